@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "elementwise.cuh"
 #include "gemm.cuh"
+#include "gemm_pair.cuh"
 #include "sampling.cuh"
 #include "draft_stream.cuh"
 
@@ -122,6 +123,19 @@ static int make_tmap(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t col
   return 0;
 }
 
+// gate | up rows [experts][2 ff, K] as {k, row of a run of 16, gate / up, run, expert}; box: 64 k x 16 rows x both x 4 runs
+static int make_tmap_glu(CUtensorMap* tm, const void* ptr, int64_t ff, int64_t K, int64_t experts) {
+  CKI(get_encode());
+  if (K % 8 != 0 || ff % kPairGluRun != 0 || ((uintptr_t)ptr & 15) != 0) return fail("TMA: gate | up rows of %lld x %lld", (long long)ff, (long long)K);
+  cuuint64_t gdim[5] = {(cuuint64_t)K, (cuuint64_t)kPairGluRun, 2, (cuuint64_t)(ff / kPairGluRun), (cuuint64_t)experts};
+  cuuint64_t gstride[4] = {(cuuint64_t)K * 2, (cuuint64_t)ff * K * 2, (cuuint64_t)kPairGluRun * K * 2, (cuuint64_t)2 * ff * K * 2};
+  cuuint32_t box[5] = {(cuuint32_t)kBlockK, (cuuint32_t)kPairGluRun, 2, 64 / kPairGluRun, 1}, estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = g_encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(ptr), gdim, gstride, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail("cuTensorMapEncodeTiled failed (%d) gate | up rows of %lld x %lld x %lld", (int)r, (long long)experts, (long long)ff, (long long)K);
+  return 0;
+}
+
 // ------------------------------------------------------------------------------------------
 // GEMM planning + launch
 // ------------------------------------------------------------------------------------------
@@ -191,6 +205,40 @@ static int launch_gemm(Launcher& L, int umma_n, int epi, const CUtensorMap& tmW,
   SSDK_GEMM_CASE(256, EPI_BF16) SSDK_GEMM_CASE(256, EPI_PARTIAL) SSDK_GEMM_CASE(256, EPI_SILU) SSDK_GEMM_CASE(256, EPI_GLU)
 #undef SSDK_GEMM_CASE
   return fail("no GEMM instance for umma_n=%d epi=%d", umma_n, epi);
+}
+
+// Word in host memory that a kernel sets when one of its bounded waits runs out; read after the stream has been waited for.
+static unsigned* g_wait_flag = nullptr;
+static int wait_flag(unsigned** out) {
+  if (!g_wait_flag) {
+    unsigned* f = nullptr;
+    CK(cudaHostAlloc(&f, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable));
+    *f = 0;
+    g_wait_flag = f;
+  }
+  *out = g_wait_flag;   // (unified addressing: the host pointer is the device's too)
+  return 0;
+}
+static int check_waits() {
+  if (g_wait_flag && *(volatile unsigned*)g_wait_flag) {
+    *(volatile unsigned*)g_wait_flag = 0;
+    return fail("a wait inside a GEMM ran out");
+  }
+  return 0;
+}
+
+// tile pairs of gemm_pair_kernel; p.timeout is filled in here
+static int launch_gemm_pair(Launcher& L, int epi, const CUtensorMap& tmW, const CUtensorMap& tmX, const CUtensorMap& tmXs, GemmPairParams p, int max_tiles) {
+  static bool attr_set = false;
+  if (!attr_set) {
+    CK(cudaFuncSetAttribute(gemm_pair_kernel<EPI_PARTIAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
+    CK(cudaFuncSetAttribute(gemm_pair_kernel<EPI_GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
+    attr_set = true;
+  }
+  CKI(wait_flag(&p.timeout));
+  const dim3 grid(2 * std::min(max_tiles, num_sms() / 2)), block(kPairThreads);
+  if (epi == EPI_GLU) return L.go(gemm_pair_kernel<EPI_GLU>, grid, block, (size_t)kPairSmem, tmW, tmX, tmXs, p);
+  return L.go(gemm_pair_kernel<EPI_PARTIAL>, grid, block, (size_t)kPairSmem, tmW, tmX, tmXs, p);
 }
 
 struct WeightMat {

@@ -68,6 +68,7 @@ struct ssdk_hyb_engine {
   bool use_tc_scores = true;    // score GEMM of latent-attention portions on the tcgen05 GEMM (SSDK_HYB_TC_SCORES=0: mma.sync tile)
   bool use_gqa_mma = true;      // grouped-query attention on the tensor cores (SSDK_HYB_GQA_MMA=0: GEMMs around a softmax, CUDA-core decode)
   bool use_tc_glu = true;       // gated feed-forward's activation in the epilogue of the tcgen05 GEMM (SSDK_HYB_TC_GLU=0: a kernel of its own)
+  int use_pair = 1;             // calls with many rows on the two-CTA GEMM: 1 by the rule of pair_ok, 2 wherever it can run, 0 never (SSDK_HYB_PAIR)
   bool use_retention_mma = true; // retention's chunks on the tensor cores (SSDK_HYB_RETENTION_MMA=0: fp32 FMA)
   bool use_decode_mma = true;   // its tensor-core form for bf16 storage (SSDK_HYB_DECODE_MMA=0: the CUDA-core form)
   std::map<std::tuple<const void*, int64_t, int, int, int>, CUtensorMap> tmaps;
@@ -79,6 +80,19 @@ struct ssdk_hyb_engine {
       if (tmaps.size() >= 8192) tmaps.clear();   // activations at changing offsets / row counts: keep the table bounded
       CUtensorMap tm;
       CKI(make_tmap(&tm, ptr, rows, K, box_rows, ld));
+      it = tmaps.emplace(key, tm).first;
+    }
+    *out = &it->second;
+    return 0;
+  }
+  // gate | up rows of `experts` matrices (keyed like a plain map, with the negative expert count for the box rows)
+  int tmap_glu(const void* ptr, int ff, int K, int experts, const CUtensorMap** out) {
+    auto key = std::make_tuple(ptr, (int64_t)2 * ff * experts, K, -experts, ff);
+    auto it = tmaps.find(key);
+    if (it == tmaps.end()) {
+      if (tmaps.size() >= 8192) tmaps.clear();
+      CUtensorMap tm;
+      CKI(make_tmap_glu(&tm, ptr, ff, K, experts));
       it = tmaps.emplace(key, tm).first;
     }
     *out = &it->second;
@@ -369,7 +383,30 @@ struct HybRun {
     return std::is_same<T, bf16>::value && e->use_tc && K % kBlockK == 0 && lda == K && ldw >= K && ldw % 8 == 0 && ldc == N &&
            ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
   }
+  // three quarters of a tile's tokens and more: below, a narrow tile streams the weights as well and split-K fills more SMs.  Measured on
+  // whole prompts (size s, m; us, one-CTA form -> pairs): 130 rows 712 -> 678, 1110 -> 1147; 200 rows 760 -> 713, 1213 -> 1193;
+  // 1024 rows 1076 -> 950, 1782 -> 1555
+  bool pair_ok(int m_total) const { return e->use_pair > 1 || (e->use_pair && m_total >= 192); }
+  // fills in the maps and launches: W holds `experts` matrices of w_rows rows (gated: gate rows, then as many up rows)
+  int go_pair(bool glu, const void* A, const void* W, int rows, int w_rows, int experts, int K, int ldw, GemmPairParams& p, int row_tiles) {
+    const CUtensorMap* tm;   // (copied: a later lookup may empty the table)
+    if (glu) CKI(e->tmap_glu(W, w_rows / 2, K, experts, &tm));
+    else CKI(e->tmap(W, (int64_t)experts * w_rows, K, 128, &tm, ldw == K ? 0 : ldw));
+    const CUtensorMap tmW = *tm;
+    CKI(e->tmap(A, rows, K, kPairXBox, &tm));
+    const CUtensorMap tmX = *tm;
+    CKI(e->tmap(A, rows, K, kPairXSmall, &tm));
+    const CUtensorMap tmXs = *tm;
+    p.N = p.ldo = glu ? w_rows / 2 : w_rows; p.num_kb = K / kBlockK; p.w_tiles = glu ? (p.N + 127) / 128 : (p.N + 255) / 256;
+    return launch_gemm_pair(L, glu ? EPI_GLU : EPI_PARTIAL, tmW, tmX, tmXs, p, p.w_tiles * row_tiles);
+  }
+  int lin_pair(bool glu, const void* A, const void* W, void* C, int m_total, int w_rows, int K, int ldw, bool gelu) {
+    GemmPairParams p = {};
+    p.out = C; p.M = m_total; p.chunks = (m_total + kPairTokens - 1) / kPairTokens; p.glu_gelu = gelu;
+    return go_pair(glu, A, W, m_total, w_rows, 1, K, ldw, p, p.chunks);
+  }
   int lin_tc(const void* A, const void* W, float* C, int m_total, int N, int K, int ldw) {
+    if (pair_ok(m_total)) return lin_pair(false, A, W, C, m_total, N, K, ldw, false);
     const CUtensorMap* tm;   // (copied: a later lookup may empty the table)
     CKI(e->tmap(W, N, K, 64, &tm, ldw == K ? 0 : ldw));
     const CUtensorMap tmW = *tm;
@@ -400,6 +437,7 @@ struct HybRun {
   }
   // y [m, ff] (bf16) = act(x Wg^T) * (x Wu^T) in the GEMM's epilogue; W holds the gate rows, then the up rows
   int lin_tc_glu(const void* A, const void* W, void* y, int m_total, int ff, int K, bool gelu) {
+    if (ff % kPairGluRun == 0 && pair_ok(m_total)) return lin_pair(true, A, W, y, m_total, 2 * ff, K, K, gelu);
     const CUtensorMap* tm;
     CKI(e->tmap(W, 2 * ff, K, 64, &tm));
     const CUtensorMap tmW = *tm;
@@ -415,6 +453,12 @@ struct HybRun {
   // C[r, :] = X[r, :] Wm[expert(r)]^T with Wm the experts' [N, K] matrices stacked by rows; glu: N holds gate rows, then as many up rows,
   // and C [rows, N / 2] (bf16) is silu(gate) * up
   int lin_tc_grouped(const void* X, const void* Wm, void* C, int rows, int N, int K, int n_experts, int un, int max_tiles, bool glu = false) {
+    if (un == kPairTokens) {
+      GemmPairParams p = {};
+      p.out = C; p.M = rows; p.g_expert_rows = N;
+      p.g_tile_expert = e->tile_expert; p.g_tile_row0 = e->tile_row0; p.g_tile_rows = e->tile_rows; p.g_n_tiles = e->n_tiles;
+      return go_pair(glu, X, Wm, rows, N, n_experts, K, K, p, max_tiles);
+    }
     const CUtensorMap* tm;
     CKI(e->tmap(Wm, (int64_t)n_experts * N, K, 64, &tm));
     const CUtensorMap tmW = *tm;
@@ -743,7 +787,7 @@ struct HybRun {
     const bool tc_moe = !kF32 && e->use_tc && e->use_tc_experts && A >= 256 && W % kBlockK == 0 && ff % kBlockK == 0 &&
                         (((uintptr_t)Lr.t[SSDK_HT_EXPERT_IN].p | (uintptr_t)Lr.t[SSDK_HT_EXPERT_OUT].p) & 15) == 0;
     const bool silu_glu = c.expert_glu && c.expert_act == SSDK_ACT_SILU, glu = tc_moe && silu_glu && e->use_tc_glu;   // activation in the GEMM's epilogue
-    const int tile = tc_moe ? 128 : ssdk::kLinBM;
+    const int tile = !tc_moe ? ssdk::kLinBM : (pair_ok(M) && (!glu || ff % kPairGluRun == 0) ? kPairTokens : 128);
     ssdk::PlanArgs pa;
     pa.sel = e->sel; pa.apos = e->apos; pa.arow = e->arow; pa.tile_expert = e->tile_expert; pa.tile_row0 = e->tile_row0;
     pa.tile_rows = e->tile_rows; pa.n_tiles = e->n_tiles; pa.n_rows = e->n_rows; pa.A = A; pa.E = Et; pa.top = top; pa.tile = tile;
@@ -1573,7 +1617,7 @@ static int hyb_forward_t(ssdk_hyb_engine* e, int n_seqs, int M, const int32_t* i
   }
   e->launches += run.L.count;
   CK(cudaStreamSynchronize(st));
-  return 0;
+  return check_waits();
 }
 
 extern "C" {
@@ -1597,6 +1641,7 @@ int ssdk_hyb_create(const ssdk_hyb_cfg* cfg, const ssdk_hyb_layer_cfg* layers, s
   e->cfg = *cfg;
   e->esz = cfg->dtype == SSDK_DT_BF16 ? 2 : 4;
   e->use_tc = env_int("SSDK_HYB_TCGEN05", 1) != 0;
+  e->use_pair = env_int("SSDK_HYB_PAIR", 1);
   e->use_decode_attn = env_int("SSDK_HYB_DECODE_ATTN", 1) != 0;
   e->use_decode_mma = env_int("SSDK_HYB_DECODE_MMA", 1) != 0;
   e->use_retention_mma = env_int("SSDK_HYB_RETENTION_MMA", 1) != 0;
