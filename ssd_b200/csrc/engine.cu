@@ -21,6 +21,7 @@
 #include "elementwise.cuh"
 #include "gemm.cuh"
 #include "gemm_pair.cuh"
+#include "gemm_split.cuh"
 #include "sampling.cuh"
 #include "draft_stream.cuh"
 
@@ -239,6 +240,16 @@ static int launch_gemm_pair(Launcher& L, int epi, const CUtensorMap& tmW, const 
   const dim3 grid(2 * std::min(max_tiles, num_sms() / 2)), block(kPairThreads);
   if (epi == EPI_GLU) return L.go(gemm_pair_kernel<EPI_GLU>, grid, block, (size_t)kPairSmem, tmW, tmX, tmXs, p);
   return L.go(gemm_pair_kernel<EPI_PARTIAL>, grid, block, (size_t)kPairSmem, tmW, tmX, tmXs, p);
+}
+
+static int launch_gemm_split(Launcher& L, const CUtensorMap& tmX, GemmSplitParams p, int max_tiles) {
+  static bool attr_set = false;
+  if (!attr_set) {
+    CK(cudaFuncSetAttribute(gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem));
+    attr_set = true;
+  }
+  CKI(wait_flag(&p.timeout));
+  return L.go(gemm_split_kernel, dim3(2 * std::min(max_tiles, num_sms() / 2)), dim3(kSplitThreads), (size_t)kSplitSmem, tmX, p);
 }
 
 struct WeightMat {

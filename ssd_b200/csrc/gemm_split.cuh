@@ -1,0 +1,291 @@
+// gemm_split.cuh — fp32 GEMM of the exact mode on the tensor cores: C[M, N] = X[M, K] · W[N, K]^T with fp32 operands and results at the
+// accuracy of a chain of fp32 FMAs.
+//
+// Every operand is the sum of three bf16 pieces, x = h + m + l (8 significant bits each, what is left over is below 2^-27 of x), and
+// a product is taken as hh + (hm + mh + mm + hl + lh): six tcgen05.mma of kind::f16 whose products are exact; the terms that are left out
+// are below 2^-26.  The tensor core truncates when it adds to its fp32 accumulator: measured against 64 bits (random signs) 2.2e-7 of
+// the result over 256 steps of k but 2.1e-6 over 2048, where a chain of FMAs is off by 1.0e-7 and 3.8e-7.  So the hh sums leave TMEM every
+// 256 k and are added up in registers (fp32, round to nearest); the five small terms, 2^-8 of the result, stay in an accumulator of
+// their own up to the end.  Relative error of 1000 x 4096 x 2048 against 64 bits: 2.4e-7, the FMA form 7.9e-7.  An infinite operand
+// gives NaN (inf - inf between its pieces).
+//
+// What bounds it: the tensor core, 24 products of 64 clocks per k-block of 64 and 128 tokens, under which everything else hides.  The
+// FMA form it takes over from (linear_kernel, 64 x 64 tiles) was bound by its shared-memory operands: 1000 x 4096 x 2048 539 us (31 TFLOP/s)
+// -> 145 us (115), 2000 x 8192 x 2048 2092 -> 459 us; with few rows the kernel streams the weights (8 x 8192 x 2048 148 -> 50 us), which is
+// why the tokens of a tile go down to 32.  Pairs of CTAs and the persistent walk as in
+// gemm_pair.cuh; the weights are read as fp32 and split on their way into shared memory (6 bytes in memory for every 4 would cost more
+// than the conversion, which needs 40 % of the issue slots), the rows of X, read by every tile, are split beforehand.
+//   warp 0      loads: the three pieces of this CTA's token half (64 rows x 64 k each)
+//   warp 1      leader only: the products
+//   warps 2-5   sums: thread = output column, up to 128 tokens in registers
+//   warps 6-9   weights: 128 rows x 64 k of fp32, the next k-block's loads in flight while this one is split and stored (128B swizzle)
+#pragma once
+#include "gemm_pair.cuh"
+
+namespace ssdk {
+
+constexpr int kSplitTokens = 128, kSplitStages = 3, kSplitThreads = 320, kSplitSegment = 4;   // segment: k-blocks between two drains
+constexpr int kSplitWPlane = 128 * 128, kSplitXPlane = 64 * 128, kSplitStageBytes = 3 * (kSplitWPlane + kSplitXPlane);
+constexpr int kSplitSmem = kSplitStages * kSplitStageBytes + 1024;
+
+struct GemmSplitParams {
+  const float* W;     // [N, ldw]
+  float* out;         // [splits][M, ldc]
+  int M, N, K, ldw, ldc;
+  int num_kb, kb_per_split, splits;
+  int w_tiles, chunks;        // tiles of 256 columns; chunks of kSplitTokens rows (dense)
+  int batch;                  // dense: products of the same shape, their weights and results w_stride and c_stride floats apart, X's rows in turn
+  int plane_rows;             // rows of one piece of X (the map holds three of them)
+  long long w_stride, c_stride;   // grouped: w_stride between two experts
+  const int* g_tile_expert;   // grouped mode: see GemmParams (tiles of up to kSplitTokens rows)
+  const int* g_tile_row0;
+  const int* g_tile_rows;
+  const int* g_n_tiles;
+  unsigned* timeout;
+};
+
+// two floats -> their three bf16 pieces, packed
+SSDK_DEVINL void split3(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
+  const __nv_bfloat162 hh = __floats2bfloat162_rn(a, b);
+  const float2 hf = __bfloat1622float2(hh);
+  const float a1 = a - hf.x, b1 = b - hf.y;
+  const __nv_bfloat162 mm = __floats2bfloat162_rn(a1, b1);
+  const float2 mf = __bfloat1622float2(mm);
+  const __nv_bfloat162 ll = __floats2bfloat162_rn(a1 - mf.x, b1 - mf.y);
+  h = *reinterpret_cast<const uint32_t*>(&hh);
+  m = *reinterpret_cast<const uint32_t*>(&mm);
+  l = *reinterpret_cast<const uint32_t*>(&ll);
+}
+
+// rows of X as three pieces: dst [3][batch * M, K] (bf16).  grid (M, batch): row r of matrix b (`stride` floats apart) is row rows[r] of src
+// if there is a list; rows from *n_rows on are left out
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ src, int ld, long long stride, const int* __restrict__ rows,
+                                                         const int* __restrict__ n_rows, __nv_bfloat16* __restrict__ dst, int K) {
+  const int r = blockIdx.x;
+  if (n_rows && r >= *n_rows) return;
+  const float4* s = reinterpret_cast<const float4*>(src + blockIdx.y * stride + (size_t)(rows ? rows[r] : r) * ld);
+  const size_t plane = (size_t)gridDim.x * gridDim.y * K;
+  __nv_bfloat16* d = dst + ((size_t)blockIdx.y * gridDim.x + r) * K;
+  for (int c = threadIdx.x; c < K / 4; c += blockDim.x) {
+    const float4 v = s[c];
+    uint2 h, m, l;
+    split3(v.x, v.y, h.x, m.x, l.x);
+    split3(v.z, v.w, h.y, m.y, l.y);
+    reinterpret_cast<uint2*>(d)[c] = h;
+    reinterpret_cast<uint2*>(d + plane)[c] = m;
+    reinterpret_cast<uint2*>(d + 2 * plane)[c] = l;
+  }
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSplitThreads, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams p) {
+  extern __shared__ uint8_t split_smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[kSplitStages];   // the leader's are used: the loads' bytes and four weight warps of both CTAs
+  __shared__ __align__(8) uint64_t empty_bar[kSplitStages];
+  __shared__ __align__(8) uint64_t main_full[2], main_empty[2], rest_full[2], rest_empty[2];
+  __shared__ uint32_t tmem_slot;
+  uint8_t* smem = split_smem_raw + ((1024u - (smem_u32(split_smem_raw) & 1023u)) & 1023u);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int pair = (int)blockIdx.x >> 1, n_pairs = (int)gridDim.x >> 1;
+
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmX);
+    for (int s = 0; s < kSplitStages; ++s) { mbar_init(&full_bar[s], 9); mbar_init(&empty_bar[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&main_full[b], 1); mbar_init(&main_empty[b], 8); mbar_init(&rest_full[b], 1); mbar_init(&rest_empty[b], 8); }
+    fence_mbar_init();
+  }
+  if (warp == 1) tmem_alloc_pair(&tmem_slot);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after();
+  const uint32_t tmem_main = tmem_slot, tmem_rest = tmem_slot + 256u;   // two accumulators of 128 columns each
+
+  pdl_launch_dependents();
+  pdl_wait();
+
+  const bool grouped = p.g_tile_expert != nullptr;
+  const int row_tiles = grouped ? *p.g_n_tiles : p.chunks;
+  const int per = row_tiles * p.splits * p.w_tiles, tiles = grouped ? per : per * p.batch;
+  struct Tile { int m0, rows, n, col, kb0, kb1, split, b; long long w0; };
+  auto tile_of = [&](int t) {   // row chunk (innermost), k range, 256 columns, matrix of the batch
+    Tile r;
+    r.b = grouped ? 0 : t / per;
+    t -= r.b * per;
+    const int u = t / row_tiles, c = t - u * row_tiles, wt = u / p.splits;
+    r.split = u - wt * p.splits;
+    if (grouped) {
+      r.m0 = p.g_tile_row0[c]; r.rows = min(kSplitTokens, p.g_tile_rows[c]); r.w0 = p.g_tile_expert[c] * p.w_stride;
+    } else {
+      r.m0 = c * kSplitTokens; r.rows = min(kSplitTokens, p.M - r.m0); r.w0 = r.b * p.w_stride;
+    }
+    r.n = (r.rows + 31) & ~31;
+    r.col = wt * 256 + (int)rank * 128;
+    r.kb0 = r.split * p.kb_per_split;
+    r.kb1 = min(p.num_kb, r.kb0 + p.kb_per_split);
+    return r;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      bool ok = true;
+      for (int t = pair; t < tiles && ok; t += n_pairs) {
+        const Tile tl = tile_of(t);
+        const int x0 = tl.b * p.M + tl.m0 + (int)rank * (tl.n >> 1);
+        for (int kb = tl.kb0; kb < tl.kb1; ++kb, ++it) {
+          const int s = it % kSplitStages;
+          if (!(ok = mbar_wait_cluster(&empty_bar[s], ((uint32_t)(it / kSplitStages) & 1u) ^ 1u, p.timeout))) break;
+          uint8_t* b_s = smem + s * kSplitStageBytes + 3 * kSplitWPlane;
+          if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2u * 3u * kSplitXPlane);
+          const uint32_t bar = map_shared(&full_bar[s], 0);
+#pragma unroll
+          for (int j = 0; j < 3; ++j) tma_load_2d_pair(b_s + j * kSplitXPlane, &tmX, bar, kb * kBlockK, j * p.plane_rows + x0, kEvictNormal);
+        }
+      }
+      for (int i = 0; i < kSplitStages && ok; ++i, ++it)   // the last commits reach this CTA before it leaves
+        ok = mbar_wait_cluster(&empty_bar[it % kSplitStages], ((uint32_t)(it / kSplitStages) & 1u) ^ 1u, p.timeout);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      int it = 0, nt = 0, sg = 0;
+      bool ok = true;
+      for (int t = pair; t < tiles && ok; t += n_pairs, ++nt) {
+        const Tile tl = tile_of(t);
+        const uint32_t idesc = make_umma_idesc_bf16(256, tl.n), rest = tmem_rest + (uint32_t)(nt & 1) * 128u;
+        if (!(ok = mbar_wait_cluster(&rest_empty[nt & 1], ((uint32_t)(nt >> 1) & 1u) ^ 1u, p.timeout))) break;
+        for (int kb = tl.kb0; kb < tl.kb1; ++kb, ++it) {
+          const int in_seg = (kb - tl.kb0) % kSplitSegment;
+          if (in_seg == 0 && !(ok = mbar_wait_cluster(&main_empty[sg & 1], ((uint32_t)(sg >> 1) & 1u) ^ 1u, p.timeout))) break;
+          const int s = it % kSplitStages;
+          if (!(ok = mbar_wait_cluster(&full_bar[s], (uint32_t)(it / kSplitStages) & 1u, p.timeout))) break;
+          tc_fence_after();
+          uint8_t* a_s = smem + s * kSplitStageBytes;
+          uint64_t wd[3], xd[3];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) { wd[j] = make_umma_desc_k128(a_s + j * kSplitWPlane); xd[j] = make_umma_desc_k128(a_s + 3 * kSplitWPlane + j * kSplitXPlane); }
+          const uint32_t acc = tmem_main + (uint32_t)(sg & 1) * 128u;
+#pragma unroll
+          for (int k = 0; k < kBlockK / 16; ++k) {
+            const uint64_t o = (uint64_t)(2 * k);
+            umma_bf16_ss_pair(acc, wd[0] + o, xd[0] + o, idesc, (uint32_t)((in_seg | k) != 0));
+            umma_bf16_ss_pair(rest, wd[0] + o, xd[1] + o, idesc, (uint32_t)(((kb - tl.kb0) | k) != 0));
+            umma_bf16_ss_pair(rest, wd[1] + o, xd[0] + o, idesc, 1u);
+            umma_bf16_ss_pair(rest, wd[1] + o, xd[1] + o, idesc, 1u);
+            umma_bf16_ss_pair(rest, wd[0] + o, xd[2] + o, idesc, 1u);
+            umma_bf16_ss_pair(rest, wd[2] + o, xd[0] + o, idesc, 1u);
+          }
+          umma_commit_pair(&empty_bar[s]);
+          if (in_seg == kSplitSegment - 1 || kb + 1 == tl.kb1) { umma_commit_pair(&main_full[sg & 1]); ++sg; }
+        }
+        if (ok) umma_commit_pair(&rest_full[nt & 1]);
+      }
+    }
+    __syncwarp();
+  } else if (warp < 6) {
+    const int q = warp & 3;
+    int nt = 0, sg = 0;
+    bool ok = true;
+    for (int t = pair; t < tiles && ok; t += n_pairs, ++nt) {
+      const Tile tl = tile_of(t);
+      float acc[kSplitTokens];
+#pragma unroll
+      for (int m = 0; m < kSplitTokens; ++m) acc[m] = 0.f;
+      auto add = [&](uint32_t src) {
+        src += (uint32_t)(q * 32) << 16;
+#pragma unroll
+        for (int c = 0; c < kSplitTokens / 32; ++c) {
+          if (c * 32 < tl.n) {
+            uint32_t r[32];
+            tmem_ld_32x32b_x16(src + c * 32, r);
+            tmem_ld_32x32b_x16(src + c * 32 + 16, r + 16);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) acc[c * 32 + i] += __uint_as_float(r[i]);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+      };
+      const int segs = (tl.kb1 - tl.kb0 + kSplitSegment - 1) / kSplitSegment;
+      for (int g = 0; g < segs; ++g, ++sg) {
+        if (!(ok = mbar_wait_cluster(&main_full[sg & 1], (uint32_t)(sg >> 1) & 1u, p.timeout))) break;
+        tc_fence_after();
+        add(tmem_main + (uint32_t)(sg & 1) * 128u);
+        if (lane == 0) mbar_arrive_cluster(map_shared(&main_empty[sg & 1], 0));
+      }
+      if (!ok || !(ok = mbar_wait_cluster(&rest_full[nt & 1], (uint32_t)(nt >> 1) & 1u, p.timeout))) break;
+      tc_fence_after();
+      add(tmem_rest + (uint32_t)(nt & 1) * 128u);
+      if (lane == 0) mbar_arrive_cluster(map_shared(&rest_empty[nt & 1], 0));
+      const int n = tl.col + q * 32 + lane;
+      if (n < p.N) {
+        float* out = p.out + tl.b * p.c_stride + ((size_t)tl.split * p.M + tl.m0) * p.ldc + n;
+#pragma unroll
+        for (int m = 0; m < kSplitTokens; ++m)
+          if (m < tl.rows) out[(size_t)m * p.ldc] = acc[m];
+      }
+    }
+    __syncwarp();
+  } else {
+    // lane: row lane / 8 of four, eight floats from column 8 (lane % 8) of the k-block; eight steps cover the warp's 32 rows
+    const int cw = warp - 6, r4 = lane >> 3, piece = lane & 7;
+    float4 v[16];
+    auto load = [&](const Tile& tl, int kb, int i) {
+      const int row = tl.col + cw * 32 + i * 4 + r4, k = kb * kBlockK + piece * 8;
+      const bool in = row < p.N && k < p.K;
+      const float4* src = reinterpret_cast<const float4*>(p.W + tl.w0 + (long long)row * p.ldw + k);
+      v[2 * i] = in ? __ldg(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[2 * i + 1] = in ? __ldg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    int it = 0, t = pair, kb = 0;
+    Tile tl = {};
+    if (t < tiles) {
+      tl = tile_of(t);
+      kb = tl.kb0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) load(tl, kb, i);
+    }
+    bool ok = true;
+    while (t < tiles && ok) {
+      Tile nx = tl;   // the k-block after this one
+      int t2 = t, kb2 = kb + 1;
+      if (kb2 >= tl.kb1) {
+        t2 += n_pairs;
+        if (t2 < tiles) { nx = tile_of(t2); kb2 = nx.kb0; }
+      }
+      const int s = it % kSplitStages;
+      if (!(ok = mbar_wait_cluster(&empty_bar[s], ((uint32_t)(it / kSplitStages) & 1u) ^ 1u, p.timeout))) break;
+      uint8_t* a_s = smem + s * kSplitStageBytes;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int row = cw * 32 + i * 4 + r4;
+        uint4 h, m, l;
+        split3(v[2 * i].x, v[2 * i].y, h.x, m.x, l.x);
+        split3(v[2 * i].z, v[2 * i].w, h.y, m.y, l.y);
+        split3(v[2 * i + 1].x, v[2 * i + 1].y, h.z, m.z, l.z);
+        split3(v[2 * i + 1].z, v[2 * i + 1].w, h.w, m.w, l.w);
+        uint8_t* dst = a_s + row * 128 + ((piece ^ (row & 7)) << 4);
+        *reinterpret_cast<uint4*>(dst) = h;
+        *reinterpret_cast<uint4*>(dst + kSplitWPlane) = m;
+        *reinterpret_cast<uint4*>(dst + 2 * kSplitWPlane) = l;
+        if (t2 < tiles) load(nx, kb2, i);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(map_shared(&full_bar[s], 0));
+      ++it; t = t2; kb = kb2; tl = nx;
+    }
+    __syncwarp();
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  if (warp == 1) tmem_dealloc_pair(tmem_slot);
+}
+
+}  // namespace ssdk

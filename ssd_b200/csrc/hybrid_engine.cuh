@@ -69,6 +69,8 @@ struct ssdk_hyb_engine {
   bool use_gqa_mma = true;      // grouped-query attention on the tensor cores (SSDK_HYB_GQA_MMA=0: GEMMs around a softmax, CUDA-core decode)
   bool use_tc_glu = true;       // gated feed-forward's activation in the epilogue of the tcgen05 GEMM (SSDK_HYB_TC_GLU=0: a kernel of its own)
   int use_pair = 1;             // calls with many rows on the two-CTA GEMM: 1 by the rule of pair_ok, 2 wherever it can run, 0 never (SSDK_HYB_PAIR)
+  int use_split = 1;            // fp32 storage: products in three bf16 pieces: 1 by the rule of split_ok, 2 wherever it can run, 0 never (SSDK_HYB_SPLIT)
+  void* pieces = nullptr; size_t piece_elems = 0;   // the pieces of X's rows (three bf16 per element)
   bool use_retention_mma = true; // retention's chunks on the tensor cores (SSDK_HYB_RETENTION_MMA=0: fp32 FMA)
   bool use_decode_mma = true;   // its tensor-core form for bf16 storage (SSDK_HYB_DECODE_MMA=0: the CUDA-core form)
   std::map<std::tuple<const void*, int64_t, int, int, int>, CUtensorMap> tmaps;
@@ -350,11 +352,16 @@ static int64_t hyb_carve(ssdk_hyb_engine* e, uint8_t* base) {
   e->temps = (float*)take(lr * 4);
   e->meta_ints = 2 * cap + 3 * (size_t)g.max_seqs + 1 + (size_t)g.max_seqs * g.max_blocks_per_seq + lr;
   e->meta = (int*)take(e->meta_ints * 4);
-  // split-K partials of the tcgen05 GEMM: up to 8 splits of a 256-row call of the widest output, bounded at 64 MB
+  // split-K partials of the tcgen05 GEMMs: up to 8 splits of a 256-row call of the widest output, bounded at 64 MB
   size_t widest = std::max<size_t>(g.vocab, g.width);
   for (int w : {e->w_p0, e->w_p1, e->w_sff2, one_norm ? 2 * g.width : 0}) widest = std::max<size_t>(widest, (size_t)w);
-  e->partial_floats = es == 2 ? std::min<size_t>(8 * std::min<size_t>(cap, 256) * widest, 16u << 20) : 0;
+  e->partial_floats = std::min<size_t>(8 * std::min<size_t>(cap, 256) * widest, 16u << 20);
   e->partials = (float*)take(e->partial_floats * 4);
+  if (es == 4) {   // the widest rows that a product reads, and one block of attention weights
+    size_t wide = std::max<size_t>({(size_t)g.width, (size_t)e->w_p1, (size_t)e->w_p2, (size_t)e->w_t0, (size_t)e->w_t1, (size_t)e->w_qcat, (size_t)e->w_sff});
+    e->piece_elems = std::max({cap * wide, A * (size_t)std::max(g.width, e->w_ff), e->att_elems, lr * (size_t)g.width});
+  }
+  e->pieces = take(e->piece_elems * 6);
   return (int64_t)off;
 }
 
@@ -475,10 +482,55 @@ struct HybRun {
     }
     return launch_gemm(L, un, EPI_PARTIAL, tmW, tmX, p, (N + kTileRows - 1) / kTileRows, 1, max_tiles);
   }
+  // ---- fp32 storage: products on the tensor cores in three bf16 pieces (gemm_split.cuh) ----
+  // Worth it from about 0.4 GFLOP (13 us of the FMA form) or K = 512 (36 us, whatever the rows): below, splitting the rows costs a launch
+  // and a pair of CTAs takes 15 us to start and drain.  us, FMA form -> this one with its split: 8 x 2048 x 2048 150 -> 30, 8 x 8192 x 2048
+  // 148 -> 56, 1000 x 4096 x 2048 539 -> 156, 2000 x 8192 x 2048 2092 -> 472; 33 x 512 x 200 19 -> 25
+  bool split_ok(const void* A, int lda, const void* W, int ldw, int m, int N, int K, int batch, long long sA, long long sW) const {
+    if (!kF32 || !e->use_split || K % 8 || lda % 4 || ldw % 4 || sA % 4 || sW % 4 || (((uintptr_t)A | (uintptr_t)W) & 15)) return false;
+    if ((size_t)m * batch * K > e->piece_elems || batch > 65535) return false;
+    return e->use_split > 1 || 2.0 * m * N * K * batch >= 4e8 || K >= 512;
+  }
+  int go_split(const void* A, int lda, long long sA, const int* gather, const int* n_rows, int m, int batch, GemmSplitParams& p, int row_tiles) {
+    CKI(L.go(ssdk::split_rows_kernel, dim3(m, batch), dim3(std::min(256, (p.K / 4 + 31) / 32 * 32)), 0, (const float*)A, lda, sA, gather, n_rows, (bf16*)e->pieces, p.K));
+    const CUtensorMap* tm;
+    CKI(e->tmap(e->pieces, 3LL * m * batch, p.K, 64, &tm));
+    p.M = m; p.plane_rows = m * batch; p.batch = batch; p.num_kb = (p.K + kBlockK - 1) / kBlockK; p.w_tiles = (p.N + 255) / 256;
+    const int tiles = p.w_tiles * row_tiles * batch;
+    // few tiles: k ranges of whole segments (dense results only; summed in the order of the ranges)
+    int S = 1;
+    if (!p.g_tile_expert && batch == 1 && p.ldc == p.N) {
+      S = std::max(1, std::min({num_sms() / 2 / tiles, p.num_kb / kSplitSegment, 8}));
+      while (S > 1 && (size_t)S * m * p.N > e->partial_floats) --S;
+    }
+    p.kb_per_split = ((p.num_kb + S - 1) / S + kSplitSegment - 1) / kSplitSegment * kSplitSegment;
+    p.splits = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;
+    float* C = p.out;
+    if (p.splits > 1) p.out = e->partials;
+    CKI(launch_gemm_split(L, *tm, p, tiles * p.splits));
+    if (p.splits > 1) {
+      const size_t n = (size_t)m * p.N;
+      CKI(L.go(ssdk::splitk_sum_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, (const float*)e->partials, C, p.splits, n));
+    }
+    return 0;
+  }
+  // C[r, :] = X[r, :] Wm[expert(r)]^T for the real experts' rows; X's rows through `gather` if given
+  int split_grouped(const void* X, int ldx, const int* gather, const void* Wm, float* C, int rows, int N, int K, int max_tiles) {
+    GemmSplitParams p = {};
+    p.W = (const float*)Wm; p.out = C; p.N = p.ldc = N; p.K = p.ldw = K; p.w_stride = (long long)N * K;
+    p.g_tile_expert = e->tile_expert; p.g_tile_row0 = e->tile_row0; p.g_tile_rows = e->tile_rows; p.g_n_tiles = e->n_tiles;
+    return go_split(X, ldx, 0, gather, e->n_rows, rows, 1, p, max_tiles);
+  }
   // C[M, N] (fp32 unless out_t) = A[M, K] W[N, K]^T
   int lin(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int m, int N, int K, bool out_t = false,
           int batch = 1, long long sA = 0, long long sW = 0, long long sC = 0, bool allow_tc = true) {
     if (allow_tc && !out_t && batch == 1 && tc_ok(A, lda, W, ldw, ldc, N, K)) return lin_tc(A, W, (float*)C, m, N, K, ldw);
+    if (split_ok(A, lda, W, ldw, m, N, K, batch, sA, sW)) {
+      GemmSplitParams p = {};
+      p.W = (const float*)W; p.out = (float*)C; p.N = N; p.K = K; p.ldw = ldw; p.ldc = ldc; p.w_stride = sW; p.c_stride = sC;
+      p.chunks = (m + kSplitTokens - 1) / kSplitTokens;
+      return go_split(A, lda, sA, nullptr, nullptr, m, batch, p, p.chunks);
+    }
     ssdk::LinearArgs a = {};
     a.A = A; a.W = W; a.C = C; a.M = m; a.N = N; a.K = K; a.lda = lda; a.ldw = ldw; a.ldc = ldc;
     a.sA = sA; a.sW = sW; a.sC = sC;
@@ -787,7 +839,8 @@ struct HybRun {
     const bool tc_moe = !kF32 && e->use_tc && e->use_tc_experts && A >= 256 && W % kBlockK == 0 && ff % kBlockK == 0 &&
                         (((uintptr_t)Lr.t[SSDK_HT_EXPERT_IN].p | (uintptr_t)Lr.t[SSDK_HT_EXPERT_OUT].p) & 15) == 0;
     const bool silu_glu = c.expert_glu && c.expert_act == SSDK_ACT_SILU, glu = tc_moe && silu_glu && e->use_tc_glu;   // activation in the GEMM's epilogue
-    const int tile = !tc_moe ? ssdk::kLinBM : (pair_ok(M) && (!glu || ff % kPairGluRun == 0) ? kPairTokens : 128);
+    const bool split = split_ok(fin, W, Lr.t[SSDK_HT_EXPERT_IN].p, W, A, Nin, W, 1, 0, 0) && split_ok(e->ey, ff, Lr.t[SSDK_HT_EXPERT_OUT].p, ff, A, W, ff, 1, 0, 0);
+    const int tile = split ? kSplitTokens : (!tc_moe ? ssdk::kLinBM : (pair_ok(M) && (!glu || ff % kPairGluRun == 0) ? kPairTokens : 128));
     ssdk::PlanArgs pa;
     pa.sel = e->sel; pa.apos = e->apos; pa.arow = e->arow; pa.tile_expert = e->tile_expert; pa.tile_row0 = e->tile_row0;
     pa.tile_rows = e->tile_rows; pa.n_tiles = e->n_tiles; pa.n_rows = e->n_rows; pa.A = A; pa.E = Et; pa.top = top; pa.tile = tile;
@@ -798,6 +851,8 @@ struct HybRun {
     if (tc_moe) {
       CKI(L.go(ssdk::gather_rows_kernel<T>, dim3(A), dim3(128), 0, (const T*)fin, (const int*)e->arow, (const int*)e->n_rows, (T*)e->xs, W));
       CKI(lin_tc_grouped(e->xs, Lr.t[SSDK_HT_EXPERT_IN].p, glu ? e->ey : (void*)e->eg, A, Nin, W, E, tile, A / tile + E + 1, glu));
+    } else if (split) {
+      CKI(split_grouped(fin, W, e->arow, Lr.t[SSDK_HT_EXPERT_IN].p, e->eg, A, Nin, W, A / tile + E + 1));
     } else {
       a.A = fin; a.W = Lr.t[SSDK_HT_EXPERT_IN].p; a.C = e->eg; a.M = A; a.N = Nin; a.K = W; a.lda = W; a.ldw = W; a.ldc = Nin;
       a.a_rows = e->arow; a.tile_expert = e->tile_expert; a.tile_row0 = e->tile_row0; a.tile_rows = e->tile_rows; a.n_tiles = e->n_tiles;
@@ -807,6 +862,8 @@ struct HybRun {
     if (!glu) CKI(expert_act(c, (const float*)e->eg, Nin, (T*)e->ey, ff, c.limit, A, n_real_rows));
     if (tc_moe) {
       CKI(lin_tc_grouped(e->ey, Lr.t[SSDK_HT_EXPERT_OUT].p, e->eo, A, W, ff, E, tile, A / tile + E + 1));
+    } else if (split) {
+      CKI(split_grouped(e->ey, ff, nullptr, Lr.t[SSDK_HT_EXPERT_OUT].p, e->eo, A, W, ff, A / tile + E + 1));
     } else {
       a.A = e->ey; a.W = Lr.t[SSDK_HT_EXPERT_OUT].p; a.C = e->eo; a.N = W; a.K = ff; a.lda = ff; a.ldw = ff; a.ldc = W; a.a_rows = nullptr;
       a.tile_expert = e->tile_expert; a.tile_row0 = e->tile_row0; a.tile_rows = e->tile_rows; a.n_tiles = e->n_tiles;
@@ -1642,6 +1699,7 @@ int ssdk_hyb_create(const ssdk_hyb_cfg* cfg, const ssdk_hyb_layer_cfg* layers, s
   e->esz = cfg->dtype == SSDK_DT_BF16 ? 2 : 4;
   e->use_tc = env_int("SSDK_HYB_TCGEN05", 1) != 0;
   e->use_pair = env_int("SSDK_HYB_PAIR", 1);
+  e->use_split = env_int("SSDK_HYB_SPLIT", 1);
   e->use_decode_attn = env_int("SSDK_HYB_DECODE_ATTN", 1) != 0;
   e->use_decode_mma = env_int("SSDK_HYB_DECODE_MMA", 1) != 0;
   e->use_retention_mma = env_int("SSDK_HYB_RETENTION_MMA", 1) != 0;
