@@ -60,6 +60,8 @@ SSDK_DEVINL float conv_at(const ConvArgs& p, const Ragged& rg, int m, int s, int
 // ACT: 0 none, 1 SiLU.  grid (M, ceil(C / blockDim))
 template <typename T, int ACT>
 __global__ void short_conv_kernel(const ConvArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= p.C) return;
   const int s = rg.tok_seq[m];
@@ -73,6 +75,8 @@ __global__ void short_conv_kernel(const ConvArgs p, const Ragged rg) {
 // entry j is read from an index above j, so one thread per channel may work in place in ascending order.
 template <typename T>
 __global__ void conv_state_kernel(const ConvArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= p.C) return;
   const int r0 = rg.cu[s], n = rg.cu[s + 1] - r0, keep = p.taps - 1;
@@ -103,6 +107,8 @@ struct InputConvArgs {
 // grid (M, ceil(C / blockDim)): one channel per thread, any number of taps
 template <typename T>
 __global__ void input_conv_kernel(const InputConvArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= p.C) return;
   const int s = rg.tok_seq[m], t = m - rg.cu[s];
@@ -130,6 +136,8 @@ __global__ void input_conv_kernel(const InputConvArgs p, const Ragged rg) {
 // rows and taps 16-byte aligned.  grid (M, ceil(C / VEC / blockDim)).  Same sums in the same order as the scalar form.
 template <typename T, int TAPS>
 __global__ void input_conv_vec_kernel(const InputConvArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int VEC = 16 / (int)sizeof(T);
   const int m = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
   if (c >= p.C) return;
@@ -175,6 +183,8 @@ __global__ void input_conv_vec_kernel(const InputConvArgs p, const Ragged rg) {
 // above j, so one thread per channel works in place in ascending order.
 template <typename T>
 __global__ void input_conv_state_kernel(const InputConvArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= p.C) return;
   const int r0 = rg.cu[s], n = rg.cu[s + 1] - r0, keep = p.taps - 1;
@@ -192,6 +202,8 @@ __global__ void input_conv_state_kernel(const InputConvArgs p, const Ragged rg) 
 // fp32 columns -> T columns (operand of a following linear layer)
 template <typename T>
 __global__ void cast_cols_kernel(const float* __restrict__ src, int ld_src, T* __restrict__ dst, int ld_dst, int cols) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x;
   for (int c = threadIdx.x; c < cols; c += blockDim.x) st_f<T>(dst + (size_t)m * ld_dst + c, src[(size_t)m * ld_src + c]);
 }
@@ -216,6 +228,8 @@ struct RglruArgs {
 // y[m] <- gelu_tanh(y[m] + bias)
 template <typename T>
 __global__ void rglru_gate_kernel(const RglruArgs p, float* __restrict__ gates, float* __restrict__ y) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= p.R) return;
   const int b = c / p.bs, cb = c - b * p.bs;
@@ -237,6 +251,7 @@ constexpr int kRglruRows = 16;  // rows whose operands are requested together
 // operands rglru_gate_kernel left (sixteen rows' loads in flight at a time).
 template <typename T>
 __global__ void rglru_scan_kernel(const RglruArgs p, const Ragged rg) {
+  pdl_wait();   // (no early start of the next kernel: its waiting blocks slow a chain of dependent steps down)
   const int s = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= p.R) return;
   const int b = c / p.bs, cb = c - b * p.bs;
@@ -279,6 +294,8 @@ struct SelScanArgs {
 template <typename T>
 __global__ void selective_gate_kernel(float* __restrict__ dtz, int ld_dt, const T* __restrict__ dt_bias, float* __restrict__ z, int ld_z,
                                       int inner) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= inner) return;
   float* d = dtz + (size_t)m * ld_dt + c;
@@ -296,6 +313,7 @@ constexpr int kSelRows = 8;  // rows whose inputs are requested (and whose B | C
 // lane per channel, the state stays in its slot (global memory).  dynamic shared memory: kSelRows * 2 N floats.
 template <typename T, int NT>
 __global__ void selective_scan_kernel(const SelScanArgs p, const Ragged rg) {
+  pdl_wait();   // (no early start of the next kernel: its waiting blocks slow a chain of dependent steps down)
   extern __shared__ float sel_sm[];
   const int s = blockIdx.x, lpc = blockDim.x, ln = threadIdx.x, N = p.N;
   const int c = blockIdx.y * blockDim.y + threadIdx.y, tid = threadIdx.y * lpc + ln, nthr = lpc * blockDim.y;
@@ -438,6 +456,8 @@ inline size_t delta_prep_smem(int D, int C) { return ((size_t)3 * C * D + 3 * C 
 // grid (chunks of the longest portion, n_seqs, H), 128 threads
 template <typename T, int C>
 __global__ void __launch_bounds__(128) delta_chunk_prep_kernel(const DeltaPrepArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float dp_sm[];
   constexpr int kThreads = 128, kSlices = kThreads / C;
   const int ci = blockIdx.x, s = blockIdx.y, h = blockIdx.z, t0 = ci * C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -604,6 +624,7 @@ inline size_t delta_scan_smem(int DP, int LC, int NC, int C) { return (size_t)2 
 // record arrives by cp.async under the current one's arithmetic.
 template <int LC, int NQ, int NC, int C>
 __global__ void __launch_bounds__(kDeltaWarps * 32, 1) delta_chunk_scan_kernel(const DeltaArgs p, const Ragged rg) {
+  pdl_wait();   // (no early start of the next kernel: its waiting blocks slow a chain of dependent steps down)
   extern __shared__ __align__(16) float ds_sm[];
   constexpr int DP = 4 * LC * NQ, kCols = kDeltaWarps * 32 / LC * NC, kThreads = kDeltaWarps * 32, kVals = NC * C;
   constexpr int kRec = (3 * C + 1) * DP + (C > 1 ? 2 * C * C : 4), kBuf = kRec + C * kCols;
@@ -801,6 +822,7 @@ __global__ void __launch_bounds__(kDeltaWarps * 32, 1) delta_chunk_scan_kernel(c
 // Any D: one thread per column, the column in shared memory ([D][blockDim], dynamic), records of single rows (C = 1) read from
 // global memory.  grid (n_seqs, H, ceil(V / blockDim))
 __global__ void delta_scan_any_kernel(const DeltaArgs p, const Ragged rg) {
+  pdl_wait();   // (no early start of the next kernel: its waiting blocks slow a chain of dependent steps down)
   extern __shared__ __align__(16) float ds_sm[];
   const int s = blockIdx.x, hd = blockIdx.y, jl = threadIdx.x, Vr = blockDim.x, j = blockIdx.z * Vr + jl;
   const int D = p.D, V = p.V, DP = p.DP, kRec = delta_record(DP, 1);
@@ -830,6 +852,8 @@ __global__ void delta_scan_any_kernel(const DeltaArgs p, const Ragged rg) {
 // fp32 columns [c0, c0 + n1) and [c0 + n1, c0 + n1 + n2) of each row -> two dense T matrices (operands of two linear layers)
 template <typename T>
 __global__ void cast_split_kernel(const float* __restrict__ src, int ld_src, T* __restrict__ d1, int n1, T* __restrict__ d2, int n2) {
+  pdl_launch_dependents();
+  pdl_wait();
   const float* r = src + (size_t)blockIdx.x * ld_src;
   for (int c = threadIdx.x; c < n1 + n2; c += blockDim.x) {
     if (c < n1) st_f<T>(d1 + (size_t)blockIdx.x * n1 + c, r[c]);

@@ -61,6 +61,8 @@ SSDK_DEVINL void split3(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l)
 // if there is a list; rows from *n_rows on are left out
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ src, int ld, long long stride, const int* __restrict__ rows,
                                                          const int* __restrict__ n_rows, __nv_bfloat16* __restrict__ dst, int K) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int r = blockIdx.x;
   if (n_rows && r >= *n_rows) return;
   const float4* s = reinterpret_cast<const float4*>(src + blockIdx.y * stride + (size_t)(rows ? rows[r] : r) * ld);

@@ -40,6 +40,8 @@ struct GqaPrepArgs {
 // grid (M, H + G), one warp: units 0 .. H-1 are query heads, H .. H+G-1 key heads (which also copy their value head)
 template <typename T>
 __global__ void gqa_prep_kernel(const GqaPrepArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x, unit = blockIdx.y, lane = threadIdx.x, s = rg.tok_seq[m];
   const int pos = rg.pos0[s] + (m - rg.cu[s]);
   const int H = p.H, G = p.G, D = p.D, V = p.V;
@@ -134,6 +136,8 @@ SSDK_DEVINL void conv_group(const ConvArgs& p, const Ragged& rg, int m, int s, i
 // VEC = 4: as conv_group, and D, V and the rotated part are multiples of 4 with adjacent pairs.
 template <typename T, int VEC, int TAPS>
 __global__ void gqa_conv_prep_kernel(const GqaConvPrepArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float gc_sm[];
   __shared__ float red[33];
   const int m = blockIdx.x, s = rg.tok_seq[m], t = m - rg.cu[s], pos = rg.pos0[s] + t;
@@ -255,6 +259,8 @@ struct GqaHeadPrepArgs {
 // rot_dims floats
 template <typename T, int VEC, int LANES>
 __global__ void gqa_head_prep_kernel(const GqaHeadPrepArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   SSDK_DYN_SMEM(float, hp_cs);
   const int m = blockIdx.x, s = rg.tok_seq[m], pos = rg.pos0[s] + (m - rg.cu[s]), lane = threadIdx.x & (LANES - 1);
   const int H = p.g.H, G = p.g.G, Gv = G / p.maps, D = p.g.D, V = p.g.V, hpg = H / G, half = (p.g.inv_freq ? p.g.rot_dims : 0) >> 1;
@@ -302,6 +308,8 @@ __global__ void gqa_head_prep_kernel(const GqaHeadPrepArgs p, const Ragged rg) {
 template <typename T>
 __global__ void kv_gather_kernel(const T* __restrict__ cache, T* __restrict__ keys, T* __restrict__ vt, const Ragged rg, int s,
                                  int lo, int kept, int ctx, int ctx_pad, int G, int D, int V, int maps) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int j = blockIdx.x;
   const size_t roww = (size_t)G * D + (size_t)(G / maps) * V;
   const T* row = j < ctx ? cache + page_row(rg, s, key_position(lo - kept + j, lo, kept)) * roww : nullptr;
@@ -336,6 +344,8 @@ SSDK_DEVINL float diff_lambda(const DiffArgs& p) {
 // o [G, M, H/G, V] fp32 (G keys = 2 per value head, H queries) -> y [M, (H / 2) V] (T), rows row0 ..; a warp per head.  grid (rows, ceil(H / 2 / warps))
 template <typename T>
 __global__ void diff_heads_kernel(const float* __restrict__ o, const DiffArgs p, T* __restrict__ y, int M, int H, int G, int V, int row0) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = row0 + blockIdx.x, hd = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31, hpg = H / G;
   if (hd >= H / 2) return;
   const float lam = diff_lambda<T>(p);
@@ -372,6 +382,8 @@ inline size_t gqa_decode_smem(int D, int V) { return ((size_t)(D + 3) / 4 * 4 + 
 // passed around by shuffle.
 template <typename T, int VPL>
 __global__ void __launch_bounds__(kGqaDecWarps * 32) gqa_decode_partial_kernel(const GqaDecodeArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float gd_sm[];
   const int s = blockIdx.x, hd = blockIdx.y, sp = blockIdx.z;
   const int row = rg.cu[s];
@@ -482,6 +494,8 @@ constexpr int kGqaMaxSplits = 32;
 // the head's learned one), times the sigmoid of the gate's pre-activation if the layer has a gate
 template <typename T>
 __global__ void gqa_decode_merge_kernel(const GqaDecodeArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float w[kGqaMaxSplits];
   const int s = blockIdx.x, hd = blockIdx.y;
   const int row = rg.cu[s];
@@ -511,6 +525,8 @@ __global__ void gqa_decode_merge_kernel(const GqaDecodeArgs p, const Ragged rg) 
 // grid (n_seqs, H / 2), differential attention: the two maps' splits are joined as above, then with each other.  dynamic shared memory: V floats
 template <typename T>
 __global__ void gqa_decode_merge_diff_kernel(const GqaDecodeArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   SSDK_DYN_SMEM(float, md_o);
   __shared__ float w[2][kGqaMaxSplits];
   __shared__ float red[33];
@@ -551,6 +567,8 @@ __global__ void gqa_decode_merge_diff_kernel(const GqaDecodeArgs p, const Ragged
 template <typename T>
 __global__ void attn_gate_kernel(const float* __restrict__ o, const float* __restrict__ gz, int ldg, T* __restrict__ y, int M, int H,
                                  int G, int V, int row0) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = row0 + blockIdx.x, hpg = H / G;
   for (int i = threadIdx.x; i < H * V; i += blockDim.x) {
     const int hd = i / V, v = i - hd * V, g = hd / hpg;

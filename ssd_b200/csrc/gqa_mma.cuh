@@ -147,6 +147,8 @@ constexpr int kGpWarps = 8, kGpRows = kGpWarps * 16;
 // per warp.  MAPS = 2 (differential attention): 64 rows, warps 0 .. 3 take their first map, warps 4 .. 7 the second
 template <int KS, int VT, int MAPS>
 __global__ void __launch_bounds__(kGpWarps * 32, 1) gqa_portion_mma_kernel(const GqaPortionArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t gm_sm[];
   typedef __nv_bfloat16 T;
   constexpr int LDK = KS * 16 + 8, LDV = VT * 8 + 8, kTile = kGmKeys * (MAPS * LDK + LDV), kRows = kGpRows / MAPS;
@@ -265,6 +267,8 @@ __global__ void __launch_bounds__(kGpWarps * 32, 1) gqa_portion_mma_kernel(const
 // grid (n_seqs, G, splits), 128 threads: warp w takes keys 16 w .. 16 w + 15 of every tile
 template <int KS, int VT>
 __global__ void __launch_bounds__(128) gqa_decode_mma_kernel(const GqaDecodeArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t gm_sm[];
   typedef __nv_bfloat16 T;
   constexpr int LDK = KS * 16 + 8, LDV = VT * 8 + 8, kTile = kGmKeys * (LDK + LDV);

@@ -57,6 +57,8 @@ SSDK_DEVINL float rope_entry(const float* zr, int c, int rot_dims, int interleav
 
 template <typename T>
 __global__ void latent_prep_kernel(const LatentPrepArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[33];
   const int m = blockIdx.x, s = rg.tok_seq[m];
   const int pos = rg.pos0[s] + (m - rg.cu[s]);
@@ -87,6 +89,8 @@ template <typename T>
 __global__ void latent_q_kernel(const float* __restrict__ q, int ldq, T* __restrict__ qn, T* __restrict__ qcat,
                                 const float* __restrict__ inv_freq, const Ragged rg, int H, int D, int R, int KR, int rot_dims,
                                 int interleaved) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x, hd = blockIdx.y, s = rg.tok_seq[m];
   const int pos = rg.pos0[s] + (m - rg.cu[s]);
   const float* src = q + (size_t)m * ldq + (size_t)hd * (D + R);
@@ -102,6 +106,8 @@ __global__ void latent_q_kernel(const float* __restrict__ q, int ldq, T* __restr
 template <typename T>
 __global__ void latent_gather_kernel(const T* __restrict__ cache, T* __restrict__ keys, T* __restrict__ lat_t, const Ragged rg,
                                      int s, int lo, int ctx, int ctx_pad, int KR, int W) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int j = blockIdx.x;
   const T* row = j < ctx ? cache + page_row(rg, s, lo + j) * (size_t)W : nullptr;
   for (int d = threadIdx.x; d < W; d += blockDim.x) {
@@ -139,6 +145,8 @@ SSDK_DEVINL int key_position(int i, int first, int kept) { return i >= first ? i
 template <typename T>
 __global__ void sink_softmax_kernel(const float* __restrict__ sc, T* __restrict__ pr, const T* __restrict__ sink, int H, int ld,
                                     int pos_first, float scale, int rows_per_batch, float sink_const, int key_first, int kept, KeyMask mask) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[33];
   const int r = blockIdx.x, batch = r / rows_per_batch, rb = r - batch * rows_per_batch;
   const int h = rb % H, pos = pos_first + rb / H;
@@ -203,6 +211,8 @@ template <> SSDK_DEVINL float2 ld_pair<__nv_bfloat16>(const __nv_bfloat16* p) {
 // heads at a time (two dimensions per lane and step), a thread accumulates one latent column for eight heads at a time.
 template <typename T>
 __global__ void __launch_bounds__(kDecThreads) latent_decode_partial_kernel(const LatentDecodeArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x, j = blockIdx.y;
   const int row = rg.cu[s];
   if (rg.cu[s + 1] - row != 1) return;
@@ -333,6 +343,8 @@ inline size_t latent_decode_mma_smem(int W) {
 
 template <int KS, int NT>
 __global__ void __launch_bounds__(kDmThreads) latent_decode_mma_kernel(const LatentDecodeArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x, j = blockIdx.y, h0 = blockIdx.z * 16;
   const int row = rg.cu[s];
   if (rg.cu[s + 1] - row != 1) return;
@@ -484,6 +496,8 @@ constexpr int kDecMaxSplits = 32;   // the host never asks for more context spli
 
 template <typename T>
 __global__ void latent_decode_merge_kernel(const LatentDecodeArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float wj[kDecMaxSplits];   // e^(m_j - m) / denominator per split (0 for a split without keys)
   const int s = blockIdx.x, h = blockIdx.y;
   const int row = rg.cu[s];

@@ -113,6 +113,8 @@ template <typename T, int VEC> SSDK_DEVINL void st_row(T* p, const float* f) {
 template <typename T>
 __global__ void embed_rows_kernel(const int* __restrict__ ids, const T* __restrict__ embed, float* __restrict__ x, int width,
                                   int vocab, float scale, T* __restrict__ xt, int copies) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x;
   int id = ids[m];
   id = min(max(id, 0), vocab - 1);
@@ -129,6 +131,8 @@ template <typename T>
 __global__ void offset_rmsnorm_kernel(const float* __restrict__ x, const T* __restrict__ w, T* __restrict__ y,
                                       const int* __restrict__ rows, int width, float eps, float offset,
                                       const T* __restrict__ w2, T* __restrict__ y2) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[33];
   const int r = blockIdx.x;
   const float* xr = x + (size_t)(rows ? rows[r] : r) * width;
@@ -149,6 +153,8 @@ template <typename T>
 __global__ void postnorm_residual_kernel(float* __restrict__ x, const float* __restrict__ y1, float s1, const float* __restrict__ y2,
                                          float s2, const T* __restrict__ w, int width, float eps, float offset, float mult,
                                          T* __restrict__ xt) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[33];
   const size_t base = (size_t)blockIdx.x * width;
   float ss = 0.f;
@@ -181,6 +187,8 @@ SSDK_DEVINL float act_f(float g) {
 // and beyond *n_rows (optional, on the device) are skipped.  VEC = 4: ff, ldz and the pointers are whole groups of four
 template <typename T, int ACT, int VEC>
 __global__ void glu_act_kernel(const float* __restrict__ z, int ldz, T* __restrict__ y, int ff, const int* __restrict__ n_rows) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int r = blockIdx.x;
   if (n_rows && r >= *n_rows) return;
   for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC; c < ff; c += gridDim.y * blockDim.x * VEC) {   // (columns may be spread over gridDim.y)
@@ -196,6 +204,8 @@ __global__ void glu_act_kernel(const float* __restrict__ z, int ldz, T* __restri
 // z [rows, ff] fp32, b [ff] (T, optional) -> y [rows, ff] (T) = act(z + b)
 template <typename T, int ACT>
 __global__ void bias_act_kernel(const float* __restrict__ z, const T* __restrict__ b, T* __restrict__ y, int ff) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int r = blockIdx.x;
   for (int c = threadIdx.x; c < ff; c += blockDim.x)
     st_f<T>(y + (size_t)r * ff + c, act_f<ACT>(z[(size_t)r * ff + c] + (b ? ld_f<T>(b + c) : 0.f)));
@@ -204,6 +214,8 @@ __global__ void bias_act_kernel(const float* __restrict__ z, const T* __restrict
 // z [rows, ldz] fp32 -> y [rows, ff] (T) = act(z); rows at and beyond *n_rows (optional, on the device) are skipped
 template <typename T, int ACT>
 __global__ void act_cols_kernel(const float* __restrict__ z, int ldz, T* __restrict__ y, int ff, const int* __restrict__ n_rows) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int r = blockIdx.x;
   if (n_rows && r >= *n_rows) return;
   for (int c = threadIdx.x; c < ff; c += blockDim.x) st_f<T>(y + (size_t)r * ff + c, act_f<ACT>(z[(size_t)r * ldz + c]));
@@ -213,6 +225,8 @@ __global__ void act_cols_kernel(const float* __restrict__ z, int ldz, T* __restr
 // r_p = sqrt(mean over the row of z^(2p) + eps): three unit-RMS powers of the row, all in fp32
 template <typename T>
 __global__ void polynorm_kernel(const float* __restrict__ z, const T* __restrict__ coef, T* __restrict__ y, int ff, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[33];
   const float* zr = z + (size_t)blockIdx.x * ff;
   float s1 = 0.f, s2 = 0.f, s3 = 0.f;
@@ -235,6 +249,8 @@ __global__ void polynorm_kernel(const float* __restrict__ z, const T* __restrict
 template <typename T>
 __global__ void token_shift_kernel(const T* __restrict__ h, const T* __restrict__ mu, const float* __restrict__ h_prev,
                                    size_t slot_stride, T* __restrict__ mixes, Ragged rg, int width, int n_mix) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x, s = rg.tok_seq[m];
   const bool first = m == rg.cu[s];
   const float* prev_state = (first && rg.pos0[s] > 0) ? h_prev + (size_t)rg.slot[s] * slot_stride : nullptr;
@@ -251,6 +267,8 @@ __global__ void token_shift_kernel(const T* __restrict__ h, const T* __restrict_
 template <typename T, int GATE>
 __global__ void head_rmsnorm_gate_kernel(const float* __restrict__ o, const float* __restrict__ g, int ldg,
                                          const T* __restrict__ w, T* __restrict__ y, int H, int V, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[33];
   const int m = blockIdx.x, hd = blockIdx.y;
   const float* orow = o + ((size_t)m * H + hd) * V;
@@ -269,6 +287,8 @@ __global__ void head_rmsnorm_gate_kernel(const float* __restrict__ o, const floa
 template <typename T>
 __global__ void clamped_glu_kernel(const float* __restrict__ z, int ldz, T* __restrict__ y, int ff, float limit,
                                    const int* __restrict__ n_rows) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int r = blockIdx.x;
   if (n_rows && r >= *n_rows) return;
   for (int c = threadIdx.x; c < ff; c += blockDim.x) {
@@ -280,17 +300,23 @@ __global__ void clamped_glu_kernel(const float* __restrict__ z, int ldz, T* __re
 
 template <typename T>
 __global__ void tanh_rows_kernel(const float* __restrict__ z, T* __restrict__ y, size_t n) {
+  pdl_launch_dependents();
+  pdl_wait();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     st_f<T>(y + i, tanhf(z[i]));
 }
 
 __global__ void f32_to_bf16_kernel(const float* __restrict__ z, __nv_bfloat16* __restrict__ y, size_t n) {
+  pdl_launch_dependents();
+  pdl_wait();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     y[i] = __float2bfloat16_rn(z[i]);
 }
 
 // out[i] = sum over s of partials[s][i] in the fixed order s = 0 .. S-1 (split-K of the tcgen05 GEMM, fp32)
 __global__ void splitk_sum_kernel(const float* __restrict__ partials, float* __restrict__ out, int S, size_t n) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float a = partials[i];
@@ -321,6 +347,8 @@ struct CombineArgs {
 };
 template <typename T>
 __global__ void block_combine_kernel(const CombineArgs p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int m = blockIdx.x;
   const float sgate = (p.shared && p.sg) ? sigmoid_f(p.sg[(size_t)m * p.ld_sg]) : 1.f;
   for (int c = threadIdx.x; c < p.width; c += blockDim.x) {
@@ -352,6 +380,8 @@ __global__ void block_combine_kernel(const CombineArgs p) {
 template <typename T>
 __global__ void stream_norm_kernel(const float* __restrict__ x, int S, const T* __restrict__ in, const T* __restrict__ w, T* __restrict__ y,
                                    const int* __restrict__ rows, int width, float eps, float offset, float mult) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float sn_u[];
   __shared__ float red[33];
   const int r = blockIdx.x;
@@ -369,6 +399,8 @@ __global__ void stream_norm_kernel(const float* __restrict__ x, int S, const T* 
 }
 
 __global__ void stream_sum_kernel(const float* __restrict__ x, float* __restrict__ y, int S, int width) {
+  pdl_launch_dependents();
+  pdl_wait();
   const float* xr = x + (size_t)blockIdx.x * S * width;
   for (int c = threadIdx.x; c < width; c += blockDim.x) {
     float u = 0.f;
@@ -398,6 +430,8 @@ struct StreamStepArgs {
 // grid (M).  SM >= S: streams held in registers; VEC = 4 needs a width that is a multiple of 4.  dynamic shared memory: width floats
 template <typename T, int SM, int VEC>
 __global__ void stream_step_kernel(const StreamStepArgs p) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float ss_u[];
   __shared__ float red[33], cmix[SM * SM], cout[SM], cin[SM];
   const int S = p.S, W = p.width;
@@ -505,6 +539,8 @@ struct SandwichArgs {
 // grid (M).  VEC = 4 needs a width that is a multiple of 4.  dynamic shared memory: width floats
 template <typename T, int VEC>
 __global__ void sandwich_step_kernel(const SandwichArgs p) {
+  pdl_launch_dependents();
+  pdl_wait();
   SSDK_DYN_SMEM(float, sw_u);
   __shared__ float red[33];
   const int m = blockIdx.x, W = p.width;

@@ -48,6 +48,8 @@ constexpr int kLinBM = 64, kLinBN = 64, kLinBK = 16, kLinThreads = 256;
 // CUDA-core tile: 64 x 64 outputs per CTA, 4 x 4 per thread, operands staged as fp32 in shared memory.
 template <typename T, typename OutT>
 __global__ void __launch_bounds__(kLinThreads) linear_kernel(const LinearArgs p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float As[kLinBK][kLinBM + 4];
   __shared__ float Ws[kLinBK][kLinBN + 4];
   int row0, nrows;
@@ -128,6 +130,8 @@ constexpr int kMmaThreads = 128, kMmaBK = 32, kMmaLd = kMmaBK + 8, kMmaStages = 
 
 template <typename OutT>
 __global__ void __launch_bounds__(kMmaThreads) linear_mma_kernel(const LinearArgs p) {
+  pdl_launch_dependents();
+  pdl_wait();
   typedef __nv_bfloat16 T;
   __shared__ __align__(16) T As[kMmaStages][kLinBM][kMmaLd];
   __shared__ __align__(16) T Ws[kMmaStages][kLinBN][kMmaLd];

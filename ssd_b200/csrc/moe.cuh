@@ -36,6 +36,8 @@ constexpr int kRouterWarps = 4;
 
 template <typename T>
 __global__ void __launch_bounds__(kRouterWarps * 32) group_topk_router_kernel(const RouterArgs p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float s_score[kRouterWarps][kRouterMaxE];    // plain scores
   __shared__ float s_choice[kRouterWarps][kRouterMaxE];   // choice scores; -inf once taken or shut out
   __shared__ float s_group[kRouterWarps][kRouterMaxE];
@@ -123,6 +125,8 @@ struct PlanArgs {
 };
 
 __global__ void __launch_bounds__(1024) expert_plan_kernel(const PlanArgs p) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ int s_cnt[kRouterMaxE];
   __shared__ int s_off[kRouterMaxE + 1];
   for (int e = threadIdx.x; e < p.E; e += blockDim.x) s_cnt[e] = 0;
@@ -162,6 +166,8 @@ __global__ void __launch_bounds__(1024) expert_plan_kernel(const PlanArgs p) {
 template <typename T>
 __global__ void gather_rows_kernel(const T* __restrict__ src, const int* __restrict__ rows, const int* __restrict__ n_rows,
                                    T* __restrict__ dst, int width) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int r = blockIdx.x;
   if (r >= *n_rows) return;
   const T* s = src + (size_t)rows[r] * width;

@@ -39,6 +39,7 @@ struct ScanShape {
 
 template <typename T>
 __global__ void wkv_scan_kernel(const WkvArgs p, const Ragged rg, const ScanShape sh) {
+  pdl_wait();   // (no early start of the next kernel: its waiting blocks slow a chain of dependent steps down)
   SSDK_DYN_SMEM(float, sm);
   const int s = blockIdx.x, hd = blockIdx.y, D = p.D, tid = threadIdx.x, nt = blockDim.x;
   const int j = tid % sh.Vr, g = tid / sh.Vr, i_lo = g * sh.Dg, i_hi = min(D, i_lo + sh.Dg);
@@ -127,6 +128,7 @@ inline size_t wkv_scan_reg_smem(int D, const ScanShape& sh, int DG) {
 
 template <typename T, int DG>
 __global__ void __launch_bounds__(512) wkv_scan_reg_kernel(const WkvArgs p, const Ragged rg, const ScanShape sh) {
+  pdl_wait();   // (no early start of the next kernel: its waiting blocks slow a chain of dependent steps down)
   SSDK_DYN_SMEM(float4, sm4);
   constexpr int C = kScanChunk;
   const int s = blockIdx.x, hd = blockIdx.y, D = p.D, tid = threadIdx.x, nt = blockDim.x;
@@ -226,6 +228,7 @@ SSDK_DEVINL float log_sigmoid_f(float x) { return fminf(x, 0.f) - log1pf(expf(-f
 
 template <typename T>
 __global__ void mlstm_scan_kernel(const MlstmArgs p, const Ragged rg, const ScanShape sh) {
+  pdl_wait();   // (no early start of the next kernel: its waiting blocks slow a chain of dependent steps down)
   SSDK_DYN_SMEM(float, sm);
   const int s = blockIdx.x, hd = blockIdx.y, D = p.D, V = p.V, tid = threadIdx.x, nt = blockDim.x;
   const int j = tid % sh.Vr, g = tid / sh.Vr, i_lo = g * sh.Dg, i_hi = min(D, i_lo + sh.Dg);
@@ -314,6 +317,7 @@ inline size_t mlstm_scan_reg_smem(int D, int V, const ScanShape& sh, int DG) {
 
 template <typename T, int DG>
 __global__ void __launch_bounds__(512) mlstm_scan_reg_kernel(const MlstmArgs p, const Ragged rg, const ScanShape sh) {
+  pdl_wait();   // (no early start of the next kernel: its waiting blocks slow a chain of dependent steps down)
   SSDK_DYN_SMEM(float2, sm2);
   constexpr int C = kScanChunk;
   const int s = blockIdx.x, hd = blockIdx.y, D = p.D, V = p.V, tid = threadIdx.x, nt = blockDim.x;

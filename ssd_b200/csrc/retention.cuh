@@ -43,6 +43,8 @@ SSDK_DEVINL int ret_record(const Ragged& rg, int s) { return rg.cu[s] / kRetChun
 // grid (M, y): the warps of a row's CTAs take its 2 H heads in turn.  dynamic shared memory: rot_dims floats
 template <int VEC>
 __global__ void retention_prep_kernel(const RetentionArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   SSDK_DYN_SMEM(float, rp_cs);
   const int m = blockIdx.x, s = rg.tok_seq[m], pos = rg.pos0[s] + (m - rg.cu[s]), half = (p.inv_freq ? p.rot_dims : 0) >> 1;
   if (rg.cu[s + 1] - rg.cu[s] == 1) return;   // (retention_decode_kernel turns its own row)
@@ -73,6 +75,8 @@ SSDK_DEVINL void ret_fma(const RetTile& t, int tx, int ty, float (&acc)[4][4]) {
 
 // grid (chunks of the longest portion, H * ceil(D / 64) * ceil(V / 64), n_seqs), 256 threads
 __global__ void __launch_bounds__(256) retention_chunk_state_any_kernel(const RetentionArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ __align__(16) RetTile t;
   const int s = blockIdx.z, c = blockIdx.x, r0 = rg.cu[s] + c * kRetChunk, left = rg.cu[s + 1] - r0;
   if (rg.cu[s + 1] - rg.cu[s] < 2 || left <= 0) return;
@@ -104,6 +108,8 @@ __global__ void __launch_bounds__(256) retention_chunk_state_any_kernel(const Re
 
 // grid (chunks of the longest portion, H * ceil(V / 64), n_seqs), 256 threads
 __global__ void __launch_bounds__(256) retention_chunk_out_any_kernel(const RetentionArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ __align__(16) RetTile t;
   __shared__ float P[kRetChunk][kRetChunk + 1];
   const int s = blockIdx.z, c = blockIdx.x, r0 = rg.cu[s] + c * kRetChunk, left = rg.cu[s + 1] - r0;
@@ -172,6 +178,7 @@ constexpr int kRetScanThreads = 128;
 // grid (n_seqs, ceil(H D V / (kRetScanThreads VEC))): VEC entries of the state per thread, eight chunks requested at a time
 template <int VEC>
 __global__ void __launch_bounds__(kRetScanThreads) retention_state_scan_kernel(const RetentionArgs p, const Ragged rg) {
+  pdl_wait();   // (no early start of the next kernel: its waiting blocks slow a chain of dependent steps down)
   const int s = blockIdx.x, rows = rg.cu[s + 1] - rg.cu[s];
   const size_t HDV = (size_t)p.H * p.D * p.V, e0 = ((size_t)blockIdx.y * kRetScanThreads + threadIdx.x) * VEC;
   if (rows < 2 || e0 >= HDV) return;
@@ -259,6 +266,8 @@ inline size_t ret_state_mma_smem(int KS, int VT) { return (size_t)kRetChunk * 2 
 // grid (chunks of the longest portion, H, n_seqs), 256 threads; D <= 16 KS, V <= 8 VT
 template <int KS, int VT>
 __global__ void __launch_bounds__(256, 2) retention_chunk_state_mma_kernel(const RetentionArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   SSDK_DYN_SMEM(uint8_t, rs_sm);
   typedef __nv_bfloat16 T;
   constexpr int LDK = KS * 16 + 8, LDV = VT * 8 + 8;
@@ -315,6 +324,8 @@ inline size_t ret_out_mma_smem(int KS, int VT) {
 // w / 4.  Shared memory: q | k, then the decayed scores | a slab of the state, then v (all as two bf16 terms)
 template <int KS, int VT>
 __global__ void __launch_bounds__(256, 2) retention_chunk_out_mma_kernel(const RetentionArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   SSDK_DYN_SMEM(uint8_t, ro_sm);
   __shared__ float s_pw[kRetChunk + 1], s_ss[2][kRetChunk];
   typedef __nv_bfloat16 T;
@@ -463,6 +474,8 @@ inline size_t ret_decode_smem(int D, int V) { return ((size_t)3 * D + V + kRetDe
 // grid (n_seqs, H), kRetDecWarps warps: the warps share the state's rows, a lane has VEC columns of it per step
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kRetDecWarps * 32) retention_decode_kernel(const RetentionArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
   SSDK_DYN_SMEM(float, rd_sm);
   __shared__ float red[33];
   const int s = blockIdx.x, hd = blockIdx.y, row = rg.cu[s];

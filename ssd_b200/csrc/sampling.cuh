@@ -53,7 +53,7 @@ struct SampleParams {
   ArgMax* partial;     // [B, n_chunks]
   unsigned* counters;  // [B], zero on entry, zero again on exit
   const uint64_t* dyn; // optional device {seed, step}: lets a static CUDA graph draw fresh numbers
-  int sub;             // call_id = step * 16 + sub when dyn != nullptr
+  int sub;             // call_id = step * 16 + sub when dyn != nullptr (sub < 0: the step itself)
 };
 
 __global__ void __launch_bounds__(256) sample_kernel(SampleParams p) {
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) sample_kernel(SampleParams p) {
   if (threadIdx.x == 0) trace_mark(TR_SAMPLE);
   if (p.dyn) {
     p.seed = p.dyn[0];
-    p.call_id = p.dyn[1] * 16ull + (uint64_t)p.sub;
+    p.call_id = p.sub < 0 ? p.dyn[1] : p.dyn[1] * 16ull + (uint64_t)p.sub;
   }
   const int b = blockIdx.y, c = blockIdx.x, nch = gridDim.x;
   const int cs = (((p.V + nch - 1) / nch) + 7) & ~7;
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kVerifyThreads) verify_kernel(VerifyParams p) 
   if (threadIdx.x == 0) trace_mark(TR_VERIFY);
   if (p.dyn) {
     p.seed = p.dyn[0];
-    p.call_id = p.dyn[1] * 16ull + (uint64_t)p.sub;
+    p.call_id = p.sub < 0 ? p.dyn[1] : p.dyn[1] * 16ull + (uint64_t)p.sub;
   }
 
   const int B = p.B, K = p.K, V = p.V, nct = gridDim.x, c = blockIdx.x;
