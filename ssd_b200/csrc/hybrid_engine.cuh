@@ -1001,6 +1001,10 @@ struct HybRun {
     a.R = R; a.bs = bs; a.decay_mult = c.decay_mult;
     CKI(L.go(ssdk::rglru_gate_kernel<T>, dim3(M, (R + 255) / 256), dim3(256), 0, a, e->p2, e->p0));
     alone();
+    if (longest() >= ssdk::kScanChunkMinRows) {
+      CKI(L.go(ssdk::rglru_chunk_scan_kernel<T>, dim3(rg.n_seqs, (R + 31) / 32), dim3(32, ssdk::kScanChunks), 0, a, rg));
+      return lin(e->t1, R, Lr.t[SSDK_HT_MIX_OUT].p, R, e->mix_out, W, M, W, R);
+    }
     const int rt = rg.n_seqs * ((R + 127) / 128) >= num_sms() ? 128 : 32;  // few sequences: one warp per CTA spreads the channels over the SMs
     CKI(L.go(ssdk::rglru_scan_kernel<T>, dim3(rg.n_seqs, (R + rt - 1) / rt), dim3(rt), 0, a, rg));
     return lin(e->t1, R, Lr.t[SSDK_HT_MIX_OUT].p, R, e->mix_out, W, M, W, R);
@@ -1037,7 +1041,11 @@ struct HybRun {
     const size_t smem = (size_t)ssdk::kSelRows * 2 * N * 4;
     CKI(L.go(ssdk::selective_gate_kernel<T>, dim3(M, (I + 255) / 256), dim3(256), 0, dtz, I, (const T*)Lr.t[SSDK_HT_SEL_DT_B].p, e->p0 + I, 2 * I, I));
     alone();
-    if (N <= 128) {
+    if (N <= 16 && longest() >= ssdk::kScanChunkMinRows) {
+      const dim3 grid(rg.n_seqs, (I + 31) / 32), block(32, ssdk::kScanChunks);
+      if (N <= 8) CKI(L.go(ssdk::selective_chunk_scan_kernel<T, 8>, grid, block, 0, a, rg));
+      else CKI(L.go(ssdk::selective_chunk_scan_kernel<T, 16>, grid, block, 0, a, rg));
+    } else if (N <= 128) {
       // NT states per lane, the lanes of a channel side by side in one warp: the fewest lanes that still give every SM
       // eight warps (a long prompt of one sequence), never more than a warp per channel
       int nt = 4;
