@@ -176,6 +176,15 @@ int ssdk_forward_tokens(ssdk_handle h, int which, int batch, int q_len,
                         const float* temps, uint64_t seed, uint64_t step_id,
                         int64_t* out_tokens, void* stream);
 
+/* The same for prompts, whose passes may carry more rows: up to ssdk_prompt_pass_rows(h, which) over the batch (2048 without
+ * tensor parallelism, 256 with it; < 0: no such model). */
+int ssdk_prompt_pass_rows(ssdk_handle h, int which);
+int ssdk_prompt_pass(ssdk_handle h, int which, int batch, int q_len,
+                     const int64_t* ids, const int32_t* ctx_len,
+                     const int32_t* block_tables, int want_sample,
+                     const float* temps, uint64_t seed, uint64_t step_id,
+                     int64_t* out_tokens, void* stream);
+
 /* Debug/parity taps: device pointers to the logits of the last spec step
  * (bf16 [batch, K+1, V] and [batch, K, V]) and of the last ssdk_forward_tokens
  * (bf16 [batch, V]).  Valid until the next call. */

@@ -270,14 +270,29 @@ static int weight_tmap(WeightMat& w) {
 // (UMMA N 16 / 32 / 64); prefill chunks and larger batches up to 256 (UMMA N 128 / 256: the weights are then streamed once
 // per 256 tokens instead of once per 64 — a 2k-token 70B prompt reads 139 GB 8 times instead of 32).
 constexpr int kMaxTokens = 256;
+// Prompt passes without tensor parallelism carry more rows: the tile pairs of gemm_pair_kernel then share the weights through L2 and a
+// layer's small kernels run once per 2048 tokens.  8B widths, 4 layers, 2003 tokens: 8141 us in passes of 256, 5125 us in one.
+constexpr int kMaxPass = 2048;
 struct XMapCache {
-  std::map<std::tuple<const void*, int, int>, CUtensorMap> maps;
-  int get(const void* ptr, int K, int umma_n, const CUtensorMap** out) {
-    auto key = std::make_tuple(ptr, K, umma_n);
+  std::map<std::tuple<const void*, int, int, int>, CUtensorMap> maps;
+  int get(const void* ptr, int K, int box_rows, const CUtensorMap** out, int rows = kMaxTokens) {
+    auto key = std::make_tuple(ptr, K, box_rows, rows);
     auto it = maps.find(key);
     if (it == maps.end()) {
       CUtensorMap tm;
-      CKI(make_tmap(&tm, ptr, kMaxTokens, K, umma_n));
+      CKI(make_tmap(&tm, ptr, rows, K, box_rows));
+      it = maps.emplace(key, tm).first;
+    }
+    *out = &it->second;
+    return 0;
+  }
+  // gate | up rows of gemm_pair_kernel's gated form
+  int get_glu(const void* ptr, int ffn, int K, const CUtensorMap** out) {
+    auto key = std::make_tuple(ptr, K, -1, ffn);
+    auto it = maps.find(key);
+    if (it == maps.end()) {
+      CUtensorMap tm;
+      CKI(make_tmap_glu(&tm, ptr, ffn, K, 1));
       it = maps.emplace(key, tm).first;
     }
     *out = &it->second;
@@ -309,6 +324,9 @@ struct Model {
   // derived (per TP rank)
   int H, KV, hd, d, ffn, qkv_dim, vocab_local;
 };
+
+// rows of one forward pass
+static int pass_rows(const Model& m) { return m.cfg.tp_size == 1 && m.ffn % kPairGluRun == 0 ? kMaxPass : kMaxTokens; }
 
 struct Workspace {
   // activations (X-operand capable: kMaxTokens rows each)
@@ -415,7 +433,7 @@ static int64_t carve(ssdk_engine* e, uint8_t* base) {
     return p;
   };
   int dmax = 0, qmax = 0, fmax = 0, vmax = 0, Hmax = 0, hdmax = 0;
-  size_t part = 0;
+  size_t part = 0, pass = kMaxTokens;
   for (int w = 0; w < 2; ++w) {
     Model& m = e->model[w];
     if (!m.present) continue;
@@ -435,15 +453,17 @@ static int64_t carve(ssdk_engine* e, uint8_t* base) {
     part = std::max(part, need(m.d, m.H * m.hd));
     part = std::max(part, need(2 * m.ffn, m.d));
     part = std::max(part, need(m.d, m.ffn));
+    if (pass_rows(m) > kMaxTokens) part = std::max(part, (size_t)pass_rows(m) * std::max(m.qkv_dim, m.d));   // one slab
+    pass = std::max<size_t>(pass, pass_rows(m));
   }
   Workspace scratch_ws;
   Workspace& w = base ? e->ws : scratch_ws;  // measuring (base == nullptr) must not clobber bound pointers
   const int K = e->rt.spec_k, MB = e->rt.max_batch;
-  w.hidden = (bf16*)take((size_t)kMaxTokens * dmax * 2);
-  w.residual = (bf16*)take((size_t)kMaxTokens * dmax * 2);
-  w.q = (bf16*)take((size_t)kMaxTokens * Hmax * hdmax * 2);
-  w.attn_out = (bf16*)take((size_t)kMaxTokens * Hmax * hdmax * 2);
-  w.act = (bf16*)take((size_t)kMaxTokens * fmax * 2);
+  w.hidden = (bf16*)take((size_t)pass * dmax * 2);
+  w.residual = (bf16*)take((size_t)pass * dmax * 2);
+  w.q = (bf16*)take((size_t)pass * Hmax * hdmax * 2);
+  w.attn_out = (bf16*)take((size_t)pass * Hmax * hdmax * 2);
+  w.act = (bf16*)take((size_t)pass * fmax * 2);
   w.last_hidden = (bf16*)take((size_t)kMaxTokens * dmax * 2);
   w.dense_tmp = (bf16*)take((size_t)kMaxTokens * std::max(dmax, qmax) * 2);
   w.partials = (float*)take(part * 4);
@@ -453,8 +473,8 @@ static int64_t carve(ssdk_engine* e, uint8_t* base) {
   w.att_counters = (unsigned*)take((size_t)kMaxTokens * 64 * 4);
   w.ar_state = (unsigned*)take(64);
   w.pub_counters = (unsigned*)take(512 * 4);
-  w.positions = (int64_t*)take(kMaxTokens * 8);
-  w.slot_mapping = (int32_t*)take(kMaxTokens * 4);
+  w.positions = (int64_t*)take(pass * 8);
+  w.slot_mapping = (int32_t*)take(pass * 4);
   w.context_lens = (int32_t*)take(kMaxTokens * 4);
   w.out_dev = take(e->out_bytes);
   w.tok_buf = (int64_t*)w.out_dev;
@@ -462,7 +482,7 @@ static int64_t carve(ssdk_engine* e, uint8_t* base) {
   w.recovery = (int64_t*)(w.out_dev ? w.out_dev + e->off_out_rec : nullptr);
   w.log_tokens = (int64_t*)take((size_t)MB * kLogCap * 8);
   w.log_len = (int32_t*)take((size_t)MB * 4);
-  w.ids_in = (int64_t*)take(kMaxTokens * 8);
+  w.ids_in = (int64_t*)take(pass * 8);
   w.out_tok = (int64_t*)take(kMaxTokens * 8);
   w.logits_q = (bf16*)take((size_t)MB * std::max(K, 1) * vmax * 2);
   w.logits_p = (bf16*)take((size_t)MB * (K + 1) * vmax * 2);
@@ -563,6 +583,20 @@ static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w
   CKI(weight_tmap(w));
   const int K = (int)w.cols;
   if (K % kBlockK) return fail("GEMM K=%d not a multiple of 64", K);
+  if (M > kMaxTokens) {   // prompt passes: one slab, summed over all of K
+    if (epi != EPI_PARTIAL && (epi != EPI_SILU || N_out % kPairGluRun)) return fail("GEMM of %d rows: unsupported form", M);
+    if (epi == EPI_PARTIAL && (size_t)M * N_out > e->ws.partial_floats) return fail("partial buffer too small");
+    const CUtensorMap *tmW, *tmX, *tmXs;
+    if (epi == EPI_SILU) CKI(e->xmaps.get_glu(w.ptr, N_out, K, &tmW));
+    else CKI(e->xmaps.get(w.ptr, K, 128, &tmW, (int)w.rows));
+    CKI(e->xmaps.get(x, K, kPairXBox, &tmX, kMaxPass));
+    CKI(e->xmaps.get(x, K, kPairXSmall, &tmXs, kMaxPass));
+    GemmPairParams p = {};
+    p.out = out; p.M = M; p.N = N_out; p.ldo = epi == EPI_SILU ? ldo : N_out; p.num_kb = K / kBlockK; p.chunks = (M + kPairTokens - 1) / kPairTokens;
+    p.w_tiles = epi == EPI_SILU ? (N_out + 127) / 128 : (N_out + 255) / 256; p.act = GLU_SILU_ROUNDED;
+    if (splits_out) *splits_out = 1;
+    return launch_gemm_pair(L, epi == EPI_SILU ? EPI_GLU : EPI_PARTIAL, *tmW, *tmX, *tmXs, p, p.w_tiles * p.chunks);
+  }
   const int un = umma_n_for(M);
   const CUtensorMap* tmX;
   CKI(e->xmaps.get(x, K, un, &tmX));
@@ -695,18 +729,19 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
   Model& m = e->model[f.which];
   Workspace& w = e->ws;
   const int M = f.B * f.Q;
-  if (M < 1 || M > kMaxTokens) return fail("forward: %d tokens (max %d)", M, kMaxTokens);
+  if (M < 1 || M > pass_rows(m)) return fail("forward: %d tokens (max %d)", M, pass_rows(m));
   const int tp = m.cfg.tp_size;
   if (tp > 1 && !e->comm) return fail("tensor parallel forward without a NCCL communicator");
   const int bs = e->rt.block_size, mb = e->rt.max_blocks_per_seq;
   const int64_t cache_layer_stride = m.num_blocks * bs * m.KV * m.hd;
 
-  CKI(L.go(prep_kernel, dim3(1), dim3(kMaxTokens), 0, f.ctx0, f.block_tables, mb, bs, f.B, f.Q, f.pos_offset,
+  CKI(L.go(prep_kernel, dim3((M + kMaxTokens - 1) / kMaxTokens), dim3(kMaxTokens), 0, f.ctx0, f.block_tables, mb, bs, f.B, f.Q, f.pos_offset,
            w.positions, w.slot_mapping, w.context_lens,
            (f.which == SSDK_TARGET && tp > 1 && e->symm_n == tp) ? w.ar_state : (unsigned*)nullptr));
 
   int TQ = 1, MT = 1, nqt = 1, nsplit = 1;
   CKI(attn_plan(m, f.B, f.Q, &TQ, &MT, &nqt, &nsplit, e->max_ctx_hint));
+  if (M > kMaxTokens) nsplit = 1;   // (the partials are sized for kMaxTokens rows; so many q tiles fill the SMs by themselves)
   const float scale = 1.0f / sqrtf((float)m.hd);
 
   const bool use_symm = tp > 1 && e->symm_n == tp;
@@ -1217,7 +1252,7 @@ int ssdk_create(const ssdk_model_cfg* target, const ssdk_model_cfg* draft, const
     return fail("pinned staging allocation failed");
   }
   memset(e->pin_in, 0, e->step_bytes);
-  e->fw_slot_bytes = align_up(e->step_bytes, 64) + (size_t)kMaxTokens * 8;
+  e->fw_slot_bytes = align_up(e->step_bytes, 64) + (size_t)kMaxPass * 8;
   if (cudaHostAlloc((void**)&e->pin_fw, e->fw_slot_bytes * ssdk_engine::kFwSlots, cudaHostAllocDefault) != cudaSuccess) {
     cudaFreeHost(e->pin_in);
     cudaFreeHost(e->pin_out);
@@ -1484,12 +1519,12 @@ int ssdk_spec_step_log(ssdk_handle h, int seq, int64_t* out_tokens, int cap, voi
   return n;
 }
 
-int ssdk_forward_tokens(ssdk_handle h, int which, int batch, int q_len, const int64_t* ids, const int32_t* ctx_len,
+static int forward_rows(ssdk_handle h, int which, int batch, int q_len, const int64_t* ids, const int32_t* ctx_len,
                         const int32_t* block_tables, int want_sample, const float* temps, uint64_t seed,
-                        uint64_t step_id, int64_t* out_tokens, void* stream) {
+                        uint64_t step_id, int64_t* out_tokens, void* stream, int most) {
   if (!h || !h->finalized) return fail("forward_tokens: engine not finalized");
   if (which < 0 || which > 1 || !h->model[which].present) return fail("forward_tokens: model %d absent", which);
-  if (batch < 1 || batch > h->rt.max_batch || q_len < 1 || batch * q_len > kMaxTokens)
+  if (batch < 1 || batch > h->rt.max_batch || q_len < 1 || q_len > most || batch * q_len > most)
     return fail("forward_tokens: batch=%d q_len=%d out of range", batch, q_len);
   cudaStream_t st = (cudaStream_t)stream;
   Workspace& w = h->ws;
@@ -1544,9 +1579,28 @@ int ssdk_forward_tokens(ssdk_handle h, int which, int batch, int q_len, const in
     CK(cudaMemcpyAsync(pin_ids, w.out_tok, (size_t)batch * 8, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (out_tokens) memcpy(out_tokens, pin_ids, (size_t)batch * 8);
+    CKI(check_waits());
   }
   h->launches += L.count;
   return 0;
+}
+
+int ssdk_forward_tokens(ssdk_handle h, int which, int batch, int q_len, const int64_t* ids, const int32_t* ctx_len,
+                        const int32_t* block_tables, int want_sample, const float* temps, uint64_t seed,
+                        uint64_t step_id, int64_t* out_tokens, void* stream) {
+  return forward_rows(h, which, batch, q_len, ids, ctx_len, block_tables, want_sample, temps, seed, step_id, out_tokens, stream, kMaxTokens);
+}
+
+int ssdk_prompt_pass_rows(ssdk_handle h, int which) {
+  if (!h || which < 0 || which > 1 || !h->model[which].present) return -1;
+  return pass_rows(h->model[which]);
+}
+
+int ssdk_prompt_pass(ssdk_handle h, int which, int batch, int q_len, const int64_t* ids, const int32_t* ctx_len,
+                     const int32_t* block_tables, int want_sample, const float* temps, uint64_t seed,
+                     uint64_t step_id, int64_t* out_tokens, void* stream) {
+  const int most = ssdk_prompt_pass_rows(h, which);
+  return forward_rows(h, which, batch, q_len, ids, ctx_len, block_tables, want_sample, temps, seed, step_id, out_tokens, stream, std::max(most, kMaxTokens));
 }
 
 // debug: route the kernels' timeline marks into `dev_buf` (uint64 [cap][2]); dev_buf = NULL disables tracing

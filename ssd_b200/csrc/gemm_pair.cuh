@@ -30,13 +30,16 @@ constexpr int kPairSmem = kPairStages * kPairStageBytes + 1024;
 // rows (a five-dimensional box picks the gated form's runs of 16) and one of the tile's token half: 128 rows, or 32-row boxes for up to 64.
 constexpr int kPairXBox = 128, kPairXSmall = 32, kPairGluRun = 16;
 
+// activations of the gated form; SILU_ROUNDED rounds gate and up to bf16 first (the dense decoders' linear layers return bf16)
+enum { GLU_SILU = 0, GLU_GELU = 1, GLU_SILU_ROUNDED = 2 };
+
 struct GemmPairParams {
   void* out;          // EPI_PARTIAL: fp32 [M, ldo]; EPI_GLU: bf16 [M, ldo]
   int M, N, ldo;      // N: output columns (EPI_GLU: of the product act(gate) * up; the up rows start N rows behind the gate rows)
   int num_kb;         // K / 64
   int w_tiles;        // tiles along the weight rows: 256 columns (EPI_PARTIAL) or 128 (EPI_GLU) of the output
   int chunks;         // row chunks of kPairTokens tokens (dense)
-  int glu_gelu;       // EPI_GLU: 0 silu, 1 gelu_tanh
+  int act;            // EPI_GLU: GLU_*
   // grouped mode: see GemmParams
   const int* g_tile_expert;
   const int* g_tile_row0;
@@ -252,8 +255,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           for (int m = 0; m < 32; m += 2) {
             const float keep = __uint_as_float(lo ? r[m] : r[m + 1]);
             const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(lo ? r[m + 1] : r[m]), 16);
-            const float g = lo ? keep : got, u = lo ? got : keep;
-            const float a = p.glu_gelu ? 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) : __fdividef(g, 1.0f + __expf(-g));
+            float g = lo ? keep : got, u = lo ? got : keep;
+            if (p.act == GLU_SILU_ROUNDED) { g = bf16_round(g); u = bf16_round(u); }
+            const float a = p.act == GLU_GELU ? 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) : __fdividef(g, 1.0f + __expf(-g));
             if (n < p.N && m + (lo ? 0 : 1) < left) out[(size_t)m * p.ldo] = f2bf(a * u);
           }
         } else {

@@ -423,7 +423,7 @@ struct HybRun {
   }
   int lin_pair(bool glu, const void* A, const void* W, void* C, int m_total, int w_rows, int K, int ldw, bool gelu) {
     GemmPairParams p = {};
-    p.out = C; p.M = m_total; p.chunks = (m_total + kPairTokens - 1) / kPairTokens; p.glu_gelu = gelu;
+    p.out = C; p.M = m_total; p.chunks = (m_total + kPairTokens - 1) / kPairTokens; p.act = gelu ? GLU_GELU : GLU_SILU;
     return go_pair(glu, A, W, m_total, w_rows, 1, K, ldw, p, p.chunks);
   }
   // (gemm_ws_kernel asks for its first weight tiles, and in grouped mode reads the tile list, before it waits for the kernel in front:

@@ -120,6 +120,9 @@ SIGNATURES: dict[str, tuple] = {
     "ssdk_spec_step_log": (C.c_int, [VP, C.c_int, c_i64p, C.c_int, VP]),
     "ssdk_forward_tokens": (C.c_int, [VP, C.c_int, C.c_int, C.c_int, c_i64p, c_i32p, c_i32p, C.c_int, c_f32p,
                                       C.c_uint64, C.c_uint64, c_i64p, VP]),
+    "ssdk_prompt_pass_rows": (C.c_int, [VP, C.c_int]),
+    "ssdk_prompt_pass": (C.c_int, [VP, C.c_int, C.c_int, C.c_int, c_i64p, c_i32p, c_i32p, C.c_int, c_f32p,
+                                   C.c_uint64, C.c_uint64, c_i64p, VP]),
     "ssdk_logits_p": (VP, [VP]),
     "ssdk_logits_q": (VP, [VP]),
     "ssdk_logits_last": (VP, [VP]),

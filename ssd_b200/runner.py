@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import ctypes as C
 from dataclasses import dataclass
+from functools import partial
 
 import numpy as np
 import torch
@@ -62,6 +63,14 @@ def rope_table(head_dim: int, rows: int, base: float, device) -> torch.Tensor:
 
 def _i32(a):
     return np.ascontiguousarray(a, dtype=np.int32)
+
+
+def _prompt_call(runner, which: int, chunk: int):
+    """(call that runs prompt rows, rows it takes at most): with the default chunk a runner that has longer passes takes those."""
+    most = runner.pass_tokens(which) if chunk == 256 and hasattr(runner, "pass_tokens") else 0
+    if most <= 256:
+        return runner.forward_tokens, chunk
+    return partial(runner.forward_tokens, rows=most), most
 
 
 class PairRunner:
@@ -161,8 +170,9 @@ class PairRunner:
         return out
 
     def forward_tokens(self, which: int, ids: list[list[int]], ctx_len: list[int], block_tables, temps=None,
-                       want_sample: bool = True, seed: int = 0) -> list[int] | None:
-        """ModelRunner.run for q_len tokens per sequence appended at ctx_len (prefill chunk or AR decode)."""
+                       want_sample: bool = True, seed: int = 0, *, rows: int = 256) -> list[int] | None:
+        """ModelRunner.run for q_len tokens per sequence appended at ctx_len (prefill chunk or AR decode).
+        rows: the rows a call may carry; prompts ask for pass_tokens."""
         if self.spec[which] is None:
             return None  # the draft replica lives on TP rank 0 only (SURVEY §8e); other ranks have nothing to do
         B, Q = len(ids), len(ids[0])
@@ -172,29 +182,37 @@ class PairRunner:
         temps_a = np.ascontiguousarray(temps if temps is not None else [0.0] * B, dtype=np.float32)
         out = np.zeros(B, dtype=np.int64)
         st = torch.cuda.current_stream().cuda_stream
-        L.check(self.lib.ssdk_forward_tokens(self.h, which, B, Q, ids_a.ctypes.data_as(L.c_i64p),
-                                             ctx_a.ctypes.data_as(L.c_i32p), bt_a.ctypes.data_as(L.c_i32p),
-                                             int(want_sample), temps_a.ctypes.data_as(L.c_f32p), seed, self.step_id,
-                                             out.ctypes.data_as(L.c_i64p), st), "ssdk_forward_tokens")
+        call = self.lib.ssdk_forward_tokens
+        if rows > 256:
+            call = self.lib.ssdk_prompt_pass
+            self.step_id += max(0, -(-B * Q // 256) - 1)  # draws are numbered by passes of 256 rows
+        L.check(call(self.h, which, B, Q, ids_a.ctypes.data_as(L.c_i64p), ctx_a.ctypes.data_as(L.c_i32p), bt_a.ctypes.data_as(L.c_i32p),
+                     int(want_sample), temps_a.ctypes.data_as(L.c_f32p), seed, self.step_id, out.ctypes.data_as(L.c_i64p), st),
+                "ssdk_forward_tokens")
         self.step_id += 1
         return out.tolist() if want_sample else None
 
     def prefill(self, which: int, tokens: list[int], block_table: list[int], start: int = 0, temp: float = 0.0,
                 want_sample: bool = True, chunk: int = 256, seed: int = 0):
-        """Prefill one sequence from position `start` in chunks of <= 256 tokens through the multi-query path: the
-        weights are streamed once per chunk (UMMA N = 128 / 256 instances of the tcgen05 GEMM), attention is the paged
-        multi-query kernel with one q tile per 4-32 query rows (layers/attention.py:85-93 semantics: causal over the
-        cache, which already holds the earlier chunks)."""
+        """Prefill one sequence from position `start` in passes through the multi-query path: the weights are streamed
+        once per pass, attention is the paged multi-query kernel with one q tile per 4-32 query rows
+        (layers/attention.py:85-93 semantics: causal over the cache, which already holds the earlier passes).
+        chunk: tokens of a pass; with the default value a pass carries what the engine takes (pass_tokens)."""
+        call, size = _prompt_call(self, which, chunk)
         tok = None
         pos = start
         n = len(tokens)
         while pos < n:
-            q = min(chunk, n - pos)
+            q = min(size, n - pos)
             last = pos + q == n
-            tok = self.forward_tokens(which, [tokens[pos:pos + q]], [pos], [block_table], [temp],
-                                      want_sample=(want_sample and last), seed=seed)
+            tok = call(which, [tokens[pos:pos + q]], [pos], [block_table], [temp],
+                       want_sample=(want_sample and last), seed=seed)
             pos += q
         return tok[0] if tok else None
+
+    def pass_tokens(self, which: int) -> int:
+        """Rows that one prompt pass of a model takes (2048; 256 under tensor parallelism)."""
+        return int(self.lib.ssdk_prompt_pass_rows(self.h, which)) if self.spec[which] is not None else 256
 
     @staticmethod
     def plan_prefill_call(remaining: list[int], max_tokens: int, max_batch: int) -> tuple[list[int], int]:
@@ -214,7 +232,7 @@ class PairRunner:
     def prefill_many(self, which: int, tokens: list[list[int]], block_tables: list[list[int]], starts: list[int],
                      temps: list[float] | None = None, want_sample: bool = True, chunk: int = 256, seed: int = 0):
         """Prefill several sequences (runner_helpers.py:123-180 batches them by cu_seqlens): every call carries up to
-        `chunk` tokens of up to max_batch sequences, the same number of tokens from each (plan_prefill_call), through the
+        a pass of tokens (`chunk` if that is less than its default) of up to max_batch sequences, the same number of tokens from each (plan_prefill_call), through the
         multi-query path; a sequence's first token is sampled by the call that holds its last prompt token.  Returns one
         token per sequence (None without want_sample)."""
         n = len(tokens)
@@ -225,15 +243,16 @@ class PairRunner:
         # (block_manager hashes a block when it is allocated, the reference stores the whole batch's K/V before any
         # attention runs): only sequences that compute their whole prompt share calls; the hits follow one by one, in order.
         packed = [i for i in range(n) if starts[i] == 0]
+        call, size = _prompt_call(self, which, min(chunk, 256))
         while True:
             idx, q = self.plan_prefill_call([len(tokens[i]) - pos[i] if i in packed else 0 for i in range(n)],
-                                            min(chunk, 256), self.max_batch)
+                                            size, self.max_batch)
             if not idx:
                 break
             done = [pos[i] + q == len(tokens[i]) for i in idx]
-            toks = self.forward_tokens(which, [tokens[i][pos[i]:pos[i] + q] for i in idx], [pos[i] for i in idx],
-                                       [block_tables[i] for i in idx], [temps[i] for i in idx],
-                                       want_sample=(want_sample and any(done)), seed=seed)
+            toks = call(which, [tokens[i][pos[i]:pos[i] + q] for i in idx], [pos[i] for i in idx],
+                        [block_tables[i] for i in idx], [temps[i] for i in idx],
+                        want_sample=(want_sample and any(done)), seed=seed)
             for j, i in enumerate(idx):
                 pos[i] += q
                 if done[j] and toks is not None:

@@ -1,0 +1,56 @@
+"""Prompt passes of more than 256 rows (gemm_pair_kernel, one slab per product) against passes of 64 rows: logits of the last row, the
+cache, several prompts in a pass, and the calls that stay refused."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# bf16 activations through two layers: both forms round the same intermediates, sums over K in another order (split-K) move some of
+# them by one unit of 2^-8
+TOL = 4 * 2.0 ** -8
+
+
+def _runner(batch=2):
+    from ssd_b200 import lib as L, synth
+    from ssd_b200.runner import ModelSpec, PairRunner
+    spec = ModelSpec(hidden=256, layers=2, heads=4, kv_heads=2, head_dim=64, ffn=576, vocab=1024, rms_eps=1e-5)
+    r = PairRunner(spec, None, spec_k=0, max_batch=batch, block_size=64, max_model_len=2560, use_graph=False, use_pdl=True)
+    w = synth.generate_weights(spec, {"seed": 3, "alpha": 0.9, "role": "target", "o_down_std": 0.05}, torch.device("cuda:0"))
+    r.bind_weights(L.TARGET, w)
+    r.finalize()
+    return r
+
+
+@pytest.mark.parametrize("n", [255, 256, 257, 320, 449, 2049])
+def test_long_pass_matches_short_ones(n):
+    from ssd_b200 import lib as L
+    r = _runner()
+    toks = torch.randint(0, 1024, (n,), generator=torch.Generator().manual_seed(n)).tolist()
+    a_pages, b_pages = list(range(40)), list(range(40, 80))
+    ta = r.prefill(L.TARGET, toks, a_pages, chunk=64)
+    la = r.logits_last(1).float()
+    tb = r.prefill(L.TARGET, toks, b_pages)
+    lb = r.logits_last(1).float()
+    assert ta == tb
+    assert ((la - lb).norm() / la.norm()).item() < TOL
+    ka, kb = (r.kv[L.TARGET][:, :, s:s + 40].flatten(2, 3)[:, :, :n].float() for s in (0, 40))
+    assert ((ka - kb).norm() / ka.norm()).item() < TOL
+
+
+def test_several_prompts_in_a_pass():
+    from ssd_b200 import lib as L
+    r = _runner()
+    g = torch.Generator().manual_seed(5)
+    prompts = [torch.randint(0, 1024, (n,), generator=g).tolist() for n in (700, 411)]
+    pages = [list(range(40)), list(range(40, 80))]
+    want = [r.prefill(L.TARGET, p, t, chunk=64) for p, t in zip(prompts, pages)]
+    assert r.prefill_many(L.TARGET, prompts, pages, [0, 0]) == want
+
+
+def test_refused_as_before():
+    from ssd_b200 import lib as L
+    r = _runner()
+    with pytest.raises(RuntimeError):
+        r.forward_tokens(L.TARGET, [[1] * 257], [0], [list(range(40))])
+    with pytest.raises(RuntimeError):
+        r.prefill(L.TARGET, [1] * 600, list(range(40)), chunk=512)
