@@ -5,28 +5,32 @@
 //   causal mask aligned to the END of the cache (query j of a sequence sees kv positions
 //   <= context_len - q_len + j), K/V read back from the paged cache (attention.py:82-83).
 //
-// Work decomposition (the problem is tiny and latency-bound at b=1, so the aim is to
-// spread a few hundred KB of KV over as many SMs as possible):
-//   grid = (kv_heads, n_split, batch * n_qtiles), 128 threads.
+// Work decomposition (at b=1 the problem is tiny and latency-bound, so the aim is to spread a few hundred KB of KV over as many
+// SMs as possible; long contexts are bound by issue slots and by the bytes in flight, so the aim is equal shares in one wave):
+//   grid = (kv_heads, ranges, n_qtiles), 128 or 256 threads.
 //   A CTA owns one kv head, up to TQ query tokens x G=H/KV query heads (R = G*tq <= 64 rows,
-//   padded to MT 16-row MMA tiles) and a contiguous range of 64-token KV chunks.
+//   padded to MT 16-row MMA tiles) and a range of 64-token KV chunks of one sequence.
+//   Ranges: the chunks of ALL sequences are cut into pieces of one length, chosen so that about two CTAs per SM get one
+//   (AttnRanges); a fixed number of splits per sequence left the longest of eight ragged 70B contexts running alone.
 //   K/V chunks are staged in shared memory with 16-byte cp.async (coalesced 256 B rows of a
-//   page), double buffered; QK^T and PV run on mma.sync m16n8k16 (bf16, fp32 accumulate)
-//   with ldmatrix fragments; softmax is online in fp32 (exp2 domain).
+//   page), two or three deep; QK^T and PV run on mma.sync m16n8k16 (bf16, fp32 accumulate)
+//   with ldmatrix fragments; softmax is online in fp32 (exp2 domain), the sums are rescaled only where a maximum moved.
 //   Warps split (m-tile, token-slice); their partial (m, l, O) are merged through smem,
 //   split-KV partials through a global fp32 scratch + attn_combine_kernel.
-// The grid is static (CUDA-graph friendly): each CTA derives its chunk range from
-// context_lens[] at run time.
+//   Two to three CTAs per SM: registers are capped and the kernels ask for the large shared-memory carve-out.  With 156 registers
+//   and the default carve-out one CTA of eight warps was resident and the SMs issued 43 % of the time.
+// The grid is static (CUDA-graph friendly): each CTA derives its range from context_lens[] at run time.
 #pragma once
 #include "common.cuh"
 
 namespace ssdk {
 
-// warps per CTA: 8 for the 32/64-row q tiles (four or two token slices per m-tile), 4 for single-m-tile decode.
-// One CTA per SM is resident, so the kernel is bound by the length of each warp's serial instruction chain (address
-// generation, softmax, epilogue merge) rather than by bandwidth: more warps = shorter chains.
+// warps per CTA: 8 for the 32/64-row q tiles (four or two token slices per m-tile), 4 for single-m-tile decode: a short context is
+// bound by the length of each warp's serial instruction chain (address generation, softmax, epilogue merge), more warps = shorter chains.
 constexpr int attn_warps(int MT) { return MT == 1 ? 4 : 8; }
 constexpr int kAttChunk = 64;
+constexpr int attn_stages(int MT) { return MT == 1 ? 2 : 3; }
+constexpr int attn_smem(int HD, int MT) { return attn_stages(MT) * 2 * kAttChunk * (HD + 8) * 2; }
 
 struct AttnParams {
   const __nv_bfloat16* q;        // [B*Q, H, hd]
@@ -37,7 +41,10 @@ struct AttnParams {
   __nv_bfloat16* out;            // [B*Q, H*hd]
   float* part_o;                 // [B*Q*H, n_split, hd]
   float* part_lse;               // [B*Q*H, n_split]
-  int B, Q, H, KV, block_size, max_blocks, n_split, TQ, n_qtiles;
+  int B, Q, H, KV, block_size, max_blocks, TQ, n_qtiles;
+  int n_split;                   // most ranges of one sequence (stride of the partials); 1: every sequence is one range, no partials
+  int target;                    // ranges aimed at over all sequences (per kv head and q tile); the grid has target + B.  0: n_split
+                                 // ranges per sequence, whatever the others' lengths; the grid has n_split B
   int g_shift;                   // log2(H / KV) when the GQA ratio is a power of two, else -1
   float scale_log2;              // softmax scale * log2(e)
 };
@@ -74,8 +81,58 @@ SSDK_DEVINL uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <int HD, int MT>
-__global__ void __launch_bounds__(attn_warps(MT) * 32) paged_attn_kernel(AttnParams p) {
+// How the batch's chunks are cut: pieces of `cps` chunks, item i = piece `split` of sequence `b` (b < 0: no such item).  Each warp works
+// it out by itself: one load per 32 sequences and a prefix sum.  `seq`: only the piece length of that sequence is asked for.
+struct AttnRanges { int cps, b, split; };
+SSDK_DEVINL AttnRanges attn_ranges(const AttnParams& p, int item, int seq = -1) {
+  AttnRanges r;
+  if (p.n_split == 1) { r.cps = 0x3fffffff; r.b = item < p.B ? item : -1; r.split = 0; return r; }
+  if (p.target == 0) {   // every sequence by itself: n_split ranges
+    const int b = seq >= 0 ? seq : item / p.n_split, n = (p.context_lens[b] + kAttChunk - 1) / kAttChunk;
+    r.cps = max(1, (n + p.n_split - 1) / p.n_split);
+    r.b = b; r.split = item - b * p.n_split;
+    return r;
+  }
+  const int lane = threadIdx.x & 31;
+  int total = 0, most = 0;
+  for (int b0 = 0; b0 < p.B; b0 += 32) {
+    const int n = b0 + lane < p.B ? (p.context_lens[b0 + lane] + kAttChunk - 1) / kAttChunk : 0;
+    total += n;
+    most = max(most, n);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    total += __shfl_xor_sync(0xffffffffu, total, o);
+    most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+  }
+  r.cps = max(1, max((total + p.target - 1) / p.target, (most + p.n_split - 1) / p.n_split));
+  r.b = -1; r.split = 0;
+  int before = 0;
+  for (int b0 = 0; b0 < p.B && item >= 0; b0 += 32) {
+    const int n = b0 + lane < p.B ? (p.context_lens[b0 + lane] + kAttChunk - 1) / kAttChunk : 0;
+    const int mine = (n + r.cps - 1) / r.cps;
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const int rel = item - before;
+    const unsigned hit = __ballot_sync(0xffffffffu, rel >= 0 && rel < upto && rel >= upto - mine);
+    if (hit) {
+      const int src = __ffs(hit) - 1;
+      r.b = b0 + src;
+      r.split = rel - __shfl_sync(0xffffffffu, upto - mine, src);
+      break;
+    }
+    before += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  return r;
+}
+
+// OCC: CTAs that are to fit an SM
+template <int HD, int MT, int OCC>
+__global__ void __launch_bounds__(attn_warps(MT) * 32, OCC) paged_attn_kernel(AttnParams p) {
   constexpr int NW = attn_warps(MT);
   constexpr int kAttThreads = NW * 32;
   constexpr int LDS = HD + 8;               // padded smem row (bf16 elements)
@@ -87,15 +144,17 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32) paged_attn_kernel(AttnPar
   constexpr int SEG = HD / 8;               // 16-byte segments per K/V row
 
   extern __shared__ __align__(16) uint8_t att_smem[];
-  __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(att_smem);            // [2][64][LDS]
-  __nv_bfloat16* sV = sK + 2 * kAttChunk * LDS;                              // [2][64][LDS]
+  constexpr int kStages = attn_stages(MT);
+  __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(att_smem);            // [kStages][64][LDS]
+  __nv_bfloat16* sV = sK + kStages * kAttChunk * LDS;                        // [kStages][64][LDS]
 
   pdl_launch_dependents();
   pdl_wait();
   if (threadIdx.x == 0) trace_mark(TR_ATTN);
 
-  const int kvh = blockIdx.x, split = blockIdx.y;
-  const int b = blockIdx.z / p.n_qtiles, qt = blockIdx.z % p.n_qtiles;
+  const AttnRanges rgs = attn_ranges(p, blockIdx.y);
+  if (rgs.b < 0) return;
+  const int kvh = blockIdx.x, split = rgs.split, b = rgs.b, qt = p.n_qtiles - 1 - (int)blockIdx.z;   // (the tiles that see most keys first)
   const int G = p.H / p.KV;
   const int tq = min(p.TQ, p.Q - qt * p.TQ);
   const int R = G * tq;
@@ -103,10 +162,10 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32) paged_attn_kernel(AttnPar
   const int ctx0 = ctx - p.Q;                         // tokens before this forward
   const int kv_max = ctx0 + qt * p.TQ + tq;           // exclusive upper bound of visible kv for this q-tile
   const int nch_total = (kv_max + kAttChunk - 1) / kAttChunk;
-  const int cps = (nch_total + p.n_split - 1) / p.n_split;
-  const int ch_begin = split * cps;
-  const int ch_end = min(nch_total, ch_begin + cps);
-  // splits without chunks own no partial: attn_combine_kernel only reads the first ceil(nch_total / cps) splits
+  const int ch_begin = split * rgs.cps;
+  const int ch_end = min(nch_total, ch_begin + min(rgs.cps, nch_total));
+  // a q tile ends before its sequence does: ranges behind it own no partial (attn_combine_kernel reads the first
+  // ceil(nch_total / cps) ranges only)
   if (p.n_split > 1 && ch_begin >= ch_end) return;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -156,23 +215,27 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32) paged_attn_kernel(AttnPar
       chunk_blk = bt[base / p.block_size];
       chunk_off = base % p.block_size;
     }
-#pragma unroll 4
+    if (page_aligned) {   // a thread keeps its 16-byte column; its rows are kAttThreads / SEG tokens apart
+      const int tok0 = threadIdx.x / SEG, seg = threadIdx.x % SEG;
+      const size_t step = (size_t)(kAttThreads / SEG) * p.KV * HD;
+      size_t off = (((size_t)max(chunk_blk, 0) * p.block_size + chunk_off + tok0) * p.KV + kvh) * HD + seg * 8;
+#pragma unroll
+      for (int tok = tok0; tok < kAttChunk; tok += kAttThreads / SEG, off += step) {
+        const bool valid = base + tok < kv_max && chunk_blk >= 0;
+        cp_async16(dk + tok * LDS + seg * 8, p.k_cache + (valid ? off : 0), valid);
+        cp_async16(dv + tok * LDS + seg * 8, p.v_cache + (valid ? off : 0), valid);
+      }
+      return;
+    }
     for (int idx = threadIdx.x; idx < kAttChunk * SEG; idx += kAttThreads) {
       const int tok = idx / SEG, seg = idx - tok * SEG;
       const int pos = base + tok;
       bool valid = pos < kv_max;
       size_t off = 0;
       if (valid) {
-        int blk, in_blk;
-        if (page_aligned) {
-          blk = chunk_blk;
-          in_blk = chunk_off + tok;
-        } else {
-          blk = bt[pos / p.block_size];
-          in_blk = pos % p.block_size;
-        }
+        const int blk = bt[pos / p.block_size], in_blk = pos % p.block_size;
         valid = blk >= 0;
-        off = (((size_t)blk * p.block_size + in_blk) * p.KV + kvh) * HD + seg * 8;
+        off = valid ? (((size_t)blk * p.block_size + in_blk) * p.KV + kvh) * HD + seg * 8 : 0;
       }
       cp_async16(dk + tok * LDS + seg * 8, p.k_cache + off, valid);
       cp_async16(dv + tok * LDS + seg * 8, p.v_cache + off, valid);
@@ -180,15 +243,25 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32) paged_attn_kernel(AttnPar
   };
 
   if (ch_begin < ch_end) {
-    load_chunk(ch_begin, 0);
-    cp_async_commit();
-    if (threadIdx.x == 0) trace_fine(TRF_ATTN + 0);  // q + first chunk requested
-    for (int ch = ch_begin; ch < ch_end; ++ch) {
-      const int stage = (ch - ch_begin) & 1;
-      if (ch + 1 < ch_end) load_chunk(ch + 1, stage ^ 1);
+#pragma unroll
+    for (int i = 0; i < kStages - 1; ++i) {
+      if (ch_begin + i < ch_end) load_chunk(ch_begin + i, i);
       cp_async_commit();
-      cp_async_wait<1>();
-      __syncthreads();
+    }
+    if (threadIdx.x == 0) trace_fine(TRF_ATTN + 0);  // q + first chunks requested
+    int stage = 0;
+    for (int ch = ch_begin; ch < ch_end; ++ch, stage = stage + 1 == kStages ? 0 : stage + 1) {
+      if (kStages == 2) {   // the next chunk is requested before this one is waited for
+        if (ch + 1 < ch_end) load_chunk(ch + 1, stage ^ 1);
+        cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
+      } else {
+        cp_async_wait<kStages - 2>();
+        __syncthreads();  // this chunk has landed, and everyone is done with the stage that is refilled now
+        if (ch + kStages - 1 < ch_end) load_chunk(ch + kStages - 1, stage == 0 ? kStages - 1 : stage - 1);
+        cp_async_commit();
+      }
       if (threadIdx.x == 0 && ch == ch_begin) trace_fine(TRF_ATTN + 1);  // first chunk landed
 
       const __nv_bfloat16* cK = sK + stage * kAttChunk * LDS;
@@ -249,12 +322,14 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32) paged_attn_kernel(AttnPar
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h) lrow[h] = lrow[h] * corr[h] + psum[h];
+      if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {   // (a factor of 1 changes no bit)
 #pragma unroll
-      for (int i = 0; i < ND; ++i) {
-        o[i][0] *= corr[0];
-        o[i][1] *= corr[0];
-        o[i][2] *= corr[1];
-        o[i][3] *= corr[1];
+        for (int i = 0; i < ND; ++i) {
+          o[i][0] *= corr[0];
+          o[i][1] *= corr[0];
+          o[i][2] *= corr[1];
+          o[i][3] *= corr[1];
+        }
       }
       // ---- O += P V ----
 #pragma unroll
@@ -274,7 +349,7 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32) paged_attn_kernel(AttnPar
           mma_bf16_16816(o[nd + 1], pa, vb[2], vb[3]);
         }
       }
-      __syncthreads();  // everyone done with this stage before it is refilled
+      if (kStages == 2) __syncthreads();  // everyone is done with this stage before it is refilled
     }
   }
   cp_async_wait<0>();
@@ -289,7 +364,7 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32) paged_attn_kernel(AttnPar
   }
   // Row stride HD + 8 floats (= 8 banks mod 32): the 8-byte fragment stores of a half-warp (rows g = 0..3, column
   // pairs t = 0..3) and the 16-byte row reads of the merge loop are both bank-conflict free.  With 8 warps the buffer
-  // is exactly as large as the K/V stages it reuses: 8 * 16 * (HD + 8) * 4 B.
+  // fits the K/V stages it reuses: 8 * 16 * (HD + 8) * 4 B.
   constexpr int LDO = HD + 8;
   float* sO = reinterpret_cast<float*>(att_smem);  // [NW warps][16 rows][LDO]: O | m | l
   {
@@ -345,7 +420,7 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32) paged_attn_kernel(AttnPar
 
 // merge split-KV partials: out = sum_s 2^(lse_s - max) o_s / sum_s 2^(lse_s - max).
 // One CTA per (token, head) row, HD/4 threads, each owning one float4 of the output.  Only the splits that had
-// chunks (n_active, recomputed from context_lens with the attention kernel's formula) are read, and every thread
+// chunks (n_active, recomputed from context_lens as the attention kernel does) are read, and every thread
 // issues all of its loads before using them, so the merge costs ~2 L2 round trips whatever n_split is.
 __global__ void attn_combine_kernel(AttnParams p, int hd) {
   __shared__ float sw[32];
@@ -359,8 +434,8 @@ __global__ void attn_combine_kernel(AttnParams p, int hd) {
   const int tq = min(p.TQ, p.Q - qt * p.TQ);
   const int kv_max = p.context_lens[b] - p.Q + qt * p.TQ + tq;
   const int nch_total = (kv_max + kAttChunk - 1) / kAttChunk;
-  const int cps = (nch_total + p.n_split - 1) / p.n_split;
-  const int n_active = (cps > 0) ? min(p.n_split, (nch_total + cps - 1) / cps) : 0;
+  const int cps = attn_ranges(p, -1, b).cps;
+  const int n_active = min(p.n_split, (nch_total + cps - 1) / cps);
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     const float lse = (lane < n_active) ? __ldcg(p.part_lse + row * p.n_split + lane) : -INFINITY;

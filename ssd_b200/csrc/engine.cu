@@ -517,7 +517,7 @@ struct Fwd {
   int64_t logits_ld;
 };
 
-static int attn_plan(const Model& m, int B, int Q, int* TQ, int* MT, int* nqt, int* nsplit, int max_ctx) {
+static int attn_plan(const Model& m, int B, int Q, int* TQ, int* MT, int* nqt, int* nsplit, int* target, int max_ctx) {
   const int G = m.H / m.KV;
   if (G < 1 || G > 16 || (m.H % m.KV) != 0) return fail("unsupported GQA ratio %d", G);
   // q tile of <= 32 rows (two 16-row MMA tiles, 8 warps = 4 token slices each): measured 7.3 us per 70B verify layer
@@ -530,31 +530,44 @@ static int attn_plan(const Model& m, int B, int Q, int* TQ, int* MT, int* nqt, i
   *TQ = tq;
   *MT = mt;
   *nqt = (Q + tq - 1) / tq;
-  const int ctas = m.KV * B * (*nqt);
-  int ns = (2 * num_sms() + ctas - 1) / ctas;
+  // a sequence is cut into at most kAttnMaxSplit ranges (one batch of loads per range in the merge)
   const int max_chunks = std::max(1, (max_ctx + kAttChunk - 1) / kAttChunk);
-  ns = std::max(1, std::min(std::min(ns, kAttnMaxSplit), max_chunks));
-  *nsplit = ns;
+  const int per = m.KV * (*nqt);
+  if (mt > 1 && B > 1) {   // equal ranges over the batch, two CTAs per SM
+    *target = std::max(1, std::min(2 * num_sms() / per, B * max_chunks));
+    *nsplit = *target <= B / 2 ? 1 : std::min({*target, kAttnMaxSplit, max_chunks});
+  } else {                 // single-row decode gains less from equal ranges than working them out costs (16 x 4000: 799 us a step, 823 with)
+    *target = 0;
+    *nsplit = std::max(1, std::min({(mt == 1 ? 3 : 2) * num_sms() / (per * B), kAttnMaxSplit, max_chunks}));
+  }
   return 0;
 }
 
-template <int HD, int MT>
+template <int HD, int MT, int OCC>
 static int launch_attn_inst(Launcher& L, const AttnParams& p, dim3 grid) {
-  const size_t smem = (size_t)2 * 2 * kAttChunk * (HD + 8) * 2;
+  const size_t smem = (size_t)attn_smem(HD, MT);
   static bool attr_set = false;
   if (!attr_set) {
-    CK(cudaFuncSetAttribute(paged_attn_kernel<HD, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaFuncSetAttribute(paged_attn_kernel<HD, MT, OCC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaFuncSetAttribute(paged_attn_kernel<HD, MT, OCC>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     attr_set = true;
   }
-  return L.go(paged_attn_kernel<HD, MT>, grid, dim3(attn_warps(MT) * 32), smem, p);
+  return L.go(paged_attn_kernel<HD, MT, OCC>, grid, dim3(attn_warps(MT) * 32), smem, p);
+}
+// More CTAs than SMs: two per SM (registers capped at 128).  8 x 8000 x 7 rows of a 70B layer 143 -> 123 us, 2003-token prompt of 4 8B
+// layers 4862 -> 4731 us; a 200-token context that one CTA per SM covers takes 1.2 us less with the registers.
+template <int HD, int MT>
+static int launch_attn_occ(Launcher& L, const AttnParams& p, dim3 grid) {
+  const long long ctas = (long long)grid.x * grid.y * grid.z;
+  return ctas > num_sms() ? launch_attn_inst<HD, MT, 2>(L, p, grid) : launch_attn_inst<HD, MT, 1>(L, p, grid);
 }
 static int launch_attn(Launcher& L, const AttnParams& p, int hd, int MT, dim3 grid) {
-  if (hd == 128 && MT == 1) return launch_attn_inst<128, 1>(L, p, grid);
-  if (hd == 128 && MT == 2) return launch_attn_inst<128, 2>(L, p, grid);
-  if (hd == 128 && MT == 4) return launch_attn_inst<128, 4>(L, p, grid);
-  if (hd == 64 && MT == 1) return launch_attn_inst<64, 1>(L, p, grid);
-  if (hd == 64 && MT == 2) return launch_attn_inst<64, 2>(L, p, grid);
-  if (hd == 64 && MT == 4) return launch_attn_inst<64, 4>(L, p, grid);
+  if (hd == 128 && MT == 1) return launch_attn_inst<128, 1, 3>(L, p, grid);
+  if (hd == 128 && MT == 2) return launch_attn_occ<128, 2>(L, p, grid);
+  if (hd == 128 && MT == 4) return launch_attn_occ<128, 4>(L, p, grid);
+  if (hd == 64 && MT == 1) return launch_attn_inst<64, 1, 3>(L, p, grid);
+  if (hd == 64 && MT == 2) return launch_attn_occ<64, 2>(L, p, grid);
+  if (hd == 64 && MT == 4) return launch_attn_occ<64, 4>(L, p, grid);
   return fail("unsupported head_dim %d (64 and 128 are built)", hd);
 }
 
@@ -562,18 +575,18 @@ static int enqueue_attention(Launcher& L, const bf16* q, const bf16* kc, const b
                              const int32_t* ctx_lens, bf16* out, float* part_o, float* part_lse, unsigned* counters,
                              int B, int Q, int H,
                              int KV, int hd, int block_size, int max_blocks, float scale, int TQ, int MT, int nqt,
-                             int nsplit) {
+                             int nsplit, int target) {
   AttnParams a;
   a.q = q; a.k_cache = kc; a.v_cache = vc; a.block_tables = bt; a.context_lens = ctx_lens; a.out = out;
   a.part_o = part_o; a.part_lse = part_lse;
   (void)counters;
   a.B = B; a.Q = Q; a.H = H; a.KV = KV; a.block_size = block_size; a.max_blocks = max_blocks;
-  a.n_split = nsplit; a.TQ = TQ; a.n_qtiles = nqt;
+  a.n_split = nsplit; a.target = target; a.TQ = TQ; a.n_qtiles = nqt;
   a.g_shift = -1;
   for (int sft = 0; sft < 5; ++sft)
     if ((H / KV) == (1 << sft)) a.g_shift = sft;
   a.scale_log2 = scale * 1.4426950408889634f;
-  CKI(launch_attn(L, a, hd, MT, dim3(KV, nsplit, B * nqt)));
+  CKI(launch_attn(L, a, hd, MT, dim3(KV, nsplit == 1 ? B : (target ? target + B : nsplit * B), nqt)));
   if (nsplit > 1) CKI(L.go(attn_combine_kernel, dim3(B * Q * H), dim3(32), 0, a, hd));
   return 0;
 }
@@ -739,8 +752,8 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
            w.positions, w.slot_mapping, w.context_lens,
            (f.which == SSDK_TARGET && tp > 1 && e->symm_n == tp) ? w.ar_state : (unsigned*)nullptr));
 
-  int TQ = 1, MT = 1, nqt = 1, nsplit = 1;
-  CKI(attn_plan(m, f.B, f.Q, &TQ, &MT, &nqt, &nsplit, e->max_ctx_hint));
+  int TQ = 1, MT = 1, nqt = 1, nsplit = 1, target = 1;
+  CKI(attn_plan(m, f.B, f.Q, &TQ, &MT, &nqt, &nsplit, &target, e->max_ctx_hint));
   if (M > kMaxTokens) nsplit = 1;   // (the partials are sized for kMaxTokens rows; so many q tiles fill the SMs by themselves)
   const float scale = 1.0f / sqrtf((float)m.hd);
 
@@ -801,7 +814,7 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
 
     // ---- attention over the paged cache ----
     CKI(enqueue_attention(L, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, w.att_o,
-                          w.att_lse, w.att_counters, f.B, f.Q, m.H, m.KV, m.hd, bs, mb, scale, TQ, MT, nqt, nsplit));
+                          w.att_lse, w.att_counters, f.B, f.Q, m.H, m.KV, m.hd, bs, mb, scale, TQ, MT, nqt, nsplit, target));
 
     // ---- output projection (row-parallel) ----
     const bool fuse_pub = use_symm && fused_publish_enabled() && M <= 64;
@@ -1181,9 +1194,11 @@ static int init_kernel_attrs() {
   SSDK_ATTR_G(128, EPI_BF16) SSDK_ATTR_G(128, EPI_PARTIAL) SSDK_ATTR_G(128, EPI_SILU) SSDK_ATTR_G(128, EPI_GLU)
   SSDK_ATTR_G(256, EPI_BF16) SSDK_ATTR_G(256, EPI_PARTIAL) SSDK_ATTR_G(256, EPI_SILU) SSDK_ATTR_G(256, EPI_GLU)
 #undef SSDK_ATTR_G
-#define SSDK_ATTR_A(HD, MT) \
-  CK(cudaFuncSetAttribute(paged_attn_kernel<HD, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 2 * kAttChunk * (HD + 8) * 2));
-  SSDK_ATTR_A(128, 1) SSDK_ATTR_A(128, 2) SSDK_ATTR_A(128, 4) SSDK_ATTR_A(64, 1) SSDK_ATTR_A(64, 2) SSDK_ATTR_A(64, 4)
+#define SSDK_ATTR_A(HD, MT, OCC) \
+  CK(cudaFuncSetAttribute(paged_attn_kernel<HD, MT, OCC>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD, MT))); \
+  CK(cudaFuncSetAttribute(paged_attn_kernel<HD, MT, OCC>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  SSDK_ATTR_A(128, 1, 3) SSDK_ATTR_A(128, 2, 1) SSDK_ATTR_A(128, 2, 2) SSDK_ATTR_A(128, 4, 1) SSDK_ATTR_A(128, 4, 2)
+  SSDK_ATTR_A(64, 1, 3) SSDK_ATTR_A(64, 2, 1) SSDK_ATTR_A(64, 2, 2) SSDK_ATTR_A(64, 4, 1) SSDK_ATTR_A(64, 4, 2)
 #undef SSDK_ATTR_A
   CK(cudaFuncSetAttribute(add_rmsnorm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
   return 0;
@@ -1703,11 +1718,11 @@ int ssdk_silu_mul(const void* gate_up, void* out, int M, int ffn, void* stream) 
   return L.go(silu_mul_kernel, dim3((M * ffn / 8 + 255) / 256), dim3(256), 0, g, (bf16*)out, M, ffn);
 }
 
-static int attn_plan_raw(int H, int KV, int B, int Q, int max_ctx, int* TQ, int* MT, int* nqt, int* nsplit) {
+static int attn_plan_raw(int H, int KV, int B, int Q, int max_ctx, int* TQ, int* MT, int* nqt, int* nsplit, int* target) {
   Model tmp;
   tmp.H = H;
   tmp.KV = KV;
-  return attn_plan(tmp, B, Q, TQ, MT, nqt, nsplit, max_ctx);
+  return attn_plan(tmp, B, Q, TQ, MT, nqt, nsplit, target, max_ctx);
 }
 
 int64_t ssdk_paged_attn_scratch_bytes(int batch, int q_len, int heads, int head_dim, int max_ctx) {
@@ -1722,15 +1737,13 @@ int ssdk_paged_attn(const void* q, const void* k_cache, const void* v_cache, con
   Launcher L;
   L.st = (cudaStream_t)stream;
   CKI(init_kernel_attrs());
-  int TQ, MT, nqt, nsplit;
-  CKI(attn_plan_raw(heads, kv_heads, batch, q_len, block_size * max_blocks_per_seq, &TQ, &MT, &nqt, &nsplit));
-  // the first 16 KB of the scratch hold the arrival counters (zero on entry)
-  CK(cudaMemsetAsync(scratch, 0, 16384, L.st));
+  int TQ, MT, nqt, nsplit, target;
+  CKI(attn_plan_raw(heads, kv_heads, batch, q_len, block_size * max_blocks_per_seq, &TQ, &MT, &nqt, &nsplit, &target));
   float* part_o = (float*)((uint8_t*)scratch + 16384);
   float* part_lse = part_o + (size_t)batch * q_len * heads * kAttnMaxSplit * head_dim;
   return enqueue_attention(L, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, block_tables, context_lens,
                            (bf16*)out, part_o, part_lse, (unsigned*)scratch, batch, q_len, heads, kv_heads, head_dim, block_size,
-                           max_blocks_per_seq, scale, TQ, MT, nqt, nsplit);
+                           max_blocks_per_seq, scale, TQ, MT, nqt, nsplit, target);
 }
 
 int ssdk_sample(const void* logits, int64_t ld, const float* temps, int B, int V, uint64_t seed, uint64_t step_id,
