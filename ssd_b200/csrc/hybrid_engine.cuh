@@ -975,6 +975,26 @@ struct HybRun {
     return n;
   }
 
+  // rows of whole 16-byte pieces (a thread then moves four channels at a time)
+  static bool whole16(int width, std::initializer_list<const void*> ps) {
+    uintptr_t a = 0;
+    for (const void* q : ps) a |= (uintptr_t)q;
+    return width % 4 == 0 && (a & 15) == 0;
+  }
+  static int row_threads(int width) { return std::max(64, std::min(512, (width / 4 + 31) / 32 * 32)); }
+  int rmsnorm(const float* x, const void* w, void* y, const int* rows, int n, float offset, const void* w2 = nullptr, void* y2 = nullptr) {
+    const int W = e->cfg.width;
+    if (whole16(W, {x, w, y, w2, y2}) && W <= 4 * ssdk::kHold * row_threads(W))
+      return L.go(ssdk::offset_rmsnorm_kernel<T, 4>, dim3(n), dim3(row_threads(W)), 0, x, (const T*)w, (T*)y, rows, W, e->cfg.eps, offset, (const T*)w2, (T*)y2);
+    return L.go(ssdk::offset_rmsnorm_kernel<T, 1>, dim3(n), dim3(256), 0, x, (const T*)w, (T*)y, rows, W, e->cfg.eps, offset, (const T*)w2, (T*)y2);
+  }
+  int postnorm(const float* y1, float s1, const float* y2, float s2, const void* w, void* xt) {
+    const int W = e->cfg.width;
+    if (whole16(W, {e->x, y1, y2, w, xt}) && W <= 4 * ssdk::kHold * row_threads(W))
+      return L.go(ssdk::postnorm_residual_kernel<T, 4>, dim3(M), dim3(row_threads(W)), 0, e->x, y1, s1, y2, s2, (const T*)w, W, e->cfg.eps, e->cfg.norm_offset, e->cfg.residual_mult, (T*)xt);
+    return L.go(ssdk::postnorm_residual_kernel<T, 1>, dim3(M), dim3(256), 0, e->x, y1, s1, y2, s2, (const T*)w, W, e->cfg.eps, e->cfg.norm_offset, e->cfg.residual_mult, (T*)xt);
+  }
+
   int rglru(HybLayer& Lr) {
     const ssdk_hyb_layer_cfg& c = Lr.c;
     const int W = e->cfg.width, R = c.inner, nb = c.blocks, bs = R / nb, taps = c.conv;
@@ -1104,7 +1124,7 @@ struct HybRun {
       else if (vec) CKI(L.go(ssdk::gqa_head_prep_kernel<T, 4, 32>, dim3(M, ys), dim3(256), smem, hp, rg));
       else CKI(L.go(ssdk::gqa_head_prep_kernel<T, 1, 32>, dim3(M, ys), dim3(256), smem, hp, rg));
     } else {
-      CKI(L.go(ssdk::gqa_prep_kernel<T>, dim3(M, H + G), dim3(32), 0, pa, rg));
+      CKI(L.go(ssdk::gqa_prep_kernel<T>, dim3(M, (H + G + ssdk::kPrepHeads - 1) / ssdk::kPrepHeads), dim3(32, ssdk::kPrepHeads), 0, pa, rg));
     }
     // tensor-core forms: bf16, heads of whole 16-byte pieces up to 128 wide, up to 16 query heads per key/value head
     const bool mma = !kF32 && e->use_gqa_mma && D % 8 == 0 && V % 8 == 0 && std::max(D, V) <= 128 && hpg <= 16 && ((uintptr_t)pool & 15) == 0;
@@ -1406,14 +1426,11 @@ struct HybRun {
       return fail("wkv, mlstm and latent attention are built for parallel blocks");
     CKI(run_mixer(Lr));
     const bool pair = Lr.c.mixer == SSDK_MIX_ATTN_DELTA;
-    CKI(L.go(ssdk::postnorm_residual_kernel<T>, dim3(M), dim3(256), 0, e->x, (const float*)e->mix_out, pair ? Lr.c.left_scale : 1.0f,
-             (const float*)(pair ? e->mix2 : nullptr), pair ? Lr.c.right_scale : 0.f, (const T*)Lr.t[SSDK_HT_NORM].p, W, g.eps, g.norm_offset,
-             g.residual_mult, xt));
+    CKI(postnorm(e->mix_out, pair ? Lr.c.left_scale : 1.0f, pair ? e->mix2 : nullptr, pair ? Lr.c.right_scale : 0.f, Lr.t[SSDK_HT_NORM].p, xt));
     if (Lr.c.mlp == SSDK_MLP_GLU) {
       CKI(check_tensor(Lr, SSDK_HT_NORM2, W, 1, "norm2"));
       CKI(glu(Lr));
-      CKI(L.go(ssdk::postnorm_residual_kernel<T>, dim3(M), dim3(256), 0, e->x, (const float*)e->mix_out, 1.0f, (const float*)nullptr, 0.f,
-               (const T*)Lr.t[SSDK_HT_NORM2].p, W, g.eps, g.norm_offset, g.residual_mult, xt));
+      CKI(postnorm(e->mix_out, 1.0f, nullptr, 0.f, Lr.t[SSDK_HT_NORM2].p, xt));
     }
     return 0;
   }
@@ -1512,8 +1529,7 @@ struct HybRun {
     if (next) CKI(check_sandwich_layer(*next));
     const void* next_w = next ? next->t[SSDK_HT_NORM].p : nullptr;
     if (li == 0)
-      CKI(L.go(ssdk::offset_rmsnorm_kernel<T>, dim3(M), dim3(256), 0, (const float*)e->x, (const T*)Lr.t[SSDK_HT_NORM].p, (T*)e->h, (const int*)nullptr,
-               g.width, g.eps, g.norm_offset, (const T*)nullptr, (T*)nullptr));
+      CKI(rmsnorm(e->x, Lr.t[SSDK_HT_NORM].p, e->h, nullptr, M, g.norm_offset));
     if (Lr.c.mixer == SSDK_MIX_ATTN_DELTA) return fail("the attention pair is built for serial blocks with one norm per sublayer");
     hin = fin = e->h;
     CKI(run_mixer(Lr));
@@ -1537,9 +1553,7 @@ struct HybRun {
     CKI(check_tensor(Lr, SSDK_HT_NORM, W, 1, "norm1"));
     if (scales) CKI(check_tensor(Lr, SSDK_HT_LS_MIX, W, 1, "ls1"));
     if (ff2) CKI(check_tensor(Lr, SSDK_HT_NORM2, W, 1, "norm2"));
-    CKI(L.go(ssdk::offset_rmsnorm_kernel<T>, dim3(M), dim3(256), 0, (const float*)e->x, (const T*)Lr.t[SSDK_HT_NORM].p, (T*)e->h,
-             (const int*)nullptr, W, e->cfg.eps, e->cfg.norm_offset, ff2 ? (const T*)Lr.t[SSDK_HT_NORM2].p : (const T*)nullptr,
-             ff2 ? (T*)e->h2 : (T*)nullptr));
+    CKI(rmsnorm(e->x, Lr.t[SSDK_HT_NORM].p, e->h, nullptr, M, e->cfg.norm_offset, ff2 ? Lr.t[SSDK_HT_NORM2].p : nullptr, ff2 ? e->h2 : nullptr));
     ssdk::CombineArgs ca = {};
     if (one) {
       const bool has_ff = Lr.c.mlp != SSDK_MLP_NONE;
@@ -1590,7 +1604,9 @@ struct HybRun {
     } else if (Lr.c.mlp != SSDK_MLP_NONE) {
       return fail("the gated dense feed-forward is built for serial blocks");
     }
-    return L.go(ssdk::block_combine_kernel<T>, dim3(M), dim3(256), 0, ca);
+    if (whole16(W, {ca.x, ca.mix, ca.ls1, ca.ls2, ca.routed, ca.shared, ca.ff_bias, ca.fin, ca.gz, ca.gz_bias}) && ca.ld_gz % 4 == 0)
+      return L.go(ssdk::block_combine_kernel<T, 4>, dim3(M, std::max(1, std::min((W / 4 + 127) / 128, 4 * num_sms() / M))), dim3(128), 0, ca);
+    return L.go(ssdk::block_combine_kernel<T, 1>, dim3(M), dim3(256), 0, ca);
   }
 };
 
@@ -1703,8 +1719,13 @@ static int hyb_forward_t(ssdk_hyb_engine* e, int n_seqs, int M, const int32_t* i
     run.L = Launcher();
     run.L.st = on; run.L.pdl = e->use_pdl;
     CK(cudaMemcpyAsync(d, hm, o * 4, cudaMemcpyHostToDevice, on));
-    CKI(run.L.go(ssdk::embed_rows_kernel<T>, dim3(M), dim3(128), 0, (const int*)(d + o_ids), (const T*)e->embed.p, e->x, g.width, g.vocab,
-                 g.embed_scale, (g.block == SSDK_BLOCK_SERIAL_POSTNORM && !std::is_same<T, float>::value) ? (T*)e->h : (T*)nullptr, run.streams()));
+    T* xt = (g.block == SSDK_BLOCK_SERIAL_POSTNORM && !std::is_same<T, float>::value) ? (T*)e->h : (T*)nullptr;
+    if (HybRun<T>::whole16(g.width, {e->embed.p, e->x}))
+      CKI(run.L.go(ssdk::embed_rows_kernel<T, 4>, dim3(M, std::max(1, std::min((g.width / 4 + 127) / 128, 4 * num_sms() / M))), dim3(128), 0, (const int*)(d + o_ids),
+                   (const T*)e->embed.p, e->x, g.width, g.vocab, g.embed_scale, xt, run.streams()));
+    else
+      CKI(run.L.go(ssdk::embed_rows_kernel<T, 1>, dim3(M), dim3(128), 0, (const int*)(d + o_ids), (const T*)e->embed.p, e->x, g.width, g.vocab,
+                   g.embed_scale, xt, run.streams()));
     for (int li = 0; li < g.n_layers; ++li) {
       CKI(run.layer(e->layers[li], li));
       if (residual_host) {
@@ -1721,8 +1742,7 @@ static int hyb_forward_t(ssdk_hyb_engine* e, int n_seqs, int M, const int32_t* i
     // (a factor on the logits is taken on the normed rows: the head is linear)
     if (g.block == SSDK_BLOCK_SERIAL_PRENORM || g.logit_scale != 1.0f)
       CKI(run.stream_norm(nullptr, e->final_norm.p, e->hn, d + o_want, n_want, g.logit_scale));
-    else CKI(run.L.go(ssdk::offset_rmsnorm_kernel<T>, dim3(n_want), dim3(256), 0, (const float*)e->x, (const T*)e->final_norm.p, (T*)e->hn,
-                 (const int*)(d + o_want), g.width, g.eps, g.norm_offset, (const T*)nullptr, (T*)nullptr));
+    else CKI(run.rmsnorm(e->x, e->final_norm.p, e->hn, d + o_want, n_want, g.norm_offset));
     CKI(run.lin(e->hn, g.width, e->head.p, g.width, e->logits, g.vocab, n_want, g.vocab, g.width));
     if (!sample) return 0;
     const size_t n = (size_t)n_want * g.vocab;
