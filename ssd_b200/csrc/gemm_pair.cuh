@@ -13,7 +13,7 @@
 //   warp 0     loads: 6 stages of {128 weight rows, up to 128 token rows} x 64 k, 128B-swizzled; both CTAs' bytes count on the
 //              leader's full barrier
 //   warp 1     leader only: tcgen05.mma.cta_group::2 M = 256, N = the tile's tokens rounded up to 64; commits free the stage in both CTAs
-//   warps 2-5  epilogue of this CTA's 128 weight rows: fp32 store, or act(gate) * up in bf16.  For the latter the weight rows of a tile
+//   warps 2-5  epilogue of this CTA's 128 weight rows: fp32 or bf16 store, or act(gate) * up in bf16.  For the latter the weight rows of a tile
 //              alternate in runs of 16 gate and 16 up rows, so that gate and up of an output column sit 16 lanes apart in one warp
 // Grouped mode (mixture of experts): a device-side list of row tiles, each of one expert, as in gemm_ws_kernel.
 // The order of the sums over K is that of gemm_ws_kernel without split-K: the results are the same bits.
@@ -34,12 +34,15 @@ constexpr int kPairXBox = 128, kPairXSmall = 32, kPairGluRun = 16;
 enum { GLU_SILU = 0, GLU_GELU = 1, GLU_SILU_ROUNDED = 2 };
 
 struct GemmPairParams {
-  void* out;          // EPI_PARTIAL: fp32 [M, ldo]; EPI_GLU: bf16 [M, ldo]
+  void* out;          // EPI_PARTIAL: fp32 [M, ldo]; EPI_GLU, EPI_BF16: bf16 [M, ldo]
   int M, N, ldo;      // N: output columns (EPI_GLU: of the product act(gate) * up; the up rows start N rows behind the gate rows)
   int num_kb;         // K / 64
   int w_tiles;        // tiles along the weight rows: 256 columns (EPI_PARTIAL) or 128 (EPI_GLU) of the output
   int chunks;         // row chunks of kPairTokens tokens (dense)
   int act;            // EPI_GLU: GLU_*
+  // dense: products of the same shape side by side (heads): product b reads X's columns from b x_step, the weight rows from b N, and
+  // writes out + b out_step
+  int batch, x_step, out_step;
   // grouped mode: see GemmParams
   const int* g_tile_expert;
   const int* g_tile_row0;
@@ -159,11 +162,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 
   const bool grouped = p.g_tile_expert != nullptr;
   const int row_tiles = grouped ? *p.g_n_tiles : p.chunks;
-  const int tiles = row_tiles * p.w_tiles;
-  // tile t: row chunk t % row_tiles (the inner index), weight rows t / row_tiles
-  struct Tile { int m0, rows, n, col, ex; };   // first token, valid tokens, multiplied tokens, this CTA's first output column, expert
+  const int per = row_tiles * p.w_tiles, tiles = grouped ? per : per * p.batch;
+  // tile t: row chunk (the inner index), weight rows, product of the batch
+  struct Tile { int m0, rows, n, col, ex, b; };   // first token, valid tokens, multiplied tokens, this CTA's first output column, expert, product
   auto tile_of = [&](int t) {
     Tile r;
+    r.b = grouped ? 0 : t / per;
+    t -= r.b * per;
     const int wt = t / row_tiles, c = t - wt * row_tiles;
     r.ex = 0;
     if (grouped) {
@@ -184,7 +189,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         const Tile tl = tile_of(t);
         const int half = tl.n >> 1, x0 = tl.m0 + (int)rank * half;
         const bool big = half > 64;
-        const int w_row = tl.ex * p.g_expert_rows + tl.col;
+        const int w_row = tl.ex * p.g_expert_rows + tl.b * p.N + tl.col, kx = tl.b * p.x_step;
         const uint32_t bytes = 2u * (16384u + (big ? (uint32_t)kPairXBox : (uint32_t)half) * 128u);
         for (int kb = 0; kb < p.num_kb; ++kb, ++it) {
           const int s = it % kPairStages;
@@ -196,9 +201,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           const int k = kb * kBlockK;
           if (EPI == EPI_GLU) tma_load_5d_pair(a_s, &tmW, bar, k, tl.col / kPairGluRun, tl.ex);
           else tma_load_2d_pair(a_s, &tmW, bar, k, w_row, kEvictNormal);
-          if (big) tma_load_2d_pair(b_s, &tmX, bar, k, x0, kEvictNormal);
+          if (big) tma_load_2d_pair(b_s, &tmX, bar, kx + k, x0, kEvictNormal);
           else
-            for (int b = 0; b < half; b += kPairXSmall) tma_load_2d_pair(b_s + b * 128, &tmXs, bar, k, x0 + b, kEvictNormal);
+            for (int b = 0; b < half; b += kPairXSmall) tma_load_2d_pair(b_s + b * 128, &tmXs, bar, kx + k, x0 + b, kEvictNormal);
         }
       }
       // the last commits of the leader reach this CTA's barriers before it leaves
@@ -260,10 +265,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             const float a = p.act == GLU_GELU ? 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) : __fdividef(g, 1.0f + __expf(-g));
             if (n < p.N && m + (lo ? 0 : 1) < left) out[(size_t)m * p.ldo] = f2bf(a * u);
           }
+        } else if (EPI == EPI_BF16) {
+          const int n = tl.col + q * 32 + lane;
+          if (n < p.N) {
+            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)tl.b * p.out_step + (size_t)(tl.m0 + m0) * p.ldo + n;
+#pragma unroll
+            for (int m = 0; m < 32; ++m)
+              if (m < left) out[(size_t)m * p.ldo] = f2bf(__uint_as_float(r[m]));
+          }
         } else {
           const int n = tl.col + q * 32 + lane;
           if (n < p.N) {
-            float* out = reinterpret_cast<float*>(p.out) + (size_t)(tl.m0 + m0) * p.ldo + n;
+            float* out = reinterpret_cast<float*>(p.out) + (size_t)tl.b * p.out_step + (size_t)(tl.m0 + m0) * p.ldo + n;
             if (left >= 32) {
 #pragma unroll
               for (int m = 0; m < 32; ++m) out[(size_t)m * p.ldo] = __uint_as_float(r[m]);

@@ -583,16 +583,27 @@ __global__ void gqa_decode_merge_diff_kernel(const GqaDecodeArgs p, const Ragged
 }
 
 // o [G, M, H/G, V] fp32 (group-major) and gate pre-activations gz[m * ldg + h * V + v] -> y [M, H V] (T) = o * sigmoid(gz), rows row0 ..
-template <typename T>
+// grid (rows, column blocks).  VEC 4: V and ldg multiples of 4, whole 16-byte pieces (8-byte ones of a bf16 y).  2000 rows of 2048: 25 -> 13 us
+template <typename T, int VEC>
 __global__ void attn_gate_kernel(const float* __restrict__ o, const float* __restrict__ gz, int ldg, T* __restrict__ y, int M, int H,
                                  int G, int V, int row0) {
   pdl_launch_dependents();
   pdl_wait();
   const int m = row0 + blockIdx.x, hpg = H / G;
-  for (int i = threadIdx.x; i < H * V; i += blockDim.x) {
+  for (int i = (blockIdx.y * blockDim.x + threadIdx.x) * VEC; i < H * V; i += gridDim.y * blockDim.x * VEC) {
     const int hd = i / V, v = i - hd * V, g = hd / hpg;
-    const float ov = o[(((size_t)g * M + m) * hpg + (hd - g * hpg)) * V + v];
-    st_f<T>(y + (size_t)m * H * V + i, gz ? ov * sigmoid_f(gz[(size_t)m * ldg + i]) : ov);
+    const float* ov = o + (((size_t)g * M + m) * hpg + (hd - g * hpg)) * V + v;
+    if constexpr (VEC == 4) {
+      const float4 f = *reinterpret_cast<const float4*>(ov);
+      float out[4] = {f.x, f.y, f.z, f.w};
+      if (gz) {
+        const float4 z = *reinterpret_cast<const float4*>(gz + (size_t)m * ldg + i);
+        out[0] *= sigmoid_f(z.x); out[1] *= sigmoid_f(z.y); out[2] *= sigmoid_f(z.z); out[3] *= sigmoid_f(z.w);
+      }
+      st_four<T>(y + (size_t)m * H * V + i, out);
+    } else {
+      st_f<T>(y + (size_t)m * H * V + i, gz ? *ov * sigmoid_f(gz[(size_t)m * ldg + i]) : *ov);
+    }
   }
 }
 

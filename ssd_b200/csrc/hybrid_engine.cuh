@@ -428,6 +428,24 @@ struct HybRun {
   }
   // (gemm_ws_kernel asks for its first weight tiles, and in grouped mode reads the tile list, before it waits for the kernel in front:
   // launches whose "weights" or list that kernel writes start after it)
+  // per head h: C[:, h out_step ..] = A[:, h x_step .. + K] W[h N .. + N, :]^T (bf16 or fp32 out); H = 1: one product with a bf16 result.
+  // Other calls take the batched tile.  2000 rows, 16 heads: 128 -> 512 columns 70 -> 27 us, 512 -> 128 columns 31 -> 20 us
+  int lin_heads(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int m, int N, int K, bool out_t, int H, int x_step, int out_step) {
+    const bool ok = std::is_same<T, bf16>::value && e->use_tc && pair_ok(m) && K % kBlockK == 0 && x_step % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 &&
+                    (H == 1 || ldw == K) && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+    if (!ok) return lin(A, lda, W, ldw, C, ldc, m, N, K, out_t, H, x_step, (long long)N * ldw, out_step, false);
+    const CUtensorMap* tm;   // (copied: a later lookup may empty the table)
+    CKI(e->tmap(W, (int64_t)H * N, K, 128, &tm, ldw == K ? 0 : ldw));
+    const CUtensorMap tmW = *tm;
+    CKI(e->tmap(A, m, lda, kPairXBox, &tm));
+    const CUtensorMap tmX = *tm;
+    CKI(e->tmap(A, m, lda, kPairXSmall, &tm));
+    const CUtensorMap tmXs = *tm;
+    GemmPairParams p = {};
+    p.out = C; p.M = m; p.N = N; p.ldo = ldc; p.num_kb = K / kBlockK; p.w_tiles = (N + 255) / 256; p.chunks = (m + kPairTokens - 1) / kPairTokens;
+    p.batch = H; p.x_step = x_step; p.out_step = out_step;
+    return launch_gemm_pair(L, out_t ? EPI_BF16 : EPI_PARTIAL, tmW, tmX, tmXs, p, p.w_tiles * p.chunks * H);
+  }
   int lin_tc(const void* A, const void* W, float* C, int m_total, int N, int K, int ldw, bool fresh_w = false) {
     if (fresh_w) L.barrier_op();
     if (pair_ok(m_total)) return lin_pair(false, A, W, C, m_total, N, K, ldw, false);
@@ -672,6 +690,23 @@ struct HybRun {
     return lin(e->t1, H * V, Lr.t[SSDK_HT_MIX_OUT].p, H * V, e->mix_out, W, M, W, H * V);
   }
 
+  int attn_gate(const float* o, const float* gate, int ldg, void* y, int n, int m_total, int H, int G, int V, int row0) {
+    const int per = row_blocks(H * V / 4, n);
+    if (V % 4 == 0 && whole16(gate ? ldg : 4, {o, gate, y}))
+      return L.go(ssdk::attn_gate_kernel<T, 4>, dim3(n, per), dim3(128), 0, o, gate, ldg, (T*)y, m_total, H, G, V, row0);
+    return L.go(ssdk::attn_gate_kernel<T, 1>, dim3(n), dim3(256), 0, o, gate, ldg, (T*)y, m_total, H, G, V, row0);
+  }
+  // att_s [n, ld] -> att_p: a row of up to 8 ld-pieces per thread stays in registers
+  int softmax(int n, const void* sink, int H, int ld, int pos_first, float scale, int rows_per_batch, float sink_const, int key_first, int kept, ssdk::KeyMask mask) {
+    const float* sc = e->att_s;
+    T* pr = (T*)e->att_p;
+    const T* sk = (const T*)sink;
+    const int threads = ld <= 1024 ? 128 : 256, hold = (ld + 4 * threads - 1) / (4 * threads);
+    if (ld % 4 == 0 && hold <= 2) return L.go(ssdk::sink_softmax_row_kernel<T, 2>, dim3(n), dim3(threads), 0, sc, pr, sk, H, ld, pos_first, scale, rows_per_batch, sink_const, key_first, kept, mask);
+    if (ld % 4 == 0 && hold <= 8) return L.go(ssdk::sink_softmax_row_kernel<T, 8>, dim3(n), dim3(threads), 0, sc, pr, sk, H, ld, pos_first, scale, rows_per_batch, sink_const, key_first, kept, mask);
+    return L.go(ssdk::sink_softmax_kernel<T>, dim3(n), dim3(256), 0, sc, pr, sk, H, ld, pos_first, scale, rows_per_batch, sink_const, key_first, kept, mask);
+  }
+
   // query rows per block of a windowed attention's portion path
   static int window_block(int win) { return std::max(128, (win + 63) / 64 * 64); }
   // rows of the query block that starts at position pos, `left` rows remain: short blocks keep the scores to the rows + the keys
@@ -753,10 +788,11 @@ struct HybRun {
       }
     }
     const int Wd = KR + R;
-    CKI(L.go(ssdk::latent_q_kernel<T>, dim3(M, H), dim3(64), 0, q, ldq, (T*)e->t1, (T*)e->qcat, (const float*)Lr.inv_freq, rg,
-             H, D, R, KR, c.rot_dims, c.rot_interleaved));
+    const bool v4 = D % 4 == 0 && R % 4 == 0 && whole16(ldq, {q, e->t1});
+    CKI(L.go(v4 ? ssdk::latent_q_kernel<T, 4> : ssdk::latent_q_kernel<T, 1>, dim3(M, (H + ssdk::kQHeads - 1) / ssdk::kQHeads),
+             dim3(32 * ssdk::kQHeads), 0, q, ldq, (T*)e->t1, (T*)e->qcat, (const float*)Lr.inv_freq, rg, H, D, R, KR, c.rot_dims, c.rot_interleaved));
     // absorption: qcat[m, h, :kv_rank] = W_uk,h^T qn[m, h, :]
-    CKI(lin(e->t1, H * D, Lr.t[SSDK_HT_LAT_UKT].p, D, e->qcat, H * Wd, M, KR, D, true, H, D, (long long)KR * D, Wd));
+    CKI(lin_heads(e->t1, H * D, Lr.t[SSDK_HT_LAT_UKT].p, D, e->qcat, H * Wd, M, KR, D, true, H, D, Wd));
     // single-token sequences (decode) share ONE fused launch + a merge; the others take the GEMM path below
     bool fused_decode = false;
     {
@@ -801,7 +837,7 @@ struct HybRun {
       by_position = true;
       // the portion's keys: positions lo .. p0 + n - 1 (the mask hides the positions before lo from every row of the portion)
       const int lo = mask.first(p0), ctx = p0 + n - lo, ctx_pad = (ctx + kpad - 1) / kpad * kpad;
-      CKI(L.go(ssdk::latent_gather_kernel<T>, dim3(ctx_pad), dim3(128), 0, (const T*)pool, (T*)e->keys, (T*)e->lat_t, rg, s, lo, ctx, ctx_pad,
+      CKI(L.go(ssdk::latent_gather_kernel<T>, dim3(ctx_pad / ssdk::kGatherKeys, (Wd + 127) / 128), dim3(128), 0, (const T*)pool, (T*)e->keys, (T*)e->lat_t, rg, s, lo, ctx, ctx_pad,
                KR, Wd));
       const int qb = (int)std::max<size_t>(1, e->att_elems / ((size_t)H * ctx_pad));
       for (int q0 = 0, nq; q0 < n; q0 += nq) {
@@ -814,10 +850,11 @@ struct HybRun {
         const T* lat_t = (const T*)e->lat_t + kb;
         // scores: keys are the 128-row operand, (query, head) rows the tokens
         CKI(lin(qrows, Wd, krows, Wd, e->att_s, cb, rows, cb, Wd, false, 1, 0, 0, 0, tc_attn, true));
-        CKI(L.go(ssdk::sink_softmax_kernel<T>, dim3(rows), dim3(256), 0, (const float*)e->att_s, (T*)e->att_p,
-                 (const T*)sink, H, cb, p0 + q0, c.attn_scale, rows, 0.f, lo + kb, 0, mask));
+        CKI(softmax(rows, sink, H, cb, p0 + q0, c.attn_scale, rows, 0.f, lo + kb, 0, mask));
         T* o_rows = (T*)e->t0 + (size_t)(r0 + q0) * H * KR;
-        if (tc_attn && tc_ok(e->att_p, cb, lat_t, ctx_pad, KR, KR, cb)) {
+        if (tc_attn && pair_ok(rows) && tc_ok(e->att_p, cb, lat_t, ctx_pad, KR, KR, cb)) {
+          CKI(lin_heads(e->att_p, cb, lat_t, ctx_pad, o_rows, KR, rows, KR, cb, true, 1, 0, 0));
+        } else if (tc_attn && tc_ok(e->att_p, cb, lat_t, ctx_pad, KR, KR, cb)) {
           // P C: the transposed latents [kv_rank, ctx_pad] are the 128-row operand, read with the row stride of the gather
           CKI(lin_tc(e->att_p, lat_t, e->att_o, rows, KR, cb, ctx_pad, true));
           CKI(L.go(ssdk::cast_cols_kernel<T>, dim3(rows), dim3(128), 0, (const float*)e->att_o, KR, o_rows, KR, KR));
@@ -829,10 +866,10 @@ struct HybRun {
     // per-head value projection of the latent output, rounded to T for the output projection (after the sigmoid gate on
     // the concatenated heads, if the layer has one: the product stays fp32 up to the gate)
     if (gate) {
-      CKI(lin(e->t0, H * KR, Lr.t[SSDK_HT_LAT_UV].p, KR, e->p1, H * V, M, V, KR, false, H, KR, (long long)V * KR, V));
-      CKI(L.go(ssdk::attn_gate_kernel<T>, dim3(M), dim3(256), 0, (const float*)e->p1, gate, ldq, (T*)e->t1, M, H, 1, V, 0));
+      CKI(lin_heads(e->t0, H * KR, Lr.t[SSDK_HT_LAT_UV].p, KR, e->p1, H * V, M, V, KR, false, H, KR, V));
+      CKI(attn_gate(e->p1, gate, ldq, e->t1, M, M, H, 1, V, 0));
     } else {
-      CKI(lin(e->t0, H * KR, Lr.t[SSDK_HT_LAT_UV].p, KR, e->t1, H * V, M, V, KR, true, H, KR, (long long)V * KR, V));
+      CKI(lin_heads(e->t0, H * KR, Lr.t[SSDK_HT_LAT_UV].p, KR, e->t1, H * V, M, V, KR, true, H, KR, V));
     }
     return lin(e->t1, H * V, Lr.t[SSDK_HT_MIX_OUT].p, H * V, e->mix_out, W, M, W, H * V);
   }
@@ -981,6 +1018,8 @@ struct HybRun {
     for (const void* q : ps) a |= (uintptr_t)q;
     return width % 4 == 0 && (a & 15) == 0;
   }
+  // CTAs of 128 threads per row of `pieces` 16-byte pieces: one per 128 pieces, about four per SM in all
+  static int row_blocks(int pieces, int rows) { return std::max(1, std::min((pieces + 127) / 128, 4 * num_sms() / rows)); }
   static int row_threads(int width) { return std::max(64, std::min(512, (width / 4 + 31) / 32 * 32)); }
   int rmsnorm(const float* x, const void* w, void* y, const int* rows, int n, float offset, const void* w2 = nullptr, void* y2 = nullptr) {
     const int W = e->cfg.width;
@@ -1204,13 +1243,12 @@ struct HybRun {
         const T* qrows = (const T*)e->qcat + (size_t)(r0 + q0) * hpg * D;
         CKI(lin(qrows, D, (const T*)e->keys + (size_t)kb * D, D, e->att_s, cb, rows, cb, D, false, G, (long long)M * hpg * D, (long long)ctx_pad * D,
                 (long long)rows * cb, false));
-        CKI(L.go(ssdk::sink_softmax_kernel<T>, dim3(G * rows), dim3(256), 0, (const float*)e->att_s, (T*)e->att_p, (const T*)sinks, hpg, cb,
-                 p0 + q0, c.attn_scale, rows, sink_const, lo + kb, kept, mask));
+        CKI(softmax(G * rows, sinks, hpg, cb, p0 + q0, c.attn_scale, rows, sink_const, lo + kb, kept, mask));
         CKI(lin(e->att_p, cb, (const T*)e->lat_t + kb, ctx_pad, og + (size_t)(r0 + q0) * hpg * V, V, rows, V, cb, false, G, (long long)rows * cb,
                 (long long)V * ctx_pad, (long long)M * hpg * V, false));
       }
       if (maps == 2) CKI(L.go(ssdk::diff_heads_kernel<T>, dim3(n, (H / 2 + 3) / 4), dim3(128), 0, (const float*)og, diff, (T*)y, M, H, G, V, r0));
-      else CKI(L.go(ssdk::attn_gate_kernel<T>, dim3(n), dim3(256), 0, (const float*)og, gate, ld_gate, (T*)y, M, H, G, V, r0));
+      else CKI(attn_gate(og, gate, ld_gate, y, n, M, H, G, V, r0));
     }
     return 0;
   }
@@ -1605,7 +1643,7 @@ struct HybRun {
       return fail("the gated dense feed-forward is built for serial blocks");
     }
     if (whole16(W, {ca.x, ca.mix, ca.ls1, ca.ls2, ca.routed, ca.shared, ca.ff_bias, ca.fin, ca.gz, ca.gz_bias}) && ca.ld_gz % 4 == 0)
-      return L.go(ssdk::block_combine_kernel<T, 4>, dim3(M, std::max(1, std::min((W / 4 + 127) / 128, 4 * num_sms() / M))), dim3(128), 0, ca);
+      return L.go(ssdk::block_combine_kernel<T, 4>, dim3(M, row_blocks(W / 4, M)), dim3(128), 0, ca);
     return L.go(ssdk::block_combine_kernel<T, 1>, dim3(M), dim3(256), 0, ca);
   }
 };
