@@ -30,6 +30,8 @@ struct HybLayer {
   float* decay_pow = nullptr; // retention: device, [heads, kRetChunk + 1] powers of the heads' decays
 };
 
+constexpr int kFewTile = 16;   // rows of a routed expert's tile in calls of few rows: the narrowest of gemm_ws_kernel
+
 struct HybGraph {            // a decode step's launches
   cudaGraphExec_t exec = nullptr;
   bool seen = false;
@@ -79,7 +81,7 @@ struct ssdk_hyb_engine {
   // tcgen05 path of the dense bf16 products: TMA descriptors by (pointer, rows, K, box rows), split-K partials
   bool use_tc = true;
   bool use_decode_attn = true;  // fused single-token latent attention (SSDK_HYB_DECODE_ATTN=0: GEMM path for every row)
-  bool use_tc_experts = true;   // routed experts of calls with many rows on the grouped tcgen05 GEMM (SSDK_HYB_TC_EXPERTS=0: mma.sync tile)
+  bool use_tc_experts = true;   // routed experts on the grouped tcgen05 GEMM (SSDK_HYB_TC_EXPERTS=0: mma.sync tile)
   bool use_tc_scores = true;    // score GEMM of latent-attention portions on the tcgen05 GEMM (SSDK_HYB_TC_SCORES=0: mma.sync tile)
   bool use_gqa_mma = true;      // grouped-query attention on the tensor cores (SSDK_HYB_GQA_MMA=0: GEMMs around a softmax, CUDA-core decode)
   bool use_tc_glu = true;       // gated feed-forward's activation in the epilogue of the tcgen05 GEMM (SSDK_HYB_TC_GLU=0: a kernel of its own)
@@ -348,7 +350,7 @@ static int64_t hyb_carve(ssdk_hyb_engine* e, uint8_t* base) {
   e->rz = (float*)take(cap * e->w_e * 4);
   e->wts = (float*)take(A * 4);
   e->sel = (int*)take(A * 4); e->apos = (int*)take(A * 4); e->arow = (int*)take(A * 4);
-  e->max_tiles = (int)(A / kLinBM + e->w_e + 1);
+  e->max_tiles = (int)(A / kFewTile + e->w_e + 1);
   e->tile_expert = (int*)take(e->max_tiles * 4); e->tile_row0 = (int*)take(e->max_tiles * 4);
   e->tile_rows = (int*)take(e->max_tiles * 4);
   e->n_tiles = (int*)take(4); e->n_rows = (int*)take(4);
@@ -391,7 +393,7 @@ struct HybRun {
 
   template <typename OutT>
   int lin_args(const ssdk::LinearArgs& a, int rows_hint, int batch) {
-    dim3 grid((a.N + ssdk::kLinBN - 1) / ssdk::kLinBN, a.tile_expert ? e->max_tiles : (rows_hint + ssdk::kLinBM - 1) / ssdk::kLinBM, batch);
+    dim3 grid((a.N + ssdk::kLinBN - 1) / ssdk::kLinBN, a.tile_expert ? rows_hint / ssdk::kLinBM + e->w_e + 1 : (rows_hint + ssdk::kLinBM - 1) / ssdk::kLinBM, batch);
     if constexpr (std::is_same<T, bf16>::value) {
       const bool vec = a.K % 8 == 0 && a.lda % 8 == 0 && a.ldw % 8 == 0 && a.sA % 8 == 0 && a.sW % 8 == 0 && a.sW_expert % 8 == 0 &&
                        ((uintptr_t)a.A & 15) == 0 && ((uintptr_t)a.W & 15) == 0;
@@ -908,13 +910,16 @@ struct HybRun {
     ra.top = top; ra.groups = c.groups; ra.keep = c.keep; ra.softmax = c.route_top_softmax ? 2 : c.route_softmax; ra.group_best = c.group_best;
     ra.renorm = c.route_renorm; ra.route_scale = c.route_scale;
     CKI(L.go(ssdk::group_topk_router_kernel<T>, dim3((M + ssdk::kRouterWarps - 1) / ssdk::kRouterWarps), dim3(ssdk::kRouterWarps * 32), 0, ra));
-    // many rows in bf16 with whole k-blocks: the grouped tcgen05 GEMM over rows gathered per expert (tiles of 128 rows);
-    // else the mma.sync / FMA tile, which gathers by index itself (tiles of kLinBM rows)
-    const bool tc_moe = !kF32 && e->use_tc && e->use_tc_experts && A >= 256 && W % kBlockK == 0 && ff % kBlockK == 0 &&
+    // bf16 with whole k-blocks: the grouped tcgen05 GEMM over rows gathered per expert; else the mma.sync / FMA tile, which gathers by
+    // index itself (tiles of kLinBM rows).  Below 256 routed rows an expert gets a few, the weights' bytes bound the call, and a tile
+    // of kFewTile rows streams them through deeper stages than the mma.sync tile does: 1, 2, 4, 8 decoding sequences, 32 experts of
+    // 2048 x 1024, top 4: 244, 267, 291, 311 -> 210, 221, 237, 265 us a call (tiles of 32: 211, 224, 239, 269); 16 experts of
+    // 1024 x 512: 168, 174, 191, 210 -> 169, 172, 180, 196; prompts of 24 and 50 tokens 293, 322 -> 266, 281
+    const bool tc_moe = !kF32 && e->use_tc && e->use_tc_experts && W % kBlockK == 0 && ff % kBlockK == 0 &&
                         (((uintptr_t)Lr.t[SSDK_HT_EXPERT_IN].p | (uintptr_t)Lr.t[SSDK_HT_EXPERT_OUT].p) & 15) == 0;
     const bool silu_glu = c.expert_glu && c.expert_act == SSDK_ACT_SILU, glu = tc_moe && silu_glu && e->use_tc_glu;   // activation in the GEMM's epilogue
     const bool split = split_ok(fin, W, Lr.t[SSDK_HT_EXPERT_IN].p, W, A, Nin, W, 1, 0, 0) && split_ok(e->ey, ff, Lr.t[SSDK_HT_EXPERT_OUT].p, ff, A, W, ff, 1, 0, 0);
-    const int tile = split ? kSplitTokens : (!tc_moe ? ssdk::kLinBM : (pair_ok(M) && (!glu || ff % kPairGluRun == 0) ? kPairTokens : 128));
+    const int tile = split ? kSplitTokens : (!tc_moe ? ssdk::kLinBM : (pair_ok(M) && (!glu || ff % kPairGluRun == 0) ? kPairTokens : A < 256 ? kFewTile : 128));
     ssdk::PlanArgs pa;
     pa.sel = e->sel; pa.apos = e->apos; pa.arow = e->arow; pa.tile_expert = e->tile_expert; pa.tile_row0 = e->tile_row0;
     pa.tile_rows = e->tile_rows; pa.n_tiles = e->n_tiles; pa.n_rows = e->n_rows; pa.A = A; pa.E = Et; pa.top = top; pa.tile = tile;
