@@ -21,6 +21,7 @@
 #include "elementwise.cuh"
 #include "gemm.cuh"
 #include "gemm_pair.cuh"
+#include "prompt_attention.cuh"
 #include "gemm_split.cuh"
 #include "sampling.cuh"
 #include "draft_stream.cuh"
@@ -134,6 +135,19 @@ static int make_tmap_glu(CUtensorMap* tm, const void* ptr, int64_t ff, int64_t K
   CUresult r = g_encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(ptr), gdim, gstride, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail("cuTensorMapEncodeTiled failed (%d) gate | up rows of %lld x %lld x %lld", (int)r, (long long)experts, (long long)ff, (long long)K);
+  return 0;
+}
+
+// rows [rows][heads][hd] as {column, head, row}; box: 64 columns x box_heads x box_rows
+static int make_tmap_heads(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t heads, int hd, int box_heads, int box_rows) {
+  CKI(get_encode());
+  if (hd % 64 != 0 || ((uintptr_t)ptr & 15) != 0) return fail("TMA: heads of %d", hd);
+  cuuint64_t gdim[3] = {(cuuint64_t)hd, (cuuint64_t)heads, (cuuint64_t)rows};
+  cuuint64_t gstride[2] = {(cuuint64_t)hd * 2, (cuuint64_t)heads * hd * 2};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_heads, (cuuint32_t)box_rows}, estr[3] = {1, 1, 1};
+  CUresult r = g_encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), gdim, gstride, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail("cuTensorMapEncodeTiled failed (%d) rows of %lld heads of %d x %lld", (int)r, (long long)heads, hd, (long long)rows);
   return 0;
 }
 
@@ -301,6 +315,18 @@ struct XMapCache {
     *out = &it->second;
     return 0;
   }
+  // rows of heads (queries, cached keys and values) of prompt_attn_kernel
+  int get_heads(const void* ptr, int64_t rows, int heads, int hd, int box_heads, int box_rows, const CUtensorMap** out) {
+    auto key = std::make_tuple(ptr, (hd << 16) | (heads << 5) | box_heads, -1 - box_rows, (int)rows);
+    auto it = maps.find(key);
+    if (it == maps.end()) {
+      CUtensorMap tm;
+      CKI(make_tmap_heads(&tm, ptr, rows, heads, hd, box_heads, box_rows));
+      it = maps.emplace(key, tm).first;
+    }
+    *out = &it->second;
+    return 0;
+  }
 };
 
 // ------------------------------------------------------------------------------------------
@@ -380,6 +406,7 @@ struct ssdk_engine {
   void* ws_base = nullptr;
   int64_t ws_bytes = 0;
   XMapCache xmaps;
+  bool use_prompt_attn = env_int("SSDK_PROMPT_ATTN", 1) != 0;   // prompt passes on tcgen05 (0: mma.sync tiles)
   ncclComm_t comm = nullptr;
   bool finalized = false;
   int64_t launches = 0;
@@ -592,6 +619,39 @@ static int enqueue_attention(Launcher& L, const bf16* q, const bf16* kc, const b
   CKI(launch_attn(L, a, hd, MT, dim3(KV, nsplit == 1 ? B : (target ? target + B : nsplit * B), nqt)));
   if (nsplit > 1) CKI(L.go(attn_combine_kernel, dim3(B * Q * H), dim3(32), 0, a, hd));
   return 0;
+}
+
+// prompt passes (more rows than kMaxTokens) whose keys come in whole chunks of a page and whose heads fill a tile
+static bool prompt_attn_ok(const Model& m, int M, int block_size) {
+  const int G = m.H / m.KV;
+  return M > kMaxTokens && (m.hd == 64 || m.hd == 128) && (G & (G - 1)) == 0 && m.H < 2048 && block_size % kPromptKeys == 0 &&
+         m.num_blocks * block_size < (1ll << 31);
+}
+template <int HD>
+static int launch_prompt_attn(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const PromptAttnParams& p, int B) {
+  static bool attr_set = false;
+  if (!attr_set) {
+    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD)));
+    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    attr_set = true;
+  }
+  const int tq = kPromptRows >> p.g_shift;
+  return L.go(prompt_attn_kernel<HD>, dim3(p.KV, (p.Q + tq - 1) / tq, B), dim3(kPromptThreads), (size_t)prompt_attn_smem(HD), tmQ, tmK, tmV, p);
+}
+static int enqueue_prompt_attention(ssdk_engine* e, Launcher& L, const Model& m, const bf16* q, const bf16* kc, const bf16* vc, const int32_t* bt,
+                                    const int32_t* ctx_lens, bf16* out, int B, int Q, int block_size, int max_blocks, float scale) {
+  PromptAttnParams p = {};
+  p.block_tables = bt; p.context_lens = ctx_lens; p.out = out; p.Q = Q; p.H = m.H; p.KV = m.KV; p.block_size = block_size; p.max_blocks = max_blocks;
+  while ((m.KV << p.g_shift) < m.H) ++p.g_shift;
+  const int64_t slots = m.num_blocks * block_size;
+  p.n_slots = (int)slots;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  CKI(wait_flag(&p.timeout));
+  const CUtensorMap *tmQ, *tmK, *tmV;
+  CKI(e->xmaps.get_heads(q, kMaxPass, m.H, m.hd, 1 << p.g_shift, kPromptRows >> p.g_shift, &tmQ));
+  CKI(e->xmaps.get_heads(kc, slots, m.KV, m.hd, 1, kPromptKeys, &tmK));
+  CKI(e->xmaps.get_heads(vc, slots, m.KV, m.hd, 1, kPromptKeys, &tmV));
+  return m.hd == 128 ? launch_prompt_attn<128>(L, *tmQ, *tmK, *tmV, p, B) : launch_prompt_attn<64>(L, *tmQ, *tmK, *tmV, p, B);
 }
 
 static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w, int M, int epi, void* out, int ldo,
@@ -816,7 +876,10 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
     CKI(launch_rope(L, M, rp));
 
     // ---- attention over the paged cache ----
-    CKI(enqueue_attention(L, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, w.att_o,
+    if (e->use_prompt_attn && prompt_attn_ok(m, M, bs))
+      CKI(enqueue_prompt_attention(e, L, m, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, f.B, f.Q, bs, mb, scale));
+    else
+      CKI(enqueue_attention(L, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, w.att_o,
                           w.att_lse, w.att_counters, f.B, f.Q, m.H, m.KV, m.hd, bs, mb, scale, TQ, MT, nqt, nsplit, target));
 
     // ---- output projection (row-parallel) ----

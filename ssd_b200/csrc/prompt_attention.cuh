@@ -1,0 +1,274 @@
+// prompt_attention.cuh — causal attention of a prompt pass over the paged KV cache on tcgen05.
+//
+// A CTA owns one kv head and a tile of 128 rows: 128 / G query tokens x the G query heads that share the kv head, so a key is loaded once
+// for all of them.  Chunks of 64 keys stream through two stages by TMA (a chunk lies in one page).  Per chunk:
+//   S = Q K^T      128 x 64, both operands K-major in shared memory, fp32 in TMEM (two buffers: the next chunk's is computed under the softmax)
+//   P = exp2(S - m) one row per thread, no shuffles; rounded to bf16 and stored over the S it came from
+//   O += P V       P from TMEM, V as it lies in the cache (MN-major operand), fp32 in TMEM
+// m is raised, and O and the sum rescaled, only when a row's maximum has grown by more than kPromptSlack (base 2): P then stays below
+// 2^kPromptSlack, which costs bf16 and fp32 nothing in relative precision.
+// Warps: 0 loads, 1 issues the products, 2-5 softmax and output.  Two CTAs per SM (97 KB, 256 TMEM columns each), so that one's products
+// run under the other's exponentials, which bound the kernel.
+// 2003 tokens, 32 heads of 128 over 8: 205 us on mma.sync tiles of 64 rows (paged_attn_kernel), 46 us here = 720 TFLOP/s of the masked work;
+// 8B widths, 4 layers: 4779 -> 4143 us a prompt.
+#pragma once
+#include "gemm_pair.cuh"
+
+namespace ssdk {
+
+constexpr int kPromptRows = 128, kPromptKeys = 64, kPromptStages = 2, kPromptThreads = 192;
+constexpr float kPromptSlack = 8.f;
+constexpr int prompt_attn_smem(int HD) { return kPromptRows * HD * 2 + kPromptStages * 2 * kPromptKeys * HD * 2 + 1024; }
+
+struct PromptAttnParams {
+  const int32_t* block_tables;   // [B, max_blocks]
+  const int32_t* context_lens;   // [B], includes the Q new tokens
+  __nv_bfloat16* out;            // [B*Q, H, hd]
+  int Q, H, KV, g_shift;         // H / KV = 1 << g_shift <= 16
+  int block_size, max_blocks;    // block_size a multiple of kPromptKeys
+  int n_slots;                   // token slots of the cache: a chunk without a page is loaded from behind them (zeros)
+  float scale_log2;              // > 0
+  unsigned* timeout;
+};
+
+// a whole warp's bounded wait: all of it goes on, or none
+SSDK_DEVINL bool warp_wait(uint64_t* bar, uint32_t parity, unsigned* timeout) {
+  return __all_sync(0xffffffffu, mbar_wait_cluster(bar, parity, timeout));
+}
+SSDK_DEVINL void tma_load_3d(void* smem_dst, const void* tmap, uint64_t* bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+// A from TMEM (a lane per row, two bf16 of K per column), B from shared memory
+SSDK_DEVINL void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// Operand that is contiguous along M or N, 128-byte swizzle: atoms of 64 elements x 8 k; the next 8 k follow 1024 B on (SBO), the next 64
+// elements `next64` bytes on (LBO)
+SSDK_DEVINL uint64_t make_umma_desc_mn128(const void* smem_tile, uint32_t next64) {
+  const uint32_t addr = smem_u32(smem_tile);
+  uint64_t d = 0;
+  d |= (uint64_t)((addr >> 4) & 0x3FFFu);
+  d |= (uint64_t)((next64 >> 4) & 0x3FFFu) << 16;
+  d |= (uint64_t)(1024u >> 4) << 32;
+  d |= (uint64_t)1u << 46;
+  d |= (uint64_t)2u << 61;
+  return d;
+}
+SSDK_DEVINL void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+SSDK_DEVINL void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// grid (kv heads, q tiles, sequences)
+template <int HD>
+__global__ void __launch_bounds__(kPromptThreads, 2)
+prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                   const PromptAttnParams p) {
+  constexpr int HALVES = HD / 64;                    // 64-column boxes of a row
+  constexpr int kQHalf = kPromptRows * 128, kKHalf = kPromptKeys * 128, kTile = HALVES * kKHalf;
+  extern __shared__ uint8_t prompt_smem_raw[];
+  __shared__ __align__(8) uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], pv_done;
+  __shared__ uint32_t tmem_slot;
+  uint8_t* smem = prompt_smem_raw + ((1024u - (smem_u32(prompt_smem_raw) & 1023u)) & 1023u);
+  uint8_t* sQ = smem;
+  uint8_t* sK = sQ + HALVES * kQHalf;
+  uint8_t* sV = sK + kPromptStages * kTile;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+    mbar_init(&q_full, 1);
+    mbar_init(&pv_done, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
+      mbar_init(&s_full[s], 1); mbar_init(&p_full[s], kPromptRows);
+    }
+    fence_mbar_init();
+  }
+  if (warp == 1) { tmem_alloc(&tmem_slot, 256); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot, tmem_o = tmem + 128;   // S / P buffers at columns 0 and 64, O behind them
+
+  pdl_launch_dependents();
+  pdl_wait();
+
+  const int kvh = blockIdx.x, qt = (int)gridDim.y - 1 - (int)blockIdx.y, b = blockIdx.z;   // (the tiles that see most keys first)
+  const int G = 1 << p.g_shift, TQ = kPromptRows >> p.g_shift;
+  const int tok0 = qt * TQ, tq = min(TQ, p.Q - tok0);
+  const int ctx0 = p.context_lens[b] - p.Q;
+  const int kv_max = ctx0 + tok0 + tq;               // exclusive upper bound of the keys the tile sees
+  const int n = (kv_max + kPromptKeys - 1) / kPromptKeys;
+  auto parity = [](int i) { return (uint32_t)(i >> 1) & 1u; };   // of the i-th use of a pair of barriers
+
+  if (warp == 0) {
+    if (lane == 0) {
+      mbar_arrive_expect_tx(&q_full, HALVES * kQHalf);
+      for (int h = 0; h < HALVES; ++h) tma_load_3d(sQ + h * kQHalf, &tmQ, &q_full, h * 64, kvh << p.g_shift, b * p.Q + tok0);
+      const int32_t* bt = p.block_tables + (size_t)b * p.max_blocks;
+      int i = 0;
+      for (; i < n; ++i) {
+        const int s = i & 1, base = i * kPromptKeys;
+        const int blk = bt[base / p.block_size];
+        const int slot = blk >= 0 ? blk * p.block_size + base % p.block_size : p.n_slots;
+        if (!mbar_wait_cluster(&k_empty[s], parity(i) ^ 1u, p.timeout)) break;
+        mbar_arrive_expect_tx(&k_full[s], kTile);
+        for (int h = 0; h < HALVES; ++h) tma_load_3d(sK + s * kTile + h * kKHalf, &tmK, &k_full[s], h * 64, kvh, slot);
+        if (!mbar_wait_cluster(&v_empty[s], parity(i) ^ 1u, p.timeout)) { mbar_wait_cluster(&k_full[s], parity(i), p.timeout); break; }
+        mbar_arrive_expect_tx(&v_full[s], kTile);
+        for (int h = 0; h < HALVES; ++h) tma_load_3d(sV + s * kTile + h * kKHalf, &tmV, &v_full[s], h * 64, kvh, slot);
+      }
+      // nothing is in flight into this CTA's memory when it leaves, also after a wait ran out
+      mbar_wait_cluster(&q_full, 0, p.timeout);
+      for (int j = max(0, i - 2); j < i; ++j) {
+        mbar_wait_cluster(&k_full[j & 1], parity(j), p.timeout);
+        mbar_wait_cluster(&v_full[j & 1], parity(j), p.timeout);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc_s = make_umma_idesc_bf16(kPromptRows, kPromptKeys);
+      constexpr uint32_t idesc_o = make_umma_idesc_bf16(kPromptRows, HD) | (1u << 16);   // V: b_major = MN
+      auto scores = [&](int i) {
+        if (!mbar_wait_cluster(&k_full[i & 1], parity(i), p.timeout)) return false;
+        tc_fence_after();
+#pragma unroll
+        for (int h = 0; h < HALVES; ++h) {
+          const uint64_t qd = make_umma_desc_k128(sQ + h * kQHalf), kd = make_umma_desc_k128(sK + (i & 1) * kTile + h * kKHalf);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_bf16_ss(tmem + (i & 1) * 64, qd + 2 * k, kd + 2 * k, idesc_s, (uint32_t)((h | k) != 0));
+        }
+        umma_commit(&k_empty[i & 1]);
+        umma_commit(&s_full[i & 1]);
+        return true;
+      };
+      bool ok = n > 0 && mbar_wait_cluster(&q_full, 0, p.timeout) && scores(0);
+      for (int i = 0; i < n && ok; ++i) {
+        // (the buffer of chunk i + 1 is free: the product that read its P was issued before, and products run in order)
+        if (i + 1 < n && !(ok = scores(i + 1))) break;
+        if (!(ok = mbar_wait_cluster(&p_full[i & 1], parity(i), p.timeout) && mbar_wait_cluster(&v_full[i & 1], parity(i), p.timeout))) break;
+        tc_fence_after();
+        const uint64_t vd = make_umma_desc_mn128(sV + (i & 1) * kTile, kKHalf);
+#pragma unroll
+        for (int k = 0; k < kPromptKeys / 16; ++k)   // 16 keys: 2048 B of V, 8 columns of P
+          umma_bf16_ts(tmem_o, tmem + (i & 1) * 64 + 8 * k, vd + 128 * k, idesc_o, (uint32_t)((i | k) != 0));
+        umma_commit(&v_empty[i & 1]);
+        umma_commit(&pv_done);
+      }
+    }
+    __syncwarp();
+  } else {
+    const int q = warp & 3, r = q * 32 + lane, tok = r >> p.g_shift;
+    const uint32_t lanes = (uint32_t)(q * 32) << 16;
+    const int lim = min(ctx0 + tok0 + tok + 1, kv_max);   // keys this row sees (rows behind the tile's tokens: some, dropped)
+    float m = -INFINITY, l = 0.f;
+    bool ok = true;
+    for (int i = 0; i < n; ++i) {
+      const int base = i * kPromptKeys;
+      const uint32_t sp = tmem + lanes + (uint32_t)(i & 1) * 64u;
+      if (!(ok = warp_wait(&s_full[i & 1], parity(i), p.timeout))) break;
+      // (phase by phase, so that a parity is never taken for the one two phases on)
+      if (i > 1 && !(ok = warp_wait(&pv_done, (uint32_t)i & 1u, p.timeout))) break;
+      tc_fence_after();
+      uint32_t u[64];
+#pragma unroll
+      for (int c = 0; c < 64; c += 16) tmem_ld_32x32b_x16(sp + c, u + c);
+      tmem_ld_wait();
+      if (base + kPromptKeys > lim) {
+#pragma unroll
+        for (int c = 0; c < 64; ++c)
+          if (base + c >= lim) u[c] = 0xff800000u;   // -inf
+      }
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c = 0; c < 64; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], __uint_as_float(u[c]));
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+      const bool grow = mx > m + kPromptSlack;
+      if (__any_sync(0xffffffffu, grow)) {
+        const float f = grow ? exp2f(m - mx) : 1.f;   // (m = -inf: 0)
+        if (grow) m = mx;
+        l *= f;
+        if (i > 0) {
+          if (!(ok = warp_wait(&pv_done, (uint32_t)(i - 1) & 1u, p.timeout))) break;
+          tc_fence_after();
+#pragma unroll 1
+          for (int c = 0; c < HD; c += 16) {
+            uint32_t o[16];
+            tmem_ld_32x32b_x16(tmem_o + lanes + c, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
+            tmem_st_32x32b_x16(tmem_o + lanes + c, o);
+          }
+        }
+      }
+      const float ms = m == -INFINITY ? 0.f : m;
+      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int c = 0; c < 64; c += 2) {
+        const float a = exp2f(fmaf(__uint_as_float(u[c]), p.scale_log2, -ms)), e = exp2f(fmaf(__uint_as_float(u[c + 1]), p.scale_log2, -ms));
+        sum4[c & 3] += a;
+        sum4[(c & 3) + 1] += e;
+        u[c >> 1] = pack_bf16x2(a, e);
+      }
+      l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+      tmem_st_32x32b_x16(sp, u);
+      tmem_st_32x32b_x16(sp + 16, u + 16);
+      tmem_st_wait();
+      if (base + kPromptKeys > kv_max) {   // the last chunk: slots behind the tile's keys hold anything, and 0 x NaN is NaN
+        if (!(ok = warp_wait(&v_full[i & 1], parity(i), p.timeout))) break;
+        const int from = kv_max - base, pieces = (kPromptKeys - from) * 8;   // 16-byte pieces per half (a row's stay in its 128 bytes)
+        for (int h = 0; h < HALVES; ++h)
+          for (int j = r; j < pieces; j += kPromptRows)
+            *reinterpret_cast<uint4*>(sV + (i & 1) * kTile + h * kKHalf + from * 128 + j * 16) = make_uint4(0u, 0u, 0u, 0u);
+        fence_proxy_async_smem();
+      }
+      tc_fence_before();
+      mbar_arrive(&p_full[i & 1]);
+    }
+    if (ok && n > 1) ok = warp_wait(&pv_done, (uint32_t)n & 1u, p.timeout);
+    if (ok && n > 0) ok = warp_wait(&pv_done, (uint32_t)(n - 1) & 1u, p.timeout);
+    if (ok) {
+      tc_fence_after();
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const bool mine = tok < tq;
+      __nv_bfloat16* dst = p.out + ((size_t)(b * p.Q + tok0 + tok) * p.H + (kvh << p.g_shift) + (r & (G - 1))) * HD;
+#pragma unroll 2
+      for (int c = 0; c < HD; c += 16) {
+        uint32_t o[16];
+        tmem_ld_32x32b_x16(tmem_o + lanes + c, o);
+        tmem_ld_wait();
+        uint32_t w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] = n <= 0 ? 0u : pack_bf16x2(__uint_as_float(o[2 * j]) * inv, __uint_as_float(o[2 * j + 1]) * inv);
+        if (mine) {
+          *reinterpret_cast<uint4*>(dst + c) = make_uint4(w[0], w[1], w[2], w[3]);
+          *reinterpret_cast<uint4*>(dst + c + 8) = make_uint4(w[4], w[5], w[6], w[7]);
+        }
+      }
+    }
+    tc_fence_before();
+  }
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) tmem_dealloc(tmem, 256);
+}
+
+}  // namespace ssdk
