@@ -176,6 +176,22 @@ struct NormParams {
   int d;
 };
 
+// One 8-element slice of a row whose input is embedded or bf16: the same sums and roundings as norm_slice
+SSDK_DEVINL void norm_slice_rows(const NormParams& p, int m, int i, const __nv_bfloat16* erow, bool zero_row, float* x) {
+  const size_t at = (size_t)m * p.d + i;
+  const uint4 none = make_uint4(0, 0, 0, 0);
+  const uint4 res = p.residual_in ? *reinterpret_cast<const uint4*>(p.residual_in + at) : none;
+  const uint4 in = p.ids ? (zero_row ? none : *reinterpret_cast<const uint4*>(erow + i)) : *reinterpret_cast<const uint4*>(p.x.dense + at);
+  unpack_bf16x8(in, x);
+  if (p.residual_in) {
+    float r[8];
+    unpack_bf16x8(res, r);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] += r[j];
+  }
+  if (p.residual_out) *reinterpret_cast<uint4*>(p.residual_out + at) = pack_bf16x8(x);
+}
+
 // One 8-element slice of the row: x = (all-reduced | embedded | GEMM) input + residual; writes the new residual.
 template <int NB>
 SSDK_DEVINL void norm_slice(const NormParams& p, int m, int i, const uint8_t* symm_slots, unsigned symm_e,
@@ -252,8 +268,11 @@ SSDK_DEVINL void norm_slice(const NormParams& p, int m, int i, const uint8_t* sy
 // one L2 round trip; the kernel is ~SLICES round trips + one block reduction.  SLICES = 0: any d, row staged in shared
 // memory.  (With a single instantiation ptxas ran out of its 128 registers at 512 threads and serialised the slab loads:
 // one round trip per slab, 3-4 us per call.)
-template <int SLICES>
-__global__ void __launch_bounds__(512) add_rmsnorm_kernel(NormParams p) {
+// ROWS: calls of many rows, whose input is an embedding or rounded to bf16 already (no slabs, no all-reduce): without their registers
+// three CTAs of 512 threads share an SM instead of one.  2003 rows of 4096: 12 us a call, and with the
+// rotation's like form a prompt of 8B widths and 4 layers takes 3934 us instead of 4143
+template <int SLICES, bool ROWS = false>
+__global__ void __launch_bounds__(512, ROWS ? 3 : 1) add_rmsnorm_kernel(NormParams p) {
   SSDK_DYN_SMEM(float, rbuf);  // d floats (SLICES == 0 only)
   SSDK_STATIC_SMEM(float, red, 32);
   pdl_launch_dependents();
@@ -262,14 +281,14 @@ __global__ void __launch_bounds__(512) add_rmsnorm_kernel(NormParams p) {
   // (which would include the acknowledgement of its remote NVLink stores, ~4 us at TP=8) — it can start polling as soon
   // as it is resident.  Seeing this rank's own flagged words implies the local chain up to the publish has run, which is
   // what protects `hidden` / `residual` (read by earlier kernels of the chain) from being overwritten too early.
-  if (!(p.symm.base && p.symm.no_dep_wait)) pdl_wait();
+  if (ROWS || !(p.symm.base && p.symm.no_dep_wait)) pdl_wait();
   if (threadIdx.x == 0) trace_mark(TR_NORM);
   const int m = blockIdx.x;
   const int d = p.d;
   // ---- one-shot all-reduce input: words carry their own flag, nothing to wait for up front ----
   const uint8_t* symm_slots = nullptr;
   unsigned symm_e = 0;
-  if (p.symm.base) {
+  if (!ROWS && p.symm.base) {
     const unsigned seq = __ldcg(p.symm.fwd_seq);
     symm_e = symm_epoch_of(seq, p.symm.call_idx);
     symm_slots = p.symm.base + symm_slot_off(symm_parity_of(seq, p.symm.call_idx, p.symm.n_calls), 0, p.symm.slot_bytes);
@@ -295,7 +314,8 @@ __global__ void __launch_bounds__(512) add_rmsnorm_kernel(NormParams p) {
     for (int c = 0; c < SLICES; ++c) {
       const int i = (c * blockDim.x + threadIdx.x) * 8;
       if (i < d) {
-        norm_slice<NB>(p, m, i, symm_slots, symm_e, erow, zero_row, xreg[c]);
+        if constexpr (ROWS) norm_slice_rows(p, m, i, erow, zero_row, xreg[c]);
+        else norm_slice<NB>(p, m, i, symm_slots, symm_e, erow, zero_row, xreg[c]);
 #pragma unroll
         for (int j = 0; j < 8; ++j) ss += xreg[c][j] * xreg[c][j];
       }
@@ -426,7 +446,8 @@ struct RopeParams {
 
 // HD is a template parameter so that the per-lane element pairs are static registers (a run-time head_dim turned the
 // x1/x2 arrays into local memory and made ptxas recycle the load registers, i.e. one L2 round trip per split-K slab).
-template <int HD>
+// ROWS: calls of many rows, whose projection is rounded to bf16 already.  2003 rows, 48 heads of 128: 26 us
+template <int HD, bool ROWS = false>
 __global__ void __launch_bounds__(128) rope_store_kernel(RopeParams p) {
   constexpr int HALF = HD / 2;
   constexpr int NP = (HALF + 63) / 64;  // (i, i+1) / (i + HALF, i + HALF + 1) pairs per lane, i = 2 * lane + 64 * t
@@ -451,7 +472,14 @@ __global__ void __launch_bounds__(128) rope_store_kernel(RopeParams p) {
   for (int t = 0; t < NP; ++t) {
     const int i = 2 * lane + 64 * t;
     if (i < HALF) {
-      gemm_out_at2x2(p.qkv, m, col0 + i, col0 + HALF + i, x1[t], x2[t]);
+      if constexpr (ROWS) {
+        const __nv_bfloat16* src = p.qkv.dense + (size_t)m * p.qkv.N + col0 + i;
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src));
+        const float2 c = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src + HALF));
+        x1[t][0] = a.x; x1[t][1] = a.y; x2[t][0] = c.x; x2[t][1] = c.y;
+      } else {
+        gemm_out_at2x2(p.qkv, m, col0 + i, col0 + HALF + i, x1[t], x2[t]);
+      }
       ss += x1[t][0] * x1[t][0] + x1[t][1] * x1[t][1] + x2[t][0] * x2[t][0] + x2[t][1] * x2[t][1];
     } else {
       x1[t][0] = x1[t][1] = x2[t][0] = x2[t][1] = 0.f;

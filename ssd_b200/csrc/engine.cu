@@ -164,17 +164,28 @@ static int num_sms() {
   }
   return g_num_sms;
 }
+// activations buffers usable as the X operand: [kMaxTokens rows, K] bf16.  Decode / verify steps use <= 64 tokens
+// (UMMA N 16 / 32 / 64); prefill chunks and larger batches up to 256 (UMMA N 128 / 256: the weights are then streamed once
+// per 256 tokens instead of once per 64 — a 2k-token 70B prompt reads 139 GB 8 times instead of 32).
+constexpr int kMaxTokens = 256;
+
 // add_rmsnorm_kernel geometry: <= 2 register-resident 8-element slices per thread (512 threads), smem staging beyond
 static int norm_threads(int d) { return std::max(32, std::min(512, ((d / 8 + 31) / 32) * 32)); }
 static int launch_norm(Launcher& L, int M, int d, const NormParams& np) {
   const int threads = norm_threads(d);
   const int slices = (d + 8 * threads - 1) / (8 * threads);
+  if (M > kMaxTokens && np.x.S == 0 && !np.symm.base && slices <= 2)
+    return L.go(slices == 1 ? add_rmsnorm_kernel<1, true> : add_rmsnorm_kernel<2, true>, dim3(M), dim3(threads), 0, np);
   if (slices == 1) return L.go(add_rmsnorm_kernel<1>, dim3(M), dim3(threads), 0, np);
   if (slices == 2) return L.go(add_rmsnorm_kernel<2>, dim3(M), dim3(threads), 0, np);
   return L.go(add_rmsnorm_kernel<0>, dim3(M), dim3(threads), (size_t)d * 4, np);
 }
 static int launch_rope(Launcher& L, int M, const RopeParams& rp) {
   const dim3 grid(M, (rp.heads + 2 * rp.kv_heads + 3) / 4), block(128);
+  if (M > kMaxTokens && rp.qkv.S == 0) {
+    if (rp.head_dim == 64) return L.go(rope_store_kernel<64, true>, grid, block, 0, rp);
+    if (rp.head_dim == 128) return L.go(rope_store_kernel<128, true>, grid, block, 0, rp);
+  }
   switch (rp.head_dim) {
     case 64: return L.go(rope_store_kernel<64>, grid, block, 0, rp);
     case 128: return L.go(rope_store_kernel<128>, grid, block, 0, rp);
@@ -283,10 +294,6 @@ static int weight_tmap(WeightMat& w) {
   return 0;
 }
 
-// activations buffers usable as the X operand: [kMaxTokens rows, K] bf16.  Decode / verify steps use <= 64 tokens
-// (UMMA N 16 / 32 / 64); prefill chunks and larger batches up to 256 (UMMA N 128 / 256: the weights are then streamed once
-// per 256 tokens instead of once per 64 — a 2k-token 70B prompt reads 139 GB 8 times instead of 32).
-constexpr int kMaxTokens = 256;
 // Prompt passes without tensor parallelism carry more rows: the tile pairs of gemm_pair_kernel then share the weights through L2 and a
 // layer's small kernels run once per 2048 tokens.  8B widths, 4 layers, 2003 tokens: 8141 us in passes of 256, 5125 us in one.
 constexpr int kMaxPass = 2048;
@@ -659,7 +666,7 @@ static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w
   CKI(weight_tmap(w));
   const int K = (int)w.cols;
   if (K % kBlockK) return fail("GEMM K=%d not a multiple of 64", K);
-  if (M > kMaxTokens) {   // prompt passes: one slab, summed over all of K
+  if (M > kMaxTokens) {   // prompt passes: summed over all of K and rounded to bf16, which their consumers do with slabs (splits 0: dense)
     if (epi != EPI_PARTIAL && (epi != EPI_SILU || N_out % kPairGluRun)) return fail("GEMM of %d rows: unsupported form", M);
     if (epi == EPI_PARTIAL && (size_t)M * N_out > e->ws.partial_floats) return fail("partial buffer too small");
     const CUtensorMap *tmW, *tmX, *tmXs;
@@ -670,8 +677,8 @@ static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w
     GemmPairParams p = {};
     p.out = out; p.M = M; p.N = N_out; p.ldo = epi == EPI_SILU ? ldo : N_out; p.num_kb = K / kBlockK; p.chunks = (M + kPairTokens - 1) / kPairTokens;
     p.w_tiles = epi == EPI_SILU ? (N_out + 127) / 128 : (N_out + 255) / 256; p.act = GLU_SILU_ROUNDED;
-    if (splits_out) *splits_out = 1;
-    return launch_gemm_pair(L, epi == EPI_SILU ? EPI_GLU : EPI_PARTIAL, *tmW, *tmX, *tmXs, p, p.w_tiles * p.chunks);
+    if (splits_out) *splits_out = 0;
+    return launch_gemm_pair(L, epi == EPI_SILU ? EPI_GLU : EPI_BF16, *tmW, *tmX, *tmXs, p, p.w_tiles * p.chunks);
   }
   const int un = umma_n_for(M);
   const CUtensorMap* tmX;
@@ -864,7 +871,7 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
     int S = 1;
     CKI(enqueue_gemm(e, L, w.hidden, lw.qkv, M, EPI_PARTIAL, w.partials, 0, m.qkv_dim, &S));
     RopeParams rp;
-    rp.qkv.dense = nullptr; rp.qkv.partial = w.partials; rp.qkv.S = S; rp.qkv.M = M; rp.qkv.N = m.qkv_dim;
+    rp.qkv.dense = (const bf16*)w.partials; rp.qkv.partial = w.partials; rp.qkv.S = S; rp.qkv.M = M; rp.qkv.N = m.qkv_dim;
     rp.positions = w.positions; rp.slot_mapping = w.slot_mapping; rp.rope_table = m.rope;
     rp.q_norm_w = m.cfg.qk_norm ? lw.q_norm : nullptr;
     rp.k_norm_w = m.cfg.qk_norm ? lw.k_norm : nullptr;
@@ -895,7 +902,7 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
     } else {
       CKI(enqueue_gemm(e, L, w.attn_out, lw.o, M, EPI_PARTIAL, w.partials, 0, m.d, &S));
     }
-    oproj.dense = nullptr; oproj.partial = w.partials; oproj.S = S; oproj.M = M; oproj.N = m.d;
+    oproj.dense = (const bf16*)w.partials; oproj.partial = w.partials; oproj.S = S; oproj.M = M; oproj.N = m.d;
     if (tp > 1 && !fuse_pub) {
       if (use_symm) {
         CKI(enqueue_ar_publish(e, L, &oproj, nullptr, M, m.d, ar_idx));
@@ -924,7 +931,7 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
     } else {
       CKI(enqueue_gemm(e, L, w.act, lw.down, M, EPI_PARTIAL, w.partials, 0, m.d, &S));
     }
-    prev.dense = nullptr; prev.partial = w.partials; prev.S = S; prev.M = M; prev.N = m.d;
+    prev.dense = (const bf16*)w.partials; prev.partial = w.partials; prev.S = S; prev.M = M; prev.N = m.d;
     if (tp > 1 && !fuse_pub) {
       if (use_symm) {
         CKI(enqueue_ar_publish(e, L, &prev, nullptr, M, m.d, ar_idx));

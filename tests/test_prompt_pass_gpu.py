@@ -54,3 +54,23 @@ def test_refused_as_before():
         r.forward_tokens(L.TARGET, [[1] * 257], [0], [list(range(40))])
     with pytest.raises(RuntimeError):
         r.prefill(L.TARGET, [1] * 600, list(range(40)), chunk=512)
+
+
+@pytest.mark.parametrize("hidden,hd,qk_norm", [(4352, 64, False), (256, 128, True), (4096, 64, True)])
+def test_row_forms(hidden, hd, qk_norm):
+    """Norms and rotation of long passes (bf16 products, one or two slices of a row per thread, head norms) against short ones."""
+    from ssd_b200 import lib as L, synth
+    from ssd_b200.runner import ModelSpec, PairRunner
+    spec = ModelSpec(hidden=hidden, layers=1, heads=4, kv_heads=2, head_dim=hd, ffn=576, vocab=1024, rms_eps=1e-5, qk_norm=qk_norm)
+    r = PairRunner(spec, None, spec_k=0, max_batch=2, block_size=64, max_model_len=640, use_graph=False, use_pdl=True)
+    w = synth.generate_weights(spec, {"seed": 4, "alpha": 0.9, "role": "target", "o_down_std": 0.05}, torch.device("cuda:0"))
+    r.bind_weights(L.TARGET, w)
+    r.finalize()
+    toks = torch.randint(0, 1024, (301,), generator=torch.Generator().manual_seed(hidden)).tolist()
+    r.prefill(L.TARGET, toks, list(range(10)), chunk=64)
+    la = r.logits_last(1).float().clone()
+    r.prefill(L.TARGET, toks, list(range(10, 20)))
+    lb = r.logits_last(1).float()
+    assert ((la - lb).norm() / la.norm()).item() < TOL
+    ka, kb = (r.kv[L.TARGET][:, 0, s:s + 10].flatten(1, 2)[:, :301].float() for s in (0, 10))
+    assert ((ka - kb).norm() / ka.norm()).item() < TOL
