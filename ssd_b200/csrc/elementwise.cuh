@@ -268,11 +268,8 @@ SSDK_DEVINL void norm_slice(const NormParams& p, int m, int i, const uint8_t* sy
 // one L2 round trip; the kernel is ~SLICES round trips + one block reduction.  SLICES = 0: any d, row staged in shared
 // memory.  (With a single instantiation ptxas ran out of its 128 registers at 512 threads and serialised the slab loads:
 // one round trip per slab, 3-4 us per call.)
-// ROWS: calls of many rows, whose input is an embedding or rounded to bf16 already (no slabs, no all-reduce): without their registers
-// three CTAs of 512 threads share an SM instead of one.  2003 rows of 4096: 12 us a call, and with the
-// rotation's like form a prompt of 8B widths and 4 layers takes 3934 us instead of 4143
-template <int SLICES, bool ROWS = false>
-__global__ void __launch_bounds__(512, ROWS ? 3 : 1) add_rmsnorm_kernel(NormParams p) {
+template <int SLICES>
+__global__ void __launch_bounds__(512) add_rmsnorm_kernel(NormParams p) {
   SSDK_DYN_SMEM(float, rbuf);  // d floats (SLICES == 0 only)
   SSDK_STATIC_SMEM(float, red, 32);
   pdl_launch_dependents();
@@ -281,14 +278,14 @@ __global__ void __launch_bounds__(512, ROWS ? 3 : 1) add_rmsnorm_kernel(NormPara
   // (which would include the acknowledgement of its remote NVLink stores, ~4 us at TP=8) — it can start polling as soon
   // as it is resident.  Seeing this rank's own flagged words implies the local chain up to the publish has run, which is
   // what protects `hidden` / `residual` (read by earlier kernels of the chain) from being overwritten too early.
-  if (ROWS || !(p.symm.base && p.symm.no_dep_wait)) pdl_wait();
+  if (!(p.symm.base && p.symm.no_dep_wait)) pdl_wait();
   if (threadIdx.x == 0) trace_mark(TR_NORM);
   const int m = blockIdx.x;
   const int d = p.d;
   // ---- one-shot all-reduce input: words carry their own flag, nothing to wait for up front ----
   const uint8_t* symm_slots = nullptr;
   unsigned symm_e = 0;
-  if (!ROWS && p.symm.base) {
+  if (p.symm.base) {
     const unsigned seq = __ldcg(p.symm.fwd_seq);
     symm_e = symm_epoch_of(seq, p.symm.call_idx);
     symm_slots = p.symm.base + symm_slot_off(symm_parity_of(seq, p.symm.call_idx, p.symm.n_calls), 0, p.symm.slot_bytes);
@@ -314,8 +311,7 @@ __global__ void __launch_bounds__(512, ROWS ? 3 : 1) add_rmsnorm_kernel(NormPara
     for (int c = 0; c < SLICES; ++c) {
       const int i = (c * blockDim.x + threadIdx.x) * 8;
       if (i < d) {
-        if constexpr (ROWS) norm_slice_rows(p, m, i, erow, zero_row, xreg[c]);
-        else norm_slice<NB>(p, m, i, symm_slots, symm_e, erow, zero_row, xreg[c]);
+        norm_slice<NB>(p, m, i, symm_slots, symm_e, erow, zero_row, xreg[c]);
 #pragma unroll
         for (int j = 0; j < 8; ++j) ss += xreg[c][j] * xreg[c][j];
       }
@@ -360,6 +356,55 @@ __global__ void __launch_bounds__(512, ROWS ? 3 : 1) add_rmsnorm_kernel(NormPara
     }
   }
   if (threadIdx.x == 0) trace_fine(TRF_NORM + 2);
+}
+
+// The same for calls of many rows, whose input is an embedding or rounded to bf16 already (no slabs, no all-reduce): without their
+// registers three CTAs of 512 threads share an SM instead of one.  2003 rows of 4096: 12 us a call; with the rotation's like form a prompt of
+// 8B widths and 4 layers takes 3934 us instead of 4143.  (A kernel of its own, so that the one above stays as it is: with
+// both in one the 8B + 1B step took 8468 us instead of 8450.)
+template <int SLICES>
+__global__ void __launch_bounds__(512, 3) add_rmsnorm_rows_kernel(NormParams p) {
+  SSDK_STATIC_SMEM(float, red, 32);
+  pdl_launch_dependents();
+  pdl_wait();
+  const int m = blockIdx.x, d = p.d;
+  const __nv_bfloat16* erow = nullptr;
+  bool zero_row = false;
+  if (p.ids) {
+    const long long id = p.ids[(size_t)m * p.ids_stride] - p.vocab_start;
+    if (id < 0 || id >= p.vocab_rows) zero_row = true;
+    else erow = p.embed + (size_t)id * d;
+  }
+  float ss = 0.f, xreg[SLICES][8];
+  uint4 wpk[SLICES];
+#pragma unroll
+  for (int c = 0; c < SLICES; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 8;
+    if (i < d && p.y) wpk[c] = *reinterpret_cast<const uint4*>(p.w + i);
+  }
+#pragma unroll
+  for (int c = 0; c < SLICES; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 8;
+    if (i < d) {
+      norm_slice_rows(p, m, i, erow, zero_row, xreg[c]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += xreg[c][j] * xreg[c][j];
+    }
+  }
+  ss = block_sum(ss, red);
+  const float rstd = rsqrtf(ss / (float)d + p.eps);
+  if (!p.y) return;
+#pragma unroll
+  for (int c = 0; c < SLICES; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 8;
+    if (i < d) {
+      float w[8], o[8];
+      unpack_bf16x8(wpk[c], w);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = xreg[c][j] * rstd * w[j];
+      *reinterpret_cast<uint4*>(p.y + (size_t)m * d + i) = pack_bf16x8(o);
+    }
+  }
 }
 
 // ----------------------------------------------------------------------------------
@@ -446,8 +491,7 @@ struct RopeParams {
 
 // HD is a template parameter so that the per-lane element pairs are static registers (a run-time head_dim turned the
 // x1/x2 arrays into local memory and made ptxas recycle the load registers, i.e. one L2 round trip per split-K slab).
-// ROWS: calls of many rows, whose projection is rounded to bf16 already.  2003 rows, 48 heads of 128: 26 us
-template <int HD, bool ROWS = false>
+template <int HD>
 __global__ void __launch_bounds__(128) rope_store_kernel(RopeParams p) {
   constexpr int HALF = HD / 2;
   constexpr int NP = (HALF + 63) / 64;  // (i, i+1) / (i + HALF, i + HALF + 1) pairs per lane, i = 2 * lane + 64 * t
@@ -472,14 +516,7 @@ __global__ void __launch_bounds__(128) rope_store_kernel(RopeParams p) {
   for (int t = 0; t < NP; ++t) {
     const int i = 2 * lane + 64 * t;
     if (i < HALF) {
-      if constexpr (ROWS) {
-        const __nv_bfloat16* src = p.qkv.dense + (size_t)m * p.qkv.N + col0 + i;
-        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src));
-        const float2 c = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src + HALF));
-        x1[t][0] = a.x; x1[t][1] = a.y; x2[t][0] = c.x; x2[t][1] = c.y;
-      } else {
-        gemm_out_at2x2(p.qkv, m, col0 + i, col0 + HALF + i, x1[t], x2[t]);
-      }
+      gemm_out_at2x2(p.qkv, m, col0 + i, col0 + HALF + i, x1[t], x2[t]);
       ss += x1[t][0] * x1[t][0] + x1[t][1] * x1[t][1] + x2[t][0] * x2[t][0] + x2[t][1] * x2[t][1];
     } else {
       x1[t][0] = x1[t][1] = x2[t][0] = x2[t][1] = 0.f;
@@ -530,6 +567,76 @@ __global__ void __launch_bounds__(128) rope_store_kernel(RopeParams p) {
     }
   }
   if (threadIdx.x == 0) trace_fine(TRF_ROPE + 1);
+}
+
+// The same for calls of many rows, whose projection is rounded to bf16 already: a warp takes kRopeHeads heads of its row, all of them asked
+// for together, the angles once.  (A head per warp: 26 us for 2003 rows and 48 heads of 128.)
+constexpr int kRopeHeads = 4;
+
+template <int HD>
+__global__ void __launch_bounds__(128) rope_store_rows_kernel(RopeParams p) {
+  constexpr int HALF = HD / 2, NP = (HALF + 63) / 64;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int m = blockIdx.x, lane = threadIdx.x & 31, H = p.heads, KV = p.kv_heads;
+  const int head0 = (blockIdx.y * 4 + (threadIdx.x >> 5)) * kRopeHeads, n = min(kRopeHeads, H + 2 * KV - head0);
+  if (n <= 0) return;
+  const int slot = p.slot_mapping[m];
+  const float* cs = p.rope_table + (size_t)p.positions[m] * HD;
+  const __nv_bfloat16* src = p.qkv.dense + (size_t)m * p.qkv.N + (size_t)head0 * HD;
+  __nv_bfloat162 a[kRopeHeads][NP], c[kRopeHeads][NP];
+  float2 co[NP], si[NP];
+#pragma unroll
+  for (int t = 0; t < NP; ++t) {
+    const int i = 2 * lane + 64 * t;
+    if (i >= HALF) continue;
+#pragma unroll
+    for (int h = 0; h < kRopeHeads; ++h)
+      if (h < n) {
+        a[h][t] = *reinterpret_cast<const __nv_bfloat162*>(src + h * HD + i);
+        c[h][t] = *reinterpret_cast<const __nv_bfloat162*>(src + h * HD + HALF + i);
+      }
+    co[t] = *reinterpret_cast<const float2*>(cs + i);
+    si[t] = *reinterpret_cast<const float2*>(cs + HALF + i);
+  }
+#pragma unroll
+  for (int h = 0; h < kRopeHeads; ++h) {
+    const int head = head0 + h, kind = head < H ? 0 : (head < H + KV ? 1 : 2);   // q, k, v
+    if (h >= n || (kind != 0 && slot < 0)) continue;
+    __nv_bfloat16* dst = kind == 0 ? p.q_out + ((size_t)m * H + head) * HD
+                                   : (kind == 1 ? p.k_cache + ((size_t)slot * KV + (head - H)) * HD : p.v_cache + ((size_t)slot * KV + (head - H - KV)) * HD);
+    const __nv_bfloat16* nw = kind == 0 ? p.q_norm_w : (kind == 1 ? p.k_norm_w : nullptr);
+    float x1[NP][2], x2[NP][2], ss = 0.f;
+#pragma unroll
+    for (int t = 0; t < NP; ++t) {
+      const bool in = 2 * lane + 64 * t < HALF;
+      const float2 u = in ? __bfloat1622float2(a[h][t]) : make_float2(0.f, 0.f), v = in ? __bfloat1622float2(c[h][t]) : make_float2(0.f, 0.f);
+      x1[t][0] = u.x; x1[t][1] = u.y; x2[t][0] = v.x; x2[t][1] = v.y;
+      ss += u.x * u.x + u.y * u.y + v.x * v.x + v.y * v.y;
+    }
+    float rstd = 1.f;
+    if (nw) rstd = rsqrtf(warp_sum(ss) / (float)HD + p.norm_eps);
+#pragma unroll
+    for (int t = 0; t < NP; ++t) {
+      const int i = 2 * lane + 64 * t;
+      if (i >= HALF) continue;
+      if (kind == 2) {
+        *reinterpret_cast<__nv_bfloat162*>(dst + i) = a[h][t];
+        *reinterpret_cast<__nv_bfloat162*>(dst + HALF + i) = c[h][t];
+        continue;
+      }
+      if (nw) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          x1[t][e] = bf16_round(x1[t][e] * rstd * bf2f(nw[i + e]));
+          x2[t][e] = bf16_round(x2[t][e] * rstd * bf2f(nw[HALF + i + e]));
+        }
+      }
+      *reinterpret_cast<__nv_bfloat162*>(dst + i) = __floats2bfloat162_rn(x1[t][0] * co[t].x - x2[t][0] * si[t].x, x1[t][1] * co[t].y - x2[t][1] * si[t].y);
+      *reinterpret_cast<__nv_bfloat162*>(dst + HALF + i) =
+          __floats2bfloat162_rn(x2[t][0] * co[t].x + x1[t][0] * si[t].x, x2[t][1] * co[t].y + x1[t][1] * si[t].y);
+    }
+  }
 }
 
 // ----------------------------------------------------------------------------------

@@ -175,7 +175,7 @@ static int launch_norm(Launcher& L, int M, int d, const NormParams& np) {
   const int threads = norm_threads(d);
   const int slices = (d + 8 * threads - 1) / (8 * threads);
   if (M > kMaxTokens && np.x.S == 0 && !np.symm.base && slices <= 2)
-    return L.go(slices == 1 ? add_rmsnorm_kernel<1, true> : add_rmsnorm_kernel<2, true>, dim3(M), dim3(threads), 0, np);
+    return L.go(slices == 1 ? add_rmsnorm_rows_kernel<1> : add_rmsnorm_rows_kernel<2>, dim3(M), dim3(threads), 0, np);
   if (slices == 1) return L.go(add_rmsnorm_kernel<1>, dim3(M), dim3(threads), 0, np);
   if (slices == 2) return L.go(add_rmsnorm_kernel<2>, dim3(M), dim3(threads), 0, np);
   return L.go(add_rmsnorm_kernel<0>, dim3(M), dim3(threads), (size_t)d * 4, np);
@@ -183,8 +183,9 @@ static int launch_norm(Launcher& L, int M, int d, const NormParams& np) {
 static int launch_rope(Launcher& L, int M, const RopeParams& rp) {
   const dim3 grid(M, (rp.heads + 2 * rp.kv_heads + 3) / 4), block(128);
   if (M > kMaxTokens && rp.qkv.S == 0) {
-    if (rp.head_dim == 64) return L.go(rope_store_kernel<64, true>, grid, block, 0, rp);
-    if (rp.head_dim == 128) return L.go(rope_store_kernel<128, true>, grid, block, 0, rp);
+    const dim3 few(M, (grid.y + kRopeHeads - 1) / kRopeHeads);
+    if (rp.head_dim == 64) return L.go(rope_store_rows_kernel<64>, few, block, 0, rp);
+    if (rp.head_dim == 128) return L.go(rope_store_rows_kernel<128>, few, block, 0, rp);
   }
   switch (rp.head_dim) {
     case 64: return L.go(rope_store_kernel<64>, grid, block, 0, rp);
@@ -586,7 +587,7 @@ static int launch_attn_inst(Launcher& L, const AttnParams& p, dim3 grid) {
   static bool attr_set = false;
   if (!attr_set) {
     CK(cudaFuncSetAttribute(paged_attn_kernel<HD, MT, OCC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CK(cudaFuncSetAttribute(paged_attn_kernel<HD, MT, OCC>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    if (OCC > 1) CK(cudaFuncSetAttribute(paged_attn_kernel<HD, MT, OCC>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     attr_set = true;
   }
   return L.go(paged_attn_kernel<HD, MT, OCC>, grid, dim3(attn_warps(MT) * 32), smem, p);
@@ -1269,7 +1270,7 @@ static int init_kernel_attrs() {
 #undef SSDK_ATTR_G
 #define SSDK_ATTR_A(HD, MT, OCC) \
   CK(cudaFuncSetAttribute(paged_attn_kernel<HD, MT, OCC>, cudaFuncAttributeMaxDynamicSharedMemorySize, attn_smem(HD, MT))); \
-  CK(cudaFuncSetAttribute(paged_attn_kernel<HD, MT, OCC>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  if (OCC > 1) CK(cudaFuncSetAttribute(paged_attn_kernel<HD, MT, OCC>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
   SSDK_ATTR_A(128, 1, 3) SSDK_ATTR_A(128, 2, 1) SSDK_ATTR_A(128, 2, 2) SSDK_ATTR_A(128, 4, 1) SSDK_ATTR_A(128, 4, 2)
   SSDK_ATTR_A(64, 1, 3) SSDK_ATTR_A(64, 2, 1) SSDK_ATTR_A(64, 2, 2) SSDK_ATTR_A(64, 4, 1) SSDK_ATTR_A(64, 4, 2)
 #undef SSDK_ATTR_A
