@@ -245,6 +245,15 @@ int ssdk_paged_attn(const void* q, const void* k_cache, const void* v_cache,
                     int batch, int q_len, int heads, int kv_heads, int head_dim,
                     int block_size, int max_blocks_per_seq, float scale, void* stream);
 
+/* The same attention as the engine's prompt passes take it (tcgen05): any number of query rows, head_dim 64 or 128, a power
+ * of two <= 16 query heads per key head, block_size a multiple of 64, num_blocks pages in the cache.  *gave_up (pinned host
+ * memory) is set if one of the kernel's bounded waits ran out; the output is then not complete. */
+int ssdk_prompt_attn(const void* q, const void* k_cache, const void* v_cache,
+                     const int32_t* block_tables, const int32_t* context_lens, void* out,
+                     int batch, int q_len, int heads, int kv_heads, int head_dim,
+                     int block_size, int max_blocks_per_seq, int64_t num_blocks, float scale,
+                     uint32_t* gave_up, void* stream);
+
 /* Sampler.forward (layers/sampler.py:14-36): greedy where temp==0, else
  * argmax(softmax(l/T) / Exp(1)) with Philox(seed, step_id) exponentials.
  * logits bf16 [B, V] with row stride ld (elements); out int64 [B]. */

@@ -629,11 +629,11 @@ static int enqueue_attention(Launcher& L, const bf16* q, const bf16* kc, const b
   return 0;
 }
 
-// prompt passes (more rows than kMaxTokens) whose keys come in whole chunks of a page and whose heads fill a tile
-static bool prompt_attn_ok(const Model& m, int M, int block_size) {
-  const int G = m.H / m.KV;
-  return M > kMaxTokens && (m.hd == 64 || m.hd == 128) && (G & (G - 1)) == 0 && m.H < 2048 && block_size % kPromptKeys == 0 &&
-         m.num_blocks * block_size < (1ll << 31);
+// keys come in whole chunks of a page, a key head's query heads fill tiles (taken by passes of more rows than kMaxTokens)
+static bool prompt_attn_ok(int H, int KV, int hd, int block_size, int64_t num_blocks) {
+  const int G = H / KV;
+  return (hd == 64 || hd == 128) && H % KV == 0 && G <= 16 && (G & (G - 1)) == 0 && H < 2048 && block_size % kPromptKeys == 0 &&
+         num_blocks * block_size < (1ll << 31);
 }
 template <int HD>
 static int launch_prompt_attn(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const PromptAttnParams& p, int B) {
@@ -646,20 +646,29 @@ static int launch_prompt_attn(Launcher& L, const CUtensorMap& tmQ, const CUtenso
   const int tq = kPromptRows >> p.g_shift;
   return L.go(prompt_attn_kernel<HD>, dim3(p.KV, (p.Q + tq - 1) / tq, B), dim3(kPromptThreads), (size_t)prompt_attn_smem(HD), tmQ, tmK, tmV, p);
 }
-static int enqueue_prompt_attention(ssdk_engine* e, Launcher& L, const Model& m, const bf16* q, const bf16* kc, const bf16* vc, const int32_t* bt,
-                                    const int32_t* ctx_lens, bf16* out, int B, int Q, int block_size, int max_blocks, float scale) {
+// maps of queries, keys and values of layer caches of `slots` token slots: {box of a tile's query tokens, kPromptKeys keys of one head}
+static int enqueue_prompt_attention(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const int32_t* bt,
+                                    const int32_t* ctx_lens, bf16* out, int B, int Q, int H, int KV, int hd, int block_size, int max_blocks,
+                                    int64_t slots, float scale, unsigned* timeout) {
   PromptAttnParams p = {};
-  p.block_tables = bt; p.context_lens = ctx_lens; p.out = out; p.Q = Q; p.H = m.H; p.KV = m.KV; p.block_size = block_size; p.max_blocks = max_blocks;
-  while ((m.KV << p.g_shift) < m.H) ++p.g_shift;
-  const int64_t slots = m.num_blocks * block_size;
+  p.block_tables = bt; p.context_lens = ctx_lens; p.out = out; p.Q = Q; p.H = H; p.KV = KV; p.block_size = block_size; p.max_blocks = max_blocks;
+  while ((KV << p.g_shift) < H) ++p.g_shift;
   p.n_slots = (int)slots;
   p.scale_log2 = scale * 1.4426950408889634f;
-  CKI(wait_flag(&p.timeout));
+  p.timeout = timeout;
+  return hd == 128 ? launch_prompt_attn<128>(L, tmQ, tmK, tmV, p, B) : launch_prompt_attn<64>(L, tmQ, tmK, tmV, p, B);
+}
+static int forward_prompt_attention(ssdk_engine* e, Launcher& L, const Model& m, const bf16* q, const bf16* kc, const bf16* vc, const int32_t* bt,
+                                    const int32_t* ctx_lens, bf16* out, int B, int Q, int block_size, int max_blocks, float scale) {
+  const int64_t slots = m.num_blocks * block_size;
+  const int G = m.H / m.KV;
+  unsigned* timeout;
+  CKI(wait_flag(&timeout));
   const CUtensorMap *tmQ, *tmK, *tmV;
-  CKI(e->xmaps.get_heads(q, kMaxPass, m.H, m.hd, 1 << p.g_shift, kPromptRows >> p.g_shift, &tmQ));
+  CKI(e->xmaps.get_heads(q, kMaxPass, m.H, m.hd, G, kPromptRows / G, &tmQ));
   CKI(e->xmaps.get_heads(kc, slots, m.KV, m.hd, 1, kPromptKeys, &tmK));
   CKI(e->xmaps.get_heads(vc, slots, m.KV, m.hd, 1, kPromptKeys, &tmV));
-  return m.hd == 128 ? launch_prompt_attn<128>(L, *tmQ, *tmK, *tmV, p, B) : launch_prompt_attn<64>(L, *tmQ, *tmK, *tmV, p, B);
+  return enqueue_prompt_attention(L, *tmQ, *tmK, *tmV, bt, ctx_lens, out, B, Q, m.H, m.KV, m.hd, block_size, max_blocks, slots, scale, timeout);
 }
 
 static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w, int M, int epi, void* out, int ldo,
@@ -884,8 +893,8 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
     CKI(launch_rope(L, M, rp));
 
     // ---- attention over the paged cache ----
-    if (e->use_prompt_attn && prompt_attn_ok(m, M, bs))
-      CKI(enqueue_prompt_attention(e, L, m, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, f.B, f.Q, bs, mb, scale));
+    if (e->use_prompt_attn && M > kMaxTokens && prompt_attn_ok(m.H, m.KV, m.hd, bs, m.num_blocks))
+      CKI(forward_prompt_attention(e, L, m, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, f.B, f.Q, bs, mb, scale));
     else
       CKI(enqueue_attention(L, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, w.att_o,
                           w.att_lse, w.att_counters, f.B, f.Q, m.H, m.KV, m.hd, bs, mb, scale, TQ, MT, nqt, nsplit, target));
@@ -1818,6 +1827,24 @@ int ssdk_paged_attn(const void* q, const void* k_cache, const void* v_cache, con
   return enqueue_attention(L, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, block_tables, context_lens,
                            (bf16*)out, part_o, part_lse, (unsigned*)scratch, batch, q_len, heads, kv_heads, head_dim, block_size,
                            max_blocks_per_seq, scale, TQ, MT, nqt, nsplit, target);
+}
+
+int ssdk_prompt_attn(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
+                     const int32_t* context_lens, void* out, int batch, int q_len, int heads, int kv_heads, int head_dim,
+                     int block_size, int max_blocks_per_seq, int64_t num_blocks, float scale, uint32_t* gave_up, void* stream) {
+  if (batch < 1 || q_len < 1 || heads < 1 || kv_heads < 1 || num_blocks < 1 || batch > 65535 || !gave_up || !(scale > 0.f) ||
+      !prompt_attn_ok(heads, kv_heads, head_dim, block_size, num_blocks) || (int64_t)batch * q_len >= (1ll << 31))
+    return fail("prompt_attn: unsupported sizes (batch=%d q_len=%d heads=%d/%d of %d, pages of %d)", batch, q_len, heads, kv_heads, head_dim, block_size);
+  Launcher L;
+  L.st = (cudaStream_t)stream;
+  const int G = heads / kv_heads;
+  const int64_t slots = num_blocks * block_size;
+  CUtensorMap tmQ, tmK, tmV;
+  CKI(make_tmap_heads(&tmQ, q, (int64_t)batch * q_len, heads, head_dim, G, kPromptRows / G));
+  CKI(make_tmap_heads(&tmK, k_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
+  CKI(make_tmap_heads(&tmV, v_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
+  return enqueue_prompt_attention(L, tmQ, tmK, tmV, block_tables, context_lens, (bf16*)out, batch, q_len, heads, kv_heads, head_dim, block_size,
+                                  max_blocks_per_seq, slots, scale, gave_up);
 }
 
 int ssdk_sample(const void* logits, int64_t ld, const float* temps, int B, int V, uint64_t seed, uint64_t step_id,

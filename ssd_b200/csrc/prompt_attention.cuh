@@ -80,7 +80,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   constexpr int HALVES = HD / 64;                    // 64-column boxes of a row
   constexpr int kQHalf = kPromptRows * 128, kKHalf = kPromptKeys * 128, kTile = HALVES * kKHalf;
   extern __shared__ uint8_t prompt_smem_raw[];
-  __shared__ __align__(8) uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], pv_done;
+  __shared__ __align__(8) uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], pv_done[2];
   __shared__ uint32_t tmem_slot;
   uint8_t* smem = prompt_smem_raw + ((1024u - (smem_u32(prompt_smem_raw) & 1023u)) & 1023u);
   uint8_t* sQ = smem;
@@ -93,10 +93,9 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
     mbar_init(&q_full, 1);
-    mbar_init(&pv_done, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
-      mbar_init(&s_full[s], 1); mbar_init(&p_full[s], kPromptRows);
+      mbar_init(&s_full[s], 1); mbar_init(&p_full[s], kPromptRows); mbar_init(&pv_done[s], 1);
     }
     fence_mbar_init();
   }
@@ -115,7 +114,12 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int ctx0 = p.context_lens[b] - p.Q;
   const int kv_max = ctx0 + tok0 + tq;               // exclusive upper bound of the keys the tile sees
   const int n = (kv_max + kPromptKeys - 1) / kPromptKeys;
-  auto parity = [](int i) { return (uint32_t)(i >> 1) & 1u; };   // of the i-th use of a pair of barriers
+  // Every pair of barriers is used in turn, chunk i on barrier i & 1; parity(i) is that use's.  A wait by parity is only right while the barrier
+  // is in that use or the one behind it.  pv_done: whoever waits for chunk j has seen s_full of chunk j + 1 or later (or issued its
+  // scores), which was committed behind the product of chunk j - 1, and the product of chunk j + 2 needs the P that this thread (or this
+  // warp's rows) has not handed over yet.  (One barrier for all chunks could run a phase ahead of a softmax warp that is held up between
+  // handing P over and asking: the wait then never ended.)
+  auto parity = [](int i) { return (uint32_t)(i >> 1) & 1u; };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -170,7 +174,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int k = 0; k < kPromptKeys / 16; ++k)   // 16 keys: 2048 B of V, 8 columns of P
           umma_bf16_ts(tmem_o, tmem + (i & 1) * 64 + 8 * k, vd + 128 * k, idesc_o, (uint32_t)((i | k) != 0));
         umma_commit(&v_empty[i & 1]);
-        umma_commit(&pv_done);
+        umma_commit(&pv_done[i & 1]);
       }
     }
     __syncwarp();
@@ -184,8 +188,6 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const int base = i * kPromptKeys;
       const uint32_t sp = tmem + lanes + (uint32_t)(i & 1) * 64u;
       if (!(ok = warp_wait(&s_full[i & 1], parity(i), p.timeout))) break;
-      // (phase by phase, so that a parity is never taken for the one two phases on)
-      if (i > 1 && !(ok = warp_wait(&pv_done, (uint32_t)i & 1u, p.timeout))) break;
       tc_fence_after();
       uint32_t u[64];
 #pragma unroll
@@ -206,7 +208,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (grow) m = mx;
         l *= f;
         if (i > 0) {
-          if (!(ok = warp_wait(&pv_done, (uint32_t)(i - 1) & 1u, p.timeout))) break;
+          if (!(ok = warp_wait(&pv_done[(i - 1) & 1], parity(i - 1), p.timeout))) break;
           tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < HD; c += 16) {
@@ -243,8 +245,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tc_fence_before();
       mbar_arrive(&p_full[i & 1]);
     }
-    if (ok && n > 1) ok = warp_wait(&pv_done, (uint32_t)n & 1u, p.timeout);
-    if (ok && n > 0) ok = warp_wait(&pv_done, (uint32_t)(n - 1) & 1u, p.timeout);
+    if (ok && n > 0) ok = warp_wait(&pv_done[(n - 1) & 1], parity(n - 1), p.timeout);
     if (ok) {
       tc_fence_after();
       const float inv = l > 0.f ? 1.f / l : 0.f;
