@@ -165,7 +165,9 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       };
       bool ok = n > 0 && mbar_wait_cluster(&q_full, 0, p.timeout) && scores(0);
       for (int i = 0; i < n && ok; ++i) {
-        // (the buffer of chunk i + 1 is free: the product that read its P was issued before, and products run in order)
+        // the scores of chunk i + 1 go over the P that the product of chunk i - 1 reads: products of different shapes and accumulators
+        // have no order of their own
+        if (i > 0 && !(ok = mbar_wait_cluster(&pv_done[(i - 1) & 1], parity(i - 1), p.timeout))) break;
         if (i + 1 < n && !(ok = scores(i + 1))) break;
         if (!(ok = mbar_wait_cluster(&p_full[i & 1], parity(i), p.timeout) && mbar_wait_cluster(&v_full[i & 1], parity(i), p.timeout))) break;
         tc_fence_after();
