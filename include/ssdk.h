@@ -195,6 +195,9 @@ const void* ssdk_logits_last(ssdk_handle h);
  * after its grid dependency resolves; replaces the reference's SSD_PROFILE perf_counter prints (engine/step.py:92-161).
  * dev_buf = NULL turns tracing off. */
 int ssdk_debug_trace(void* dev_buf, int cap);
+/* Host word that this engine's kernels set when one of their bounded waits runs out.  Every call that waits for the stream fails
+ * once (and clears it) if it is set. */
+uint32_t* ssdk_debug_wait_word(ssdk_handle h);
 /* number of kernels this library launched (or replayed inside graphs) so far */
 int64_t ssdk_launch_count(ssdk_handle h);
 
@@ -514,6 +517,7 @@ int ssdk_hyb_forward(ssdk_hyb_handle h, int n_seqs, int n_tokens, const int32_t*
                      const float* temps, uint64_t seed, uint64_t step_id, int64_t* out_tokens,
                      float* residual_host, void* stream);
 int64_t ssdk_hyb_launch_count(ssdk_hyb_handle h);
+uint32_t* ssdk_hyb_debug_wait_word(ssdk_hyb_handle h);   /* as ssdk_debug_wait_word */
 
 #ifdef __cplusplus
 }

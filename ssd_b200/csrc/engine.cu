@@ -68,6 +68,7 @@ static int env_int(const char* name, int dflt) {
 // ------------------------------------------------------------------------------------------
 struct Launcher {
   cudaStream_t st = nullptr;
+  unsigned* gave_up = nullptr;   // the engine's word for waits that run out (WaitWord)
   bool pdl = false;       // PDL enabled at all
   bool prev_kernel = false;  // the previous op on the stream was one of our kernels
   int64_t count = 0;
@@ -234,25 +235,25 @@ static int launch_gemm(Launcher& L, int umma_n, int epi, const CUtensorMap& tmW,
   return fail("no GEMM instance for umma_n=%d epi=%d", umma_n, epi);
 }
 
-// Word in host memory that a kernel sets when one of its bounded waits runs out; read after the stream has been waited for.
-static unsigned* g_wait_flag = nullptr;
-static int wait_flag(unsigned** out) {
-  if (!g_wait_flag) {
-    unsigned* f = nullptr;
-    CK(cudaHostAlloc(&f, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable));
-    *f = 0;
-    g_wait_flag = f;
+// Word in host memory that the kernels of one engine set when a bounded wait of theirs runs out.  Read wherever a call has waited for the
+// stream: a call that does not wait (prompt passes without a token) leaves its report to the next one that does.
+struct WaitWord {
+  unsigned* word = nullptr;   // (unified addressing: the host pointer is the device's too)
+  WaitWord() = default;
+  WaitWord(const WaitWord&) = delete;
+  ~WaitWord() { if (word) cudaFreeHost(word); }
+  bool make() {
+    if (cudaHostAlloc(&word, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) { word = nullptr; return false; }
+    *word = 0;
+    return true;
   }
-  *out = g_wait_flag;   // (unified addressing: the host pointer is the device's too)
-  return 0;
-}
-static int check_waits() {
-  if (g_wait_flag && *(volatile unsigned*)g_wait_flag) {
-    *(volatile unsigned*)g_wait_flag = 0;
-    return fail("a wait inside a GEMM ran out");
+  int check() {
+    volatile unsigned* w = word;
+    if (!*w) return 0;
+    *w = 0;
+    return fail("a bounded wait in a tile-pair product or the prompt attention ran out: what this engine's calls left since the last check is not complete");
   }
-  return 0;
-}
+};
 
 // tile pairs of gemm_pair_kernel; p.timeout is filled in here
 static int launch_gemm_pair(Launcher& L, int epi, const CUtensorMap& tmW, const CUtensorMap& tmX, const CUtensorMap& tmXs, GemmPairParams p, int max_tiles) {
@@ -263,7 +264,7 @@ static int launch_gemm_pair(Launcher& L, int epi, const CUtensorMap& tmW, const 
     CK(cudaFuncSetAttribute(gemm_pair_kernel<EPI_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
     attr_set = true;
   }
-  CKI(wait_flag(&p.timeout));
+  p.timeout = L.gave_up;
   if (p.batch < 1) p.batch = 1;
   const dim3 grid(2 * std::min(max_tiles, num_sms() / 2)), block(kPairThreads);
   if (epi == EPI_BF16) return L.go(gemm_pair_kernel<EPI_BF16>, grid, block, (size_t)kPairSmem, tmW, tmX, tmXs, p);
@@ -277,7 +278,7 @@ static int launch_gemm_split(Launcher& L, const CUtensorMap& tmX, GemmSplitParam
     CK(cudaFuncSetAttribute(gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem));
     attr_set = true;
   }
-  CKI(wait_flag(&p.timeout));
+  p.timeout = L.gave_up;
   return L.go(gemm_split_kernel, dim3(2 * std::min(max_tiles, num_sms() / 2)), dim3(kSplitThreads), (size_t)kSplitSmem, tmX, p);
 }
 
@@ -414,6 +415,7 @@ struct ssdk_engine {
   void* ws_base = nullptr;
   int64_t ws_bytes = 0;
   XMapCache xmaps;
+  WaitWord waits;
   bool use_prompt_attn = env_int("SSDK_PROMPT_ATTN", 1) != 0;   // prompt passes on tcgen05 (0: mma.sync tiles)
   ncclComm_t comm = nullptr;
   bool finalized = false;
@@ -662,13 +664,11 @@ static int forward_prompt_attention(ssdk_engine* e, Launcher& L, const Model& m,
                                     const int32_t* ctx_lens, bf16* out, int B, int Q, int block_size, int max_blocks, float scale) {
   const int64_t slots = m.num_blocks * block_size;
   const int G = m.H / m.KV;
-  unsigned* timeout;
-  CKI(wait_flag(&timeout));
   const CUtensorMap *tmQ, *tmK, *tmV;
   CKI(e->xmaps.get_heads(q, kMaxPass, m.H, m.hd, G, kPromptRows / G, &tmQ));
   CKI(e->xmaps.get_heads(kc, slots, m.KV, m.hd, 1, kPromptKeys, &tmK));
   CKI(e->xmaps.get_heads(vc, slots, m.KV, m.hd, 1, kPromptKeys, &tmV));
-  return enqueue_prompt_attention(L, *tmQ, *tmK, *tmV, bt, ctx_lens, out, B, Q, m.H, m.KV, m.hd, block_size, max_blocks, slots, scale, timeout);
+  return enqueue_prompt_attention(L, *tmQ, *tmK, *tmV, bt, ctx_lens, out, B, Q, m.H, m.KV, m.hd, block_size, max_blocks, slots, scale, L.gave_up);
 }
 
 static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w, int M, int epi, void* out, int ldo,
@@ -1344,7 +1344,7 @@ int ssdk_create(const ssdk_model_cfg* target, const ssdk_model_cfg* draft, const
   }
   layout_step(e);
   e->max_ctx_hint = rt->max_blocks_per_seq * rt->block_size;
-  if (cudaHostAlloc((void**)&e->pin_in, e->step_bytes, cudaHostAllocDefault) != cudaSuccess ||
+  if (!e->waits.make() || cudaHostAlloc((void**)&e->pin_in, e->step_bytes, cudaHostAllocDefault) != cudaSuccess ||
       cudaHostAlloc((void**)&e->pin_out, e->out_bytes + 64 * 8, cudaHostAllocDefault) != cudaSuccess) {
     delete e;
     return fail("pinned staging allocation failed");
@@ -1546,6 +1546,7 @@ int ssdk_spec_step(ssdk_handle h, int batch, const int32_t* ctx_len, const int64
     h->launches += L.count;
   }
   CK(cudaStreamSynchronize(st));
+  CKI(h->waits.check());
   read_step(h, batch, out_tokens, out_n_accept, out_recovery);
   return 0;
 }
@@ -1560,7 +1561,7 @@ int ssdk_spec_step_stage(ssdk_handle h, int batch, const int32_t* ctx_len, const
   CK(cudaMemcpyAsync(h->ws.step_dev, h->pin_in, h->step_bytes, cudaMemcpyHostToDevice, st));
   CK(cudaMemsetAsync(h->ws.log_len, 0, (size_t)h->rt.max_batch * 4, st));
   CK(cudaStreamSynchronize(st));
-  return 0;
+  return h->waits.check();
 }
 
 int ssdk_spec_step_resident(ssdk_handle h, int batch, void* stream) {
@@ -1597,6 +1598,7 @@ int ssdk_spec_step_fetch(ssdk_handle h, int batch, int64_t* out_tokens, int32_t*
   int32_t* lens = (int32_t*)(h->pin_out + h->out_bytes);
   CK(cudaMemcpyAsync(lens, h->ws.log_len, (size_t)batch * 4, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  CKI(h->waits.check());
   read_step(h, batch, out_tokens, nullptr, out_recovery);
   if (out_n_accept) memcpy(out_n_accept, lens, (size_t)batch * 4);
   return 0;
@@ -1609,6 +1611,7 @@ int ssdk_spec_step_log(ssdk_handle h, int seq, int64_t* out_tokens, int cap, voi
   int32_t len = 0;
   CK(cudaMemcpyAsync(&len, h->ws.log_len + seq, 4, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  CKI(h->waits.check());
   const int n = std::min(std::min((int)len, cap), kLogCap);
   if (n > 0) {
     CK(cudaMemcpyAsync(out_tokens, h->ws.log_tokens + (size_t)seq * kLogCap, (size_t)n * 8, cudaMemcpyDeviceToHost, st));
@@ -1654,6 +1657,7 @@ static int forward_rows(ssdk_handle h, int which, int batch, int q_len, const in
   Launcher L;
   L.st = st;
   L.pdl = h->rt.use_pdl != 0;
+  L.gave_up = h->waits.word;
   Model& m = h->model[which];
   Fwd f;
   f.which = which; f.B = batch; f.Q = q_len; f.ids = w.ids_in; f.ids_stride = 1;
@@ -1677,7 +1681,7 @@ static int forward_rows(ssdk_handle h, int which, int batch, int q_len, const in
     CK(cudaMemcpyAsync(pin_ids, w.out_tok, (size_t)batch * 8, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (out_tokens) memcpy(out_tokens, pin_ids, (size_t)batch * 8);
-    CKI(check_waits());
+    CKI(h->waits.check());
   }
   h->launches += L.count;
   return 0;
@@ -1700,6 +1704,8 @@ int ssdk_prompt_pass(ssdk_handle h, int which, int batch, int q_len, const int64
   const int most = ssdk_prompt_pass_rows(h, which);
   return forward_rows(h, which, batch, q_len, ids, ctx_len, block_tables, want_sample, temps, seed, step_id, out_tokens, stream, std::max(most, kMaxTokens));
 }
+
+uint32_t* ssdk_debug_wait_word(ssdk_handle h) { return h ? h->waits.word : nullptr; }
 
 // debug: route the kernels' timeline marks into `dev_buf` (uint64 [cap][2]); dev_buf = NULL disables tracing
 int ssdk_debug_trace(void* dev_buf, int cap) {

@@ -119,6 +119,7 @@ struct ssdk_hyb_engine {
   }
   int64_t launches = 0;
   bool smem_attr_done = false;
+  WaitWord waits;
 };
 
 // delta rule: lanes per pair of state columns (LC) and 16-byte pieces per lane and column (NQ) of delta_chunk_scan_kernel,
@@ -1760,7 +1761,7 @@ static int hyb_forward_t(ssdk_hyb_engine* e, int n_seqs, int M, const int32_t* i
   // everything up to the logits on the device and the sampled tokens in pinned memory
   auto enqueue = [&](cudaStream_t on) -> int {
     run.L = Launcher();
-    run.L.st = on; run.L.pdl = e->use_pdl;
+    run.L.st = on; run.L.pdl = e->use_pdl; run.L.gave_up = e->waits.word;
     CK(cudaMemcpyAsync(d, hm, o * 4, cudaMemcpyHostToDevice, on));
     T* xt = (g.block == SSDK_BLOCK_SERIAL_POSTNORM && !std::is_same<T, float>::value) ? (T*)e->h : (T*)nullptr;
     if (HybRun<T>::whole16(g.width, {e->embed.p, e->x}))
@@ -1839,7 +1840,7 @@ static int hyb_forward_t(ssdk_hyb_engine* e, int n_seqs, int M, const int32_t* i
   if (logits_host && n_want > 0) CK(cudaMemcpyAsync(logits_host, e->logits, (size_t)n_want * g.vocab * 4, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   if (sample) memcpy(out_tokens, e->h_tokens, (size_t)n_want * 8);
-  return check_waits();
+  return e->waits.check();
 }
 
 extern "C" {
@@ -1915,7 +1916,7 @@ int ssdk_hyb_create(const ssdk_hyb_cfg* cfg, const ssdk_hyb_layer_cfg* layers, s
     }
   }
   e->ws_bytes = hyb_carve(e, nullptr);
-  if (cudaMallocHost(&e->h_meta, e->meta_ints * 4) != cudaSuccess || cudaMallocHost(&e->h_tokens, (size_t)cfg->max_logit_rows * 8) != cudaSuccess) {
+  if (!e->waits.make() || cudaMallocHost(&e->h_meta, e->meta_ints * 4) != cudaSuccess || cudaMallocHost(&e->h_tokens, (size_t)cfg->max_logit_rows * 8) != cudaSuccess) {
     if (e->h_meta) cudaFreeHost(e->h_meta);
     delete e;
     return fail("ssdk_hyb_create: pinned staging allocation failed");
@@ -2031,6 +2032,7 @@ int ssdk_hyb_forward(ssdk_hyb_handle e, int n_seqs, int n_tokens, const int32_t*
                               out_tokens, residual_host, st);
 }
 
+uint32_t* ssdk_hyb_debug_wait_word(ssdk_hyb_handle e) { return e ? e->waits.word : nullptr; }
 int64_t ssdk_hyb_launch_count(ssdk_hyb_handle e) { return e ? e->launches : -1; }
 
 }  // extern "C"

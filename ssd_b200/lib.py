@@ -127,6 +127,7 @@ SIGNATURES: dict[str, tuple] = {
     "ssdk_logits_q": (VP, [VP]),
     "ssdk_logits_last": (VP, [VP]),
     "ssdk_debug_trace": (C.c_int, [VP, C.c_int]),
+    "ssdk_debug_wait_word": (C.POINTER(C.c_uint32), [VP]),
     "ssdk_launch_count": (C.c_int64, [VP]),
     "ssdk_gemm_small_m": (C.c_int, [VP, VP, VP, VP, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, VP]),
     "ssdk_gemm_gate_up_silu": (C.c_int, [VP, VP, VP, C.c_int, C.c_int, C.c_int, VP]),
@@ -153,6 +154,7 @@ SIGNATURES: dict[str, tuple] = {
     "ssdk_hyb_bind_pools": (C.c_int, [VP, VP, C.c_int64, VP, C.c_int64, VP, C.c_int64]),
     "ssdk_hyb_forward": (C.c_int, [VP, C.c_int, C.c_int, c_i32p, c_i32p, c_i32p, c_i32p, c_i32p, C.c_int, c_i32p, c_f32p,
                                    c_f32p, C.c_uint64, C.c_uint64, c_i64p, c_f32p, VP]),
+    "ssdk_hyb_debug_wait_word": (C.POINTER(C.c_uint32), [VP]),
     "ssdk_hyb_launch_count": (C.c_int64, [VP]),
 }
 
