@@ -6,8 +6,12 @@
 // are below 2^-26.  The tensor core truncates when it adds to its fp32 accumulator: measured against 64 bits (random signs) 2.2e-7 of
 // the result over 256 steps of k but 2.1e-6 over 2048, where a chain of FMAs is off by 1.0e-7 and 3.8e-7.  So the hh sums leave TMEM every
 // 256 k and are added up in registers (fp32, round to nearest); the five small terms, 2^-8 of the result, stay in an accumulator of
-// their own up to the end.  Relative error of 1000 x 4096 x 2048 against 64 bits: 2.4e-7, the FMA form 7.9e-7.  An infinite operand
-// gives NaN (inf - inf between its pieces).
+// their own up to the end.  Relative error of 1000 x 4096 x 2048 against 64 bits: 2.4e-7, the FMA form 7.9e-7.
+//
+// Where pieces do not do: an operand that is infinite or above bf16's largest number (3.39e38) has an infinite first piece, so that its
+// products are infinite or NaN, and pieces below bf16's normal range (2^-126) may be lost, which is below 2^-24 of a result from 2^-70
+// on (as long as K times the largest other operand is below 2^30).  Results that are not finite, and results below 2^-70 that are not zero, are
+// therefore taken again as the FMA chain over k that linear_kernel walks (see split_again).  What still differs: a result below 2^-126 may be zero.
 //
 // What bounds it: the tensor core, 24 products of 64 clocks per k-block of 64 and 128 tokens, under which everything else hides.  The
 // FMA form it takes over from (linear_kernel, 64 x 64 tiles) was bound by its shared-memory operands: 1000 x 4096 x 2048 539 us (31 TFLOP/s)
@@ -36,6 +40,10 @@ struct GemmSplitParams {
   int w_tiles, chunks;        // tiles of 256 columns; chunks of kSplitTokens rows (dense)
   int batch;                  // dense: products of the same shape, their weights and results w_stride and c_stride floats apart, X's rows in turn
   int plane_rows;             // rows of one piece of X (the map holds three of them)
+  const float* X;             // the rows themselves, for results that are taken again: row r of matrix b is row x_rows[r] (or r) from X + b x_stride
+  const int* x_rows;
+  long long x_stride;
+  int ldx;
   long long w_stride, c_stride;   // grouped: w_stride between two experts
   const int* g_tile_expert;   // grouped mode: see GemmParams (tiles of up to kSplitTokens rows)
   const int* g_tile_row0;
@@ -79,6 +87,13 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
   }
 }
 
+// a result that the pieces cannot vouch for: infinite, NaN, or below 2^-70 and not zero
+SSDK_DEVINL bool split_again(float v) {
+  constexpr uint32_t lo = (127u - 70u) << 24, hi = 255u << 24;
+  const uint32_t u = __float_as_uint(v) << 1;
+  return u != 0u && u - lo >= hi - lo;
+}
+
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSplitThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams p) {
   extern __shared__ uint8_t split_smem_raw[];
@@ -86,6 +101,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
   __shared__ __align__(8) uint64_t empty_bar[kSplitStages];
   __shared__ __align__(8) uint64_t main_full[2], main_empty[2], rest_full[2], rest_empty[2];
   __shared__ uint32_t tmem_slot;
+  __shared__ int s_again;   // some result of this CTA's is to be taken again
   uint8_t* smem = split_smem_raw + ((1024u - (smem_u32(split_smem_raw) & 1023u)) & 1023u);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -97,6 +113,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
     for (int s = 0; s < kSplitStages; ++s) { mbar_init(&full_bar[s], 9); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&main_full[b], 1); mbar_init(&main_empty[b], 8); mbar_init(&rest_full[b], 1); mbar_init(&rest_empty[b], 8); }
     fence_mbar_init();
+    s_again = 0;
   }
   if (warp == 1) tmem_alloc_pair(&tmem_slot);
   tc_fence_before();
@@ -226,9 +243,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
       const int n = tl.col + q * 32 + lane;
       if (n < p.N) {
         float* out = p.out + tl.b * p.c_stride + ((size_t)tl.split * p.M + tl.m0) * p.ldc + n;
+        bool again = false;
 #pragma unroll
         for (int m = 0; m < kSplitTokens; ++m)
-          if (m < tl.rows) out[(size_t)m * p.ldc] = acc[m];
+          if (m < tl.rows) { out[(size_t)m * p.ldc] = acc[m]; again |= split_again(acc[m]); }
+        if (again) s_again = 1;
       }
     }
     __syncwarp();
@@ -286,6 +305,26 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
 
   tc_fence_before();
   __syncthreads();
+  if (s_again) {   // (nothing waits for this CTA any more but its partner's exit)
+    for (int t = pair; t < tiles; t += n_pairs) {
+      const Tile tl = tile_of(t);
+      for (int i = threadIdx.x; i < tl.rows * 128; i += kSplitThreads) {
+        const int r = tl.m0 + (i >> 7), n = tl.col + (i & 127);
+        if (n >= p.N) continue;
+        float* out = p.out + tl.b * p.c_stride + ((size_t)tl.split * p.M + r) * p.ldc + n;
+        if (!split_again(*out)) continue;
+        const float* x = p.X + tl.b * p.x_stride + (size_t)(p.x_rows ? p.x_rows[r] : r) * p.ldx;
+        const float* w = p.W + tl.w0 + (long long)n * p.ldw;
+        const int k1 = min(p.K, tl.kb1 * kBlockK);
+        float s = 0.f;
+        for (int k = tl.kb0 * kBlockK; k < k1; k += 4) {
+          const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(w + k);
+          s = fmaf(a.x, b.x, s); s = fmaf(a.y, b.y, s); s = fmaf(a.z, b.z, s); s = fmaf(a.w, b.w, s);
+        }
+        *out = s;
+      }
+    }
+  }
   cluster_sync_all();
   if (warp == 1) tmem_dealloc_pair(tmem_slot);
 }

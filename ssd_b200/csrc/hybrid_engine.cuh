@@ -534,6 +534,7 @@ struct HybRun {
     CKI(L.go(ssdk::split_rows_kernel, dim3(m, batch), dim3(std::min(256, (p.K / 4 + 31) / 32 * 32)), 0, (const float*)A, lda, sA, gather, n_rows, (bf16*)e->pieces, p.K));
     const CUtensorMap* tm;
     CKI(e->tmap(e->pieces, 3LL * m * batch, p.K, 64, &tm));
+    p.X = (const float*)A; p.ldx = lda; p.x_stride = sA; p.x_rows = gather;
     p.M = m; p.plane_rows = m * batch; p.batch = batch; p.num_kb = (p.K + kBlockK - 1) / kBlockK; p.w_tiles = (p.N + 255) / 256;
     const int tiles = p.w_tiles * row_tiles * batch;
     // few tiles: k ranges of whole segments (dense results only; summed in the order of the ranges)

@@ -50,3 +50,50 @@ def test_three_pieces_match_the_oracle(tmp_path, monkeypatch, arch):
                 at += n
             errs[mode] = U.rel_err(np.concatenate(got), want)
         assert errs["2"] < TOL and errs["2"] < max(1e-6, 1.5 * errs["0"]), (cuts, errs)
+
+
+def test_infinite_largest_and_tiny_operands(tmp_path, monkeypatch):
+    """Operands that three bf16 pieces cannot hold give what the FMA form gives: the same infinities and NaNs, the same numbers for values
+    above bf16's largest and for results of any size.  Wide head rows (whole products), few and many rows, split k, and one expert."""
+    from ssd_b200.hybrid import HybridRunner, HybridSpec, load_hybrid_weights
+    U, cfg, _ = _model("vegilix")
+    path = U.write_checkpoint(str(tmp_path / "ckpt"), cfg, U.random_tensors(cfg, 1))
+    spec = HybridSpec.from_dir(path)
+    inf, big, g = float("inf"), 3.395e38, torch.Generator().manual_seed(4)
+    small = [1e-20, 1e-27, 1e-33, 1e-36]
+
+    def run(mode, change):
+        monkeypatch.setenv("SSDK_HYB_SPLIT", mode)
+        w = load_hybrid_weights(path, spec, torch.float32, "cuda:0")
+        change(w)
+        r = HybridRunner(spec, w, dtype="float32", max_tokens=300, max_seqs=2, block_size=16, num_blocks=40, n_slots=2, max_model_len=320)
+        toks = torch.randint(0, cfg["vocab"], (261,), generator=torch.Generator().manual_seed(2)).tolist()
+        out = [r.forward([(toks[:n], 0, 0, list(range(20)), list(range(n)))])[0] for n in (1, 7, 261)]
+        r.close()
+        return np.concatenate(out)
+
+    def head(w):
+        h = w["HEAD"]
+        h[3, 7] = inf
+        h[5, 0], h[5, 599] = inf, -inf
+        h[9, 64] = big
+        h[10] = h[10] * 1e-3
+        h[10, 300] = -big
+        h[11, 1] = float("nan")
+        for i, f in enumerate(small):
+            h[20 + i] = h[20 + i] * f
+
+    def expert(w):
+        w["layers"][0]["EXPERT_IN"].view(-1, 600)[17, 5] = inf
+
+    with np.errstate(all="ignore"):
+        for change in (head, expert):
+            a, b = run("0", change), run("2", change)
+            assert not np.isfinite(a).all()
+            assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(np.where(np.isinf(a), np.sign(a), 0), np.where(np.isinf(b), np.sign(b), 0))
+        a, b = (run(mode, head).astype(np.float64) for mode in ("0", "2"))
+    for col in [9, 10, 20, 21, 22, 23]:
+        ok = np.isfinite(a[:, col])
+        x, y = a[ok, col], b[ok, col]
+        size = np.abs(x).max()   # (the squares of 1e-36 are not numbers)
+        assert ok.any() and np.linalg.norm((x - y) / size) < TOL * np.linalg.norm(x / size), col
