@@ -287,7 +287,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         const int j = idx & 63, m = idx >> 6, n = col_lo + j;
         if (n < p.N) {
           const float g = ex[j * LD + m], u = ex[(64 + j) * LD + m];
-          const float a = p.glu_gelu ? 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) : __fdividef(g, 1.0f + __expf(-g));
+          const float a = p.glu_gelu ? 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) : g / (1.0f + expf(-g));
           out[(size_t)(m_base + m0 + m) * p.ldo + n] = f2bf(a * u);
         }
       }

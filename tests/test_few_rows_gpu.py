@@ -49,3 +49,27 @@ def test_latent_decoding_at_tile_edges(tmp_path, monkeypatch):
     for n, a, b in zip(lens, rows["1"], rows["0"]):
         assert np.isfinite(a).all()
         assert U.rel_err(a, b) < 2.0 ** -8, f"{n} keys"
+
+
+def test_gate_far_below_zero(tmp_path, monkeypatch):
+    """silu(g) for g around -88, where 1 + e^-g is near fp32's largest number and silu(g) is not zero yet, under an up projection that
+    makes it visible.  One nonzero weight per gate and up row and an identity behind them: both forms compute the same numbers."""
+    ff = W = 192
+    mlp = U.moe(experts=3, identity=1, top=2, groups=2, keep=2, ff=ff, shared_ff=None)
+    cfg = U.config([U.latent(heads=2, dim=16, rot_dim=16, vdim=16, kv_rank=48, mlp=mlp)], width=W)
+    t = U.random_tensors(cfg, 13, correction=1.0)
+    size = torch.logspace(np.log10(60.0), np.log10(200.0), ff // 2)
+    for e in range(3):
+        gate, up = torch.zeros(ff, W), torch.zeros(ff, W)
+        gate[:, 0] = torch.cat([size, -size])
+        up[:, 1] = 2.0 ** 117
+        t[f"l0.mlp.e{e}.gate"], t[f"l0.mlp.e{e}.up"], t[f"l0.mlp.e{e}.down"] = gate.bfloat16().float(), up, torch.eye(W)
+    path = U.write_checkpoint(str(tmp_path / "c"), cfg, t)
+    none = U.write_checkpoint(str(tmp_path / "d"), cfg, {k: torch.zeros_like(v) if ".down" in k else v for k, v in t.items()})
+    toks, rows = _tokens(16, cfg["vocab"], 5), []
+    for tc, p in (("1", path), ("0", path), ("0", none)):
+        monkeypatch.setenv("SSDK_HYB_TC_EXPERTS", tc)
+        rows.append(_load(p, "bfloat16", max_tokens=64, num_blocks=24).forward([(toks, 0, 0, _pages(16, 16), [0])], residual=True)[2][0])
+    size = np.abs(rows[1] - rows[2])
+    assert ((size > 1e-4) & (size < 1)).any()   # (what the gates around -88 leave)
+    assert np.array_equal(rows[0], rows[1])
