@@ -228,7 +228,9 @@ __global__ void sink_softmax_row_kernel(const float* __restrict__ sc, T* __restr
   const int jk = min(min(mask.keep, j0), n);
   const float* srow = sc + (size_t)r * ld;
   const float sk = sink ? ld_f<T>(sink + batch * H + h) : (sink_const > 0.f ? logf(sink_const) : -INFINITY);
+  static_assert(HOLD <= 8, "a bit per held column");
   float v[HOLD][4], mx = sk;
+  uint32_t seen = 0;   // the visible ones among the held columns (a visible score may be -inf itself)
 #pragma unroll
   for (int i = 0; i < HOLD; ++i) {
     const int j = (i * blockDim.x + threadIdx.x) * 4;
@@ -237,8 +239,9 @@ __global__ void sink_softmax_row_kernel(const float* __restrict__ sc, T* __restr
     v[i][0] = f.x; v[i][1] = f.y; v[i][2] = f.z; v[i][3] = f.w;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const bool seen = (j + e >= j0 && j + e < n) || j + e < jk;
-      v[i][e] = seen ? v[i][e] * scale : -INFINITY;
+      const bool s = (j + e >= j0 && j + e < n) || j + e < jk;
+      seen |= (uint32_t)s << (4 * i + e);
+      v[i][e] = s ? v[i][e] * scale : -INFINITY;
       mx = fmaxf(mx, v[i][e]);
     }
   }
@@ -252,7 +255,7 @@ __global__ void sink_softmax_row_kernel(const float* __restrict__ sc, T* __restr
   for (int i = 0; i < HOLD; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const float x = v[i][e] == -INFINITY ? 0.f : expf(v[i][e] - mx);
+      const float x = seen >> (4 * i + e) & 1u ? expf(v[i][e] - mx) : 0.f;
       v[i][e] = x;
       sum += x;
     }
@@ -264,7 +267,7 @@ __global__ void sink_softmax_row_kernel(const float* __restrict__ sc, T* __restr
     if (j >= ld) continue;
     float o[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) o[e] = v[i][e] == 0.f ? 0.f : v[i][e] * inv;   // (a row that sees nothing has no finite inv)
+    for (int e = 0; e < 4; ++e) o[e] = seen >> (4 * i + e) & 1u ? v[i][e] * inv : 0.f;   // (a row that sees nothing has no finite inv)
     st_four<T>(pr + (size_t)r * ld + j, o);
   }
 }

@@ -56,3 +56,15 @@ def test_softmax_row_edges(tmp_path, n):
         rows.append(r.forward([(toks[at:], at, slot, pages, [last - 1])])[0][-1])
     assert np.isfinite(rows[0]).all()
     assert U.rel_err(rows[0], rows[1]) < 16 * max(n, 16) ** 0.5 * 2.0 ** -23
+
+
+def test_softmax_over_infinite_scores(tmp_path):
+    """A row whose only visible score is -inf has no softmax (NaN, as inf - inf), like one whose score is +inf; both rows of a prompt of
+    two tokens whose keys hold an infinity in an entry that is not rotated."""
+    cfg = U.config([U.latent(heads=1, rot_dim=8, dims=4, scale=1.0)])
+    t = U.random_tensors(cfg, 3)
+    t["l0.mix.dkv"][20 + 6, 0] = float("inf")   # (kv_rank 20, then the key's 8 entries)
+    r = _load(U.write_checkpoint(str(tmp_path / "ckpt"), cfg, t), max_tokens=64)
+    for tok in range(16):
+        rows = r.forward([([tok, 2 * tok + 1], 0, 0, _pages(2, 16), [0, 1])])[0]
+        assert np.isnan(rows[0]).all(), tok
