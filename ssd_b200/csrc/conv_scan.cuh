@@ -438,12 +438,6 @@ __global__ void selective_scan_kernel(const SelScanArgs p, const Ragged rg) {
   }
 }
 
-// 2^x as the instruction gives it (error 2^-22; results below the normal range are zero)
-SSDK_DEVINL float ex2_approx(float x) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
 // Portions of many rows, N <= NT <= 16: pieces of a sequence's rows as in rglru_chunk_scan_kernel, a channel's states in the registers of
 // one lane.  A piece's decay of state n is exp(A_n sum dt).  Six rows are taken together: their B | C rows (one coalesced load each)
 // wait in shared memory for all lanes, the next six rows' loads are in flight under them.  Bound by issue slots and by the exponentials
@@ -511,7 +505,7 @@ __global__ void __launch_bounds__(kScanChunks * 32) selective_chunk_scan_kernel(
             const float4 b = B[n / 4];
             const float bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) S[n + i] = fmaf(ex2_approx(d[k] * A2[n + i]), S[n + i], dx * bv[i]);
+            for (int i = 0; i < 4; ++i) S[n + i] = fmaf(exp2f(d[k] * A2[n + i]), S[n + i], dx * bv[i]);
             if (kOut) {
               const float4 cv = B[(NT + n) / 4];
               y = fmaf(S[n], cv.x, y); y = fmaf(S[n + 1], cv.y, y); y = fmaf(S[n + 2], cv.z, y); y = fmaf(S[n + 3], cv.w, y);
@@ -533,7 +527,7 @@ __global__ void __launch_bounds__(kScanChunks * 32) selective_chunk_scan_kernel(
   for (int v = 0; v < w; ++v) {
     const float d = s_dt[v][lane];
 #pragma unroll
-    for (int n = 0; n < NT; ++n) S[n] = fmaf(ex2_approx(d * A2[n]), S[n], s_state[v][n][lane]);
+    for (int n = 0; n < NT; ++n) S[n] = fmaf(exp2f(d * A2[n]), S[n], s_state[v][n][lane]);
   }
   walk(std::true_type{});
   if (live && m0 < m1 && m1 == r1) {
