@@ -517,6 +517,7 @@ int ssdk_hyb_forward(ssdk_hyb_handle h, int n_seqs, int n_tokens, const int32_t*
                      const float* temps, uint64_t seed, uint64_t step_id, int64_t* out_tokens,
                      float* residual_host, void* stream);
 int64_t ssdk_hyb_launch_count(ssdk_hyb_handle h);
+int64_t ssdk_hyb_graphs_made(ssdk_hyb_handle h);   /* graphs of decode steps made so far */
 uint32_t* ssdk_hyb_debug_wait_word(ssdk_hyb_handle h);   /* as ssdk_debug_wait_word */
 
 #ifdef __cplusplus

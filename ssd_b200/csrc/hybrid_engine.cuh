@@ -34,9 +34,13 @@ constexpr int kFewTile = 16;   // rows of a routed expert's tile in calls of few
 
 struct HybGraph {            // a decode step's launches
   cudaGraphExec_t exec = nullptr;
-  bool seen = false;
-  int64_t launches = 0;
+  int plain = 0;             // steps of this kind that ran as plain launches
+  int64_t launches = 0, last = 0;   // last: the step that used it last
 };
+// Making a graph costs about two steps, replaying one saves a twentieth of a step and more: kinds that come up only a few times stay plain
+// launches, and a step costs 1.5 times its launches at worst.  Kinds are counts and context splits (up to 32 of them over the first 2048
+// tokens of a batch); the least used one makes room.
+constexpr int kGraphAfter = 4, kGraphKinds = 64;
 
 struct ssdk_hyb_engine {
   ssdk_hyb_cfg cfg;
@@ -72,6 +76,20 @@ struct ssdk_hyb_engine {
   int64_t* h_tokens = nullptr; // pinned: the sampled tokens
   bool use_graph = true, use_pdl = true;   // decode steps replayed as graphs; programmatic dependent launch (SSDK_HYB_GRAPH=0, SSDK_HYB_PDL=0)
   std::map<std::vector<int>, HybGraph> graphs;
+  int64_t graph_clock = 0, graphs_made = 0;
+  HybGraph* graph_of(const std::vector<int>& key) {
+    auto it = graphs.find(key);
+    if (it == graphs.end()) {
+      if (graphs.size() >= kGraphKinds) {
+        auto old = std::min_element(graphs.begin(), graphs.end(), [](const auto& a, const auto& b) { return a.second.last < b.second.last; });
+        if (old->second.exec) cudaGraphExecDestroy(old->second.exec);   // (every call waits for its stream: nothing is in flight)
+        graphs.erase(old);
+      }
+      it = graphs.emplace(key, HybGraph()).first;
+    }
+    it->second.last = ++graph_clock;
+    return &it->second;
+  }
   cudaStream_t cap_stream = nullptr;
   void drop_graphs() {       // also when a buffer that their launches name is bound anew
     for (auto& kv : graphs)
@@ -734,18 +752,30 @@ struct HybRun {
   }
 
   bool by_position = false;   // some launch followed from positions in another way than decode_key knows (attention without a fused decode form)
-  // the sizes that the launches of a decode step depend on beside the counts: every attention layer's context splits follow from the
-  // longest visible context in tiles of 64 keys
+  uint8_t* layer_pool(const HybLayer& Lr) const { return e->cache + (size_t)e->num_blocks * e->cfg.block_size * Lr.cache_rows_before * e->esz; }
+  // context splits of the single-token rows of a latent layer: ~2 CTAs per SM over all sequences, at least 64 keys per split
+  static int latent_splits(int n_dec, int ctx_max) { return std::max(1, std::min({ssdk::kDecMaxSplits, 2 * num_sms() / n_dec, (ctx_max + 63) / 64})); }
+  // grouped-query attention on the tensor cores: bf16, heads of whole 16-byte pieces up to 128 wide, up to 16 query heads per key/value head
+  bool gqa_on_mma(const HybLayer& Lr) const {
+    const ssdk_hyb_layer_cfg& c = Lr.c;
+    return !kF32 && e->use_gqa_mma && c.dim % 8 == 0 && c.vdim % 8 == 0 && std::max(c.dim, c.vdim) <= 128 && c.heads / c.kv_heads <= 16 &&
+           ((uintptr_t)layer_pool(Lr) & 15) == 0;
+  }
+  // its splits.  Tensor cores: ~3 four-warp CTAs per SM, at least a tile of keys each; CUDA cores: ~8 per SM (a CTA per head)
+  int gqa_splits(const HybLayer& Lr, int n_dec, int ctx_max) const {
+    const int H = Lr.c.heads * Lr.c.maps, G = Lr.c.kv_heads * Lr.c.maps;
+    return std::max(1, gqa_on_mma(Lr) ? std::min({ssdk::kGqaMaxSplits, 3 * num_sms() / std::max(1, n_dec * G), (ctx_max + ssdk::kGmKeys - 1) / ssdk::kGmKeys})
+                                      : std::min({ssdk::kGqaMaxSplits, 8 * num_sms() / std::max(1, n_dec * H), (ctx_max + 127) / 128}));
+  }
+  // what the launches of a decode step depend on beside the counts: every attention layer's context splits
   void decode_key(std::vector<int>& key) const {
-    int last[3] = {-1, -1, -1};
     for (const HybLayer& Lr : e->layers) {
       const ssdk_hyb_layer_cfg& c = Lr.c;
-      if (!Lr.cache_row && !(c.mixer == SSDK_MIX_LATENT_ATTN)) continue;
-      if (c.window == last[0] && c.chunk == last[1] && c.keep_first == last[2]) continue;
-      last[0] = c.window; last[1] = c.chunk; last[2] = c.keep_first;
+      const bool latent = c.mixer == SSDK_MIX_LATENT_ATTN;
+      if (!Lr.cache_row && !latent) continue;
       int ctx = 0;
-      decode_rows(ssdk::KeyMask{c.window, c.chunk, c.keep_first}, &ctx);
-      key.push_back(std::min((ctx + 63) / 64, 64));   // (at most 32 splits of 64 or 128 keys)
+      const int n_dec = decode_rows(ssdk::KeyMask{c.window, c.chunk, latent ? 0 : c.keep_first}, &ctx);
+      key.push_back(latent ? latent_splits(n_dec, ctx) : gqa_splits(Lr, n_dec, ctx));
     }
   }
 
@@ -760,7 +790,7 @@ struct HybRun {
     if (own) CKI(check_tensor(Lr, SSDK_HT_LAT_KVNORM, KR, 1, "dkv.norm"));
     if (c.learned_sink) CKI(check_tensor(Lr, SSDK_HT_LAT_SINK, H, 1, "sink"));
     if (!e->cache) return fail("hybrid: latent cache not bound");
-    uint8_t* pool = e->cache + (size_t)e->num_blocks * e->cfg.block_size * Lr.cache_rows_before * e->esz;
+    uint8_t* pool = layer_pool(Lr);
     const void* sink = c.learned_sink ? Lr.t[SSDK_HT_LAT_SINK].p : nullptr;
     const float* q = nullptr;       // fp32 query rows [H, D + R] with leading dimension ldq
     const float* gate = nullptr;    // fp32 pre-activations of the output gate [H V], leading dimension ldq
@@ -809,8 +839,7 @@ struct HybRun {
       const int ks_per = ((Wd + 15) / 16 + 3) / 4, nt_per = ((KR + 7) / 8 + 3) / 4;
       const bool mma = !kF32 && e->use_decode_mma && pool_aligned && Wd % 8 == 0 && KR % 8 == 0 && ks_per <= 9 && nt_per <= 16;
       if (n_dec > 0 && (mma || smem <= 200 * 1024) && e->use_decode_attn) {
-        // ~2 CTAs per SM over all sequences, at least 64 keys per split, partials within the score buffer
-        int splits = std::max(1, std::min({ssdk::kDecMaxSplits, 2 * num_sms() / n_dec, (ctx_max + 63) / 64}));
+        int splits = latent_splits(n_dec, ctx_max);   // (partials within the score buffer)
         const size_t per_split = (size_t)rg.n_seqs * H * (KR + 2);
         splits = (int)std::min<size_t>(splits, e->att_elems / per_split);
         if (splits >= 1) {
@@ -1142,7 +1171,7 @@ struct HybRun {
     const ssdk::DiffArgs diff = {Lr.t[SSDK_HT_ATTN_DIFF].p, D, c.diff, e->cfg.eps};
     const float sink_const = sinks ? 0.f : c.sink;
     if (!e->cache) return fail("hybrid: attention cache not bound");
-    uint8_t* pool = e->cache + (size_t)e->num_blocks * e->cfg.block_size * Lr.cache_rows_before * e->esz;
+    uint8_t* pool = layer_pool(Lr);
     ssdk::GqaPrepArgs pa;
     pa.z = z; pa.ldz = ldz; pa.q = e->qcat; pa.cache = pool; pa.inv_freq = c.rot_dims >= 2 ? Lr.inv_freq : nullptr;
     pa.H = H; pa.G = G; pa.D = D; pa.V = V; pa.rot_dims = c.rot_dims; pa.qk_norm = c.qk_norm; pa.rot_mult = Lr.rot_mult; pa.eps = e->cfg.eps;
@@ -1172,8 +1201,7 @@ struct HybRun {
     } else {
       CKI(L.go(ssdk::gqa_prep_kernel<T>, dim3(M, (H + G + ssdk::kPrepHeads - 1) / ssdk::kPrepHeads), dim3(32, ssdk::kPrepHeads), 0, pa, rg));
     }
-    // tensor-core forms: bf16, heads of whole 16-byte pieces up to 128 wide, up to 16 query heads per key/value head
-    const bool mma = !kF32 && e->use_gqa_mma && D % 8 == 0 && V % 8 == 0 && std::max(D, V) <= 128 && hpg <= 16 && ((uintptr_t)pool & 15) == 0;
+    const bool mma = gqa_on_mma(Lr);
     const int ks = std::max(D, V) <= 32 ? 2 : (std::max(D, V) <= 64 || (maps == 2 && D <= 64) ? 4 : 8);
     const int vt = V <= 64 && ks < 8 ? 2 * ks : 16;   // (two maps: value heads are often twice as wide as the keys)
     bool fused_decode = false;
@@ -1182,10 +1210,7 @@ struct HybRun {
       const int n_dec = decode_rows(mask, &ctx_max);
       const int vpl = (V + 31) / 32;
       if (n_dec > 0 && (mma || vpl <= 8) && e->use_decode_attn) {
-        // tensor cores: ~3 four-warp CTAs per SM, at least a tile of keys each; CUDA cores: ~8 per SM (a CTA per head)
-        int splits = mma ? std::min({ssdk::kGqaMaxSplits, 3 * num_sms() / std::max(1, n_dec * G), (ctx_max + ssdk::kGmKeys - 1) / ssdk::kGmKeys})
-                         : std::min({ssdk::kGqaMaxSplits, 8 * num_sms() / std::max(1, n_dec * H), (ctx_max + 127) / 128});
-        splits = std::max(1, splits);
+        int splits = gqa_splits(Lr, n_dec, ctx_max);
         const size_t per_split = (size_t)rg.n_seqs * H * (V + 2);
         splits = (int)std::min<size_t>(splits, e->att_elems / per_split);
         if (splits >= 1) {
@@ -1812,10 +1837,9 @@ static int hyb_forward_t(ssdk_hyb_engine* e, int n_seqs, int M, const int32_t* i
   if (e->use_graph && M == n_seqs && !residual_host) {
     std::vector<int> key = {n_seqs, n_want, (int)sample};
     run.decode_key(key);
-    if (e->graphs.size() >= 64 && !e->graphs.count(key)) e->drop_graphs();
-    hg = &e->graphs[key];
+    hg = e->graph_of(key);
   }
-  if (hg && !hg->exec && hg->seen) {   // (the first step of a kind is launched as it is: a graph costs about two steps to make)
+  if (hg && !hg->exec && hg->plain >= kGraphAfter) {
     if (!e->cap_stream) CK(cudaStreamCreateWithFlags(&e->cap_stream, cudaStreamNonBlocking));
     CK(cudaStreamBeginCapture(e->cap_stream, cudaStreamCaptureModeRelaxed));
     const int rc = enqueue(e->cap_stream);
@@ -1827,6 +1851,7 @@ static int hyb_forward_t(ssdk_hyb_engine* e, int n_seqs, int M, const int32_t* i
       e->use_graph = false;
     } else {
       hg->launches = run.L.count;
+      ++e->graphs_made;
     }
     if (graph) cudaGraphDestroy(graph);
   }
@@ -1836,7 +1861,7 @@ static int hyb_forward_t(ssdk_hyb_engine* e, int n_seqs, int M, const int32_t* i
   } else {
     CKI(enqueue(st));
     e->launches += run.L.count;
-    if (hg) hg->seen = !run.by_position;
+    if (hg) hg->plain = run.by_position ? 0 : hg->plain + 1;
   }
   if (logits_host && n_want > 0) CK(cudaMemcpyAsync(logits_host, e->logits, (size_t)n_want * g.vocab * 4, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
@@ -2034,6 +2059,7 @@ int ssdk_hyb_forward(ssdk_hyb_handle e, int n_seqs, int n_tokens, const int32_t*
 }
 
 uint32_t* ssdk_hyb_debug_wait_word(ssdk_hyb_handle e) { return e ? e->waits.word : nullptr; }
+int64_t ssdk_hyb_graphs_made(ssdk_hyb_handle e) { return e ? e->graphs_made : -1; }
 int64_t ssdk_hyb_launch_count(ssdk_hyb_handle e) { return e ? e->launches : -1; }
 
 }  // extern "C"

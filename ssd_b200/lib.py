@@ -155,6 +155,7 @@ SIGNATURES: dict[str, tuple] = {
     "ssdk_hyb_forward": (C.c_int, [VP, C.c_int, C.c_int, c_i32p, c_i32p, c_i32p, c_i32p, c_i32p, C.c_int, c_i32p, c_f32p,
                                    c_f32p, C.c_uint64, C.c_uint64, c_i64p, c_f32p, VP]),
     "ssdk_hyb_debug_wait_word": (C.POINTER(C.c_uint32), [VP]),
+    "ssdk_hyb_graphs_made": (C.c_int64, [VP]),
     "ssdk_hyb_launch_count": (C.c_int64, [VP]),
 }
 

@@ -43,3 +43,43 @@ def test_same_bits_as_plain_launches(monkeypatch, arch, dtype):
     assert n == n_plain
     for i, (a, b) in enumerate(zip(want, got)):
         assert np.array_equal(a, b), f"output {i}"
+
+
+def _decode(r, n, pos, sample):
+    temps = [0.0] * n if sample else None
+    return r.forward([([7 + i], pos, i, [i], [0]) for i in range(n)], temps=temps)
+
+
+def test_kinds_of_steps_keep_their_graphs(monkeypatch):
+    """A kind of step gets its graph once: not again while other kinds come and go (more of them than are kept), nor along a context whose
+    splits stay; kinds that come up a few times get none.  The numbers are those of plain launches throughout."""
+    from ssd_b200 import hybrid_bench as hb
+    from ssd_b200.hybrid import HybridRunner, random_hybrid_weights
+    spec = hb.kokatar_spec(dict(hb.SIZES["s"], layers=1, vocab=512))
+    w = random_hybrid_weights(spec, torch.bfloat16, "cuda:0", seed=2)
+    runners = []
+    for plain in (True, False):
+        monkeypatch.setenv("SSDK_HYB_GRAPH", "0" if plain else "1")
+        runners.append(HybridRunner(spec, w, max_tokens=64, max_seqs=40, block_size=1024, num_blocks=40, n_slots=40, max_model_len=1024))
+    made = lambda: runners[1].lib.ssdk_hyb_graphs_made(runners[1].h)
+
+    def both(*a):
+        (la, ta), (lb, tb) = (_decode(r, *a) for r in runners)
+        assert np.array_equal(la, lb) and ta == tb
+
+    for _ in range(3):
+        both(3, 5, True)
+    assert made() == 0
+    for n in (1, 2, 3):
+        for _ in range(8):
+            both(n, 5, True)
+    assert made() == 3
+    for n in range(4, 41):   # 74 other kinds, each of them twice, the first three in between
+        for sample in (True, False):
+            both(n, 5, sample)
+            both(n, 5, sample)
+        both(1 + n % 3, 6, True)
+    assert made() == 3
+    for pos in range(64, 128):   # one, then two tiles of keys: one more kind at most
+        both(2, pos, True)
+    assert made() <= 4
