@@ -83,7 +83,7 @@ DESIGNS = {
                 "attention": {"rot_half": 1, "learned_sink": 0, "maps": 2, "qk_norm": 3},
                 "moe": {"route_top_softmax": 1, "group_best": 1, "expert_act": L.ACT_SILU, "expert_glu": 1, "shared_gate": 0}},
 }
-PINNED_LOGITS = 1 << 18  # floats of a pinned result buffer (8 rows of 32768); a runner has two
+PINNED_LOGITS = 1 << 22  # floats of a pinned result buffer at most; a runner has two, each as large as a decode step's logits
 RGLRU_DECAY_MULT = 8.0  # log a = -8 r softplus(lam)
 
 
@@ -775,7 +775,7 @@ class HybridRunner:
         L.check(self.lib.ssdk_hyb_bind_pools(self.h, self.cache.data_ptr(), num_blocks, self.state.data_ptr(), n_slots,
                                              self.workspace.data_ptr() + off, nb_w), "ssdk_hyb_bind_pools")
         self.step_id = 0
-        rows = min(self.max_logit_rows, max(1, PINNED_LOGITS // spec.vocab))
+        rows = min(max_seqs, self.max_logit_rows, max(1, PINNED_LOGITS // spec.vocab))
         self._pinned = [torch.empty(rows * spec.vocab, dtype=torch.float32, pin_memory=True).numpy() for _ in range(2)]
         self._idle_refs = max(sys.getrefcount(buf) for buf in self._pinned)
 

@@ -83,3 +83,25 @@ def test_kinds_of_steps_keep_their_graphs(monkeypatch):
     for pos in range(64, 128):   # one, then two tiles of keys: one more kind at most
         both(2, pos, True)
     assert made() <= 4
+
+
+def test_held_results_stay_as_they_were():
+    """Results are handed out in buffers that later calls use again: not while a caller still holds an array, a view or a tensor of them."""
+    from ssd_b200 import hybrid_bench as hb
+    from ssd_b200.hybrid import HybridRunner, random_hybrid_weights
+    spec = hb.kokatar_spec(dict(hb.SIZES["s"], layers=1, vocab=512))
+    r = HybridRunner(spec, random_hybrid_weights(spec, torch.bfloat16, "cuda:0", seed=2), max_tokens=64, max_seqs=9, block_size=64, num_blocks=9, n_slots=9, max_model_len=64)
+    assert all(buf.size == 9 * 512 for buf in r._pinned)   # a row per sequence
+    call = lambda k: r.forward([([k + i], 0, i, [i], [0]) for i in range(9)])[0]
+    held, copies = [], []
+    for k, keep in enumerate((lambda a: a, lambda a: a[3:5], lambda a: torch.from_numpy(a), lambda a: a.T, lambda a: memoryview(a), lambda a: a.reshape(-1)[::2])):
+        got = keep(call(20 * k))
+        held.append(got)
+        copies.append(np.asarray(got).copy())
+    for k in range(4):
+        call(300 + k)
+    for a, b in zip(held, copies):
+        assert np.array_equal(np.asarray(a), b)
+    pinned = [buf.ctypes.data for buf in r._pinned]
+    del held, got, a
+    assert call(1).ctypes.data in pinned   # and they come back once nobody holds them
