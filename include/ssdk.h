@@ -185,6 +185,13 @@ int ssdk_prompt_pass(ssdk_handle h, int which, int batch, int q_len,
                      const float* temps, uint64_t seed, uint64_t step_id,
                      int64_t* out_tokens, void* stream);
 
+/* ssdk_prompt_pass whose row b draws the random numbers of row draws[2 b + 1] of the call with step_id draws[2 b]. */
+int ssdk_prompt_pass_draws(ssdk_handle h, int which, int batch, int q_len,
+                           const int64_t* ids, const int32_t* ctx_len,
+                           const int32_t* block_tables, int want_sample,
+                           const float* temps, uint64_t seed, const uint64_t* draws,
+                           int64_t* out_tokens, void* stream);
+
 /* Debug/parity taps: device pointers to the logits of the last spec step
  * (bf16 [batch, K+1, V] and [batch, K, V]) and of the last ssdk_forward_tokens
  * (bf16 [batch, V]).  Valid until the next call. */

@@ -379,6 +379,7 @@ struct Workspace {
   // step state
   uint8_t* out_dev;     // [tok_buf | n_accept | recovery] — one D2H per step
   int64_t* tok_buf;     // [max_batch, K+1]
+  uint64_t* draws;      // [max_batch][2]: SampleParams::draws
   int64_t* ids_in;      // [kMaxTokens]  (forward_tokens input)
   int64_t* out_tok;     // [max_batch]   (forward_tokens sampled output)
   bf16 *logits_q, *logits_p, *logits_last;
@@ -524,6 +525,7 @@ static int64_t carve(ssdk_engine* e, uint8_t* base) {
   w.log_len = (int32_t*)take((size_t)MB * 4);
   w.ids_in = (int64_t*)take(pass * 8);
   w.out_tok = (int64_t*)take(kMaxTokens * 8);
+  w.draws = (uint64_t*)take((size_t)MB * 16);
   w.logits_q = (bf16*)take((size_t)MB * std::max(K, 1) * vmax * 2);
   w.logits_p = (bf16*)take((size_t)MB * (K + 1) * vmax * 2);
   w.logits_last = (bf16*)take((size_t)kMaxTokens * vmax * 2);
@@ -1350,7 +1352,7 @@ int ssdk_create(const ssdk_model_cfg* target, const ssdk_model_cfg* draft, const
     return fail("pinned staging allocation failed");
   }
   memset(e->pin_in, 0, e->step_bytes);
-  e->fw_slot_bytes = align_up(e->step_bytes, 64) + (size_t)kMaxPass * 8;
+  e->fw_slot_bytes = align_up(e->step_bytes, 64) + (size_t)kMaxPass * 8 + (size_t)rt->max_batch * 16;
   if (cudaHostAlloc((void**)&e->pin_fw, e->fw_slot_bytes * ssdk_engine::kFwSlots, cudaHostAllocDefault) != cudaSuccess) {
     cudaFreeHost(e->pin_in);
     cudaFreeHost(e->pin_out);
@@ -1622,7 +1624,7 @@ int ssdk_spec_step_log(ssdk_handle h, int seq, int64_t* out_tokens, int cap, voi
 
 static int forward_rows(ssdk_handle h, int which, int batch, int q_len, const int64_t* ids, const int32_t* ctx_len,
                         const int32_t* block_tables, int want_sample, const float* temps, uint64_t seed,
-                        uint64_t step_id, int64_t* out_tokens, void* stream, int most) {
+                        uint64_t step_id, const uint64_t* draws, int64_t* out_tokens, void* stream, int most) {
   if (!h || !h->finalized) return fail("forward_tokens: engine not finalized");
   if (which < 0 || which > 1 || !h->model[which].present) return fail("forward_tokens: model %d absent", which);
   if (batch < 1 || batch > h->rt.max_batch || q_len < 1 || q_len > most || batch * q_len > most)
@@ -1649,6 +1651,12 @@ static int forward_rows(ssdk_handle h, int which, int batch, int q_len, const in
   int64_t* pin_ids_in = (int64_t*)(pin + align_up(h->step_bytes, 64));
   memcpy(pin_ids_in, ids, (size_t)batch * q_len * 8);
   CK(cudaMemcpyAsync(w.ids_in, pin_ids_in, (size_t)batch * q_len * 8, cudaMemcpyHostToDevice, st));
+  const bool own_draws = draws && want_sample && temps && *std::max_element(temps, temps + batch) > 0.f;
+  if (own_draws) {
+    uint64_t* pin_draws = (uint64_t*)(pin + align_up(h->step_bytes, 64) + (size_t)kMaxPass * 8);
+    for (int b = 0; b < batch; ++b) { pin_draws[2 * b] = draws[2 * b] * 16ull + 14ull; pin_draws[2 * b + 1] = draws[2 * b + 1]; }
+    CK(cudaMemcpyAsync(w.draws, pin_draws, (size_t)batch * 16, cudaMemcpyHostToDevice, st));
+  }
   CK(cudaEventRecord(h->fw_ev[slot], st));
   h->fw_ev_pending[slot] = true;
   // sampled tokens come back through the tail of the result staging buffer (read after the synchronize below)
@@ -1673,7 +1681,7 @@ static int forward_rows(ssdk_handle h, int which, int batch, int q_len, const in
     SampleParams sp;
     sp.logits = w.logits_last; sp.ld = m.cfg.vocab; sp.temps = (const float*)(w.step_dev + h->off_tt);
     sp.V = m.cfg.vocab; sp.seed = seed; sp.call_id = step_id * 16ull + 14ull; sp.out = w.out_tok; sp.out_stride = 1;
-    sp.partial = w.samp_partial; sp.counters = w.samp_counters; sp.dyn = nullptr; sp.sub = 0;
+    sp.partial = w.samp_partial; sp.counters = w.samp_counters; sp.dyn = nullptr; sp.sub = 0; sp.draws = own_draws ? w.draws : nullptr;
     CKI(L.go(sample_kernel, dim3(kSampleChunks, batch), dim3(256), 0, sp));
   }
   if (want_sample) {
@@ -1690,7 +1698,7 @@ static int forward_rows(ssdk_handle h, int which, int batch, int q_len, const in
 int ssdk_forward_tokens(ssdk_handle h, int which, int batch, int q_len, const int64_t* ids, const int32_t* ctx_len,
                         const int32_t* block_tables, int want_sample, const float* temps, uint64_t seed,
                         uint64_t step_id, int64_t* out_tokens, void* stream) {
-  return forward_rows(h, which, batch, q_len, ids, ctx_len, block_tables, want_sample, temps, seed, step_id, out_tokens, stream, kMaxTokens);
+  return forward_rows(h, which, batch, q_len, ids, ctx_len, block_tables, want_sample, temps, seed, step_id, nullptr, out_tokens, stream, kMaxTokens);
 }
 
 int ssdk_prompt_pass_rows(ssdk_handle h, int which) {
@@ -1702,7 +1710,15 @@ int ssdk_prompt_pass(ssdk_handle h, int which, int batch, int q_len, const int64
                      const int32_t* block_tables, int want_sample, const float* temps, uint64_t seed,
                      uint64_t step_id, int64_t* out_tokens, void* stream) {
   const int most = ssdk_prompt_pass_rows(h, which);
-  return forward_rows(h, which, batch, q_len, ids, ctx_len, block_tables, want_sample, temps, seed, step_id, out_tokens, stream, std::max(most, kMaxTokens));
+  return forward_rows(h, which, batch, q_len, ids, ctx_len, block_tables, want_sample, temps, seed, step_id, nullptr, out_tokens, stream, std::max(most, kMaxTokens));
+}
+
+int ssdk_prompt_pass_draws(ssdk_handle h, int which, int batch, int q_len, const int64_t* ids, const int32_t* ctx_len,
+                           const int32_t* block_tables, int want_sample, const float* temps, uint64_t seed,
+                           const uint64_t* draws, int64_t* out_tokens, void* stream) {
+  if (!draws) return fail("prompt_pass_draws: null draws");
+  const int most = ssdk_prompt_pass_rows(h, which);
+  return forward_rows(h, which, batch, q_len, ids, ctx_len, block_tables, want_sample, temps, seed, 0, draws, out_tokens, stream, std::max(most, kMaxTokens));
 }
 
 uint32_t* ssdk_debug_wait_word(ssdk_handle h) { return h ? h->waits.word : nullptr; }

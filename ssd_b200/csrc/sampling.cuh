@@ -54,6 +54,7 @@ struct SampleParams {
   unsigned* counters;  // [B], zero on entry, zero again on exit
   const uint64_t* dyn; // optional device {seed, step}: lets a static CUDA graph draw fresh numbers
   int sub;             // call_id = step * 16 + sub when dyn != nullptr (sub < 0: the step itself)
+  const uint64_t* draws = nullptr;  // optional device [B][2]: call id and row that a row's random numbers are taken for
 };
 
 __global__ void __launch_bounds__(256) sample_kernel(SampleParams p) {
@@ -67,6 +68,11 @@ __global__ void __launch_bounds__(256) sample_kernel(SampleParams p) {
     p.call_id = p.sub < 0 ? p.dyn[1] : p.dyn[1] * 16ull + (uint64_t)p.sub;
   }
   const int b = blockIdx.y, c = blockIdx.x, nch = gridDim.x;
+  uint32_t row_id = (uint32_t)b;
+  if (p.draws) {
+    p.call_id = p.draws[2 * b];
+    row_id = (uint32_t)p.draws[2 * b + 1];
+  }
   const int cs = (((p.V + nch - 1) / nch) + 7) & ~7;
   const int beg = c * cs, end = min(p.V, beg + cs);
   const float T = p.temps[b];
@@ -76,7 +82,7 @@ __global__ void __launch_bounds__(256) sample_kernel(SampleParams p) {
   ArgMax best{-INFINITY, 0x7fffffff};
   for (int i = beg + threadIdx.x * 4; i < end; i += blockDim.x * 4) {
     uint4 rnd = make_uint4(0, 0, 0, 0);
-    if (!greedy) rnd = philox_draw((uint32_t)(i >> 2), (uint32_t)b, p.call_id, TAG_SAMPLE, p.seed);
+    if (!greedy) rnd = philox_draw((uint32_t)(i >> 2), row_id, p.call_id, TAG_SAMPLE, p.seed);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int idx = i + j;

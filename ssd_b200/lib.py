@@ -123,6 +123,8 @@ SIGNATURES: dict[str, tuple] = {
     "ssdk_prompt_pass_rows": (C.c_int, [VP, C.c_int]),
     "ssdk_prompt_pass": (C.c_int, [VP, C.c_int, C.c_int, C.c_int, c_i64p, c_i32p, c_i32p, C.c_int, c_f32p,
                                    C.c_uint64, C.c_uint64, c_i64p, VP]),
+    "ssdk_prompt_pass_draws": (C.c_int, [VP, C.c_int, C.c_int, C.c_int, c_i64p, c_i32p, c_i32p, C.c_int, c_f32p,
+                                         C.c_uint64, C.POINTER(C.c_uint64), c_i64p, VP]),
     "ssdk_logits_p": (VP, [VP]),
     "ssdk_logits_q": (VP, [VP]),
     "ssdk_logits_last": (VP, [VP]),

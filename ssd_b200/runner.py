@@ -65,11 +65,20 @@ def _i32(a):
     return np.ascontiguousarray(a, dtype=np.int32)
 
 
+class _WholePass(int):
+    """The default chunk of a prompt: equal to 256, what a pass carries under tensor parallelism, and told by its type from a
+    caller's own 256, which bounds a pass there."""
+
+
+WHOLE_PASS = _WholePass(256)
+
+
 def _prompt_call(runner, which: int, chunk: int):
-    """(call that runs prompt rows, rows it takes at most): with the default chunk a runner that has longer passes takes those."""
-    most = runner.pass_tokens(which) if chunk == 256 and hasattr(runner, "pass_tokens") else 0
+    """(call that runs prompt rows, rows it takes at most): without a chunk of the caller's, what the engine takes.  (Host tests
+    run the planners on objects without an engine, whose calls take the chunk.)"""
+    most = runner.pass_tokens(which) if isinstance(chunk, _WholePass) and hasattr(runner, "pass_tokens") else 0
     if most <= 256:
-        return runner.forward_tokens, chunk
+        return runner.forward_tokens, int(chunk)
     return partial(runner.forward_tokens, rows=most), most
 
 
@@ -170,9 +179,10 @@ class PairRunner:
         return out
 
     def forward_tokens(self, which: int, ids: list[list[int]], ctx_len: list[int], block_tables, temps=None,
-                       want_sample: bool = True, seed: int = 0, *, rows: int = 256) -> list[int] | None:
+                       want_sample: bool = True, seed: int = 0, *, rows: int = 256, draws=None) -> list[int] | None:
         """ModelRunner.run for q_len tokens per sequence appended at ctx_len (prefill chunk or AR decode).
-        rows: the rows a call may carry; prompts ask for pass_tokens."""
+        rows: the rows a call may carry; prompts ask for pass_tokens.  draws: per sequence, the call number and the row that
+        its random draw is taken for (draw_numbers), if those are not this call's own."""
         if self.spec[which] is None:
             return None  # the draft replica lives on TP rank 0 only (SURVEY §8e); other ranks have nothing to do
         B, Q = len(ids), len(ids[0])
@@ -182,22 +192,28 @@ class PairRunner:
         temps_a = np.ascontiguousarray(temps if temps is not None else [0.0] * B, dtype=np.float32)
         out = np.zeros(B, dtype=np.int64)
         st = torch.cuda.current_stream().cuda_stream
+        args = (self.h, which, B, Q, ids_a.ctypes.data_as(L.c_i64p), ctx_a.ctypes.data_as(L.c_i32p), bt_a.ctypes.data_as(L.c_i32p),
+                int(want_sample), temps_a.ctypes.data_as(L.c_f32p), seed)
+        if draws is not None:
+            draws_a = np.ascontiguousarray(draws, dtype=np.uint64).reshape(-1)
+            L.check(self.lib.ssdk_prompt_pass_draws(*args, draws_a.ctypes.data_as(C.POINTER(C.c_uint64)), out.ctypes.data_as(L.c_i64p), st),
+                    "ssdk_prompt_pass_draws")
+            return out.tolist() if want_sample else None
         call = self.lib.ssdk_forward_tokens
         if rows > 256:
             call = self.lib.ssdk_prompt_pass
             self.step_id += max(0, -(-B * Q // 256) - 1)  # draws are numbered by passes of 256 rows
-        L.check(call(self.h, which, B, Q, ids_a.ctypes.data_as(L.c_i64p), ctx_a.ctypes.data_as(L.c_i32p), bt_a.ctypes.data_as(L.c_i32p),
-                     int(want_sample), temps_a.ctypes.data_as(L.c_f32p), seed, self.step_id, out.ctypes.data_as(L.c_i64p), st),
-                "ssdk_forward_tokens")
+        L.check(call(*args, self.step_id, out.ctypes.data_as(L.c_i64p), st), "ssdk_forward_tokens")
         self.step_id += 1
         return out.tolist() if want_sample else None
 
     def prefill(self, which: int, tokens: list[int], block_table: list[int], start: int = 0, temp: float = 0.0,
-                want_sample: bool = True, chunk: int = 256, seed: int = 0):
+                want_sample: bool = True, chunk: int = WHOLE_PASS, seed: int = 0):
         """Prefill one sequence from position `start` in passes through the multi-query path: the weights are streamed
-        once per pass, attention is the paged multi-query kernel with one q tile per 4-32 query rows
-        (layers/attention.py:85-93 semantics: causal over the cache, which already holds the earlier passes).
-        chunk: tokens of a pass; with the default value a pass carries what the engine takes (pass_tokens)."""
+        once per pass, attention is causal over the cache, which already holds the earlier passes
+        (layers/attention.py:85-93): tcgen05 tiles of 128 rows in passes of more than 256, the paged multi-query kernel with
+        tiles of up to 64 rows in shorter ones.
+        chunk: tokens of a pass at most, up to 256; if not given, a pass carries what the engine takes (pass_tokens)."""
         call, size = _prompt_call(self, which, chunk)
         tok = None
         pos = start
@@ -229,12 +245,28 @@ class PairRunner:
                 best, best_q = order[:nb], q
         return sorted(best), best_q
 
+    @staticmethod
+    def draw_numbers(lens: list[int], max_batch: int) -> tuple[list[tuple[int, int]], int]:
+        """Per prompt, the call and the row of that call that would sample its first token if prompts of these lengths ran in
+        calls of 256 tokens, and the number of those calls: random draws are numbered so whatever a pass carries."""
+        left, at, calls = list(lens), [(0, 0)] * len(lens), 0
+        while True:
+            idx, q = PairRunner.plan_prefill_call(left, 256, max_batch)
+            if not idx:
+                return at, calls
+            for row, i in enumerate(idx):
+                left[i] -= q
+                if left[i] == 0:
+                    at[i] = (calls, row)
+            calls += 1
+
     def prefill_many(self, which: int, tokens: list[list[int]], block_tables: list[list[int]], starts: list[int],
-                     temps: list[float] | None = None, want_sample: bool = True, chunk: int = 256, seed: int = 0):
+                     temps: list[float] | None = None, want_sample: bool = True, chunk: int = WHOLE_PASS, seed: int = 0):
         """Prefill several sequences (runner_helpers.py:123-180 batches them by cu_seqlens): every call carries up to
-        a pass of tokens (`chunk` if that is less than its default) of up to max_batch sequences, the same number of tokens from each (plan_prefill_call), through the
-        multi-query path; a sequence's first token is sampled by the call that holds its last prompt token.  Returns one
-        token per sequence (None without want_sample)."""
+        `chunk` tokens (at most 256; if not given, what the engine takes) of up to max_batch sequences, the same number of
+        tokens from each (plan_prefill_call), through the multi-query path; a sequence's first token is sampled by the call
+        that holds its last prompt token, with the draw that calls of 256 tokens would give it.  Returns one token per
+        sequence (None without want_sample)."""
         n = len(tokens)
         pos = list(starts)
         temps = list(temps) if temps is not None else [0.0] * n
@@ -244,15 +276,20 @@ class PairRunner:
         # attention runs): only sequences that compute their whole prompt share calls; the hits follow one by one, in order.
         packed = [i for i in range(n) if starts[i] == 0]
         call, size = _prompt_call(self, which, min(chunk, 256))
+        numbers = None
+        if size > 256:
+            numbers, calls = self.draw_numbers([len(tokens[i]) if i in packed else 0 for i in range(n)], self.max_batch)
+            first, self.step_id = self.step_id, self.step_id + calls
         while True:
             idx, q = self.plan_prefill_call([len(tokens[i]) - pos[i] if i in packed else 0 for i in range(n)],
                                             size, self.max_batch)
             if not idx:
                 break
             done = [pos[i] + q == len(tokens[i]) for i in idx]
+            more = {} if numbers is None else {"draws": [(first + numbers[i][0], numbers[i][1]) for i in idx]}
             toks = call(which, [tokens[i][pos[i]:pos[i] + q] for i in idx], [pos[i] for i in idx],
                         [block_tables[i] for i in idx], [temps[i] for i in idx],
-                        want_sample=(want_sample and any(done)), seed=seed)
+                        want_sample=(want_sample and any(done)), seed=seed, **more)
             for j, i in enumerate(idx):
                 pos[i] += q
                 if done[j] and toks is not None:

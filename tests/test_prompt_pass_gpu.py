@@ -74,3 +74,17 @@ def test_row_forms(hidden, hd, qk_norm):
     assert ((la - lb).norm() / la.norm()).item() < TOL
     ka, kb = (r.kv[L.TARGET][:, 0, s:s + 10].flatten(1, 2)[:, :301].float() for s in (0, 10))
     assert ((ka - kb).norm() / ka.norm()).item() < TOL
+
+
+def test_sampled_prompts_draw_as_in_short_passes():
+    """Flat logits under a high temperature: a token is decided by its random numbers, so that equal tokens mean equal draws."""
+    from ssd_b200 import lib as L
+    g = torch.Generator().manual_seed(5)
+    prompts = [torch.randint(0, 1024, (n,), generator=g).tolist() for n in (700, 300, 300, 411, 90)]
+    pages = [list(range(12 * i, 12 * (i + 1))) for i in range(5)]
+    got = []
+    for kw in ({"chunk": 256}, {}):
+        r = _runner(batch=5)
+        first = r.prefill_many(L.TARGET, prompts, pages, [0] * 5, [50.0, 0.0, 50.0, 50.0, 50.0], seed=9, **kw)
+        got.append((first, r.forward_tokens(L.TARGET, [[t] for t in first], [len(p) for p in prompts], pages, [50.0] * 5, seed=9), r.step_id))
+    assert got[0] == got[1]
