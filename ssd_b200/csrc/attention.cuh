@@ -6,12 +6,11 @@
 //   <= context_len - q_len + j), K/V read back from the paged cache (attention.py:82-83).
 //
 // Work decomposition (at b=1 the problem is tiny and latency-bound, so the aim is to spread a few hundred KB of KV over as many
-// SMs as possible; long contexts are bound by issue slots and by the bytes in flight, so the aim is equal shares in one wave):
-//   grid = (kv_heads, ranges, n_qtiles), 128 or 256 threads.
+// SMs as possible; long contexts are bound by issue slots and by the bytes in flight):
+//   grid = (kv_heads, batch * n_split, n_qtiles), 128 or 256 threads.
 //   A CTA owns one kv head, up to TQ query tokens x G=H/KV query heads (R = G*tq <= 64 rows,
-//   padded to MT 16-row MMA tiles) and a range of 64-token KV chunks of one sequence.
-//   Ranges: the chunks of ALL sequences are cut into pieces of one length, chosen so that about two CTAs per SM get one
-//   (AttnRanges); a fixed number of splits per sequence left the longest of eight ragged 70B contexts running alone.
+//   padded to MT 16-row MMA tiles) and one of n_split ranges of the 64-token KV chunks of one sequence.  How a sequence is cut follows from
+//   its own length and the shape of the call, so that its result does not depend on what it is batched with.
 //   K/V chunks are staged in shared memory with 16-byte cp.async (coalesced 256 B rows of a
 //   page), two or three deep; QK^T and PV run on mma.sync m16n8k16 (bf16, fp32 accumulate)
 //   with ldmatrix fragments; softmax is online in fp32 (exp2 domain), the sums are rescaled only where a maximum moved.
@@ -19,7 +18,7 @@
 //   split-KV partials through a global fp32 scratch + attn_combine_kernel.
 //   Two to three CTAs per SM: registers are capped and the kernels ask for the large shared-memory carve-out.  With 156 registers
 //   and the default carve-out one CTA of eight warps was resident and the SMs issued 43 % of the time.
-// The grid is static (CUDA-graph friendly): each CTA derives its range from context_lens[] at run time.
+// The grid is static (CUDA-graph friendly): each CTA derives its chunk range from context_lens[] at run time.
 #pragma once
 #include "common.cuh"
 
@@ -42,9 +41,7 @@ struct AttnParams {
   float* part_o;                 // [B*Q*H, n_split, hd]
   float* part_lse;               // [B*Q*H, n_split]
   int B, Q, H, KV, block_size, max_blocks, TQ, n_qtiles;
-  int n_split;                   // most ranges of one sequence (stride of the partials); 1: every sequence is one range, no partials
-  int target;                    // ranges aimed at over all sequences (per kv head and q tile); the grid has target + B.  0: n_split
-                                 // ranges per sequence, whatever the others' lengths; the grid has n_split B
+  int n_split;                   // ranges of one sequence; 1: no partials
   int g_shift;                   // log2(H / KV) when the GQA ratio is a power of two, else -1
   float scale_log2;              // softmax scale * log2(e)
 };
@@ -81,55 +78,6 @@ SSDK_DEVINL uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// How the batch's chunks are cut: pieces of `cps` chunks, item i = piece `split` of sequence `b` (b < 0: no such item).  Each warp works
-// it out by itself: one load per 32 sequences and a prefix sum.  `seq`: only the piece length of that sequence is asked for.
-struct AttnRanges { int cps, b, split; };
-SSDK_DEVINL AttnRanges attn_ranges(const AttnParams& p, int item, int seq = -1) {
-  AttnRanges r;
-  if (p.n_split == 1) { r.cps = 0x3fffffff; r.b = item < p.B ? item : -1; r.split = 0; return r; }
-  if (p.target == 0) {   // every sequence by itself: n_split ranges
-    const int b = seq >= 0 ? seq : item / p.n_split, n = (p.context_lens[b] + kAttChunk - 1) / kAttChunk;
-    r.cps = max(1, (n + p.n_split - 1) / p.n_split);
-    r.b = b; r.split = item - b * p.n_split;
-    return r;
-  }
-  const int lane = threadIdx.x & 31;
-  int total = 0, most = 0;
-  for (int b0 = 0; b0 < p.B; b0 += 32) {
-    const int n = b0 + lane < p.B ? (p.context_lens[b0 + lane] + kAttChunk - 1) / kAttChunk : 0;
-    total += n;
-    most = max(most, n);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    total += __shfl_xor_sync(0xffffffffu, total, o);
-    most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-  }
-  r.cps = max(1, max((total + p.target - 1) / p.target, (most + p.n_split - 1) / p.n_split));
-  r.b = -1; r.split = 0;
-  int before = 0;
-  for (int b0 = 0; b0 < p.B && item >= 0; b0 += 32) {
-    const int n = b0 + lane < p.B ? (p.context_lens[b0 + lane] + kAttChunk - 1) / kAttChunk : 0;
-    const int mine = (n + r.cps - 1) / r.cps;
-    int upto = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, upto, o);
-      if (lane >= o) upto += v;
-    }
-    const int rel = item - before;
-    const unsigned hit = __ballot_sync(0xffffffffu, rel >= 0 && rel < upto && rel >= upto - mine);
-    if (hit) {
-      const int src = __ffs(hit) - 1;
-      r.b = b0 + src;
-      r.split = rel - __shfl_sync(0xffffffffu, upto - mine, src);
-      break;
-    }
-    before += __shfl_sync(0xffffffffu, upto, 31);
-  }
-  return r;
-}
-
 // OCC: CTAs that are to fit an SM
 template <int HD, int MT, int OCC>
 __global__ void __launch_bounds__(attn_warps(MT) * 32, OCC) paged_attn_kernel(AttnParams p) {
@@ -152,9 +100,7 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32, OCC) paged_attn_kernel(At
   pdl_wait();
   if (threadIdx.x == 0) trace_mark(TR_ATTN);
 
-  const AttnRanges rgs = attn_ranges(p, blockIdx.y);
-  if (rgs.b < 0) return;
-  const int kvh = blockIdx.x, split = rgs.split, b = rgs.b, qt = p.n_qtiles - 1 - (int)blockIdx.z;   // (the tiles that see most keys first)
+  const int kvh = blockIdx.x, b = blockIdx.y / p.n_split, split = blockIdx.y - b * p.n_split, qt = p.n_qtiles - 1 - (int)blockIdx.z;   // (the tiles that see most keys first)
   const int G = p.H / p.KV;
   const int tq = min(p.TQ, p.Q - qt * p.TQ);
   const int R = G * tq;
@@ -162,10 +108,10 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32, OCC) paged_attn_kernel(At
   const int ctx0 = ctx - p.Q;                         // tokens before this forward
   const int kv_max = ctx0 + qt * p.TQ + tq;           // exclusive upper bound of visible kv for this q-tile
   const int nch_total = (kv_max + kAttChunk - 1) / kAttChunk;
-  const int ch_begin = split * rgs.cps;
-  const int ch_end = min(nch_total, ch_begin + min(rgs.cps, nch_total));
-  // a q tile ends before its sequence does: ranges behind it own no partial (attn_combine_kernel reads the first
-  // ceil(nch_total / cps) ranges only)
+  const int cps = (nch_total + p.n_split - 1) / p.n_split;
+  const int ch_begin = split * cps;
+  const int ch_end = min(nch_total, ch_begin + cps);
+  // ranges without chunks own no partial: attn_combine_kernel only reads the first ceil(nch_total / cps)
   if (p.n_split > 1 && ch_begin >= ch_end) return;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -420,7 +366,7 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32, OCC) paged_attn_kernel(At
 
 // merge split-KV partials: out = sum_s 2^(lse_s - max) o_s / sum_s 2^(lse_s - max).
 // One CTA per (token, head) row, HD/4 threads, each owning one float4 of the output.  Only the splits that had
-// chunks (n_active, recomputed from context_lens as the attention kernel does) are read, and every thread
+// chunks (n_active, recomputed from context_lens with the attention kernel's formula) are read, and every thread
 // issues all of its loads before using them, so the merge costs ~2 L2 round trips whatever n_split is.
 __global__ void attn_combine_kernel(AttnParams p, int hd) {
   __shared__ float sw[32];
@@ -434,8 +380,8 @@ __global__ void attn_combine_kernel(AttnParams p, int hd) {
   const int tq = min(p.TQ, p.Q - qt * p.TQ);
   const int kv_max = p.context_lens[b] - p.Q + qt * p.TQ + tq;
   const int nch_total = (kv_max + kAttChunk - 1) / kAttChunk;
-  const int cps = attn_ranges(p, -1, b).cps;
-  const int n_active = min(p.n_split, (nch_total + cps - 1) / cps);
+  const int cps = (nch_total + p.n_split - 1) / p.n_split;
+  const int n_active = (cps > 0) ? min(p.n_split, (nch_total + cps - 1) / cps) : 0;
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     const float lse = (lane < n_active) ? __ldcg(p.part_lse + row * p.n_split + lane) : -INFINITY;

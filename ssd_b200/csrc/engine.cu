@@ -559,7 +559,7 @@ struct Fwd {
   int64_t logits_ld;
 };
 
-static int attn_plan(const Model& m, int B, int Q, int* TQ, int* MT, int* nqt, int* nsplit, int* target, int max_ctx) {
+static int attn_plan(const Model& m, int B, int Q, int* TQ, int* MT, int* nqt, int* nsplit, int max_ctx) {
   const int G = m.H / m.KV;
   if (G < 1 || G > 16 || (m.H % m.KV) != 0) return fail("unsupported GQA ratio %d", G);
   // q tile of <= 32 rows (two 16-row MMA tiles, 8 warps = 4 token slices each): measured 7.3 us per 70B verify layer
@@ -572,16 +572,14 @@ static int attn_plan(const Model& m, int B, int Q, int* TQ, int* MT, int* nqt, i
   *TQ = tq;
   *MT = mt;
   *nqt = (Q + tq - 1) / tq;
-  // a sequence is cut into at most kAttnMaxSplit ranges (one batch of loads per range in the merge)
+  // (at most kAttnMaxSplit ranges: one batch of loads each in the merge)
   const int max_chunks = std::max(1, (max_ctx + kAttChunk - 1) / kAttChunk);
-  const int per = m.KV * (*nqt);
-  if (mt > 1 && B > 1) {   // equal ranges over the batch, two CTAs per SM
-    *target = std::max(1, std::min(2 * num_sms() / per, B * max_chunks));
-    *nsplit = *target <= B / 2 ? 1 : std::min({*target, kAttnMaxSplit, max_chunks});
-  } else {                 // single-row decode gains less from equal ranges than working them out costs (16 x 4000: 799 us a step, 823 with)
-    *target = 0;
-    *nsplit = std::max(1, std::min({(mt == 1 ? 3 : 2) * num_sms() / (per * B), kAttnMaxSplit, max_chunks}));
-  }
+  const int ctas = m.KV * B * (*nqt);
+  // ranges per sequence: enough for two CTAs per SM (one row per head: three are resident, and one range less than would fill them).
+  // 8 x 7 rows of a 70B layer, contexts of 4500 to 8000: 110 us, 121 with a range less; with the chunks of all sequences cut into equal pieces,
+  // which every CTA had to work out from all contexts, 124, and a sequence's bits then followed from its neighbours' lengths.
+  const int ns = mt == 1 ? 3 * num_sms() / ctas : (2 * num_sms() + ctas - 1) / ctas;
+  *nsplit = std::max(1, std::min({ns, kAttnMaxSplit, max_chunks}));
   return 0;
 }
 
@@ -596,7 +594,7 @@ static int launch_attn_inst(Launcher& L, const AttnParams& p, dim3 grid) {
   }
   return L.go(paged_attn_kernel<HD, MT, OCC>, grid, dim3(attn_warps(MT) * 32), smem, p);
 }
-// More CTAs than SMs: two per SM (registers capped at 128).  8 x 8000 x 7 rows of a 70B layer 143 -> 123 us, 2003-token prompt of 4 8B
+// More CTAs than SMs: two per SM (registers capped at 128).  8 x 8000 x 7 rows of a 70B layer 143 -> 110 us, 2003-token prompt of 4 8B
 // layers 4862 -> 4731 us; a 200-token context that one CTA per SM covers takes 1.2 us less with the registers.
 template <int HD, int MT>
 static int launch_attn_occ(Launcher& L, const AttnParams& p, dim3 grid) {
@@ -617,18 +615,18 @@ static int enqueue_attention(Launcher& L, const bf16* q, const bf16* kc, const b
                              const int32_t* ctx_lens, bf16* out, float* part_o, float* part_lse, unsigned* counters,
                              int B, int Q, int H,
                              int KV, int hd, int block_size, int max_blocks, float scale, int TQ, int MT, int nqt,
-                             int nsplit, int target) {
+                             int nsplit) {
   AttnParams a;
   a.q = q; a.k_cache = kc; a.v_cache = vc; a.block_tables = bt; a.context_lens = ctx_lens; a.out = out;
   a.part_o = part_o; a.part_lse = part_lse;
   (void)counters;
   a.B = B; a.Q = Q; a.H = H; a.KV = KV; a.block_size = block_size; a.max_blocks = max_blocks;
-  a.n_split = nsplit; a.target = target; a.TQ = TQ; a.n_qtiles = nqt;
+  a.n_split = nsplit; a.TQ = TQ; a.n_qtiles = nqt;
   a.g_shift = -1;
   for (int sft = 0; sft < 5; ++sft)
     if ((H / KV) == (1 << sft)) a.g_shift = sft;
   a.scale_log2 = scale * 1.4426950408889634f;
-  CKI(launch_attn(L, a, hd, MT, dim3(KV, nsplit == 1 ? B : (target ? target + B : nsplit * B), nqt)));
+  CKI(launch_attn(L, a, hd, MT, dim3(KV, nsplit * B, nqt)));
   if (nsplit > 1) CKI(L.go(attn_combine_kernel, dim3(B * Q * H), dim3(32), 0, a, hd));
   return 0;
 }
@@ -834,8 +832,8 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
            w.positions, w.slot_mapping, w.context_lens,
            (f.which == SSDK_TARGET && tp > 1 && e->symm_n == tp) ? w.ar_state : (unsigned*)nullptr));
 
-  int TQ = 1, MT = 1, nqt = 1, nsplit = 1, target = 1;
-  CKI(attn_plan(m, f.B, f.Q, &TQ, &MT, &nqt, &nsplit, &target, e->max_ctx_hint));
+  int TQ = 1, MT = 1, nqt = 1, nsplit = 1;
+  CKI(attn_plan(m, f.B, f.Q, &TQ, &MT, &nqt, &nsplit, e->max_ctx_hint));
   if (M > kMaxTokens) nsplit = 1;   // (the partials are sized for kMaxTokens rows; so many q tiles fill the SMs by themselves)
   const float scale = 1.0f / sqrtf((float)m.hd);
 
@@ -899,7 +897,7 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
       CKI(forward_prompt_attention(e, L, m, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, f.B, f.Q, bs, mb, scale));
     else
       CKI(enqueue_attention(L, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, w.att_o,
-                          w.att_lse, w.att_counters, f.B, f.Q, m.H, m.KV, m.hd, bs, mb, scale, TQ, MT, nqt, nsplit, target));
+                          w.att_lse, w.att_counters, f.B, f.Q, m.H, m.KV, m.hd, bs, mb, scale, TQ, MT, nqt, nsplit));
 
     // ---- output projection (row-parallel) ----
     const bool fuse_pub = use_symm && fused_publish_enabled() && M <= 64;
@@ -1823,11 +1821,11 @@ int ssdk_silu_mul(const void* gate_up, void* out, int M, int ffn, void* stream) 
   return L.go(silu_mul_kernel, dim3((M * ffn / 8 + 255) / 256), dim3(256), 0, g, (bf16*)out, M, ffn);
 }
 
-static int attn_plan_raw(int H, int KV, int B, int Q, int max_ctx, int* TQ, int* MT, int* nqt, int* nsplit, int* target) {
+static int attn_plan_raw(int H, int KV, int B, int Q, int max_ctx, int* TQ, int* MT, int* nqt, int* nsplit) {
   Model tmp;
   tmp.H = H;
   tmp.KV = KV;
-  return attn_plan(tmp, B, Q, TQ, MT, nqt, nsplit, target, max_ctx);
+  return attn_plan(tmp, B, Q, TQ, MT, nqt, nsplit, max_ctx);
 }
 
 int64_t ssdk_paged_attn_scratch_bytes(int batch, int q_len, int heads, int head_dim, int max_ctx) {
@@ -1842,13 +1840,13 @@ int ssdk_paged_attn(const void* q, const void* k_cache, const void* v_cache, con
   Launcher L;
   L.st = (cudaStream_t)stream;
   CKI(init_kernel_attrs());
-  int TQ, MT, nqt, nsplit, target;
-  CKI(attn_plan_raw(heads, kv_heads, batch, q_len, block_size * max_blocks_per_seq, &TQ, &MT, &nqt, &nsplit, &target));
+  int TQ, MT, nqt, nsplit;
+  CKI(attn_plan_raw(heads, kv_heads, batch, q_len, block_size * max_blocks_per_seq, &TQ, &MT, &nqt, &nsplit));
   float* part_o = (float*)((uint8_t*)scratch + 16384);
   float* part_lse = part_o + (size_t)batch * q_len * heads * kAttnMaxSplit * head_dim;
   return enqueue_attention(L, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, block_tables, context_lens,
                            (bf16*)out, part_o, part_lse, (unsigned*)scratch, batch, q_len, heads, kv_heads, head_dim, block_size,
-                           max_blocks_per_seq, scale, TQ, MT, nqt, nsplit, target);
+                           max_blocks_per_seq, scale, TQ, MT, nqt, nsplit);
 }
 
 int ssdk_prompt_attn(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,

@@ -230,3 +230,17 @@ def test_verify_full_vocab_sizes(dev):
         t = torch.full((1,), 0.8, device=dev)
         n, rec = ops.verify(lp.to(dev), lp[:, :K].contiguous().to(dev), spec.to(dev), t, t, None, True, 1, 2)
         assert int(n) == K and 0 <= int(rec) < V_
+
+
+@pytest.mark.parametrize("rows", [1, 3, 7])
+def test_attention_of_a_sequence_does_not_follow_from_its_neighbours(dev, rows):
+    """The same sequence in batches whose other contexts are short, long or ragged: the same bits."""
+    from ssd_b200 import ops
+    H, KV, hd, bs, pages = 32, 4, 128, 64, 64
+    g = torch.Generator(device="cuda").manual_seed(3)
+    kc, vc = (torch.randn(4 * pages, bs, KV, hd, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(4 * rows, H, hd, generator=g, device="cuda").to(torch.bfloat16)
+    tables = torch.arange(4 * pages, dtype=torch.int32, device="cuda").view(4, pages)
+    out = [ops.paged_attention(q, kc, vc, tables, torch.tensor([lens[0], 1700, *lens[1:]], dtype=torch.int32, device="cuda"), rows, hd ** -0.5).view(4, rows, -1)[1]
+           for lens in ([rows, rows, rows], [4096, 4096, 4096], [100, 4000, 901])]
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
