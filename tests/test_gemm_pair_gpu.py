@@ -38,3 +38,23 @@ def test_same_as_one_cta_form(monkeypatch, kind):
         assert np.isfinite(b).all()
         err = np.sqrt(((a - b) ** 2).mean(-1) / (a ** 2).mean(-1))
         assert err.max() < TOL, f"{kind}, {n} rows: row {err.argmax()} off by {err.max():.2e}"
+
+
+def test_many_tiles_per_pair(monkeypatch):
+    """1999 rows through a gated feed-forward of 6000 columns and a head of 8000: five and four tiles per pair of CTAs on 148 SMs, so that
+    the load ring and both accumulators run on from tile to tile, with remainders in rows and columns."""
+    from ssd_b200 import hybrid_bench as hb
+    from ssd_b200.hybrid import HybridRunner, random_hybrid_weights
+    spec = hb.kefurax_spec(dict(hb.SIZES["s"], layers=1, vocab=8000, sff=6000 - 2 * 512), ("rglru",))
+    assert spec.layers[0].ff == 6000
+    w = random_hybrid_weights(spec, torch.bfloat16, "cuda:0", seed=5)
+    toks = torch.randint(0, spec.vocab, (1999,), generator=torch.Generator().manual_seed(5)).tolist()
+    out = []
+    for mode in ("0", "2"):
+        monkeypatch.setenv("SSDK_HYB_PAIR", mode)
+        r = HybridRunner(spec, w, max_tokens=2000, max_seqs=1, block_size=64, num_blocks=32, n_slots=1, max_model_len=2048)
+        out.append(r.forward([(toks, 0, 0, list(range(32)), list(range(1999)))])[0].copy())
+        r.close()
+    a, b = out
+    err = np.sqrt(((a - b) ** 2).mean(-1) / (a ** 2).mean(-1))
+    assert np.isfinite(b).all() and err.max() < TOL, f"row {err.argmax()} off by {err.max():.2e}"

@@ -97,3 +97,44 @@ def test_infinite_largest_and_tiny_operands(tmp_path, monkeypatch):
         x, y = a[ok, col], b[ok, col]
         size = np.abs(x).max()   # (the squares of 1e-36 are not numbers)
         assert ok.any() and np.linalg.norm((x - y) / size) < TOL * np.linalg.norm(x / size), col
+
+
+def test_many_tiles_per_pair(tmp_path, monkeypatch):
+    """1000 rows through a head of 8000 columns and k = 328: 256 tiles, three and four per pair of CTAs on 148 SMs, so that rings and
+    accumulators run on from tile to tile; against the float64 oracle."""
+    from ssd_b200.hybrid import HybridRunner, HybridSpec, load_hybrid_weights
+    U = importlib.import_module("tests.kefurax_util")
+    cfg = U.config([U.rglru(width=48, blocks=2)], width=328, vocab=8000)
+    tensors = U.random_tensors(cfg, 6)
+    path = U.write_checkpoint(str(tmp_path / "ckpt"), cfg, tensors)
+    spec = HybridSpec.from_dir(path)
+    w = load_hybrid_weights(path, spec, torch.float32, "cuda:0")
+    toks = torch.randint(0, cfg["vocab"], (1000,), generator=torch.Generator().manual_seed(2)).tolist()
+    want = U.PlainModel(cfg, tensors).run(toks).numpy()
+    errs = {}
+    for mode in ("0", "2"):
+        monkeypatch.setenv("SSDK_HYB_SPLIT", mode)
+        r = HybridRunner(spec, w, dtype="float32", max_tokens=1000, max_seqs=1, block_size=16, num_blocks=64, n_slots=1, max_model_len=1024)
+        got = r.forward([(toks, 0, 0, list(range(63)), list(range(1000)))])[0]
+        errs[mode] = np.sqrt(((got - want) ** 2).mean(-1) / (want ** 2).mean(-1)).max()   # the worst row
+        r.close()
+    assert errs["2"] < TOL and errs["2"] < max(1e-6, 1.5 * errs["0"]), errs
+
+
+def test_many_expert_tiles(tmp_path, monkeypatch):
+    """40 experts of 520 columns over 1000 rows: 200 grouped tiles of 5 to 100 rows, against the FMA form (its error is 1e-6)."""
+    from ssd_b200.hybrid import HybridRunner, HybridSpec, load_hybrid_weights
+    U = importlib.import_module("tests.vegilix_util")
+    cfg = U.config([U.retention(heads=2, dim=16, vdim=8, dims=8, mlp=U.moe(experts=40, top=2, ff=520, shared_ff=16))], width=600, vocab=64)
+    path = U.write_checkpoint(str(tmp_path / "ckpt"), cfg, U.random_tensors(cfg, 1))
+    spec = HybridSpec.from_dir(path)
+    w = load_hybrid_weights(path, spec, torch.float32, "cuda:0")
+    toks = torch.randint(0, cfg["vocab"], (1000,), generator=torch.Generator().manual_seed(2)).tolist()
+    out = []
+    for mode in ("0", "2"):
+        monkeypatch.setenv("SSDK_HYB_SPLIT", mode)
+        r = HybridRunner(spec, w, dtype="float32", max_tokens=1000, max_seqs=1, block_size=16, num_blocks=64, n_slots=1, max_model_len=1024)
+        out.append(r.forward([(toks, 0, 0, list(range(63)), list(range(1000)))])[0].copy())
+        r.close()
+    err = np.sqrt(((out[0] - out[1]) ** 2).mean(-1) / (out[0] ** 2).mean(-1))
+    assert np.isfinite(out[1]).all() and err.max() < TOL, f"row {err.argmax()} off by {err.max():.2e}"

@@ -88,3 +88,22 @@ def test_sampled_prompts_draw_as_in_short_passes():
         first = r.prefill_many(L.TARGET, prompts, pages, [0] * 5, [50.0, 0.0, 50.0, 50.0, 50.0], seed=9, **kw)
         got.append((first, r.forward_tokens(L.TARGET, [[t] for t in first], [len(p) for p in prompts], pages, [50.0] * 5, seed=9), r.step_id))
     assert got[0] == got[1]
+
+
+def test_many_tiles_per_pair():
+    """Projections of 6144 columns and a gated feed-forward of 6016 over 2003 rows: up to three and six tiles per pair of CTAs on 148 SMs."""
+    from ssd_b200 import lib as L, synth
+    from ssd_b200.runner import ModelSpec, PairRunner
+    spec = ModelSpec(hidden=2048, layers=1, heads=64, kv_heads=16, head_dim=64, ffn=6016, vocab=1024, rms_eps=1e-5)
+    r = PairRunner(spec, None, spec_k=0, max_batch=2, block_size=64, max_model_len=2048, use_graph=False, use_pdl=True)
+    w = synth.generate_weights(spec, {"seed": 4, "alpha": 0.9, "role": "target", "o_down_std": 0.05}, torch.device("cuda:0"))
+    r.bind_weights(L.TARGET, w)
+    r.finalize()
+    toks = torch.randint(0, 1024, (2003,), generator=torch.Generator().manual_seed(8)).tolist()
+    r.prefill(L.TARGET, toks, list(range(32)), chunk=64)
+    la = r.logits_last(1).float().clone()
+    r.prefill(L.TARGET, toks, list(range(32, 64)))
+    lb = r.logits_last(1).float()
+    assert ((la - lb).norm() / la.norm()).item() < TOL
+    ka, kb = (r.kv[L.TARGET][:, 0, s:s + 32].flatten(1, 2)[:, :2003].float() for s in (0, 32))
+    assert ((ka - kb).norm(dim=(-1, -2)) / ka.norm(dim=(-1, -2))).max().item() < TOL   # every row's keys and values
