@@ -494,7 +494,7 @@ static int64_t carve(ssdk_engine* e, uint8_t* base) {
     part = std::max(part, need(m.d, m.H * m.hd));
     part = std::max(part, need(2 * m.ffn, m.d));
     part = std::max(part, need(m.d, m.ffn));
-    if (pass_rows(m) > kMaxTokens) part = std::max(part, (size_t)pass_rows(m) * std::max(m.qkv_dim, m.d));   // one slab
+    if (pass_rows(m) > kMaxTokens) part = std::max(part, (size_t)pass_rows(m) * std::max(m.qkv_dim, m.d) / 2);   // one result in bf16
     pass = std::max<size_t>(pass, pass_rows(m));
   }
   Workspace scratch_ws;
@@ -678,7 +678,7 @@ static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w
   if (K % kBlockK) return fail("GEMM K=%d not a multiple of 64", K);
   if (M > kMaxTokens) {   // prompt passes: summed over all of K and rounded to bf16, which their consumers do with slabs (splits 0: dense)
     if (epi != EPI_PARTIAL && (epi != EPI_SILU || N_out % kPairGluRun)) return fail("GEMM of %d rows: unsupported form", M);
-    if (epi == EPI_PARTIAL && (size_t)M * N_out > e->ws.partial_floats) return fail("partial buffer too small");
+    if (epi == EPI_PARTIAL && (size_t)M * N_out > 2 * e->ws.partial_floats) return fail("partial buffer too small");
     const CUtensorMap *tmW, *tmX, *tmXs;
     if (epi == EPI_SILU) CKI(e->xmaps.get_glu(w.ptr, N_out, K, &tmW));
     else CKI(e->xmaps.get(w.ptr, K, 128, &tmW, (int)w.rows));
