@@ -6,9 +6,9 @@ API — `ssd.LLM(...)`, `add_request`, `create_inference_step`, `step` — on th
 its CUDA-graph capture / replay (`capture_cudagraph`, `run_decode_cudagraph`, `run_verify_cudagraph`), its `Sampler`,
 `verify()`, `Scheduler` and `BlockManager`.  None of ssd_b200's kernels or engine code is on this path.
 
-What has to be supplied from outside, because the image is not the reference's pinned environment (SURVEY §7/§8c):
+What has to be supplied from outside, because the image is not the reference's pinned environment:
   1. `sgl_kernel.flash_attn` (FA3 wheel, absent, Hopper-only): two functions backed by flash_attn 2.8.3, which ships
-     sm_100 SASS — the stub BASELINE.md §4.2 prescribes;
+     sm_100 kernels;
   2. checkpoints: none exist in the image, so `ssd.engine.model_runner.load_model` is replaced by a filler that writes
      ssd_b200.synth's seeded synthetic weights (the same tensors our engine runs on) into the reference's own
      nn.Parameters, and `AutoTokenizer.from_pretrained` returns the synthetic "<id>" tokenizer for synthetic dirs;

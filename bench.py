@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""bench.py — decode tokens/s of the sync speculative-decoding hot path (BASELINE.json metric).
+"""bench.py — decode tokens/s of the sync speculative-decoding hot path.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference|reference-gpu]
                     [--workload 70b|8b|qwen32b|tiny] [--temp T] [--lm-scale S]
@@ -13,7 +13,7 @@ temp 0, synthetic "bigram agreement" weights at the exact shapes (there are no c
   e2e       the same metric through the public engine API (LLMEngine.step: scheduler + ssdk_spec_step with HOST
             buffers: per-step H2D of ctx/recovery/block tables and D2H of tokens/accept count inside the timing)
   roofline  achieved HBM GB/s of the dominant kernel (weight-streaming tcgen05 GEMM, largest instance) vs the
-            measured peak, plus the whole-step fraction of the HBM roofline of SURVEY §8(d)
+            measured peak, plus the whole-step fraction of the HBM roofline (bytes_per_step)
   cpu_baseline  the oracle (CPU restatement of the reference path) timed on the host cores on a bounded sample
   parity_check  temp 0: the tokens of the timed device-resident loop AND of the engine (e2e) loop against the closed-form
             greedy chain of the synthetic target (t_{i+1} = pi_t(t_i)) — token-for-token, at every N
@@ -43,7 +43,7 @@ WORKLOADS = {
     "qwen32b": ("qwen3-32b", "qwen3-0.6b", "Qwen3-32B target + Qwen3-0.6B draft"),
     "tiny": ("llama-tiny-target", "llama-tiny-draft", "tiny Llama pair (plumbing)"),
 }
-# forward weight bytes (bf16, body + lm_head) and KV bytes/token: SURVEY §2 / BASELINE.md §3
+# forward weight bytes (bf16, body + lm_head) and KV bytes/token
 W_BYTES = {"llama-3.2-1b": 2.472e9, "llama-3.1-8b": 15.010e9, "llama-3.1-70b": 139.006e9, "qwen3-0.6b": 1.192e9,
            "qwen3-32b": 63.968e9}
 KV_BYTES = {"llama-3.2-1b": 32768, "llama-3.1-8b": 131072, "llama-3.1-70b": 327680, "qwen3-0.6b": 114688,
@@ -136,7 +136,7 @@ def run_reference_gpu_subprocess(args, timeout_s: int = 480):
 
 
 def bytes_per_step(tshape, dshape, K, ctx, tp):
-    """(K+1)(W_draft + ctx*kv_d) + (W_target + ctx*kv_t)/TP + (2K+1)*V*2."""
+    """Bytes that a step cannot do without: (K+1)(W_draft + ctx*kv_d) + (W_target + ctx*kv_t)/TP + (2K+1)*V*2."""
     V = 151936 if "qwen" in tshape else 128256
     if tshape not in W_BYTES:
         return None
@@ -324,7 +324,7 @@ def run_ours(args):
 
 def gemm_roofline(runner, peak):
     """Dominant kernel = gemm_ws_kernel; its largest instance is the target's gate|up projection at M=K+1.
-    achieved = algorithmic bytes (weight bytes of that matrix, SURVEY §8d: out*in*2) / CUDA-event time."""
+    achieved = algorithmic bytes (weight bytes of that matrix: out*in*2) / CUDA-event time."""
     import torch
     from ssd_b200 import lib as L, ops
     w = runner.weights[L.TARGET]["layers"][0]["gate_up"]
@@ -454,7 +454,7 @@ def main():
     ap.add_argument("--steps", type=int, default=48)
     ap.add_argument("--warmup", type=int, default=6)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference", "reference-gpu"])
-    ap.add_argument("--temp", type=float, default=0.0, help="sampling temperature of target and draft (BASELINE config 4: 0.7)")
+    ap.add_argument("--temp", type=float, default=0.0, help="sampling temperature of target and draft (0.7: the sampled configuration)")
     ap.add_argument("--lm-scale", type=float, default=None, help="synthetic lm_head scale (softens the distribution for temp>0)")
     ap.add_argument("--no-ref-gpu", action="store_true", help="skip the reference GPU arm inside the default line")
     ap.add_argument("--workload", default="70b", choices=sorted(WORKLOADS))

@@ -5,7 +5,7 @@ Runs only in the build container (the reference does not travel to the GPU box).
     CXX=/usr/bin/g++ python oracle/gen_golden.py            # compiled (Inductor) numerics + everything else
     TORCHDYNAMO_DISABLE=1 python oracle/gen_golden.py eager  # eager numerics of the @torch.compile regions
 
-Three stubs are needed to run the reference on CPU (SURVEY §8c): the absent `sgl_kernel.flash_attn`
+Three stubs are needed to run the reference on CPU: the absent `sgl_kernel.flash_attn`
 wheel (two functions, replaced by a pure-torch paged attention with FlashAttention's documented
 semantics) and the Triton `store_kvcache` (replaced by an index scatter).  Everything else —
 ssd.utils.verify.verify, ssd.layers.sampler.Sampler, ssd.layers.{layernorm,rotary_embedding,activation},
@@ -295,7 +295,7 @@ def _hf_cfg(family, c):
     cfg = Cfg(hidden_size=c.hidden, intermediate_size=c.ffn, num_hidden_layers=c.layers, num_attention_heads=c.heads,
               num_key_value_heads=c.kv_heads, head_dim=c.head_dim, vocab_size=c.vocab, rms_norm_eps=c.rms_eps,
               max_position_embeddings=c.max_pos, tie_word_embeddings=c.tie_embed, hidden_act="silu")
-    cfg.rope_scaling = None  # SURVEY §8c(iv): transformers 5.5 makes this a dict; the reference needs None
+    cfg.rope_scaling = None  # transformers 5.5 makes this a dict; the reference needs None
     cfg.rope_theta = c.rope_theta
     cfg.torch_dtype = torch.bfloat16
     return cfg

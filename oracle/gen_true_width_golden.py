@@ -1,4 +1,4 @@
-"""Generate tests/golden/true_width_<cfg>.npz: the ORACLE's sync-SD steps at the TRUE widths of the BASELINE models.
+"""Generate tests/golden/true_width_<cfg>.npz: the ORACLE's sync-SD steps at the TRUE widths of the benchmark's models.
 
     python oracle/gen_true_width_golden.py [llama70b llama8b qwen32b]
 
@@ -30,7 +30,7 @@ OUT = REPO / "tests" / "golden"
 
 # name: (target shape, draft shape, batch, prompt lengths, K, spec steps)
 CONFIGS = {
-    "llama70b": ("llama-3.1-70b", "llama-3.2-1b", 1, [200], 6, 2),   # 200-token prompt: 4 prefill chunks (ADVICE r1 #1)
+    "llama70b": ("llama-3.1-70b", "llama-3.2-1b", 1, [200], 6, 2),   # 200-token prompt: 4 prefill chunks
     "llama8b": ("llama-3.1-8b", "llama-3.2-1b", 2, [40, 23], 6, 2),
     "qwen32b": ("qwen3-32b", "qwen3-0.6b", 2, [33, 48], 6, 2),
 }

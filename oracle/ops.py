@@ -2,7 +2,7 @@
 
 `compiled=True` (default) follows the numerics the reference actually runs with — its
 RMSNorm / SiluAndMul are @torch.compile regions, and Inductor keeps the in-kernel
-`.to(bf16)` in fp32, i.e. ONE rounding (SURVEY §8a checklist 2); `compiled=False` is the eager
+`.to(bf16)` in fp32, i.e. ONE rounding; `compiled=False` is the eager
 (double-rounding) reading of the same source, used to pin against eager goldens.
 """
 from __future__ import annotations

@@ -1,4 +1,4 @@
-"""Bookkeeping-level driver for differential tests of Scheduler / BlockManager / Sequence (SURVEY §8 row a19).
+"""Bookkeeping-level driver for differential tests of Scheduler / BlockManager / Sequence.
 
 TEST INFRASTRUCTURE ONLY.  The same scripted workload is pushed through the reference's own classes
 (oracle/gen_sched_golden.py, in the build container) and through ssd_b200.engine (tests/test_sched_golden.py); the model

@@ -90,7 +90,7 @@ class SpecSession:
         return suffixes, rec, logits_p, logits_q, spec
 
 
-    # ---- teacher-forced replay (tolerance protocol of SURVEY §7 "hard parts") ----
+    # ---- teacher-forced replay (tolerance protocol) ----
     def spec_step_forced(self, spec: torch.Tensor):
         """Run the K+1 draft forwards and the verify forward on GIVEN speculation tokens [B, K+1] without
         advancing the session. Returns (logits_p [B,K+1,V], logits_q [B,K,V])."""
@@ -120,8 +120,7 @@ def check_greedy_step(spec: torch.Tensor, n_accept: list[int], recovery: list[in
                       eps: float):
     """Compare a teacher's greedy (temp 0) step outcome with logits computed by a checker on the same tokens.
     Returns (hard_mismatches, near_tie_mismatches): a decision only counts as hard when the checker's own
-    top-2 margin at that position is >= eps (bf16 logits tie within a few ulps far too often for exact match;
-    SURVEY §7)."""
+    top-2 margin at that position is >= eps (bf16 logits tie within a few ulps far too often for exact match)."""
     B, Kp1 = spec.shape
     K = Kp1 - 1
     hard, soft = [], []

@@ -60,7 +60,7 @@ class Config:
         if not 1 <= self.num_gpus <= 8:
             raise AssertionError("single node only: 1 <= num_gpus <= 8 (config.py:55)")
         if self.draft_async:
-            raise NotImplementedError("draft_async (async SSD) is a SURVEY §8(f) 'next' row, not built yet")
+            raise NotImplementedError("draft_async (asynchronous speculation) is not built")
         if self.use_eagle:
             raise NotImplementedError("EAGLE-3 drafts are out of scope of the sync-SD hot path")
         if self.enforce_eager:
@@ -87,7 +87,7 @@ class Config:
             self.max_model_len = min(self.max_model_len, self.draft_hf_config.max_position_embeddings)
         if self.max_num_batched_tokens < self.max_model_len:
             raise AssertionError("max_num_batched_tokens < max_model_len (config.py:94)")
-        # limits of libssdk (DESIGN.md "Limits"), reported here rather than at the first step
+        # limits of libssdk, reported here rather than at the first step
         k1 = (self.speculate_k + 1) if self.speculate else 1
         if self.speculate and not 1 <= self.speculate_k <= 7:
             raise ValueError(f"speculate_k={self.speculate_k}: libssdk supports 1 <= k <= 7")

@@ -75,7 +75,6 @@ SSDK_DEVINL float block_sum(float v, float* red) {
 }
 
 // (value, index) argmax with lowest-index tie-break == torch.argmax semantics
-// (SURVEY §8a checklist 6).
 struct ArgMax {
   float v;
   int i;
@@ -126,7 +125,7 @@ SSDK_DEVINL float u32_to_exp1(uint32_t x) { return -__logf(u32_to_unit_open0(x))
 // epoch / slot parity of the one-shot all-reduce number call_idx of target forward number seq (n_calls all-reduces per
 // forward).  The slot parity runs on ACROSS forwards: a forward has 2L+1 all-reduces — an odd number — so a per-forward
 // parity would put the last all-reduce of forward n and the first one of forward n+1 into the same slot back to back, and
-// a fast rank could overwrite words a slow peer is still polling (ADVICE r1).  With a continuous parity a slot is reused at
+// a fast rank could overwrite words a slow peer is still polling.  With a continuous parity a slot is reused at
 // distance 2 only, which the data dependence already protects (a rank needs every peer's words of all-reduce i+1 before
 // it can publish i+2).
 SSDK_DEVINL unsigned symm_epoch_of(unsigned seq, int call_idx) { return seq * 512u + (unsigned)call_idx + 1u; }

@@ -442,7 +442,7 @@ __global__ void selective_scan_kernel(const SelScanArgs p, const Ragged rg) {
 // one lane.  A piece's decay of state n is exp(A_n sum dt).  Six rows are taken together: their B | C rows (one coalesced load each)
 // wait in shared memory for all lanes, the next six rows' loads are in flight under them.  Bound by issue slots and by the exponentials
 // (two per state and row, 16 per clock and SM).  The walk over all rows with states spread over lanes was a chain of 0.39 us per row:
-// 2048 rows x 4096 channels x 16 states 802 -> 107 us (299 us with a row at a time).
+// 2048 rows x 4096 channels x 16 states 802 -> 126 us (299 us with a row at a time).
 template <typename T, int NT>
 __global__ void __launch_bounds__(kScanChunks * 32) selective_chunk_scan_kernel(const SelScanArgs p, const Ragged rg) {
   pdl_wait();

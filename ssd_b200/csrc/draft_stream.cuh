@@ -2,7 +2,7 @@
 // K+1 single-token draft forwards + K samplings) as ONE persistent kernel, batch 1.
 //
 // Why: the 1B draft streams 2.47 GB per forward (0.376 ms at the measured HBM peak) but the kernel-per-op path needs
-// 0.79 ms — nine kernel boundaries per layer, during each of which HBM idles (profiles/r01_small_kernels.md).  The weights
+// 0.79 ms — nine kernel boundaries per layer, during each of which HBM idles.  The weights
 // do not depend on the activations, so here every CTA (one per SM) streams ITS share of every matrix, in program order
 // and without ever waiting for a phase, through a ring of 32 KB shared-memory slots:
 //   * a PRODUCER warp requests slot after slot with bulk async copies (cp.async.bulk global -> shared, mbarrier
@@ -12,7 +12,7 @@
 //   * 8 CONSUMER warps run the phases.  A projection at one token is a GEMV: each warp keeps its 64-float slice of x in
 //     registers for the whole phase and owns whole rows (K <= 2048: no cross-warp traffic at all), reads 16 bytes per
 //     lane per step from the slot (conflict-free), and releases the slot with one mbarrier arrive per warp.
-// History (profiles/r02_draft_stream.md): persistent kernel with weights read straight from global memory 0.85 ms per
+// History: persistent kernel with weights read straight from global memory 0.85 ms per
 // forward; first ring version (thread 0 issuing the copies between block-wide barriers, x read from shared memory)
 // 1.05-1.15 ms: the consume loop, not HBM, was the bottleneck (1.2 us per 32 KB slot against 0.73 us of HBM time).
 //
@@ -26,7 +26,7 @@
 // then final norm -> lm_head rows -> in-kernel sampling (greedy argmax over the bf16 logits, lowest index wins, or the
 // Philox exponential race of layers/sampler.py:27-34 — the SAME scores sample_kernel computes, so the tokens are identical)
 // -> the next forward starts inside the same launch.  The last forward of a step only writes KV (speculator_sync.py:52-56).
-// Rounding points are the reference's (SURVEY §8a checklist 1-4): every linear output, the residual, the norm output, q/k
+// Rounding points are the reference's: every linear output, the residual, the norm output, q/k
 // after RoPE and the attention output are rounded to bf16; accumulation is fp32.
 //
 // Jobs: rows are dealt to CTAs in jobs of consecutive rows; job s of a matrix belongs to CTA s mod #CTAs.
@@ -99,7 +99,7 @@ SSDK_DEVINL void ds_sync() {
 // has arrived, so every CTA computes the same base).  Arrival = one release-add without a return value; waiting = relaxed
 // polling loads + one acquire fence at the end.  (A first version — acq_rel fetch-adds for arrival, counter reset and
 // generation bump, acquire loads for polling — compiled to MEMBAR.ALL.GPU + ATOMG + CCTL.IVALL three times in a row on the
-// last arriver and an L1 invalidation per poll: 2.9 us per barrier, 15 us per layer; profiles/r02_draft_stream.md.)
+// last arriver and an L1 invalidation per poll: 2.9 us per barrier, 15 us per layer.)
 // ---------------------------------------------------------------------------------------------
 struct DsGridBar {
   unsigned long long* counter;
@@ -192,7 +192,7 @@ SSDK_DEVINL void ds_cursor_settle(const DsParams& p, const DsGeom* geom, DsCurso
 
 // the producer: one lane walks the job sequence of this CTA and refills slots as the consumers release them.  (An L2
 // window beyond the ring — `cp.async.bulk.prefetch.L2` of the next jobs, continuously or only while every requested copy
-// had landed — was measured twice and removed: 8B + 1B 8.53 / 8.63 vs 8.34 / 8.48 ms per step, profiles/r02_draft_stream.md.)
+// had landed — was measured twice and removed: 8B + 1B 8.53 / 8.63 vs 8.34 / 8.48 ms per step.)
 SSDK_DEVINL void ds_cursor_next(const DsParams& p, const DsGeom* geom, DsCursor& c) {
   c.s += (int)gridDim.x;
   if (c.s >= geom[c.m].nj) ds_cursor_settle(p, geom, c);

@@ -2,7 +2,7 @@
 // per-head norm + RoPE + KV-cache scatter, SiLU*mul, and the per-forward index prep.
 // Every kernel also folds in the fixed-order reduction of the producer GEMM's split-K
 // partials (fp32 [S, M, N]) and the bf16 rounding the reference applies to every
-// F.linear output (SURVEY §8a checklist 1).
+// F.linear output.
 #pragma once
 #include "common.cuh"
 
@@ -152,7 +152,7 @@ struct SymmIn {
   unsigned slot_bytes;
 };
 constexpr int kSymmMaxRanks = 8;
-// NOTE (robustness item for the next round): fwd_seq is bumped by prep_kernel at the START of the forward.  A dataflow
+// NOTE: fwd_seq is bumped by prep_kernel at the START of the forward.  A dataflow
 // consumer reads it without a grid-dependency wait, i.e. formally it could run before prep_kernel has finished if the
 // whole PDL chain (>= 9 launches) were co-resident and launched within prep's ~2 us — impossible at model shapes
 // (the GEMM grids serialise the chain) and never observed, but not excluded by construction.  Moving the bump into a
@@ -360,8 +360,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_kernel(NormParams p) {
 
 // The same for calls of many rows, whose input is an embedding or rounded to bf16 already (no slabs, no all-reduce): without their
 // registers three CTAs of 512 threads share an SM instead of one.  2003 rows of 4096: 12 us a call; with the rotation's like form a prompt of
-// 8B widths and 4 layers takes 3934 us instead of 4143.  (A kernel of its own, so that the one above stays as it is: with
-// both in one the 8B + 1B step took 8468 us instead of 8450.)
+// 8B widths and 4 layers takes 3934 us instead of 4143.  (A kernel of its own, so that the decode step's above keeps its code.)
 template <int SLICES>
 __global__ void __launch_bounds__(512, 3) add_rmsnorm_rows_kernel(NormParams p) {
   SSDK_STATIC_SMEM(float, red, 32);
@@ -570,7 +569,7 @@ __global__ void __launch_bounds__(128) rope_store_kernel(RopeParams p) {
 }
 
 // The same for calls of many rows, whose projection is rounded to bf16 already: a warp takes kRopeHeads heads of its row, all of them asked
-// for together, the angles once.  (A head per warp: 26 us for 2003 rows and 48 heads of 128.)
+// for together, the angles once.  2003 rows, 48 heads of 128: 10.6 us (a head per warp: 26).
 constexpr int kRopeHeads = 4;
 
 template <int HD>

@@ -13,7 +13,9 @@
 // on (as long as K times the largest other operand is below 2^30).  Results that are not finite, and results below 2^-70 that are not zero, are
 // therefore taken again as the FMA chain over k that linear_kernel walks (see split_again).  What still differs: a result below 2^-126 may be zero.
 //
-// What bounds it: the tensor core, 24 products of 64 clocks per k-block of 64 and 128 tokens, under which everything else hides.  The
+// What bounds it: 24 products of 64 clocks per k-block of 64 and 128 tokens are a floor that it is 2.6 times above (tensor pipe active 38 % of
+// the time on the SMs that have two tiles of 1000 x 3072 x 2048, 25 % on all: 96 tiles on 74 pairs), DRAM and issue slots are further
+// away (3 and 16 %): three stages of 72 KB do not cover the way of the weights through registers.  The
 // FMA form it takes over from (linear_kernel, 64 x 64 tiles) was bound by its shared-memory operands: 1000 x 4096 x 2048 539 us (31 TFLOP/s)
 // -> 145 us (115), 2000 x 8192 x 2048 2092 -> 459 us; with few rows the kernel streams the weights (8 x 8192 x 2048 148 -> 50 us), which is
 // why the tokens of a tile go down to 32.  Pairs of CTAs and the persistent walk as in

@@ -447,8 +447,6 @@ struct HybRun {
     p.out = C; p.M = m_total; p.chunks = (m_total + kPairTokens - 1) / kPairTokens; p.act = gelu ? GLU_GELU : GLU_SILU;
     return go_pair(glu, A, W, m_total, w_rows, 1, K, ldw, p, p.chunks);
   }
-  // (gemm_ws_kernel asks for its first weight tiles, and in grouped mode reads the tile list, before it waits for the kernel in front:
-  // launches whose "weights" or list that kernel writes start after it)
   // per head h: C[:, h out_step ..] = A[:, h x_step .. + K] W[h N .. + N, :]^T (bf16 or fp32 out); H = 1: one product with a bf16 result.
   // Other calls take the batched tile.  2000 rows, 16 heads: 128 -> 512 columns 70 -> 27 us, 512 -> 128 columns 31 -> 20 us
   int lin_heads(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int m, int N, int K, bool out_t, int H, int x_step, int out_step) {
@@ -467,6 +465,8 @@ struct HybRun {
     p.batch = H; p.x_step = x_step; p.out_step = out_step;
     return launch_gemm_pair(L, out_t ? EPI_BF16 : EPI_PARTIAL, tmW, tmX, tmXs, p, p.w_tiles * p.chunks * H);
   }
+  // (gemm_ws_kernel asks for its first weight tiles, and in grouped mode reads the tile list, before it waits for the kernel in front:
+  // launches whose "weights" (fresh_w) or list that kernel writes start after it)
   int lin_tc(const void* A, const void* W, float* C, int m_total, int N, int K, int ldw, bool fresh_w = false) {
     if (fresh_w) L.barrier_op();
     if (pair_ok(m_total)) return lin_pair(false, A, W, C, m_total, N, K, ldw, false);

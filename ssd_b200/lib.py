@@ -201,6 +201,6 @@ def last_error() -> str:
 
 
 def check(rc: int, what: str = "ssdk call") -> None:
-    """Reference error convention is Python exceptions: map rc<0 to RuntimeError."""
+    """The reference reports errors as Python exceptions: map rc<0 to RuntimeError."""
     if rc != 0:
         raise RuntimeError(f"{what} failed: {last_error()}")

@@ -164,7 +164,7 @@ def build_runner(config, tp_size: int = 1, tp_rank: int = 0, device=None, finali
     wt = load_weights(config.model, tspec, device, tp_size, tp_rank)
     wd = load_weights(config.draft, dspec, device) if (dspec is not None and tp_rank == 0) else None
     if dspec is not None and tp_rank != 0:
-        dspec = None  # the draft is a replica pinned to rank 0 (SURVEY §8e)
+        dspec = None  # the draft is a replica pinned to rank 0
     nbt = kv_blocks_for(config, tspec, tp_size, 0.8 if dspec else 1.0)
     nbd = kv_blocks_for(config, dspec, 1, 0.75, reserved=nbt * kv_block_bytes(config, tspec, tp_size)) if dspec else None
     config.num_kvcache_blocks = nbt

@@ -184,7 +184,7 @@ class PairRunner:
         rows: the rows a call may carry; prompts ask for pass_tokens.  draws: per sequence, the call number and the row that
         its random draw is taken for (draw_numbers), if those are not this call's own."""
         if self.spec[which] is None:
-            return None  # the draft replica lives on TP rank 0 only (SURVEY §8e); other ranks have nothing to do
+            return None  # the draft replica lives on TP rank 0 only; other ranks have nothing to do
         B, Q = len(ids), len(ids[0])
         assert all(len(x) == Q for x in ids)
         ids_a = np.ascontiguousarray(np.array(ids, dtype=np.int64).reshape(-1))

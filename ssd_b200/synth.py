@@ -2,7 +2,7 @@
 
 There are no model weights in the image, so throughput is measured on synthetic weights at the true shapes
 (every kernel streams the real byte count).  To make speculative decoding behave like a real target/draft pair the
-weights are built with the "bigram agreement" construction of SURVEY §8(d):
+weights are built with the "bigram agreement" construction:
 
   * token embeddings e_t ~ N(0,1)^d (near-orthogonal), lm_head[pi(t)] = e_t  => greedy next token = pi(t);
   * o_proj / down_proj are scaled to ~0 so the residual stream stays the embedding (they are still streamed);
@@ -85,7 +85,7 @@ def permutations(vocab: int, seed: int, alpha: float, device, draft_mode: str = 
     draft_mode "perm" (default): on the other tokens the draft follows a DIFFERENT next-token map with the same large
     margin — pi_draft(t) = pi_target(sigma(t)) with sigma a cyclic shift inside the disagreeing set — so pi_draft is a
     permutation too, every draft decision is as clear-cut as the target's and a whole run is reproducible token for
-    token (engine vs oracle vs the reference engine on the same weights).  "noise" (round 1): pi_draft = -1 there, the
+    token (engine vs oracle vs the reference engine on the same weights).  "noise": pi_draft = -1 there, the
     draft's lm_head row is missing and its guess is the argmax of noise (a near-tie a few per cent of the time)."""
     g = torch.Generator(device="cpu").manual_seed(seed * 7919 + 13)
     pi_t = torch.randperm(vocab, generator=g, device="cpu")  # explicit: the caller may run under set_default_device("cuda")
@@ -197,7 +197,7 @@ def iter_weights(spec, meta: dict, device, tp_size: int = 1, tp_rank: int = 0):
             "post_norm": torch.ones(d, dtype=bf, device=device),
             "qkv": randn((H + 2 * KV) * hd, d, 0.02, gl),
             # default ~0: keeps the residual stream == embedding (accept-len control); `o_down_std` in the
-            # directory's meta switches the attention / MLP branches on (parity tests, DESIGN §4)
+            # directory's meta switches the attention / MLP branches on (parity tests)
             "o": randn(d, H * hd, o_std, gl),
             "gate_up": randn(2 * ffn, d, 0.02, gl),
             "down": randn(d, ffn, down_std, gl),

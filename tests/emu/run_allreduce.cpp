@@ -24,7 +24,7 @@ int main(int argc, char** argv) {
   std::ifstream f(argv[1], std::ios::binary);
   auto hdr = rd<int32_t>(f, 7);
   // n_calls all-reduces per forward (odd, like the 2L+1 of a real forward), n_fwd forwards back to back with NO other
-  // cross-rank synchronisation in between; rank `slow` dawdles in the last consumer of every forward (ADVICE r1 #2)
+  // cross-rank synchronisation in between; rank `slow` dawdles in the last consumer of every forward
   const int R = hdr[0], M = hdr[1], d = hdr[2], S = hdr[3], per_fwd = hdr[4], threads = hdr[5], n_fwd = hdr[6];
   const int n_calls = per_fwd * n_fwd, slow = R - 1;
   const float eps = rd<float>(f, 1)[0];

@@ -2,7 +2,7 @@
 `add_rmsnorm_kernel` (csrc/elementwise.cuh) — executed from SOURCE for 2 and 8 emulated ranks that share host memory the
 way peer-mapped symmetric buffers share HBM (tests/emu/run_allreduce.cpp).  Ranks are skewed against each other with
 random delays, three forwards of five all-reduces each (an ODD count per forward, like the 2L+1 of the real model, with the
-last rank dawdling in the last consumer of every forward — the slot-reuse case across forwards of ADVICE r1 #2) reuse the
+last rank dawdling in the last consumer of every forward — the slot-reuse case across forwards) reuse the
 two parity slots, and every rank must produce
 bf16( sum over ranks, in rank order, of that rank's bf16-rounded split-K reduction ) -> residual add -> RMSNorm,
 bit-identically on all ranks.  Covers the 1-slice and the 2-slice norm instantiations."""

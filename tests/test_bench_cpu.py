@@ -1,4 +1,4 @@
-"""CPU checks of bench.py's bookkeeping: the HBM step-roofline formula reproduces BASELINE.md §3, and the reference arm
+"""CPU checks of bench.py's bookkeeping: the HBM step-roofline formula reproduces the bytes of the model table, and the reference arm
 (`--impl reference`, the oracle port on host cores) runs end to end on a tiny workload and prints the required keys."""
 import json
 import os

@@ -92,7 +92,7 @@ def test_spec_steps_match_oracle(family, use_graph):
 
 
 # golden steps (of 10, two sequences each) that must be reproduced EXACTLY — speculations, accept counts and recovery
-# tokens of both sequences — before any near-tie may end the comparison; measured on B200 (profiles/r02_pytest_gpu.txt)
+# tokens of both sequences — before any near-tie may end the comparison; measured on B200
 MIN_EXACT_GOLDEN_STEPS = {"llama": 2, "qwen": 4}
 
 
@@ -213,7 +213,7 @@ def test_streaming_draft_kernel_matches_kernel_per_op_path():
 
 @pytest.mark.parametrize("chunk", [32, 64, 256])
 def test_long_prompt_prefill_in_unsynchronised_chunks(chunk):
-    """ADVICE r1 #1: ssdk_forward_tokens does not synchronise for non-final prefill chunks, so its pinned staging must not be
+    """ssdk_forward_tokens does not synchronise for non-final prefill chunks, so its pinned staging must not be
     reused before the queued H2D copy has run.  A 450-token prompt goes through 15 / 8 / 2 chunks (the first ones without a
     host sync); the sampled token and the last-position logits must match the oracle's single-pass prefill, and the KV it
     left behind must carry a correct decode step."""

@@ -1,5 +1,5 @@
 """End-to-end through the public API (LLM.generate, the call bench/bench.py makes): the speculative-decoding invariant
-— sync-SD output == autoregressive output of the target, token for token at temperature 0 (SURVEY §8c) — plus the
+— sync-SD output == autoregressive output of the target, token for token at temperature 0 — plus the
 METRICS contract, EOS / max_new_tokens truncation and prefix-cache reuse, on synthetic tiny Llama pairs."""
 import pytest
 import torch

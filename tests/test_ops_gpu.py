@@ -210,7 +210,7 @@ def test_verify_ratio_matches_oracle(dev):
 
 
 def test_verify_full_vocab_sizes(dev):
-    """BASELINE sizes: V = 128256 (Llama) and 151936 (Qwen), K = 6; size-independent properties."""
+    """Full vocabularies: V = 128256 (Llama) and 151936 (Qwen), K = 6; size-independent properties."""
     from ssd_b200 import ops
     for V_, K in ((128256, 6), (151936, 6)):
         g = torch.Generator().manual_seed(V_)

@@ -63,7 +63,7 @@ def test_layers_match_reference(tag, compiled):
     x, res, w = bf16(z["norm_x"]), bf16(z["norm_res"]), bf16(z["norm_w"])
     y = ops.rms_norm(x, w, 1e-5, compiled=compiled)
     y2, r2 = ops.rms_norm(x, w, 1e-5, res, compiled=compiled)
-    # reduction order inside Inductor differs: allow a vanishing fraction of 1-ulp flips (SURVEY §8a: 1.7e-5)
+    # reduction order inside Inductor differs: allow a vanishing fraction of 1-ulp flips (1.7e-5)
     assert ulp_mismatch_fraction(y, bf16(z["norm_y"])) < 2e-3
     assert ulp_mismatch_fraction(y2, bf16(z["norm_add_y"])) < 2e-3
     assert torch.equal(r2, bf16(z["norm_add_res"]))
@@ -126,10 +126,10 @@ def test_sync_sd_trace_matches_reference(family):
 
 
 def test_baseline_config0_plumbing_1b_shapes_on_cpu():
-    """BASELINE.json configs[0] — 'Llama-3 1B AR greedy b=1 on CPU (plumbing, no GPU)': the reference itself cannot
+    """Llama-3 1B, autoregressive, greedy, b=1 on CPU: the reference itself cannot
     run on CPU (engine/model_runner.py:88-89 hard-require CUDA), so the plumbing check is the oracle driving the
     Llama-3.2-1B layer shapes (2 of 16 layers, reduced vocab to keep the CPU suite fast) autoregressively and being
-    reproduced exactly by its own speculative path (SD == AR, SURVEY §8c)."""
+    reproduced exactly by its own speculative path (SD == AR)."""
     from oracle.model import ModelCfg, random_weights
     cfg = ModelCfg(hidden=2048, layers=2, heads=32, kv_heads=8, head_dim=64, ffn=8192, vocab=4096, max_pos=512)
     w = random_weights(cfg, 3)

@@ -1,9 +1,9 @@
-"""The reference's OWN acceptance harness (bench/bench.py, unmodified, SURVEY §2 item 19) driven on top of the
+"""The reference's OWN acceptance harness (bench/bench.py, unmodified) driven on top of the
 ssd_b200 host engine through the `ssd` compat shim — on CPU, with the device runner replaced by a deterministic test
 double.  Checks the drop-in boundary end to end: `import ssd.paths`, `from ssd import LLM, SamplingParams`,
 `from ssd.engine.llm_engine import METRICS`, the kwargs of `create_llm_kwargs`, `generate()`'s return value, the sweep
 path that pokes `llm.config.max_num_seqs` / `llm.scheduler.max_num_seqs`, and the scheduler / block-manager bookkeeping
-under random accept lengths.  Skipped where the reference checkout is absent (the GPU box)."""
+under random accept lengths.  Skipped where the reference checkout is absent."""
 import importlib
 import json
 import os

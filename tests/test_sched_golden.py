@@ -1,4 +1,4 @@
-"""Scheduler / BlockManager / Sequence against the reference's own classes (SURVEY §8 row a19): the scripted workloads of
+"""Scheduler / BlockManager / Sequence against the reference's own classes: the scripted workloads of
 oracle/sched_driver.py were run through the unmodified ssd/engine/{scheduler,block_manager,sequence}.py
 (oracle/gen_sched_golden.py); here the same driver runs ssd_b200.engine and every recorded state must be identical —
 block tables and free-list order included, because the block tables are hot-path inputs of the kernels."""

@@ -1,4 +1,4 @@
-"""Engine-level parity at the TRUE widths of the BASELINE models.
+"""Engine-level parity at the TRUE widths of the benchmark's models.
 
 Two decoder layers at the real dimensions of Llama-3.1-70B / 8B / Qwen3-32B (+ their drafts), full vocabulary,
 NON-degenerate o_proj / down_proj, a 200-token prompt (4 prefill chunks, none of the first three synchronises) — the
