@@ -1,4 +1,4 @@
-"""Micro-benchmark of the weight-streaming GEMM at the shapes of the BASELINE models: achieved HBM GB/s
+"""Micro-benchmark of the weight-streaming GEMM at the shapes of the benchmark's models: achieved HBM GB/s
 (weight bytes / CUDA-event time, L2 flushed between launches) next to torch (cuBLAS) on the same shapes."""
 import json
 import os
@@ -49,7 +49,7 @@ def main():
             print(json.dumps(rec), flush=True)
             out.append(rec)
         del w
-    json.dump(out, open("gpurun_out/gemm_bench.json", "w"), indent=1)
+    json.dump(out, open("gemm_bench.json", "w"), indent=1)
 
 
 if __name__ == "__main__":

@@ -1,4 +1,4 @@
-"""Prefill (TTFT) timing of ssdk_forward_tokens in chunks of 64 (round 1) vs 256 tokens (UMMA N = 256 instances of the GEMM):
+"""Prefill (TTFT) timing of ssdk_forward_tokens in chunks of 64 vs 256 tokens (UMMA N = 256 instances of the GEMM):
 a 2048-token prompt through the 8B-width target (full depth) and an 8-layer 70B-width target; then the reference bench's
 prompt set (16 prompts x 128 tokens) one prompt per call vs packed two to a call (PairRunner.prefill_many)."""
 import os

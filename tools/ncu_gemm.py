@@ -1,5 +1,5 @@
 """Launch the dominant kernel (weight-streaming GEMM, SiLU epilogue) at the 70B gate|up shape a few times — target of
-`ncu --set full -k regex:gemm_ws` (see tools/gpu_ncu.sh)."""
+`ncu --set full --clock-control none -k regex:gemm_ws`."""
 import os
 import sys
 

@@ -1,4 +1,4 @@
-"""Workload for the per-kernel-family `ncu --set full` captures (tools/gpu_ncu_families.sh).
+"""Workload for the per-kernel-family `ncu --set full` captures.
 
     python tools/ncu_workload.py engine   # eager (no CUDA graph) spec steps: every kernel family of the hot path at the
                                           # widths of Llama-3.1-70B (2 layers) + Llama-3.2-1B (2 layers), full vocabulary

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Run the reference's unmodified bench/bench.py on top of ssd_b200 (the acceptance harness).
+"""Run the reference's unmodified bench/bench.py on top of ssd_b200 (its acceptance harness).
 
     python tools/run_reference_bench.py --ref /path/to/ssd [--synthetic] -- --size 8 --spec --k 6 --random --numseqs 8 --b 1
 
