@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Reference GPU arm: the UNMODIFIED reference engine (tanishqkumar/ssd, installed under baseline/_ref by
 `__graft_entry__.build()` with `pip install --no-deps --target baseline/_ref /root/reference`) driven through its own public
-API — `ssd.LLM(...)`, `add_request`, `create_inference_step`, `step` — on this box's GPU: its `LlamaForCausalLM` /
+API — `ssd.LLM(...)`, `add_request`, `create_inference_step`, `step` — on the local GPU: its `LlamaForCausalLM` /
 `Qwen3ForCausalLM`, `F.linear` (cuBLAS), its `@torch.compile` regions (Inductor -> Triton), its Triton `store_kvcache`,
 its CUDA-graph capture / replay (`capture_cudagraph`, `run_decode_cudagraph`, `run_verify_cudagraph`), its `Sampler`,
 `verify()`, `Scheduler` and `BlockManager`.  None of ssd_b200's kernels or engine code is on this path.

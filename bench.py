@@ -18,7 +18,7 @@ temp 0, synthetic "bigram agreement" weights at the exact shapes (there are no c
   parity_check  temp 0: the tokens of the timed device-resident loop AND of the engine (e2e) loop against the closed-form
             greedy chain of the synthetic target (t_{i+1} = pi_t(t_i)) — token-for-token, at every N
   allreduce "symm" (one-shot NVLink all-reduce, ssd_b200's own kernels) | "nccl" (SSD_B200_NO_SYMM=1) | "none" (N=1)
-  reference_gpu  (N=1) the UNMODIFIED reference engine on this box's GPU (baseline/ref_gpu.py: torch.compile, cuBLAS,
+  reference_gpu  (N=1) the UNMODIFIED reference engine on the same GPU (baseline/ref_gpu.py: torch.compile, cuBLAS,
             its CUDA graphs, flash_attn 2.8.3 stub) on the same weights and prompt: its tokens/s, and whether its tokens
             equal ours; `--impl reference-gpu` prints that arm alone
 """
@@ -99,7 +99,7 @@ class ClockSampler:
 
 def usable_cores() -> int:
     """Threads the CPU arm may really use: min(CPU affinity, cgroup cpu.max quota).  os.cpu_count() reports the host's
-    128 logical CPUs while the container's quota is 16 — 128 oversubscribed threads made the round-1 CPU arm swing 13x."""
+    128 logical CPUs while the container's quota is 16 — 128 oversubscribed threads made the CPU arm swing 13x."""
     n = len(os.sched_getaffinity(0)) if hasattr(os, "sched_getaffinity") else (os.cpu_count() or 1)
     try:
         with open("/sys/fs/cgroup/cpu.max") as f:
@@ -431,7 +431,7 @@ def cpu_baseline(tshape, dshape, K, alpha, sample_steps=3, t_layers=2, d_layers=
 
 def run_reference(args):
     """Reference arm of this tier: the reference's own CPU implementation of the path = the oracle port
-    (the Python reference cannot travel to the GPU box), all host threads, bounded sample per step."""
+    (the reference need not be installed), all host threads, bounded sample per step."""
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return

@@ -1,6 +1,6 @@
 """Generate tests/golden/*.npz by importing and running the UNMODIFIED reference (/root/reference).
 
-Runs only in the build container (the reference does not travel to the GPU box).  Usage:
+Runs where the reference is mounted.  Usage:
 
     CXX=/usr/bin/g++ python oracle/gen_golden.py            # compiled (Inductor) numerics + everything else
     TORCHDYNAMO_DISABLE=1 python oracle/gen_golden.py eager  # eager numerics of the @torch.compile regions

@@ -1,5 +1,5 @@
 """Generate tests/golden/sched_*.json.gz by running the UNMODIFIED reference Scheduler / BlockManager / Sequence
-(ssd/engine/{scheduler,block_manager,sequence}.py) through oracle/sched_driver.py.  Build container only.
+(ssd/engine/{scheduler,block_manager,sequence}.py) through oracle/sched_driver.py.  Needs the reference.
 
     python oracle/gen_sched_golden.py
 

@@ -2,7 +2,7 @@
 
     python oracle/gen_true_width_golden.py [llama70b llama8b qwen32b]
 
-TEST INFRASTRUCTURE (like everything under oracle/).  Runs in the build container (CPU, minutes per config); the GPU
+TEST INFRASTRUCTURE (like everything under oracle/).  Runs on the CPU (minutes per config); the GPU
 test `tests/test_true_width_gpu.py` regenerates the very same weights on the device — `ssd_b200.synth` with
 `rng="hash"` is a pure integer function of (stream, row, column), bit-identical on CPU and GPU — runs the same prompt
 through `ssdk_forward_tokens` / `ssdk_spec_step`, and compares tokens, accept counts, recovery tokens and the logits at

@@ -1,7 +1,7 @@
 """Bookkeeping-level driver for differential tests of Scheduler / BlockManager / Sequence.
 
 TEST INFRASTRUCTURE ONLY.  The same scripted workload is pushed through the reference's own classes
-(oracle/gen_sched_golden.py, in the build container) and through ssd_b200.engine (tests/test_sched_golden.py); the model
+(oracle/gen_sched_golden.py) and through ssd_b200.engine (tests/test_sched_golden.py); the model
 is replaced by a deterministic token chain with seeded accept lengths, exactly where LLMEngine.step
 (engine/llm_engine.py:186-236) would call ModelRunner / Speculator / Verifier:
 

@@ -5,7 +5,7 @@
 
 The library links only against libcudart (static) and NCCL; it has no torch or Python
 dependency.  The built .so lives next to the sources (ssd_b200/_lib/libssdk.so) so it
-travels with the repo snapshot to the GPU box.
+travels with a copy of the tree.
 """
 from __future__ import annotations
 

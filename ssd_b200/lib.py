@@ -179,7 +179,7 @@ def load(build_if_missing: bool = True) -> C.CDLL:
         try:
             if _build.is_stale():
                 _build.build(verbose=False)
-        except Exception as exc:  # no nvcc on this box: the prebuilt .so must be there
+        except Exception as exc:  # no nvcc here: the prebuilt .so must be there
             if not _LIB_PATH.exists():
                 raise RuntimeError(f"libssdk.so is missing and could not be built: {exc}") from exc
     if not _LIB_PATH.exists():

@@ -103,8 +103,8 @@ def permutations(vocab: int, seed: int, alpha: float, device, draft_mode: str = 
 def hash_uniform(rows: int, cols: int, std: float, stream: int, device, row0: int = 0) -> torch.Tensor:
     """Device-independent pseudo-random bf16 matrix [rows, cols], zero mean, standard deviation `std` (uniform): element
     (r, c) is a pure integer function of (stream, r + row0, c) — splitmix64-style, wrapping int64 arithmetic — so the
-    same bits come out on CPU and GPU.  Used where a fixture generated in the (GPU-less) build container must be
-    regenerated bit-for-bit on the GPU box (tests/golden/true_width_*.npz)."""
+    same bits come out on CPU and GPU.  Used where a fixture generated without a GPU must be
+    regenerated bit-for-bit on a GPU (tests/golden/true_width_*.npz)."""
     out = torch.empty(rows, cols, dtype=torch.bfloat16, device=device)
     step = max(1, (1 << 25) // max(cols, 1))
     c = torch.arange(cols, dtype=torch.int64, device=device)[None, :]

@@ -2,7 +2,7 @@
 
 Two decoder layers at the real dimensions of Llama-3.1-70B / 8B / Qwen3-32B (+ their drafts), full vocabulary,
 NON-degenerate o_proj / down_proj, a 200-token prompt (4 prefill chunks, none of the first three synchronises) — the
-oracle ran the same prompts on the same weights in the build container (oracle/gen_true_width_golden.py; the weights are
+oracle ran the same prompts on the same weights on the CPU (oracle/gen_true_width_golden.py; the weights are
 a pure integer function of (stream, row, column) and are regenerated here bit-for-bit on the device).  Checked, through
 the C-ABI (ssdk_forward_tokens / ssdk_spec_step):
   * the first sampled token, every speculated token, accept count and recovery token: EXACT (all margins are in the
