@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "elementwise.cuh"
 #include "gemm.cuh"
+#include "gemm_few.cuh"
 #include "gemm_pair.cuh"
 #include "prompt_attention.cuh"
 #include "gemm_split.cuh"
@@ -280,6 +281,24 @@ static int launch_gemm_split(Launcher& L, const CUtensorMap& tmX, GemmSplitParam
   }
   p.timeout = L.gave_up;
   return L.go(gemm_split_kernel, dim3(2 * std::min(max_tiles, num_sms() / 2)), dim3(kSplitThreads), (size_t)kSplitSmem, tmX, p);
+}
+
+// Up to 30 MB of weights: what is asked for before the kernel in front is done then covers a good part of them (64 KB per CTA).  Above, the deeper ring of
+// gemm_ws_kernel streams better behind a wait: four layers of 8B widths with rows of 8 sequences 628 us either way up to 30 MB, 691 with their 33 MB
+// matrices here; qwen3-0.6b, 4 layers, one sequence 283 -> 262 (up to 9 MB), 244 (13 and 30 MB).  M <= 8 is the token side of the instruction: two
+// tiles of tokens cost registers for the loads in flight (16 rows of llama-3.2-1b 412 -> 430 us).
+static bool few_rows(int M, int64_t N, int K) { return M <= kFewTokens && N * K * 2 <= (30 << 20); }
+// fp32, bf16 or act(gate) * up in bf16; W and X start on 16-byte boundaries, their strides are whole 16-byte pieces, K % 64 == 0
+static int launch_gemm_few(Launcher& L, int epi, const void* X, int ldx, const void* W, int ldw, void* out, int ldo, int M, int N, int K, bool gelu = false) {
+  GemmFewParams p;
+  p.W = (const bf16*)W; p.X = (const bf16*)X; p.out = out; p.M = M; p.N = N; p.K = K; p.ldw = ldw; p.ldx = ldx; p.ldo = ldo; p.gelu = gelu;
+  const int cols = epi == FEW_SILU || epi == FEW_GLU ? kFewRows / 2 : kFewRows, tiles = (N + cols - 1) / cols;
+  const int warps = K <= 1024 ? kFewWarps / 2 : kFewWarps;   // (at least four units of k per warp)
+  const dim3 grid(std::min(tiles, num_sms() * 2 * kFewWarps / warps)), block(32 * warps);
+  if (epi == FEW_F32) return L.go(gemm_few_kernel<FEW_F32>, grid, block, 0, p);
+  if (epi == FEW_BF16) return L.go(gemm_few_kernel<FEW_BF16>, grid, block, 0, p);
+  if (epi == FEW_SILU) return L.go(gemm_few_kernel<FEW_SILU>, grid, block, 0, p);
+  return L.go(gemm_few_kernel<FEW_GLU>, grid, block, 0, p);
 }
 
 struct WeightMat {
@@ -689,6 +708,10 @@ static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w
     p.w_tiles = epi == EPI_SILU ? (N_out + 127) / 128 : (N_out + 255) / 256; p.act = GLU_SILU_ROUNDED;
     if (splits_out) *splits_out = 0;
     return launch_gemm_pair(L, epi == EPI_SILU ? EPI_GLU : EPI_BF16, *tmW, *tmX, *tmXs, p, p.w_tiles * p.chunks);
+  }
+  if (epi != EPI_PUBLISH && few_rows(M, w.rows, K)) {
+    if (splits_out) *splits_out = 1;
+    return launch_gemm_few(L, epi == EPI_SILU ? FEW_SILU : epi == EPI_BF16 ? FEW_BF16 : FEW_F32, x, K, w.ptr, K, out, epi == EPI_PARTIAL ? N_out : ldo, M, N_out, K);
   }
   const int un = umma_n_for(M);
   const CUtensorMap* tmX;
@@ -1753,6 +1776,7 @@ int ssdk_gemm_small_m(const void* x, const void* w, void* y, float* partials, in
   const int num_kb = K / kBlockK;
   int S = split_k > 0 ? std::min(split_k, num_kb) : auto_splits(tiles, num_kb, un <= 64 ? 2 : 1);
   if (S > 1 && !partials) return fail("gemm_small_m: split_k=%d needs a partials buffer", S);
+  if (split_k <= 0 && few_rows(M, N, K)) return launch_gemm_few(L, FEW_BF16, x, K, w, K, y, ldy, M, N, K);
   GemmParams p;
   p.M = M; p.N = N; p.ldo = ldy; p.num_kb = num_kb; p.tile_rows = kTileRows; p.hi_row_offset = 64;
   p.kb_per_split = (num_kb + S - 1) / S;
@@ -1776,6 +1800,7 @@ int ssdk_gemm_gate_up_silu(const void* x, const void* w_gate_up, void* hout, int
   CKI(make_tmap(&tmW, w_gate_up, 2 * (int64_t)ffn, K, 64));
   const int un = umma_n_for(M);
   CKI(make_tmap(&tmX, x, M, K, un));
+  if (few_rows(M, 2 * (int64_t)ffn, K)) return launch_gemm_few(L, FEW_SILU, x, K, w_gate_up, K, hout, ffn, M, ffn, K);
   GemmParams p;
   p.out = hout; p.M = M; p.N = ffn; p.ldo = ffn; p.num_kb = K / kBlockK; p.kb_per_split = p.num_kb;
   p.tile_rows = 64; p.hi_row_offset = ffn;

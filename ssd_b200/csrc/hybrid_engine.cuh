@@ -469,6 +469,7 @@ struct HybRun {
   // launches whose "weights" (fresh_w) or list that kernel writes start after it)
   int lin_tc(const void* A, const void* W, float* C, int m_total, int N, int K, int ldw, bool fresh_w = false) {
     if (fresh_w) L.barrier_op();
+    if (few_rows(m_total, N, K)) return launch_gemm_few(L, FEW_F32, A, K, W, ldw, C, N, m_total, N, K);
     if (pair_ok(m_total)) return lin_pair(false, A, W, C, m_total, N, K, ldw, false);
     const CUtensorMap* tm;   // (copied: a later lookup may empty the table)
     CKI(e->tmap(W, N, K, 64, &tm, ldw == K ? 0 : ldw));
@@ -500,6 +501,7 @@ struct HybRun {
   }
   // y [m, ff] (bf16) = act(x Wg^T) * (x Wu^T) in the GEMM's epilogue; W holds the gate rows, then the up rows
   int lin_tc_glu(const void* A, const void* W, void* y, int m_total, int ff, int K, bool gelu) {
+    if (few_rows(m_total, 2 * ff, K)) return launch_gemm_few(L, FEW_GLU, A, K, W, K, y, ff, m_total, ff, K, gelu);
     if (ff % kPairGluRun == 0 && pair_ok(m_total)) return lin_pair(true, A, W, y, m_total, 2 * ff, K, K, gelu);
     const CUtensorMap* tm;
     CKI(e->tmap(W, 2 * ff, K, 64, &tm));
