@@ -255,6 +255,13 @@ int ssdk_paged_attn(const void* q, const void* k_cache, const void* v_cache,
                     int batch, int q_len, int heads, int kv_heads, int head_dim,
                     int block_size, int max_blocks_per_seq, float scale, void* stream);
 
+/* ssdk_paged_attn for a cache of num_blocks pages whose size the caller knows. */
+int ssdk_paged_attn_pages(const void* q, const void* k_cache, const void* v_cache,
+                          const int32_t* block_tables, const int32_t* context_lens,
+                          void* out, void* scratch,
+                          int batch, int q_len, int heads, int kv_heads, int head_dim,
+                          int block_size, int max_blocks_per_seq, int64_t num_blocks, float scale, void* stream);
+
 /* The same attention as the engine's prompt passes take it (tcgen05): any number of query rows, head_dim 64 or 128, a power
  * of two <= 16 query heads per key head, block_size a multiple of 64, num_blocks pages in the cache.  *gave_up (pinned host
  * memory) is set if one of the kernel's bounded waits ran out; the output is then not complete. */

@@ -656,38 +656,63 @@ static bool prompt_attn_ok(int H, int KV, int hd, int block_size, int64_t num_bl
   return (hd == 64 || hd == 128) && H % KV == 0 && G <= 16 && (G & (G - 1)) == 0 && H < 2048 && block_size % kPromptKeys == 0 &&
          num_blocks * block_size < (1ll << 31);
 }
+// Calls of few rows on the same tiles, their keys in ranges.  A tile holds all query heads of a key head for up to 128 rows, where paged_attn_kernel
+// reads the keys once per 32 rows and is bound by its instructions; it costs 2 us more to start.  us with the merge, 32-row tiles -> this one:
+// 7 rows x 8 query heads of 128 per key head, 8 x 8000 keys 106 -> 56, 4 x 2000 26 -> 19, 1 x 1000 12.7 -> 10.7, 1 x 500 9.8 -> 9.7, 1 x 200 9.5 -> 10.0;
+// 7 x 4, 8 x 8000 66 -> 52, 1 x 2000 13.5 -> 12.4, 1 x 1000 10.0 -> 10.7.  Up to 16 rows (one m16 tile) the instructions fit: 1 x 8, 8 x 8000 46 -> 51.
+// The line follows from the sizes of the call and the table alone, so that a sequence's result does not depend on what it is batched with.
+static bool attn_on_tiles(int H, int KV, int hd, int B, int Q, int block_size, int64_t num_blocks, int max_ctx) {
+  if (!prompt_attn_ok(H, KV, hd, block_size, num_blocks) || H / KV * Q <= 16) return false;
+  const int tokens = std::max(1, 32 / (H / KV));
+  return (int64_t)B * ((Q + tokens - 1) / tokens) * max_ctx >= 2000;
+}
+// ranges per sequence: three CTAs for two SMs (two are resident; 8 x 8000 keys 65.7 us with one per SM, 56.4, 58.7 with two)
+static int tile_splits(int H, int KV, int B, int Q, int max_ctx) {
+  const int tokens = kPromptRows / (H / KV), ctas = KV * B * ((Q + tokens - 1) / tokens);
+  return std::max(1, std::min({(3 * num_sms() + 2 * ctas - 1) / (2 * ctas), kAttnMaxSplit, (max_ctx + kPromptKeys - 1) / kPromptKeys}));
+}
 template <int HD>
 static int launch_prompt_attn(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const PromptAttnParams& p, int B) {
   static bool attr_set = false;
   if (!attr_set) {
-    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD)));
-    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD)));
+    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD)));
+    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     attr_set = true;
   }
-  const int tq = kPromptRows >> p.g_shift;
-  return L.go(prompt_attn_kernel<HD>, dim3(p.KV, (p.Q + tq - 1) / tq, B), dim3(kPromptThreads), (size_t)prompt_attn_smem(HD), tmQ, tmK, tmV, p);
+  const int tq = kPromptRows >> p.g_shift, nqt = (p.Q + tq - 1) / tq;
+  if (p.n_split > 1) return L.go(prompt_attn_kernel<HD, true>, dim3(p.KV, nqt, B * p.n_split), dim3(kPromptThreads), (size_t)prompt_attn_smem(HD), tmQ, tmK, tmV, p);
+  return L.go(prompt_attn_kernel<HD, false>, dim3(p.KV, nqt, B), dim3(kPromptThreads), (size_t)prompt_attn_smem(HD), tmQ, tmK, tmV, p);
 }
 // maps of queries, keys and values of layer caches of `slots` token slots: {box of a tile's query tokens, kPromptKeys keys of one head}
 static int enqueue_prompt_attention(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const int32_t* bt,
                                     const int32_t* ctx_lens, bf16* out, int B, int Q, int H, int KV, int hd, int block_size, int max_blocks,
-                                    int64_t slots, float scale, unsigned* timeout) {
+                                    int64_t slots, float scale, unsigned* timeout, int n_split = 1, float* part_o = nullptr, float* part_lse = nullptr) {
   PromptAttnParams p = {};
+  p.n_split = n_split; p.part_o = part_o; p.part_lse = part_lse;
   p.block_tables = bt; p.context_lens = ctx_lens; p.out = out; p.Q = Q; p.H = H; p.KV = KV; p.block_size = block_size; p.max_blocks = max_blocks;
   while ((KV << p.g_shift) < H) ++p.g_shift;
   p.n_slots = (int)slots;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.timeout = timeout;
-  return hd == 128 ? launch_prompt_attn<128>(L, tmQ, tmK, tmV, p, B) : launch_prompt_attn<64>(L, tmQ, tmK, tmV, p, B);
+  CKI(hd == 128 ? launch_prompt_attn<128>(L, tmQ, tmK, tmV, p, B) : launch_prompt_attn<64>(L, tmQ, tmK, tmV, p, B));
+  if (n_split > 1) {
+    AttnParams a = {};
+    a.context_lens = ctx_lens; a.out = out; a.part_o = part_o; a.part_lse = part_lse; a.B = B; a.Q = Q; a.H = H; a.KV = KV; a.TQ = kPromptRows >> p.g_shift; a.n_split = n_split;
+    CKI(L.go(attn_combine_kernel, dim3(B * Q * H), dim3(32), 0, a, hd));
+  }
+  return 0;
 }
 static int forward_prompt_attention(ssdk_engine* e, Launcher& L, const Model& m, const bf16* q, const bf16* kc, const bf16* vc, const int32_t* bt,
-                                    const int32_t* ctx_lens, bf16* out, int B, int Q, int block_size, int max_blocks, float scale) {
+                                    const int32_t* ctx_lens, bf16* out, int B, int Q, int block_size, int max_blocks, float scale, int n_split) {
   const int64_t slots = m.num_blocks * block_size;
   const int G = m.H / m.KV;
   const CUtensorMap *tmQ, *tmK, *tmV;
-  CKI(e->xmaps.get_heads(q, kMaxPass, m.H, m.hd, G, kPromptRows / G, &tmQ));
+  CKI(e->xmaps.get_heads(q, B * Q > kMaxTokens ? kMaxPass : kMaxTokens, m.H, m.hd, G, kPromptRows / G, &tmQ));
   CKI(e->xmaps.get_heads(kc, slots, m.KV, m.hd, 1, kPromptKeys, &tmK));
   CKI(e->xmaps.get_heads(vc, slots, m.KV, m.hd, 1, kPromptKeys, &tmV));
-  return enqueue_prompt_attention(L, *tmQ, *tmK, *tmV, bt, ctx_lens, out, B, Q, m.H, m.KV, m.hd, block_size, max_blocks, slots, scale, L.gave_up);
+  return enqueue_prompt_attention(L, *tmQ, *tmK, *tmV, bt, ctx_lens, out, B, Q, m.H, m.KV, m.hd, block_size, max_blocks, slots, scale, L.gave_up, n_split, e->ws.att_o, e->ws.att_lse);
 }
 
 static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w, int M, int epi, void* out, int ldo,
@@ -857,6 +882,9 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
 
   int TQ = 1, MT = 1, nqt = 1, nsplit = 1;
   CKI(attn_plan(m, f.B, f.Q, &TQ, &MT, &nqt, &nsplit, e->max_ctx_hint));
+  const bool att_tiles = e->use_prompt_attn && (M > kMaxTokens ? prompt_attn_ok(m.H, m.KV, m.hd, bs, m.num_blocks)
+                                                               : attn_on_tiles(m.H, m.KV, m.hd, f.B, f.Q, bs, m.num_blocks, e->max_ctx_hint));
+  if (att_tiles) nsplit = tile_splits(m.H, m.KV, f.B, f.Q, e->max_ctx_hint);
   if (M > kMaxTokens) nsplit = 1;   // (the partials are sized for kMaxTokens rows; so many q tiles fill the SMs by themselves)
   const float scale = 1.0f / sqrtf((float)m.hd);
 
@@ -916,8 +944,8 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
     CKI(launch_rope(L, M, rp));
 
     // ---- attention over the paged cache ----
-    if (e->use_prompt_attn && M > kMaxTokens && prompt_attn_ok(m.H, m.KV, m.hd, bs, m.num_blocks))
-      CKI(forward_prompt_attention(e, L, m, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, f.B, f.Q, bs, mb, scale));
+    if (att_tiles)
+      CKI(forward_prompt_attention(e, L, m, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, f.B, f.Q, bs, mb, scale, nsplit));
     else
       CKI(enqueue_attention(L, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, w.att_o,
                           w.att_lse, w.att_counters, f.B, f.Q, m.H, m.KV, m.hd, bs, mb, scale, TQ, MT, nqt, nsplit));
@@ -1270,6 +1298,7 @@ static int get_spec_graph(ssdk_engine* e, int B, bool host_io, bool stream_draft
   Launcher L;
   L.st = e->cap_stream;
   L.pdl = e->rt.use_pdl != 0;
+  L.gave_up = e->waits.word;
   cudaGraph_t graph = nullptr;
   CK(cudaStreamBeginCapture(e->cap_stream, cudaStreamCaptureModeThreadLocal));
   const int rc = enqueue_spec_step(e, L, B, host_io, !host_io, stream_draft);
@@ -1306,6 +1335,11 @@ static int init_kernel_attrs() {
   SSDK_ATTR_A(128, 1, 3) SSDK_ATTR_A(128, 2, 1) SSDK_ATTR_A(128, 2, 2) SSDK_ATTR_A(128, 4, 1) SSDK_ATTR_A(128, 4, 2)
   SSDK_ATTR_A(64, 1, 3) SSDK_ATTR_A(64, 2, 1) SSDK_ATTR_A(64, 2, 2) SSDK_ATTR_A(64, 4, 1) SSDK_ATTR_A(64, 4, 2)
 #undef SSDK_ATTR_A
+#define SSDK_ATTR_P(HD, SPLIT) \
+  CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD))); \
+  CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  SSDK_ATTR_P(64, false) SSDK_ATTR_P(64, true) SSDK_ATTR_P(128, false) SSDK_ATTR_P(128, true)
+#undef SSDK_ATTR_P
   CK(cudaFuncSetAttribute(add_rmsnorm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
   return 0;
 }
@@ -1565,6 +1599,7 @@ int ssdk_spec_step(ssdk_handle h, int batch, const int32_t* ctx_len, const int64
     Launcher L;
     L.st = st;
     L.pdl = h->rt.use_pdl != 0;
+    L.gave_up = h->waits.word;
     CKI(enqueue_spec_step(h, L, batch, true, false, stream_draft));
     h->launches += L.count;
   }
@@ -1604,6 +1639,7 @@ int ssdk_spec_step_resident(ssdk_handle h, int batch, void* stream) {
     Launcher L;
     L.st = st;
     L.pdl = h->rt.use_pdl != 0;
+    L.gave_up = h->waits.word;
     CKI(enqueue_spec_step(h, L, batch, false, true, stream_draft));
     h->launches += L.count;
   }
@@ -1872,6 +1908,28 @@ int ssdk_paged_attn(const void* q, const void* k_cache, const void* v_cache, con
   return enqueue_attention(L, (const bf16*)q, (const bf16*)k_cache, (const bf16*)v_cache, block_tables, context_lens,
                            (bf16*)out, part_o, part_lse, (unsigned*)scratch, batch, q_len, heads, kv_heads, head_dim, block_size,
                            max_blocks_per_seq, scale, TQ, MT, nqt, nsplit);
+}
+
+int ssdk_paged_attn_pages(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
+                          const int32_t* context_lens, void* out, void* scratch, int batch, int q_len, int heads, int kv_heads,
+                          int head_dim, int block_size, int max_blocks_per_seq, int64_t num_blocks, float scale, void* stream) {
+  const int max_ctx = block_size * max_blocks_per_seq;
+  if (batch * q_len > kMaxTokens || !(scale > 0.f) || (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) || num_blocks < 1 ||
+      !attn_on_tiles(heads, kv_heads, head_dim, batch, q_len, block_size, num_blocks, max_ctx))
+    return ssdk_paged_attn(q, k_cache, v_cache, block_tables, context_lens, out, scratch, batch, q_len, heads, kv_heads, head_dim, block_size,
+                           max_blocks_per_seq, scale, stream);
+  Launcher L;
+  L.st = (cudaStream_t)stream;
+  float* part_o = (float*)((uint8_t*)scratch + 16384);
+  float* part_lse = part_o + (size_t)batch * q_len * heads * kAttnMaxSplit * head_dim;
+  const int G = heads / kv_heads;
+  const int64_t slots = num_blocks * block_size;
+  CUtensorMap tmQ, tmK, tmV;
+  CKI(make_tmap_heads(&tmQ, q, (int64_t)batch * q_len, heads, head_dim, G, kPromptRows / G));
+  CKI(make_tmap_heads(&tmK, k_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
+  CKI(make_tmap_heads(&tmV, v_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
+  return enqueue_prompt_attention(L, tmQ, tmK, tmV, block_tables, context_lens, (bf16*)out, batch, q_len, heads, kv_heads, head_dim, block_size,
+                                  max_blocks_per_seq, slots, scale, nullptr, tile_splits(heads, kv_heads, batch, q_len, max_ctx), part_o, part_lse);
 }
 
 int ssdk_prompt_attn(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,

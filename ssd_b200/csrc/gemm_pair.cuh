@@ -85,7 +85,7 @@ SSDK_DEVINL bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, unsigned* tim
         : "memory");
     if (ok) return true;
     if (clock64() - t0 > 4000000000LL) {   // ~2 s
-      *(volatile unsigned*)timeout = 1u;
+      if (timeout) *(volatile unsigned*)timeout = 1u;
       return false;
     }
   }

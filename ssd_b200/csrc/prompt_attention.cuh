@@ -28,7 +28,12 @@ struct PromptAttnParams {
   int block_size, max_blocks;    // block_size a multiple of kPromptKeys
   int n_slots;                   // token slots of the cache: a chunk without a page is loaded from behind them (zeros)
   float scale_log2;              // > 0
-  unsigned* timeout;
+  unsigned* timeout;             // (nullptr: calls without an engine; rows whose waits ran out are NaN)
+  // SPLIT: the keys of a sequence in n_split ranges of whole chunks, as paged_attn_kernel cuts them; what a range gives goes to
+  // part_o [B*Q*H, n_split, hd] and part_lse [B*Q*H, n_split] (fp32, see attn_combine_kernel)
+  int n_split;
+  float* part_o;
+  float* part_lse;
 };
 
 // a whole warp's bounded wait: all of it goes on, or none
@@ -72,8 +77,8 @@ SSDK_DEVINL void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t* r) {
 }
 SSDK_DEVINL void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// grid (kv heads, q tiles, sequences)
-template <int HD>
+// grid (kv heads, q tiles, sequences x ranges)
+template <int HD, bool SPLIT>
 __global__ void __launch_bounds__(kPromptThreads, 2)
 prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                    const PromptAttnParams p) {
@@ -87,6 +92,11 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint8_t* sK = sQ + HALVES * kQHalf;
   uint8_t* sV = sK + kPromptStages * kTile;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kvh = blockIdx.x, qt = (int)gridDim.y - 1 - (int)blockIdx.y;   // (the tiles that see most keys first)
+  const int b = SPLIT ? (int)blockIdx.z / p.n_split : (int)blockIdx.z, split = SPLIT ? (int)blockIdx.z - b * p.n_split : 0;
+  const int G = 1 << p.g_shift, TQ = kPromptRows >> p.g_shift;
+  const int tok0 = qt * TQ, tq = min(TQ, p.Q - tok0);
+  const int live = SPLIT ? ((tq << p.g_shift) + 31) & ~31 : kPromptRows;   // rows of the warps that have some
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmQ);
@@ -95,7 +105,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     mbar_init(&q_full, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
-      mbar_init(&s_full[s], 1); mbar_init(&p_full[s], kPromptRows); mbar_init(&pv_done[s], 1);
+      mbar_init(&s_full[s], 1); mbar_init(&p_full[s], live); mbar_init(&pv_done[s], 1);
     }
     fence_mbar_init();
   }
@@ -108,12 +118,14 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   pdl_launch_dependents();
   pdl_wait();
 
-  const int kvh = blockIdx.x, qt = (int)gridDim.y - 1 - (int)blockIdx.y, b = blockIdx.z;   // (the tiles that see most keys first)
-  const int G = 1 << p.g_shift, TQ = kPromptRows >> p.g_shift;
-  const int tok0 = qt * TQ, tq = min(TQ, p.Q - tok0);
   const int ctx0 = p.context_lens[b] - p.Q;
   const int kv_max = ctx0 + tok0 + tq;               // exclusive upper bound of the keys the tile sees
-  const int n = (kv_max + kPromptKeys - 1) / kPromptKeys;
+  int n = (kv_max + kPromptKeys - 1) / kPromptKeys, first = 0;   // chunks of this CTA, and the first key of the first one
+  if (SPLIT) {   // (a range without chunks leaves no partial: the merge reads those that have some)
+    const int per = (n + p.n_split - 1) / p.n_split;
+    first = split * per * kPromptKeys;
+    n = max(0, min(per, n - split * per));
+  }
   // Every pair of barriers is used in turn, chunk i on barrier i & 1; parity(i) is that use's.  A wait by parity is only right while the barrier
   // is in that use or the one behind it.  pv_done: whoever waits for chunk j has seen s_full of chunk j + 1 or later (or issued its
   // scores), which was committed behind the product of chunk j - 1, and the product of chunk j + 2 needs the P that this thread (or this
@@ -122,13 +134,13 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   auto parity = [](int i) { return (uint32_t)(i >> 1) & 1u; };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (lane == 0 && n > 0) {
       mbar_arrive_expect_tx(&q_full, HALVES * kQHalf);
       for (int h = 0; h < HALVES; ++h) tma_load_3d(sQ + h * kQHalf, &tmQ, &q_full, h * 64, kvh << p.g_shift, b * p.Q + tok0);
       const int32_t* bt = p.block_tables + (size_t)b * p.max_blocks;
       int i = 0;
       for (; i < n; ++i) {
-        const int s = i & 1, base = i * kPromptKeys;
+        const int s = i & 1, base = first + i * kPromptKeys;
         const int blk = bt[base / p.block_size];
         const int slot = blk >= 0 ? blk * p.block_size + base % p.block_size : p.n_slots;
         if (!mbar_wait_cluster(&k_empty[s], parity(i) ^ 1u, p.timeout)) break;
@@ -185,9 +197,10 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const uint32_t lanes = (uint32_t)(q * 32) << 16;
     const int lim = min(ctx0 + tok0 + tok + 1, kv_max);   // keys this row sees (rows behind the tile's tokens: some, dropped)
     float m = -INFINITY, l = 0.f;
-    bool ok = true;
-    for (int i = 0; i < n; ++i) {
-      const int base = i * kPromptKeys;
+    const bool in = !SPLIT || q * 32 < live;   // (a warp without rows: what the products make of its lanes, nobody reads)
+    bool ok = in;
+    for (int i = 0; i < n && in; ++i) {
+      const int base = first + i * kPromptKeys;
       const uint32_t sp = tmem + lanes + (uint32_t)(i & 1) * 64u;
       if (!(ok = warp_wait(&s_full[i & 1], parity(i), p.timeout))) break;
       tc_fence_after();
@@ -240,7 +253,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (!(ok = warp_wait(&v_full[i & 1], parity(i), p.timeout))) break;
         const int from = kv_max - base, pieces = (kPromptKeys - from) * 8;   // 16-byte pieces per half (a row's stay in its 128 bytes)
         for (int h = 0; h < HALVES; ++h)
-          for (int j = r; j < pieces; j += kPromptRows)
+          for (int j = r; j < pieces; j += live)
             *reinterpret_cast<uint4*>(sV + (i & 1) * kTile + h * kKHalf + from * 128 + j * 16) = make_uint4(0u, 0u, 0u, 0u);
         fence_proxy_async_smem();
       }
@@ -248,11 +261,30 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       mbar_arrive(&p_full[i & 1]);
     }
     if (ok && n > 0) ok = warp_wait(&pv_done[(n - 1) & 1], parity(n - 1), p.timeout);
-    if (ok) {
-      tc_fence_after();
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-      const bool mine = tok < tq;
-      __nv_bfloat16* dst = p.out + ((size_t)(b * p.Q + tok0 + tok) * p.H + (kvh << p.g_shift) + (r & (G - 1))) * HD;
+    tc_fence_after();
+    const float inv = !ok ? __int_as_float(0x7fffffff) : l > 0.f ? 1.f / l : 0.f;   // NaN: a wait ran out
+    const bool mine = in && tok < tq;
+    const size_t row = (size_t)(b * p.Q + tok0 + tok) * p.H + (kvh << p.g_shift) + (r & (G - 1));
+    if (SPLIT) {
+      if (n > 0 && in) {
+        float* dst = p.part_o + (row * p.n_split + split) * HD;
+#pragma unroll 2
+        for (int c = 0; c < HD; c += 16) {
+          uint32_t o[16];
+          tmem_ld_32x32b_x16(tmem_o + lanes + c, o);
+          tmem_ld_wait();
+          float f[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(o[j]) * inv;
+          if (mine) {
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(dst + c + j) = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
+          }
+        }
+        if (mine) p.part_lse[row * p.n_split + split] = l > 0.f ? m + log2f(l) : -INFINITY;
+      }
+    } else {
+      __nv_bfloat16* dst = p.out + row * HD;
 #pragma unroll 2
       for (int c = 0; c < HD; c += 16) {
         uint32_t o[16];

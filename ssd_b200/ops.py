@@ -126,15 +126,15 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
     _req(context_lens, torch.int32, "context_lens")
     Mq, H, hd = q.shape
     B = Mq // q_len
-    _, block_size, KV, _ = k_cache.shape
+    num_blocks, block_size, KV, _ = k_cache.shape
     max_blocks = block_tables.shape[1]
     lib = _L.load()
     nbytes = lib.ssdk_paged_attn_scratch_bytes(B, q_len, H, hd, max_blocks * block_size)
     scratch = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
     out = torch.empty(Mq, H * hd, dtype=torch.bfloat16, device=q.device)
-    _L.check(lib.ssdk_paged_attn(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), _ptr(context_lens), _ptr(out),
-                                 _ptr(scratch), B, q_len, H, KV, hd, block_size, max_blocks, float(scale), _stream()),
-             "ssdk_paged_attn")
+    _L.check(lib.ssdk_paged_attn_pages(_ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), _ptr(context_lens), _ptr(out),
+                                       _ptr(scratch), B, q_len, H, KV, hd, block_size, max_blocks, num_blocks, float(scale), _stream()),
+             "ssdk_paged_attn_pages")
     return out
 
 
