@@ -30,8 +30,9 @@
 
 namespace ssdk {
 
-constexpr int kSplitTokens = 128, kSplitStages = 3, kSplitThreads = 320, kSplitSegment = 4;   // segment: k-blocks between two drains
-constexpr int kSplitWPlane = 128 * 128, kSplitXPlane = 64 * 128, kSplitStageBytes = 3 * (kSplitWPlane + kSplitXPlane);
+constexpr int kSplitTokens = 192, kSplitStages = 2, kSplitThreads = 512, kSplitSegment = 4;   // segment: k-blocks between two drains
+constexpr int kSplitXBox = 32;
+constexpr int kSplitWPlane = 128 * 128, kSplitXPlane = kSplitTokens / 2 * 128, kSplitStageBytes = 3 * (kSplitWPlane + kSplitXPlane);
 constexpr int kSplitSmem = kSplitStages * kSplitStageBytes + 1024;
 
 struct GemmSplitParams {
@@ -39,7 +40,7 @@ struct GemmSplitParams {
   float* out;         // [splits][M, ldc]
   int M, N, K, ldw, ldc;
   int num_kb, kb_per_split, splits;
-  int w_tiles, chunks;        // tiles of 256 columns; chunks of kSplitTokens rows (dense)
+  int w_tiles, chunks, tokens;   // tiles of 256 columns; dense: chunks of `tokens` rows (a multiple of 32, at most kSplitTokens)
   int batch;                  // dense: products of the same shape, their weights and results w_stride and c_stride floats apart, X's rows in turn
   int plane_rows;             // rows of one piece of X (the map holds three of them)
   const float* X;             // the rows themselves, for results that are taken again: row r of matrix b is row x_rows[r] (or r) from X + b x_stride
@@ -96,12 +97,18 @@ SSDK_DEVINL bool split_again(float v) {
   return u != 0u && u - lo >= hi - lo;
 }
 
+// registers of a warpgroup: 56 + 232 + 2 x 112 = 4 x 128, what the block is launched with
+template <int R>
+SSDK_DEVINL void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
+template <int R>
+SSDK_DEVINL void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
+
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSplitThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams p) {
   extern __shared__ uint8_t split_smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[kSplitStages];   // the leader's are used: the loads' bytes and four weight warps of both CTAs
+  __shared__ __align__(8) uint64_t full_bar[kSplitStages];   // the leader's are used: the loads' bytes and eight weight warps of both CTAs
   __shared__ __align__(8) uint64_t empty_bar[kSplitStages];
-  __shared__ __align__(8) uint64_t main_full[2], main_empty[2], rest_full[2], rest_empty[2];
+  __shared__ __align__(8) uint64_t main_full, main_empty, rest_full, rest_empty;
   __shared__ uint32_t tmem_slot;
   __shared__ int s_again;   // some result of this CTA's is to be taken again
   uint8_t* smem = split_smem_raw + ((1024u - (smem_u32(split_smem_raw) & 1023u)) & 1023u);
@@ -112,8 +119,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmX);
-    for (int s = 0; s < kSplitStages; ++s) { mbar_init(&full_bar[s], 9); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&main_full[b], 1); mbar_init(&main_empty[b], 8); mbar_init(&rest_full[b], 1); mbar_init(&rest_empty[b], 8); }
+    for (int s = 0; s < kSplitStages; ++s) { mbar_init(&full_bar[s], 17); mbar_init(&empty_bar[s], 1); }
+    mbar_init(&main_full, 1); mbar_init(&main_empty, 8); mbar_init(&rest_full, 1); mbar_init(&rest_empty, 8);   // four sum warps in each CTA
     fence_mbar_init();
     s_again = 0;
   }
@@ -122,7 +129,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
   __syncthreads();
   cluster_sync_all();
   tc_fence_after();
-  const uint32_t tmem_main = tmem_slot, tmem_rest = tmem_slot + 256u;   // two accumulators of 128 columns each
+  const uint32_t tmem_main = tmem_slot, tmem_rest = tmem_slot + 256u;
 
   pdl_launch_dependents();
   pdl_wait();
@@ -140,7 +147,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
     if (grouped) {
       r.m0 = p.g_tile_row0[c]; r.rows = min(kSplitTokens, p.g_tile_rows[c]); r.w0 = p.g_tile_expert[c] * p.w_stride;
     } else {
-      r.m0 = c * kSplitTokens; r.rows = min(kSplitTokens, p.M - r.m0); r.w0 = r.b * p.w_stride;
+      r.m0 = c * p.tokens; r.rows = min(p.tokens, p.M - r.m0); r.w0 = r.b * p.w_stride;
     }
     r.n = (r.rows + 31) & ~31;
     r.col = wt * 256 + (int)rank * 128;
@@ -149,64 +156,69 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
     return r;
   };
 
-  if (warp == 0) {
-    if (lane == 0) {
+  if (warp < 4) {
+    regs_down<56>();
+    if (warp == 0 && lane == 0) {
       int it = 0;
       bool ok = true;
       for (int t = pair; t < tiles && ok; t += n_pairs) {
         const Tile tl = tile_of(t);
-        const int x0 = tl.b * p.M + tl.m0 + (int)rank * (tl.n >> 1);
+        const int half = tl.n >> 1, x0 = tl.b * p.M + tl.m0 + (int)rank * half, boxes = (half + kSplitXBox - 1) / kSplitXBox;
         for (int kb = tl.kb0; kb < tl.kb1; ++kb, ++it) {
           const int s = it % kSplitStages;
           if (!(ok = mbar_wait_cluster(&empty_bar[s], ((uint32_t)(it / kSplitStages) & 1u) ^ 1u, p.timeout))) break;
           uint8_t* b_s = smem + s * kSplitStageBytes + 3 * kSplitWPlane;
-          if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2u * 3u * kSplitXPlane);
+          if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2u * 3u * (uint32_t)boxes * kSplitXBox * 128u);
           const uint32_t bar = map_shared(&full_bar[s], 0);
+          for (int i = 0; i < boxes; ++i)
 #pragma unroll
-          for (int j = 0; j < 3; ++j) tma_load_2d_pair(b_s + j * kSplitXPlane, &tmX, bar, kb * kBlockK, j * p.plane_rows + x0, kEvictNormal);
+            for (int j = 0; j < 3; ++j)
+              tma_load_2d_pair(b_s + j * kSplitXPlane + i * kSplitXBox * 128, &tmX, bar, kb * kBlockK, j * p.plane_rows + x0 + i * kSplitXBox, kEvictNormal);
         }
       }
       for (int i = 0; i < kSplitStages && ok; ++i, ++it)   // the last commits reach this CTA before it leaves
         ok = mbar_wait_cluster(&empty_bar[it % kSplitStages], ((uint32_t)(it / kSplitStages) & 1u) ^ 1u, p.timeout);
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    } else if (warp == 1 && lane == 0 && rank == 0) {
       int it = 0, nt = 0, sg = 0;
       bool ok = true;
       for (int t = pair; t < tiles && ok; t += n_pairs, ++nt) {
         const Tile tl = tile_of(t);
-        const uint32_t idesc = make_umma_idesc_bf16(256, tl.n), rest = tmem_rest + (uint32_t)(nt & 1) * 128u;
-        if (!(ok = mbar_wait_cluster(&rest_empty[nt & 1], ((uint32_t)(nt >> 1) & 1u) ^ 1u, p.timeout))) break;
+        const uint32_t idesc = make_umma_idesc_bf16(256, tl.n);
+        if (!(ok = mbar_wait_cluster(&rest_empty, ((uint32_t)nt & 1u) ^ 1u, p.timeout))) break;
         for (int kb = tl.kb0; kb < tl.kb1; ++kb, ++it) {
-          const int in_seg = (kb - tl.kb0) % kSplitSegment;
-          if (in_seg == 0 && !(ok = mbar_wait_cluster(&main_empty[sg & 1], ((uint32_t)(sg >> 1) & 1u) ^ 1u, p.timeout))) break;
-          const int s = it % kSplitStages;
+          const int in_seg = (kb - tl.kb0) % kSplitSegment, s = it % kSplitStages;
           if (!(ok = mbar_wait_cluster(&full_bar[s], (uint32_t)(it / kSplitStages) & 1u, p.timeout))) break;
           tc_fence_after();
           uint8_t* a_s = smem + s * kSplitStageBytes;
           uint64_t wd[3], xd[3];
 #pragma unroll
           for (int j = 0; j < 3; ++j) { wd[j] = make_umma_desc_k128(a_s + j * kSplitWPlane); xd[j] = make_umma_desc_k128(a_s + 3 * kSplitWPlane + j * kSplitXPlane); }
-          const uint32_t acc = tmem_main + (uint32_t)(sg & 1) * 128u;
+          // the small terms first: the sums of the segment before are fetched from their accumulator meanwhile
 #pragma unroll
           for (int k = 0; k < kBlockK / 16; ++k) {
             const uint64_t o = (uint64_t)(2 * k);
-            umma_bf16_ss_pair(acc, wd[0] + o, xd[0] + o, idesc, (uint32_t)((in_seg | k) != 0));
-            umma_bf16_ss_pair(rest, wd[0] + o, xd[1] + o, idesc, (uint32_t)(((kb - tl.kb0) | k) != 0));
-            umma_bf16_ss_pair(rest, wd[1] + o, xd[0] + o, idesc, 1u);
-            umma_bf16_ss_pair(rest, wd[1] + o, xd[1] + o, idesc, 1u);
-            umma_bf16_ss_pair(rest, wd[0] + o, xd[2] + o, idesc, 1u);
-            umma_bf16_ss_pair(rest, wd[2] + o, xd[0] + o, idesc, 1u);
+            umma_bf16_ss_pair(tmem_rest, wd[0] + o, xd[1] + o, idesc, (uint32_t)(((kb - tl.kb0) | k) != 0));
+            umma_bf16_ss_pair(tmem_rest, wd[1] + o, xd[0] + o, idesc, 1u);
+            umma_bf16_ss_pair(tmem_rest, wd[1] + o, xd[1] + o, idesc, 1u);
+            umma_bf16_ss_pair(tmem_rest, wd[0] + o, xd[2] + o, idesc, 1u);
+            umma_bf16_ss_pair(tmem_rest, wd[2] + o, xd[0] + o, idesc, 1u);
           }
+          if (in_seg == 0) {
+            if (!(ok = mbar_wait_cluster(&main_empty, ((uint32_t)sg & 1u) ^ 1u, p.timeout))) break;
+            tc_fence_after();
+          }
+#pragma unroll
+          for (int k = 0; k < kBlockK / 16; ++k)
+            umma_bf16_ss_pair(tmem_main, wd[0] + (uint64_t)(2 * k), xd[0] + (uint64_t)(2 * k), idesc, (uint32_t)((in_seg | k) != 0));
           umma_commit_pair(&empty_bar[s]);
-          if (in_seg == kSplitSegment - 1 || kb + 1 == tl.kb1) { umma_commit_pair(&main_full[sg & 1]); ++sg; }
+          if (in_seg == kSplitSegment - 1 || kb + 1 == tl.kb1) { umma_commit_pair(&main_full); ++sg; }
         }
-        if (ok) umma_commit_pair(&rest_full[nt & 1]);
+        if (ok) umma_commit_pair(&rest_full);
       }
     }
     __syncwarp();
-  } else if (warp < 6) {
+  } else if (warp < 8) {
+    regs_up<232>();
     const int q = warp & 3;
     int nt = 0, sg = 0;
     bool ok = true;
@@ -218,14 +230,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
       auto add = [&](uint32_t src) {
         src += (uint32_t)(q * 32) << 16;
 #pragma unroll
-        for (int c = 0; c < kSplitTokens / 32; ++c) {
-          if (c * 32 < tl.n) {
-            uint32_t r[32];
-            tmem_ld_32x32b_x16(src + c * 32, r);
-            tmem_ld_32x32b_x16(src + c * 32 + 16, r + 16);
+        for (int c = 0; c < kSplitTokens / 16; ++c) {
+          if (c * 16 < tl.n) {
+            uint32_t r[16];
+            tmem_ld_32x32b_x16(src + c * 16, r);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) acc[c * 32 + i] += __uint_as_float(r[i]);
+            for (int i = 0; i < 16; ++i) acc[c * 16 + i] += __uint_as_float(r[i]);
           }
         }
         tc_fence_before();
@@ -233,15 +244,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
       };
       const int segs = (tl.kb1 - tl.kb0 + kSplitSegment - 1) / kSplitSegment;
       for (int g = 0; g < segs; ++g, ++sg) {
-        if (!(ok = mbar_wait_cluster(&main_full[sg & 1], (uint32_t)(sg >> 1) & 1u, p.timeout))) break;
+        if (!(ok = mbar_wait_cluster(&main_full, (uint32_t)sg & 1u, p.timeout))) break;
         tc_fence_after();
-        add(tmem_main + (uint32_t)(sg & 1) * 128u);
-        if (lane == 0) mbar_arrive_cluster(map_shared(&main_empty[sg & 1], 0));
+        add(tmem_main);
+        if (lane == 0) mbar_arrive_cluster(map_shared(&main_empty, 0));
       }
-      if (!ok || !(ok = mbar_wait_cluster(&rest_full[nt & 1], (uint32_t)(nt >> 1) & 1u, p.timeout))) break;
+      if (!ok || !(ok = mbar_wait_cluster(&rest_full, (uint32_t)nt & 1u, p.timeout))) break;
       tc_fence_after();
-      add(tmem_rest + (uint32_t)(nt & 1) * 128u);
-      if (lane == 0) mbar_arrive_cluster(map_shared(&rest_empty[nt & 1], 0));
+      add(tmem_rest);
+      if (lane == 0) mbar_arrive_cluster(map_shared(&rest_empty, 0));
       const int n = tl.col + q * 32 + lane;
       if (n < p.N) {
         float* out = p.out + tl.b * p.c_stride + ((size_t)tl.split * p.M + tl.m0) * p.ldc + n;
@@ -254,53 +265,58 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
     }
     __syncwarp();
   } else {
-    // lane: row lane / 8 of four, eight floats from column 8 (lane % 8) of the k-block; eight steps cover the warp's 32 rows
-    const int cw = warp - 6, r4 = lane >> 3, piece = lane & 7;
-    float4 v[16];
-    auto load = [&](const Tile& tl, int kb, int i) {
-      const int row = tl.col + cw * 32 + i * 4 + r4, k = kb * kBlockK + piece * 8;
-      const bool in = row < p.N && k < p.K;
-      const float4* src = reinterpret_cast<const float4*>(p.W + tl.w0 + (long long)row * p.ldw + k);
-      v[2 * i] = in ? __ldg(src) : make_float4(0.f, 0.f, 0.f, 0.f);
-      v[2 * i + 1] = in ? __ldg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+    regs_down<112>();
+    // lane: row lane / 8 of four, eight floats from column 8 (lane % 8) of the k-block; four steps cover the warp's 16 rows
+    const int r0 = (warp - 8) * 16 + (lane >> 3), piece = lane & 7;
+    const float* src[4];   // this thread's four weight rows of the tile whose loads are asked for
+    auto rows_of = [&](const Tile& tl) {   // (rows behind the matrix: the last one's, whose results nobody takes)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) src[i] = p.W + tl.w0 + (long long)min(tl.col + r0 + i * 4, p.N - 1) * p.ldw + piece * 8;
+    };
+    float4 v[8];
+    auto load = [&](int kb, int i) {
+      const bool in = kb * kBlockK + piece * 8 < p.K;
+      const float4* at = reinterpret_cast<const float4*>(src[i] + kb * kBlockK);
+      v[2 * i] = in ? __ldg(at) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[2 * i + 1] = in ? __ldg(at + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     int it = 0, t = pair, kb = 0;
     Tile tl = {};
     if (t < tiles) {
       tl = tile_of(t);
       kb = tl.kb0;
+      rows_of(tl);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) load(tl, kb, i);
+      for (int i = 0; i < 4; ++i) load(kb, i);
     }
     bool ok = true;
     while (t < tiles && ok) {
-      Tile nx = tl;   // the k-block after this one
-      int t2 = t, kb2 = kb + 1;
+      int t2 = t, kb2 = kb + 1;   // the k-block after this one
       if (kb2 >= tl.kb1) {
         t2 += n_pairs;
-        if (t2 < tiles) { nx = tile_of(t2); kb2 = nx.kb0; }
+        if (t2 < tiles) { tl = tile_of(t2); kb2 = tl.kb0; rows_of(tl); }
       }
       const int s = it % kSplitStages;
       if (!(ok = mbar_wait_cluster(&empty_bar[s], ((uint32_t)(it / kSplitStages) & 1u) ^ 1u, p.timeout))) break;
       uint8_t* a_s = smem + s * kSplitStageBytes;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int row = cw * 32 + i * 4 + r4;
+      for (int i = 0; i < 4; ++i) {
+        const int row = r0 + i * 4;
         uint4 h, m, l;
         split3(v[2 * i].x, v[2 * i].y, h.x, m.x, l.x);
         split3(v[2 * i].z, v[2 * i].w, h.y, m.y, l.y);
         split3(v[2 * i + 1].x, v[2 * i + 1].y, h.z, m.z, l.z);
         split3(v[2 * i + 1].z, v[2 * i + 1].w, h.w, m.w, l.w);
+        if (t2 < tiles) load(kb2, i);
         uint8_t* dst = a_s + row * 128 + ((piece ^ (row & 7)) << 4);
         *reinterpret_cast<uint4*>(dst) = h;
         *reinterpret_cast<uint4*>(dst + kSplitWPlane) = m;
         *reinterpret_cast<uint4*>(dst + 2 * kSplitWPlane) = l;
-        if (t2 < tiles) load(nx, kb2, i);
       }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_shared(&full_bar[s], 0));
-      ++it; t = t2; kb = kb2; tl = nx;
+      ++it; t = t2; kb = kb2;
     }
     __syncwarp();
   }

@@ -550,21 +550,34 @@ struct HybRun {
     if ((size_t)m * batch * K > e->piece_elems || batch > 65535) return false;
     return e->use_split > 1 || 2.0 * m * N * K * batch >= 4e8 || K >= 512;
   }
+  // rows of a chunk and k ranges (of whole segments, summed in order behind the product) of a dense call: the fewest clocks over the rounds that the
+  // pairs of CTAs take.  A k-block takes 3100 clocks and 7.5 per token (measured, 960 x 4096 x 2048: 3800, 4090, 4410, 4520 at 96, 128, 160, 192 tokens), a
+  // tile 5000 to start and drain; the sum of the ranges a launch and its traffic.
+  static int split_plan(GemmSplitParams& p, size_t partial_floats) {
+    double best = 0;
+    const int pairs = num_sms() / 2;
+    for (int tok = kSplitTokens; tok >= 32; tok -= 32) {
+      const int chunks = (p.M + tok - 1) / tok, tiles = p.w_tiles * chunks * p.batch;
+      for (int s = 1; s <= 8; ++s) {
+        const int per = ((p.num_kb + s - 1) / s + kSplitSegment - 1) / kSplitSegment * kSplitSegment, S = (p.num_kb + per - 1) / per;
+        if (S != s || (S > 1 && (p.batch > 1 || (size_t)S * p.M * p.N > partial_floats))) continue;
+        double cost = (double)((tiles * S + pairs - 1) / pairs) * (std::min(per, p.num_kb) * (3100.0 + 7.5 * tok) + 5000.0);
+        if (S > 1) cost += 5000.0 + (S + 1) * (double)p.M * p.N * 4 / 1600;
+        if (best == 0 || cost < best) { best = cost; p.tokens = tok; p.chunks = chunks; p.kb_per_split = per; p.splits = S; }
+      }
+    }
+    return p.chunks;
+  }
   int go_split(const void* A, int lda, long long sA, const int* gather, const int* n_rows, int m, int batch, GemmSplitParams& p, int row_tiles) {
     CKI(L.go(ssdk::split_rows_kernel, dim3(m, batch), dim3(std::min(256, (p.K / 4 + 31) / 32 * 32)), 0, (const float*)A, lda, sA, gather, n_rows, (bf16*)e->pieces, p.K));
     const CUtensorMap* tm;
-    CKI(e->tmap(e->pieces, 3LL * m * batch, p.K, 64, &tm));
+    CKI(e->tmap(e->pieces, 3LL * m * batch, p.K, kSplitXBox, &tm));
     p.X = (const float*)A; p.ldx = lda; p.x_stride = sA; p.x_rows = gather;
     p.M = m; p.plane_rows = m * batch; p.batch = batch; p.num_kb = (p.K + kBlockK - 1) / kBlockK; p.w_tiles = (p.N + 255) / 256;
+    p.kb_per_split = (p.num_kb + kSplitSegment - 1) / kSplitSegment * kSplitSegment;
+    p.splits = 1;
+    if (!p.g_tile_expert) row_tiles = split_plan(p, p.ldc == p.N ? e->partial_floats : 0);
     const int tiles = p.w_tiles * row_tiles * batch;
-    // few tiles: k ranges of whole segments (dense results only; summed in the order of the ranges)
-    int S = 1;
-    if (!p.g_tile_expert && batch == 1 && p.ldc == p.N) {
-      S = std::max(1, std::min({num_sms() / 2 / tiles, p.num_kb / kSplitSegment, 8}));
-      while (S > 1 && (size_t)S * m * p.N > e->partial_floats) --S;
-    }
-    p.kb_per_split = ((p.num_kb + S - 1) / S + kSplitSegment - 1) / kSplitSegment * kSplitSegment;
-    p.splits = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;
     float* C = p.out;
     if (p.splits > 1) p.out = e->partials;
     CKI(launch_gemm_split(L, *tm, p, tiles * p.splits));
@@ -588,8 +601,7 @@ struct HybRun {
     if (split_ok(A, lda, W, ldw, m, N, K, batch, sA, sW)) {
       GemmSplitParams p = {};
       p.W = (const float*)W; p.out = (float*)C; p.N = N; p.K = K; p.ldw = ldw; p.ldc = ldc; p.w_stride = sW; p.c_stride = sC;
-      p.chunks = (m + kSplitTokens - 1) / kSplitTokens;
-      return go_split(A, lda, sA, nullptr, nullptr, m, batch, p, p.chunks);
+      return go_split(A, lda, sA, nullptr, nullptr, m, batch, p, 0);
     }
     ssdk::LinearArgs a = {};
     a.A = A; a.W = W; a.C = C; a.M = m; a.N = N; a.K = K; a.lda = lda; a.ldw = ldw; a.ldc = ldc;
