@@ -6,6 +6,7 @@
 #include "conv_scan.cuh"
 #include "gqa_attention.cuh"
 #include "gqa_mma.cuh"
+#include "gqa_prompt.cuh"
 #include "latent_attention.cuh"
 #include "layer_ops.cuh"
 #include "linear.cuh"
@@ -793,6 +794,37 @@ struct HybRun {
     }
   }
 
+  // prompt portions on tcgen05: keys in whole chunks of a page, a key head's query heads fill tiles.  Whole prompts, us, mma.sync tiles -> these, one layer:
+  // kefurax m 24 tokens 194 -> 195, 200 317 -> 310, 800 544 -> 525; vegilix m 24 228 -> 228, 200 326 -> 322, 800 409 -> 386; 2000 633 -> 543
+  bool gqa_on_tiles(const HybLayer& Lr, const float* gate, int ld_gate) const {
+    const ssdk_hyb_layer_cfg& c = Lr.c;
+    const int hpg = c.heads / c.kv_heads;
+    auto whole = [](int d) { return d == 64 || d == 128; };
+    return c.attn_scale > 0.f && e->cfg.block_size % ssdk::kPromptKeys == 0 && (hpg & (hpg - 1)) == 0 && hpg <= 16 && whole(c.vdim) && (c.maps == 2 ? c.dim == 64 : whole(c.dim)) &&
+           e->num_blocks * e->cfg.block_size < (1ll << 31) && (int64_t)M * c.heads * c.maps < (1ll << 31) && whole16(gate ? ld_gate : 4, {gate});
+  }
+  template <int DK, int VD, int MAPS>
+  int gqa_prompt_go(const CUtensorMap& tmQ, const CUtensorMap& tmKV, const ssdk::GqaPromptArgs& a, int n_max) {
+    const int tile = ssdk::kPromptRows / MAPS;
+    return L.go(ssdk::gqa_prompt_kernel<DK, VD, MAPS>, dim3(((n_max << a.g_shift) + tile - 1) / tile, a.G / MAPS, rg.n_seqs), dim3(ssdk::kPromptThreads),
+                (size_t)ssdk::gqa_prompt_smem(DK, VD), tmQ, tmKV, a, rg);
+  }
+  int gqa_prompt(const HybLayer& Lr, int n_max, const void* pool, void* y, const float* gate, int ld_gate, const void* sinks, float sink_const, const ssdk::DiffArgs& diff) {
+    const ssdk_hyb_layer_cfg& c = Lr.c;
+    ssdk::GqaPromptArgs a = {};
+    a.y = y; a.gate = gate; a.ld_gate = ld_gate; a.G = c.kv_heads * c.maps; a.D = c.dim;
+    while ((c.kv_heads << a.g_shift) < c.heads) ++a.g_shift;
+    a.scale_log2 = c.attn_scale * ssdk::kLog2e; a.sink = sink_const; a.sinks = sinks; a.mask = ssdk::KeyMask{c.window, c.chunk, c.keep_first}; a.diff = diff; a.timeout = L.gave_up;
+    const CUtensorMap* tm;   // (copied: a later lookup may empty the table)
+    CKI(e->tmap(e->qcat, (int64_t)M * c.heads * c.maps, c.dim, ssdk::kPromptRows / c.maps, &tm));
+    const CUtensorMap tmQ = *tm;
+    CKI(e->tmap(pool, e->num_blocks * e->cfg.block_size, (int)Lr.cache_row, ssdk::kPromptKeys, &tm));
+    const CUtensorMap tmKV = *tm;
+    if (c.maps == 2) return c.vdim == 128 ? gqa_prompt_go<128, 128, 2>(tmQ, tmKV, a, n_max) : gqa_prompt_go<128, 64, 2>(tmQ, tmKV, a, n_max);
+    if (c.dim == 128) return c.vdim == 128 ? gqa_prompt_go<128, 128, 1>(tmQ, tmKV, a, n_max) : gqa_prompt_go<128, 64, 1>(tmQ, tmKV, a, n_max);
+    return c.vdim == 128 ? gqa_prompt_go<64, 128, 1>(tmQ, tmKV, a, n_max) : gqa_prompt_go<64, 64, 1>(tmQ, tmKV, a, n_max);
+  }
+
   int latent(HybLayer& Lr) {
     const ssdk_hyb_layer_cfg& c = Lr.c;
     const int H = c.heads, D = c.dim, V = c.vdim, R = c.rot_dim, KR = c.kv_rank, QR = c.q_rank, W = e->cfg.width;
@@ -1250,7 +1282,9 @@ struct HybRun {
     if (mma) {   // all portions in one launch
       int n_max = 0;
       for (int s = 0; s < rg.n_seqs; ++s) n_max = std::max(n_max, h_cu[s + 1] - h_cu[s]);
-      if (n_max > 1) {
+      if (n_max > 1 && gqa_on_tiles(Lr, gate, ld_gate)) {
+        CKI(gqa_prompt(Lr, n_max, pool, y, gate, ld_gate, sinks, sink_const, diff));
+      } else if (n_max > 1) {
         ssdk::GqaPortionArgs fa;
         fa.q = e->qcat; fa.cache = pool; fa.y = y; fa.gate = gate; fa.ld_gate = ld_gate; fa.H = H; fa.G = G; fa.D = D; fa.V = V;
         fa.scale = c.attn_scale; fa.sink = sink_const; fa.sinks = sinks; fa.mask = mask; fa.diff = diff;
@@ -1734,6 +1768,11 @@ static int hyb_smem_attrs(ssdk_hyb_engine* e) {
   CK(cudaFuncSetAttribute(ssdk::gqa_portion_mma_kernel<2, 4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   CK(cudaFuncSetAttribute(ssdk::gqa_portion_mma_kernel<4, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   CK(cudaFuncSetAttribute(ssdk::gqa_portion_mma_kernel<8, 16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+#define SSDK_TILE_ATTR(DK, VD, MAPS) \
+  CK(cudaFuncSetAttribute(ssdk::gqa_prompt_kernel<DK, VD, MAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, ssdk::gqa_prompt_smem(DK, VD))); \
+  CK(cudaFuncSetAttribute(ssdk::gqa_prompt_kernel<DK, VD, MAPS>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  SSDK_TILE_ATTR(128, 128, 2) SSDK_TILE_ATTR(128, 64, 2) SSDK_TILE_ATTR(128, 128, 1) SSDK_TILE_ATTR(128, 64, 1) SSDK_TILE_ATTR(64, 128, 1) SSDK_TILE_ATTR(64, 64, 1)
+#undef SSDK_TILE_ATTR
 #define SSDK_RET_ATTR(KS, VT) \
   CK(cudaFuncSetAttribute(ssdk::retention_chunk_state_mma_kernel<KS, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, big)); \
   CK(cudaFuncSetAttribute(ssdk::retention_chunk_out_mma_kernel<KS, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
