@@ -65,7 +65,7 @@ struct ssdk_hyb_engine {
   void *ey = nullptr, *sy = nullptr, *xs = nullptr;   // xs: routed rows gathered per expert (grouped tcgen05 GEMM)
   int *sel = nullptr, *apos = nullptr, *arow = nullptr, *tile_expert = nullptr, *tile_row0 = nullptr, *tile_rows = nullptr,
       *n_tiles = nullptr, *n_rows = nullptr;
-  void* hn = nullptr; float* logits = nullptr; bf16* logits16 = nullptr; int64_t* tokens = nullptr;
+  void* hn = nullptr; float* logits = nullptr;
   int* meta = nullptr; size_t meta_ints = 0;
   int max_tiles = 0;
   // widths of the shared buffers (elements per row)
@@ -384,9 +384,7 @@ static int64_t hyb_carve(ssdk_hyb_engine* e, uint8_t* base) {
   const size_t lr = g.max_logit_rows;
   e->hn = take(lr * g.width * es);
   e->logits = (float*)take(lr * g.vocab * 4);
-  e->logits16 = (bf16*)take(lr * g.vocab * 2);
-  e->tokens = (int64_t*)take(lr * 8);
-  e->meta_ints = 4 + 2 * cap + 3 * (size_t)g.max_seqs + 1 + (size_t)g.max_seqs * g.max_blocks_per_seq + 2 * lr;
+  e->meta_ints = 6 + 2 * cap + 3 * (size_t)g.max_seqs + 1 + (size_t)g.max_seqs * g.max_blocks_per_seq + 2 * lr;
   e->meta = (int*)take(e->meta_ints * 4);
   // split-K partials of the tcgen05 GEMMs: up to 8 splits of a 256-row call of the widest output, bounded at 64 MB
   size_t widest = std::max<size_t>(g.vocab, g.width);
@@ -1817,11 +1815,18 @@ static int hyb_forward_t(ssdk_hyb_engine* e, int n_seqs, int M, const int32_t* i
   void* scr = nullptr;
   const bool sample = temps && out_tokens && n_want > 0;
   if (sample) CKI(op_scratch(&scr, st));
-  // stage the step's numbers: seed, step | ids | tok_seq | cu | pos0 | slot | tables | want_rows | temperatures
+  // sampled rows: the sampler, which reads all logits, also takes them to pinned host memory (other memory: a copy behind it)
+  float* logits_dev = nullptr;
+  if (sample && logits_host) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, logits_host) == cudaSuccess && at.type == cudaMemoryTypeHost) logits_dev = (float*)at.devicePointer;
+    else (void)cudaGetLastError();
+  }
+  // stage the step's numbers: seed, step, where the logits go | ids | tok_seq | cu | pos0 | slot | tables | want_rows | temperatures
   int* hm = e->h_meta;
   int* d = e->meta;
   size_t o = 0;
-  memcpy(hm + o, &seed, 8); memcpy(hm + o + 2, &step_id, 8); o += 4;
+  memcpy(hm + o, &seed, 8); memcpy(hm + o + 2, &step_id, 8); memcpy(hm + o + 4, &logits_dev, 8); o += 6;
   const size_t o_ids = o; memcpy(hm + o, ids, (size_t)M * 4); o += M;
   const size_t o_seq = o;
   for (int s = 0; s < n_seqs; ++s)
@@ -1868,18 +1873,14 @@ static int hyb_forward_t(ssdk_hyb_engine* e, int n_seqs, int M, const int32_t* i
     else CKI(run.rmsnorm(e->x, e->final_norm.p, e->hn, d + o_want, n_want, g.norm_offset));
     CKI(run.lin(e->hn, g.width, e->head.p, g.width, e->logits, g.vocab, n_want, g.vocab, g.width));
     if (!sample) return 0;
-    const size_t n = (size_t)n_want * g.vocab;
-    CKI(run.L.go(ssdk::f32_to_bf16_kernel, dim3((unsigned)std::min<size_t>((n + 255) / 256, 8192)), dim3(256), 0, (const float*)e->logits,
-                 e->logits16, n));
     for (int r0 = 0; r0 < n_want; r0 += 256) {
       const int nb = std::min(256, n_want - r0);
       SampleParams sp;
-      sp.logits = e->logits16 + (size_t)r0 * g.vocab; sp.ld = g.vocab; sp.temps = (const float*)(d + o_temp) + r0; sp.V = g.vocab; sp.seed = seed;
-      sp.call_id = step_id; sp.out = e->tokens + r0; sp.out_stride = 1; sp.counters = (unsigned*)scr;
+      sp.logits = nullptr; sp.ld = g.vocab; sp.logits32 = e->logits + (size_t)r0 * g.vocab; sp.copy_to = (float* const*)(d + 4); sp.copy_row = r0; sp.temps = (const float*)(d + o_temp) + r0; sp.V = g.vocab; sp.seed = seed;
+      sp.call_id = step_id; sp.out = e->h_tokens + r0; sp.out_stride = 1; sp.counters = (unsigned*)scr;
       sp.partial = (ArgMax*)((uint8_t*)scr + 4096); sp.dyn = (const uint64_t*)d; sp.sub = -1;
       CKI(run.L.go(sample_kernel, dim3(kSampleChunks, nb), dim3(256), 0, sp));
     }
-    CK(cudaMemcpyAsync(e->h_tokens, e->tokens, (size_t)n_want * 8, cudaMemcpyDeviceToHost, on));
     return 0;
   };
   // Decode steps (one token per sequence) are a hundred launches of a few microseconds, which the host issues slower than the GPU runs
@@ -1916,7 +1917,7 @@ static int hyb_forward_t(ssdk_hyb_engine* e, int n_seqs, int M, const int32_t* i
     e->launches += run.L.count;
     if (hg) hg->plain = run.by_position ? 0 : hg->plain + 1;
   }
-  if (logits_host && n_want > 0) CK(cudaMemcpyAsync(logits_host, e->logits, (size_t)n_want * g.vocab * 4, cudaMemcpyDeviceToHost, st));
+  if (logits_host && n_want > 0 && !logits_dev) CK(cudaMemcpyAsync(logits_host, e->logits, (size_t)n_want * g.vocab * 4, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   if (sample) memcpy(out_tokens, e->h_tokens, (size_t)n_want * 8);
   return e->waits.check();

@@ -393,13 +393,6 @@ __global__ void tanh_rows_kernel(const float* __restrict__ z, T* __restrict__ y,
     st_f<T>(y + i, tanhf(z[i]));
 }
 
-__global__ void f32_to_bf16_kernel(const float* __restrict__ z, __nv_bfloat16* __restrict__ y, size_t n) {
-  pdl_launch_dependents();
-  pdl_wait();
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    y[i] = __float2bfloat16_rn(z[i]);
-}
-
 // out[i] = sum over s of partials[s][i] in the fixed order s = 0 .. S-1 (split-K of the tcgen05 GEMM, fp32)
 __global__ void splitk_sum_kernel(const float* __restrict__ partials, float* __restrict__ out, int S, size_t n) {
   pdl_launch_dependents();

@@ -55,6 +55,11 @@ struct SampleParams {
   const uint64_t* dyn; // optional device {seed, step}: lets a static CUDA graph draw fresh numbers
   int sub;             // call_id = step * 16 + sub when dyn != nullptr (sub < 0: the step itself)
   const uint64_t* draws = nullptr;  // optional device [B][2]: call id and row that a row's random numbers are taken for
+  // optional: fp32 logits [B, V] (rounded to bf16 here, instead of `logits`) that are copied on the way to where the word at `copy_to` points
+  // (pinned host memory; 0: nowhere), rows from copy_row on
+  const float* logits32 = nullptr;
+  float* const* copy_to = nullptr;
+  int copy_row = 0;
 };
 
 __global__ void __launch_bounds__(256) sample_kernel(SampleParams p) {
@@ -78,16 +83,32 @@ __global__ void __launch_bounds__(256) sample_kernel(SampleParams p) {
   const float T = p.temps[b];
   const bool greedy = (T == 0.f);
   const float invT = greedy ? 1.f : 1.f / T;
-  const __nv_bfloat16* row = p.logits + (size_t)b * p.ld;
+  const __nv_bfloat16* row = p.logits32 ? nullptr : p.logits + (size_t)b * p.ld;
+  const float* row32 = p.logits32 ? p.logits32 + (size_t)b * p.V : nullptr;
+  float* copy = row32 && p.copy_to ? *p.copy_to : nullptr;
+  if (copy) copy += (size_t)(p.copy_row + b) * p.V;
+  const bool whole = (p.V & 3) == 0 && ((uintptr_t)copy & 15) == 0;   // (logits32 starts on a 16-byte boundary)
   ArgMax best{-INFINITY, 0x7fffffff};
   for (int i = beg + threadIdx.x * 4; i < end; i += blockDim.x * 4) {
     uint4 rnd = make_uint4(0, 0, 0, 0);
     if (!greedy) rnd = philox_draw((uint32_t)(i >> 2), row_id, p.call_id, TAG_SAMPLE, p.seed);
+    float v[4];
+    if (row32 && whole) {   // (chunks start and end on multiples of four)
+      const float4 f = *reinterpret_cast<const float4*>(row32 + i);
+      v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+      if (copy) *reinterpret_cast<float4*>(copy + i) = f;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v[j] = i + j >= end ? 0.f : row32 ? row32[i + j] : bf2f(row[i + j]);
+        if (copy && i + j < end) copy[i + j] = v[j];
+      }
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int idx = i + j;
       if (idx < end) {
-        const float l = bf2f(row[idx]);
+        const float l = row32 ? bf16_round(v[j]) : v[j];
         float sc = l;
         if (!greedy) {
           // scores = softmax(l/T) / (E + 1e-10)   (sampler.py:27-34), log domain
