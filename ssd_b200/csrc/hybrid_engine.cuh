@@ -91,7 +91,8 @@ struct ssdk_hyb_engine {
     it->second.last = ++graph_clock;
     return &it->second;
   }
-  cudaStream_t cap_stream = nullptr;
+  cudaStream_t cap_stream = nullptr, side = nullptr;   // side: see HybRun::beside
+  cudaEvent_t side_begin = nullptr, side_end = nullptr;
   void drop_graphs() {       // also when a buffer that their launches name is bound anew
     for (auto& kv : graphs)
       if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
@@ -1435,52 +1436,88 @@ struct HybRun {
     CKI(lin(hin, W, Lr.t[SSDK_HT_PAIR_IN].p, W, e->p0, Ntot, M, Ntot, W));
     // left: attention
     const float* agate = c.pair_gate ? e->p0 + o_g : nullptr;
-    if (c.pair_conv || c.qk_norm == 2 || Lr.t[SSDK_HT_ATTN_IN_B].p) {
-      if (c.qk_norm == 1) return fail("attention pair: the per-head unit norm is built for projections without a bias");
-      ssdk::ConvArgs ca = {};
-      ca.in = e->p0; ca.ld_in = Ntot; ca.in_bias = Lr.t[SSDK_HT_ATTN_IN_B].p; ca.w = c.pair_conv ? Lr.t[SSDK_HT_ATTN_CONV_W].p : nullptr;
-      ca.hist = e->state + Lr.attn_hist_off; ca.slot_stride = e->slot_floats; ca.C = Ca; ca.taps = std::max(1, c.pair_conv);
-      CKI(gqa_attention(Lr, e->p0, Ntot, e->t0, e->p1, agate, Ntot, nullptr, &ca, Lr.t[SSDK_HT_ATTN_QK_NORM].p));
-    } else {
-      CKI(gqa_attention(Lr, e->p0, Ntot, e->t0, e->p1, agate, Ntot));
-    }
-    CKI(lin(e->t0, HV, Lr.t[SSDK_HT_ATTN_OUT].p, HV, e->mix_out, W, M, W, HV));
-    // right: gated delta rule
-    float* st = e->state + Lr.state_off;
-    ssdk::DeltaPrepArgs dp = {};
-    dp.conv.in = e->p0 + o_dq; dp.conv.ld_in = Ntot; dp.conv.w = Lr.t[SSDK_HT_CONV_W].p; dp.conv.hist = st + (size_t)Hd * Dd * Vd;
-    dp.conv.slot_stride = e->slot_floats; dp.conv.C = Cd; dp.conv.taps = taps;
-    dp.v = e->p2; dp.rec = e->delta_rec;
-    float* dz = dp.v + (size_t)M * dHV;                            // decay pre-activations [M, Hd Dd]
-    float* gz = dz + (Ra ? (size_t)M * Hd * Dd : 0);               // gate pre-activations [M, Hd Vd]
-    dp.b = e->p0 + o_b; dp.ld_b = Ntot;
-    if (Ra || Rg) {   // second halves of the low-rank projections
-      const void *za = e->p0 + o_a, *zg = e->p0 + o_g1;
-      int lda = Ntot, ldg = Ntot;
-      if (!kF32) {
-        T* ta = (T*)e->t1;
-        T* tg = ta + (size_t)M * Ra;
-        CKI(L.go(ssdk::cast_split_kernel<T>, dim3(M), dim3(Ra + Rg <= 128 ? 128 : 256), 0, (const float*)e->p0 + (Ra ? o_a : o_g1), Ntot, ta, Ra, tg, Rg));
-        za = ta; zg = tg; lda = Ra; ldg = Rg;
+    auto left = [&]() -> int {
+      if (c.pair_conv || c.qk_norm == 2 || Lr.t[SSDK_HT_ATTN_IN_B].p) {
+        if (c.qk_norm == 1) return fail("attention pair: the per-head unit norm is built for projections without a bias");
+        ssdk::ConvArgs ca = {};
+        ca.in = e->p0; ca.ld_in = Ntot; ca.in_bias = Lr.t[SSDK_HT_ATTN_IN_B].p; ca.w = c.pair_conv ? Lr.t[SSDK_HT_ATTN_CONV_W].p : nullptr;
+        ca.hist = e->state + Lr.attn_hist_off; ca.slot_stride = e->slot_floats; ca.C = Ca; ca.taps = std::max(1, c.pair_conv);
+        CKI(gqa_attention(Lr, e->p0, Ntot, e->t0, e->p1, agate, Ntot, nullptr, &ca, Lr.t[SSDK_HT_ATTN_QK_NORM].p));
+      } else {
+        CKI(gqa_attention(Lr, e->p0, Ntot, e->t0, e->p1, agate, Ntot));
       }
-      if (Ra) CKI(lin(za, lda, Lr.t[SSDK_HT_DELTA_A2].p, Ra, dz, Hd * Dd, M, Hd * Dd, Ra));
-      if (Rg) CKI(lin(zg, ldg, Lr.t[SSDK_HT_DELTA_G2].p, Rg, gz, dHV, M, dHV, Rg));
-    }
-    dp.a = Ra ? dz : e->p0 + o_a; dp.ld_a = Ra ? Hd * Dd : Ntot; dp.per_channel = Ra > 0;
-    dp.A_log = Lr.t[SSDK_HT_DELTA_ALOG].p; dp.dt_bias = Lr.t[SSDK_HT_DELTA_DT_B].p;
-    dp.H = Hd; dp.G = Gd; dp.D = Dd; dp.V = Vd; dp.DP = delta_padded(Dd); dp.q_scale = 1.0f / sqrtf((float)Dd); dp.unit_eps = 1e-6f;
-    ssdk::DeltaArgs da;
-    da.rec = e->delta_rec; da.v = dp.v; da.o = e->p1; da.S = st; da.slot_stride = e->slot_floats; da.H = Hd; da.D = Dd; da.V = Vd; da.DP = dp.DP;
-    da.vec = Dd % 4 == 0;
-    CKI(delta_rule(dp, da));
-    if (taps > 1) CKI(L.go(ssdk::conv_state_kernel<T>, dim3(rg.n_seqs, (Cd + 255) / 256), dim3(256), 0, dp.conv, rg));
-    const dim3 ngrid(M, Hd), nblock(std::min(256, (Vd + 31) / 32 * 32));
-    const float* gate = Rg ? gz : e->p0 + o_dg;
-    const int ld_gate = Rg ? dHV : Ntot;
-    const T* nw = (const T*)Lr.t[SSDK_HT_MIX_NORM].p;
-    if (c.d_gate_act) CKI(L.go(ssdk::head_rmsnorm_gate_kernel<T, 1>, ngrid, nblock, 0, (const float*)e->p1, gate, ld_gate, nw, (T*)e->t1, Hd, Vd, e->cfg.eps));
-    else CKI(L.go(ssdk::head_rmsnorm_gate_kernel<T, 0>, ngrid, nblock, 0, (const float*)e->p1, gate, ld_gate, nw, (T*)e->t1, Hd, Vd, e->cfg.eps));
-    return lin(e->t1, dHV, Lr.t[SSDK_HT_MIX_OUT].p, dHV, e->mix2, W, M, W, dHV);
+      return lin(e->t0, HV, Lr.t[SSDK_HT_ATTN_OUT].p, HV, e->mix_out, W, M, W, HV);
+    };
+    const bool aside = beside_ok(Lr, HV, W);
+    if (aside) CKI(beside(left));
+    else CKI(left());
+    auto right = [&]() -> int {
+      // right: gated delta rule
+      float* st = e->state + Lr.state_off;
+      ssdk::DeltaPrepArgs dp = {};
+      dp.conv.in = e->p0 + o_dq; dp.conv.ld_in = Ntot; dp.conv.w = Lr.t[SSDK_HT_CONV_W].p; dp.conv.hist = st + (size_t)Hd * Dd * Vd;
+      dp.conv.slot_stride = e->slot_floats; dp.conv.C = Cd; dp.conv.taps = taps;
+      dp.v = e->p2; dp.rec = e->delta_rec;
+      float* dz = dp.v + (size_t)M * dHV;                            // decay pre-activations [M, Hd Dd]
+      float* gz = dz + (Ra ? (size_t)M * Hd * Dd : 0);               // gate pre-activations [M, Hd Vd]
+      dp.b = e->p0 + o_b; dp.ld_b = Ntot;
+      if (Ra || Rg) {   // second halves of the low-rank projections
+        const void *za = e->p0 + o_a, *zg = e->p0 + o_g1;
+        int lda = Ntot, ldg = Ntot;
+        if (!kF32) {
+          T* ta = (T*)e->t1;
+          T* tg = ta + (size_t)M * Ra;
+          CKI(L.go(ssdk::cast_split_kernel<T>, dim3(M), dim3(Ra + Rg <= 128 ? 128 : 256), 0, (const float*)e->p0 + (Ra ? o_a : o_g1), Ntot, ta, Ra, tg, Rg));
+          za = ta; zg = tg; lda = Ra; ldg = Rg;
+        }
+        if (Ra) CKI(lin(za, lda, Lr.t[SSDK_HT_DELTA_A2].p, Ra, dz, Hd * Dd, M, Hd * Dd, Ra));
+        if (Rg) CKI(lin(zg, ldg, Lr.t[SSDK_HT_DELTA_G2].p, Rg, gz, dHV, M, dHV, Rg));
+      }
+      dp.a = Ra ? dz : e->p0 + o_a; dp.ld_a = Ra ? Hd * Dd : Ntot; dp.per_channel = Ra > 0;
+      dp.A_log = Lr.t[SSDK_HT_DELTA_ALOG].p; dp.dt_bias = Lr.t[SSDK_HT_DELTA_DT_B].p;
+      dp.H = Hd; dp.G = Gd; dp.D = Dd; dp.V = Vd; dp.DP = delta_padded(Dd); dp.q_scale = 1.0f / sqrtf((float)Dd); dp.unit_eps = 1e-6f;
+      ssdk::DeltaArgs da;
+      da.rec = e->delta_rec; da.v = dp.v; da.o = e->p1; da.S = st; da.slot_stride = e->slot_floats; da.H = Hd; da.D = Dd; da.V = Vd; da.DP = dp.DP;
+      da.vec = Dd % 4 == 0;
+      CKI(delta_rule(dp, da));
+      if (taps > 1) CKI(L.go(ssdk::conv_state_kernel<T>, dim3(rg.n_seqs, (Cd + 255) / 256), dim3(256), 0, dp.conv, rg));
+      const float* gate = Rg ? gz : e->p0 + o_dg;
+      const int ld_gate = Rg ? dHV : Ntot;
+      const T* nw = (const T*)Lr.t[SSDK_HT_MIX_NORM].p;
+      const dim3 ngrid(M, Hd), nblock(std::min(256, (Vd + 31) / 32 * 32));
+      if (c.d_gate_act) CKI(L.go(ssdk::head_rmsnorm_gate_kernel<T, 1>, ngrid, nblock, 0, (const float*)e->p1, gate, ld_gate, nw, (T*)e->t1, Hd, Vd, e->cfg.eps));
+      else CKI(L.go(ssdk::head_rmsnorm_gate_kernel<T, 0>, ngrid, nblock, 0, (const float*)e->p1, gate, ld_gate, nw, (T*)e->t1, Hd, Vd, e->cfg.eps));
+      return lin(e->t1, dHV, Lr.t[SSDK_HT_MIX_OUT].p, dHV, e->mix2, W, M, W, dHV);
+    };
+    const int rc = right();
+    if (aside) CKI(beside_end());   // (also after an error: nothing of this call outlives it)
+    return rc;
+  }
+
+  // A pair's attention on a stream of its own beside its delta rule, whose walk leaves most of the machine idle.  The two share what they read (the
+  // projection) and nothing that they write as long as the attention runs in its fused kernels (which leave p1 alone) and its output product
+  // needs no split-K partials.
+  bool beside_ok(const HybLayer& Lr, int K, int N) const {
+    return e->side && longest() == 1 && !kF32 && gqa_on_mma(Lr) && e->use_decode_attn && (few_rows(M, N, K) || pair_ok(M) || !tc_ok(e->t0, K, Lr.t[SSDK_HT_ATTN_OUT].p, K, N, N, K));
+  }
+  template <typename F>
+  int beside(F&& branch) {
+    const cudaStream_t main = L.st;
+    CK(cudaEventRecord(e->side_begin, main));
+    CK(cudaStreamWaitEvent(e->side, e->side_begin, 0));
+    L.st = e->side;
+    L.barrier_op();
+    const int rc = branch();
+    L.st = main;
+    L.barrier_op();
+    if (rc) return rc;
+    CK(cudaEventRecord(e->side_end, e->side));
+    return 0;
+  }
+  int beside_end() {
+    CK(cudaStreamWaitEvent(L.st, e->side_end, 0));
+    L.barrier_op();
+    return 0;
   }
 
   // the delta rule over this step's rows: state-independent products per chunk, then the walk
@@ -2001,6 +2038,11 @@ int ssdk_hyb_create(const ssdk_hyb_cfg* cfg, const ssdk_hyb_layer_cfg* layers, s
     delete e;
     return fail("ssdk_hyb_create: pinned staging allocation failed");
   }
+  if (e->any_pair && (cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking) != cudaSuccess || cudaEventCreateWithFlags(&e->side_begin, cudaEventDisableTiming) != cudaSuccess ||
+                      cudaEventCreateWithFlags(&e->side_end, cudaEventDisableTiming) != cudaSuccess)) {
+    ssdk_hyb_destroy(e);
+    return fail("ssdk_hyb_create: could not make a stream");
+  }
   *out = e;
   return 0;
 }
@@ -2016,6 +2058,9 @@ int ssdk_hyb_destroy(ssdk_hyb_handle e) {
   if (e->h_tokens) cudaFreeHost(e->h_tokens);
   e->drop_graphs();
   if (e->cap_stream) cudaStreamDestroy(e->cap_stream);
+  if (e->side) cudaStreamDestroy(e->side);
+  if (e->side_begin) cudaEventDestroy(e->side_begin);
+  if (e->side_end) cudaEventDestroy(e->side_end);
   delete e;
   return 0;
 }
