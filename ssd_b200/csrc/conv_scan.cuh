@@ -72,6 +72,55 @@ __global__ void short_conv_kernel(const ConvArgs p, const Ragged rg) {
   if (p.out_t) st_f<T>((T*)p.out_t + (size_t)m * p.ld_t + c, v);
 }
 
+// The same over kConvRows consecutive rows per thread and four channels (taps of kConvTaps): a row's inputs are read once and not once per tap.  Channels,
+// strides and buffers are whole 16-byte pieces.  grid (ceil(M / kConvRows), ceil(C / 4 / blockDim)).  Same sums in the same order.
+// 2048 rows of 4096 channels: 64 -> 20 us (a thread per element read every input four times and waited for each).
+constexpr int kConvRows = 8, kConvTaps = 4;
+template <typename T, int ACT>
+__global__ void __launch_bounds__(128) short_conv_rows_kernel(const ConvArgs p, const Ragged rg) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int m0 = blockIdx.x * kConvRows, c = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
+  if (c >= p.C) return;
+  float w[4 * kConvTaps], bias[4] = {0.f, 0.f, 0.f, 0.f}, ib[4] = {0.f, 0.f, 0.f, 0.f};   // w[e kConvTaps + j]: channel c + e, tap j
+  ld_contig<T, 4 * kConvTaps>((const T*)p.w + (size_t)c * kConvTaps, w);
+  if (p.bias) ld_contig<T, 4>((const T*)p.bias + c, bias);
+  if (p.in_bias) ld_contig<T, 4>((const T*)p.in_bias + c, ib);
+  float x[kConvRows + kConvTaps - 1][4];   // x[i]: row m0 - (kConvTaps - 1) + i
+#pragma unroll
+  for (int i = 0; i < kConvRows + kConvTaps - 1; ++i) {
+    const int m = m0 - (kConvTaps - 1) + i;
+    const float4 v = m >= 0 && m < rg.M ? *reinterpret_cast<const float4*>(p.in + (size_t)m * p.ld_in + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    x[i][0] = v.x + ib[0]; x[i][1] = v.y + ib[1]; x[i][2] = v.z + ib[2]; x[i][3] = v.w + ib[3];
+  }
+#pragma unroll
+  for (int i = 0; i < kConvRows; ++i) {
+    const int m = m0 + i;
+    if (m >= rg.M) return;
+    const int s = rg.tok_seq[m], t = m - rg.cu[s];
+    float y[4] = {bias[0], bias[1], bias[2], bias[3]};
+#pragma unroll
+    for (int j = 0; j < kConvTaps; ++j) {
+      const int back = kConvTaps - 1 - j;
+      float v[4] = {x[i + j][0], x[i + j][1], x[i + j][2], x[i + j][3]};
+      if (back > t) {   // before the portion: the slot's rows, zeros before the sequence
+        const float* h = p.hist + (size_t)rg.slot[s] * p.slot_stride + (size_t)(kConvTaps - 1 - (back - t)) * p.C + c;
+        const bool carried = rg.pos0[s] > 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = carried ? h[e] : 0.f;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[e] = fmaf(w[e * kConvTaps + j], v[e], y[e]);
+    }
+    if (ACT == 1) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[e] = silu_f(y[e]);
+    }
+    if (p.out) st_row<float, 4>(p.out + (size_t)m * p.ld_out + c, y);
+    if (p.out_t) st_row<T, 4>((T*)p.out_t + (size_t)m * p.ld_t + c, y);
+  }
+}
+
 // grid (n_seqs, ceil(C / blockDim)).  New history = the last taps - 1 entries of (old history ++ this portion's inputs);
 // entry j is read from an index above j, so one thread per channel may work in place in ascending order.
 template <typename T>
@@ -227,23 +276,33 @@ struct RglruArgs {
 // grid (M, ceil(R / blockDim)): everything of a row that does not depend on the state, for all rows at once and in place:
 // gates[m][recurrence slot] <- a = exp(-c r softplus(lam)), gates[m][input slot] <- sqrt(1 - a^2) i u,
 // y[m] <- gelu_tanh(y[m] + bias)
-template <typename T>
+// VEC = 4: channels of a block, strides and buffers are whole 16-byte pieces (2048 rows of 2048 channels: 46 -> 22 us)
+template <typename T, int VEC>
 __global__ void rglru_gate_kernel(const RglruArgs p, float* __restrict__ gates, float* __restrict__ y) {
   pdl_launch_dependents();
   pdl_wait();
-  const int m = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
+  const int m = blockIdx.x, c = VEC * (blockIdx.y * blockDim.x + threadIdx.x);
   if (c >= p.R) return;
   const int b = c / p.bs, cb = c - b * p.bs;
   const int gr = b * 2 * p.bs + cb, gi = gr + p.bs;
-  const float sp = softplus_f(ld_f<T>((const T*)p.lam + c)) * p.decay_mult;
-  float* grow = gates + (size_t)m * p.ld_g;
-  const float log_a = -sigmoid_f(grow[gr] + ld_f<T>((const T*)p.gate_bias + gr)) * sp;
-  const float i = sigmoid_f(grow[gi] + ld_f<T>((const T*)p.gate_bias + gi));
-  grow[gr] = expf(log_a);
-  // 1 - a^2 through expm1: exact also where a is within an ulp of 1
-  grow[gi] = sqrtf(-expm1f(2.0f * log_a)) * i * p.u[(size_t)m * p.ld_u + c];
-  float* yp = y + (size_t)m * p.ld_y + c;
-  *yp = gelu_tanh_f(*yp + ld_f<T>((const T*)p.y_bias + c));
+  float *rp = gates + (size_t)m * p.ld_g + gr, *ip = gates + (size_t)m * p.ld_g + gi, *yp = y + (size_t)m * p.ld_y + c;
+  float lam[VEC], r[VEC], rb[VEC], i[VEC], ib[VEC], u[VEC], yv[VEC], yb[VEC];
+  ld_contig<T, VEC>((const T*)p.lam + c, lam);
+  ld_vec<VEC>(rp, r); ld_contig<T, VEC>((const T*)p.gate_bias + gr, rb);
+  ld_vec<VEC>(ip, i); ld_contig<T, VEC>((const T*)p.gate_bias + gi, ib);
+  ld_vec<VEC>(p.u + (size_t)m * p.ld_u + c, u);
+  ld_vec<VEC>(yp, yv); ld_contig<T, VEC>((const T*)p.y_bias + c, yb);
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) {
+    const float log_a = -sigmoid_f(r[e] + rb[e]) * (softplus_f(lam[e]) * p.decay_mult);
+    r[e] = expf(log_a);
+    // 1 - a^2 through expm1: exact also where a is within an ulp of 1
+    i[e] = sqrtf(-expm1f(2.0f * log_a)) * sigmoid_f(i[e] + ib[e]) * u[e];
+    yv[e] = gelu_tanh_f(yv[e] + yb[e]);
+  }
+  st_vec<VEC>(rp, r);
+  st_vec<VEC>(ip, i);
+  st_vec<VEC>(yp, yv);
 }
 
 constexpr int kRglruRows = 16;  // rows whose operands are requested together
@@ -344,18 +403,23 @@ struct SelScanArgs {
   int inner, N;
 };
 
-// grid (M, ceil(inner / blockDim)): the state-independent part of a row, in place: dtz <- softplus(dtz + bias), z <- silu(z)
-template <typename T>
+// grid (M, ceil(inner / VEC / blockDim)): the state-independent part of a row, in place: dtz <- softplus(dtz + bias), z <- silu(z).
+// VEC = 4: strides and buffers are whole 16-byte pieces
+template <typename T, int VEC>
 __global__ void selective_gate_kernel(float* __restrict__ dtz, int ld_dt, const T* __restrict__ dt_bias, float* __restrict__ z, int ld_z,
                                       int inner) {
   pdl_launch_dependents();
   pdl_wait();
-  const int m = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
+  const int m = blockIdx.x, c = VEC * (blockIdx.y * blockDim.x + threadIdx.x);
   if (c >= inner) return;
-  float* d = dtz + (size_t)m * ld_dt + c;
-  *d = softplus_f(*d + ld_f<T>(dt_bias + c));
-  float* zp = z + (size_t)m * ld_z + c;
-  *zp = silu_f(*zp);
+  float d[VEC], zv[VEC], b[VEC];
+  ld_vec<VEC>(dtz + (size_t)m * ld_dt + c, d);
+  ld_vec<VEC>(z + (size_t)m * ld_z + c, zv);
+  ld_contig<T, VEC>(dt_bias + c, b);
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) { d[e] = softplus_f(d[e] + b[e]); zv[e] = silu_f(zv[e]); }
+  st_vec<VEC>(dtz + (size_t)m * ld_dt + c, d);
+  st_vec<VEC>(z + (size_t)m * ld_z + c, zv);
 }
 
 constexpr int kSelRows = 8;  // rows whose inputs are requested (and whose B | C are staged) together

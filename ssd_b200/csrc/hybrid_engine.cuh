@@ -638,6 +638,22 @@ struct HybRun {
     return sh;
   }
 
+  // y [M, H V] (T) = unit RMS of every head of o [M, H V], times a channel weight, times silu (0) or sigmoid (1) of a gate pre-activation
+  template <int GATE>
+  int head_norm_gate(const float* o, const float* gate, int ld_gate, const T* w, void* y, int H, int V) {
+    if (V == 128 && whole16(ld_gate, {o, gate, w, y}) && (int64_t)M * H < (1ll << 31))
+      return L.go(ssdk::head_rmsnorm_gate_warp_kernel<T, GATE>, dim3((M * H + 7) / 8), dim3(256), 0, o, gate, ld_gate, w, (T*)y, M * H, H, e->cfg.eps);
+    return L.go(ssdk::head_rmsnorm_gate_kernel<T, GATE>, dim3(M, H), dim3(std::min(256, (V + 31) / 32 * 32)), 0, o, gate, ld_gate, w, (T*)y, H, V, e->cfg.eps);
+  }
+  // from a few rows per thread on (the grid of the row form then still covers the SMs); others: a thread per element
+  template <int ACT>
+  int short_conv(const ssdk::ConvArgs& ca) {
+    if (M >= 16 * ssdk::kConvRows && ca.taps == ssdk::kConvTaps && ca.C % 4 == 0 && ca.ld_in % 4 == 0 && ca.ld_out % 4 == 0 && ca.ld_t % 4 == 0 && ca.w &&
+        whole16(4, {ca.in, ca.w, ca.bias, ca.in_bias, ca.out, ca.out_t}))
+      return L.go(ssdk::short_conv_rows_kernel<T, ACT>, dim3((M + ssdk::kConvRows - 1) / ssdk::kConvRows, (ca.C / 4 + 127) / 128), dim3(128), 0, ca, rg);
+    return L.go(ssdk::short_conv_kernel<T, ACT>, dim3(M, (ca.C + 255) / 256), dim3(256), 0, ca, rg);
+  }
+
   int wkv(HybLayer& Lr) {
     const ssdk_hyb_layer_cfg& c = Lr.c;
     const int H = c.heads, D = c.dim, HD = H * D, W = e->cfg.width;
@@ -1129,8 +1145,8 @@ struct HybRun {
     ca.in = e->p0 + R; ca.ld_in = 2 * R; ca.in_bias = w_at(Lr.t[SSDK_HT_RGLRU_IN_B], R); ca.w = Lr.t[SSDK_HT_CONV_W].p;
     ca.bias = Lr.t[SSDK_HT_CONV_B].p; ca.out = e->p1; ca.ld_out = R; ca.out_t = kF32 ? nullptr : e->t0; ca.ld_t = R;
     ca.hist = st + R; ca.slot_stride = e->slot_floats; ca.C = R; ca.taps = taps;
-    const dim3 cgrid(M, (R + 255) / 256), sgrid(rg.n_seqs, (R + 255) / 256);
-    CKI(L.go(ssdk::short_conv_kernel<T, 0>, cgrid, dim3(256), 0, ca, rg));
+    const dim3 sgrid(rg.n_seqs, (R + 255) / 256);
+    CKI(short_conv<0>(ca));
     CKI(L.go(ssdk::conv_state_kernel<T>, sgrid, dim3(256), 0, ca, rg));
     // block-diagonal gates: per block one [2 bs, bs] product, all blocks in one batched launch
     const void* u_t = kF32 ? (const void*)e->p1 : (const void*)e->t0;
@@ -1139,7 +1155,8 @@ struct HybRun {
     a.u = e->p1; a.ld_u = R; a.gates = e->p2; a.ld_g = 2 * R; a.gate_bias = Lr.t[SSDK_HT_RGLRU_GATE_B].p; a.lam = Lr.t[SSDK_HT_RGLRU_LAM].p;
     a.y = e->p0; a.ld_y = 2 * R; a.y_bias = Lr.t[SSDK_HT_RGLRU_IN_B].p; a.out = e->t1; a.S = st; a.slot_stride = e->slot_floats;
     a.R = R; a.bs = bs; a.decay_mult = c.decay_mult;
-    CKI(L.go(ssdk::rglru_gate_kernel<T>, dim3(M, (R + 255) / 256), dim3(256), 0, a, e->p2, e->p0));
+    if (bs % 4 == 0 && whole16(4, {a.u, a.gates, a.y, a.gate_bias, a.lam, a.y_bias})) CKI(L.go(ssdk::rglru_gate_kernel<T, 4>, dim3(M, (R / 4 + 127) / 128), dim3(128), 0, a, e->p2, e->p0));
+    else CKI(L.go(ssdk::rglru_gate_kernel<T, 1>, dim3(M, (R + 255) / 256), dim3(256), 0, a, e->p2, e->p0));
     alone();
     if (longest() >= ssdk::kScanChunkMinRows) {
       CKI(L.go(ssdk::rglru_chunk_scan_kernel<T>, dim3(rg.n_seqs, (R + 31) / 32), dim3(32, ssdk::kScanChunks), 0, a, rg));
@@ -1163,7 +1180,7 @@ struct HybRun {
     ssdk::ConvArgs ca = {};
     ca.in = e->p0; ca.ld_in = 2 * I; ca.w = Lr.t[SSDK_HT_CONV_W].p; ca.bias = Lr.t[SSDK_HT_CONV_B].p; ca.out = e->p1; ca.ld_out = I;
     ca.out_t = kF32 ? nullptr : e->t0; ca.ld_t = I; ca.hist = st + (size_t)I * N; ca.slot_stride = e->slot_floats; ca.C = I; ca.taps = taps;
-    CKI(L.go(ssdk::short_conv_kernel<T, 1>, dim3(M, (I + 255) / 256), dim3(256), 0, ca, rg));
+    CKI(short_conv<1>(ca));
     CKI(L.go(ssdk::conv_state_kernel<T>, dim3(rg.n_seqs, (I + 255) / 256), dim3(256), 0, ca, rg));
     const void* x_t = kF32 ? (const void*)e->p1 : (const void*)e->t0;
     CKI(lin(x_t, I, Lr.t[SSDK_HT_SEL_X].p, I, e->p2, Nx, M, Nx, I));          // dt (low rank) | B | C
@@ -1179,7 +1196,9 @@ struct HybRun {
     a.A_log = Lr.t[SSDK_HT_SEL_ALOG].p; a.Dw = Lr.t[SSDK_HT_SEL_D].p; a.z = e->p0 + I; a.ld_z = 2 * I; a.out = e->t1;
     a.S = st; a.slot_stride = e->slot_floats; a.inner = I; a.N = N;
     const size_t smem = (size_t)ssdk::kSelRows * 2 * N * 4;
-    CKI(L.go(ssdk::selective_gate_kernel<T>, dim3(M, (I + 255) / 256), dim3(256), 0, dtz, I, (const T*)Lr.t[SSDK_HT_SEL_DT_B].p, e->p0 + I, 2 * I, I));
+    const T* dt_b = (const T*)Lr.t[SSDK_HT_SEL_DT_B].p;
+    if (I % 4 == 0 && whole16(4, {dtz, e->p0, dt_b})) CKI(L.go(ssdk::selective_gate_kernel<T, 4>, dim3(M, (I / 4 + 127) / 128), dim3(128), 0, dtz, I, dt_b, e->p0 + I, 2 * I, I));
+    else CKI(L.go(ssdk::selective_gate_kernel<T, 1>, dim3(M, (I + 255) / 256), dim3(256), 0, dtz, I, dt_b, e->p0 + I, 2 * I, I));
     alone();
     if (N <= 16 && longest() >= ssdk::kScanChunkMinRows) {
       const dim3 grid(rg.n_seqs, (I + 31) / 32), block(32, ssdk::kScanChunks);
@@ -1244,7 +1263,10 @@ struct HybRun {
       else if (vec) CKI(L.go(ssdk::gqa_head_prep_kernel<T, 4, 32>, dim3(M, ys), dim3(256), smem, hp, rg));
       else CKI(L.go(ssdk::gqa_head_prep_kernel<T, 1, 32>, dim3(M, ys), dim3(256), smem, hp, rg));
     } else {
-      CKI(L.go(ssdk::gqa_prep_kernel<T>, dim3(M, (H + G + ssdk::kPrepHeads - 1) / ssdk::kPrepHeads), dim3(32, ssdk::kPrepHeads), 0, pa, rg));
+      // (the row form where rows fill the machine: few rows take a warp per head)
+      const bool rows = M >= num_sms() && !c.rot_half && D % 4 == 0 && V % 4 == 0 && D <= 128 && c.rot_dims % 4 == 0 && whole16(ldz, {z, pool, e->qcat});
+      if (rows) CKI(L.go(ssdk::gqa_prep_rows_kernel<T>, dim3(M), dim3(256), (size_t)c.rot_dims * 4, pa, rg));
+      else CKI(L.go(ssdk::gqa_prep_kernel<T>, dim3(M, (H + G + ssdk::kPrepHeads - 1) / ssdk::kPrepHeads), dim3(32, ssdk::kPrepHeads), 0, pa, rg));
     }
     const bool mma = gqa_on_mma(Lr);
     const int ks = std::max(D, V) <= 32 ? 2 : (std::max(D, V) <= 64 || (maps == 2 && D <= 64) ? 4 : 8);
@@ -1484,9 +1506,7 @@ struct HybRun {
       const float* gate = Rg ? gz : e->p0 + o_dg;
       const int ld_gate = Rg ? dHV : Ntot;
       const T* nw = (const T*)Lr.t[SSDK_HT_MIX_NORM].p;
-      const dim3 ngrid(M, Hd), nblock(std::min(256, (Vd + 31) / 32 * 32));
-      if (c.d_gate_act) CKI(L.go(ssdk::head_rmsnorm_gate_kernel<T, 1>, ngrid, nblock, 0, (const float*)e->p1, gate, ld_gate, nw, (T*)e->t1, Hd, Vd, e->cfg.eps));
-      else CKI(L.go(ssdk::head_rmsnorm_gate_kernel<T, 0>, ngrid, nblock, 0, (const float*)e->p1, gate, ld_gate, nw, (T*)e->t1, Hd, Vd, e->cfg.eps));
+      CKI(c.d_gate_act ? head_norm_gate<1>(e->p1, gate, ld_gate, nw, e->t1, Hd, Vd) : head_norm_gate<0>(e->p1, gate, ld_gate, nw, e->t1, Hd, Vd));
       return lin(e->t1, dHV, Lr.t[SSDK_HT_MIX_OUT].p, dHV, e->mix2, W, M, W, dHV);
     };
     const int rc = right();

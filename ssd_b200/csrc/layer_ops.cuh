@@ -370,6 +370,27 @@ __global__ void head_rmsnorm_gate_kernel(const float* __restrict__ o, const floa
   }
 }
 
+// The same for heads of 128 channels, a warp per head, four channels per lane (strides and buffers are whole 16-byte pieces): one pass, no block-wide sum.
+// 2048 rows of 16 heads: 38 -> 10 us.  grid ceil(rows H / warps)
+template <typename T, int GATE>
+__global__ void __launch_bounds__(256) head_rmsnorm_gate_warp_kernel(const float* __restrict__ o, const float* __restrict__ g, int ldg,
+                                                                     const T* __restrict__ w, T* __restrict__ y, int n, int H, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), c = 4 * (threadIdx.x & 31);
+  if (u >= n) return;
+  const int m = u / H, hd = u - m * H;
+  float x[4], gz[4], wv[4] = {1.f, 1.f, 1.f, 1.f};
+  ld_vec<4>(o + (size_t)u * 128 + c, x);
+  ld_vec<4>(g + (size_t)m * ldg + hd * 128 + c, gz);
+  if (w) ld_contig<T, 4>(w + hd * 128 + c, wv);
+  const float ss = warp_sum(fmaf(x[0], x[0], fmaf(x[1], x[1], fmaf(x[2], x[2], x[3] * x[3]))));
+  const float inv = 1.0f / sqrtf(ss / 128.0f + eps);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) x[e] = x[e] * inv * wv[e] * (GATE == 0 ? gz[e] * sigmoid_f(gz[e]) : sigmoid_f(gz[e]));
+  st_row<T, 4>(y + (size_t)u * 128 + c, x);
+}
+
 // z [rows, ldz] fp32 with gate columns [0, ff) and up columns [ff, 2 ff) -> y [rows, ff] (T)
 template <typename T>
 __global__ void clamped_glu_kernel(const float* __restrict__ z, int ldz, T* __restrict__ y, int ff, float limit,
