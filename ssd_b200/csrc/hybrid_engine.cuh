@@ -72,7 +72,7 @@ struct ssdk_hyb_engine {
   int w_p0 = 0, w_p1 = 0, w_p2 = 0, w_t0 = 0, w_t1 = 0, w_e = 0, w_top = 0, w_ff2 = 0, w_ff = 0, w_sff2 = 0, w_sff = 0;
   size_t delta_floats = 0; float* delta_rec = nullptr;   // chunk records of the delta rule
   size_t ret_floats = 0; float* ret_rec = nullptr;       // chunk records of the retention
-  bool any_wkv = false, any_pair = false, any_ffn = false, vec_state = false;   // vec_state: slots are whole 16-byte pieces
+  bool any_wkv = false, any_pair = false, any_ffn = false, any_shared = false, vec_state = false;   // vec_state: slots are whole 16-byte pieces
   int* h_meta = nullptr;     // pinned staging of the step's numbers
   int64_t* h_tokens = nullptr; // pinned: the sampled tokens
   bool use_graph = true, use_pdl = true;   // decode steps replayed as graphs; programmatic dependent launch (SSDK_HYB_GRAPH=0, SSDK_HYB_PDL=0)
@@ -325,7 +325,7 @@ static int hyb_derive(ssdk_hyb_engine* e) {
       }
       const long long mats = c.expert_glu ? 2 : 1;   // stacked input matrices of an expert
       up(e->w_e, Et); up(e->w_top, c.top); up(e->w_ff2, mats * c.ff); up(e->w_ff, c.ff);
-      if (c.shared_ff > 0) { up(e->w_sff2, mats * c.shared_ff + 1); up(e->w_sff, c.shared_ff); }
+      if (c.shared_ff > 0) { up(e->w_sff2, mats * c.shared_ff + 1); up(e->w_sff, c.shared_ff); e->any_shared = true; }
     } else if (c.mlp != SSDK_MLP_NONE) {
       return fail("hybrid layer: unknown feed-forward kind %d", c.mlp);
     }
@@ -997,62 +997,75 @@ struct HybRun {
     CKI(check_tensor(Lr, SSDK_HT_EXPERT_OUT, (int64_t)E * W, ff, "experts.out"));
     if (c.route_bias) CKI(check_tensor(Lr, SSDK_HT_ROUTER_BIAS, Et, 1, "router.bias"));
     CKI(lin(fin, W, Lr.t[SSDK_HT_ROUTER].p, W, e->rz, Et, M, Et, W));
-    ssdk::RouterArgs ra;
-    ra.z = e->rz; ra.bias = c.route_bias ? Lr.t[SSDK_HT_ROUTER_BIAS].p : nullptr; ra.sel = e->sel; ra.wts = e->wts; ra.M = M; ra.E = Et;
-    ra.top = top; ra.groups = c.groups; ra.keep = c.keep; ra.softmax = c.route_top_softmax ? 2 : c.route_softmax; ra.group_best = c.group_best;
-    ra.renorm = c.route_renorm; ra.route_scale = c.route_scale;
-    CKI(L.go(ssdk::group_topk_router_kernel<T>, dim3((M + ssdk::kRouterWarps - 1) / ssdk::kRouterWarps), dim3(ssdk::kRouterWarps * 32), 0, ra));
-    // bf16 with whole k-blocks: the grouped tcgen05 GEMM over rows gathered per expert; else the mma.sync / FMA tile, which gathers by
-    // index itself (tiles of kLinBM rows).  Below 256 routed rows an expert gets a few, the weights' bytes bound the call, and a tile
-    // of kFewTile rows streams them through deeper stages than the mma.sync tile does: 1, 2, 4, 8 decoding sequences, 32 experts of
-    // 2048 x 1024, top 4: 244, 267, 291, 311 -> 210, 221, 237, 265 us a call (tiles of 32: 211, 224, 239, 269); 16 experts of
-    // 1024 x 512: 168, 174, 191, 210 -> 169, 172, 180, 196; prompts of 24 and 50 tokens 293, 322 -> 266, 281
-    const bool tc_moe = !kF32 && e->use_tc && e->use_tc_experts && W % kBlockK == 0 && ff % kBlockK == 0 &&
-                        (((uintptr_t)Lr.t[SSDK_HT_EXPERT_IN].p | (uintptr_t)Lr.t[SSDK_HT_EXPERT_OUT].p) & 15) == 0;
-    const bool silu_glu = c.expert_glu && c.expert_act == SSDK_ACT_SILU, glu = tc_moe && silu_glu && e->use_tc_glu;   // activation in the GEMM's epilogue
-    const bool split = split_ok(fin, W, Lr.t[SSDK_HT_EXPERT_IN].p, W, A, Nin, W, 1, 0, 0) && split_ok(e->ey, ff, Lr.t[SSDK_HT_EXPERT_OUT].p, ff, A, W, ff, 1, 0, 0);
-    const int tile = split ? kSplitTokens : (!tc_moe ? ssdk::kLinBM : (pair_ok(M) && (!glu || ff % kPairGluRun == 0) ? kPairTokens : A < 256 ? kFewTile : 128));
-    ssdk::PlanArgs pa;
-    pa.sel = e->sel; pa.apos = e->apos; pa.arow = e->arow; pa.tile_expert = e->tile_expert; pa.tile_row0 = e->tile_row0;
-    pa.tile_rows = e->tile_rows; pa.n_tiles = e->n_tiles; pa.n_rows = e->n_rows; pa.A = A; pa.E = Et; pa.top = top; pa.tile = tile;
-    pa.E_real = E;
-    CKI(L.go(ssdk::expert_plan_kernel, dim3(1), dim3(1024), 0, pa));
-    const int* n_real_rows = c.identity > 0 ? e->n_rows : nullptr;   // rows behind them belong to identity experts: nothing to compute
-    ssdk::LinearArgs a = {};
-    if (tc_moe) {
-      CKI(L.go(ssdk::gather_rows_kernel<T>, dim3(A), dim3(128), 0, (const T*)fin, (const int*)e->arow, (const int*)e->n_rows, (T*)e->xs, W));
-      CKI(lin_tc_grouped(e->xs, Lr.t[SSDK_HT_EXPERT_IN].p, glu ? e->ey : (void*)e->eg, A, Nin, W, E, tile, A / tile + E + 1, glu));
-    } else if (split) {
-      CKI(split_grouped(fin, W, e->arow, Lr.t[SSDK_HT_EXPERT_IN].p, e->eg, A, Nin, W, A / tile + E + 1));
-    } else {
-      a.A = fin; a.W = Lr.t[SSDK_HT_EXPERT_IN].p; a.C = e->eg; a.M = A; a.N = Nin; a.K = W; a.lda = W; a.ldw = W; a.ldc = Nin;
-      a.a_rows = e->arow; a.tile_expert = e->tile_expert; a.tile_row0 = e->tile_row0; a.tile_rows = e->tile_rows; a.n_tiles = e->n_tiles;
-      a.sW_expert = (long long)Nin * W;
-      CKI(lin_args<float>(a, A, 1));
-    }
-    if (!glu) CKI(expert_act(c, (const float*)e->eg, Nin, (T*)e->ey, ff, c.limit, A, n_real_rows));
-    if (tc_moe) {
-      CKI(lin_tc_grouped(e->ey, Lr.t[SSDK_HT_EXPERT_OUT].p, e->eo, A, W, ff, E, tile, A / tile + E + 1));
-    } else if (split) {
-      CKI(split_grouped(e->ey, ff, nullptr, Lr.t[SSDK_HT_EXPERT_OUT].p, e->eo, A, W, ff, A / tile + E + 1));
-    } else {
-      a.A = e->ey; a.W = Lr.t[SSDK_HT_EXPERT_OUT].p; a.C = e->eo; a.N = W; a.K = ff; a.lda = ff; a.ldw = ff; a.ldc = W; a.a_rows = nullptr;
-      a.tile_expert = e->tile_expert; a.tile_row0 = e->tile_row0; a.tile_rows = e->tile_rows; a.n_tiles = e->n_tiles;
-      a.M = A; a.sW_expert = (long long)W * ff;
-      CKI(lin_args<float>(a, A, 1));
-    }
-    if (c.shared_ff > 0) {
-      const int sff = c.shared_ff, Ns = (c.expert_glu ? 2 : 1) * sff + (c.shared_gate ? 1 : 0);
+    const bool silu_glu = c.expert_glu && c.expert_act == SSDK_ACT_SILU;
+    const int sff = c.shared_ff, Ns = (c.expert_glu ? 2 : 1) * sff + (c.shared_gate ? 1 : 0);
+    const bool shared_glu = sff > 0 && silu_glu && !c.shared_gate && tc_glu_ok(fin, Lr.t[SSDK_HT_SHARED_IN].p, sff, W);
+    auto shared = [&]() -> int {
+      if (sff <= 0) return 0;
       CKI(check_tensor(Lr, SSDK_HT_SHARED_IN, Ns, W, "shared.in")); CKI(check_tensor(Lr, SSDK_HT_SHARED_OUT, W, sff, "shared.out"));
-      if (silu_glu && !c.shared_gate && tc_glu_ok(fin, Lr.t[SSDK_HT_SHARED_IN].p, sff, W)) {
+      if (shared_glu) {
         CKI(lin_tc_glu(fin, Lr.t[SSDK_HT_SHARED_IN].p, e->sy, M, sff, W, false));
       } else {
         CKI(lin(fin, W, Lr.t[SSDK_HT_SHARED_IN].p, W, e->sz, Ns, M, Ns, W));
         CKI(expert_act(c, (const float*)e->sz, Ns, (T*)e->sy, sff, c.shared_limit, M, (const int*)nullptr));
       }
       CKI(lin(e->sy, sff, Lr.t[SSDK_HT_SHARED_OUT].p, sff, e->so, W, M, W, sff));
-    }
-    return 0;
+      return 0;
+    };
+    // the shared expert beside the routing, which is a chain of small kernels: prompts of vegilix m, 2001 tokens 540 -> 521 us, of lisenex m 876 -> 853,
+    // eight of its sequences decoding 248 -> 235
+    const bool aside = sff > 0 && beside_ok(e->sy, Lr.t[SSDK_HT_SHARED_OUT].p, sff, W) && (shared_glu || beside_ok(fin, Lr.t[SSDK_HT_SHARED_IN].p, W, Ns));
+    if (aside) CKI(beside(shared));
+    auto routed = [&]() -> int {
+      ssdk::RouterArgs ra;
+      ra.z = e->rz; ra.bias = c.route_bias ? Lr.t[SSDK_HT_ROUTER_BIAS].p : nullptr; ra.sel = e->sel; ra.wts = e->wts; ra.M = M; ra.E = Et;
+      ra.top = top; ra.groups = c.groups; ra.keep = c.keep; ra.softmax = c.route_top_softmax ? 2 : c.route_softmax; ra.group_best = c.group_best;
+      ra.renorm = c.route_renorm; ra.route_scale = c.route_scale;
+      CKI(L.go(ssdk::group_topk_router_kernel<T>, dim3((M + ssdk::kRouterWarps - 1) / ssdk::kRouterWarps), dim3(ssdk::kRouterWarps * 32), 0, ra));
+      // bf16 with whole k-blocks: the grouped tcgen05 GEMM over rows gathered per expert; else the mma.sync / FMA tile, which gathers by
+      // index itself (tiles of kLinBM rows).  Below 256 routed rows an expert gets a few, the weights' bytes bound the call, and a tile
+      // of kFewTile rows streams them through deeper stages than the mma.sync tile does: 1, 2, 4, 8 decoding sequences, 32 experts of
+      // 2048 x 1024, top 4: 244, 267, 291, 311 -> 210, 221, 237, 265 us a call (tiles of 32: 211, 224, 239, 269); 16 experts of
+      // 1024 x 512: 168, 174, 191, 210 -> 169, 172, 180, 196; prompts of 24 and 50 tokens 293, 322 -> 266, 281
+      const bool tc_moe = !kF32 && e->use_tc && e->use_tc_experts && W % kBlockK == 0 && ff % kBlockK == 0 &&
+                          (((uintptr_t)Lr.t[SSDK_HT_EXPERT_IN].p | (uintptr_t)Lr.t[SSDK_HT_EXPERT_OUT].p) & 15) == 0;
+      const bool glu = tc_moe && silu_glu && e->use_tc_glu;   // activation in the GEMM's epilogue
+      const bool split = split_ok(fin, W, Lr.t[SSDK_HT_EXPERT_IN].p, W, A, Nin, W, 1, 0, 0) && split_ok(e->ey, ff, Lr.t[SSDK_HT_EXPERT_OUT].p, ff, A, W, ff, 1, 0, 0);
+      const int tile = split ? kSplitTokens : (!tc_moe ? ssdk::kLinBM : (pair_ok(M) && (!glu || ff % kPairGluRun == 0) ? kPairTokens : A < 256 ? kFewTile : 128));
+      ssdk::PlanArgs pa;
+      pa.sel = e->sel; pa.apos = e->apos; pa.arow = e->arow; pa.tile_expert = e->tile_expert; pa.tile_row0 = e->tile_row0;
+      pa.tile_rows = e->tile_rows; pa.n_tiles = e->n_tiles; pa.n_rows = e->n_rows; pa.A = A; pa.E = Et; pa.top = top; pa.tile = tile;
+      pa.E_real = E;
+      CKI(L.go(ssdk::expert_plan_kernel, dim3(1), dim3(1024), 0, pa));
+      const int* n_real_rows = c.identity > 0 ? e->n_rows : nullptr;   // rows behind them belong to identity experts: nothing to compute
+      ssdk::LinearArgs a = {};
+      if (tc_moe) {
+        CKI(L.go(ssdk::gather_rows_kernel<T>, dim3(A), dim3(128), 0, (const T*)fin, (const int*)e->arow, (const int*)e->n_rows, (T*)e->xs, W));
+        CKI(lin_tc_grouped(e->xs, Lr.t[SSDK_HT_EXPERT_IN].p, glu ? e->ey : (void*)e->eg, A, Nin, W, E, tile, A / tile + E + 1, glu));
+      } else if (split) {
+        CKI(split_grouped(fin, W, e->arow, Lr.t[SSDK_HT_EXPERT_IN].p, e->eg, A, Nin, W, A / tile + E + 1));
+      } else {
+        a.A = fin; a.W = Lr.t[SSDK_HT_EXPERT_IN].p; a.C = e->eg; a.M = A; a.N = Nin; a.K = W; a.lda = W; a.ldw = W; a.ldc = Nin;
+        a.a_rows = e->arow; a.tile_expert = e->tile_expert; a.tile_row0 = e->tile_row0; a.tile_rows = e->tile_rows; a.n_tiles = e->n_tiles;
+        a.sW_expert = (long long)Nin * W;
+        CKI(lin_args<float>(a, A, 1));
+      }
+      if (!glu) CKI(expert_act(c, (const float*)e->eg, Nin, (T*)e->ey, ff, c.limit, A, n_real_rows));
+      if (tc_moe) {
+        CKI(lin_tc_grouped(e->ey, Lr.t[SSDK_HT_EXPERT_OUT].p, e->eo, A, W, ff, E, tile, A / tile + E + 1));
+      } else if (split) {
+        CKI(split_grouped(e->ey, ff, nullptr, Lr.t[SSDK_HT_EXPERT_OUT].p, e->eo, A, W, ff, A / tile + E + 1));
+      } else {
+        a.A = e->ey; a.W = Lr.t[SSDK_HT_EXPERT_OUT].p; a.C = e->eo; a.N = W; a.K = ff; a.lda = ff; a.ldw = ff; a.ldc = W; a.a_rows = nullptr;
+        a.tile_expert = e->tile_expert; a.tile_row0 = e->tile_row0; a.tile_rows = e->tile_rows; a.n_tiles = e->n_tiles;
+        a.M = A; a.sW_expert = (long long)W * ff;
+        CKI(lin_args<float>(a, A, 1));
+      }
+      return 0;
+    };
+    const int rc = routed();
+    if (aside) CKI(beside_end());   // (also after an error: nothing of this call outlives it)
+    return rc || aside ? rc : shared();
   }
 
   // dense feed-forward without a gate: so = W_down act(W_up h + b_up); b_down joins in the block's combine
@@ -1470,7 +1483,10 @@ struct HybRun {
       }
       return lin(e->t0, HV, Lr.t[SSDK_HT_ATTN_OUT].p, HV, e->mix_out, W, M, W, HV);
     };
-    const bool aside = beside_ok(Lr, HV, W);
+    // A decoding step's attention beside its delta rule: chains of five small kernels each.  In prompts the walk of the delta rule, a warp per scheduler, would
+    // take 427 us instead of 263 beside anything (2048 tokens, 4 layers: 2616 -> 2795 us a call; decoding 209 -> 186).  The attention runs in its
+    // fused kernels, which leave p1 alone.
+    const bool aside = longest() == 1 && gqa_on_mma(Lr) && e->use_decode_attn && beside_ok(e->t0, Lr.t[SSDK_HT_ATTN_OUT].p, HV, W);
     if (aside) CKI(beside(left));
     else CKI(left());
     auto right = [&]() -> int {
@@ -1514,11 +1530,10 @@ struct HybRun {
     return rc;
   }
 
-  // A pair's attention on a stream of its own beside its delta rule, whose walk leaves most of the machine idle.  The two share what they read (the
-  // projection) and nothing that they write as long as the attention runs in its fused kernels (which leave p1 alone) and its output product
-  // needs no split-K partials.
-  bool beside_ok(const HybLayer& Lr, int K, int N) const {
-    return e->side && longest() == 1 && !kF32 && gqa_on_mma(Lr) && e->use_decode_attn && (few_rows(M, N, K) || pair_ok(M) || !tc_ok(e->t0, K, Lr.t[SSDK_HT_ATTN_OUT].p, K, N, N, K));
+  // A branch of a layer on a stream of its own beside the rest of it: the two share what they read and nothing that they write.  Among that are the
+  // split-K partials and the pieces of fp32 rows, so that a product x[M, K] w[N, K]^T may be taken aside only where it needs neither.
+  bool beside_ok(const void* x, const void* w, int K, int N) const {
+    return e->side && !kF32 && (few_rows(M, N, K) || pair_ok(M) || !tc_ok(x, K, w, K, N, N, K));
   }
   template <typename F>
   int beside(F&& branch) {
@@ -2058,7 +2073,7 @@ int ssdk_hyb_create(const ssdk_hyb_cfg* cfg, const ssdk_hyb_layer_cfg* layers, s
     delete e;
     return fail("ssdk_hyb_create: pinned staging allocation failed");
   }
-  if (e->any_pair && (cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking) != cudaSuccess || cudaEventCreateWithFlags(&e->side_begin, cudaEventDisableTiming) != cudaSuccess ||
+  if ((e->any_pair || e->any_shared) && (cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking) != cudaSuccess || cudaEventCreateWithFlags(&e->side_begin, cudaEventDisableTiming) != cudaSuccess ||
                       cudaEventCreateWithFlags(&e->side_end, cudaEventDisableTiming) != cudaSuccess)) {
     ssdk_hyb_destroy(e);
     return fail("ssdk_hyb_create: could not make a stream");
