@@ -263,11 +263,13 @@ static int launch_gemm_pair(Launcher& L, int epi, const CUtensorMap& tmW, const 
     CK(cudaFuncSetAttribute(gemm_pair_kernel<EPI_PARTIAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
     CK(cudaFuncSetAttribute(gemm_pair_kernel<EPI_GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
     CK(cudaFuncSetAttribute(gemm_pair_kernel<EPI_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
+    CK(cudaFuncSetAttribute(gemm_pair_kernel<EPI_BF16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
     attr_set = true;
   }
   p.timeout = L.gave_up;
   if (p.batch < 1) p.batch = 1;
   const dim3 grid(2 * std::min(max_tiles, num_sms() / 2)), block(kPairThreads);
+  if (epi == EPI_BF16 && p.w_head > 0) return L.go(gemm_pair_kernel<EPI_BF16, true>, grid, block, (size_t)kPairSmem, tmW, tmX, tmXs, p);
   if (epi == EPI_BF16) return L.go(gemm_pair_kernel<EPI_BF16>, grid, block, (size_t)kPairSmem, tmW, tmX, tmXs, p);
   if (epi == EPI_GLU) return L.go(gemm_pair_kernel<EPI_GLU>, grid, block, (size_t)kPairSmem, tmW, tmX, tmXs, p);
   return L.go(gemm_pair_kernel<EPI_PARTIAL>, grid, block, (size_t)kPairSmem, tmW, tmX, tmXs, p);

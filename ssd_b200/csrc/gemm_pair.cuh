@@ -43,6 +43,8 @@ struct GemmPairParams {
   // dense: products of the same shape side by side (heads): product b reads X's columns from b x_step, the weight rows from b N, and
   // writes out + b out_step
   int batch, x_step, out_step;
+  // W_COLS (dense): the weights are [heads][K][w_head] (w_head a multiple of 64): output column n is column n % w_head of head n / w_head
+  int w_head;
   // grouped mode: see GemmParams
   const int* g_tile_expert;
   const int* g_tile_row0;
@@ -127,7 +129,21 @@ SSDK_DEVINL void tmem_dealloc_pair(uint32_t taddr) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(512) : "memory");
 }
 
-template <int EPI>
+// Operand that is contiguous along M or N, 128-byte swizzle: atoms of 64 elements x 8 k; the next 8 k follow 1024 B on (SBO), the next 64
+// elements `next64` bytes on (LBO)
+SSDK_DEVINL uint64_t make_umma_desc_mn128(const void* smem_tile, uint32_t next64) {
+  const uint32_t addr = smem_u32(smem_tile);
+  uint64_t d = 0;
+  d |= (uint64_t)((addr >> 4) & 0x3FFFu);
+  d |= (uint64_t)((next64 >> 4) & 0x3FFFu) << 16;
+  d |= (uint64_t)(1024u >> 4) << 32;
+  d |= (uint64_t)1u << 46;
+  d |= (uint64_t)2u << 61;
+  return d;
+}
+
+// W_COLS: weights whose output columns are contiguous and not their k (two boxes of 64 columns x 64 k per stage)
+template <int EPI, bool W_COLS = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmXs,
                  const GemmPairParams p) {
@@ -200,6 +216,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           const uint32_t bar = map_shared(&full_bar[s], 0);
           const int k = kb * kBlockK;
           if (EPI == EPI_GLU) tma_load_5d_pair(a_s, &tmW, bar, k, tl.col / kPairGluRun, tl.ex);
+          else if (W_COLS)
+            for (int b = 0; b < 2; ++b) {
+              const int n = tl.col + b * 64, head = n / p.w_head;
+              tma_load_2d_pair(a_s + b * 8192, &tmW, bar, n - head * p.w_head, head * p.num_kb * kBlockK + k, kEvictNormal);
+            }
           else tma_load_2d_pair(a_s, &tmW, bar, k, w_row, kEvictNormal);
           if (big) tma_load_2d_pair(b_s, &tmX, bar, kx + k, x0, kEvictNormal);
           else
@@ -217,7 +238,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       bool ok = true;
       for (int t = pair; t < tiles && ok; t += n_pairs, ++nt) {
         const Tile tl = tile_of(t);
-        const uint32_t idesc = make_umma_idesc_bf16(256, tl.n), acc = tmem_d + (uint32_t)(nt & 1) * 256u;
+        const uint32_t idesc = make_umma_idesc_bf16(256, tl.n) | (W_COLS ? 1u << 15 : 0u), acc = tmem_d + (uint32_t)(nt & 1) * 256u;
         if (!(ok = mbar_wait_cluster(&acc_empty[nt & 1], ((uint32_t)(nt >> 1) & 1u) ^ 1u, p.timeout))) break;
         tc_fence_after();
         for (int kb = 0; kb < p.num_kb; ++kb, ++it) {
@@ -225,10 +246,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           if (!(ok = mbar_wait_cluster(&full_bar[s], (uint32_t)(it / kPairStages) & 1u, p.timeout))) break;
           tc_fence_after();
           uint8_t* a_s = smem + s * kPairStageBytes;
-          const uint64_t adesc = make_umma_desc_k128(a_s), bdesc = make_umma_desc_k128(a_s + 16384);
+          const uint64_t adesc = W_COLS ? make_umma_desc_mn128(a_s, 8192) : make_umma_desc_k128(a_s), bdesc = make_umma_desc_k128(a_s + 16384);
 #pragma unroll
-          for (int k = 0; k < kBlockK / 16; ++k)
-            umma_bf16_ss_pair(acc, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (uint32_t)((kb | k) != 0));
+          for (int k = 0; k < kBlockK / 16; ++k)   // 16 k: 32 B of a row, 16 rows of 128 B of W_COLS
+            umma_bf16_ss_pair(acc, adesc + (uint64_t)((W_COLS ? 128 : 2) * k), bdesc + (uint64_t)(2 * k), idesc, (uint32_t)((kb | k) != 0));
           umma_commit_pair(&empty_bar[s]);
         }
         if (ok) umma_commit_pair(&acc_full[nt & 1]);

@@ -818,11 +818,11 @@ struct HybRun {
     return c.attn_scale > 0.f && e->cfg.block_size % ssdk::kPromptKeys == 0 && (hpg & (hpg - 1)) == 0 && hpg <= 16 && whole(c.vdim) && (c.maps == 2 ? c.dim == 64 : whole(c.dim)) &&
            e->num_blocks * e->cfg.block_size < (1ll << 31) && (int64_t)M * c.heads * c.maps < (1ll << 31) && whole16(gate ? ld_gate : 4, {gate});
   }
-  template <int DK, int VD, int MAPS>
-  int gqa_prompt_go(const CUtensorMap& tmQ, const CUtensorMap& tmKV, const ssdk::GqaPromptArgs& a, int n_max) {
+  template <int DK, int VD, int MAPS, bool LATENT = false>
+  int gqa_prompt_go(const CUtensorMap& tmQ, const CUtensorMap& tmKV, const ssdk::GqaPromptArgs& a, int n_max, const ssdk::GqaLatentMaps& lm = {}) {
     const int tile = ssdk::kPromptRows / MAPS;
-    return L.go(ssdk::gqa_prompt_kernel<DK, VD, MAPS>, dim3(((n_max << a.g_shift) + tile - 1) / tile, a.G / MAPS, rg.n_seqs), dim3(ssdk::kPromptThreads),
-                (size_t)ssdk::gqa_prompt_smem(DK, VD), tmQ, tmKV, a, rg);
+    return L.go(ssdk::gqa_prompt_kernel<DK, VD, MAPS, LATENT>, dim3(((n_max << a.g_shift) + tile - 1) / tile, a.G / MAPS, rg.n_seqs), dim3(ssdk::kPromptThreads),
+                (size_t)ssdk::gqa_prompt_smem(DK, VD), tmQ, tmKV, lm, a, rg);
   }
   int gqa_prompt(const HybLayer& Lr, int n_max, const void* pool, void* y, const float* gate, int ld_gate, const void* sinks, float sink_const, const ssdk::DiffArgs& diff) {
     const ssdk_hyb_layer_cfg& c = Lr.c;
@@ -838,6 +838,51 @@ struct HybRun {
     if (c.maps == 2) return c.vdim == 128 ? gqa_prompt_go<128, 128, 2>(tmQ, tmKV, a, n_max) : gqa_prompt_go<128, 64, 2>(tmQ, tmKV, a, n_max);
     if (c.dim == 128) return c.vdim == 128 ? gqa_prompt_go<128, 128, 1>(tmQ, tmKV, a, n_max) : gqa_prompt_go<128, 64, 1>(tmQ, tmKV, a, n_max);
     return c.vdim == 128 ? gqa_prompt_go<64, 128, 1>(tmQ, tmKV, a, n_max) : gqa_prompt_go<64, 64, 1>(tmQ, tmKV, a, n_max);
+  }
+
+  // Latent attention of whole prompts (every sequence of the call starts in it): keys and values of every head are made first, 2 x kv_rank products per
+  // entry, and a (query, key) pair then costs dim + rot + vdim of them instead of 2 kv_rank + rot.
+  bool latent_whole(const HybLayer& Lr, const uint8_t* pool, const float* gate, int ldq) const {
+    const ssdk_hyb_layer_cfg& c = Lr.c;
+    const int H = c.heads, Wd = c.kv_rank + c.rot_dim;
+    if (kF32 || !e->use_tc || !e->use_tc_scores || !pair_ok(M) || c.rot_dim != 64 || !(c.attn_scale > 0.f) || !((c.dim == 128 && c.vdim == 128) || (c.dim == 64 && c.vdim == 64))) return false;
+    if (c.kv_rank % kBlockK || c.vdim > c.kv_rank || (((uintptr_t)pool | (uintptr_t)Lr.t[SSDK_HT_LAT_UKT].p | (uintptr_t)Lr.t[SSDK_HT_LAT_UV].p) & 15) || !whole16(gate ? ldq : 4, {gate})) return false;
+    if ((size_t)M * H * c.dim > 2 * e->att_elems || (size_t)M * H * c.vdim > e->att_elems || (size_t)M * Wd > 2 * (size_t)e->cfg.max_tokens * e->w_lat_o) return false;   // att_s, att_p, att_o
+    for (int s = 0; s < rg.n_seqs; ++s)
+      if (h_pos0[s] != 0 || h_cu[s + 1] - h_cu[s] < 2) return false;
+    return true;
+  }
+  int latent_prompt(const HybLayer& Lr, const uint8_t* pool, const float* gate, int ldq, const void* sink, const ssdk::KeyMask& mask) {
+    const ssdk_hyb_layer_cfg& c = Lr.c;
+    const int H = c.heads, D = c.dim, V = c.vdim, R = c.rot_dim, KR = c.kv_rank, Wd = KR + R;
+    T *rows = (T*)e->att_o, *keys = (T*)e->att_s, *vals = (T*)e->att_p;
+    by_position = true;
+    if constexpr (!kF32) CKI(L.go(ssdk::latent_rows_kernel, dim3(M), dim3(128), 0, (const bf16*)pool, (bf16*)rows, rg, Wd));
+    auto map = [&](const void* p, int64_t n, int cols, int box, CUtensorMap* out) {
+      const CUtensorMap* tm;
+      CKI(e->tmap(p, n, cols, box, &tm));
+      *out = *tm;   // (copied: a later lookup may empty the table)
+      return 0;
+    };
+    CUtensorMap tmW, tmX, tmXs, tmQ, tmK;
+    ssdk::GqaLatentMaps lm;
+    // keys [M, H D] = rows' latents . uk^T, whose columns are contiguous; values [M, H V]
+    CKI(map(Lr.t[SSDK_HT_LAT_UKT].p, (int64_t)H * KR, D, 64, &tmW));
+    CKI(map(rows, M, Wd, kPairXBox, &tmX));
+    CKI(map(rows, M, Wd, kPairXSmall, &tmXs));
+    GemmPairParams p = {};
+    p.out = keys; p.M = M; p.N = p.ldo = H * D; p.num_kb = KR / kBlockK; p.w_tiles = (p.N + 255) / 256; p.chunks = (M + kPairTokens - 1) / kPairTokens; p.w_head = D;
+    CKI(launch_gemm_pair(L, EPI_BF16, tmW, tmX, tmXs, p, p.w_tiles * p.chunks));
+    CKI(lin_heads(rows, Wd, Lr.t[SSDK_HT_LAT_UV].p, KR, vals, H * V, M, H * V, KR, true, 1, 0, 0));
+    ssdk::GqaPromptArgs a = {};
+    a.y = e->t0; a.gate = gate; a.ld_gate = ldq; a.G = H; a.D = D; a.scale_log2 = c.attn_scale * ssdk::kLog2e; a.sinks = sink; a.mask = mask; a.timeout = L.gave_up;
+    a.key_rot = a.query_rot = KR; a.query_ld = Wd;
+    CKI(map(e->t1, M, H * D, ssdk::kPromptRows, &tmQ));
+    CKI(map(e->qcat, M, H * Wd, ssdk::kPromptRows, &lm.q_rot));
+    CKI(map(keys, M, H * D, ssdk::kPromptKeys, &tmK));
+    CKI(map(rows, M, Wd, ssdk::kPromptKeys, &lm.k_rot));
+    CKI(map(vals, M, H * V, ssdk::kPromptKeys, &lm.v));
+    return D == 128 ? gqa_prompt_go<192, 128, 1, true>(tmQ, tmK, a, longest(), lm) : gqa_prompt_go<128, 64, 1, true>(tmQ, tmK, a, longest(), lm);
   }
 
   int latent(HybLayer& Lr) {
@@ -886,6 +931,10 @@ struct HybRun {
     const bool v4 = D % 4 == 0 && R % 4 == 0 && whole16(ldq, {q, e->t1});
     CKI(L.go(v4 ? ssdk::latent_q_kernel<T, 4> : ssdk::latent_q_kernel<T, 1>, dim3(M, (H + ssdk::kQHeads - 1) / ssdk::kQHeads),
              dim3(32 * ssdk::kQHeads), 0, q, ldq, (T*)e->t1, (T*)e->qcat, (const float*)Lr.inv_freq, rg, H, D, R, KR, c.rot_dims, c.rot_interleaved));
+    if (latent_whole(Lr, pool, gate, ldq)) {
+      CKI(latent_prompt(Lr, pool, gate, ldq, sink, mask));
+      return lin(e->t0, H * V, Lr.t[SSDK_HT_MIX_OUT].p, H * V, e->mix_out, W, M, W, H * V);
+    }
     // absorption: qcat[m, h, :kv_rank] = W_uk,h^T qn[m, h, :]
     CKI(lin_heads(e->t1, H * D, Lr.t[SSDK_HT_LAT_UKT].p, D, e->qcat, H * Wd, M, KR, D, true, H, D, Wd));
     // single-token sequences (decode) share ONE fused launch + a merge; the others take the GEMM path below
@@ -1838,10 +1887,11 @@ static int hyb_smem_attrs(ssdk_hyb_engine* e) {
   CK(cudaFuncSetAttribute(ssdk::gqa_portion_mma_kernel<2, 4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   CK(cudaFuncSetAttribute(ssdk::gqa_portion_mma_kernel<4, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   CK(cudaFuncSetAttribute(ssdk::gqa_portion_mma_kernel<8, 16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-#define SSDK_TILE_ATTR(DK, VD, MAPS) \
-  CK(cudaFuncSetAttribute(ssdk::gqa_prompt_kernel<DK, VD, MAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, ssdk::gqa_prompt_smem(DK, VD))); \
-  CK(cudaFuncSetAttribute(ssdk::gqa_prompt_kernel<DK, VD, MAPS>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-  SSDK_TILE_ATTR(128, 128, 2) SSDK_TILE_ATTR(128, 64, 2) SSDK_TILE_ATTR(128, 128, 1) SSDK_TILE_ATTR(128, 64, 1) SSDK_TILE_ATTR(64, 128, 1) SSDK_TILE_ATTR(64, 64, 1)
+#define SSDK_TILE_ATTR(DK, VD, MAPS, LATENT) \
+  CK(cudaFuncSetAttribute(ssdk::gqa_prompt_kernel<DK, VD, MAPS, LATENT>, cudaFuncAttributeMaxDynamicSharedMemorySize, ssdk::gqa_prompt_smem(DK, VD))); \
+  CK(cudaFuncSetAttribute(ssdk::gqa_prompt_kernel<DK, VD, MAPS, LATENT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  SSDK_TILE_ATTR(128, 128, 2, false) SSDK_TILE_ATTR(128, 64, 2, false) SSDK_TILE_ATTR(128, 128, 1, false) SSDK_TILE_ATTR(128, 64, 1, false) SSDK_TILE_ATTR(64, 128, 1, false)
+  SSDK_TILE_ATTR(64, 64, 1, false) SSDK_TILE_ATTR(192, 128, 1, true) SSDK_TILE_ATTR(128, 64, 1, true)
 #undef SSDK_TILE_ATTR
 #define SSDK_RET_ATTR(KS, VT) \
   CK(cudaFuncSetAttribute(ssdk::retention_chunk_state_mma_kernel<KS, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, big)); \

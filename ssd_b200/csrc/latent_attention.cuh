@@ -156,6 +156,15 @@ __global__ void latent_gather_kernel(const T* __restrict__ cache, T* __restrict_
   }
 }
 
+// dst[m, :] = the pool row of token m (rows of whole 16-byte pieces).  grid M
+__global__ void latent_rows_kernel(const __nv_bfloat16* __restrict__ cache, __nv_bfloat16* __restrict__ dst, const Ragged rg, int W) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int m = blockIdx.x, s = rg.tok_seq[m];
+  const uint4* src = reinterpret_cast<const uint4*>(cache + page_row(rg, s, rg.pos0[s] + (m - rg.cu[s])) * W);
+  for (int c = threadIdx.x; c < W / 8; c += blockDim.x) reinterpret_cast<uint4*>(dst + (size_t)m * W)[c] = src[c];
+}
+
 // Which keys a causal query sees: those at first(pos) .. pos, and those before position `keep`.  A sliding window keeps the last
 // `window` positions, chunks are counted from the sequence's start and end at the query's own chunk; 0 = no window, no chunks,
 // no kept first keys.

@@ -55,18 +55,6 @@ SSDK_DEVINL void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, 
       ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Operand that is contiguous along M or N, 128-byte swizzle: atoms of 64 elements x 8 k; the next 8 k follow 1024 B on (SBO), the next 64
-// elements `next64` bytes on (LBO)
-SSDK_DEVINL uint64_t make_umma_desc_mn128(const void* smem_tile, uint32_t next64) {
-  const uint32_t addr = smem_u32(smem_tile);
-  uint64_t d = 0;
-  d |= (uint64_t)((addr >> 4) & 0x3FFFu);
-  d |= (uint64_t)((next64 >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)(1024u >> 4) << 32;
-  d |= (uint64_t)1u << 46;
-  d |= (uint64_t)2u << 61;
-  return d;
-}
 SSDK_DEVINL void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
