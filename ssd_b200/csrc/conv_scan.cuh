@@ -817,19 +817,6 @@ struct DeltaArgs {
   int vec;                           // D and the slot's columns are whole 16-byte pieces
 };
 
-// two fp32 products and sums at once
-SSDK_DEVINL uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-SSDK_DEVINL uint64_t pack2(float x, float y) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
-  return d;
-}
-SSDK_DEVINL void unpack2(uint64_t v, float* x, float* y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(*x), "=f"(*y) : "l"(v)); }
-
 constexpr int kDeltaWarps = 4;
 inline __host__ __device__ int delta_cols(int LC, int NC) { return kDeltaWarps * 32 / LC * NC; }   // value columns of a CTA
 inline size_t delta_scan_smem(int DP, int LC, int NC, int C) { return (size_t)2 * (delta_record(DP, C) + C * delta_cols(LC, NC)) * 4; }

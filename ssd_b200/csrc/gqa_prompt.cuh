@@ -184,10 +184,7 @@ gqa_prompt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         for (int c = 0; c < 64; ++c)
           if (base + c > hi || (base + c < lo && base + c >= p.mask.keep)) u[c] = 0xff800000u;   // -inf
       }
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int c = 0; c < 64; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], __uint_as_float(u[c]));
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+      const float mx = row_max(u) * p.scale_log2;
       const bool grow = mx > m + kPromptSlack;
       if (__any_sync(0xffffffffu, grow)) {
         const float f = grow ? exp2f(m - mx) : 1.f;   // (m = -inf: 0)
@@ -208,15 +205,7 @@ gqa_prompt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         }
       }
       const float ms = m == -INFINITY ? 0.f : m;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int c = 0; c < 64; c += 2) {
-        const float a = exp2f(fmaf(__uint_as_float(u[c]), p.scale_log2, -ms)), e = exp2f(fmaf(__uint_as_float(u[c + 1]), p.scale_log2, -ms));
-        sum4[c & 3] += a;
-        sum4[(c & 3) + 1] += e;
-        u[c >> 1] = pack_bf16x2(a, e);
-      }
-      l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+      l += row_exp(u, p.scale_log2, ms);
       tmem_st_32x32b_x16(sp, u);
       tmem_st_32x32b_x16(sp + 16, u + 16);
       tmem_st_wait();

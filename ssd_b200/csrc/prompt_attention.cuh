@@ -65,6 +65,36 @@ SSDK_DEVINL void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t* r) {
 }
 SSDK_DEVINL void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// largest of a row's 64 scores
+SSDK_DEVINL float row_max(const uint32_t (&u)[64]) {
+  float m[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) m[c] = max3(__uint_as_float(u[c]), __uint_as_float(u[c + 4]), __uint_as_float(u[c + 8]));
+#pragma unroll
+  for (int c = 12; c < 60; c += 8)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) m[e] = max3(m[e], __uint_as_float(u[c + e]), __uint_as_float(u[c + 4 + e]));
+  return fmaxf(max3(m[0], m[1], __uint_as_float(u[60])), max3(m[2], m[3], max3(__uint_as_float(u[61]), __uint_as_float(u[62]), __uint_as_float(u[63]))));
+}
+// 2^(score * scale - ms) of a row: rounded to bf16 in the first 32 words, their sum (of the unrounded ones) back.  Products and sums two at a time; a probability
+// below 2^-126 is zero (the row's largest is at least 2^-kPromptSlack).
+SSDK_DEVINL float row_exp(uint32_t (&u)[64], float scale, float ms) {
+  const uint64_t sc = pack2(scale, scale), off = pack2(-ms, -ms);
+  uint64_t sum[2] = {0, 0};
+#pragma unroll
+  for (int c = 0; c < 64; c += 2) {
+    float a, e;
+    unpack2(fma2(pack2(__uint_as_float(u[c]), __uint_as_float(u[c + 1])), sc, off), &a, &e);
+    a = ex2_ftz(a); e = ex2_ftz(e);
+    sum[(c >> 1) & 1] = add2(sum[(c >> 1) & 1], pack2(a, e));
+    u[c >> 1] = pack_bf16x2(a, e);
+  }
+  float s0, s1, s2, s3;
+  unpack2(sum[0], &s0, &s1);
+  unpack2(sum[1], &s2, &s3);
+  return (s0 + s1) + (s2 + s3);
+}
+
 // grid (kv heads, q tiles, sequences x ranges)
 template <int HD, bool SPLIT>
 __global__ void __launch_bounds__(kPromptThreads, 2)
@@ -201,10 +231,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int c = 0; c < 64; ++c)
           if (base + c >= lim) u[c] = 0xff800000u;   // -inf
       }
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int c = 0; c < 64; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], __uint_as_float(u[c]));
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+      const float mx = row_max(u) * p.scale_log2;
       const bool grow = mx > m + kPromptSlack;
       if (__any_sync(0xffffffffu, grow)) {
         const float f = grow ? exp2f(m - mx) : 1.f;   // (m = -inf: 0)
@@ -225,15 +252,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
       }
       const float ms = m == -INFINITY ? 0.f : m;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int c = 0; c < 64; c += 2) {
-        const float a = exp2f(fmaf(__uint_as_float(u[c]), p.scale_log2, -ms)), e = exp2f(fmaf(__uint_as_float(u[c + 1]), p.scale_log2, -ms));
-        sum4[c & 3] += a;
-        sum4[(c & 3) + 1] += e;
-        u[c >> 1] = pack_bf16x2(a, e);
-      }
-      l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+      l += row_exp(u, p.scale_log2, ms);
       tmem_st_32x32b_x16(sp, u);
       tmem_st_32x32b_x16(sp + 16, u + 16);
       tmem_st_wait();
