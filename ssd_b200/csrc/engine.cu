@@ -291,12 +291,13 @@ static int launch_gemm_split(Launcher& L, const CUtensorMap& tmX, GemmSplitParam
 // tiles of tokens cost registers for the loads in flight (16 rows of llama-3.2-1b 412 -> 430 us).
 static bool few_rows(int M, int64_t N, int K) { return M <= kFewTokens && N * K * 2 <= (30 << 20); }
 // fp32, bf16 or act(gate) * up in bf16; W and X start on 16-byte boundaries, their strides are whole 16-byte pieces, K % 64 == 0
-static int launch_gemm_few(Launcher& L, int epi, const void* X, int ldx, const void* W, int ldw, void* out, int ldo, int M, int N, int K, bool gelu = false) {
+static int launch_gemm_few(Launcher& L, int epi, const void* X, int ldx, const void* W, int ldw, void* out, int ldo, int M, int N, int K, bool gelu = false,
+                           int heads = 1, int x_step = 0, int out_step = 0) {
   GemmFewParams p;
-  p.W = (const bf16*)W; p.X = (const bf16*)X; p.out = out; p.M = M; p.N = N; p.K = K; p.ldw = ldw; p.ldx = ldx; p.ldo = ldo; p.gelu = gelu;
+  p.W = (const bf16*)W; p.X = (const bf16*)X; p.out = out; p.M = M; p.N = N; p.K = K; p.ldw = ldw; p.ldx = ldx; p.ldo = ldo; p.gelu = gelu; p.x_step = x_step; p.out_step = out_step;
   const int cols = epi == FEW_SILU || epi == FEW_GLU ? kFewRows / 2 : kFewRows, tiles = (N + cols - 1) / cols;
   const int warps = K <= 1024 ? kFewWarps / 2 : kFewWarps;   // (at least four units of k per warp)
-  const dim3 grid(std::min(tiles, num_sms() * 2 * kFewWarps / warps)), block(32 * warps);
+  const dim3 grid(std::min(tiles, std::max(1, num_sms() * 2 * kFewWarps / warps / heads)), heads), block(32 * warps);
   if (epi == FEW_F32) return L.go(gemm_few_kernel<FEW_F32>, grid, block, 0, p);
   if (epi == FEW_BF16) return L.go(gemm_few_kernel<FEW_BF16>, grid, block, 0, p);
   if (epi == FEW_SILU) return L.go(gemm_few_kernel<FEW_SILU>, grid, block, 0, p);

@@ -29,6 +29,7 @@ struct GemmFewParams {
   void* out;                // [M, ldo]: fp32 or bf16
   int M, N, K, ldw, ldx, ldo;
   int gelu;                 // FEW_GLU: gelu_tanh instead of silu
+  int x_step, out_step;     // products side by side (heads): product b reads X's columns from b x_step, the weight rows from b N, and writes out + b out_step
 };
 
 template <int EPI>
@@ -40,13 +41,14 @@ __global__ void __launch_bounds__(kFewWarps * 32, 2) gemm_few_kernel(const GemmF
   const int g = lane >> 2, t = lane & 3;
   const int tiles = (p.N + COLS - 1) / COLS;
   const int units = p.K / kFewUnit, u0 = warp * units / nw, u1 = (warp + 1) * units / nw;
+  const __nv_bfloat16 *W = p.W + (size_t)blockIdx.y * p.N * p.ldw, *X = p.X + (size_t)blockIdx.y * p.x_step;
   const bool keep_x = u1 - u0 <= D;   // this warp's part of X stays in its registers
 
   const __nv_bfloat16 *wa, *wb;       // this thread's two weight rows of a tile
   auto rows_of = [&](int tile) {
     const int r = min(tile * COLS + g, p.N - 1);   // (columns behind N are multiplied and dropped)
-    wa = p.W + (size_t)r * p.ldw + t * 8;
-    wb = p.W + (size_t)(GATED ? r + p.N : min(tile * COLS + g + 8, p.N - 1)) * p.ldw + t * 8;
+    wa = W + (size_t)r * p.ldw + t * 8;
+    wb = W + (size_t)(GATED ? r + p.N : min(tile * COLS + g + 8, p.N - 1)) * p.ldw + t * 8;
   };
   uint4 w[D][4], x[D][2];
   auto load_w = [&](uint4* v, int u) {
@@ -56,7 +58,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 2) gemm_few_kernel(const GemmF
     v[3] = ld_nc_v4_evict_first(wb + u * kFewUnit + 32);
   };
   auto load_x = [&](uint4* v, int u) {
-    const uint4* src = reinterpret_cast<const uint4*>(p.X + (size_t)g * p.ldx + u * kFewUnit + t * 8);
+    const uint4* src = reinterpret_cast<const uint4*>(X + (size_t)g * p.ldx + u * kFewUnit + t * 8);
     v[0] = g < p.M ? src[0] : make_uint4(0u, 0u, 0u, 0u);
     v[1] = g < p.M ? src[4] : make_uint4(0u, 0u, 0u, 0u);
   };
@@ -113,7 +115,7 @@ __global__ void __launch_bounds__(kFewWarps * 32, 2) gemm_few_kernel(const GemmF
         if (col >= 8) src += up;
         for (int q = 0; q < nw; ++q) s += src[q * 132];
       }
-      const size_t at = (size_t)m * p.ldo + n;
+      const size_t at = (size_t)m * p.ldo + (size_t)blockIdx.y * p.out_step + n;
       if (EPI == FEW_F32) {
         reinterpret_cast<float*>(p.out)[at] = s;
       } else if (EPI == FEW_BF16) {
