@@ -31,7 +31,7 @@
 namespace ssdk {
 
 constexpr int kSplitTokens = 192, kSplitStages = 2, kSplitThreads = 512, kSplitSegment = 4;   // segment: k-blocks between two drains
-constexpr int kSplitXBox = 32;
+constexpr int kSplitXBox = 32, kSplitSeeTiles = 128;
 constexpr int kSplitWPlane = 128 * 128, kSplitXPlane = kSplitTokens / 2 * 128, kSplitStageBytes = 3 * (kSplitWPlane + kSplitXPlane);
 constexpr int kSplitSmem = kSplitStages * kSplitStageBytes + 1024;
 
@@ -52,6 +52,10 @@ struct GemmSplitParams {
   const int* g_tile_row0;
   const int* g_tile_rows;
   const int* g_n_tiles;
+  // Attention (dense, splits 1): row r of a matrix has to do with columns (see_k: steps of k) below see + r / see_heads only.  Tiles beyond are left
+  // out, or k ends there (X holds what lies between a row's own end and that of its chunk's last row; chunks then go from the longest to the
+  // shortest, there and back over the pairs).  see_heads 0: all of it
+  int see, see_heads, see_k;
   unsigned* timeout;
 };
 
@@ -68,17 +72,17 @@ SSDK_DEVINL void split3(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l)
   l = *reinterpret_cast<const uint32_t*>(&ll);
 }
 
-// rows of X as three pieces: dst [3][batch * M, K] (bf16).  grid (M, batch): row r of matrix b (`stride` floats apart) is row rows[r] of src
-// if there is a list; rows from *n_rows on are left out
+// rows of X as three pieces: dst [3][batch * M, K] (bf16).  grid (ceil(M / blockDim.y), batch): row r of matrix b (`stride` floats apart) is row rows[r]
+// of src if there is a list; rows from *n_rows on are left out.  Narrow rows share a block: 25152 rows of 64 columns 25 -> 4 us
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ src, int ld, long long stride, const int* __restrict__ rows,
-                                                         const int* __restrict__ n_rows, __nv_bfloat16* __restrict__ dst, int K) {
+                                                         const int* __restrict__ n_rows, __nv_bfloat16* __restrict__ dst, int M, int K) {
   pdl_launch_dependents();
   pdl_wait();
-  const int r = blockIdx.x;
-  if (n_rows && r >= *n_rows) return;
+  const int r = blockIdx.x * blockDim.y + threadIdx.y;
+  if (r >= M || (n_rows && r >= *n_rows)) return;
   const float4* s = reinterpret_cast<const float4*>(src + blockIdx.y * stride + (size_t)(rows ? rows[r] : r) * ld);
-  const size_t plane = (size_t)gridDim.x * gridDim.y * K;
-  __nv_bfloat16* d = dst + ((size_t)blockIdx.y * gridDim.x + r) * K;
+  const size_t plane = (size_t)M * gridDim.y * K;
+  __nv_bfloat16* d = dst + ((size_t)blockIdx.y * M + r) * K;
   for (int c = threadIdx.x; c < K / 4; c += blockDim.x) {
     const float4 v = s[c];
     uint2 h, m, l;
@@ -111,6 +115,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
   __shared__ __align__(8) uint64_t main_full, main_empty, rest_full, rest_empty;
   __shared__ uint32_t tmem_slot;
   __shared__ int s_again;   // some result of this CTA's is to be taken again
+  __shared__ int s_seen[kSplitSeeTiles + 1];   // tiles in front of a column tile's, where some are left out
   uint8_t* smem = split_smem_raw + ((1024u - (smem_u32(split_smem_raw) & 1023u)) & 1023u);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -123,6 +128,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
     mbar_init(&main_full, 1); mbar_init(&main_empty, 8); mbar_init(&rest_full, 1); mbar_init(&rest_empty, 8);   // four sum warps in each CTA
     fence_mbar_init();
     s_again = 0;
+    if (p.see_heads && !p.see_k) {   // column tile w: the chunks from that of the first row which sees column 256 w
+      s_seen[0] = 0;
+      for (int w = 0; w < p.w_tiles; ++w) s_seen[w + 1] = s_seen[w] + max(0, p.chunks - max(0, w * 256 - p.see + 1) * p.see_heads / p.tokens);
+    }
   }
   if (warp == 1) tmem_alloc_pair(&tmem_slot);
   tc_fence_before();
@@ -136,14 +145,31 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
 
   const bool grouped = p.g_tile_expert != nullptr;
   const int row_tiles = grouped ? *p.g_n_tiles : p.chunks;
-  const int per = row_tiles * p.splits * p.w_tiles, tiles = grouped ? per : per * p.batch;
+  const bool see_k = p.see_heads && p.see_k, see_cols = p.see_heads && !p.see_k;
+  const int per = see_cols ? s_seen[p.w_tiles] : row_tiles * p.splits * p.w_tiles, tiles = grouped ? per : per * p.batch;
+  // this pair's i-th tile
+  auto tile_at = [&](int i) { return i * n_pairs + (see_k && (i & 1) ? n_pairs - 1 - pair : pair); };
   struct Tile { int m0, rows, n, col, kb0, kb1, split, b; long long w0; };
   auto tile_of = [&](int t) {   // row chunk (innermost), k range, 256 columns, matrix of the batch
     Tile r;
-    r.b = grouped ? 0 : t / per;
-    t -= r.b * per;
-    const int u = t / row_tiles, c = t - u * row_tiles, wt = u / p.splits;
-    r.split = u - wt * p.splits;
+    int c, wt;
+    r.split = 0;
+    if (see_k) {
+      r.b = t % p.batch;
+      t /= p.batch;
+      wt = t % p.w_tiles; c = p.chunks - 1 - t / p.w_tiles;
+    } else {
+      r.b = grouped ? 0 : t / per;
+      t -= r.b * per;
+      if (see_cols) {
+        for (wt = 0; s_seen[wt + 1] <= t; ++wt);
+        c = p.chunks - (s_seen[wt + 1] - t);
+      } else {
+        const int u = t / row_tiles;
+        c = t - u * row_tiles; wt = u / p.splits;
+        r.split = u - wt * p.splits;
+      }
+    }
     if (grouped) {
       r.m0 = p.g_tile_row0[c]; r.rows = min(kSplitTokens, p.g_tile_rows[c]); r.w0 = p.g_tile_expert[c] * p.w_stride;
     } else {
@@ -153,6 +179,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
     r.col = wt * 256 + (int)rank * 128;
     r.kb0 = r.split * p.kb_per_split;
     r.kb1 = min(p.num_kb, r.kb0 + p.kb_per_split);
+    if (see_k) r.kb1 = min(r.kb1, (p.see + (r.m0 + r.rows - 1) / p.see_heads + kBlockK - 1) / kBlockK);
     return r;
   };
 
@@ -161,7 +188,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
     if (warp == 0 && lane == 0) {
       int it = 0;
       bool ok = true;
-      for (int t = pair; t < tiles && ok; t += n_pairs) {
+      for (int i = 0, t; (t = tile_at(i)) < tiles && ok; ++i) {
         const Tile tl = tile_of(t);
         const int half = tl.n >> 1, x0 = tl.b * p.M + tl.m0 + (int)rank * half, boxes = (half + kSplitXBox - 1) / kSplitXBox;
         for (int kb = tl.kb0; kb < tl.kb1; ++kb, ++it) {
@@ -181,7 +208,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
     } else if (warp == 1 && lane == 0 && rank == 0) {
       int it = 0, nt = 0, sg = 0;
       bool ok = true;
-      for (int t = pair; t < tiles && ok; t += n_pairs, ++nt) {
+      for (int t; (t = tile_at(nt)) < tiles && ok; ++nt) {
         const Tile tl = tile_of(t);
         const uint32_t idesc = make_umma_idesc_bf16(256, tl.n);
         if (!(ok = mbar_wait_cluster(&rest_empty, ((uint32_t)nt & 1u) ^ 1u, p.timeout))) break;
@@ -222,7 +249,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
     const int q = warp & 3;
     int nt = 0, sg = 0;
     bool ok = true;
-    for (int t = pair; t < tiles && ok; t += n_pairs, ++nt) {
+    for (int t; (t = tile_at(nt)) < tiles && ok; ++nt) {
       const Tile tl = tile_of(t);
       float acc[kSplitTokens];
 #pragma unroll
@@ -280,7 +307,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
       v[2 * i] = in ? __ldg(at) : make_float4(0.f, 0.f, 0.f, 0.f);
       v[2 * i + 1] = in ? __ldg(at + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
-    int it = 0, t = pair, kb = 0;
+    int it = 0, step = 0, t = tile_at(0), kb = 0;
     Tile tl = {};
     if (t < tiles) {
       tl = tile_of(t);
@@ -293,7 +320,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
     while (t < tiles && ok) {
       int t2 = t, kb2 = kb + 1;   // the k-block after this one
       if (kb2 >= tl.kb1) {
-        t2 += n_pairs;
+        t2 = tile_at(++step);
         if (t2 < tiles) { tl = tile_of(t2); kb2 = tl.kb0; rows_of(tl); }
       }
       const int s = it % kSplitStages;
@@ -324,7 +351,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
   tc_fence_before();
   __syncthreads();
   if (s_again) {   // (nothing waits for this CTA any more but its partner's exit)
-    for (int t = pair; t < tiles; t += n_pairs) {
+    for (int j = 0, t; (t = tile_at(j)) < tiles; ++j) {
       const Tile tl = tile_of(t);
       for (int i = threadIdx.x; i < tl.rows * 128; i += kSplitThreads) {
         const int r = tl.m0 + (i >> 7), n = tl.col + (i & 127);

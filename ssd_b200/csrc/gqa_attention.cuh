@@ -369,23 +369,37 @@ __global__ void gqa_head_prep_kernel(const GqaHeadPrepArgs p, const Ragged rg) {
   }
 }
 
-// grid (ctx_pad): the key of index lo - kept + j of sequence s (KeyMask) -> keys[g][j][:] and vt[g][:][j] (a value head once per map that
-// shares it); zero from ctx up to ctx_pad
+// grid (ceil(ctx_pad / kKvKeys), G), block (32, 8): the keys of indexes lo - kept + j of sequence s (KeyMask) -> keys[g][j][:] and vt[g][:][j] (a value head
+// once per map that shares it); zero from ctx up to ctx_pad.  The values turn in shared memory, so that both sides move whole lines: 8 heads of 64 and
+// 128 columns, 1000 keys in 32 bits 17 -> 13 us
+constexpr int kKvKeys = 32;
 template <typename T>
-__global__ void kv_gather_kernel(const T* __restrict__ cache, T* __restrict__ keys, T* __restrict__ vt, const Ragged rg, int s,
-                                 int lo, int kept, int ctx, int ctx_pad, int G, int D, int V, int maps) {
+__global__ void __launch_bounds__(256) kv_gather_kernel(const T* __restrict__ cache, T* __restrict__ keys, T* __restrict__ vt, const Ragged rg, int s,
+                                                        int lo, int kept, int ctx, int ctx_pad, int G, int D, int V, int maps) {
+  __shared__ T tile[kKvKeys][kKvKeys + 1];
   pdl_launch_dependents();
   pdl_wait();
-  const int j = blockIdx.x;
+  const int j0 = blockIdx.x * kKvKeys, g = blockIdx.y, x = threadIdx.x, y = threadIdx.y;
   const size_t roww = (size_t)G * D + (size_t)(G / maps) * V;
-  const T* row = j < ctx ? cache + page_row(rg, s, key_position(lo - kept + j, lo, kept)) * roww : nullptr;
-  for (int i = threadIdx.x; i < G * D; i += blockDim.x) {
-    const int g = i / D, d = i - g * D;
-    keys[((size_t)g * ctx_pad + j) * D + d] = row ? row[i] : T(0.f);
+  const T* row[kKvKeys / 8];   // this warp's keys y, y + 8, ..
+#pragma unroll
+  for (int i = 0; i < kKvKeys / 8; ++i) {
+    const int j = j0 + y + 8 * i;
+    row[i] = j < ctx ? cache + page_row(rg, s, key_position(lo - kept + j, lo, kept)) * roww : nullptr;
+    if (j < ctx_pad)
+      for (int d = x; d < D; d += 32) keys[((size_t)g * ctx_pad + j) * D + d] = row[i] ? row[i][(size_t)g * D + d] : T(0.f);
   }
-  for (int i = threadIdx.x; i < G * V; i += blockDim.x) {
-    const int g = i / V, v = i - g * V;
-    vt[(size_t)i * ctx_pad + j] = row ? row[(size_t)G * D + (size_t)(g / maps) * V + v] : T(0.f);
+  const size_t v_at = (size_t)G * D + (size_t)(g / maps) * V;
+  for (int v0 = 0; v0 < V; v0 += 32) {
+#pragma unroll
+    for (int i = 0; i < kKvKeys / 8; ++i) tile[y + 8 * i][x] = row[i] && v0 + x < V ? row[i][v_at + v0 + x] : T(0.f);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int v = v0 + y + 8 * i;
+      if (v < V && j0 + x < ctx_pad) vt[((size_t)g * V + v) * ctx_pad + j0 + x] = tile[x][y + 8 * i];
+    }
+    __syncthreads();
   }
 }
 

@@ -573,15 +573,19 @@ struct HybRun {
     }
     return p.chunks;
   }
-  int go_split(const void* A, int lda, long long sA, const int* gather, const int* n_rows, int m, int batch, GemmSplitParams& p, int row_tiles) {
-    CKI(L.go(ssdk::split_rows_kernel, dim3(m, batch), dim3(std::min(256, (p.K / 4 + 31) / 32 * 32)), 0, (const float*)A, lda, sA, gather, n_rows, (bf16*)e->pieces, p.K));
+  // ready: the pieces of A are there
+  int go_split(const void* A, int lda, long long sA, const int* gather, const int* n_rows, int m, int batch, GemmSplitParams& p, int row_tiles, bool ready = false) {
+    int tx = 256;   // threads of a row
+    while (tx > 8 && tx >= p.K / 2) tx /= 2;
+    if (!ready)
+      CKI(L.go(ssdk::split_rows_kernel, dim3((m + 256 / tx - 1) / (256 / tx), batch), dim3(tx, 256 / tx), 0, (const float*)A, lda, sA, gather, n_rows, (bf16*)e->pieces, m, p.K));
     const CUtensorMap* tm;
     CKI(e->tmap(e->pieces, 3LL * m * batch, p.K, kSplitXBox, &tm));
     p.X = (const float*)A; p.ldx = lda; p.x_stride = sA; p.x_rows = gather;
     p.M = m; p.plane_rows = m * batch; p.batch = batch; p.num_kb = (p.K + kBlockK - 1) / kBlockK; p.w_tiles = (p.N + 255) / 256;
     p.kb_per_split = (p.num_kb + kSplitSegment - 1) / kSplitSegment * kSplitSegment;
     p.splits = 1;
-    if (!p.g_tile_expert) row_tiles = split_plan(p, p.ldc == p.N ? e->partial_floats : 0);
+    if (!p.g_tile_expert) row_tiles = split_plan(p, p.ldc == p.N && !p.see_heads ? e->partial_floats : 0);
     const int tiles = p.w_tiles * row_tiles * batch;
     float* C = p.out;
     if (p.splits > 1) p.out = e->partials;
@@ -598,6 +602,16 @@ struct HybRun {
     p.W = (const float*)Wm; p.out = C; p.N = p.ldc = N; p.K = p.ldw = K; p.w_stride = (long long)N * K;
     p.g_tile_expert = e->tile_expert; p.g_tile_row0 = e->tile_row0; p.g_tile_rows = e->tile_rows; p.g_n_tiles = e->n_tiles;
     return go_split(X, ldx, 0, gather, e->n_rows, rows, 1, p, max_tiles);
+  }
+  // attention in 32 bits, per key head: rows x keys (in_k false) and weights x values (in_k true), where row r has to do with the first see + r / heads keys
+  // only: up to half of the work of a prompt (786 queries of 32 maps: products of 64 columns 98 -> 52 us, with the values 93 -> 73).  `ready`: the softmax left
+  // the weights' pieces
+  int lin_seen(const void* A, int lda, const void* W, int ldw, float* C, int ldc, int m, int N, int K, int batch, long long sA, long long sW, long long sC, int see, int heads,
+               bool in_k, bool ready) {
+    GemmSplitParams p = {};
+    p.W = (const float*)W; p.out = C; p.N = N; p.K = K; p.ldw = ldw; p.ldc = ldc; p.w_stride = sW; p.c_stride = sC;
+    if (in_k || (N + 255) / 256 <= kSplitSeeTiles) { p.see = see; p.see_heads = heads; p.see_k = in_k; }
+    return go_split(A, lda, sA, nullptr, nullptr, m, batch, p, 0, ready);
   }
   // C[M, N] (fp32 unless out_t) = A[M, K] W[N, K]^T
   int lin(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int m, int N, int K, bool out_t = false,
@@ -753,14 +767,20 @@ struct HybRun {
       return L.go(ssdk::attn_gate_kernel<T, 4>, dim3(n, per), dim3(128), 0, o, gate, ldg, (T*)y, m_total, H, G, V, row0);
     return L.go(ssdk::attn_gate_kernel<T, 1>, dim3(n), dim3(256), 0, o, gate, ldg, (T*)y, m_total, H, G, V, row0);
   }
-  // att_s [n, ld] -> att_p: a row of up to 8 ld-pieces per thread stays in registers
-  int softmax(int n, const void* sink, int H, int ld, int pos_first, float scale, int rows_per_batch, float sink_const, int key_first, int kept, ssdk::KeyMask mask) {
+  static bool softmax_holds(int ld) { return ld % 4 == 0 && ld <= 8192; }   // (the forms that also leave the pieces)
+  // att_s [n, ld] -> att_p: a row stays in the registers of a warp or of a block
+  int softmax(int n, const void* sink, int H, int ld, int pos_first, float scale, int rows_per_batch, float sink_const, int key_first, int kept, ssdk::KeyMask mask,
+              bool pieces = false) {
     const float* sc = e->att_s;
     T* pr = (T*)e->att_p;
     const T* sk = (const T*)sink;
-    const int threads = ld <= 1024 ? 128 : 256, hold = (ld + 4 * threads - 1) / (4 * threads);
-    if (ld % 4 == 0 && hold <= 2) return L.go(ssdk::sink_softmax_row_kernel<T, 2>, dim3(n), dim3(threads), 0, sc, pr, sk, H, ld, pos_first, scale, rows_per_batch, sink_const, key_first, kept, mask);
-    if (ld % 4 == 0 && hold <= 8) return L.go(ssdk::sink_softmax_row_kernel<T, 8>, dim3(n), dim3(threads), 0, sc, pr, sk, H, ld, pos_first, scale, rows_per_batch, sink_const, key_first, kept, mask);
+    bf16* to = pieces ? (bf16*)e->pieces : nullptr;
+    const size_t plane = (size_t)n * ld;
+    if (ld % 4 == 0 && ld <= ssdk::kSoftmaxWarpLd)
+      return L.go(ssdk::sink_softmax_warp_kernel<T>, dim3((n + ssdk::kSoftmaxWarps - 1) / ssdk::kSoftmaxWarps), dim3(ssdk::kSoftmaxWarps * 32), 0, sc, pr, sk, n, H, ld, pos_first, scale,
+                  rows_per_batch, sink_const, key_first, kept, mask, to, plane);
+    if (softmax_holds(ld))
+      return L.go(ssdk::sink_softmax_row_kernel<T, 8>, dim3(n), dim3(256), 0, sc, pr, sk, H, ld, pos_first, scale, rows_per_batch, sink_const, key_first, kept, mask, to, plane);
     return L.go(ssdk::sink_softmax_kernel<T>, dim3(n), dim3(256), 0, sc, pr, sk, H, ld, pos_first, scale, rows_per_batch, sink_const, key_first, kept, mask);
   }
 
@@ -997,10 +1017,15 @@ struct HybRun {
         const T* krows = (const T*)e->keys + (size_t)kb * Wd;
         const T* lat_t = (const T*)e->lat_t + kb;
         // scores: keys are the 128-row operand, (query, head) rows the tokens
-        CKI(lin(qrows, Wd, krows, Wd, e->att_s, cb, rows, cb, Wd, false, 1, 0, 0, 0, tc_attn, true));
-        CKI(softmax(rows, sink, H, cb, p0 + q0, c.attn_scale, rows, 0.f, lo + kb, 0, mask));
+        const int see = p0 + q0 - (lo + kb) + 1;
+        if (split_ok(qrows, Wd, krows, Wd, rows, cb, Wd, 1, 0, 0)) CKI(lin_seen(qrows, Wd, krows, Wd, e->att_s, cb, rows, cb, Wd, 1, 0, 0, 0, see, H, false, false));
+        else CKI(lin(qrows, Wd, krows, Wd, e->att_s, cb, rows, cb, Wd, false, 1, 0, 0, 0, tc_attn, true));
+        const bool pv = softmax_holds(cb) && split_ok(e->att_p, cb, lat_t, ctx_pad, rows, KR, cb, 1, 0, 0);
+        CKI(softmax(rows, sink, H, cb, p0 + q0, c.attn_scale, rows, 0.f, lo + kb, 0, mask, pv));
         T* o_rows = (T*)e->t0 + (size_t)(r0 + q0) * H * KR;
-        if (tc_attn && pair_ok(rows) && tc_ok(e->att_p, cb, lat_t, ctx_pad, KR, KR, cb)) {
+        if (pv) {
+          CKI(lin_seen(e->att_p, cb, lat_t, ctx_pad, (float*)o_rows, KR, rows, KR, cb, 1, 0, 0, 0, see, H, true, true));
+        } else if (tc_attn && pair_ok(rows) && tc_ok(e->att_p, cb, lat_t, ctx_pad, KR, KR, cb)) {
           CKI(lin_heads(e->att_p, cb, lat_t, ctx_pad, o_rows, KR, rows, KR, cb, true, 1, 0, 0));
         } else if (tc_attn && tc_ok(e->att_p, cb, lat_t, ctx_pad, KR, KR, cb)) {
           // P C: the transposed latents [kv_rank, ctx_pad] are the 128-row operand, read with the row stride of the gather
@@ -1396,7 +1421,8 @@ struct HybRun {
       int lo = mask.first(p0), kept = mask.kept(lo), ctx = p0 + n - lo + kept, ctx_pad = (ctx + 7) / 8 * 8;   // the kept keys, then lo .. p0 + n - 1
       const bool per_block = mask.keep > 0;   // kept keys must lie beside a block's own: every query block is gathered by itself
       auto gather = [&]() {
-        return L.go(ssdk::kv_gather_kernel<T>, dim3(ctx_pad), dim3(128), 0, (const T*)pool, (T*)e->keys, (T*)e->lat_t, rg, s, lo, kept, ctx, ctx_pad, G, D, V, maps);
+        return L.go(ssdk::kv_gather_kernel<T>, dim3((ctx_pad + ssdk::kKvKeys - 1) / ssdk::kKvKeys, G), dim3(32, 8), 0, (const T*)pool, (T*)e->keys, (T*)e->lat_t, rg, s, lo, kept, ctx,
+                    ctx_pad, G, D, V, maps);
       };
       if (!per_block) CKI(gather());
       const int qb = (int)std::max<size_t>(1, e->att_elems / ((size_t)H * ctx_pad));
@@ -1409,11 +1435,16 @@ struct HybRun {
         const int rows = nq * hpg, kb = (mask.first(p0 + q0) - lo) / 8 * 8;
         const int cb = (p0 + q0 + nq - lo + kept - kb + 7) / 8 * 8;   // gathered keys kb .. kb + cb - 1 are what this block can see
         const T* qrows = (const T*)e->qcat + (size_t)(r0 + q0) * hpg * D;
-        CKI(lin(qrows, D, (const T*)e->keys + (size_t)kb * D, D, e->att_s, cb, rows, cb, D, false, G, (long long)M * hpg * D, (long long)ctx_pad * D,
-                (long long)rows * cb, false));
-        CKI(softmax(G * rows, sinks, hpg, cb, p0 + q0, c.attn_scale, rows, sink_const, lo + kb, kept, mask));
-        CKI(lin(e->att_p, cb, (const T*)e->lat_t + kb, ctx_pad, og + (size_t)(r0 + q0) * hpg * V, V, rows, V, cb, false, G, (long long)rows * cb,
-                (long long)V * ctx_pad, (long long)M * hpg * V, false));
+        const T *krows = (const T*)e->keys + (size_t)kb * D, *values = (const T*)e->lat_t + kb;
+        const long long sq = (long long)M * hpg * D, sk = (long long)ctx_pad * D, ss = (long long)rows * cb, sv = (long long)V * ctx_pad, so = (long long)M * hpg * V;
+        float* o = og + (size_t)(r0 + q0) * hpg * V;
+        const int see = p0 + q0 - (lo + kb) + kept + 1;
+        if (split_ok(qrows, D, krows, D, rows, cb, D, G, sq, sk)) CKI(lin_seen(qrows, D, krows, D, e->att_s, cb, rows, cb, D, G, sq, sk, ss, see, hpg, false, false));
+        else CKI(lin(qrows, D, krows, D, e->att_s, cb, rows, cb, D, false, G, sq, sk, ss, false));
+        const bool pv = softmax_holds(cb) && split_ok(e->att_p, cb, values, ctx_pad, rows, V, cb, G, ss, sv);
+        CKI(softmax(G * rows, sinks, hpg, cb, p0 + q0, c.attn_scale, rows, sink_const, lo + kb, kept, mask, pv));
+        if (pv) CKI(lin_seen(e->att_p, cb, values, ctx_pad, o, V, rows, V, cb, G, ss, sv, so, see, hpg, true, true));
+        else CKI(lin(e->att_p, cb, values, ctx_pad, o, V, rows, V, cb, false, G, ss, sv, so, false));
       }
       if (maps == 2) CKI(L.go(ssdk::diff_heads_kernel<T>, dim3(n, (H / 2 + 3) / 4), dim3(128), 0, (const float*)og, diff, (T*)y, M, H, G, V, r0));
       else CKI(attn_gate(og, gate, ld_gate, y, n, M, H, G, V, r0));

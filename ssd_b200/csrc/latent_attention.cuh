@@ -21,6 +21,7 @@
 //                        sequences in one launch, split along the context (scores, running maximum and P C per split,
 //                        fp32), latent_decode_merge_kernel joins the splits and adds the sink to the denominator.
 #pragma once
+#include "gemm_split.cuh"  // split3, kSplitTokens
 #include "layer_ops.cuh"
 
 namespace ssdk {
@@ -221,12 +222,24 @@ __global__ void sink_softmax_kernel(const float* __restrict__ sc, T* __restrict_
     st_f<T>(pr + (size_t)r * ld + j, ((j >= j0 && j < n) || j < jk) ? expf(srow[j] * scale - mx) * inv : 0.f);
 }
 
+// four weights' three bf16 pieces (see gemm_split.cuh), a plane apart
+SSDK_DEVINL void store_pieces(__nv_bfloat16* d, size_t plane, const float (&o)[4]) {
+  uint2 h, m, l;
+  split3(o[0], o[1], h.x, m.x, l.x);
+  split3(o[2], o[3], h.y, m.y, l.y);
+  *reinterpret_cast<uint2*>(d) = h;
+  *reinterpret_cast<uint2*>(d + plane) = m;
+  *reinterpret_cast<uint2*>(d + 2 * plane) = l;
+}
+
 // The same for rows of up to 4 HOLD blockDim columns (ld a multiple of 4): four columns per thread and piece, held in registers, so that a
 // score is read once and its exponential taken once.  Only visible columns are read; all are written.  16 heads x 1000 rows x 1000
-// keys: 44 -> 27 us
+// keys: 44 -> 27 us.  With `pieces` ([3][rows, ld], `plane` elements each) the weights' three bf16 pieces for gemm_split_kernel are written too, and of a row
+// only what a chunk of kSplitTokens rows from it on takes: the product ends k there
 template <typename T, int HOLD>
 __global__ void sink_softmax_row_kernel(const float* __restrict__ sc, T* __restrict__ pr, const T* __restrict__ sink, int H, int ld,
-                                        int pos_first, float scale, int rows_per_batch, float sink_const, int key_first, int kept, KeyMask mask) {
+                                        int pos_first, float scale, int rows_per_batch, float sink_const, int key_first, int kept, KeyMask mask,
+                                        __nv_bfloat16* __restrict__ pieces, size_t plane) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float red[33];
@@ -270,14 +283,84 @@ __global__ void sink_softmax_row_kernel(const float* __restrict__ sc, T* __restr
     }
   sum = block_sum(sum, red) + expf(sk - mx);
   const float inv = 1.0f / sum;
+  const int end = pieces ? min(ld, (n + (min(rb + kSplitTokens, rows_per_batch) - 1) / H - rb / H + kBlockK - 1) / kBlockK * kBlockK) : ld;
 #pragma unroll
   for (int i = 0; i < HOLD; ++i) {
     const int j = (i * blockDim.x + threadIdx.x) * 4;
-    if (j >= ld) continue;
+    if (j >= end) continue;
     float o[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[e] = seen >> (4 * i + e) & 1u ? v[i][e] * inv : 0.f;   // (a row that sees nothing has no finite inv)
     st_four<T>(pr + (size_t)r * ld + j, o);
+    if constexpr (sizeof(T) == 4) {
+      if (pieces) store_pieces(pieces + (size_t)r * ld + j, plane, o);
+    }
+  }
+}
+
+// The same for rows of up to 1024 columns (ld a multiple of 4), a warp per row: no barriers, a row's loads all in flight.  25152 rows of 792 columns with their pieces: 57 us
+// with a block per row, 43 so; with the pieces split by a launch of their own 64 + 38
+constexpr int kSoftmaxWarpLd = 1024, kSoftmaxWarps = 8;
+template <typename T>
+__global__ void __launch_bounds__(kSoftmaxWarps * 32) sink_softmax_warp_kernel(const float* __restrict__ sc, T* __restrict__ pr, const T* __restrict__ sink, int rows, int H, int ld,
+                                        int pos_first, float scale, int rows_per_batch, float sink_const, int key_first, int kept, KeyMask mask,
+                                        __nv_bfloat16* __restrict__ pieces, size_t plane) {
+  constexpr int HOLD = kSoftmaxWarpLd / 128;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int r = blockIdx.x * kSoftmaxWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  const int batch = r / rows_per_batch, rb = r - batch * rows_per_batch;
+  const int q = rb / H, h = rb - q * H, pos = pos_first + q;
+  const int n = pos - key_first + kept + 1;
+  const int j0 = max(0, mask.first(pos) - key_first + kept);
+  const int jk = min(min(mask.keep, j0), n);
+  const float* srow = sc + (size_t)r * ld;
+  const float sk = sink ? ld_f<T>(sink + batch * H + h) : (sink_const > 0.f ? logf(sink_const) : -INFINITY);
+  const int end = pieces ? min(ld, (n + (min(rb + kSplitTokens, rows_per_batch) - 1) / H - q + kBlockK - 1) / kBlockK * kBlockK) : ld;
+  float v[HOLD][4], mx = sk;
+  uint32_t seen = 0;
+#pragma unroll
+  for (int i = 0; i < HOLD; ++i) {
+    const int j = (i * 32 + lane) * 4;
+    const bool any = j < n && (j + 4 > j0 || j < jk);
+    const float4 f = any ? *reinterpret_cast<const float4*>(srow + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[i][0] = f.x; v[i][1] = f.y; v[i][2] = f.z; v[i][3] = f.w;
+  }
+#pragma unroll
+  for (int i = 0; i < HOLD; ++i) {
+    const int j = (i * 32 + lane) * 4;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const bool s = (j + e >= j0 && j + e < n) || j + e < jk;
+      seen |= (uint32_t)s << (4 * i + e);
+      v[i][e] = s ? v[i][e] * scale : -INFINITY;
+      mx = fmaxf(mx, v[i][e]);
+    }
+  }
+  mx = warp_max(mx);
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < HOLD; ++i)
+    if (i * 128 < end)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float x = seen >> (4 * i + e) & 1u ? expf(v[i][e] - mx) : 0.f;
+        v[i][e] = x;
+        sum += x;
+      }
+  const float inv = 1.0f / (warp_sum(sum) + expf(sk - mx));
+#pragma unroll
+  for (int i = 0; i < HOLD; ++i) {
+    const int j = (i * 32 + lane) * 4;
+    if (j >= end) continue;
+    float o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = seen >> (4 * i + e) & 1u ? v[i][e] * inv : 0.f;
+    st_four<T>(pr + (size_t)r * ld + j, o);
+    if constexpr (sizeof(T) == 4) {
+      if (pieces) store_pieces(pieces + (size_t)r * ld + j, plane, o);
+    }
   }
 }
 
