@@ -31,6 +31,8 @@ constexpr int kAttChunk = 64;
 constexpr int attn_stages(int MT) { return MT == 1 ? 2 : 3; }
 constexpr int attn_smem(int HD, int MT) { return attn_stages(MT) * 2 * kAttChunk * (HD + 8) * 2; }
 
+constexpr int kAttnAhead = 4;    // chunks of keys asked for before the wait
+
 struct AttnParams {
   const __nv_bfloat16* q;        // [B*Q, H, hd]
   const __nv_bfloat16* k_cache;  // [slots, KV, hd]
@@ -44,6 +46,7 @@ struct AttnParams {
   int n_split;                   // ranges of one sequence; 1: no partials
   int g_shift;                   // log2(H / KV) when the GQA ratio is a power of two, else -1
   float scale_log2;              // softmax scale * log2(e)
+  int pages;                     // of the caches, if they are known (0: nothing is asked for ahead)
 };
 
 SSDK_DEVINL void cp_async16(void* smem_dst, const void* gsrc, bool valid) {
@@ -97,6 +100,25 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32, OCC) paged_attn_kernel(At
   __nv_bfloat16* sV = sK + kStages * kAttChunk * LDS;                        // [kStages][64][LDS]
 
   pdl_launch_dependents();
+  // While the kernel in front (the rotation) runs, the first keys and values of this CTA's range are asked for into L2: a hint that reads nothing, so that it
+  // does not matter that lengths and table may still be those of the step before (bounded by the caches here, read past L1).
+  // Four contexts of 1500, 28 layers of 8 key heads: a step of five draft passes 5822 -> 5682 us; 16 contexts of 4000, four 8B layers 795 -> 789.
+  if (p.pages > 0 && p.block_size % kAttChunk == 0) {
+    const int b = blockIdx.y / p.n_split, split = blockIdx.y - b * p.n_split;
+    const int nch = (min(max(__ldcg(p.context_lens + b), 0), p.max_blocks * p.block_size) + kAttChunk - 1) / kAttChunk, cps = (nch + p.n_split - 1) / p.n_split;
+    const int c1 = min(min((split + 1) * cps, nch), split * cps + kAttnAhead);
+    constexpr int LINES = HD / 64;   // 128-byte lines of a row
+    for (int ch = split * cps; ch < c1; ++ch) {
+      const int page = __ldcg(p.block_tables + (size_t)b * p.max_blocks + ch * kAttChunk / p.block_size);
+      if (page < 0 || page >= p.pages) continue;
+      const size_t row0 = (size_t)page * p.block_size + ch * kAttChunk % p.block_size;
+      for (int i = threadIdx.x; i < kAttChunk * LINES; i += kAttThreads) {
+        const size_t at = ((row0 + i / LINES) * p.KV + blockIdx.x) * HD + i % LINES * 64;
+        prefetch_l2(p.k_cache + at);
+        prefetch_l2(p.v_cache + at);
+      }
+    }
+  }
   pdl_wait();
   if (threadIdx.x == 0) trace_mark(TR_ATTN);
 

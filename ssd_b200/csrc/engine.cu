@@ -637,8 +637,9 @@ static int enqueue_attention(Launcher& L, const bf16* q, const bf16* kc, const b
                              const int32_t* ctx_lens, bf16* out, float* part_o, float* part_lse, unsigned* counters,
                              int B, int Q, int H,
                              int KV, int hd, int block_size, int max_blocks, float scale, int TQ, int MT, int nqt,
-                             int nsplit) {
+                             int nsplit, int64_t pages = 0) {
   AttnParams a;
+  a.pages = (int)std::min<int64_t>(pages, 1 << 30);
   a.q = q; a.k_cache = kc; a.v_cache = vc; a.block_tables = bt; a.context_lens = ctx_lens; a.out = out;
   a.part_o = part_o; a.part_lse = part_lse;
   (void)counters;
@@ -951,7 +952,7 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
       CKI(forward_prompt_attention(e, L, m, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, f.B, f.Q, bs, mb, scale, nsplit));
     else
       CKI(enqueue_attention(L, w.q, rp.k_cache, rp.v_cache, f.block_tables, w.context_lens, w.attn_out, w.att_o,
-                          w.att_lse, w.att_counters, f.B, f.Q, m.H, m.KV, m.hd, bs, mb, scale, TQ, MT, nqt, nsplit));
+                          w.att_lse, w.att_counters, f.B, f.Q, m.H, m.KV, m.hd, bs, mb, scale, TQ, MT, nqt, nsplit, m.num_blocks));
 
     // ---- output projection (row-parallel) ----
     const bool fuse_pub = use_symm && fused_publish_enabled() && M <= 64;
