@@ -292,8 +292,11 @@ static int launch_gemm_split(Launcher& L, const CUtensorMap& tmX, GemmSplitParam
 static bool few_rows(int M, int64_t N, int K) { return M <= kFewTokens && N * K * 2 <= (30 << 20); }
 // fp32, bf16 or act(gate) * up in bf16; W and X start on 16-byte boundaries, their strides are whole 16-byte pieces, K % 64 == 0
 static int launch_gemm_few(Launcher& L, int epi, const void* X, int ldx, const void* W, int ldw, void* out, int ldo, int M, int N, int K, bool gelu = false,
-                           int heads = 1, int x_step = 0, int out_step = 0) {
+                           int heads = 1, int x_step = 0, int out_step = 0,
+                           const void* ahead = nullptr, int64_t ahead_bytes = 0, const void* ahead2 = nullptr, int64_t ahead_bytes2 = 0) {
   GemmFewParams p;
+  p.ahead[0] = (const bf16*)ahead; p.ahead_lines[0] = (int)(ahead_bytes / 128);
+  p.ahead[1] = (const bf16*)ahead2; p.ahead_lines[1] = (int)(ahead_bytes2 / 128);
   p.W = (const bf16*)W; p.X = (const bf16*)X; p.out = out; p.M = M; p.N = N; p.K = K; p.ldw = ldw; p.ldx = ldx; p.ldo = ldo; p.gelu = gelu; p.x_step = x_step; p.out_step = out_step;
   const int cols = epi == FEW_SILU || epi == FEW_GLU ? kFewRows / 2 : kFewRows, tiles = (N + cols - 1) / cols;
   const int warps = K <= 1024 ? kFewWarps / 2 : kFewWarps;   // (at least four units of k per warp)
@@ -720,7 +723,7 @@ static int forward_prompt_attention(ssdk_engine* e, Launcher& L, const Model& m,
 }
 
 static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w, int M, int epi, void* out, int ldo,
-                        int N_out, int* splits_out, const PublishParams* pub = nullptr) {
+                        int N_out, int* splits_out, const PublishParams* pub = nullptr, const WeightMat* next = nullptr, const WeightMat* next2 = nullptr) {
   CKI(weight_tmap(w));
   const int K = (int)w.cols;
   if (K % kBlockK) return fail("GEMM K=%d not a multiple of 64", K);
@@ -740,7 +743,10 @@ static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w
   }
   if (epi != EPI_PUBLISH && few_rows(M, w.rows, K)) {
     if (splits_out) *splits_out = 1;
-    return launch_gemm_few(L, epi == EPI_SILU ? FEW_SILU : epi == EPI_BF16 ? FEW_BF16 : FEW_F32, x, K, w.ptr, K, out, epi == EPI_PARTIAL ? N_out : ldo, M, N_out, K);
+    const bool ahead2 = next2 && few_rows(M, next2->rows, (int)next2->cols);
+    const bool ahead = next && few_rows(M, next->rows, (int)next->cols);
+    return launch_gemm_few(L, epi == EPI_SILU ? FEW_SILU : epi == EPI_BF16 ? FEW_BF16 : FEW_F32, x, K, w.ptr, K, out, epi == EPI_PARTIAL ? N_out : ldo, M, N_out, K, false, 1, 0, 0,
+                           ahead ? next->ptr : nullptr, ahead ? next->rows * next->cols * 2 : 0, ahead2 ? next2->ptr : nullptr, ahead2 ? next2->rows * next2->cols * 2 : 0);
   }
   const int un = umma_n_for(M);
   const CUtensorMap* tmX;
@@ -934,7 +940,7 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
 
     // ---- QKV projection -> RoPE (+qk norm) -> KV store ----
     int S = 1;
-    CKI(enqueue_gemm(e, L, w.hidden, lw.qkv, M, EPI_PARTIAL, w.partials, 0, m.qkv_dim, &S));
+    CKI(enqueue_gemm(e, L, w.hidden, lw.qkv, M, EPI_PARTIAL, w.partials, 0, m.qkv_dim, &S, nullptr, &lw.o));
     RopeParams rp;
     rp.qkv.dense = (const bf16*)w.partials; rp.qkv.partial = w.partials; rp.qkv.S = S; rp.qkv.M = M; rp.qkv.N = m.qkv_dim;
     rp.positions = w.positions; rp.slot_mapping = w.slot_mapping; rp.rope_table = m.rope;
@@ -987,7 +993,7 @@ static int enqueue_forward(ssdk_engine* e, Launcher& L, const Fwd& f) {
     CKI(launch_norm(L, M, m.d, pn));
 
     // ---- MLP: gate|up with fused SiLU*mul (split-K inside the kernel when the shard is too narrow to fill the machine) ----
-    CKI(enqueue_gemm(e, L, w.hidden, lw.gate_up, M, EPI_SILU, w.act, m.ffn, m.ffn, nullptr));
+    CKI(enqueue_gemm(e, L, w.hidden, lw.gate_up, M, EPI_SILU, w.act, m.ffn, m.ffn, nullptr, nullptr, &lw.down, l + 1 < m.cfg.layers ? &m.layers[l + 1].qkv : nullptr));
     if (fuse_pub) {
       const PublishParams pb = publish_params(e, ar_idx);
       CKI(enqueue_gemm(e, L, w.act, lw.down, M, EPI_PUBLISH, w.partials, 0, m.d, &S, &pb));

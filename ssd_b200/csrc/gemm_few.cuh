@@ -29,6 +29,8 @@ struct GemmFewParams {
   void* out;                // [M, ldo]: fp32 or bf16
   int M, N, K, ldw, ldx, ldo;
   int gelu;                 // FEW_GLU: gelu_tanh instead of silu
+  const __nv_bfloat16* ahead[2];   // weights of products behind this one, asked for into L2: ahead_lines of 128 bytes each
+  int ahead_lines[2];
   int x_step, out_step;     // products side by side (heads): product b reads X's columns from b x_step, the weight rows from b N, and writes out + b out_step
 };
 
@@ -72,6 +74,9 @@ __global__ void __launch_bounds__(kFewWarps * 32, 2) gemm_few_kernel(const GemmF
   if (p.ldx < 0) pdl_launch_dependents();
   pdl_wait();
   if (threadIdx.x == 0) trace_mark(TR_GEMM);
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.ahead_lines[a]; i += gridDim.x * blockDim.x) prefetch_l2(p.ahead[a] + (size_t)i * 64);
 #pragma unroll
   for (int j = 0; j < D; ++j)
     if (u0 + j < u1) load_x(x[j], u0 + j);
