@@ -822,6 +822,16 @@ struct HybRun {
     return std::max(1, gqa_on_mma(Lr) ? std::min({ssdk::kGqaMaxSplits, 3 * num_sms() / std::max(1, n_dec * G), (ctx_max + ssdk::kGmKeys - 1) / ssdk::kGmKeys})
                                       : std::min({ssdk::kGqaMaxSplits, 8 * num_sms() / std::max(1, n_dec * H), (ctx_max + 127) / 128}));
   }
+  // context splits with which a grouped-query layer's single-token rows take the fused decode form; 0: they do not (no such rows, or the score buffer
+  // holds not even one split's partials), and go through gathers and products with a scratch of their own
+  int gqa_decode_splits(const HybLayer& Lr) const {
+    const ssdk_hyb_layer_cfg& c = Lr.c;
+    int ctx_max = 0;
+    const int n_dec = decode_rows(ssdk::KeyMask{c.window, c.chunk, c.keep_first}, &ctx_max);
+    if (n_dec < 1 || !e->use_decode_attn || !(gqa_on_mma(Lr) || (c.vdim + 31) / 32 <= 8)) return 0;
+    const size_t per_split = (size_t)rg.n_seqs * c.heads * c.maps * (c.vdim + 2);
+    return (int)std::min<size_t>(gqa_splits(Lr, n_dec, ctx_max), e->att_elems / per_split);
+  }
   // what the launches of a decode step depend on beside the counts: every attention layer's context splits
   void decode_key(std::vector<int>& key) const {
     for (const HybLayer& Lr : e->layers) {
@@ -1363,34 +1373,24 @@ struct HybRun {
     const bool mma = gqa_on_mma(Lr);
     const int ks = std::max(D, V) <= 32 ? 2 : (std::max(D, V) <= 64 || (maps == 2 && D <= 64) ? 4 : 8);
     const int vt = V <= 64 && ks < 8 ? 2 * ks : 16;   // (two maps: value heads are often twice as wide as the keys)
-    bool fused_decode = false;
-    {
-      int ctx_max = 0;
-      const int n_dec = decode_rows(mask, &ctx_max);
-      const int vpl = (V + 31) / 32;
-      if (n_dec > 0 && (mma || vpl <= 8) && e->use_decode_attn) {
-        int splits = gqa_splits(Lr, n_dec, ctx_max);
-        const size_t per_split = (size_t)rg.n_seqs * H * (V + 2);
-        splits = (int)std::min<size_t>(splits, e->att_elems / per_split);
-        if (splits >= 1) {
-          ssdk::GqaDecodeArgs da;
-          da.q = e->qcat; da.cache = pool; da.part = e->att_s; da.y = y; da.gate = gate; da.ld_gate = ld_gate; da.H = H; da.G = G; da.D = D; da.V = V; da.splits = splits;
-          da.scale = c.attn_scale; da.sink = sink_const; da.sinks = sinks; da.mask = mask; da.maps = maps; da.diff = diff;
-          const dim3 grid(rg.n_seqs, H, splits), block(ssdk::kGqaDecWarps * 32), mgrid(rg.n_seqs, G, splits), mblock(128);
-          const size_t smem = ssdk::gqa_decode_smem(D, V), msmem = ssdk::gqa_decode_mma_smem(ks, vt, V);
-          if (mma && ks == 2) CKI(L.go(ssdk::gqa_decode_mma_kernel<2, 4>, mgrid, mblock, msmem, da, rg));
-          else if (mma && ks == 4 && vt == 16) CKI(L.go(ssdk::gqa_decode_mma_kernel<4, 16>, mgrid, mblock, msmem, da, rg));
-          else if (mma && ks == 4) CKI(L.go(ssdk::gqa_decode_mma_kernel<4, 8>, mgrid, mblock, msmem, da, rg));
-          else if (mma) CKI(L.go(ssdk::gqa_decode_mma_kernel<8, 16>, mgrid, mblock, msmem, da, rg));
-          else if (vpl <= 1) CKI(L.go(ssdk::gqa_decode_partial_kernel<T, 1>, grid, block, smem, da, rg));
-          else if (vpl <= 2) CKI(L.go(ssdk::gqa_decode_partial_kernel<T, 2>, grid, block, smem, da, rg));
-          else if (vpl <= 4) CKI(L.go(ssdk::gqa_decode_partial_kernel<T, 4>, grid, block, smem, da, rg));
-          else CKI(L.go(ssdk::gqa_decode_partial_kernel<T, 8>, grid, block, smem, da, rg));
-          if (maps == 2) CKI(L.go(ssdk::gqa_decode_merge_diff_kernel<T>, dim3(rg.n_seqs, H / 2), dim3(V <= 64 ? 64 : 128), (size_t)V * 4, da, rg));
-          else CKI(L.go(ssdk::gqa_decode_merge_kernel<T>, dim3(rg.n_seqs, H), dim3(V <= 64 ? 64 : 128), 0, da, rg));
-          fused_decode = true;
-        }
-      }
+    const int splits = gqa_decode_splits(Lr), vpl = (V + 31) / 32;
+    const bool fused_decode = splits >= 1;
+    if (fused_decode) {
+      ssdk::GqaDecodeArgs da;
+      da.q = e->qcat; da.cache = pool; da.part = e->att_s; da.y = y; da.gate = gate; da.ld_gate = ld_gate; da.H = H; da.G = G; da.D = D; da.V = V; da.splits = splits;
+      da.scale = c.attn_scale; da.sink = sink_const; da.sinks = sinks; da.mask = mask; da.maps = maps; da.diff = diff;
+      const dim3 grid(rg.n_seqs, H, splits), block(ssdk::kGqaDecWarps * 32), mgrid(rg.n_seqs, G, splits), mblock(128);
+      const size_t smem = ssdk::gqa_decode_smem(D, V), msmem = ssdk::gqa_decode_mma_smem(ks, vt, V);
+      if (mma && ks == 2) CKI(L.go(ssdk::gqa_decode_mma_kernel<2, 4>, mgrid, mblock, msmem, da, rg));
+      else if (mma && ks == 4 && vt == 16) CKI(L.go(ssdk::gqa_decode_mma_kernel<4, 16>, mgrid, mblock, msmem, da, rg));
+      else if (mma && ks == 4) CKI(L.go(ssdk::gqa_decode_mma_kernel<4, 8>, mgrid, mblock, msmem, da, rg));
+      else if (mma) CKI(L.go(ssdk::gqa_decode_mma_kernel<8, 16>, mgrid, mblock, msmem, da, rg));
+      else if (vpl <= 1) CKI(L.go(ssdk::gqa_decode_partial_kernel<T, 1>, grid, block, smem, da, rg));
+      else if (vpl <= 2) CKI(L.go(ssdk::gqa_decode_partial_kernel<T, 2>, grid, block, smem, da, rg));
+      else if (vpl <= 4) CKI(L.go(ssdk::gqa_decode_partial_kernel<T, 4>, grid, block, smem, da, rg));
+      else CKI(L.go(ssdk::gqa_decode_partial_kernel<T, 8>, grid, block, smem, da, rg));
+      if (maps == 2) CKI(L.go(ssdk::gqa_decode_merge_diff_kernel<T>, dim3(rg.n_seqs, H / 2), dim3(V <= 64 ? 64 : 128), (size_t)V * 4, da, rg));
+      else CKI(L.go(ssdk::gqa_decode_merge_kernel<T>, dim3(rg.n_seqs, H), dim3(V <= 64 ? 64 : 128), 0, da, rg));
     }
     if (mma) {   // all portions in one launch
       int n_max = 0;
@@ -1569,9 +1569,9 @@ struct HybRun {
       return lin(e->t0, HV, Lr.t[SSDK_HT_ATTN_OUT].p, HV, e->mix_out, W, M, W, HV);
     };
     // A decoding step's attention beside its delta rule: chains of five small kernels each.  In prompts the walk of the delta rule, a warp per scheduler, would
-    // take 427 us instead of 263 beside anything (2048 tokens, 4 layers: 2616 -> 2795 us a call; decoding 209 -> 186).  The attention runs in its
-    // fused kernels, which leave p1 alone.
-    const bool aside = longest() == 1 && gqa_on_mma(Lr) && e->use_decode_attn && beside_ok(e->t0, Lr.t[SSDK_HT_ATTN_OUT].p, HV, W);
+    // take 427 us instead of 263 beside anything (2048 tokens, 4 layers: 2616 -> 2795 us a call; decoding 209 -> 186).  Only where the attention runs in
+    // its fused kernels: the other form's scratch is p1, which the delta rule's results lie in.
+    const bool aside = longest() == 1 && gqa_on_mma(Lr) && gqa_decode_splits(Lr) >= 1 && beside_ok(e->t0, Lr.t[SSDK_HT_ATTN_OUT].p, HV, W);
     if (aside) CKI(beside(left));
     else CKI(left());
     auto right = [&]() -> int {
