@@ -1630,9 +1630,9 @@ struct HybRun {
     const int rc = branch();
     L.st = main;
     L.barrier_op();
-    if (rc) return rc;
     CK(cudaEventRecord(e->side_end, e->side));
-    return 0;
+    if (rc) CKI(beside_end());   // what the branch had launched before its error is waited for like all the rest (a capture ends with its streams joined)
+    return rc;
   }
   int beside_end() {
     CK(cudaStreamWaitEvent(L.st, e->side_end, 0));
