@@ -56,12 +56,7 @@ gqa_prompt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   uint8_t* sV = sK + kPromptStages * HK * kHalf;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  pdl_launch_dependents();
-  pdl_wait();
-  const int gv = blockIdx.y, s = blockIdx.z, r0 = rg.cu[s], p0 = rg.pos0[s], shift = p.g_shift;
-  const int rows = (rg.cu[s + 1] - r0) << shift, row0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * R;   // (the tiles that see most keys first)
-  if (rows < 2 << shift || row0 >= rows) return;
-
+  // (in front of the trigger: a product that this kernel lets start early finds its tensor memory taken, and not the other way round)
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmKV);
@@ -78,6 +73,15 @@ gqa_prompt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot, tmem_o = tmem + 128;   // S / P buffers at columns 0 and 64, O behind them
+
+  pdl_launch_dependents();
+  pdl_wait();
+  const int gv = blockIdx.y, s = blockIdx.z, r0 = rg.cu[s], p0 = rg.pos0[s], shift = p.g_shift;
+  const int rows = (rg.cu[s + 1] - r0) << shift, row0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * R;   // (the tiles that see most keys first)
+  if (rows < 2 << shift || row0 >= rows) {   // (the whole CTA)
+    if (warp == 1) tmem_dealloc(tmem, 256);
+    return;
+  }
 
   // keys that the tile's rows see together: those below `keep`, and first .. k_end - 1
   const int first = p.mask.first(p0 + (row0 >> shift)), keep = p.mask.kept(first), k_end = p0 + ((min(rows, row0 + R) - 1) >> shift) + 1;
