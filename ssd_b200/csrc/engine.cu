@@ -678,24 +678,26 @@ static int tile_splits(int H, int KV, int B, int Q, int max_ctx) {
   const int tokens = kPromptRows / (H / KV), ctas = KV * B * ((Q + tokens - 1) / tokens);
   return std::max(1, std::min({(3 * num_sms() + 2 * ctas - 1) / (2 * ctas), kAttnMaxSplit, (max_ctx + kPromptKeys - 1) / kPromptKeys}));
 }
-template <int HD>
-static int launch_prompt_attn(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const PromptAttnParams& p, int B) {
+template <int HD, bool SPLIT, bool FINE>
+static int launch_prompt_inst(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const PromptAttnParams& p, int B) {
   static bool attr_set = false;
   if (!attr_set) {
-    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD)));
-    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD)));
-    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD)));
+    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT, FINE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     attr_set = true;
   }
   const int tq = kPromptRows >> p.g_shift, nqt = (p.Q + tq - 1) / tq;
-  if (p.n_split > 1) return L.go(prompt_attn_kernel<HD, true>, dim3(p.KV, nqt, B * p.n_split), dim3(kPromptThreads), (size_t)prompt_attn_smem(HD), tmQ, tmK, tmV, p);
-  return L.go(prompt_attn_kernel<HD, false>, dim3(p.KV, nqt, B), dim3(kPromptThreads), (size_t)prompt_attn_smem(HD), tmQ, tmK, tmV, p);
+  return L.go(prompt_attn_kernel<HD, SPLIT, FINE>, dim3(p.KV, nqt, B * p.n_split), dim3(kPromptThreads), (size_t)prompt_attn_smem(HD), tmQ, tmK, tmV, p);
+}
+template <int HD>
+static int launch_prompt_attn(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const PromptAttnParams& p, int B, bool fine) {
+  if (p.n_split > 1) return launch_prompt_inst<HD, true, true>(L, tmQ, tmK, tmV, p, B);
+  return fine ? launch_prompt_inst<HD, false, true>(L, tmQ, tmK, tmV, p, B) : launch_prompt_inst<HD, false, false>(L, tmQ, tmK, tmV, p, B);
 }
 // maps of queries, keys and values of layer caches of `slots` token slots: {box of a tile's query tokens, kPromptKeys keys of one head}
 static int enqueue_prompt_attention(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const int32_t* bt,
                                     const int32_t* ctx_lens, bf16* out, int B, int Q, int H, int KV, int hd, int block_size, int max_blocks,
-                                    int64_t slots, float scale, unsigned* timeout, int n_split = 1, float* part_o = nullptr, float* part_lse = nullptr) {
+                                    int64_t slots, float scale, unsigned* timeout, bool fine, int n_split = 1, float* part_o = nullptr, float* part_lse = nullptr) {
   PromptAttnParams p = {};
   p.n_split = n_split; p.part_o = part_o; p.part_lse = part_lse;
   p.block_tables = bt; p.context_lens = ctx_lens; p.out = out; p.Q = Q; p.H = H; p.KV = KV; p.block_size = block_size; p.max_blocks = max_blocks;
@@ -703,7 +705,7 @@ static int enqueue_prompt_attention(Launcher& L, const CUtensorMap& tmQ, const C
   p.n_slots = (int)slots;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.timeout = timeout;
-  CKI(hd == 128 ? launch_prompt_attn<128>(L, tmQ, tmK, tmV, p, B) : launch_prompt_attn<64>(L, tmQ, tmK, tmV, p, B));
+  CKI(hd == 128 ? launch_prompt_attn<128>(L, tmQ, tmK, tmV, p, B, fine) : launch_prompt_attn<64>(L, tmQ, tmK, tmV, p, B, fine));
   if (n_split > 1) {
     AttnParams a = {};
     a.context_lens = ctx_lens; a.out = out; a.part_o = part_o; a.part_lse = part_lse; a.B = B; a.Q = Q; a.H = H; a.KV = KV; a.TQ = kPromptRows >> p.g_shift; a.n_split = n_split;
@@ -719,7 +721,8 @@ static int forward_prompt_attention(ssdk_engine* e, Launcher& L, const Model& m,
   CKI(e->xmaps.get_heads(q, B * Q > kMaxTokens ? kMaxPass : kMaxTokens, m.H, m.hd, G, kPromptRows / G, &tmQ));
   CKI(e->xmaps.get_heads(kc, slots, m.KV, m.hd, 1, kPromptKeys, &tmK));
   CKI(e->xmaps.get_heads(vc, slots, m.KV, m.hd, 1, kPromptKeys, &tmV));
-  return enqueue_prompt_attention(L, *tmQ, *tmK, *tmV, bt, ctx_lens, out, B, Q, m.H, m.KV, m.hd, block_size, max_blocks, slots, scale, L.gave_up, n_split, e->ws.att_o, e->ws.att_lse);
+  return enqueue_prompt_attention(L, *tmQ, *tmK, *tmV, bt, ctx_lens, out, B, Q, m.H, m.KV, m.hd, block_size, max_blocks, slots, scale, L.gave_up, B * Q <= kMaxTokens, n_split,
+                                  e->ws.att_o, e->ws.att_lse);
 }
 
 static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w, int M, int epi, void* out, int ldo,
@@ -1345,10 +1348,10 @@ static int init_kernel_attrs() {
   SSDK_ATTR_A(128, 1, 3) SSDK_ATTR_A(128, 2, 1) SSDK_ATTR_A(128, 2, 2) SSDK_ATTR_A(128, 4, 1) SSDK_ATTR_A(128, 4, 2)
   SSDK_ATTR_A(64, 1, 3) SSDK_ATTR_A(64, 2, 1) SSDK_ATTR_A(64, 2, 2) SSDK_ATTR_A(64, 4, 1) SSDK_ATTR_A(64, 4, 2)
 #undef SSDK_ATTR_A
-#define SSDK_ATTR_P(HD, SPLIT) \
-  CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD))); \
-  CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-  SSDK_ATTR_P(64, false) SSDK_ATTR_P(64, true) SSDK_ATTR_P(128, false) SSDK_ATTR_P(128, true)
+#define SSDK_ATTR_P(HD, SPLIT, FINE) \
+  CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD))); \
+  CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT, FINE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  SSDK_ATTR_P(64, false, false) SSDK_ATTR_P(64, false, true) SSDK_ATTR_P(64, true, true) SSDK_ATTR_P(128, false, false) SSDK_ATTR_P(128, false, true) SSDK_ATTR_P(128, true, true)
 #undef SSDK_ATTR_P
   CK(cudaFuncSetAttribute(add_rmsnorm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
   return 0;
@@ -1939,7 +1942,7 @@ int ssdk_paged_attn_pages(const void* q, const void* k_cache, const void* v_cach
   CKI(make_tmap_heads(&tmK, k_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
   CKI(make_tmap_heads(&tmV, v_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
   return enqueue_prompt_attention(L, tmQ, tmK, tmV, block_tables, context_lens, (bf16*)out, batch, q_len, heads, kv_heads, head_dim, block_size,
-                                  max_blocks_per_seq, slots, scale, nullptr, tile_splits(heads, kv_heads, batch, q_len, max_ctx), part_o, part_lse);
+                                  max_blocks_per_seq, slots, scale, nullptr, true, tile_splits(heads, kv_heads, batch, q_len, max_ctx), part_o, part_lse);
 }
 
 int ssdk_prompt_attn(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
@@ -1957,7 +1960,7 @@ int ssdk_prompt_attn(const void* q, const void* k_cache, const void* v_cache, co
   CKI(make_tmap_heads(&tmK, k_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
   CKI(make_tmap_heads(&tmV, v_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
   return enqueue_prompt_attention(L, tmQ, tmK, tmV, block_tables, context_lens, (bf16*)out, batch, q_len, heads, kv_heads, head_dim, block_size,
-                                  max_blocks_per_seq, slots, scale, gave_up);
+                                  max_blocks_per_seq, slots, scale, gave_up, false);
 }
 
 int ssdk_sample(const void* logits, int64_t ld, const float* temps, int B, int V, uint64_t seed, uint64_t step_id,

@@ -209,7 +209,7 @@ gqa_prompt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         }
       }
       const float ms = m == -INFINITY ? 0.f : m;
-      l += row_exp(u, p.scale_log2, ms);
+      l += row_exp<false>(u, p.scale_log2, ms);
       tmem_st_32x32b_x16(sp, u);
       tmem_st_32x32b_x16(sp + 16, u + 16);
       tmem_st_wait();

@@ -6,7 +6,11 @@
 //   P = exp2(S - m) one row per thread, no shuffles; rounded to bf16 and stored over the S it came from
 //   O += P V       P from TMEM, V as it lies in the cache (MN-major operand), fp32 in TMEM
 // m is raised, and O and the sum rescaled, only when a row's maximum has grown by more than kPromptSlack (base 2): P then stays below
-// 2^kPromptSlack, which costs bf16 and fp32 nothing in relative precision.
+// 2^kPromptSlack, where bf16 and fp32 are as fine relative to a value as below 1.  But a row's largest weight is no longer exactly 1, and is rounded like all others;
+// paged_attn_kernel follows the maximum of every token slice and rounds none of those.  FINE (the calls that this kernel takes over from it) therefore gives P
+// as two bf16 pieces, 16 significant bits, and multiplies each with V.  Relative error of a 70B layer's attention against 64 bits, 8 x 7 rows of contexts of 4500
+// to 8000 / 4 x 8 of 1880 to 3000 / 2 x 8 of 220 to 300: 0.00275, 0.00268, 0.00252 in paged_attn_kernel, 0.00289, 0.00286, 0.00264 with one piece, 0.00237,
+// 0.00237, 0.0023 with two, which cost 12 % of the first (60 -> 67 us; paged_attn_kernel 109).  Pieces cut off instead of rounded: the same time.
 // Warps: 0 loads, 1 issues the products, 2-5 softmax and output.  Two CTAs per SM (97 KB, 256 TMEM columns each), so that one's products
 // run under the other's exponentials, which bound the kernel.
 // 2003 tokens, 32 heads of 128 over 8: 205 us on mma.sync tiles of 64 rows (paged_attn_kernel), 47 us here = 700 TFLOP/s of the masked work;
@@ -76,18 +80,31 @@ SSDK_DEVINL float row_max(const uint32_t (&u)[64]) {
     for (int e = 0; e < 4; ++e) m[e] = max3(m[e], __uint_as_float(u[c + e]), __uint_as_float(u[c + 4 + e]));
   return fmaxf(max3(m[0], m[1], __uint_as_float(u[60])), max3(m[2], m[3], max3(__uint_as_float(u[61]), __uint_as_float(u[62]), __uint_as_float(u[63]))));
 }
-// 2^(score * scale - ms) of a row: rounded to bf16 in the first 32 words, their sum (of the unrounded ones) back.  Products and sums two at a time; a probability
-// below 2^-126 is zero (the row's largest is at least 2^-kPromptSlack).
+// 2^(score * scale - ms) of a row: rounded to bf16 in the first 32 words (FINE: what that leaves, rounded to bf16, in the others), their sum (of the unrounded ones)
+// back.  Products and sums two at a time; a probability below 2^-126 is zero (the row's largest is at least 2^-kPromptSlack).
+template <bool FINE>
 SSDK_DEVINL float row_exp(uint32_t (&u)[64], float scale, float ms) {
   const uint64_t sc = pack2(scale, scale), off = pack2(-ms, -ms);
+  const uint64_t minus = pack2(-1.f, -1.f);
   uint64_t sum[2] = {0, 0};
+  uint32_t low[32];
 #pragma unroll
   for (int c = 0; c < 64; c += 2) {
     float a, e;
     unpack2(fma2(pack2(__uint_as_float(u[c]), __uint_as_float(u[c + 1])), sc, off), &a, &e);
     a = ex2_ftz(a); e = ex2_ftz(e);
     sum[(c >> 1) & 1] = add2(sum[(c >> 1) & 1], pack2(a, e));
-    u[c >> 1] = pack_bf16x2(a, e);
+    const uint32_t h = pack_bf16x2(a, e);
+    u[c >> 1] = h;
+    if (FINE) {   // (exact differences)
+      float x, y;
+      unpack2(fma2(pack2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), minus, pack2(a, e)), &x, &y);
+      low[c >> 1] = pack_bf16x2(x, y);
+    }
+  }
+  if (FINE) {
+#pragma unroll
+    for (int c = 0; c < 32; ++c) u[32 + c] = low[c];
   }
   float s0, s1, s2, s3;
   unpack2(sum[0], &s0, &s1);
@@ -95,8 +112,8 @@ SSDK_DEVINL float row_exp(uint32_t (&u)[64], float scale, float ms) {
   return (s0 + s1) + (s2 + s3);
 }
 
-// grid (kv heads, q tiles, sequences x ranges)
-template <int HD, bool SPLIT>
+// grid (kv heads, q tiles, sequences x ranges).  FINE: P in two pieces
+template <int HD, bool SPLIT, bool FINE>
 __global__ void __launch_bounds__(kPromptThreads, 2)
 prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                    const PromptAttnParams p) {
@@ -205,6 +222,10 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
         for (int k = 0; k < kPromptKeys / 16; ++k)   // 16 keys: 2048 B of V, 8 columns of P
           umma_bf16_ts(tmem_o, tmem + (i & 1) * 64 + 8 * k, vd + 128 * k, idesc_o, (uint32_t)((i | k) != 0));
+        if (FINE) {
+#pragma unroll
+          for (int k = 0; k < kPromptKeys / 16; ++k) umma_bf16_ts(tmem_o, tmem + (i & 1) * 64 + 32 + 8 * k, vd + 128 * k, idesc_o, 1u);
+        }
         umma_commit(&v_empty[i & 1]);
         umma_commit(&pv_done[i & 1]);
       }
@@ -252,9 +273,9 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
       }
       const float ms = m == -INFINITY ? 0.f : m;
-      l += row_exp(u, p.scale_log2, ms);
-      tmem_st_32x32b_x16(sp, u);
-      tmem_st_32x32b_x16(sp + 16, u + 16);
+      l += row_exp<FINE>(u, p.scale_log2, ms);
+#pragma unroll
+      for (int c = 0; c < (FINE ? 64 : 32); c += 16) tmem_st_32x32b_x16(sp + c, u + c);
       tmem_st_wait();
       if (base + kPromptKeys > kv_max) {   // the last chunk: slots behind the tile's keys hold anything, and 0 x NaN is NaN
         if (!(ok = warp_wait(&v_full[i & 1], parity(i), p.timeout))) break;

@@ -39,6 +39,31 @@ def test_against_float64(heads, kv_heads, hd, q_len, ctx):
             assert torch.isfinite(off).all() and off.max().item() < 1, (b, h, off.max().item())
 
 
+@pytest.mark.parametrize("heads,kv_heads,hd,q_len,ctx", [(64, 8, 128, 7, [1500, 64, 1, 700]), (32, 8, 64, 8, [300, 2, 900]), (16, 1, 128, 3, [60, 130, 4000]),
+                                                         (32, 32, 128, 100, [50, 400])])
+def test_weights_keep_sixteen_bits(heads, kv_heads, hd, q_len, ctx):
+    """The output is rounded to bf16 (eight significant bits: 2^-8 of it at most); weights are not (two pieces: 2^-17), and fp32 sums of scores and products move them
+    by less than 2^-15: together 2^-14 of sum p |v|.  Weights of one bf16 piece are off by up to 2^-8 each, which short contexts show."""
+    from ssd_b200 import ops
+    G, B, bs = heads // kv_heads, len(ctx), 64
+    g = torch.Generator(device="cuda").manual_seed(heads * 1000 + q_len)
+    pages = -(-(max(max(ctx) + q_len, 2048)) // bs)   # (the table's capacity takes the call to the tiles)
+    tables = torch.arange(B * pages, dtype=torch.int32, device="cuda").view(B, pages)
+    q = torch.randn(B * q_len, heads, hd, generator=g, device="cuda").to(torch.bfloat16)
+    kc, vc = (torch.randn(B * pages, bs, kv_heads, hd, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    lens = torch.tensor([n + q_len for n in ctx], dtype=torch.int32, device="cuda")
+    out = ops.paged_attention(q, kc, vc, tables, lens, q_len, hd ** -0.5).view(B, q_len, heads, hd).double()
+    for b, n0 in enumerate(ctx):
+        k, v = (c.view(B, pages * bs, kv_heads, hd)[b, :n0 + q_len].double() for c in (kc, vc))
+        hidden = torch.arange(n0 + q_len, device="cuda")[None, :] > torch.arange(n0, n0 + q_len, device="cuda")[:, None]
+        for h in range(0, heads, max(1, heads // 8)):
+            s = (q.view(B, q_len, heads, hd)[b, :, h].double() @ k[:, h // G].T) * hd ** -0.5
+            p = torch.softmax(s.masked_fill(hidden, float("-inf")), -1)
+            y = p @ v[:, h // G]
+            bound = 2.0 ** -8 * y.abs() + 2.0 ** -14 * (p @ v[:, h // G].abs())
+            assert ((out[b, :, h] - y).abs() <= bound).all(), (b, h, ((out[b, :, h] - y).abs() / bound).max().item())
+
+
 def test_pages_that_a_table_does_not_name_count_as_zero_keys():
     """As in the tiles that this form takes over from: a chunk behind a table entry of -1 scores 0 and has no value."""
     from ssd_b200 import ops
