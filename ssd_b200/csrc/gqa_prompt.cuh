@@ -45,6 +45,10 @@ __global__ void __launch_bounds__(kPromptThreads, 2)
 gqa_prompt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ GqaLatentMaps lm, const GqaPromptArgs p,
                   const Ragged rg) {
   constexpr int HK = DK / 64, HV = VD / 64, R = kPromptRows / MAPS;   // 64-column boxes of keys and values, rows of a map
+  // Weights as two bf16 pieces (see prompt_attention.cuh): the tiles that this form took over from keep the largest weights of their slices unrounded.  vegilix m,
+  // prompts of 2001 and 2 x 700 tokens against 64 bits: 0.00338, 0.00328 with one piece, 0.00324, 0.00313 with two; 518 -> 523 us.  Latent attention: the absorbed form that
+  // whole prompts took before rounds its weights once as well
+  constexpr bool FINE = !LATENT;
   constexpr int kQHalf = kPromptRows * 128, kHalf = kPromptKeys * 128;
   static_assert(MAPS == 1 || (DK == 128 && !LATENT), "two maps of 64");
   extern __shared__ uint8_t prompt_smem_raw[];
@@ -154,6 +158,10 @@ gqa_prompt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 #pragma unroll
         for (int k = 0; k < kPromptKeys / 16; ++k)   // 16 keys: 2048 B of V, 8 columns of P
           umma_bf16_ts(tmem_o, tmem + (i & 1) * 64 + 8 * k, vd + 128 * k, idesc_o, (uint32_t)((i | k) != 0));
+        if (FINE) {
+#pragma unroll
+          for (int k = 0; k < kPromptKeys / 16; ++k) umma_bf16_ts(tmem_o, tmem + (i & 1) * 64 + 32 + 8 * k, vd + 128 * k, idesc_o, 1u);
+        }
         umma_commit(&v_empty[i & 1]);
         umma_commit(&pv_done[i & 1]);
       }
@@ -209,9 +217,9 @@ gqa_prompt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         }
       }
       const float ms = m == -INFINITY ? 0.f : m;
-      l += row_exp<false>(u, p.scale_log2, ms);
-      tmem_st_32x32b_x16(sp, u);
-      tmem_st_32x32b_x16(sp + 16, u + 16);
+      l += row_exp<FINE>(u, p.scale_log2, ms);
+#pragma unroll
+      for (int c = 0; c < (FINE ? 64 : 32); c += 16) tmem_st_32x32b_x16(sp + c, u + c);
       tmem_st_wait();
       // values that no row of the tile sees may be anything, and 0 x NaN is NaN: those between the kept keys and the first one, those behind the last
       const int gap0 = min(max(keep - base, 0), kPromptKeys), gap1 = min(max(first - base, gap0), kPromptKeys), end = min(k_end - base, kPromptKeys);

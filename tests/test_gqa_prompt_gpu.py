@@ -1,4 +1,4 @@
-"""Prompts of grouped-query attention on tcgen05 tiles (gqa_prompt_kernel) against the path of separate products and a softmax: one and two maps, head
+"""Prompts of grouped-query attention on tcgen05 tiles (gqa_prompt_kernel) against 64 bits and the path of separate products and a softmax: one and two maps, head
 sizes, groups, windows and kept keys around chunks, constant and learned sinks, output gates, two sequences, portions behind earlier ones, a pool
 that holds NaN wherever nothing was stored."""
 import importlib
@@ -30,7 +30,9 @@ def test_matches_separate_products(tmp_path, monkeypatch, arch, a):
     rounded, which shows as one unit (2^-8) of a head's entries, and again behind the output projection's rounding and the norm: 2^-6 covers it."""
     from ssd_b200.hybrid import HybridRunner, HybridSpec, load_hybrid_weights
     U, cfg = _model(arch, a)
-    path = U.write_checkpoint(str(tmp_path / "c"), cfg, U.random_tensors(cfg, 3))
+    tensors = U.random_tensors(cfg, 3)
+    path = U.write_checkpoint(str(tmp_path / "c"), cfg, tensors)
+    plain = (U if arch == "kefurax" else importlib.import_module(f"tests.{arch}_plain")).PlainModel(cfg, tensors)
     spec = HybridSpec.from_dir(path)
     runners = {}
     for on in ("1", "0"):
@@ -41,10 +43,19 @@ def test_matches_separate_products(tmp_path, monkeypatch, arch, a):
         runners[on] = r
     toks = [torch.randint(0, cfg["vocab"], (n,), generator=torch.Generator().manual_seed(n)).tolist() for n in (700, 321, 193)]
     pages = [list(range(i * 16, (i + 1) * 16))[::-1] for i in range(3)]
-    at = [0, 0, 0]
+    want = [plain.run(t).numpy() for t in toks]
+    at, rows = [0, 0, 0], {"1": [], "0": [], "want": []}
     for part in ((2, 128, 64), (255, 1, 65), (63, 129, 1), (380, 63, 63)):   # rows of the three sequences in turn
         entries = [(toks[i][at[i]:at[i] + n], at[i], i, pages[i], list(range(n))) for i, n in enumerate(part)]
+        rows["want"] += [want[i][at[i]:at[i] + n] for i, n in enumerate(part)]
         at = [x + n for x, n in zip(at, part)]
-        got = {on: r.forward(entries, residual=True)[2][0] for on, r in runners.items()}
+        got = {}
+        for on, r in runners.items():
+            logits, _, residual = r.forward(entries, residual=True)
+            got[on] = residual[0]
+            rows[on].append(logits)
         assert np.isfinite(got["1"]).all()
         assert U.rel_err(got["1"], got["0"]) < 2.0 ** -6, part
+    # all rows against 64 bits: no further off than the separate products, which round a weight once as well (a tenth for the order of sums)
+    off = {on: U.rel_err(np.concatenate(rows[on]), np.concatenate(rows["want"])) for on in ("1", "0")}
+    assert off["1"] < 2.0 ** -6 and off["1"] <= 1.1 * off["0"], off
