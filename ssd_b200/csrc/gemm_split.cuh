@@ -13,18 +13,18 @@
 // on (as long as K times the largest other operand is below 2^30).  Results that are not finite, and results below 2^-70 that are not zero, are
 // therefore taken again as the FMA chain over k that linear_kernel walks (see split_again).  What still differs: a result below 2^-126 may be zero.
 //
-// What bounds it: 24 products of 64 clocks per k-block of 64 and 128 tokens are a floor that it is 2.6 times above (tensor pipe active 38 % of
-// the time on the SMs that have two tiles of 1000 x 3072 x 2048, 25 % on all: 96 tiles on 74 pairs), DRAM and issue slots are further
-// away (3 and 16 %): three stages of 72 KB do not cover the way of the weights through registers.  The
-// FMA form it takes over from (linear_kernel, 64 x 64 tiles) was bound by its shared-memory operands: 1000 x 4096 x 2048 539 us (31 TFLOP/s)
-// -> 145 us (115), 2000 x 8192 x 2048 2092 -> 459 us; with few rows the kernel streams the weights (8 x 8192 x 2048 148 -> 50 us), which is
-// why the tokens of a tile go down to 32.  Pairs of CTAs and the persistent walk as in
+// What bounds it: the tensor core takes about 85 clocks for an instruction and one more for four tokens, so that a k-block of 64 (24 products) is 2040 clocks
+// and 6 a token; measured, with what the stages do not cover, 3100 and 7.5 (960 x 4096 x 2048 with chunks of 96, 128, 160, 192 tokens: 3800, 4090, 4410, 4520).
+// Chunks of up to 192 tokens therefore (of 128, in three stages: 1000 x 3072 x 2048 137 us, 82 here).  The FMA form that it took over from (linear_kernel,
+// 64 x 64 tiles) was bound by its shared-memory operands: 1000 x 4096 x 2048 539 us (31 TFLOP/s), 2000 x 8192 x 2048 2092.  With few rows the kernel streams
+// the weights (8 x 8192 x 2048 148 us in the FMA form), which is why the tokens of a tile go down to 32.  Pairs of CTAs and the persistent walk as in
 // gemm_pair.cuh; the weights are read as fp32 and split on their way into shared memory (6 bytes in memory for every 4 would cost more
-// than the conversion, which needs 40 % of the issue slots), the rows of X, read by every tile, are split beforehand.
-//   warp 0      loads: the three pieces of this CTA's token half (64 rows x 64 k each)
-//   warp 1      leader only: the products
-//   warps 2-5   sums: thread = output column, up to 128 tokens in registers
-//   warps 6-9   weights: 128 rows x 64 k of fp32, the next k-block's loads in flight while this one is split and stored (128B swizzle)
+// than the conversion), the rows of X, read by every tile, are split beforehand.  Two stages of 84 KB.  The large sums (hh) and the five small ones have an accumulator
+// of 192 columns each; the small terms of a k-block go first, so that the large sums of the segment before leave tensor memory under them.
+//   warp 0       loads: the three pieces of this CTA's token half (up to 96 rows x 64 k each, in boxes of 32 rows)
+//   warp 1       leader only: the products
+//   warps 4-7    sums: thread = output column, up to 192 tokens in registers (232 of them)
+//   warps 8-15   weights: 128 rows x 64 k of fp32, the next k-block's loads in flight while this one is split and stored (128B swizzle)
 #pragma once
 #include "gemm_pair.cuh"
 
@@ -285,8 +285,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const GemmSplitParams
         float* out = p.out + tl.b * p.c_stride + ((size_t)tl.split * p.M + tl.m0) * p.ldc + n;
         bool again = false;
 #pragma unroll
-        for (int m = 0; m < kSplitTokens; ++m)
-          if (m < tl.rows) { out[(size_t)m * p.ldc] = acc[m]; again |= split_again(acc[m]); }
+        for (int c = 0; c < kSplitTokens; c += 16) {
+          if (c >= tl.rows) break;   // (few rows fetch no more instructions than they need: with those of 192 rows a decoding step took 4 us more per product: kefurax s, 3 layers, 2 sequences 657 us, 473 so)
+#pragma unroll
+          for (int m = c; m < c + 16; ++m)
+            if (m < tl.rows) { out[(size_t)m * p.ldc] = acc[m]; again |= split_again(acc[m]); }
+        }
         if (again) s_again = 1;
       }
     }
