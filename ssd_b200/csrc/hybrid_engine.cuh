@@ -876,7 +876,8 @@ struct HybRun {
   }
 
   // Latent attention of whole prompts (every sequence of the call starts in it): keys and values of every head are made first, 2 x kv_rank products per
-  // entry, and a (query, key) pair then costs dim + rot + vdim of them instead of 2 kv_rank + rot.
+  // entry, and a (query, key) pair then costs dim + rot + vdim of them instead of 2 kv_rank + rot.  A call with a single token or a later portion in it
+  // takes the absorbed form for all its sequences, so that a prompt's bits depend on whether such a one is beside it.
   bool latent_whole(const HybLayer& Lr, const uint8_t* pool, const float* gate, int ldq) const {
     const ssdk_hyb_layer_cfg& c = Lr.c;
     const int H = c.heads, Wd = c.kv_rank + c.rot_dim;
@@ -1421,7 +1422,7 @@ struct HybRun {
       int lo = mask.first(p0), kept = mask.kept(lo), ctx = p0 + n - lo + kept, ctx_pad = (ctx + 7) / 8 * 8;   // the kept keys, then lo .. p0 + n - 1
       const bool per_block = mask.keep > 0;   // kept keys must lie beside a block's own: every query block is gathered by itself
       auto gather = [&]() {
-        return L.go(ssdk::kv_gather_kernel<T>, dim3((ctx_pad + ssdk::kKvKeys - 1) / ssdk::kKvKeys, G), dim3(32, 8), 0, (const T*)pool, (T*)e->keys, (T*)e->lat_t, rg, s, lo, kept, ctx,
+        return L.go(ssdk::kv_gather_kernel<T>, dim3((ctx_pad + ssdk::kKvKeys - 1) / ssdk::kKvKeys, G, (std::max(D, V) + 31) / 32), dim3(32, 8), 0, (const T*)pool, (T*)e->keys, (T*)e->lat_t, rg, s, lo, kept, ctx,
                     ctx_pad, G, D, V, maps);
       };
       if (!per_block) CKI(gather());
