@@ -290,6 +290,11 @@ static int launch_gemm_split(Launcher& L, const CUtensorMap& tmX, GemmSplitParam
 // matrices here; qwen3-0.6b, 4 layers, one sequence 283 -> 262 (up to 9 MB), 244 (13 and 30 MB).  M <= 8 is the token side of the instruction: two
 // tiles of tokens cost registers for the loads in flight (16 rows of llama-3.2-1b 412 -> 430 us).
 static bool few_rows(int M, int64_t N, int K) { return M <= kFewTokens && N * K * 2 <= (30 << 20); }
+// The dense decoders' products, whose split-K partials the kernel behind sums on its way, so that less is saved: above four rows only with few k or small matrices
+// (a CTA reads M K of x behind its wait for every 16 K of weights).  Steps of the 8B + 1B pair, whose 1B layers have matrices of 8 and 13 MB over k = 2048:
+// 3, 5, 8 sequences 6334, 6454, 6844 us on gemm_ws_kernel, 6331, 6626, 7089 here.  Of the Qwen pair (13 and 8 MB over k = 1024, 4 and 6 MB above): 2, 4, 5, 8
+// sequences 5048, 5256, 5358, 5850 -> 4105, 4223, 4438, 4662; without the 13 MB matrix at five and eight rows 5275, 5652.
+static bool few_rows_dense(int M, int64_t N, int K) { return few_rows(M, N, K) && (M <= 4 || K <= 1024 || N * K * 2 < (8 << 20)); }
 // fp32, bf16 or act(gate) * up in bf16; W and X start on 16-byte boundaries, their strides are whole 16-byte pieces, K % 64 == 0
 static int launch_gemm_few(Launcher& L, int epi, const void* X, int ldx, const void* W, int ldw, void* out, int ldo, int M, int N, int K, bool gelu = false,
                            int heads = 1, int x_step = 0, int out_step = 0,
@@ -744,10 +749,13 @@ static int enqueue_gemm(ssdk_engine* e, Launcher& L, const bf16* x, WeightMat& w
     if (splits_out) *splits_out = 0;
     return launch_gemm_pair(L, epi == EPI_SILU ? EPI_GLU : EPI_BF16, *tmW, *tmX, *tmXs, p, p.w_tiles * p.chunks);
   }
-  if (epi != EPI_PUBLISH && few_rows(M, w.rows, K)) {
+  if (epi != EPI_PUBLISH && few_rows_dense(M, w.rows, K)) {
     if (splits_out) *splits_out = 1;
-    const bool ahead2 = next2 && few_rows(M, next2->rows, (int)next2->cols);
-    const bool ahead = next && few_rows(M, next->rows, (int)next->cols);
+    // The weights of the products behind this one that this form takes are asked for into L2 meanwhile: attention and norms in between leave the memory idle.  Steps of the
+    // Qwen pair (16 draft layers), 2, 4, 8 sequences 4220, 4275, 4770 us without, 4110, 4221, 4665 so; of the 8B + 1B pair, 2 sequences 6178, 6122; a token through
+    // four layers of the 0.6B model 251, 245, of the 1B model 356, 354
+    const bool ahead2 = next2 && few_rows_dense(M, next2->rows, (int)next2->cols);
+    const bool ahead = next && few_rows_dense(M, next->rows, (int)next->cols);
     return launch_gemm_few(L, epi == EPI_SILU ? FEW_SILU : epi == EPI_BF16 ? FEW_BF16 : FEW_F32, x, K, w.ptr, K, out, epi == EPI_PARTIAL ? N_out : ldo, M, N_out, K, false, 1, 0, 0,
                            ahead ? next->ptr : nullptr, ahead ? next->rows * next->cols * 2 : 0, ahead2 ? next2->ptr : nullptr, ahead2 ? next2->rows * next2->cols * 2 : 0);
   }
