@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(attn_warps(MT) * 32, OCC) paged_attn_kernel(At
   pdl_launch_dependents();
   // While the kernel in front (the rotation) runs, the first keys and values of this CTA's range are asked for into L2: a hint that reads nothing, so that it
   // does not matter that lengths and table may still be those of the step before (bounded by the caches here, read past L1).
-  // Four contexts of 1500, 28 layers of 8 key heads: a step of five draft passes 5822 -> 5682 us; 16 contexts of 4000, four 8B layers 795 -> 789.
+  // Four contexts of 1500, 28 layers of 8 key heads: a step of five draft passes 5822 -> 5682 us; 16 contexts of 4000, four 8B layers the same.
   if (p.pages > 0 && p.block_size % kAttChunk == 0) {
     const int b = blockIdx.y / p.n_split, split = blockIdx.y - b * p.n_split;
     const int nch = (min(max(__ldcg(p.context_lens + b), 0), p.max_blocks * p.block_size) + kAttChunk - 1) / kAttChunk, cps = (nch + p.n_split - 1) / p.n_split;

@@ -662,21 +662,28 @@ static int enqueue_attention(Launcher& L, const bf16* q, const bf16* kc, const b
   return 0;
 }
 
-// keys come in whole chunks of a page, a key head's query heads fill tiles (taken by passes of more rows than kMaxTokens)
+// keys come in whole chunks of a page, a key head's query heads fill tiles (taken by passes of more rows than kMaxTokens, and by the shorter ones that attn_on_tiles names)
 static bool prompt_attn_ok(int H, int KV, int hd, int block_size, int64_t num_blocks) {
   const int G = H / KV;
   return (hd == 64 || hd == 128) && H % KV == 0 && G <= 16 && (G & (G - 1)) == 0 && H < 2048 && block_size % kPromptKeys == 0 &&
          num_blocks * block_size < (1ll << 31);
 }
 // Calls of few rows on the same tiles, their keys in ranges.  A tile holds all query heads of a key head for up to 128 rows, where paged_attn_kernel
-// reads the keys once per 32 rows and is bound by its instructions; it costs 2 us more to start.  us with the merge, 32-row tiles -> this one:
-// 7 rows x 8 query heads of 128 per key head, 8 x 8000 keys 106 -> 56, 4 x 2000 26 -> 19, 1 x 1000 12.7 -> 10.7, 1 x 500 9.8 -> 9.7, 1 x 200 9.5 -> 10.0;
-// 7 x 4, 8 x 8000 66 -> 52, 1 x 2000 13.5 -> 12.4, 1 x 1000 10.0 -> 10.7.  Up to 16 rows (one m16 tile) the instructions fit: 1 x 8, 8 x 8000 46 -> 51.
-// The line follows from the sizes of the call and the table alone, so that a sequence's result does not depend on what it is batched with.
+// reads the keys once per 32 rows and is bound by its instructions; it costs 2 us more to start.  What decides are the 32-row tiles of the other form (key heads x
+// sequences x tiles of a sequence): from 16 of them on heads of 128 gain with long contexts and lose little with short ones; heads of 64 halve the instructions
+// per key, so that only several tiles of one sequence gain.  us with the merge, 32-row tiles -> this one, tables of 8192 keys, heads / key heads x size:
+//   64/8 x 128, 5 rows of contexts of 100, 500, 2000, 6000: 1 sequence (16 tiles) 10.5 -> 9.9, 10.7 -> 10.0, 13.1 -> 12.3, 25.0 -> 18.1; 4 (64) 10.6 -> 11.3,
+//     13.5 -> 12.8, 28.7 -> 19.7, 66.3 -> 32.2; 8 (128) 13.2 -> 11.2, 22.3 -> 13.6, 47.0 -> 23.3, 105 -> 47; 3 rows, 1 sequence (8) 8.7 -> 9.8, 8.9 -> 9.5, 12.3 -> 11.9, 17.2 -> 16.7
+//   32/8 x 128, 8 rows: 1 sequence (8) 9.4 -> 10.1, 9.5 -> 9.9, 13.5 -> 11.9, 18.2 -> 17.4; 2 (16) 11.7 -> 10.1, 11.9 -> 10.7, 14.9 -> 14.8, 27.9 -> 21.3
+//   32/8 x 64, uneven contexts up to 400, 2000, 6000: 8 rows, 8 sequences (64) 9.9 -> 10.5, 18.4 -> 17.9, 36.8 -> 35.3, 16 (128) 16.2 -> 13.2, 28.8 -> 27.6, 58.6 -> 61.2;
+//     5 rows, 4 sequences (32) 8.5 -> 9.4, 11.9 -> 13.1, 20.2 -> 23.8; 16 rows, 4 sequences (64) 10.2 -> 11.1, 18.4 -> 14.8, 32.9 -> 25.4
+// Up to 16 rows per key head (one m16 tile) the instructions fit.  Tables too short for the ranges to matter stay.  The line follows from the number of sequences and rows and
+// the table's size, not from the contexts: lengths of the neighbours do not move a sequence's result, their number may.
 static bool attn_on_tiles(int H, int KV, int hd, int B, int Q, int block_size, int64_t num_blocks, int max_ctx) {
   if (!prompt_attn_ok(H, KV, hd, block_size, num_blocks) || H / KV * Q <= 16) return false;
-  const int tokens = std::max(1, 32 / (H / KV));
-  return (int64_t)B * ((Q + tokens - 1) / tokens) * max_ctx >= 2000;
+  const int tokens = std::max(1, 32 / (H / KV)), per_seq = (Q + tokens - 1) / tokens;
+  const int64_t tiles = (int64_t)KV * B * per_seq;
+  return (int64_t)B * per_seq * max_ctx >= 2000 && (hd == 128 ? tiles >= 16 : per_seq > 1 && tiles >= 64);
 }
 // ranges per sequence: three CTAs for two SMs (two are resident; 8 x 8000 keys 65.7 us with one per SM, 56.4, 58.7 with two)
 static int tile_splits(int H, int KV, int B, int Q, int max_ctx) {

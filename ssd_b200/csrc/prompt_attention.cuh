@@ -32,7 +32,7 @@ struct PromptAttnParams {
   int block_size, max_blocks;    // block_size a multiple of kPromptKeys
   int n_slots;                   // token slots of the cache: a chunk without a page is loaded from behind them (zeros)
   float scale_log2;              // > 0
-  unsigned* timeout;             // (nullptr: calls without an engine; rows whose waits ran out are NaN)
+  unsigned* timeout;             // (rows whose waits ran out are NaN)
   // SPLIT: the keys of a sequence in n_split ranges of whole chunks, as paged_attn_kernel cuts them; what a range gives goes to
   // part_o [B*Q*H, n_split, hd] and part_lse [B*Q*H, n_split] (fp32, see attn_combine_kernel)
   int n_split;

@@ -211,8 +211,8 @@ class PairRunner:
                 want_sample: bool = True, chunk: int = WHOLE_PASS, seed: int = 0):
         """Prefill one sequence from position `start` in passes through the multi-query path: the weights are streamed
         once per pass, attention is causal over the cache, which already holds the earlier passes
-        (layers/attention.py:85-93): tcgen05 tiles of 128 rows in passes of more than 256, the paged multi-query kernel with
-        tiles of up to 64 rows in shorter ones.
+        (layers/attention.py:85-93): tcgen05 tiles of 128 rows in passes of more than 256 and, with the keys
+        cut into ranges, in shorter ones of enough rows and heads, else the paged multi-query kernel with tiles of up to 32 rows.
         chunk: tokens of a pass at most, up to 256; if not given, a pass carries what the engine takes (pass_tokens)."""
         call, size = _prompt_call(self, which, chunk)
         tok = None

@@ -39,7 +39,7 @@ def test_against_float64(heads, kv_heads, hd, q_len, ctx):
             assert torch.isfinite(off).all() and off.max().item() < 1, (b, h, off.max().item())
 
 
-@pytest.mark.parametrize("heads,kv_heads,hd,q_len,ctx", [(64, 8, 128, 7, [1500, 64, 1, 700]), (32, 8, 64, 8, [300, 2, 900]), (16, 1, 128, 3, [60, 130, 4000]),
+@pytest.mark.parametrize("heads,kv_heads,hd,q_len,ctx", [(64, 8, 128, 7, [1500, 64, 1, 700]), (32, 8, 64, 16, [300, 2, 900, 40]), (16, 1, 128, 3, [60, 130, 4000, 7, 1000, 2, 300, 64]),
                                                          (32, 32, 128, 100, [50, 400])])
 def test_weights_keep_sixteen_bits(heads, kv_heads, hd, q_len, ctx):
     """The output is rounded to bf16 (eight significant bits: 2^-8 of it at most); weights are not (two pieces: 2^-17), and fp32 sums of scores and products move them
