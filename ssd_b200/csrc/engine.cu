@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cstdarg>
 #include <cstdio>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <map>
@@ -1348,7 +1349,12 @@ static int get_spec_graph(ssdk_engine* e, int B, bool host_io, bool stream_draft
 }
 
 // pre-set >48 KB dynamic smem opt-ins so nothing but launches happens during capture
+// (once per device: thirty calls of the runtime are 4 us, which a stand-alone op would pay every time)
 static int init_kernel_attrs() {
+  static std::atomic<bool> done[64];
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  if (dev < 64 && done[dev].load(std::memory_order_acquire)) return 0;
 #define SSDK_ATTR_G(UN, EP) \
   CK(cudaFuncSetAttribute(gemm_ws_kernel<UN, EP>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<UN>::kSmemBytes));
   SSDK_ATTR_G(16, EPI_BF16) SSDK_ATTR_G(16, EPI_PARTIAL) SSDK_ATTR_G(16, EPI_SILU) SSDK_ATTR_G(16, EPI_GLU) SSDK_ATTR_G(16, EPI_PUBLISH)
@@ -1369,6 +1375,7 @@ static int init_kernel_attrs() {
   SSDK_ATTR_P(64, false, false) SSDK_ATTR_P(64, false, true) SSDK_ATTR_P(64, true, true) SSDK_ATTR_P(128, false, false) SSDK_ATTR_P(128, false, true) SSDK_ATTR_P(128, true, true)
 #undef SSDK_ATTR_P
   CK(cudaFuncSetAttribute(add_rmsnorm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+  if (dev < 64) done[dev].store(true, std::memory_order_release);
   return 0;
 }
 
@@ -1948,6 +1955,7 @@ int ssdk_paged_attn_pages(const void* q, const void* k_cache, const void* v_cach
                            max_blocks_per_seq, scale, stream);
   Launcher L;
   L.st = (cudaStream_t)stream;
+  CKI(init_kernel_attrs());
   float* part_o = (float*)((uint8_t*)scratch + 16384);
   float* part_lse = part_o + (size_t)batch * q_len * heads * kAttnMaxSplit * head_dim;
   const int G = heads / kv_heads;
