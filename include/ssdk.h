@@ -255,7 +255,8 @@ int ssdk_paged_attn(const void* q, const void* k_cache, const void* v_cache,
                     int batch, int q_len, int heads, int kv_heads, int head_dim,
                     int block_size, int max_blocks_per_seq, float scale, void* stream);
 
-/* ssdk_paged_attn for a cache of num_blocks pages whose size the caller knows. */
+/* ssdk_paged_attn for a cache of num_blocks pages whose size the caller knows.  Some calls take kernels with bounded waits: a wait that runs out leaves
+ * NaN rows, and the next such call of the process returns an error. */
 int ssdk_paged_attn_pages(const void* q, const void* k_cache, const void* v_cache,
                           const int32_t* block_tables, const int32_t* context_lens,
                           void* out, void* scratch,

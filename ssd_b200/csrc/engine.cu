@@ -249,13 +249,26 @@ struct WaitWord {
     *word = 0;
     return true;
   }
-  int check() {
+  int check(const char* whose = "this engine's calls left since the last check is not complete") {
     volatile unsigned* w = word;
     if (!*w) return 0;
     *w = 0;
-    return fail("a bounded wait in a tile-pair product or the prompt attention ran out: what this engine's calls left since the last check is not complete");
+    return fail("a bounded wait in a tile-pair product or the prompt attention ran out: what %s", whose);
   }
 };
+// The same for calls without an engine, which do not wait for the stream: rows whose waits ran out are NaN, and the next such call reports it.  One word for the
+// process that is never freed (a kernel in flight may still write to it); made under relaxed capture rules, since the first such call may be a captured one.
+static WaitWord* op_waits() {
+  static WaitWord* const w = [] {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    WaitWord* made = new WaitWord;
+    if (!made->make()) { delete made; made = nullptr; }
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    return made;
+  }();
+  return w;
+}
 
 // tile pairs of gemm_pair_kernel; p.timeout is filled in here
 static int launch_gemm_pair(Launcher& L, int epi, const CUtensorMap& tmW, const CUtensorMap& tmX, const CUtensorMap& tmXs, GemmPairParams p, int max_tiles) {
@@ -1956,6 +1969,9 @@ int ssdk_paged_attn_pages(const void* q, const void* k_cache, const void* v_cach
   Launcher L;
   L.st = (cudaStream_t)stream;
   CKI(init_kernel_attrs());
+  WaitWord* waits = op_waits();
+  if (!waits) return fail("paged_attn: pinned word for bounded waits not allocated");
+  CKI(waits->check("an earlier call of paged attention without an engine left is not complete (NaN rows)"));
   float* part_o = (float*)((uint8_t*)scratch + 16384);
   float* part_lse = part_o + (size_t)batch * q_len * heads * kAttnMaxSplit * head_dim;
   const int G = heads / kv_heads;
@@ -1965,7 +1981,7 @@ int ssdk_paged_attn_pages(const void* q, const void* k_cache, const void* v_cach
   CKI(make_tmap_heads(&tmK, k_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
   CKI(make_tmap_heads(&tmV, v_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
   return enqueue_prompt_attention(L, tmQ, tmK, tmV, block_tables, context_lens, (bf16*)out, batch, q_len, heads, kv_heads, head_dim, block_size,
-                                  max_blocks_per_seq, slots, scale, nullptr, true, tile_splits(heads, kv_heads, batch, q_len, max_ctx), part_o, part_lse);
+                                  max_blocks_per_seq, slots, scale, waits->word, true, tile_splits(heads, kv_heads, batch, q_len, max_ctx), part_o, part_lse);
 }
 
 int ssdk_prompt_attn(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
