@@ -704,26 +704,34 @@ static int tile_splits(int H, int KV, int B, int Q, int max_ctx) {
   const int tokens = kPromptRows / (H / KV), ctas = KV * B * ((Q + tokens - 1) / tokens);
   return std::max(1, std::min({(3 * num_sms() + 2 * ctas - 1) / (2 * ctas), kAttnMaxSplit, (max_ctx + kPromptKeys - 1) / kPromptKeys}));
 }
-template <int HD, bool SPLIT, bool FINE>
+// How a call of few rows keeps its weights (see prompt_attn_kernel).  Rows of their own cost 1 us a call, a second product 0.2 us a chunk of keys.  64/8 heads x 128, 5 rows, one
+// product more -> twin rows, us: 16 sequences of up to 6000 keys 91 -> 84, 4 of 6000 (18 chunks a range) 32.2 -> 30.7, 4 of 100 11.4 -> 12.6, 8 of 100 11.2 -> 12.3
+static int prompt_pieces(int H, int KV, int Q, int max_ctx, int n_split) {
+  return H / KV * Q <= kPromptRows / 2 && max_ctx / kPromptKeys >= 24 * n_split ? kPromptTwin : kPromptTwo;
+}
+static int prompt_box(int H, int KV, int pieces) { return (pieces == kPromptTwin ? kPromptRows / 2 : kPromptRows) / (H / KV); }   // query tokens of a tile
+template <int HD, bool SPLIT, int P>
 static int launch_prompt_inst(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const PromptAttnParams& p, int B) {
   static bool attr_set = false;
   if (!attr_set) {
-    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD)));
-    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT, FINE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD)));
+    CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT, P>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     attr_set = true;
   }
-  const int tq = kPromptRows >> p.g_shift, nqt = (p.Q + tq - 1) / tq;
-  return L.go(prompt_attn_kernel<HD, SPLIT, FINE>, dim3(p.KV, nqt, B * p.n_split), dim3(kPromptThreads), (size_t)prompt_attn_smem(HD), tmQ, tmK, tmV, p);
+  const int tq = (P == kPromptTwin ? kPromptRows / 2 : kPromptRows) >> p.g_shift, nqt = (p.Q + tq - 1) / tq;
+  return L.go(prompt_attn_kernel<HD, SPLIT, P>, dim3(p.KV, nqt, B * p.n_split), dim3(kPromptThreads), (size_t)prompt_attn_smem(HD), tmQ, tmK, tmV, p);
 }
 template <int HD>
-static int launch_prompt_attn(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const PromptAttnParams& p, int B, bool fine) {
-  if (p.n_split > 1) return launch_prompt_inst<HD, true, true>(L, tmQ, tmK, tmV, p, B);
-  return fine ? launch_prompt_inst<HD, false, true>(L, tmQ, tmK, tmV, p, B) : launch_prompt_inst<HD, false, false>(L, tmQ, tmK, tmV, p, B);
+static int launch_prompt_attn(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const PromptAttnParams& p, int B, int pieces) {
+  if (pieces == kPromptOne) return launch_prompt_inst<HD, false, kPromptOne>(L, tmQ, tmK, tmV, p, B);
+  if (pieces == kPromptTwin)
+    return p.n_split > 1 ? launch_prompt_inst<HD, true, kPromptTwin>(L, tmQ, tmK, tmV, p, B) : launch_prompt_inst<HD, false, kPromptTwin>(L, tmQ, tmK, tmV, p, B);
+  return p.n_split > 1 ? launch_prompt_inst<HD, true, kPromptTwo>(L, tmQ, tmK, tmV, p, B) : launch_prompt_inst<HD, false, kPromptTwo>(L, tmQ, tmK, tmV, p, B);
 }
 // maps of queries, keys and values of layer caches of `slots` token slots: {box of a tile's query tokens, kPromptKeys keys of one head}
 static int enqueue_prompt_attention(Launcher& L, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const int32_t* bt,
                                     const int32_t* ctx_lens, bf16* out, int B, int Q, int H, int KV, int hd, int block_size, int max_blocks,
-                                    int64_t slots, float scale, unsigned* timeout, bool fine, int n_split = 1, float* part_o = nullptr, float* part_lse = nullptr) {
+                                    int64_t slots, float scale, unsigned* timeout, int pieces, int n_split = 1, float* part_o = nullptr, float* part_lse = nullptr) {
   PromptAttnParams p = {};
   p.n_split = n_split; p.part_o = part_o; p.part_lse = part_lse;
   p.block_tables = bt; p.context_lens = ctx_lens; p.out = out; p.Q = Q; p.H = H; p.KV = KV; p.block_size = block_size; p.max_blocks = max_blocks;
@@ -731,7 +739,7 @@ static int enqueue_prompt_attention(Launcher& L, const CUtensorMap& tmQ, const C
   p.n_slots = (int)slots;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.timeout = timeout;
-  CKI(hd == 128 ? launch_prompt_attn<128>(L, tmQ, tmK, tmV, p, B, fine) : launch_prompt_attn<64>(L, tmQ, tmK, tmV, p, B, fine));
+  CKI(hd == 128 ? launch_prompt_attn<128>(L, tmQ, tmK, tmV, p, B, pieces) : launch_prompt_attn<64>(L, tmQ, tmK, tmV, p, B, pieces));
   if (n_split > 1) {
     AttnParams a = {};
     a.context_lens = ctx_lens; a.out = out; a.part_o = part_o; a.part_lse = part_lse; a.B = B; a.Q = Q; a.H = H; a.KV = KV; a.TQ = kPromptRows >> p.g_shift; a.n_split = n_split;
@@ -744,10 +752,11 @@ static int forward_prompt_attention(ssdk_engine* e, Launcher& L, const Model& m,
   const int64_t slots = m.num_blocks * block_size;
   const int G = m.H / m.KV;
   const CUtensorMap *tmQ, *tmK, *tmV;
-  CKI(e->xmaps.get_heads(q, B * Q > kMaxTokens ? kMaxPass : kMaxTokens, m.H, m.hd, G, kPromptRows / G, &tmQ));
+  const int pieces = B * Q > kMaxTokens ? kPromptOne : prompt_pieces(m.H, m.KV, Q, max_blocks * block_size, n_split);
+  CKI(e->xmaps.get_heads(q, B * Q > kMaxTokens ? kMaxPass : kMaxTokens, m.H, m.hd, G, prompt_box(m.H, m.KV, pieces), &tmQ));
   CKI(e->xmaps.get_heads(kc, slots, m.KV, m.hd, 1, kPromptKeys, &tmK));
   CKI(e->xmaps.get_heads(vc, slots, m.KV, m.hd, 1, kPromptKeys, &tmV));
-  return enqueue_prompt_attention(L, *tmQ, *tmK, *tmV, bt, ctx_lens, out, B, Q, m.H, m.KV, m.hd, block_size, max_blocks, slots, scale, L.gave_up, B * Q <= kMaxTokens, n_split,
+  return enqueue_prompt_attention(L, *tmQ, *tmK, *tmV, bt, ctx_lens, out, B, Q, m.H, m.KV, m.hd, block_size, max_blocks, slots, scale, L.gave_up, pieces, n_split,
                                   e->ws.att_o, e->ws.att_lse);
 }
 
@@ -1382,10 +1391,11 @@ static int init_kernel_attrs() {
   SSDK_ATTR_A(128, 1, 3) SSDK_ATTR_A(128, 2, 1) SSDK_ATTR_A(128, 2, 2) SSDK_ATTR_A(128, 4, 1) SSDK_ATTR_A(128, 4, 2)
   SSDK_ATTR_A(64, 1, 3) SSDK_ATTR_A(64, 2, 1) SSDK_ATTR_A(64, 2, 2) SSDK_ATTR_A(64, 4, 1) SSDK_ATTR_A(64, 4, 2)
 #undef SSDK_ATTR_A
-#define SSDK_ATTR_P(HD, SPLIT, FINE) \
-  CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD))); \
-  CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT, FINE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-  SSDK_ATTR_P(64, false, false) SSDK_ATTR_P(64, false, true) SSDK_ATTR_P(64, true, true) SSDK_ATTR_P(128, false, false) SSDK_ATTR_P(128, false, true) SSDK_ATTR_P(128, true, true)
+#define SSDK_ATTR_P(HD, SPLIT, P) \
+  CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, prompt_attn_smem(HD))); \
+  CK(cudaFuncSetAttribute(prompt_attn_kernel<HD, SPLIT, P>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  SSDK_ATTR_P(64, false, kPromptOne) SSDK_ATTR_P(64, false, kPromptTwo) SSDK_ATTR_P(64, true, kPromptTwo) SSDK_ATTR_P(64, false, kPromptTwin) SSDK_ATTR_P(64, true, kPromptTwin)
+  SSDK_ATTR_P(128, false, kPromptOne) SSDK_ATTR_P(128, false, kPromptTwo) SSDK_ATTR_P(128, true, kPromptTwo) SSDK_ATTR_P(128, false, kPromptTwin) SSDK_ATTR_P(128, true, kPromptTwin)
 #undef SSDK_ATTR_P
   CK(cudaFuncSetAttribute(add_rmsnorm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
   if (dev < 64) done[dev].store(true, std::memory_order_release);
@@ -1977,11 +1987,12 @@ int ssdk_paged_attn_pages(const void* q, const void* k_cache, const void* v_cach
   const int G = heads / kv_heads;
   const int64_t slots = num_blocks * block_size;
   CUtensorMap tmQ, tmK, tmV;
-  CKI(make_tmap_heads(&tmQ, q, (int64_t)batch * q_len, heads, head_dim, G, kPromptRows / G));
+  const int n_split = tile_splits(heads, kv_heads, batch, q_len, max_ctx), pieces = prompt_pieces(heads, kv_heads, q_len, max_ctx, n_split);
+  CKI(make_tmap_heads(&tmQ, q, (int64_t)batch * q_len, heads, head_dim, G, prompt_box(heads, kv_heads, pieces)));
   CKI(make_tmap_heads(&tmK, k_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
   CKI(make_tmap_heads(&tmV, v_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
   return enqueue_prompt_attention(L, tmQ, tmK, tmV, block_tables, context_lens, (bf16*)out, batch, q_len, heads, kv_heads, head_dim, block_size,
-                                  max_blocks_per_seq, slots, scale, waits->word, true, tile_splits(heads, kv_heads, batch, q_len, max_ctx), part_o, part_lse);
+                                  max_blocks_per_seq, slots, scale, waits->word, pieces, n_split, part_o, part_lse);
 }
 
 int ssdk_prompt_attn(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables,
@@ -1999,7 +2010,7 @@ int ssdk_prompt_attn(const void* q, const void* k_cache, const void* v_cache, co
   CKI(make_tmap_heads(&tmK, k_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
   CKI(make_tmap_heads(&tmV, v_cache, slots, kv_heads, head_dim, 1, kPromptKeys));
   return enqueue_prompt_attention(L, tmQ, tmK, tmV, block_tables, context_lens, (bf16*)out, batch, q_len, heads, kv_heads, head_dim, block_size,
-                                  max_blocks_per_seq, slots, scale, gave_up, false);
+                                  max_blocks_per_seq, slots, scale, gave_up, kPromptOne);
 }
 
 int ssdk_sample(const void* logits, int64_t ld, const float* temps, int B, int V, uint64_t seed, uint64_t step_id,

@@ -217,7 +217,7 @@ gqa_prompt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         }
       }
       const float ms = m == -INFINITY ? 0.f : m;
-      l += row_exp<FINE>(u, p.scale_log2, ms);
+      l += row_exp<true, FINE>(u, p.scale_log2, ms);
 #pragma unroll
       for (int c = 0; c < (FINE ? 64 : 32); c += 16) tmem_st_32x32b_x16(sp + c, u + c);
       tmem_st_wait();

@@ -7,10 +7,12 @@
 //   O += P V       P from TMEM, V as it lies in the cache (MN-major operand), fp32 in TMEM
 // m is raised, and O and the sum rescaled, only when a row's maximum has grown by more than kPromptSlack (base 2): P then stays below
 // 2^kPromptSlack, where bf16 and fp32 are as fine relative to a value as below 1.  But a row's largest weight is no longer exactly 1, and is rounded like all others;
-// paged_attn_kernel follows the maximum of every token slice and rounds none of those.  FINE (the calls that this kernel takes over from it) therefore gives P
-// as two bf16 pieces, 16 significant bits, and multiplies each with V.  Relative error of a 70B layer's attention against 64 bits, 8 x 7 rows of contexts of 4500
+// paged_attn_kernel follows the maximum of every token slice and rounds none of those.  The calls that this kernel takes over from it therefore give P
+// as two bf16 pieces, 16 significant bits, which both meet V.  Relative error of a 70B layer's attention against 64 bits, 8 x 7 rows of contexts of 4500
 // to 8000 / 4 x 8 of 1880 to 3000 / 2 x 8 of 220 to 300: 0.00275, 0.00268, 0.00252 in paged_attn_kernel, 0.00289, 0.00286, 0.00264 with one piece, 0.00237,
-// 0.00237, 0.0023 with two, which cost 12 % of the first (60 -> 67 us; paged_attn_kernel 109).  Pieces cut off instead of rounded: the same time.
+// 0.00237, 0.0023 with two.  The softmax hardly notices; what costs is a second product per chunk (the first: 60 -> 67 us, 109 in paged_attn_kernel).  Calls of up to 64 rows
+// and long tables load their queries twice: rows 64 .. 127 are the same rows again, give the low pieces and add up in accumulator lanes of their own, so that one product
+// takes both, and the warps that would idle do the work (62 us).
 // Warps: 0 loads, 1 issues the products, 2-5 softmax and output.  Two CTAs per SM (97 KB, 256 TMEM columns each), so that one's products
 // run under the other's exponentials, which bound the kernel.
 // 2003 tokens, 32 heads of 128 over 8: 205 us on mma.sync tiles of 64 rows (paged_attn_kernel), 47 us here = 700 TFLOP/s of the masked work;
@@ -80,12 +82,14 @@ SSDK_DEVINL float row_max(const uint32_t (&u)[64]) {
     for (int e = 0; e < 4; ++e) m[e] = max3(m[e], __uint_as_float(u[c + e]), __uint_as_float(u[c + 4 + e]));
   return fmaxf(max3(m[0], m[1], __uint_as_float(u[60])), max3(m[2], m[3], max3(__uint_as_float(u[61]), __uint_as_float(u[62]), __uint_as_float(u[63]))));
 }
-// 2^(score * scale - ms) of a row: rounded to bf16 in the first 32 words (FINE: what that leaves, rounded to bf16, in the others), their sum (of the unrounded ones)
-// back.  Products and sums two at a time; a probability below 2^-126 is zero (the row's largest is at least 2^-kPromptSlack).
-template <bool FINE>
+// Weights of a product with V: one bf16 piece; two, side by side in the columns of their scores; two, in rows of their own
+enum { kPromptOne = 0, kPromptTwo = 1, kPromptTwin = 2 };
+
+// 2^(score * scale - ms) of a row, and their sum (of the unrounded ones) back.  HIGH: rounded to bf16 in the first 32 words; LOW: what that leaves, rounded, in the
+// others (without HIGH in the first).  Products and sums two at a time; a probability below 2^-126 is zero (the row's largest is at least 2^-kPromptSlack).
+template <bool HIGH, bool LOW>
 SSDK_DEVINL float row_exp(uint32_t (&u)[64], float scale, float ms) {
-  const uint64_t sc = pack2(scale, scale), off = pack2(-ms, -ms);
-  const uint64_t minus = pack2(-1.f, -1.f);
+  const uint64_t sc = pack2(scale, scale), off = pack2(-ms, -ms), minus = pack2(-1.f, -1.f);
   uint64_t sum[2] = {0, 0};
   uint32_t low[32];
 #pragma unroll
@@ -95,14 +99,14 @@ SSDK_DEVINL float row_exp(uint32_t (&u)[64], float scale, float ms) {
     a = ex2_ftz(a); e = ex2_ftz(e);
     sum[(c >> 1) & 1] = add2(sum[(c >> 1) & 1], pack2(a, e));
     const uint32_t h = pack_bf16x2(a, e);
-    u[c >> 1] = h;
-    if (FINE) {   // (exact differences)
+    if (HIGH) u[c >> 1] = h;
+    if (LOW) {   // (exact differences)
       float x, y;
       unpack2(fma2(pack2(__uint_as_float(h << 16), __uint_as_float(h & 0xffff0000u)), minus, pack2(a, e)), &x, &y);
-      low[c >> 1] = pack_bf16x2(x, y);
+      (HIGH ? low : u)[c >> 1] = pack_bf16x2(x, y);
     }
   }
-  if (FINE) {
+  if (HIGH && LOW) {
 #pragma unroll
     for (int c = 0; c < 32; ++c) u[32 + c] = low[c];
   }
@@ -112,8 +116,8 @@ SSDK_DEVINL float row_exp(uint32_t (&u)[64], float scale, float ms) {
   return (s0 + s1) + (s2 + s3);
 }
 
-// grid (kv heads, q tiles, sequences x ranges).  FINE: P in two pieces
-template <int HD, bool SPLIT, bool FINE>
+// grid (kv heads, q tiles, sequences x ranges).  P: kPromptTwin takes tiles of up to 64 rows (their map's boxes hold as many)
+template <int HD, bool SPLIT, int P>
 __global__ void __launch_bounds__(kPromptThreads, 2)
 prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                    const PromptAttnParams p) {
@@ -122,6 +126,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   extern __shared__ uint8_t prompt_smem_raw[];
   __shared__ __align__(8) uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], pv_done[2];
   __shared__ uint32_t tmem_slot;
+  __shared__ int s_failed;   // TWIN: a wait of the low pieces' warps ran out
   uint8_t* smem = prompt_smem_raw + ((1024u - (smem_u32(prompt_smem_raw) & 1023u)) & 1023u);
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + HALVES * kQHalf;
@@ -129,9 +134,12 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.x, qt = (int)gridDim.y - 1 - (int)blockIdx.y;   // (the tiles that see most keys first)
   const int b = SPLIT ? (int)blockIdx.z / p.n_split : (int)blockIdx.z, split = SPLIT ? (int)blockIdx.z - b * p.n_split : 0;
-  const int G = 1 << p.g_shift, TQ = kPromptRows >> p.g_shift;
+  constexpr bool TWIN = P == kPromptTwin;
+  constexpr int ROWS = TWIN ? kPromptRows / 2 : kPromptRows;
+  const int G = 1 << p.g_shift, TQ = ROWS >> p.g_shift;
   const int tok0 = qt * TQ, tq = min(TQ, p.Q - tok0);
-  const int live = SPLIT ? ((tq << p.g_shift) + 31) & ~31 : kPromptRows;   // rows of the warps that have some
+  const int half = ((tq << p.g_shift) + 31) & ~31;                       // rows of the warps that have some
+  const int live = TWIN ? 2 * half : SPLIT ? half : kPromptRows;         // threads that hand P over
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmQ);
@@ -143,6 +151,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       mbar_init(&s_full[s], 1); mbar_init(&p_full[s], live); mbar_init(&pv_done[s], 1);
     }
     fence_mbar_init();
+    s_failed = 0;
   }
   if (warp == 1) { tmem_alloc(&tmem_slot, 256); tmem_relinquish(); }
   tc_fence_before();
@@ -171,7 +180,8 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   if (warp == 0) {
     if (lane == 0 && n > 0) {
       mbar_arrive_expect_tx(&q_full, HALVES * kQHalf);
-      for (int h = 0; h < HALVES; ++h) tma_load_3d(sQ + h * kQHalf, &tmQ, &q_full, h * 64, kvh << p.g_shift, b * p.Q + tok0);
+      for (int h = 0; h < HALVES; ++h)
+        for (int r = 0; r < kPromptRows; r += ROWS) tma_load_3d(sQ + h * kQHalf + r * 128, &tmQ, &q_full, h * 64, kvh << p.g_shift, b * p.Q + tok0);
       const int32_t* bt = p.block_tables + (size_t)b * p.max_blocks;
       int i = 0;
       for (; i < n; ++i) {
@@ -222,7 +232,7 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
         for (int k = 0; k < kPromptKeys / 16; ++k)   // 16 keys: 2048 B of V, 8 columns of P
           umma_bf16_ts(tmem_o, tmem + (i & 1) * 64 + 8 * k, vd + 128 * k, idesc_o, (uint32_t)((i | k) != 0));
-        if (FINE) {
+        if (P == kPromptTwo) {
 #pragma unroll
           for (int k = 0; k < kPromptKeys / 16; ++k) umma_bf16_ts(tmem_o, tmem + (i & 1) * 64 + 32 + 8 * k, vd + 128 * k, idesc_o, 1u);
         }
@@ -232,11 +242,12 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
     __syncwarp();
   } else {
-    const int q = warp & 3, r = q * 32 + lane, tok = r >> p.g_shift;
+    const int q = warp & 3, r = TWIN ? (q & 1) * 32 + lane : q * 32 + lane, tok = r >> p.g_shift;
+    const bool low = TWIN && q >= 2;   // (the whole warp) the same row as two warps before, its low pieces
     const uint32_t lanes = (uint32_t)(q * 32) << 16;
     const int lim = min(ctx0 + tok0 + tok + 1, kv_max);   // keys this row sees (rows behind the tile's tokens: some, dropped)
     float m = -INFINITY, l = 0.f;
-    const bool in = !SPLIT || q * 32 < live;   // (a warp without rows: what the products make of its lanes, nobody reads)
+    const bool in = !(SPLIT || TWIN) || (r & ~31) < half;   // (a warp without rows: what the products make of its lanes, nobody reads)
     bool ok = in;
     for (int i = 0; i < n && in; ++i) {
       const int base = first + i * kPromptKeys;
@@ -273,15 +284,15 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
       }
       const float ms = m == -INFINITY ? 0.f : m;
-      l += row_exp<FINE>(u, p.scale_log2, ms);
+      l += low ? row_exp<false, true>(u, p.scale_log2, ms) : row_exp<true, P == kPromptTwo>(u, p.scale_log2, ms);
 #pragma unroll
-      for (int c = 0; c < (FINE ? 64 : 32); c += 16) tmem_st_32x32b_x16(sp + c, u + c);
+      for (int c = 0; c < (P == kPromptTwo ? 64 : 32); c += 16) tmem_st_32x32b_x16(sp + c, u + c);
       tmem_st_wait();
       if (base + kPromptKeys > kv_max) {   // the last chunk: slots behind the tile's keys hold anything, and 0 x NaN is NaN
         if (!(ok = warp_wait(&v_full[i & 1], parity(i), p.timeout))) break;
         const int from = kv_max - base, pieces = (kPromptKeys - from) * 8;   // 16-byte pieces per half (a row's stay in its 128 bytes)
         for (int h = 0; h < HALVES; ++h)
-          for (int j = r; j < pieces; j += live)
+          for (int j = low ? half + r : r; j < pieces; j += live)
             *reinterpret_cast<uint4*>(sV + (i & 1) * kTile + h * kKHalf + from * 128 + j * 16) = make_uint4(0u, 0u, 0u, 0u);
         fence_proxy_async_smem();
       }
@@ -290,37 +301,62 @@ prompt_attn_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
     if (ok && n > 0) ok = warp_wait(&pv_done[(n - 1) & 1], parity(n - 1), p.timeout);
     tc_fence_after();
-    const float inv = !ok ? __int_as_float(0x7fffffff) : l > 0.f ? 1.f / l : 0.f;   // NaN: a wait ran out
-    const bool mine = in && tok < tq;
-    const size_t row = (size_t)(b * p.Q + tok0 + tok) * p.H + (kvh << p.g_shift) + (r & (G - 1));
-    if (SPLIT) {
-      if (n > 0 && in) {
-        float* dst = p.part_o + (row * p.n_split + split) * HD;
-#pragma unroll 2
+    constexpr int LDO = HD + 4;
+    float* o2 = reinterpret_cast<float*>(sK) + (size_t)(r & (ROWS - 1)) * LDO;   // (the stages: every product has read them)
+    if (TWIN && n > 0 && in) {   // what the low pieces gave goes to the warps of the high ones
+      if (low && !ok) s_failed = 1;
+      if (low && ok) {
         for (int c = 0; c < HD; c += 16) {
           uint32_t o[16];
           tmem_ld_32x32b_x16(tmem_o + lanes + c, o);
           tmem_ld_wait();
-          float f[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(o[j]) * inv;
+          for (int j = 0; j < 16; j += 4) *reinterpret_cast<uint4*>(o2 + c + j) = make_uint4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+        }
+      }
+      asm volatile("bar.sync 1, %0;" ::"r"(live) : "memory");
+      ok = ok && !*(volatile int*)&s_failed;
+    }
+    auto sums = [&](int c, float (&f)[16]) {   // 16 columns of this row
+      uint32_t o[16];
+      tmem_ld_32x32b_x16(tmem_o + lanes + c, o);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(o[j]);
+      if (TWIN && n > 0) {
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(o2 + c + j);
+          f[j] += x.x; f[j + 1] += x.y; f[j + 2] += x.z; f[j + 3] += x.w;
+        }
+      }
+    };
+    const float inv = !ok ? __int_as_float(0x7fffffff) : l > 0.f ? 1.f / l : 0.f;   // NaN: a wait ran out
+    const bool mine = in && !low && tok < tq;
+    const size_t row = (size_t)(b * p.Q + tok0 + tok) * p.H + (kvh << p.g_shift) + (r & (G - 1));
+    if (SPLIT) {
+      if (n > 0 && in && !low) {
+        float* dst = p.part_o + (row * p.n_split + split) * HD;
+#pragma unroll 2
+        for (int c = 0; c < HD; c += 16) {
+          float f[16];
+          sums(c, f);
           if (mine) {
 #pragma unroll
-            for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(dst + c + j) = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
+            for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(dst + c + j) = make_float4(f[j] * inv, f[j + 1] * inv, f[j + 2] * inv, f[j + 3] * inv);
           }
         }
         if (mine) p.part_lse[row * p.n_split + split] = l > 0.f ? m + log2f(l) : -INFINITY;
       }
-    } else {
+    } else if (!low) {
       __nv_bfloat16* dst = p.out + row * HD;
 #pragma unroll 2
       for (int c = 0; c < HD; c += 16) {
-        uint32_t o[16];
-        tmem_ld_32x32b_x16(tmem_o + lanes + c, o);
-        tmem_ld_wait();
+        float f[16];
+        sums(c, f);
         uint32_t w[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) w[j] = n <= 0 ? 0u : pack_bf16x2(__uint_as_float(o[2 * j]) * inv, __uint_as_float(o[2 * j + 1]) * inv);
+        for (int j = 0; j < 8; ++j) w[j] = n <= 0 ? 0u : pack_bf16x2(f[2 * j] * inv, f[2 * j + 1] * inv);
         if (mine) {
           *reinterpret_cast<uint4*>(dst + c) = make_uint4(w[0], w[1], w[2], w[3]);
           *reinterpret_cast<uint4*>(dst + c + 8) = make_uint4(w[4], w[5], w[6], w[7]);

@@ -40,15 +40,19 @@ def test_against_float64(heads, kv_heads, hd, q_len, ctx):
 
 
 @pytest.mark.parametrize("heads,kv_heads,hd,q_len,ctx", [(64, 8, 128, 7, [1500, 64, 1, 700]), (32, 8, 64, 16, [300, 2, 900, 40]), (16, 1, 128, 3, [60, 130, 4000, 7, 1000, 2, 300, 64]),
-                                                         (32, 32, 128, 100, [50, 400])])
-def test_weights_keep_sixteen_bits(heads, kv_heads, hd, q_len, ctx):
+                                                         (32, 32, 128, 100, [50, 400]),
+                                                         (32, 8, 64, 16, [100, 2500, 30, 700, 64, 9, 1, 333]), (64, 8, 128, 8, [700, 128, 63, 4, 2000, 1, 40, 350]), (64, 8, 128, 7, [90, 500, 3, 1700, 57, 58, 2, 250]),
+                                                         (64, 8, 128, 4, [40, 300] * 8), (64, 8, 128, 3, [77] * 32)])
+@pytest.mark.parametrize("table", [2048, 8192])   # (long tables: the low pieces in rows of their own)
+def test_weights_keep_sixteen_bits(heads, kv_heads, hd, q_len, ctx, table):
     """The output is rounded to bf16 (eight significant bits: 2^-8 of it at most); weights are not (two pieces: 2^-17), and fp32 sums of scores and products move them
     by less than 2^-15: together 2^-14 of sum p |v|.  Weights of one bf16 piece are off by up to 2^-8 each, which short contexts show."""
     from ssd_b200 import ops
     G, B, bs = heads // kv_heads, len(ctx), 64
     g = torch.Generator(device="cuda").manual_seed(heads * 1000 + q_len)
-    pages = -(-(max(max(ctx) + q_len, 2048)) // bs)   # (the table's capacity takes the call to the tiles)
-    tables = torch.arange(B * pages, dtype=torch.int32, device="cuda").view(B, pages)
+    pages = -(-(max(ctx) + q_len) // bs)
+    tables = torch.full((B, max(pages, table // bs)), -1, dtype=torch.int32, device="cuda")   # (its capacity takes the call to the tiles)
+    tables[:, :pages] = torch.arange(B * pages, dtype=torch.int32, device="cuda").view(B, pages)
     q = torch.randn(B * q_len, heads, hd, generator=g, device="cuda").to(torch.bfloat16)
     kc, vc = (torch.randn(B * pages, bs, kv_heads, hd, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
     lens = torch.tensor([n + q_len for n in ctx], dtype=torch.int32, device="cuda")
