@@ -308,7 +308,7 @@ def run_ours(args):
         "parity_check": parity,
         "allreduce": ("none" if world == 1 else ("symm" if getattr(runner, "symm", False) else "nccl")),
         "draft_path": "kernel-per-op" if os.environ.get("SSDK_DRAFT_STREAM", "1") == "0"
-        else "draft_stream_kernel (one launch per step; kernel-per-op graph beyond 1024 tokens of context)",
+        else "draft_stream_kernel (one launch per step; kernel-per-op graph for long contexts)",
         "reference_gpu": ref_gpu,
     }
     if args.lm_scale:

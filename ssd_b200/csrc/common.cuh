@@ -49,6 +49,11 @@ SSDK_DEVINL uint4 pack_bf16x8(const float* f) {
   return v;
 }
 
+SSDK_DEVINL uint32_t pack_bf16x2(float lo, float hi) {
+  __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&v);
+}
+
 // ----------------------------------------------------------------------------------
 // warp / block reductions
 // ----------------------------------------------------------------------------------
@@ -401,6 +406,34 @@ SSDK_DEVINL uint4 ld_volatile_v4(const void* p) {
   return r;
 }
 
+// D[16, 8] += A[16, 16] B[16, 8]
+SSDK_DEVINL void mma_bf16_16816(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// registers of a warpgroup's threads (all of its warps; the shares of a block add up to what it was launched with at most)
+template <int N>
+SSDK_DEVINL void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+SSDK_DEVINL void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+// flag-in-word exchange between the CTAs of one launch: payload and tag travel in one word, so that neither side needs a fence
+SSDK_DEVINL void st_relaxed_gpu_u64(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+SSDK_DEVINL uint4 ld_relaxed_gpu_v4(const void* p) {   // four words, each whole
+  uint4 r;
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+  return r;
+}
+SSDK_DEVINL uint32_t ld_relaxed_gpu_u32(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 #else  // SSDK_HOST_EMU: host stand-ins for the few PTX helpers the emulated kernels use
 enum { TR_PREP = 1, TR_NORM, TR_GEMM, TR_ROPE, TR_ATTN, TR_SAMPLE, TR_VERIFY, TR_MISC };
 enum { TRF_ATTN = 16, TRF_NORM = 24, TRF_ROPE = 32, TRF_COMB = 40, TRF_GEMM = 48 };
@@ -486,6 +519,71 @@ SSDK_DEVINL uint4 ld_volatile_v4(const void* p) {
   const uint64_t a = __atomic_load_n(q, __ATOMIC_ACQUIRE), b = __atomic_load_n(q + 1, __ATOMIC_ACQUIRE);
   std::this_thread::yield();
   return make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
+}
+template <int N>
+SSDK_DEVINL void reg_inc() {}
+template <int N>
+SSDK_DEVINL void reg_dec() {}
+SSDK_DEVINL void st_relaxed_gpu_u64(unsigned long long* p, unsigned long long v) { __atomic_store_n(p, v, __ATOMIC_RELAXED); }
+SSDK_DEVINL uint32_t ld_relaxed_gpu_u32(const uint32_t* p) {
+  std::this_thread::sleep_for(std::chrono::microseconds(20));   // (pollers that only yield keep the threads they wait for off the cores)
+  return __atomic_load_n(p, __ATOMIC_RELAXED);
+}
+SSDK_DEVINL uint4 ld_relaxed_gpu_v4(const void* p) {
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(p);
+  uint4 r;
+  r.x = __atomic_load_n(q, __ATOMIC_RELAXED); r.y = __atomic_load_n(q + 1, __ATOMIC_RELAXED);
+  r.z = __atomic_load_n(q + 2, __ATOMIC_RELAXED); r.w = __atomic_load_n(q + 3, __ATOMIC_RELAXED);
+  std::this_thread::sleep_for(std::chrono::microseconds(20));
+  return r;
+}
+// every lane's word of a warp
+inline void emu_gather(uint32_t v, uint32_t* all) {
+  emu::Warp& w = *emu::tctx.cta->warps[threadIdx.x >> 5];
+  w.slot[threadIdx.x & 31] = v;
+  w.bar.arrive_and_wait();
+  std::memcpy(all, w.slot, sizeof(w.slot));
+  w.bar.arrive_and_wait();
+}
+SSDK_DEVINL float __shfl_sync(unsigned, float v, int src) {
+  uint32_t u, all[32];
+  std::memcpy(&u, &v, 4);
+  emu_gather(u, all);
+  std::memcpy(&v, &all[src], 4);
+  return v;
+}
+SSDK_DEVINL uint32_t __byte_perm(uint32_t a, uint32_t b, uint32_t sel) {
+  const uint64_t v = ((uint64_t)b << 32) | a;
+  uint32_t r = 0;
+  for (int i = 0; i < 4; ++i) r |= (uint32_t)((v >> (8 * ((sel >> (4 * i)) & 7))) & 0xffu) << (8 * i);
+  return r;
+}
+SSDK_DEVINL void mma_bf16_16816(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  struct Words { uint32_t w[32][6]; };
+  static std::mutex mu;
+  static std::map<emu::Warp*, std::unique_ptr<Words>> all;
+  emu::Warp* warp = emu::tctx.cta->warps[threadIdx.x >> 5].get();
+  Words* x;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    auto& slot = all[warp];
+    if (!slot) slot = std::make_unique<Words>();
+    x = slot.get();
+  }
+  uint32_t* mine = x->w[threadIdx.x & 31];
+  for (int i = 0; i < 4; ++i) mine[i] = a[i];
+  mine[4] = b0; mine[5] = b1;
+  warp->bar.arrive_and_wait();
+  auto val = [](uint32_t w, int half) { return __bfloat162float(__nv_bfloat16{(uint16_t)(half ? w >> 16 : w & 0xffffu)}); };
+  const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+  for (int e = 0; e < 4; ++e) {
+    const int row = g, hi = e >> 1, col = 2 * t + (e & 1);   // rows behind the eighth: A's odd words
+    for (int k = 0; k < 16; ++k) {
+      const int lane_k = (k & 7) >> 1, part = k >> 3;
+      c[e] += val(x->w[row * 4 + lane_k][2 * part + hi], k & 1) * val(x->w[col * 4 + lane_k][4 + part], k & 1);
+    }
+  }
+  warp->bar.arrive_and_wait();
 }
 #endif
 

@@ -442,9 +442,8 @@ struct Workspace {
   RecPart* ver_rec;
   unsigned* ver_counters;
   size_t partial_floats = 0;
-  // streaming draft kernel (draft_stream.cuh): inter-phase vectors, split-KV partials, device-wide barrier state
-  bf16* ds_vec;
-  float* ds_attn;
+  // streaming draft kernel (draft_stream.cuh): exchange words, device-wide barrier state
+  uint32_t* ds_words;
   unsigned* ds_sync;
 };
 
@@ -506,6 +505,32 @@ static void derive(Model& m) {
   m.ffn = c.ffn / c.tp_size;
   m.qkv_dim = (m.H + 2 * m.KV) * m.hd;
   m.vocab_local = c.vocab / c.tp_size;
+}
+
+// ---- streaming draft kernel: which models and batches it serves, and with what shared memory ----
+constexpr int kMaxDynSmem = 227 * 1024 - (int)sizeof(DsShared) - 256;  // opt-in limit per CTA minus the kernel's static shared memory
+static int ds_tokens(int B) { return B == 1 ? 1 : (B <= 4 ? 4 : 8); }   // the kernel's instances
+// slots of up to 2048 columns; narrow models: 1024 (twice as many slots in the same room, and no half-empty ones)
+static int ds_max_chunk(const Model& m) { return m.d <= 1024 ? 1024 : kDsMaxChunk; }
+static size_t ds_fixed_smem(const Model& m, int B) {
+  const int MT = ds_tokens(B);
+  size_t scratch = std::max((size_t)B * (2 * m.d + kDsPad), ds_attn_bytes(m.H / m.KV, m.hd));
+  for (int K : {m.H * m.hd, m.ffn})
+    if (ds_staged(MT, B, K)) scratch = std::max(scratch, ds_stage_bytes(B, K));
+  return ds_part_bytes(MT) + (size_t)B * m.d * 2 + scratch + 64;
+}
+static int ds_ring_slots(const Model& m, int B) {
+  const size_t fixed = ds_fixed_smem(m, B);
+  const int slot = ds_slot_bytes(ds_max_chunk(m));
+  return fixed > (size_t)kMaxDynSmem ? 0 : (int)std::min<size_t>(kDsMaxSlots, ((size_t)kMaxDynSmem - fixed) / slot);
+}
+static bool draft_stream_supported(const Model& m, int B) {
+  const int G = m.KV ? m.H / m.KV : 0, mc = ds_max_chunk(m);
+  DsGeom g;
+  // (a row of every matrix on every CTA is what makes the exchange without barriers sound, see draft_stream.cuh)
+  return B >= 1 && B <= kDsMaxBatch && m.cfg.tp_size == 1 && m.cfg.layers <= kDsMaxLayers && (m.hd == 64 || m.hd == 128) && G >= 1 && G <= 8 &&
+         m.H % m.KV == 0 && m.KV <= 32 && m.d <= 8 * kDsConsumers && m.d >= num_sms() && m.ffn >= num_sms() && m.cfg.vocab >= num_sms() &&
+         ds_geometry(m.d, m.qkv_dim, mc, &g) && ds_geometry(m.H * m.hd, m.d, mc, &g) && ds_geometry(m.ffn, m.d, mc, &g) && ds_ring_slots(m, B) >= 4;
 }
 
 // workspace carve-up (pass base = nullptr to measure)
@@ -581,8 +606,13 @@ static int64_t carve(ssdk_engine* e, uint8_t* base) {
   w.ver_rows = (RowPart*)take((size_t)kVerifyMaxRows * kVerifyCtas * sizeof(RowPart));
   w.ver_rec = (RecPart*)take((size_t)kVerifyMaxBatch * kVerifyCtas * sizeof(RecPart));
   w.ver_counters = (unsigned*)take(64);
-  w.ds_vec = (bf16*)take((size_t)(qmax + 4 * dmax + fmax + Hmax * hdmax + 64) * 2);
-  w.ds_attn = (float*)take((size_t)Hmax * kDsSplits * (hdmax + 2) * 4);
+  long long words = 0;
+  if (e->model[SSDK_DRAFT].present) {
+    const Model& m = e->model[SSDK_DRAFT];
+    for (int b = 1; b <= std::min(MB, kDsMaxBatch); ++b)
+      if (draft_stream_supported(m, b)) words = std::max(words, ds_words(b, m.d, m.H, m.KV, m.hd, m.ffn, num_sms()));
+  }
+  w.ds_words = (uint32_t*)take((size_t)words * 4);
   w.ds_sync = (unsigned*)take(256);
   return (int64_t)align_up(off, 1024);
 }
@@ -1153,68 +1183,44 @@ static bool draft_stream_enabled() {
   if (v < 0) v = env_int("SSDK_DRAFT_STREAM", 1) != 0 ? 1 : 0;
   return v == 1;
 }
-constexpr int kMaxDynSmem = 227 * 1024 - 2048;  // opt-in limit per CTA minus the kernel's static shared memory (1.8 KB)
-static size_t ds_fixed_smem(const Model& m) {
-  const int G = m.H / m.KV, gmax = G <= 4 ? 4 : 8;
-  const size_t xs = (size_t)std::max(std::max(m.d, m.ffn), m.H * m.hd);
-  const size_t scratch = (size_t)gmax * m.hd + 2 * m.hd + (size_t)kDsWarps * gmax * (m.hd + 2);
-  return (xs + scratch) * 4 + 256;
-}
-static int ds_ring_slots(const Model& m) {
-  const size_t fixed = ds_fixed_smem(m);
-  if (fixed + 3 * (size_t)kDsSlotBytes > (size_t)kMaxDynSmem) return 0;
-  return (int)std::min<size_t>(kDsMaxSlots, ((size_t)kMaxDynSmem - fixed) / kDsSlotBytes);
-}
-static bool draft_stream_supported(const Model& m, int B) {
-  const int G = m.KV ? m.H / m.KV : 0;
-  DsGeom g;
-  return B == 1 && m.cfg.tp_size == 1 && m.cfg.layers <= kDsMaxLayers && (m.hd == 64 || m.hd == 128) && G >= 1 && G <= 8 &&
-         m.H % m.KV == 0 && m.KV <= 32 && m.d % 8 == 0 && (m.H * m.hd) % 8 == 0 && m.ffn % 8 == 0 &&
-         ds_geometry(m.d, m.qkv_dim, false, &g) && ds_geometry(m.H * m.hd, m.d, false, &g) &&
-         ds_geometry(m.d, m.ffn, true, &g) && ds_geometry(m.ffn, m.d, false, &g) && ds_geometry(m.d, m.cfg.vocab, false, &g) &&
-         ds_ring_slots(m) >= 3;
-}
-// Which draft path a step takes.  The streaming kernel wins while the attention phase of a KV split is ONE round of loads
-// (16 splits x 8 warps x 8 tokens = 1024 tokens); every further round costs more than the kernel-per-op draft's tensor-core
-// attention (measured at ~3k tokens: +2.4 ms per step), so longer contexts take the
-// kernel-per-op graph.  Both graphs compute the same step; ctx_bound = the longest context of the batch before the step.
-static int draft_stream_max_ctx() {
-  static int v = -1;
-  if (v < 0) v = std::max(0, env_int("SSDK_DRAFT_STREAM_MAX_CTX", 1024));
-  return v;
-}
+// Which draft path a step takes (both compute the same step; ctx_bound = the longest context of the batch before it).  Steps of k = 4 with two target layers, us, kernels per op -> streaming kernel:
+//   1B draft (16 layers, d = 2048): 1 sequence of 200, 900, 2000, 8000 tokens 4364 -> 3194, 4436 -> 3355, 4565 -> 3478, 4827 -> 4054; 2 of 200, 2000 4463 -> 3841, 4718 -> 4445;
+//     4 of 200, 2000 4699 -> 3804, 5005 -> 4395; 5 of 900, 2000 4872 -> 4657, 4938 -> 4901; 8 of 200, 900, 2000 4851 -> 4547, 4969 -> 4919, 5221 -> 5412
+//   0.6B draft (28 layers, d = 1024, heads of 128): 1 of 60, 200, 500, 900 4439 -> 4213, 4484 -> 4376, 4512 -> 4738, 4723 -> 4771; 2, 4, 8 of 200 4652 -> 5777, 4719 -> 5850, 5047 -> 7595
+// Wide models stream their weights for most of a layer, so that what the kernel saves between stages counts; its attention, a few CTAs per sequence, costs more per key, which
+// bounds the keys of a call.  Narrow ones are all exchange, and from two sequences on every CTA reads more words than the weights it multiplies.
+// SSDK_DRAFT_STREAM_MAX_CTX replaces the rule by a bound on the context alone.
 static bool use_draft_stream(ssdk_engine* e, int B, int ctx_bound) {
-  const Model& drf = e->model[SSDK_DRAFT];
-  return drf.present && draft_stream_enabled() && draft_stream_supported(drf, B) &&
-         ctx_bound + e->rt.spec_k + 1 <= draft_stream_max_ctx();
+  const Model& m = e->model[SSDK_DRAFT];
+  if (!m.present || !draft_stream_enabled() || !draft_stream_supported(m, B)) return false;
+  const int keys = ctx_bound + e->rt.spec_k + 1;
+  static const int forced = env_int("SSDK_DRAFT_STREAM_MAX_CTX", -1);
+  if (forced >= 0) return keys <= forced;
+  if (m.d > 1024) return (int64_t)B * keys <= 8192;
+  return B == 1 && keys <= (m.hd == 128 ? 256 : 1024);
 }
-template <int HD, int GMAX>
+template <int HD, int MT>
 static int launch_draft_stream(Launcher& L, const DsParams& p, size_t smem) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    CK(cudaFuncSetAttribute(draft_stream_kernel<HD, GMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_set = true;
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(num_sms());
   cfg.blockDim = dim3(kDsThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = L.st;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;  // all CTAs must be co-resident: the phases meet at device-wide barriers
+  attr[0].id = cudaLaunchAttributeCooperative;  // all CTAs must be co-resident: they wait for one another
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;  // (a plain launch measured the same step time: 5.70 vs 5.66 ms — the attribute costs nothing between steps)
-  cudaError_t err = cudaLaunchKernelEx(&cfg, draft_stream_kernel<HD, GMAX>, p);
+  cudaError_t err = cudaLaunchKernelEx(&cfg, draft_stream_kernel<HD, MT>, p);
   if (err != cudaSuccess) return fail("draft stream launch failed: %s", cudaGetErrorString(err));
   L.barrier_op();  // not a PDL primary: the next kernel starts after this grid has drained
   ++L.count;
   return 0;
 }
 // forwards 0 .. n_fwd-1 of the draft on tok_buf[0 ..]; samples tok_buf[f + 1] after every forward but (optionally) the last
-static int enqueue_draft_stream(ssdk_engine* e, Launcher& L, int64_t* tok_buf, int n_fwd, bool skip_last_head,
+static int enqueue_draft_stream(ssdk_engine* e, Launcher& L, int B, int64_t* tok_buf, int tok_ld, int n_fwd, bool skip_last_head,
                                 const int32_t* ctx0, const int32_t* block_table, const float* temp, const uint64_t* dyn,
-                                bf16* logits, int64_t logits_ld) {
+                                bf16* logits, int64_t logits_ld, int64_t logits_seq_ld) {
   Model& m = e->model[SSDK_DRAFT];
   Workspace& w = e->ws;
   DsParams p;
@@ -1228,31 +1234,23 @@ static int enqueue_draft_stream(ssdk_engine* e, Launcher& L, int64_t* tok_buf, i
   p.block_size = e->rt.block_size; p.max_blocks = e->rt.max_blocks_per_seq;
   p.tok_buf = tok_buf; p.n_fwd = n_fwd; p.skip_last_head = skip_last_head ? 1 : 0;
   p.ctx0 = ctx0; p.block_table = block_table;
-  bf16* v = w.ds_vec;
-  p.vec_qkv = v; v += align_up((size_t)m.qkv_dim, 8);
-  p.vec_attn = v; v += (size_t)m.H * m.hd;
-  p.vec_o = v; v += m.d;
-  p.vec_down = v; v += m.d;
-  p.resid0 = v; v += m.d;
-  p.resid1 = v; v += m.d;
-  p.vec_act = v;
-  p.attn_part = w.ds_attn;
+  p.batch = B; p.tok_ld = tok_ld; p.logits_seq_ld = logits_seq_ld;
   p.logits = logits; p.logits_ld = logits_ld;
   p.temp = temp; p.dyn = dyn;
   p.samp_partial = w.samp_partial;
   p.bar_state = w.ds_sync;
-  p.attn_ticket = w.ds_sync + 8;
-  p.n_slots = ds_ring_slots(m);
+  p.words = w.ds_words;
+  p.timeout = L.gave_up;
+  p.max_chunk = ds_max_chunk(m);
+  p.slot_bytes = ds_slot_bytes(p.max_chunk);
+  p.n_slots = ds_ring_slots(m, B);
   for (int l = 0; l < p.L; ++l) {
     const LayerW& lw = m.layers[l];
     p.layers[l] = DsLayer{lw.qkv.ptr, lw.o.ptr, lw.gate_up.ptr, lw.down.ptr, lw.input_norm, lw.post_norm, lw.q_norm, lw.k_norm};
   }
-  const int G = m.H / m.KV, gmax = G <= 4 ? 4 : 8;
-  const size_t smem = ds_fixed_smem(m) + (size_t)p.n_slots * kDsSlotBytes;
-  if (m.hd == 64 && gmax == 4) return launch_draft_stream<64, 4>(L, p, smem);
-  if (m.hd == 64 && gmax == 8) return launch_draft_stream<64, 8>(L, p, smem);
-  if (m.hd == 128 && gmax == 4) return launch_draft_stream<128, 4>(L, p, smem);
-  return launch_draft_stream<128, 8>(L, p, smem);
+  const size_t smem = ds_fixed_smem(m, B) + (size_t)p.n_slots * p.slot_bytes;
+  if (m.hd == 64) return B == 1 ? launch_draft_stream<64, 1>(L, p, smem) : (B <= 4 ? launch_draft_stream<64, 4>(L, p, smem) : launch_draft_stream<64, 8>(L, p, smem));
+  return B == 1 ? launch_draft_stream<128, 1>(L, p, smem) : (B <= 4 ? launch_draft_stream<128, 4>(L, p, smem) : launch_draft_stream<128, 8>(L, p, smem));
 }
 
 static int enqueue_spec_step(ssdk_engine* e, Launcher& L, int B, bool host_io, bool advance, bool stream_draft) {
@@ -1278,7 +1276,7 @@ static int enqueue_spec_step(ssdk_engine* e, Launcher& L, int B, bool host_io, b
   if (tp_rank == 0 && !drf.present) return fail("rank 0 needs the draft model");
   if (drf.present) CKI(L.go(init_tokens_kernel, dim3(1), dim3(64), 0, (const int64_t*)rec_in, w.tok_buf, B, K + 1));
   if (stream_draft)
-    CKI(enqueue_draft_stream(e, L, w.tok_buf, K + 1, true, ctx, btd, tq, seed_step, w.logits_q, (int64_t)V));
+    CKI(enqueue_draft_stream(e, L, B, w.tok_buf, K + 1, K + 1, true, ctx, btd, tq, seed_step, w.logits_q, (int64_t)V, (int64_t)K * V));
   for (int k = 0; k <= K && drf.present && !stream_draft; ++k) {
     Fwd f;
     f.which = SSDK_DRAFT; f.B = B; f.Q = 1; f.ids = w.tok_buf + k; f.ids_stride = K + 1;
@@ -1397,6 +1395,15 @@ static int init_kernel_attrs() {
   SSDK_ATTR_P(64, false, kPromptOne) SSDK_ATTR_P(64, false, kPromptTwo) SSDK_ATTR_P(64, true, kPromptTwo) SSDK_ATTR_P(64, false, kPromptTwin) SSDK_ATTR_P(64, true, kPromptTwin)
   SSDK_ATTR_P(128, false, kPromptOne) SSDK_ATTR_P(128, false, kPromptTwo) SSDK_ATTR_P(128, true, kPromptTwo) SSDK_ATTR_P(128, false, kPromptTwin) SSDK_ATTR_P(128, true, kPromptTwin)
 #undef SSDK_ATTR_P
+#define SSDK_ATTR_D(HD, MT) \
+  CK(cudaFuncSetAttribute(draft_stream_kernel<HD, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem)); \
+  { /* (a register split above what the block is launched with would wait for ever) */ \
+    cudaFuncAttributes a; \
+    CK(cudaFuncGetAttributes(&a, draft_stream_kernel<HD, MT>)); \
+    if (a.numRegs != kDsRegsLaunch) return fail("draft_stream_kernel: built with %d registers", a.numRegs); \
+  }
+  SSDK_ATTR_D(64, 1) SSDK_ATTR_D(64, 4) SSDK_ATTR_D(64, 8) SSDK_ATTR_D(128, 1) SSDK_ATTR_D(128, 4) SSDK_ATTR_D(128, 8)
+#undef SSDK_ATTR_D
   CK(cudaFuncSetAttribute(add_rmsnorm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
   if (dev < 64) done[dev].store(true, std::memory_order_release);
   return 0;

@@ -1,0 +1,102 @@
+"""csrc/draft_stream.cuh on host threads with the exchange of the product (tagged words that their readers poll; tests/test_draft_stream_emu_cpu.py runs the
+same source with barriers in their place), for one sequence and for batches of uneven contexts: logits of every forward, keys and values, tokens (greedy and Philox)
+against the oracle, two launches over the same words.  What it cannot show is the device's memory model and speed."""
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+import torch
+
+from oracle.model import ModelCfg, OracleModel, random_weights
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SRC = os.path.join(ROOT, "tests", "emu", "run_draft_words.cpp")
+BIN = os.path.join(ROOT, "tests", "emu", "_build", "run_draft_words")
+
+pytestmark = pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++ (C++20)")
+
+
+def _build():
+    deps = [SRC, os.path.join(ROOT, "tests", "emu", "cuda_emu.h")] + [os.path.join(ROOT, "ssd_b200", "csrc", n) for n in ("draft_stream.cuh", "common.cuh", "sampling.cuh")]
+    if os.path.exists(BIN) and all(os.path.getmtime(BIN) >= os.path.getmtime(d) for d in deps):
+        return
+    os.makedirs(os.path.dirname(BIN), exist_ok=True)
+    subprocess.run(["g++", "-std=c++20", "-O1", "-pthread", "-Wno-unknown-pragmas", "-Wno-attributes", "-o", BIN, SRC], check=True)
+
+
+def _u16(t):
+    return t.contiguous().view(torch.int16).numpy().astype(np.uint16)
+
+
+@pytest.mark.parametrize("hd,kv,grid,ffn,ctx,temp,chunk", [
+    (64, 2, 3, 512, [21], 0.0, 1024),                # one sequence, a range per key head
+    (64, 1, 2, 512, [300], 0.7, 256),                # two ranges: exchange of partial results; two slots per tile
+    (128, 1, 3, 768, [270, 5, 33], 0.0, 256),        # three sequences on the instance of four, three slots per tile
+    (64, 2, 2, 512, [9, 255, 256, 1, 30], 0.8, 512), # five: fragments straight from the words; more units than CTAs, contexts around a round of keys
+    (64, 1, 2, 4608, [40, 3, 7], 0.0, 2048),         # an intermediate row too long for the shared memory of four tokens' instance
+])
+def test_tagged_exchange_matches_the_oracle(tmp_path, hd, kv, grid, ffn, ctx, temp, chunk):
+    from oracle import verify as V
+    _build()
+    torch.manual_seed(3)
+    B, n_fwd, bs = len(ctx), 2, 16
+    cfg = ModelCfg(hidden=256, layers=1 if ffn > 4096 else 2, heads=256 // hd, kv_heads=kv, head_dim=hd, ffn=ffn, vocab=264, max_pos=512, rms_eps=1e-6, rope_theta=500000.0, qk_norm=hd == 128)
+    w = random_weights(cfg, seed=9)
+    per = (max(ctx) + n_fwd) // bs + 1
+    nblk = B * per
+    order = torch.randperm(nblk).tolist()
+    tables = [order[b * per:(b + 1) * per] for b in range(B)]
+    model = OracleModel(cfg, w, num_blocks=nblk, block_size=bs)
+    for b, n in enumerate(ctx):
+        slots = torch.tensor([tables[b][p // bs] * bs + p % bs for p in range(n)], dtype=torch.int32)
+        model.forward(torch.randint(0, cfg.vocab, (n,)), torch.arange(n), slots, torch.tensor([n], dtype=torch.int32), torch.tensor([tables[b]], dtype=torch.int32), n)
+    kv0 = model.kv_cache.clone()
+    seed, call_base = 1234, 7 * 16
+    temps = [temp if b != 1 else 0.0 for b in range(B)]
+    blob, out = tmp_path / "in.bin", tmp_path / "out.bin"
+    with open(blob, "wb") as f:
+        np.array([B, cfg.hidden, cfg.layers, cfg.heads, cfg.kv_heads, hd, cfg.ffn, cfg.vocab, int(cfg.qk_norm), bs, per, nblk * bs, n_fwd, grid, cfg.max_pos, 4, chunk], dtype=np.int32).tofile(f)
+        np.array([cfg.rms_eps] + temps, dtype=np.float32).tofile(f)
+        np.array([seed, call_base], dtype=np.uint64).tofile(f)
+        np.array([77 + b for b in range(B)], dtype=np.int64).tofile(f)
+        np.array(ctx, dtype=np.int32).tofile(f)
+        np.array(tables, dtype=np.int32).tofile(f)
+        for t in (w["embed"], w["final_norm"], w["lm_head"]):
+            _u16(t).tofile(f)
+        model.rope.numpy().astype(np.float32).tofile(f)
+        ones = torch.ones(hd, dtype=torch.bfloat16)
+        for lw in w["layers"]:
+            for k in ("qkv", "o", "gate_up", "down", "input_norm", "post_norm"):
+                _u16(lw[k]).tofile(f)
+            _u16(lw.get("q_norm", ones)).tofile(f)
+            _u16(lw.get("k_norm", ones)).tofile(f)
+        _u16(kv0[0]).tofile(f)
+        _u16(kv0[1]).tofile(f)
+    res = subprocess.run([BIN, str(blob), str(out)], capture_output=True, text=True, timeout=600)
+    assert res.returncode == 0, res.stderr[-2000:]
+    raw = np.fromfile(out, dtype=np.uint16)
+    nl, nc = B * n_fwd * cfg.vocab, cfg.layers * nblk * bs * kv * hd
+    bf = torch.from_numpy(raw[:nl + 2 * nc].astype(np.int16)).view(torch.bfloat16)
+    logits, kc, vc = bf[:nl].reshape(B, n_fwd, cfg.vocab), bf[nl:nl + nc].float(), bf[nl + nc:].float()
+    toks = np.frombuffer(raw[nl + 2 * nc:].tobytes(), dtype=np.int64).reshape(B, n_fwd + 1)
+    for b, n in enumerate(ctx):
+        bt = torch.tensor([tables[b]], dtype=torch.int32)
+        for step in range(n_fwd):
+            p = n + step
+            slot = torch.tensor([tables[b][p // bs] * bs + p % bs], dtype=torch.int32)
+            h = model.forward(torch.tensor([int(toks[b, step])]), torch.tensor([p]), slot, torch.tensor([p + 1], dtype=torch.int32), bt, 1)
+            if step == n_fwd - 1:
+                assert toks[b, step + 1] == -1   # the last forward has no head
+                break
+            want, got = model.compute_logits(h)[0].float(), logits[b, step].float()
+            # bf16 roundings of the hidden state (2^-9 each, about sixteen of them on the way) on logits of unit scale
+            assert (got - want).abs().max() <= 0.02 * want.abs().max() + 0.02, (b, step)
+            # the token is what the sampler's rule makes of the kernel's own logits
+            row = logits[:, step] if temps[b] else logits[b, step][None]
+            mine = V.sample(row, torch.tensor(temps if temps[b] else [0.0]), seed, call_base + step)
+            assert toks[b, step + 1] == int(mine[b if temps[b] else 0]), (b, step)
+    ref = model.kv_cache.float()
+    for got, want in ((kc, ref[0].reshape(-1)), (vc, ref[1].reshape(-1))):
+        assert (got - want).abs().max() <= 0.02 * want.abs().max() + 1e-3
