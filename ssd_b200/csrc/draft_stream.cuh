@@ -485,7 +485,7 @@ SSDK_DEVINL void ds_consume(DsRing& ring, const DsGeom& g, int mode, int M, floa
 // xs[m] = bf16r( r * rsqrt(mean r^2 + eps) * w ),  r = a (+ resid) in fp32;  resid = bf16(r), which every CTA keeps for itself (thread t only touches elements 8 t .. 8 t + 8).
 // a: a stage's results, or (src == nullptr) rows of the embedding, which are their own residual.
 template <int MT>
-SSDK_DEVINL void ds_norm(const DsVec* src, const __nv_bfloat16* embed, const int* tok, uint8_t* resid, const __nv_bfloat16* w, float eps, int d, int M, uint32_t tag,
+SSDK_DEVINL void ds_norm(const DsVec* src, const __nv_bfloat16* embed, int vocab, const int* tok, uint8_t* resid, const __nv_bfloat16* w, float eps, int d, int M, uint32_t tag,
                          const DsWait& wait, uint8_t* xs, float* red) {
   const int tid = ds_tid(), i0 = tid * 8, warp = tid >> 5, lane = tid & 31;
   const bool on = i0 < d;
@@ -518,7 +518,7 @@ SSDK_DEVINL void ds_norm(const DsVec* src, const __nv_bfloat16* embed, const int
   } else {
 #pragma unroll
     for (int m = 0; m < MT; ++m)
-      if (m < M && on) unpack_bf16x8(*reinterpret_cast<const uint4*>(embed + (size_t)tok[m] * d + i0), x[m]);
+      if (m < M && on && (unsigned)tok[m] < (unsigned)vocab) unpack_bf16x8(*reinterpret_cast<const uint4*>(embed + (size_t)tok[m] * d + i0), x[m]);
   }
 #pragma unroll
   for (int m = 0; m < MT; ++m) {
@@ -981,7 +981,7 @@ SSDK_DEVINL unsigned ds_stage(int kind, int l, int f, uint32_t tag, unsigned st)
   } else {
     const __nv_bfloat16* w = kind == DS_QKV ? S.p.layers[l].in_norm : (kind == DS_GU ? S.p.layers[l].post_norm : S.p.final_norm);
     const bool embed = kind == DS_QKV && l == 0;   // first layer: hidden = norm(embed), residual = embed (models/llama3.py:192-193)
-    ds_norm<MT>(embed ? nullptr : &src, S.p.embed, S.tok, S.resid, w, S.p.eps, S.p.d, M, kind == DS_QKV ? tag - 1u : tag, wait, S.scratch, S.red);
+    ds_norm<MT>(embed ? nullptr : &src, S.p.embed, S.p.vocab, S.tok, S.resid, w, S.p.eps, S.p.d, M, kind == DS_QKV ? tag - 1u : tag, wait, S.scratch, S.red);
     xrow = S.scratch + (tid >> 5) * (g.ck >> 2);   // (one chunk)
     pitch = 2 * g.K + kDsPad;
   }
@@ -1059,7 +1059,10 @@ __global__ void __launch_bounds__(kDsThreads, 1) draft_stream_kernel(const __gri
   const bool staged = p.max_blocks <= kDsBtSmem;
   if (staged)
     for (int i = threadIdx.x; i < M * p.max_blocks; i += kDsThreads) S.bt[i / p.max_blocks * kDsBtSmem + i % p.max_blocks] = p.block_table[i];
-  if ((int)threadIdx.x < M) S.tok[threadIdx.x] = (int)p.tok_buf[(size_t)threadIdx.x * p.tok_ld];
+  if ((int)threadIdx.x < M) {
+    const int64_t t = p.tok_buf[(size_t)threadIdx.x * p.tok_ld];
+    S.tok[threadIdx.x] = t >= 0 && t < p.vocab ? (int)t : -1;   // (ids outside the vocabulary: zero rows)
+  }
   if (threadIdx.x == 0) {
     trace_mark(TR_MISC);
     ds_geometry(p.d, (p.H + 2 * p.KV) * HD, max_chunk, &S.geom[DS_QKV]);

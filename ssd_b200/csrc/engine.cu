@@ -607,8 +607,9 @@ static int64_t carve(ssdk_engine* e, uint8_t* base) {
   w.ver_rec = (RecPart*)take((size_t)kVerifyMaxBatch * kVerifyCtas * sizeof(RecPart));
   w.ver_counters = (unsigned*)take(64);
   long long words = 0;
-  if (e->model[SSDK_DRAFT].present) {
-    const Model& m = e->model[SSDK_DRAFT];
+  for (int i = 0; i < 2; ++i) {
+    const Model& m = e->model[i];
+    if (!m.present) continue;
     for (int b = 1; b <= std::min(MB, kDsMaxBatch); ++b)
       if (draft_stream_supported(m, b)) words = std::max(words, ds_words(b, m.d, m.H, m.KV, m.hd, m.ffn, num_sms()));
   }
@@ -1199,6 +1200,12 @@ static bool use_draft_stream(ssdk_engine* e, int B, int ctx_bound) {
   if (m.d > 1024) return (int64_t)B * keys <= 8192;
   return B == 1 && keys <= (m.hd == 128 ? 256 : 1024);
 }
+// One token per sequence of plain decoding, for the wide models of the rule above: a forward is one launch instead of eight per layer, and no graph.  1B model, 16 layers, us a call with its token:
+//   1 sequence of 200, 2000, 7000 tokens 898 -> 665, 938 -> 731, 990 -> 838; 2 of 200, 4000 924 -> 798, 998 -> 983; 4 of 200, 2000 959 -> 772, 1023 -> 912; 8 of 200, 1000 986 -> 919, 1042 -> 1027;
+//   two layers of it: 1, 4, 8 of 200 279 -> 255, 268 -> 257, 280 -> 282
+static bool stream_decode(ssdk_engine* e, const Model& m, int B, int q_len, const int32_t* ctx_len) {
+  return q_len == 1 && m.d > 1024 && draft_stream_enabled() && draft_stream_supported(m, B) && (int64_t)B * (*std::max_element(ctx_len, ctx_len + B) + 1) <= 8192;
+}
 template <int HD, int MT>
 static int launch_draft_stream(Launcher& L, const DsParams& p, size_t smem) {
   cudaLaunchConfig_t cfg = {};
@@ -1217,11 +1224,11 @@ static int launch_draft_stream(Launcher& L, const DsParams& p, size_t smem) {
   ++L.count;
   return 0;
 }
-// forwards 0 .. n_fwd-1 of the draft on tok_buf[0 ..]; samples tok_buf[f + 1] after every forward but (optionally) the last
-static int enqueue_draft_stream(ssdk_engine* e, Launcher& L, int B, int64_t* tok_buf, int tok_ld, int n_fwd, bool skip_last_head,
+// forwards 0 .. n_fwd-1 of a model on tok_buf[0 ..] of every sequence; samples tok_buf[f + 1] after every forward but (optionally) the last
+static int enqueue_draft_stream(ssdk_engine* e, Launcher& L, int which, int B, int64_t* tok_buf, int tok_ld, int n_fwd, bool skip_last_head,
                                 const int32_t* ctx0, const int32_t* block_table, const float* temp, const uint64_t* dyn,
                                 bf16* logits, int64_t logits_ld, int64_t logits_seq_ld) {
-  Model& m = e->model[SSDK_DRAFT];
+  Model& m = e->model[which];
   Workspace& w = e->ws;
   DsParams p;
   memset(&p, 0, sizeof(p));
@@ -1276,7 +1283,7 @@ static int enqueue_spec_step(ssdk_engine* e, Launcher& L, int B, bool host_io, b
   if (tp_rank == 0 && !drf.present) return fail("rank 0 needs the draft model");
   if (drf.present) CKI(L.go(init_tokens_kernel, dim3(1), dim3(64), 0, (const int64_t*)rec_in, w.tok_buf, B, K + 1));
   if (stream_draft)
-    CKI(enqueue_draft_stream(e, L, B, w.tok_buf, K + 1, K + 1, true, ctx, btd, tq, seed_step, w.logits_q, (int64_t)V, (int64_t)K * V));
+    CKI(enqueue_draft_stream(e, L, SSDK_DRAFT, B, w.tok_buf, K + 1, K + 1, true, ctx, btd, tq, seed_step, w.logits_q, (int64_t)V, (int64_t)K * V));
   for (int k = 0; k <= K && drf.present && !stream_draft; ++k) {
     Fwd f;
     f.which = SSDK_DRAFT; f.B = B; f.Q = 1; f.ids = w.tok_buf + k; f.ids_stride = K + 1;
@@ -1797,7 +1804,10 @@ static int forward_rows(ssdk_handle h, int which, int batch, int q_len, const in
   f.logits_mode = want_sample ? 2 : 0;
   f.logits_out = w.logits_last;
   f.logits_ld = m.cfg.vocab;
-  CKI(enqueue_forward(h, L, f));
+  if (stream_decode(h, m, batch, q_len, ctx_len))   // (its own choice, the best logit, goes behind each token that it has read: ids_in is written anew by every call)
+    CKI(enqueue_draft_stream(h, L, which, batch, w.ids_in, 1, 1, !want_sample, f.ctx0, f.block_tables, nullptr, nullptr, want_sample ? w.logits_last : nullptr, 0, m.cfg.vocab));
+  else
+    CKI(enqueue_forward(h, L, f));
   const bool do_sample = want_sample && m.cfg.tp_rank == 0;
   if (do_sample) {
     SampleParams sp;
