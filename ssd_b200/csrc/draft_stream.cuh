@@ -28,7 +28,8 @@
 //
 // Measured, us a forward of the 1B draft (16 layers, context 203): with device-wide barriers between the stages and one warp per row on CUDA cores 738 (40.8 a layer, 18.6 of them weights at
 // copy bandwidth); tags 705; all reads of a slot in front of its products, which then go in four chains 665; one rolled copy of the code for all stages, which stays in the instruction
-// caches 622; two steps of k per product and missing words asked for again together 552.  What is left, of 30 us a layer: attention 5 (one CTA per key head fetches the keys), the four other
+// caches 622; two steps of k per product and missing words asked for again together 552; no
+// first piece asked for alone in front of gate|up's words 532.  What is left, of 28 us a layer: attention 5 (one CTA per key head fetches the keys), the four other
 // exchanges 1.2 each and a wait of up to 2.5 for the CTA whose weights come last, slots at 0.45 (0.73 is the memory's rate).  Contexts of 60 to 8000 tokens and other batches: use_draft_stream (engine.cu).
 //
 // Tags.  tag = forward * L + layer + 1; the words are zeroed at kernel start (a device-wide barrier follows), so no word of another launch is taken for this one's.
@@ -501,7 +502,6 @@ SSDK_DEVINL void ds_norm(const DsVec* src, const __nv_bfloat16* embed, int vocab
       uint4 v[2 * MT];   // (tokens that the batch has not ask for the first one's; every register of a stage is written in full: one that is written here and there
                          // stays alive from layer to layer, and all stages' together spill, 1250 us a forward)
       auto ask = [&](int i) { return ds_ask(*src, (i >> 1) < M ? i >> 1 : 0, i0 + 4 * (i & 1), tag); };
-      if (MT > 1) ds_wait_first(*src, 0, i0, tag, wait);
 #pragma unroll
       for (int i = 0; i < 2 * MT; ++i) v[i] = ask(i);
       ds_have(v, tag, wait, ask);
@@ -551,16 +551,17 @@ SSDK_DEVINL void ds_norm(const DsVec* src, const __nv_bfloat16* embed, int vocab
   ds_sync();
 }
 // A stage's results as they are, up to four tokens: a warp asks for its columns with all its lanes (all requests in flight at once) and lays them out
-// in shared memory of its own.
+// in shared memory of its own.  patient: asks for one piece until there is something.  Behind the attention, where most CTAs wait while a few fetch keys (asking for everything takes 8 %
+// of a 0.6B forward); behind gate|up the CTAs arrive together, and one token's first piece would cost a trip to L2 more than it saves (8B + 1B, k = 6, two target layers: 4428 -> 4167 us).
 template <int MT>
-SSDK_DEVINL const uint8_t* ds_stage_vec(const DsVec& v, const DsGeom& g, int M, uint32_t tag, const DsWait& wait, uint8_t* stage) {
+SSDK_DEVINL const uint8_t* ds_stage_vec(const DsVec& v, const DsGeom& g, int M, uint32_t tag, const DsWait& wait, uint8_t* stage, bool patient) {
   const int tid = ds_tid(), warp = tid >> 5, lane = tid & 31;
   const int part = g.ck >> 3, pitch = g.K / kDsWarps * 2 + kDsPad;   // this warp's columns of a chunk; bytes of a token
   uint8_t* mine = stage + (size_t)warp * M * pitch;
   constexpr int N = MT == 1 ? 8 : 16;   // requests in flight
   const int halves = part > 128 ? 2 : 1, n = M * g.chunks * halves;   // pieces of 128 words: half, chunk, token
   const int last = (part - 1) & ~3;   // (lanes behind the last column ask for it)
-  ds_wait_first(v, 0, warp * part + min(4 * lane, last), tag, wait);
+  if (MT > 1 || patient) ds_wait_first(v, 0, warp * part + min(4 * lane, last), tag, wait);
   for (int e = 0; e < n; e += N) {
     auto where = [&](int i, int& b, int& c, int& col) {
       const int u = min(e + i, n - 1);   // (n <= 4 x 4 x 2)
@@ -973,7 +974,7 @@ SSDK_DEVINL unsigned ds_stage(int kind, int l, int f, uint32_t tag, unsigned st)
   const int tid = ds_tid(), lane = tid & 31;
   if (kind == DS_O || kind == DS_DOWN) {
     if constexpr (MT <= 4) {
-      if (MT == 1 || ds_staged(MT, M, g.K)) { xrow = ds_stage_vec<MT>(src, g, M, tag, wait, S.scratch); pitch = g.K / kDsWarps * 2 + kDsPad; }   // (one token always fits)
+      if (MT == 1 || ds_staged(MT, M, g.K)) { xrow = ds_stage_vec<MT>(src, g, M, tag, wait, S.scratch, kind == DS_O); pitch = g.K / kDsWarps * 2 + kDsPad; }   // (one token always fits)
       else direct = true;
     } else {
       direct = true;
