@@ -1185,26 +1185,28 @@ static bool draft_stream_enabled() {
   return v == 1;
 }
 // Which draft path a step takes (both compute the same step; ctx_bound = the longest context of the batch before it).  Steps of k = 4 with two target layers, us, kernels per op -> streaming kernel:
-//   1B draft (16 layers, d = 2048): 1 sequence of 200, 900, 2000, 8000 tokens 4364 -> 3194, 4436 -> 3355, 4565 -> 3478, 4827 -> 4054; 2 of 200, 2000 4463 -> 3841, 4718 -> 4445;
-//     4 of 200, 2000 4699 -> 3804, 5005 -> 4395; 5 of 900, 2000 4872 -> 4657, 4938 -> 4901; 8 of 200, 900, 2000 4851 -> 4547, 4969 -> 4919, 5221 -> 5412
-//   0.6B draft (28 layers, d = 1024, heads of 128): 1 of 60, 200, 500, 900 4439 -> 4213, 4484 -> 4376, 4512 -> 4738, 4723 -> 4771; 2, 4, 8 of 200 4652 -> 5777, 4719 -> 5850, 5047 -> 7595
+//   1B draft (16 layers, d = 2048): 1 sequence of 200, 900, 2000, 8000 tokens 4364 -> 3101, 4444 -> 3339, 4565 -> 3500, 4827 -> 3982; 2 of 500, 2000 4512 -> 4072, 4688 -> 4434;
+//     4 of 200, 2000 4699 -> 3821, 5005 -> 4451; 5 of 500, 900, 1500 4735 -> 4437, 4861 -> 4696, 4910 -> 4796; 8 of 200, 500, 900 4872 -> 4631, 4964 -> 4836, 5056 -> 5122
+//   0.6B draft (28 layers, d = 1024, heads of 128): 1 of 60, 200, 500, 900 4439 -> 3988, 4484 -> 4136, 4512 -> 4738, 4723 -> 4708; 2, 4, 8 of 200 4652 -> 5777, 4719 -> 5850, 5047 -> 7595
 // Wide models stream their weights for most of a layer, so that what the kernel saves between stages counts; its attention, a few CTAs per sequence, costs more per key, which
-// bounds the keys of a call.  Narrow ones are all exchange, and from two sequences on every CTA reads more words than the weights it multiplies.
+// bounds the keys of a call (more than four sequences: half of the tokens' fragments come from other CTAs' words one chunk at a time, and the line lies lower).  Narrow ones are all exchange, and from two sequences on every CTA reads more words than the weights it multiplies.
 // SSDK_DRAFT_STREAM_MAX_CTX replaces the rule by a bound on the context alone.
+static int64_t stream_keys(int B) { return B > 4 ? 5120 : 8192; }   // of all sequences
 static bool use_draft_stream(ssdk_engine* e, int B, int ctx_bound) {
   const Model& m = e->model[SSDK_DRAFT];
   if (!m.present || !draft_stream_enabled() || !draft_stream_supported(m, B)) return false;
   const int keys = ctx_bound + e->rt.spec_k + 1;
   static const int forced = env_int("SSDK_DRAFT_STREAM_MAX_CTX", -1);
   if (forced >= 0) return keys <= forced;
-  if (m.d > 1024) return (int64_t)B * keys <= 8192;
+  if (m.d > 1024) return (int64_t)B * keys <= stream_keys(B);
   return B == 1 && keys <= (m.hd == 128 ? 256 : 1024);
 }
 // One token per sequence of plain decoding, for the wide models of the rule above: a forward is one launch instead of eight per layer, and no graph.  1B model, 16 layers, us a call with its token:
-//   1 sequence of 200, 2000, 7000 tokens 898 -> 665, 938 -> 731, 990 -> 838; 2 of 200, 4000 924 -> 798, 998 -> 983; 4 of 200, 2000 959 -> 772, 1023 -> 912; 8 of 200, 1000 986 -> 919, 1042 -> 1027;
-//   two layers of it: 1, 4, 8 of 200 279 -> 255, 268 -> 257, 280 -> 282
+//   1 sequence of 200, 2000, 7000 tokens 898 -> 626, 938 -> 699, 990 -> 807; 2 of 200, 4000 924 -> 792, 998 -> 980; 4 of 200, 2000 959 -> 766, 1023 -> 926; 8 of 200 986 -> 917;
+//   two layers of it: 1, 4, 8 of 200 279 -> 248, 268 -> 255, 280 -> 285 (the launch itself, its first barrier and the words of eight tokens: more than four sequences from four layers on)
 static bool stream_decode(ssdk_engine* e, const Model& m, int B, int q_len, const int32_t* ctx_len) {
-  return q_len == 1 && m.d > 1024 && draft_stream_enabled() && draft_stream_supported(m, B) && (int64_t)B * (*std::max_element(ctx_len, ctx_len + B) + 1) <= 8192;
+  return q_len == 1 && m.d > 1024 && (B <= 4 || m.cfg.layers >= 4) && draft_stream_enabled() && draft_stream_supported(m, B) &&
+         (int64_t)B * (*std::max_element(ctx_len, ctx_len + B) + 1) <= stream_keys(B);
 }
 template <int HD, int MT>
 static int launch_draft_stream(Launcher& L, const DsParams& p, size_t smem) {

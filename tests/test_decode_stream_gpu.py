@@ -16,7 +16,7 @@ def test_one_token_per_sequence_matches_the_oracle(lens, temp):
     dev = torch.device("cuda:0")
     B, bs = len(lens), 64
     mb = (max(lens) + 4) // bs + 1
-    cfg = ModelCfg(hidden=1280, layers=2, heads=20, kv_heads=5, head_dim=64, ffn=2560, vocab=1024, max_pos=bs * mb)
+    cfg = ModelCfg(hidden=1280, layers=4 if B > 4 else 2, heads=20, kv_heads=5, head_dim=64, ffn=2560, vocab=1024, max_pos=bs * mb)
     w = random_weights(cfg, 33)
     r = PairRunner(_spec(cfg), None, spec_k=0, max_batch=B, block_size=bs, max_model_len=bs * mb)
     r.bind_weights(L.TARGET, _to_dev(w, dev))
@@ -38,9 +38,11 @@ def test_one_token_per_sequence_matches_the_oracle(lens, temp):
     out = r.forward_tokens(L.TARGET, [[t] for t in toks], lens, tables.tolist(), temps=[temp] * B, seed=7)
     assert r.launch_count - n0 <= 2
     got = r.logits_last(B).float().cpu()
+    # 0.08 for two layers (as in the other engine tests), 0.05 for the last one's keys; the bf16 roundings of further layers are independent and add in quadrature
+    deeper = (cfg.layers / 2) ** 0.5
     for b, n in enumerate(lens):
         h = model.forward(torch.tensor([toks[b]]), torch.tensor([n]), slots(b, [n]), torch.tensor([n + 1], dtype=torch.int32), tables[b:b + 1], 1)
-        torch.testing.assert_close(got[b], model.compute_logits(h)[0].float(), atol=0.08, rtol=0.03)
+        torch.testing.assert_close(got[b], model.compute_logits(h)[0].float(), atol=0.08 * deeper, rtol=0.03)
     mine = V.sample(r.logits_last(B).cpu(), torch.tensor([temp] * B), 7, step * 16 + 14)
     assert list(out) == mine.tolist()
     kv = r.kv[L.TARGET].float().cpu()
@@ -48,5 +50,5 @@ def test_one_token_per_sequence_matches_the_oracle(lens, temp):
     for b, n in enumerate(lens):
         s = int(slots(b, [n])[0])
         for i in range(2):
-            torch.testing.assert_close(kv[i].reshape(cfg.layers, -1, cfg.kv_heads, 64)[:, s], ref[i].reshape(cfg.layers, -1, cfg.kv_heads, 64)[:, s], atol=0.05, rtol=0.02)
+            torch.testing.assert_close(kv[i].reshape(cfg.layers, -1, cfg.kv_heads, 64)[:, s], ref[i].reshape(cfg.layers, -1, cfg.kv_heads, 64)[:, s], atol=0.05 * deeper, rtol=0.02)
     r.close()
