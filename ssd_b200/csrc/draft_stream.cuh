@@ -630,27 +630,44 @@ struct DsPages {
   const int32_t* table;   // of the sequence
   const int* staged;      // its copy in shared memory, or null
   int block_size, shift;  // (shift < 0: not a power of two)
-  SSDK_DEVINL size_t slot(int t) const {
+  SSDK_DEVINL int page(int t) const {   // negative: the table names none
     const int i = shift >= 0 ? t >> shift : t / block_size;
-    const int blk = staged ? staged[i] : table[i];
-    return (size_t)blk * block_size + (t - i * block_size);
+    return staged ? staged[i] : table[i];
   }
+  SSDK_DEVINL size_t slot(int t, int page) const { return (size_t)page * block_size + (shift >= 0 ? t & (block_size - 1) : t % block_size); }
 };
+// Keys and values of tokens without a page are zeros, as in paged_attn_kernel: they are read from here (a flag or a bit per key next to the loads in flight spills: with heads of 128
+// 212 bytes -> 536 and more).
+__device__ uint4 ds_no_page[16];
 // Keys tb .. tb + 32 of a warp: tb is a multiple of 32, so that with pages of whole 32 one page holds them.  Keys behind the range and the new one (pos) are zero; whoever has
 // none reads an earlier key, so that no load waits for a branch (1.2 us to get sixteen loads under way with one).
-SSDK_DEVINL const __nv_bfloat16* ds_key_row(const __nv_bfloat16* base, const DsPages& pg, int ld, const __nv_bfloat16* page_row, int tb, int t) {
-  return page_row ? page_row + (t - tb) * ld : base + pg.slot(t) * ld;
-}
+struct DsRows {
+  const __nv_bfloat16* row;   // of the first of 32 keys, or of every cache's first row: keys look for their own pages
+  const DsPages& pg;
+  int ld, from;
+  bool whole;                 // one page holds them
+  SSDK_DEVINL DsRows(const __nv_bfloat16* base, const DsPages& g, int stride, int first) : row(base), pg(g), ld(stride), from(first), whole(g.block_size % 32 == 0) {
+    if (whole) {
+      const int page = pg.page(from);
+      row = page < 0 ? reinterpret_cast<const __nv_bfloat16*>(ds_no_page) : base + pg.slot(from, page) * ld;
+      if (page < 0) ld = 0;
+    }
+  }
+  SSDK_DEVINL const __nv_bfloat16* at(int t) const {
+    if (whole) return row + (t - from) * ld;
+    const int page = pg.page(t);
+    return page < 0 ? reinterpret_cast<const __nv_bfloat16*>(ds_no_page) : row + pg.slot(t, page) * ld;
+  }
+};
 SSDK_DEVINL uint4 ds_keep(const uint4& v, bool on) { return make_uint4(on ? v.x : 0u, on ? v.y : 0u, on ? v.z : 0u, on ? v.w : 0u); }
 // keys tb + 8 j + lane / 4, dims 32 k + 8 (lane & 3) .. + 8
 template <int HD>
 SSDK_DEVINL void ds_load_k(const __nv_bfloat16* base, const DsPages& pg, int ld, int lane, int tb, int t1, int pos, uint4 (&k)[4][HD / 32]) {
   const int most = max(min(t1, pos) - 1, 0);   // (the last key that is in the cache; none: the new one's slot, not used)
-  const __nv_bfloat16* page_row = pg.block_size % 32 == 0 ? base + pg.slot(min(tb, most)) * ld : nullptr;
-  const int from = min(tb, most);
+  const DsRows rows(base, pg, ld, min(tb, most));
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const __nv_bfloat16* s = ds_key_row(base, pg, ld, page_row, from, min(tb + 8 * j + (lane >> 2), most)) + 8 * (lane & 3);
+    const __nv_bfloat16* s = rows.at(min(tb + 8 * j + (lane >> 2), most)) + 8 * (lane & 3);
 #pragma unroll
     for (int i = 0; i < HD / 32; ++i) k[j][i] = ds_ldcg16(s + 32 * i);
   }
@@ -659,13 +676,12 @@ SSDK_DEVINL void ds_load_k(const __nv_bfloat16* base, const DsPages& pg, int ld,
 template <int HD>
 SSDK_DEVINL void ds_load_v(const __nv_bfloat16* base, const DsPages& pg, int ld, int lane, int tb, int t1, int pos, uint4 (&v)[2][4][HD / 64]) {
   const int most = max(min(t1, pos) - 1, 0);
-  const __nv_bfloat16* page_row = pg.block_size % 32 == 0 ? base + pg.slot(min(tb, most)) * ld : nullptr;
-  const int from = min(tb, most);
+  const DsRows rows(base, pg, ld, min(tb, most));
 #pragma unroll
   for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const __nv_bfloat16* s = ds_key_row(base, pg, ld, page_row, from, min(tb + 16 * kk + 2 * (lane & 3) + (j & 1) + 8 * (j >> 1), most)) + 8 * (lane >> 2);
+      const __nv_bfloat16* s = rows.at(min(tb + 16 * kk + 2 * (lane & 3) + (j & 1) + 8 * (j >> 1), most)) + 8 * (lane >> 2);
 #pragma unroll
       for (int i = 0; i < HD / 64; ++i) v[kk][j][i] = ds_ldcg16(s + 64 * i);
     }
@@ -742,11 +758,6 @@ SSDK_DEVINL void ds_attention_unit(const DsParams& p, int layer, int b, int h, i
       } while (!ok && !wait.give_up(w0));
       __syncwarp();
     }
-    if (kind == 2) {
-#pragma unroll
-      for (int t = 0; t < PT; ++t) { sv[lane + 32 * t] = f2bf(x1[t]); sv[HALF + lane + 32 * t] = f2bf(x2[t]); }
-      continue;
-    }
     if (nw) {
       float ss = 0.f;
 #pragma unroll
@@ -755,6 +766,15 @@ SSDK_DEVINL void ds_attention_unit(const DsParams& p, int layer, int b, int h, i
       const float rstd = rsqrtf(ss / (float)HD + p.eps);
 #pragma unroll
       for (int t = 0; t < PT; ++t) { x1[t] = bf16_round(x1[t] * rstd * n1[t]); x2[t] = bf16_round(x2[t] * rstd * n2[t]); }
+    }
+    if (kind > 0 && pg.page(pos) < 0) {   // a new token without a page counts like any other
+#pragma unroll
+      for (int t = 0; t < PT; ++t) x1[t] = x2[t] = 0.f;
+    }
+    if (kind == 2) {
+#pragma unroll
+      for (int t = 0; t < PT; ++t) { sv[lane + 32 * t] = f2bf(x1[t]); sv[HALF + lane + 32 * t] = f2bf(x2[t]); }
+      continue;
     }
     __nv_bfloat16* dst = kind == 0 ? reinterpret_cast<__nv_bfloat16*>(sq + (size_t)row * LDQ) : sk;
 #pragma unroll
@@ -768,11 +788,11 @@ SSDK_DEVINL void ds_attention_unit(const DsParams& p, int layer, int b, int h, i
 
   // ---- KV store of the new token (one unit per kv head) ----
   if (s == 0 && tid < HD / 4) {
-    const int i = pg.shift >= 0 ? pos >> pg.shift : pos / pg.block_size;
-    if ((pg.staged ? pg.staged[i] : pg.table[i]) >= 0) {
+    const int page = pg.page(pos);
+    if (page >= 0) {
       const int e = tid % (HD / 8) * 8;
       const bool val = tid >= HD / 8;
-      *reinterpret_cast<uint4*>((val ? vbase : kbase) + pg.slot(pos) * ld + e) = *reinterpret_cast<const uint4*>((val ? sv : sk) + e);
+      *reinterpret_cast<uint4*>((val ? vbase : kbase) + pg.slot(pos, page) * ld + e) = *reinterpret_cast<const uint4*>((val ? sv : sk) + e);
     }
   }
 

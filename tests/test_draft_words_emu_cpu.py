@@ -14,34 +14,30 @@ from oracle.model import ModelCfg, OracleModel, random_weights
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SRC = os.path.join(ROOT, "tests", "emu", "run_draft_words.cpp")
 BIN = os.path.join(ROOT, "tests", "emu", "_build", "run_draft_words")
+ASAN = BIN + "_asan"   # every access outside an array of the runner ends the process
 
 pytestmark = pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++ (C++20)")
 
 
-def _build():
+def _build(binary=BIN):
+    flags = ["-fsanitize=address", "-g"] if binary == ASAN else []
     deps = [SRC, os.path.join(ROOT, "tests", "emu", "cuda_emu.h")] + [os.path.join(ROOT, "ssd_b200", "csrc", n) for n in ("draft_stream.cuh", "common.cuh", "sampling.cuh")]
-    if os.path.exists(BIN) and all(os.path.getmtime(BIN) >= os.path.getmtime(d) for d in deps):
+    if os.path.exists(binary) and all(os.path.getmtime(binary) >= os.path.getmtime(d) for d in deps):
         return
-    os.makedirs(os.path.dirname(BIN), exist_ok=True)
-    subprocess.run(["g++", "-std=c++20", "-O1", "-pthread", "-Wno-unknown-pragmas", "-Wno-attributes", "-o", BIN, SRC], check=True)
+    os.makedirs(os.path.dirname(binary), exist_ok=True)
+    subprocess.run(["g++", "-std=c++20", "-O1", "-pthread", "-Wno-unknown-pragmas", "-Wno-attributes", *flags, "-o", binary, SRC], check=True)
 
 
 def _u16(t):
     return t.contiguous().view(torch.int16).numpy().astype(np.uint16)
 
 
-@pytest.mark.parametrize("hd,kv,grid,ffn,ctx,temp,chunk", [
-    (64, 2, 3, 512, [21], 0.0, 1024),                # one sequence, a range per key head
-    (64, 1, 2, 512, [300], 0.7, 256),                # two ranges: exchange of partial results; two slots per tile
-    (128, 1, 3, 768, [270, 5, 33], 0.0, 256),        # three sequences on the instance of four, three slots per tile
-    (64, 2, 2, 512, [9, 255, 256, 1, 30], 0.8, 512), # five: fragments straight from the words; more units than CTAs, contexts around a round of keys
-    (64, 1, 2, 4608, [40, 3, 7], 0.0, 2048),         # an intermediate row too long for the shared memory of four tokens' instance
-])
-def test_tagged_exchange_matches_the_oracle(tmp_path, hd, kv, grid, ffn, ctx, temp, chunk):
+def _check(tmp_path, hd, kv, grid, ffn, ctx, temp, chunk, bs=16, unnamed=(), binary=BIN):
+    """One launch against the oracle.  unnamed: (sequence, entry) pairs of the page tables that name no page."""
     from oracle import verify as V
-    _build()
+    _build(binary)
     torch.manual_seed(3)
-    B, n_fwd, bs = len(ctx), 2, 16
+    B, n_fwd = len(ctx), 2
     cfg = ModelCfg(hidden=256, layers=1 if ffn > 4096 else 2, heads=256 // hd, kv_heads=kv, head_dim=hd, ffn=ffn, vocab=264, max_pos=512, rms_eps=1e-6, rope_theta=500000.0, qk_norm=hd == 128)
     w = random_weights(cfg, seed=9)
     per = (max(ctx) + n_fwd) // bs + 1
@@ -49,10 +45,17 @@ def test_tagged_exchange_matches_the_oracle(tmp_path, hd, kv, grid, ffn, ctx, te
     order = torch.randperm(nblk).tolist()
     tables = [order[b * per:(b + 1) * per] for b in range(B)]
     model = OracleModel(cfg, w, num_blocks=nblk, block_size=bs)
+    given = [[-1 if (b, i) in unnamed else t for i, t in enumerate(row)] for b, row in enumerate(tables)]
     for b, n in enumerate(ctx):
+        if not n:
+            continue
         slots = torch.tensor([tables[b][p // bs] * bs + p % bs for p in range(n)], dtype=torch.int32)
         model.forward(torch.randint(0, cfg.vocab, (n,)), torch.arange(n), slots, torch.tensor([n], dtype=torch.int32), torch.tensor([tables[b]], dtype=torch.int32), n)
+    for b, i in unnamed:   # tokens without a page: keys and values of zeros, and nothing is stored (the oracle reads a page of zeros that the kernel does not know)
+        model.kv_cache[:, :, tables[b][i]] = 0
     kv0 = model.kv_cache.clone()
+    for b, i in unnamed:
+        kv0[:, :, tables[b][i]] = 3.0
     seed, call_base = 1234, 7 * 16
     temps = [temp if b != 1 else 0.0 for b in range(B)]
     blob, out = tmp_path / "in.bin", tmp_path / "out.bin"
@@ -62,7 +65,7 @@ def test_tagged_exchange_matches_the_oracle(tmp_path, hd, kv, grid, ffn, ctx, te
         np.array([seed, call_base], dtype=np.uint64).tofile(f)
         np.array([77 + b for b in range(B)], dtype=np.int64).tofile(f)
         np.array(ctx, dtype=np.int32).tofile(f)
-        np.array(tables, dtype=np.int32).tofile(f)
+        np.array(given, dtype=np.int32).tofile(f)
         for t in (w["embed"], w["final_norm"], w["lm_head"]):
             _u16(t).tofile(f)
         model.rope.numpy().astype(np.float32).tofile(f)
@@ -74,7 +77,7 @@ def test_tagged_exchange_matches_the_oracle(tmp_path, hd, kv, grid, ffn, ctx, te
             _u16(lw.get("k_norm", ones)).tofile(f)
         _u16(kv0[0]).tofile(f)
         _u16(kv0[1]).tofile(f)
-    res = subprocess.run([BIN, str(blob), str(out)], capture_output=True, text=True, timeout=600)
+    res = subprocess.run([binary, str(blob), str(out)], capture_output=True, text=True, timeout=600)
     assert res.returncode == 0, res.stderr[-2000:]
     raw = np.fromfile(out, dtype=np.uint16)
     nl, nc = B * n_fwd * cfg.vocab, cfg.layers * nblk * bs * kv * hd
@@ -85,7 +88,7 @@ def test_tagged_exchange_matches_the_oracle(tmp_path, hd, kv, grid, ffn, ctx, te
         bt = torch.tensor([tables[b]], dtype=torch.int32)
         for step in range(n_fwd):
             p = n + step
-            slot = torch.tensor([tables[b][p // bs] * bs + p % bs], dtype=torch.int32)
+            slot = torch.tensor([given[b][p // bs] * bs + p % bs if given[b][p // bs] >= 0 else -1], dtype=torch.int32)
             h = model.forward(torch.tensor([int(toks[b, step])]), torch.tensor([p]), slot, torch.tensor([p + 1], dtype=torch.int32), bt, 1)
             if step == n_fwd - 1:
                 assert toks[b, step + 1] == -1   # the last forward has no head
@@ -97,6 +100,30 @@ def test_tagged_exchange_matches_the_oracle(tmp_path, hd, kv, grid, ffn, ctx, te
             row = logits[:, step] if temps[b] else logits[b, step][None]
             mine = V.sample(row, torch.tensor(temps if temps[b] else [0.0]), seed, call_base + step)
             assert toks[b, step + 1] == int(mine[b if temps[b] else 0]), (b, step)
+    for b, i in unnamed:
+        model.kv_cache[:, :, tables[b][i]] = 3.0   # (untouched)
     ref = model.kv_cache.float()
     for got, want in ((kc, ref[0].reshape(-1)), (vc, ref[1].reshape(-1))):
         assert (got - want).abs().max() <= 0.02 * want.abs().max() + 1e-3
+
+
+@pytest.mark.parametrize("hd,kv,grid,ffn,ctx,temp,chunk", [
+    (64, 2, 3, 512, [21], 0.0, 1024),                # one sequence, a range per key head
+    (64, 1, 2, 512, [300], 0.7, 256),                # two ranges: exchange of partial results; two slots per tile
+    (128, 1, 3, 768, [270, 5, 33], 0.0, 256),        # three sequences on the instance of four, three slots per tile
+    (64, 2, 2, 512, [9, 255, 256, 1, 30], 0.8, 512), # five: fragments straight from the words; more units than CTAs, contexts around a round of keys
+    (64, 1, 2, 4608, [40, 3, 7], 0.0, 2048),         # an intermediate row too long for the shared memory of four tokens' instance
+])
+def test_tagged_exchange_matches_the_oracle(tmp_path, hd, kv, grid, ffn, ctx, temp, chunk):
+    _check(tmp_path, hd, kv, grid, ffn, ctx, temp, chunk)
+
+
+@pytest.mark.parametrize("hd,ctx,bs,unnamed", [
+    (64, [0], 16, [(0, 0)]),                           # no token in the cache and no page for the first
+    (128, [0, 30], 32, [(0, 0)]),                      # the same beside a sequence that has pages, pages of whole 32 keys
+    (64, [15, 40], 16, [(0, 0), (1, 1)]),              # a first page, whose last slot the new token would take; one inside a context
+    (64, [70, 40], 32, [(0, 1), (0, 2), (1, 1)]),      # pages of whole 32 keys, among them the new token's
+])
+def test_tokens_without_a_page_are_zeros(tmp_path, hd, ctx, bs, unnamed):
+    """The rule of paged_attn_kernel, and no read outside the cache (address sanitizer)."""
+    _check(tmp_path, hd, 2 if hd == 64 else 1, 2, 512, ctx, 0.0, 512, bs=bs, unnamed=unnamed, binary=ASAN)
