@@ -450,7 +450,7 @@ SSDK_DEVINL unsigned ld_acquire_u32(const unsigned* p) {
 SSDK_DEVINL unsigned atom_add_acq_rel_gpu(unsigned* p, unsigned v) { return __atomic_fetch_add(p, v, __ATOMIC_ACQ_REL); }
 SSDK_DEVINL void red_add_release_gpu_u64(unsigned long long* p, unsigned long long v) { __atomic_fetch_add(p, v, __ATOMIC_RELEASE); }
 SSDK_DEVINL unsigned long long ld_relaxed_gpu_u64(const unsigned long long* p) {
-  std::this_thread::yield();
+  emu::polled(p);
 #if defined(__SANITIZE_THREAD__)
   // ThreadSanitizer does not model atomic_thread_fence: the "relaxed poll + one acquire fence" of the device-wide barrier
   // would show up as races on everything the barrier orders.  Under TSan the poll itself acquires.
@@ -483,27 +483,18 @@ SSDK_DEVINL void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
   w = (w & ~0xFFFFFFFFull) | (uint32_t)((uint32_t)w + bytes);
   w -= (1ull << 32);
   emu_mbar_settle(w);
-  *bar = w;
+  __atomic_store_n(bar, w, __ATOMIC_RELEASE);
 }
 SSDK_DEVINL void mbar_arrive(uint64_t* bar) {
   std::lock_guard<std::mutex> g(emu_mbar_mu());
   uint64_t w = *bar;
   w -= (1ull << 32);
   emu_mbar_settle(w);
-  *bar = w;
+  __atomic_store_n(bar, w, __ATOMIC_RELEASE);
 }
-SSDK_DEVINL bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  std::lock_guard<std::mutex> g(emu_mbar_mu());
-  return (uint32_t)(*bar >> 63) != parity;
-}
+SSDK_DEVINL bool mbar_try_wait(uint64_t* bar, uint32_t parity) { return (uint32_t)(__atomic_load_n(bar, __ATOMIC_ACQUIRE) >> 63) != parity; }
 SSDK_DEVINL void mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (;;) {
-    {
-      std::lock_guard<std::mutex> g(emu_mbar_mu());
-      if ((uint32_t)(*bar >> 63) != parity) return;
-    }
-    std::this_thread::yield();
-  }
+  while (!mbar_try_wait(bar, parity)) std::this_thread::sleep_for(std::chrono::microseconds(200));
 }
 SSDK_DEVINL void bulk_load_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
   std::memcpy(smem_dst, gsrc, bytes);
@@ -511,7 +502,7 @@ SSDK_DEVINL void bulk_load_g2s(void* smem_dst, const void* gsrc, uint32_t bytes,
   uint64_t w = *bar;
   w = (w & ~0xFFFFFFFFull) | (uint32_t)((uint32_t)w - bytes);
   emu_mbar_settle(w);
-  *bar = w;
+  __atomic_store_n(bar, w, __ATOMIC_RELEASE);
 }
 SSDK_DEVINL uint4 ld_volatile_v4(const void* p) {
   // two aligned 8-byte words {2 x bf16, epoch}: each is read atomically, like the device's 8-byte store granularity
@@ -526,15 +517,15 @@ template <int N>
 SSDK_DEVINL void reg_dec() {}
 SSDK_DEVINL void st_relaxed_gpu_u64(unsigned long long* p, unsigned long long v) { __atomic_store_n(p, v, __ATOMIC_RELAXED); }
 SSDK_DEVINL uint32_t ld_relaxed_gpu_u32(const uint32_t* p) {
-  std::this_thread::sleep_for(std::chrono::microseconds(20));   // (pollers that only yield keep the threads they wait for off the cores)
+  emu::polled(p);
   return __atomic_load_n(p, __ATOMIC_RELAXED);
 }
 SSDK_DEVINL uint4 ld_relaxed_gpu_v4(const void* p) {
+  emu::polled(p);
   const uint32_t* q = reinterpret_cast<const uint32_t*>(p);
   uint4 r;
   r.x = __atomic_load_n(q, __ATOMIC_RELAXED); r.y = __atomic_load_n(q + 1, __ATOMIC_RELAXED);
   r.z = __atomic_load_n(q + 2, __ATOMIC_RELAXED); r.w = __atomic_load_n(q + 3, __ATOMIC_RELAXED);
-  std::this_thread::sleep_for(std::chrono::microseconds(20));
   return r;
 }
 // every lane's word of a warp
@@ -559,31 +550,21 @@ SSDK_DEVINL uint32_t __byte_perm(uint32_t a, uint32_t b, uint32_t sel) {
   return r;
 }
 SSDK_DEVINL void mma_bf16_16816(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-  struct Words { uint32_t w[32][6]; };
-  static std::mutex mu;
-  static std::map<emu::Warp*, std::unique_ptr<Words>> all;
-  emu::Warp* warp = emu::tctx.cta->warps[threadIdx.x >> 5].get();
-  Words* x;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    auto& slot = all[warp];
-    if (!slot) slot = std::make_unique<Words>();
-    x = slot.get();
-  }
-  uint32_t* mine = x->w[threadIdx.x & 31];
+  emu::Warp* x = emu::tctx.cta->warps[threadIdx.x >> 5].get();
+  uint32_t* mine = x->operands[threadIdx.x & 31];
   for (int i = 0; i < 4; ++i) mine[i] = a[i];
   mine[4] = b0; mine[5] = b1;
-  warp->bar.arrive_and_wait();
+  x->bar.arrive_and_wait();
   auto val = [](uint32_t w, int half) { return __bfloat162float(__nv_bfloat16{(uint16_t)(half ? w >> 16 : w & 0xffffu)}); };
   const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
   for (int e = 0; e < 4; ++e) {
     const int row = g, hi = e >> 1, col = 2 * t + (e & 1);   // rows behind the eighth: A's odd words
     for (int k = 0; k < 16; ++k) {
       const int lane_k = (k & 7) >> 1, part = k >> 3;
-      c[e] += val(x->w[row * 4 + lane_k][2 * part + hi], k & 1) * val(x->w[col * 4 + lane_k][4 + part], k & 1);
+      c[e] += val(x->operands[row * 4 + lane_k][2 * part + hi], k & 1) * val(x->operands[col * 4 + lane_k][4 + part], k & 1);
     }
   }
-  warp->bar.arrive_and_wait();
+  x->bar.arrive_and_wait();
 }
 #endif
 

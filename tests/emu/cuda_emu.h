@@ -68,7 +68,7 @@ using std::min;
 
 namespace emu {
 struct Warp {
-  uint32_t slot[32];
+  uint32_t slot[32], operands[32][6];   // of shuffles; of mma
   std::barrier<> bar{32};
 };
 struct Cta {
@@ -92,10 +92,15 @@ inline void* dyn_smem() {
 }
 template <typename T>
 T* static_smem(size_t n, int key) {
-  std::lock_guard<std::mutex> g(tctx.cta->mu);
-  auto& v = tctx.cta->statics[key];
-  if (v.empty()) v.resize(n * sizeof(T) + 64);
-  return reinterpret_cast<T*>((reinterpret_cast<uintptr_t>(v.data()) + 63) & ~uintptr_t(63));
+  thread_local std::map<int, void*> known;   // (a thread belongs to one CTA)
+  void*& p = known[key];
+  if (!p) {
+    std::lock_guard<std::mutex> g(tctx.cta->mu);
+    auto& v = tctx.cta->statics[key];
+    if (v.empty()) v.resize(n * sizeof(T) + 64);
+    p = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(v.data()) + 63) & ~uintptr_t(63));
+  }
+  return reinterpret_cast<T*>(p);
 }
 }  // namespace emu
 
@@ -138,6 +143,19 @@ inline T __shfl_xor_sync(unsigned, T v, int lane_mask) {
   w.bar.arrive_and_wait();
   return r;
 }
+namespace emu {
+// A thread that asks for an address again sleeps: some hundred pollers that only yield, or sleep for a few microseconds, take all cores from the threads that they wait for.
+inline void polled(const void* p) {
+  thread_local const void* last[64];
+  thread_local unsigned n = 0;
+  for (const void* q : last)
+    if (q == p) {
+      std::this_thread::sleep_for(std::chrono::microseconds(500));
+      return;
+    }
+  last[n++ % 64] = p;
+}
+}  // namespace emu
 inline unsigned atomicAdd(unsigned* p, unsigned v) { return __atomic_fetch_add(p, v, __ATOMIC_SEQ_CST); }
 template <typename T>
 inline T __ldcg(const T* p) { return *p; }
