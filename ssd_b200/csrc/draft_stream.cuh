@@ -20,7 +20,10 @@
 // Philox exponential race of layers/sampler.py:27-34 — the SAME scores sample_kernel computes, so the tokens are identical)
 // -> the next forward starts inside the same launch.  The last forward of a step only writes KV (speculator_sync.py:52-56).
 // Rounding points are the reference's: every linear output, the residual, the norm output, q/k
-// after RoPE and the attention output are rounded to bf16; accumulation is fp32.
+// after RoPE and the attention output are rounded to bf16; accumulation is fp32, in the tensor cores for chains of two products of 16 columns (more than
+// four sequences: four), which fp32 adds bring together.  Of logits of
+// 2048 columns 7.2e-5 (one sequence), 8.7e-5 (three), 8.6e-5 (eight) are not the rounded exact sum; chains of fp32 FMA that one warp per row ran before left 7.8e-5, the kernel-by-kernel
+// form, which batches took before, 8.7e-4 .. 9.1e-4.
 //
 // Products: a CTA owns a run of consecutive rows of every matrix (N / #CTAs, to one row), walked in tiles of 8 rows x up to 2048 columns = one slot.
 // mma.sync m16n8k16; the eight warps take an eighth of the columns each and meet in shared memory once per group of tiles.  The order of k inside a product is free as long
@@ -619,7 +622,7 @@ SSDK_DEVINL void ds_frag_vec(const DsVec& v, const DsGeom& g, int c, int M, uint
 // ---------------------------------------------------------------------------------------------
 // stage B unit: sequence b, kv head h, split s.  Rebuilds the rotated q rows of the head group and the new token's k / v from the
 // q|k|v words, stores k / v into the page slot (split 0 only) and runs its token range: warp w takes 32 keys at a time, scores on mma.sync (q as A, keys as B), online
-// softmax in registers, weights in two bf16 pieces (the rest is 2^-18 of a weight) times the values as the other operand.  A thread's 16-byte loads ARE its fragments: eight
+// softmax in registers, weights in three bf16 pieces (all of their bits) times the values as the other operand.  A thread's 16-byte loads ARE its fragments: eight
 // dims of one key; of a value row, eight dims of which each product takes two.  The cached keys and values do not depend on this layer's stages, so they are asked for before
 // the wait for q|k|v; the next 32 keys' are asked for as soon as their registers are free.
 // (A lane per head dim with a five-shuffle sum per key and head, partials, a ticket and a merge by the last split: 4.8 us per layer at contexts of 135.)
@@ -685,6 +688,15 @@ SSDK_DEVINL void ds_load_v(const __nv_bfloat16* base, const DsPages& pg, int ld,
 #pragma unroll
       for (int i = 0; i < HD / 64; ++i) v[kk][j][i] = ds_ldcg16(s + 64 * i);
     }
+}
+// Two weights in three bf16 pieces each, whose sum is the weight in all of its 24 bits (what is left of it has 16 bits, then 8)
+SSDK_DEVINL void ds_pieces(float p0, float p1, uint32_t (&w)[3]) {
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    w[q] = pack_bf16x2(p0, p1);
+    p0 -= ds_bits_f(w[q] & 0xffffu);
+    p1 -= ds_bits_f(w[q] >> 16);
+  }
 }
 SSDK_DEVINL uint32_t ds_word(const uint4& v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
 
@@ -852,22 +864,21 @@ SSDK_DEVINL void ds_attention_unit(const DsParams& p, int layer, int b, int h, i
     for (int j = 0; j < HD / 16; ++j) { o[j][0] *= corr0; o[j][1] *= corr1; o[j][2] *= corr0; o[j][3] *= corr1; }
 #pragma unroll
     for (int kk = 0; kk < 2; ++kk) {
-      uint32_t hi[2], lo[2];
+      uint32_t w[2][3];
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const float p0 = exp2f(sc[2 * kk + e][0] - base), p1 = exp2f(sc[2 * kk + e][1] - base);
         l += p0 + p1;
-        hi[e] = pack_bf16x2(p0, p1);
-        lo[e] = pack_bf16x2(p0 - ds_bits_f(hi[e] & 0xffffu), p1 - ds_bits_f(hi[e] >> 16));
+        ds_pieces(p0, p1, w[e]);
       }
 #pragma unroll
       for (int i = 0; i < HD / 64; ++i)
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          const uint32_t u0 = ds_word(vf[kk][0][i], w), u1 = ds_word(vf[kk][1][i], w), u2 = ds_word(vf[kk][2][i], w), u3 = ds_word(vf[kk][3][i], w);
+        for (int d = 0; d < 4; ++d) {
+          const uint32_t u0 = ds_word(vf[kk][0][i], d), u1 = ds_word(vf[kk][1][i], d), u2 = ds_word(vf[kk][2][i], d), u3 = ds_word(vf[kk][3][i], d);
           const uint32_t a[4] = {__byte_perm(u0, u1, 0x5410), __byte_perm(u0, u1, 0x7632), __byte_perm(u2, u3, 0x5410), __byte_perm(u2, u3, 0x7632)};
-          mma_bf16_16816(o[4 * i + w], a, hi[0], hi[1]);
-          mma_bf16_16816(o[4 * i + w], a, lo[0], lo[1]);
+#pragma unroll
+          for (int q = 0; q < 3; ++q) mma_bf16_16816(o[4 * i + d], a, w[0][q], w[1][q]);
         }
     }
     if (more) ds_load_v<HD>(vbase, pg, ld, lane, tb + kDsUnitKeys, t1, pos, vf);

@@ -1,6 +1,7 @@
 // Runs the SOURCE of csrc/draft_stream.cuh on host threads (cuda_emu.h) with the exchange that the product uses (tagged words instead of barriers), for a
 // batch of sequences.  TEST INFRASTRUCTURE.
 //   run_draft_words <input blob> <output blob>
+//   run_draft_words pieces           the attention's weights against the sum of their pieces
 // blob layout: see tests/test_draft_words_emu_cpu.py (the writer).
 #include "cuda_emu.h"
 #define SSDK_HOST_EMU 1
@@ -8,6 +9,7 @@
 
 #include <fstream>
 #include <iostream>
+#include <string>
 
 using bf16 = __nv_bfloat16;
 
@@ -27,7 +29,31 @@ struct Reader {
   int i32() { return vec<int32_t>(1)[0]; }
 };
 
+static int check_pieces() {
+  uint32_t x = 12345u;
+  for (int i = 0; i < 1000000; ++i) {
+    float p[2];
+    for (float& v : p) {
+      x = x * 1664525u + 1013904223u;
+      v = std::exp2((float)-(int)(x >> 25)) * (1.0f + (float)(x & 0x7fffffu) * 0x1p-23f);   // all mantissas, 2^-127 .. 2
+      if (v > 1.0f) v *= 0.5f;
+    }
+    uint32_t w[3];
+    ssdk::ds_pieces(p[0], p[1], w);
+    for (int h = 0; h < 2; ++h) {
+      double sum = 0;
+      for (uint32_t q : w) sum += (double)ssdk::ds_bits_f(h ? q >> 16 : q & 0xffffu);
+      if (std::abs(sum - (double)p[h]) > 0x1p-133) {   // (below that a bf16 has no bits)
+        std::cerr << "weight " << p[h] << " is " << sum << "\n";
+        return 1;
+      }
+    }
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
+  if (argc == 2 && std::string(argv[1]) == "pieces") return check_pieces();
   if (argc != 3) return 2;
   Reader r(argv[1]);
   const int B = r.i32(), d = r.i32(), L = r.i32(), H = r.i32(), KV = r.i32(), hd = r.i32(), ffn = r.i32(), vocab = r.i32();

@@ -127,3 +127,10 @@ def test_tagged_exchange_matches_the_oracle(tmp_path, hd, kv, grid, ffn, ctx, te
 def test_tokens_without_a_page_are_zeros(tmp_path, hd, ctx, bs, unnamed):
     """The rule of paged_attn_kernel, and no read outside the cache (address sanitizer)."""
     _check(tmp_path, hd, 2 if hd == 64 else 1, 2, 512, ctx, 0.0, 512, bs=bs, unnamed=unnamed, binary=ASAN)
+
+
+def test_attention_weights_keep_all_their_bits():
+    """The products take a weight as bf16 pieces; their sum is the 32-bit weight."""
+    _build()
+    res = subprocess.run([BIN, "pieces"], capture_output=True, text=True, timeout=60)
+    assert res.returncode == 0, res.stderr[-500:]
