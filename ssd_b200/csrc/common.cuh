@@ -460,7 +460,7 @@ SSDK_DEVINL unsigned long long ld_relaxed_gpu_u64(const unsigned long long* p) {
 #endif
 }
 SSDK_DEVINL void fence_acq_rel_gpu() { std::atomic_thread_fence(std::memory_order_acq_rel); }
-SSDK_DEVINL void st_relaxed_gpu_u32(unsigned* p, unsigned v) { __atomic_store_n(p, v, __ATOMIC_RELAXED); }
+SSDK_DEVINL void st_relaxed_gpu_u32(unsigned* p, unsigned v) { if (!emu::lost(emu::lost_words)) __atomic_store_n(p, v, __ATOMIC_RELAXED); }
 SSDK_DEVINL void prefetch_l2(const void*) {}
 // mbarrier + bulk copy stand-ins: one 64-bit word = {phase bit 63 | pending arrivals 32..47 | init count 48..62 | tx bytes 0..31},
 // updated under one global lock (test infrastructure; the bulk copy is a synchronous memcpy by the issuing thread)
@@ -492,11 +492,16 @@ SSDK_DEVINL void mbar_arrive(uint64_t* bar) {
   emu_mbar_settle(w);
   __atomic_store_n(bar, w, __ATOMIC_RELEASE);
 }
-SSDK_DEVINL bool mbar_try_wait(uint64_t* bar, uint32_t parity) { return (uint32_t)(__atomic_load_n(bar, __ATOMIC_ACQUIRE) >> 63) != parity; }
+SSDK_DEVINL bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+  if ((uint32_t)(__atomic_load_n(bar, __ATOMIC_ACQUIRE) >> 63) != parity) return true;
+  std::this_thread::sleep_for(std::chrono::microseconds(200));   // (a waiter that spins takes the cores from the threads that it waits for)
+  return (uint32_t)(__atomic_load_n(bar, __ATOMIC_ACQUIRE) >> 63) != parity;
+}
 SSDK_DEVINL void mbar_wait(uint64_t* bar, uint32_t parity) {
-  while (!mbar_try_wait(bar, parity)) std::this_thread::sleep_for(std::chrono::microseconds(200));
+  while (!mbar_try_wait(bar, parity)) {}
 }
 SSDK_DEVINL void bulk_load_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
+  if (emu::lost(emu::lost_copies)) return;
   std::memcpy(smem_dst, gsrc, bytes);
   std::lock_guard<std::mutex> g(emu_mbar_mu());
   uint64_t w = *bar;
@@ -536,7 +541,9 @@ inline void emu_gather(uint32_t v, uint32_t* all) {
   std::memcpy(all, w.slot, sizeof(w.slot));
   w.bar.arrive_and_wait();
 }
-SSDK_DEVINL float __shfl_sync(unsigned, float v, int src) {
+template <typename T>
+SSDK_DEVINL T __shfl_sync(unsigned, T v, int src) {
+  static_assert(sizeof(T) == 4, "32-bit shuffles only");
   uint32_t u, all[32];
   std::memcpy(&u, &v, 4);
   emu_gather(u, all);

@@ -65,9 +65,9 @@ constexpr int kDsStage = 33 * 1024;   // vectors up to this many bytes are laid 
 constexpr int kDsBtSmem = 32;         // page-table entries of a sequence staged in shared memory at kernel start (the table is launch-constant)
 
 #ifdef SSDK_HOST_EMU
-constexpr long long kDsWaitCycles = 4000000000000LL;
+inline long long ds_wait_cycles = 4000000000000LL;   // (tests set it)
 #else
-constexpr long long kDsWaitCycles = 4000000000LL;
+constexpr long long ds_wait_cycles = 4000000000LL;   // of clock64: about two seconds
 #endif
 
 struct DsLayer {
@@ -129,19 +129,29 @@ SSDK_DEVINL int ds_tid() {
 }
 
 // ---------------------------------------------------------------------------------------------
-// waits: about two seconds, then the launch's word is set and every later wait of the CTA returns at once (its results are garbage that stays in bounds)
+// waits: all have a limit.  One that runs out sets the launch's word (the host's next look at it is an error of the call) and the CTA goes on without what it waited for: its results are
+// garbage that stays in bounds, under the tags that other CTAs wait for, and it arrives at every barrier, so that the launch ends and leaves the next one a whole count.
+// `dead`: words and barriers, which other CTAs bring; every later wait of the CTA for one returns at once, while its weights, which it fetches itself, are waited for as ever.
+// `broken`: slots of the ring; neither side waits for them any more, and the producer asks for nothing more and waits, again with a limit, for what is in flight.
 // ---------------------------------------------------------------------------------------------
 struct DsWait {
   volatile int* dead;   // shared by the CTA
   unsigned* timeout;
   SSDK_DEVINL bool give_up(long long t0) const {
     if (*dead) return true;
-    if (clock64() - t0 < kDsWaitCycles) return false;
+    if (clock64() - t0 < ds_wait_cycles) return false;
     *dead = 1;
     if (timeout) *reinterpret_cast<volatile unsigned*>(timeout) = 1u;
     return true;
   }
 };
+SSDK_DEVINL bool ds_ring_wait(uint64_t* bar, uint32_t parity, const DsWait& broken) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity))
+    if (broken.give_up(t0)) return false;
+  return true;
+}
 
 // ---------------------------------------------------------------------------------------------
 // device-wide barrier of the consumers (kernel start, and once per forward behind the sampling, where it also orders the new keys and values): ONE 64-bit arrival
@@ -237,9 +247,11 @@ struct DsProducer {
   uint8_t* ring;
   uint64_t *full, *empty;
   unsigned n_slots, slot_bytes, slot, phase;
+  DsWait broken;
+  unsigned used;   // slots that have been asked for at least once
 };
 template <int MT>
-SSDK_DEVINL void ds_feed(DsProducer& r, const DsGeom& g, const __nv_bfloat16* w, bool pair) {
+SSDK_DEVINL bool ds_feed(DsProducer& r, const DsGeom& g, const __nv_bfloat16* w, bool pair) {
   constexpr int group = ds_group(MT);
   const int lane = threadIdx.x & 31, sub = pair ? 2 : 1, r1 = g.r1;
   for (int t0 = g.r0; t0 < r1; t0 += kDsTile * group / sub)   // the order of ds_consume: groups, chunks, tiles
@@ -247,28 +259,37 @@ SSDK_DEVINL void ds_feed(DsProducer& r, const DsGeom& g, const __nv_bfloat16* w,
       for (int i = 0; i < group; ++i) {
         const int t = t0 + i / sub * kDsTile, n = min(kDsTile, r1 - t);
         if (n <= 0) break;
+        int ok = 1;
         if (lane == 0) {
-          mbar_wait(&r.empty[r.slot], r.phase ^ 1u);  // a fresh barrier passes the first round at once
-          mbar_arrive_expect_tx(&r.full[r.slot], (unsigned)(n * g.ck * 2));
+          ok = ds_ring_wait(&r.empty[r.slot], r.phase ^ 1u, r.broken);  // a fresh barrier passes the first round at once
+          if (ok) mbar_arrive_expect_tx(&r.full[r.slot], (unsigned)(n * g.ck * 2));
         }
-        __syncwarp();
+        if (!__shfl_sync(0xffffffffu, ok, 0)) return false;
         if (lane < n)
           bulk_load_g2s(r.ring + (size_t)r.slot * r.slot_bytes + (size_t)lane * (g.ck * 2 + kDsPad),
                         w + ((size_t)(i % sub ? g.rows : 0) + t + lane) * g.K + (size_t)c * g.ck, (unsigned)g.ck * 2u, &r.full[r.slot]);
-        if (++r.slot == r.n_slots) { r.slot = 0; r.phase ^= 1u; }
+        if (++r.slot == r.n_slots) { r.slot = 0; r.phase ^= 1u; r.used = r.n_slots; }
+        r.used = max(r.used, r.slot);
       }
+  return true;
 }
 template <int MT>
 SSDK_DEVINL void ds_producer(const DsParams& p, const DsGeom* geom, DsProducer& r) {
-  for (int f = 0; f < p.n_fwd; ++f) {
-    for (int l = 0; l < p.L; ++l) {
+  bool ok = true;
+  for (int f = 0; ok && f < p.n_fwd; ++f) {
+    for (int l = 0; ok && l < p.L; ++l) {
       const DsLayer& lw = p.layers[l];
-      ds_feed<MT>(r, geom[DS_QKV], lw.qkv, false);
-      ds_feed<MT>(r, geom[DS_O], lw.o, false);
-      ds_feed<MT>(r, geom[DS_GU], lw.gate_up, true);
-      ds_feed<MT>(r, geom[DS_DOWN], lw.down, false);
+      ok = ds_feed<MT>(r, geom[DS_QKV], lw.qkv, false) && ds_feed<MT>(r, geom[DS_O], lw.o, false) && ds_feed<MT>(r, geom[DS_GU], lw.gate_up, true) &&
+           ds_feed<MT>(r, geom[DS_DOWN], lw.down, false);
     }
-    if (ds_has_head(p, f)) ds_feed<MT>(r, geom[DS_HEAD], p.lm_head, false);
+    if (ok && ds_has_head(p, f)) ok = ds_feed<MT>(r, geom[DS_HEAD], p.lm_head, false);
+  }
+  // no copy is in flight when the CTA leaves: the last one into every slot
+  for (unsigned s = threadIdx.x & 31; s < r.used; s += 32) {
+    const uint32_t parity = s < r.slot ? r.phase : r.phase ^ 1u;
+    const long long t0 = clock64();
+    while (!mbar_try_wait(&r.full[s], parity))
+      if (clock64() - t0 > ds_wait_cycles) break;
   }
 }
 
@@ -328,6 +349,8 @@ struct DsRing {
   const uint8_t* base;
   uint64_t *full, *empty;
   unsigned n_slots, slot_bytes, slot, phase;
+  DsWait broken;
+  bool gone;   // this thread has given up a slot: it takes and gives back no more (a slot needs all warps to be given back, so that the producer stops too)
 };
 // x of a chunk, this thread's fragments, steps of 32 columns of the warp's ck / 8.  Five tokens and more: step j, columns 32 j + 8 (lane & 3) .. + 8 of token lane / 4.
 // Up to four: steps 2 j (lanes 0 .. 15) and 2 j + 1 (16 .. 31) of token (lane / 4) & 3.
@@ -369,7 +392,7 @@ SSDK_DEVINL void ds_slot(DsRing& ring, int steps, int at, int lane, const DsX<MT
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) c[i][e] = 0.f;
-  mbar_wait(&ring.full[ring.slot], ring.phase);
+  ring.gone = ring.gone || !ds_ring_wait(&ring.full[ring.slot], ring.phase, ring.broken);
   const uint8_t* w = ring.base + (unsigned)(ring.slot * ring.slot_bytes + at);
   if (steps == 8) {
     ds_steps<MT, 8>(w, x.v, c);
@@ -389,7 +412,7 @@ SSDK_DEVINL void ds_slot(DsRing& ring, int steps, int at, int lane, const DsX<MT
     }
   }
   __syncwarp();
-  if (lane == 0) mbar_arrive(&ring.empty[ring.slot]);   // one arrive per consumer warp, after its last read
+  if (lane == 0 && !ring.gone) mbar_arrive(&ring.empty[ring.slot]);   // one arrive per consumer warp, after its last read
   if (++ring.slot == ring.n_slots) { ring.slot = 0; ring.phase ^= 1u; }
   float s[4];
 #pragma unroll
@@ -965,14 +988,14 @@ SSDK_DEVINL void ds_attention_merge(const DsParams& p, int b, int h, int s, int 
 }
 
 // ---------------------------------------------------------------------------------------------
-// the stages.  What they share is in shared memory.  `st`: ring slot | ring phase << 8.
+// the stages.  What they share is in shared memory.  `st`: ring slot | ring phase << 8 | ring given up << 9.
 // ---------------------------------------------------------------------------------------------
 struct DsShared {
   DsParams p;
   DsGeom geom[5];
   DsVec vec[5];             // results of the stages: q|k|v, attention, o, act, down
   DsPartial part;
-  int M, shift, staged, dead;
+  int M, shift, staged, dead, broken;
   unsigned slot_bytes;
   uint8_t *sums, *resid, *scratch;
   int tok[kDsMaxBatch];
@@ -1041,7 +1064,7 @@ SSDK_DEVINL unsigned ds_stage(int kind, int l, int f, uint32_t tag, unsigned st)
     smp.call_id = (S.p.dyn ? S.p.dyn[1] * 16ull : S.p.call_base) + (uint64_t)f;
     if (S.p.logits) smp.logits = S.p.logits + (size_t)f * S.p.logits_ld + (size_t)tok * S.p.logits_seq_ld;
   }
-  DsRing ring{ds_smem, S.full, S.empty, (unsigned)S.p.n_slots, S.slot_bytes, st & 0xffu, st >> 8};
+  DsRing ring{ds_smem, S.full, S.empty, (unsigned)S.p.n_slots, S.slot_bytes, st & 0xffu, st >> 8 & 1u, DsWait{&S.broken, S.p.timeout}, st >> 9 != 0u};
   ds_consume<MT>(ring, g, kind == DS_GU ? DS_GATED : (kind == DS_HEAD ? DS_LOGITS : DS_ROWS), M, reinterpret_cast<float*>(S.sums), out, tag, load, smp);
   ds_mark(f, 2 * kind + 1);
   if (kind == DS_HEAD) {   // eight threads of a warp per sequence -> per-CTA best
@@ -1061,7 +1084,7 @@ SSDK_DEVINL unsigned ds_stage(int kind, int l, int f, uint32_t tag, unsigned st)
       S.p.samp_partial[(size_t)tid * gridDim.x + blockIdx.x] = c;
     }
   }
-  return ring.slot | ring.phase << 8;
+  return ring.slot | ring.phase << 8 | (ring.gone ? 1u : 0u) << 9;
 }
 // B: units of this CTA (pass 0), their merges (pass 1: behind all units of a CTA, since a merge waits for units of other CTAs)
 template <int HD>
@@ -1104,7 +1127,7 @@ __global__ void __launch_bounds__(kDsThreads, 1) draft_stream_kernel(const __gri
     ds_geometry(p.d, p.vocab, max_chunk, &S.geom[DS_HEAD]);
     for (int i = 0; i < 5; ++i) ds_own_rows(&S.geom[i]);
     // dynamic shared memory: [ring][sums of the tiles][residual rows][normed rows / fragments / attention scratch]
-    S.M = M; S.dead = 0; S.staged = staged; S.slot_bytes = slot_bytes;
+    S.M = M; S.dead = S.broken = 0; S.staged = staged; S.slot_bytes = slot_bytes;
     S.sums = ds_smem + (size_t)p.n_slots * slot_bytes;
     S.resid = S.sums + ds_part_bytes(MT);
     S.scratch = S.resid + (size_t)M * p.d * 2;
@@ -1133,7 +1156,7 @@ __global__ void __launch_bounds__(kDsThreads, 1) draft_stream_kernel(const __gri
     reg_dec<kDsRegsProducer>();
     if (threadIdx.x >= kDsConsumers + 32) return;
     // ===================== producer warp: the weight stream never waits for a stage =====================
-    DsProducer r{ds_smem, S.full, S.empty, (unsigned)p.n_slots, slot_bytes, 0u, 0u};
+    DsProducer r{ds_smem, S.full, S.empty, (unsigned)p.n_slots, slot_bytes, 0u, 0u, DsWait{&S.broken, p.timeout}, 0u};
     ds_producer<MT>(p, S.geom, r);
     return;
   }
@@ -1189,7 +1212,7 @@ __global__ void __launch_bounds__(kDsThreads, 1) draft_stream_kernel(const __gri
       }
       a = warp_argmax(a);
       if ((threadIdx.x & 31) == 0) {
-        const int t = min(a.i, p.vocab - 1);   // (logits that are all NaN have no best)
+        const int t = min(max(a.i, 0), p.vocab - 1);   // (logits that are all NaN have no best; behind a wait that ran out there may be anything)
         S.tok[b] = t;
         if (blockIdx.x == 0) p.tok_buf[(size_t)b * p.tok_ld + f + 1] = t;
       }

@@ -253,7 +253,7 @@ struct WaitWord {
     volatile unsigned* w = word;
     if (!*w) return 0;
     *w = 0;
-    return fail("a bounded wait in a tile-pair product or the prompt attention ran out: what %s", whose);
+    return fail("a bounded wait in a tile-pair product, the prompt attention or the streaming kernel ran out: what %s", whose);
   }
 };
 // The same for calls without an engine, which do not wait for the stream: rows whose waits ran out are NaN, and the next such call reports it.  One word for the

@@ -156,6 +156,11 @@ inline void polled(const void* p) {
   last[n++ % 64] = p;
 }
 }  // namespace emu
+namespace emu {
+// failures that a test asks for: of the last CTA, what follows the n-th word it stores or copy it makes (-1: none) is lost
+inline std::atomic<int> lost_words{-1}, lost_copies{-1};
+inline bool lost(std::atomic<int>& left) { return blockIdx.x + 1 == gridDim.x && left.load() >= 0 && left.fetch_sub(left.load() > 0 ? 1 : 0) == 0; }
+}  // namespace emu
 inline unsigned atomicAdd(unsigned* p, unsigned v) { return __atomic_fetch_add(p, v, __ATOMIC_SEQ_CST); }
 template <typename T>
 inline T __ldcg(const T* p) { return *p; }

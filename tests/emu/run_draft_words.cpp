@@ -1,6 +1,7 @@
 // Runs the SOURCE of csrc/draft_stream.cuh on host threads (cuda_emu.h) with the exchange that the product uses (tagged words instead of barriers), for a
 // batch of sequences.  TEST INFRASTRUCTURE.
 //   run_draft_words <input blob> <output blob>
+//   run_draft_words <input blob> <output blob> words|copies <n>   in the first of two launches the last CTA's words, or copies of weights, are lost from the n-th on
 //   run_draft_words pieces           the attention's weights against the sum of their pieces
 // blob layout: see tests/test_draft_words_emu_cpu.py (the writer).
 #include "cuda_emu.h"
@@ -54,7 +55,8 @@ static int check_pieces() {
 
 int main(int argc, char** argv) {
   if (argc == 2 && std::string(argv[1]) == "pieces") return check_pieces();
-  if (argc != 3) return 2;
+  if (argc != 3 && argc != 5) return 2;
+  const bool lose = argc == 5;
   Reader r(argv[1]);
   const int B = r.i32(), d = r.i32(), L = r.i32(), H = r.i32(), KV = r.i32(), hd = r.i32(), ffn = r.i32(), vocab = r.i32();
   const int qk_norm = r.i32(), block_size = r.i32(), max_blocks = r.i32(), nslots = r.i32(), n_fwd = r.i32(), grid = r.i32(), max_pos = r.i32(), ring = r.i32(), max_chunk = r.i32();
@@ -104,7 +106,13 @@ int main(int argc, char** argv) {
   p.n_slots = ring; p.batch = B; p.max_chunk = max_chunk; p.slot_bytes = ssdk::ds_slot_bytes(max_chunk); p.words = words;
   for (int l = 0; l < L; ++l)
     p.layers[l] = ssdk::DsLayer{lw[l].w[0].data(), lw[l].w[1].data(), lw[l].w[2].data(), lw[l].w[3].data(), lw[l].w[4].data(), lw[l].w[5].data(), lw[l].w[6].data(), lw[l].w[7].data()};
+  unsigned gave_up = 0;
+  p.timeout = &gave_up;
   for (int rep = 0; rep < 2; ++rep) {   // a second launch finds the words and tags of the first
+    if (lose) {
+      ssdk::ds_wait_cycles = rep == 0 ? 1000000000LL : 4000000000000LL;   // half a second
+      (std::string(argv[3]) == "words" ? emu::lost_words : emu::lost_copies) = rep == 0 ? std::atoi(argv[4]) : -1;
+    }
     for (int b = 0; b < B; ++b) {
       std::fill(tok.begin() + (size_t)b * (n_fwd + 1), tok.begin() + (size_t)(b + 1) * (n_fwd + 1), -1);
       tok[(size_t)b * (n_fwd + 1)] = first[b];
@@ -112,6 +120,23 @@ int main(int argc, char** argv) {
 #define RUN(HD, T) emu::launch(ssdk::draft_stream_kernel<HD, T>, p, grid, ssdk::kDsThreads, smem)
     if (hd == 64) { if (MT == 1) RUN(64, 1); else if (MT == 4) RUN(64, 4); else RUN(64, 8); }
     else { if (MT == 1) RUN(128, 1); else if (MT == 4) RUN(128, 4); else RUN(128, 8); }
+    unsigned long long arrivals;
+    std::memcpy(&arrivals, sync, 8);
+    if (arrivals % (unsigned long long)grid != 0) {
+      std::cerr << "barrier arrival counter is not a whole number of barriers\n";
+      return 3;
+    }
+    if (gave_up != (lose && rep == 0 ? 1u : 0u)) {
+      std::cerr << (gave_up ? "a wait ran out\n" : "no wait ran out\n");
+      return 3;
+    }
+    gave_up = 0;
+    for (int b = 0; b < B; ++b)
+      for (int f = 1; f < n_fwd; ++f)
+        if (tok[(size_t)b * (n_fwd + 1) + f] < 0 || tok[(size_t)b * (n_fwd + 1) + f] >= vocab) {
+          std::cerr << "token out of range\n";
+          return 3;
+        }
   }
   std::ofstream o(argv[2], std::ios::binary);
   o.write(reinterpret_cast<const char*>(logits.data()), (std::streamsize)(logits.size() * 2));

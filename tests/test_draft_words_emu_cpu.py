@@ -32,7 +32,7 @@ def _u16(t):
     return t.contiguous().view(torch.int16).numpy().astype(np.uint16)
 
 
-def _check(tmp_path, hd, kv, grid, ffn, ctx, temp, chunk, bs=16, unnamed=(), binary=BIN):
+def _check(tmp_path, hd, kv, grid, ffn, ctx, temp, chunk, bs=16, unnamed=(), binary=BIN, lose=()):
     """One launch against the oracle.  unnamed: (sequence, entry) pairs of the page tables that name no page."""
     from oracle import verify as V
     _build(binary)
@@ -77,7 +77,7 @@ def _check(tmp_path, hd, kv, grid, ffn, ctx, temp, chunk, bs=16, unnamed=(), bin
             _u16(lw.get("k_norm", ones)).tofile(f)
         _u16(kv0[0]).tofile(f)
         _u16(kv0[1]).tofile(f)
-    res = subprocess.run([binary, str(blob), str(out)], capture_output=True, text=True, timeout=600)
+    res = subprocess.run([binary, str(blob), str(out), *lose], capture_output=True, text=True, timeout=600)
     assert res.returncode == 0, res.stderr[-2000:]
     raw = np.fromfile(out, dtype=np.uint16)
     nl, nc = B * n_fwd * cfg.vocab, cfg.layers * nblk * bs * kv * hd
@@ -134,3 +134,10 @@ def test_attention_weights_keep_all_their_bits():
     _build()
     res = subprocess.run([BIN, "pieces"], capture_output=True, text=True, timeout=60)
     assert res.returncode == 0, res.stderr[-500:]
+
+
+@pytest.mark.parametrize("lose", [("words", "0"), ("words", "700"), ("copies", "0"), ("copies", "60"), ("copies", "900")])
+def test_waits_that_run_out_end_the_launch(tmp_path, lose):
+    """What the last CTA sends, or the weights that it fetches, is lost on the way: every wait for it has a limit, the launch ends with its word set, and the next one is right (the
+    runner looks at the word, the barrier's count and the range of the tokens behind both)."""
+    _check(tmp_path, 64, 1, 2, 512, [40, 300], 0.7, 256, lose=lose)
