@@ -259,9 +259,9 @@ SSDK_DEVINL bool ds_feed(DsProducer& r, const DsGeom& g, const __nv_bfloat16* w,
       for (int i = 0; i < group; ++i) {
         const int t = t0 + i / sub * kDsTile, n = min(kDsTile, r1 - t);
         if (n <= 0) break;
-        int ok = 1;
+        int ok = 1;   // (consumers that have given up say so before they give a slot back: a slot whose last copy may be in flight is not asked for again)
         if (lane == 0) {
-          ok = ds_ring_wait(&r.empty[r.slot], r.phase ^ 1u, r.broken);  // a fresh barrier passes the first round at once
+          ok = ds_ring_wait(&r.empty[r.slot], r.phase ^ 1u, r.broken) && !*r.broken.dead;  // a fresh barrier passes the first round at once
           if (ok) mbar_arrive_expect_tx(&r.full[r.slot], (unsigned)(n * g.ck * 2));
         }
         if (!__shfl_sync(0xffffffffu, ok, 0)) return false;
@@ -350,7 +350,6 @@ struct DsRing {
   uint64_t *full, *empty;
   unsigned n_slots, slot_bytes, slot, phase;
   DsWait broken;
-  bool gone;   // this thread has given up a slot: it takes and gives back no more (a slot needs all warps to be given back, so that the producer stops too)
 };
 // x of a chunk, this thread's fragments, steps of 32 columns of the warp's ck / 8.  Five tokens and more: step j, columns 32 j + 8 (lane & 3) .. + 8 of token lane / 4.
 // Up to four: steps 2 j (lanes 0 .. 15) and 2 j + 1 (16 .. 31) of token (lane / 4) & 3.
@@ -392,7 +391,7 @@ SSDK_DEVINL void ds_slot(DsRing& ring, int steps, int at, int lane, const DsX<MT
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) c[i][e] = 0.f;
-  ring.gone = ring.gone || !ds_ring_wait(&ring.full[ring.slot], ring.phase, ring.broken);
+  ds_ring_wait(&ring.full[ring.slot], ring.phase, ring.broken);   // (given up: whatever lies there)
   const uint8_t* w = ring.base + (unsigned)(ring.slot * ring.slot_bytes + at);
   if (steps == 8) {
     ds_steps<MT, 8>(w, x.v, c);
@@ -412,7 +411,7 @@ SSDK_DEVINL void ds_slot(DsRing& ring, int steps, int at, int lane, const DsX<MT
     }
   }
   __syncwarp();
-  if (lane == 0 && !ring.gone) mbar_arrive(&ring.empty[ring.slot]);   // one arrive per consumer warp, after its last read
+  if (lane == 0) mbar_arrive(&ring.empty[ring.slot]);   // one arrive per consumer warp, after its last read
   if (++ring.slot == ring.n_slots) { ring.slot = 0; ring.phase ^= 1u; }
   float s[4];
 #pragma unroll
@@ -988,7 +987,7 @@ SSDK_DEVINL void ds_attention_merge(const DsParams& p, int b, int h, int s, int 
 }
 
 // ---------------------------------------------------------------------------------------------
-// the stages.  What they share is in shared memory.  `st`: ring slot | ring phase << 8 | ring given up << 9.
+// the stages.  What they share is in shared memory.  `st`: ring slot | ring phase << 8.
 // ---------------------------------------------------------------------------------------------
 struct DsShared {
   DsParams p;
@@ -1064,7 +1063,7 @@ SSDK_DEVINL unsigned ds_stage(int kind, int l, int f, uint32_t tag, unsigned st)
     smp.call_id = (S.p.dyn ? S.p.dyn[1] * 16ull : S.p.call_base) + (uint64_t)f;
     if (S.p.logits) smp.logits = S.p.logits + (size_t)f * S.p.logits_ld + (size_t)tok * S.p.logits_seq_ld;
   }
-  DsRing ring{ds_smem, S.full, S.empty, (unsigned)S.p.n_slots, S.slot_bytes, st & 0xffu, st >> 8 & 1u, DsWait{&S.broken, S.p.timeout}, st >> 9 != 0u};
+  DsRing ring{ds_smem, S.full, S.empty, (unsigned)S.p.n_slots, S.slot_bytes, st & 0xffu, st >> 8, DsWait{&S.broken, S.p.timeout}};
   ds_consume<MT>(ring, g, kind == DS_GU ? DS_GATED : (kind == DS_HEAD ? DS_LOGITS : DS_ROWS), M, reinterpret_cast<float*>(S.sums), out, tag, load, smp);
   ds_mark(f, 2 * kind + 1);
   if (kind == DS_HEAD) {   // eight threads of a warp per sequence -> per-CTA best
@@ -1084,7 +1083,7 @@ SSDK_DEVINL unsigned ds_stage(int kind, int l, int f, uint32_t tag, unsigned st)
       S.p.samp_partial[(size_t)tid * gridDim.x + blockIdx.x] = c;
     }
   }
-  return ring.slot | ring.phase << 8 | (ring.gone ? 1u : 0u) << 9;
+  return ring.slot | ring.phase << 8;
 }
 // B: units of this CTA (pass 0), their merges (pass 1: behind all units of a CTA, since a merge waits for units of other CTAs)
 template <int HD>
