@@ -87,9 +87,6 @@ struct DsParams {
   int skip_last_head;            // 1: the last forward runs without lm_head / sampling (it only writes KV)
   const int32_t* ctx0;           // [batch]: tokens in the cache before the first forward
   const int32_t* block_table;    // [batch][max_blocks]
-  // host emulation without `words` only: the vectors as plain bf16, stages meet at the device-wide barrier (one sequence)
-  __nv_bfloat16 *vec_qkv, *vec_attn, *vec_o, *vec_act, *vec_down, *resid0, *resid1;
-  float* attn_part;              // [H][kDsSplits][hd + 2]: o | m | l
   __nv_bfloat16* logits;         // row of sequence b and forward f at logits + b * logits_seq_ld + f * logits_ld (may be null: no logits kept)
   long long logits_ld;
   const float* temp;             // draft temperatures [batch] (device)
@@ -97,7 +94,6 @@ struct DsParams {
   uint64_t seed, call_base;      // used when dyn == nullptr: call_id = call_base + f
   ArgMax* samp_partial;          // [batch][#CTAs]
   unsigned* bar_state;           // one 64-bit arrival counter (8-byte aligned), only ever grows; zero before the first launch
-  unsigned* attn_ticket;         // (unused)
   int n_slots;                   // ring depth
   int batch;                     // sequences (0: one)
   int tok_ld;
@@ -106,6 +102,12 @@ struct DsParams {
   int slot_bytes;                // ring stride (0: that of kDsMaxChunk columns)
   uint32_t* words;               // ds_words() words: exchange of the stages
   unsigned* timeout;             // set when a bounded wait runs out
+#ifdef SSDK_HOST_EMU
+  // a test's second form, without `words`: the vectors as plain bf16, stages meet at the device-wide barrier (one sequence)
+  __nv_bfloat16 *vec_qkv, *vec_attn, *vec_o, *vec_act, *vec_down, *resid0, *resid1;
+  float* attn_part;              // [H][kDsSplits][hd + 2]: o | m | l
+  unsigned* attn_ticket;
+#endif
   DsLayer layers[kDsMaxLayers];
 };
 
@@ -298,28 +300,35 @@ SSDK_DEVINL void ds_producer(const DsParams& p, const DsGeom* geom, DsProducer& 
 // ---------------------------------------------------------------------------------------------
 struct DsVec {                // one stage's results: [batch][n]
   uint32_t* words;
-  __nv_bfloat16* plain;       // (host emulation without words)
   int n;
-};
 #ifdef SSDK_HOST_EMU
-#define DS_PLAIN(v) ((v).words == nullptr)
-#else
-#define DS_PLAIN(v) false
+  __nv_bfloat16* plain;       // without words
 #endif
+};
 SSDK_DEVINL void ds_put(const DsVec& v, int b, int i, uint32_t tag, float x) {
-  if (DS_PLAIN(v)) v.plain[(size_t)b * v.n + i] = f2bf(x);
-  else st_relaxed_gpu_u32(v.words + (size_t)b * v.n + i, (tag << 16) | ds_f_bits(x));
+#ifdef SSDK_HOST_EMU
+  if (!v.words) { v.plain[(size_t)b * v.n + i] = f2bf(x); return; }
+#endif
+  st_relaxed_gpu_u32(v.words + (size_t)b * v.n + i, (tag << 16) | ds_f_bits(x));
 }
 SSDK_DEVINL bool ds_tagged(const uint4& w, uint32_t tag) {
   return (w.x >> 16) == tag && (w.y >> 16) == tag && (w.z >> 16) == tag && (w.w >> 16) == tag;
 }
 SSDK_DEVINL uint2 ds_pack4(const uint4& w) { return make_uint2(__byte_perm(w.x, w.y, 0x5410), __byte_perm(w.z, w.w, 0x5410)); }
-// four consecutive words of sequence b, at i (the tag is the one that is waited for: host emulation without words)
+// four consecutive words of sequence b, at i; one (the tag is the one that is waited for: host emulation without words)
+SSDK_DEVINL uint32_t ds_ask_one(const DsVec& v, size_t at, uint32_t tag) {
+#ifdef SSDK_HOST_EMU
+  if (!v.words) return tag << 16 | ds_f_bits(bf2f(v.plain[at]));
+#endif
+  return ld_relaxed_gpu_u32(v.words + at);
+}
 SSDK_DEVINL uint4 ds_ask(const DsVec& v, int b, int i, uint32_t tag) {
-  if (DS_PLAIN(v)) {
-    const __nv_bfloat16* s = v.plain + (size_t)b * v.n + i;
-    return make_uint4(tag << 16 | ds_f_bits(bf2f(s[0])), tag << 16 | ds_f_bits(bf2f(s[1])), tag << 16 | ds_f_bits(bf2f(s[2])), tag << 16 | ds_f_bits(bf2f(s[3])));
+#ifdef SSDK_HOST_EMU
+  if (!v.words) {
+    const size_t at = (size_t)b * v.n + i;
+    return make_uint4(ds_ask_one(v, at, tag), ds_ask_one(v, at + 1, tag), ds_ask_one(v, at + 2, tag), ds_ask_one(v, at + 3, tag));
   }
+#endif
   return ld_relaxed_gpu_v4(v.words + (size_t)b * v.n + i);
 }
 // waits until every piece of r carries the tag: all that are missing are asked for again at once (one after another costs a trip to L2 each: 5 us per norm of four tokens)
@@ -724,15 +733,21 @@ SSDK_DEVINL uint32_t ds_word(const uint4& v, int i) { return i == 0 ? v.x : (i =
 
 struct DsPartial {            // partial results of the splits: per sequence, head and split hd sums, maximum, sum of weights
   unsigned long long* words;  // {fp32, tag}
-  float* plain;               // (host emulation without words)
   int most;                   // splits that there is room for
+#ifdef SSDK_HOST_EMU
+  float* plain;               // without words
+#endif
 };
 SSDK_DEVINL void ds_put_part(const DsPartial& q, size_t i, uint32_t tag, float x) {
+#ifdef SSDK_HOST_EMU
   if (!q.words) { q.plain[i] = x; return; }
+#endif
   st_relaxed_gpu_u64(q.words + i, ((unsigned long long)tag << 32) | *reinterpret_cast<const uint32_t*>(&x));
 }
 SSDK_DEVINL unsigned long long ds_ask_part(const DsPartial& q, size_t i, uint32_t tag) {
+#ifdef SSDK_HOST_EMU
   if (!q.words) return ((unsigned long long)tag << 32) | *reinterpret_cast<const uint32_t*>(q.plain + i);
+#endif
   return ld_relaxed_gpu_u64(q.words + i);
 }
 SSDK_DEVINL float ds_part_value(unsigned long long w) {
@@ -774,24 +789,19 @@ SSDK_DEVINL void ds_attention_unit(const DsParams& p, int layer, int b, int h, i
       c[t] = cs[i]; sn[t] = cs[HALF + i];
       n1[t] = nw ? bf2f(nw[i]) : 1.f; n2[t] = nw ? bf2f(nw[HALF + i]) : 1.f;
     }
-    if (DS_PLAIN(qkv)) {
+    const size_t src = (size_t)b * qkv.n + col0 + lane;
+    const long long w0 = clock64();
+    bool ok;
+    do {
+      ok = true;
 #pragma unroll
-      for (int t = 0; t < PT; ++t) { x1[t] = bf2f(qkv.plain[(size_t)b * qkv.n + col0 + lane + 32 * t]); x2[t] = bf2f(qkv.plain[(size_t)b * qkv.n + col0 + HALF + lane + 32 * t]); }
-    } else {
-      const uint32_t* src = qkv.words + (size_t)b * qkv.n + col0 + lane;
-      const long long w0 = clock64();
-      bool ok;
-      do {
-        ok = true;
-#pragma unroll
-        for (int t = 0; t < PT; ++t) {
-          const uint32_t u1 = ld_relaxed_gpu_u32(src + 32 * t), u2 = ld_relaxed_gpu_u32(src + HALF + 32 * t);
-          ok = ok && (u1 >> 16) == tag && (u2 >> 16) == tag;
-          x1[t] = ds_bits_f(u1); x2[t] = ds_bits_f(u2);
-        }
-      } while (!ok && !wait.give_up(w0));
-      __syncwarp();
-    }
+      for (int t = 0; t < PT; ++t) {
+        const uint32_t u1 = ds_ask_one(qkv, src + 32 * t, tag), u2 = ds_ask_one(qkv, src + HALF + 32 * t, tag);
+        ok = ok && (u1 >> 16) == tag && (u2 >> 16) == tag;
+        x1[t] = ds_bits_f(u1 & 0xffffu); x2[t] = ds_bits_f(u2 & 0xffffu);
+      }
+    } while (!ok && !wait.give_up(w0));
+    __syncwarp();
     if (nw) {
       float ss = 0.f;
 #pragma unroll
@@ -1133,16 +1143,22 @@ __global__ void __launch_bounds__(kDsThreads, 1) draft_stream_kernel(const __gri
     S.shift = -1;
     for (int i = 0; i < 20; ++i)
       if (p.block_size == (1 << i)) S.shift = i;
-    S.vec[DS_VQKV] = DsVec{p.words, p.vec_qkv, (p.H + 2 * p.KV) * HD};
-    S.vec[DS_VATTN] = DsVec{nullptr, p.vec_attn, p.H * HD};
-    S.vec[DS_VO] = DsVec{nullptr, p.vec_o, p.d};
-    S.vec[DS_VACT] = DsVec{nullptr, p.vec_act, p.ffn};
-    S.vec[DS_VDOWN] = DsVec{nullptr, p.vec_down, p.d};
-    S.part = DsPartial{nullptr, p.attn_part, p.words ? ds_max_splits(M, p.KV, (int)gridDim.x) : kDsSplits};
-    if (p.words) {
-      for (int i = 1; i < 5; ++i) S.vec[i].words = S.vec[i - 1].words + (size_t)M * S.vec[i - 1].n;
-      S.part.words = reinterpret_cast<unsigned long long*>(S.vec[4].words + (size_t)M * S.vec[4].n);
+    const int rows[5] = {(p.H + 2 * p.KV) * HD, p.H * HD, p.d, p.ffn, p.d};   // DS_VQKV ..
+    uint32_t* words = p.words;
+    for (int i = 0; i < 5; ++i) {
+      S.vec[i].words = words;
+      S.vec[i].n = rows[i];
+      words += (size_t)M * rows[i];
     }
+    S.part.words = reinterpret_cast<unsigned long long*>(words);
+    S.part.most = ds_max_splits(M, p.KV, (int)gridDim.x);
+#ifdef SSDK_HOST_EMU
+    if (!p.words) {
+      __nv_bfloat16* const plain[5] = {p.vec_qkv, p.vec_attn, p.vec_o, p.vec_act, p.vec_down};
+      for (int i = 0; i < 5; ++i) { S.vec[i].words = nullptr; S.vec[i].plain = plain[i]; }
+      S.part.words = nullptr; S.part.plain = p.attn_part; S.part.most = kDsSplits;
+    }
+#endif
     for (int s = 0; s < p.n_slots; ++s) {
       mbar_init(&S.full[s], 1);           // the producer's arrive.expect_tx + the copies' transaction bytes
       mbar_init(&S.empty[s], kDsWarps);   // one arrive per consumer warp
@@ -1167,7 +1183,10 @@ __global__ void __launch_bounds__(kDsThreads, 1) draft_stream_kernel(const __gri
   bar.counter = reinterpret_cast<unsigned long long*>(p.bar_state);
   bar.target = 0;
   bar.init();
-  if (p.words) {
+#ifdef SSDK_HOST_EMU
+  if (p.words)
+#endif
+  {
     const long long n = ds_words(M, p.d, p.H, p.KV, HD, p.ffn, (int)gridDim.x) / 4;   // (vectors of whole 8 words, partial results of whole four)
     for (long long i = (long long)blockIdx.x * kDsConsumers + threadIdx.x; i < n; i += (long long)gridDim.x * kDsConsumers)
       reinterpret_cast<uint4*>(p.words)[i] = make_uint4(0u, 0u, 0u, 0u);
