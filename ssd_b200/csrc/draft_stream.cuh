@@ -85,6 +85,7 @@ struct DsParams {
   int64_t* tok_buf;              // sequence b at tok_buf + b * tok_ld: [n_fwd (+1)]: [0] = first input token; the kernel writes [f + 1]
   int n_fwd;                     // forwards in this launch
   int skip_last_head;            // 1: the last forward runs without lm_head / sampling (it only writes KV)
+  int logits_only;               // 1: nobody reads tokens (one forward, whose logits another kernel samples)
   const int32_t* ctx0;           // [batch]: tokens in the cache before the first forward
   const int32_t* block_table;    // [batch][max_blocks]
   __nv_bfloat16* logits;         // row of sequence b and forward f at logits + b * logits_seq_ld + f * logits_ld (may be null: no logits kept)
@@ -1076,7 +1077,7 @@ SSDK_DEVINL unsigned ds_stage(int kind, int l, int f, uint32_t tag, unsigned st)
   DsRing ring{ds_smem, S.full, S.empty, (unsigned)S.p.n_slots, S.slot_bytes, st & 0xffu, st >> 8, DsWait{&S.broken, S.p.timeout}};
   ds_consume<MT>(ring, g, kind == DS_GU ? DS_GATED : (kind == DS_HEAD ? DS_LOGITS : DS_ROWS), M, reinterpret_cast<float*>(S.sums), out, tag, load, smp);
   ds_mark(f, 2 * kind + 1);
-  if (kind == DS_HEAD) {   // eight threads of a warp per sequence -> per-CTA best
+  if (kind == DS_HEAD && !S.p.logits_only) {   // eight threads of a warp per sequence -> per-CTA best
     ArgMax a = smp.best;
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) {
@@ -1217,7 +1218,7 @@ __global__ void __launch_bounds__(kDsThreads, 1) draft_stream_kernel(const __gri
       st = ds_stage<MT>(kind, l, f, tag, st);
       if (kind != DS_HEAD) meet();
     }
-    if (!ds_has_head(p, f)) break;
+    if (!ds_has_head(p, f) || p.logits_only) break;
     bar.sync(wait);
     if ((int)(threadIdx.x >> 5) < M) {   // device-wide reduction: every CTA learns the tokens
       const int b = threadIdx.x >> 5;

@@ -1226,8 +1226,8 @@ static int launch_draft_stream(Launcher& L, const DsParams& p, size_t smem) {
   ++L.count;
   return 0;
 }
-// forwards 0 .. n_fwd-1 of a model on tok_buf[0 ..] of every sequence; samples tok_buf[f + 1] after every forward but (optionally) the last
-static int enqueue_draft_stream(ssdk_engine* e, Launcher& L, int which, int B, int64_t* tok_buf, int tok_ld, int n_fwd, bool skip_last_head,
+// forwards 0 .. n_fwd-1 of a model on tok_buf[0 ..] of every sequence; samples tok_buf[f + 1] after every forward but (optionally) the last; or (logits_only) one forward that leaves its logits
+static int enqueue_draft_stream(ssdk_engine* e, Launcher& L, int which, int B, int64_t* tok_buf, int tok_ld, int n_fwd, bool skip_last_head, bool logits_only,
                                 const int32_t* ctx0, const int32_t* block_table, const float* temp, const uint64_t* dyn,
                                 bf16* logits, int64_t logits_ld, int64_t logits_seq_ld) {
   Model& m = e->model[which];
@@ -1241,7 +1241,7 @@ static int enqueue_draft_stream(ssdk_engine* e, Launcher& L, int which, int B, i
   p.k_cache = m.k_cache; p.v_cache = m.v_cache;
   p.cache_layer_stride = (long long)m.num_blocks * e->rt.block_size * m.KV * m.hd;
   p.block_size = e->rt.block_size; p.max_blocks = e->rt.max_blocks_per_seq;
-  p.tok_buf = tok_buf; p.n_fwd = n_fwd; p.skip_last_head = skip_last_head ? 1 : 0;
+  p.tok_buf = tok_buf; p.n_fwd = n_fwd; p.skip_last_head = skip_last_head ? 1 : 0; p.logits_only = logits_only ? 1 : 0;
   p.ctx0 = ctx0; p.block_table = block_table;
   p.batch = B; p.tok_ld = tok_ld; p.logits_seq_ld = logits_seq_ld;
   p.logits = logits; p.logits_ld = logits_ld;
@@ -1285,7 +1285,7 @@ static int enqueue_spec_step(ssdk_engine* e, Launcher& L, int B, bool host_io, b
   if (tp_rank == 0 && !drf.present) return fail("rank 0 needs the draft model");
   if (drf.present) CKI(L.go(init_tokens_kernel, dim3(1), dim3(64), 0, (const int64_t*)rec_in, w.tok_buf, B, K + 1));
   if (stream_draft)
-    CKI(enqueue_draft_stream(e, L, SSDK_DRAFT, B, w.tok_buf, K + 1, K + 1, true, ctx, btd, tq, seed_step, w.logits_q, (int64_t)V, (int64_t)K * V));
+    CKI(enqueue_draft_stream(e, L, SSDK_DRAFT, B, w.tok_buf, K + 1, K + 1, true, false, ctx, btd, tq, seed_step, w.logits_q, (int64_t)V, (int64_t)K * V));
   for (int k = 0; k <= K && drf.present && !stream_draft; ++k) {
     Fwd f;
     f.which = SSDK_DRAFT; f.B = B; f.Q = 1; f.ids = w.tok_buf + k; f.ids_stride = K + 1;
@@ -1806,8 +1806,8 @@ static int forward_rows(ssdk_handle h, int which, int batch, int q_len, const in
   f.logits_mode = want_sample ? 2 : 0;
   f.logits_out = w.logits_last;
   f.logits_ld = m.cfg.vocab;
-  if (stream_decode(h, m, batch, q_len, ctx_len))   // (its own choice, the best logit, goes behind each token that it has read: ids_in is written anew by every call)
-    CKI(enqueue_draft_stream(h, L, which, batch, w.ids_in, 1, 1, !want_sample, f.ctx0, f.block_tables, nullptr, nullptr, want_sample ? w.logits_last : nullptr, 0, m.cfg.vocab));
+  if (stream_decode(h, m, batch, q_len, ctx_len))
+    CKI(enqueue_draft_stream(h, L, which, batch, w.ids_in, 1, 1, !want_sample, true, f.ctx0, f.block_tables, nullptr, nullptr, want_sample ? w.logits_last : nullptr, 0, m.cfg.vocab));
   else
     CKI(enqueue_forward(h, L, f));
   const bool do_sample = want_sample && m.cfg.tp_rank == 0;
