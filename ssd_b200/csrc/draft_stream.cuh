@@ -671,52 +671,39 @@ struct DsPages {
   }
   SSDK_DEVINL size_t slot(int t, int page) const { return (size_t)page * block_size + (shift >= 0 ? t & (block_size - 1) : t % block_size); }
 };
-// Keys and values of tokens without a page are zeros, as in paged_attn_kernel: they are read from here (a flag or a bit per key next to the loads in flight spills: with heads of 128
-// 212 bytes -> 536 and more).
+// Keys tb .. tb + 32 of a warp.  Every lane looks one of them up and the loads take its row from there.  Keys behind the range and the new one (pos) are zero; whoever has none reads an
+// earlier key, so that no load waits for a branch (1.2 us to get sixteen loads under way with one).  Tokens without a page count as zeros, as in paged_attn_kernel: they are read from
+// ds_no_page (a flag or a bit per key next to the loads in flight spills: with heads of 128 212 bytes -> 536 and more).
 __device__ uint4 ds_no_page[16];
-// Keys tb .. tb + 32 of a warp: tb is a multiple of 32, so that with pages of whole 32 one page holds them.  Keys behind the range and the new one (pos) are zero; whoever has
-// none reads an earlier key, so that no load waits for a branch (1.2 us to get sixteen loads under way with one).
-struct DsRows {
-  const __nv_bfloat16* row;   // of the first of 32 keys, or of every cache's first row: keys look for their own pages
-  const DsPages& pg;
-  int ld, from;
-  bool whole;                 // one page holds them
-  SSDK_DEVINL DsRows(const __nv_bfloat16* base, const DsPages& g, int stride, int first) : row(base), pg(g), ld(stride), from(first), whole(g.block_size % 32 == 0) {
-    if (whole) {
-      const int page = pg.page(from);
-      row = page < 0 ? reinterpret_cast<const __nv_bfloat16*>(ds_no_page) : base + pg.slot(from, page) * ld;
-      if (page < 0) ld = 0;
-    }
-  }
-  SSDK_DEVINL const __nv_bfloat16* at(int t) const {
-    if (whole) return row + (t - from) * ld;
-    const int page = pg.page(t);
-    return page < 0 ? reinterpret_cast<const __nv_bfloat16*>(ds_no_page) : row + pg.slot(t, page) * ld;
-  }
-};
+constexpr uint32_t kDsNoSlot = 0xffffffffu;   // (a cache of that many rows is larger than the memory)
+SSDK_DEVINL uint32_t ds_slots(const DsPages& pg, int lane, int tb, int t1, int pos) {
+  const int t = min(tb + lane, max(min(t1, pos) - 1, 0));   // (at most the last key that is in the cache; none: the new one's slot, not used)
+  const int page = pg.page(t);
+  return page < 0 ? kDsNoSlot : (uint32_t)pg.slot(t, page);
+}
+SSDK_DEVINL const __nv_bfloat16* ds_key_row(const __nv_bfloat16* base, uint32_t slots, int key, int ld) {
+  const uint32_t slot = __shfl_sync(0xffffffffu, slots, key);
+  return slot == kDsNoSlot ? reinterpret_cast<const __nv_bfloat16*>(ds_no_page) : base + (size_t)slot * ld;
+}
 SSDK_DEVINL uint4 ds_keep(const uint4& v, bool on) { return make_uint4(on ? v.x : 0u, on ? v.y : 0u, on ? v.z : 0u, on ? v.w : 0u); }
 // keys tb + 8 j + lane / 4, dims 32 k + 8 (lane & 3) .. + 8
 template <int HD>
-SSDK_DEVINL void ds_load_k(const __nv_bfloat16* base, const DsPages& pg, int ld, int lane, int tb, int t1, int pos, uint4 (&k)[4][HD / 32]) {
-  const int most = max(min(t1, pos) - 1, 0);   // (the last key that is in the cache; none: the new one's slot, not used)
-  const DsRows rows(base, pg, ld, min(tb, most));
+SSDK_DEVINL void ds_load_k(const __nv_bfloat16* base, uint32_t slots, int ld, int lane, uint4 (&k)[4][HD / 32]) {
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const __nv_bfloat16* s = rows.at(min(tb + 8 * j + (lane >> 2), most)) + 8 * (lane & 3);
+    const __nv_bfloat16* s = ds_key_row(base, slots, 8 * j + (lane >> 2), ld) + 8 * (lane & 3);
 #pragma unroll
     for (int i = 0; i < HD / 32; ++i) k[j][i] = ds_ldcg16(s + 32 * i);
   }
 }
 // value rows tb + 16 kk + {2q, 2q + 1, 2q + 8, 2q + 9} (q = lane & 3), dims 64 i + 8 (lane / 4) .. + 8
 template <int HD>
-SSDK_DEVINL void ds_load_v(const __nv_bfloat16* base, const DsPages& pg, int ld, int lane, int tb, int t1, int pos, uint4 (&v)[2][4][HD / 64]) {
-  const int most = max(min(t1, pos) - 1, 0);
-  const DsRows rows(base, pg, ld, min(tb, most));
+SSDK_DEVINL void ds_load_v(const __nv_bfloat16* base, uint32_t slots, int ld, int lane, uint4 (&v)[2][4][HD / 64]) {
 #pragma unroll
   for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const __nv_bfloat16* s = rows.at(min(tb + 16 * kk + 2 * (lane & 3) + (j & 1) + 8 * (j >> 1), most)) + 8 * (lane >> 2);
+      const __nv_bfloat16* s = ds_key_row(base, slots, 16 * kk + 2 * (lane & 3) + (j & 1) + 8 * (j >> 1), ld) + 8 * (lane >> 2);
 #pragma unroll
       for (int i = 0; i < HD / 64; ++i) v[kk][j][i] = ds_ldcg16(s + 64 * i);
     }
@@ -774,8 +761,11 @@ SSDK_DEVINL void ds_attention_unit(const DsParams& p, int layer, int b, int h, i
   __nv_bfloat16* vbase = p.v_cache + (size_t)layer * p.cache_layer_stride + (size_t)h * HD;
   uint4 kf[4][KB], vf[2][4][HD / 64];
   int tb = t0 + warp * 32;
-  ds_load_k<HD>(kbase, pg, ld, lane, tb, t1, pos, kf);
-  ds_load_v<HD>(vbase, pg, ld, lane, tb, t1, pos, vf);
+  uint32_t slots = ds_slots(pg, lane, tb, t1, pos);
+  ds_load_k<HD>(kbase, slots, ld, lane, kf);
+  ds_load_v<HD>(vbase, slots, ld, lane, vf);
+
+  const int new_page = pg.page(pos);   // (in front of the wait)
 
   // ---- q rows, k, v: one warp per row, rotate-half pairs (i, i + HALF) ----
   const float* cs = p.rope + (size_t)pos * HD;
@@ -812,7 +802,7 @@ SSDK_DEVINL void ds_attention_unit(const DsParams& p, int layer, int b, int h, i
 #pragma unroll
       for (int t = 0; t < PT; ++t) { x1[t] = bf16_round(x1[t] * rstd * n1[t]); x2[t] = bf16_round(x2[t] * rstd * n2[t]); }
     }
-    if (kind > 0 && pg.page(pos) < 0) {   // a new token without a page counts like any other
+    if (kind > 0 && new_page < 0) {   // a new token without a page counts like any other
 #pragma unroll
       for (int t = 0; t < PT; ++t) x1[t] = x2[t] = 0.f;
     }
@@ -832,13 +822,10 @@ SSDK_DEVINL void ds_attention_unit(const DsParams& p, int layer, int b, int h, i
   ds_sync();
 
   // ---- KV store of the new token (one unit per kv head) ----
-  if (s == 0 && tid < HD / 4) {
-    const int page = pg.page(pos);
-    if (page >= 0) {
-      const int e = tid % (HD / 8) * 8;
-      const bool val = tid >= HD / 8;
-      *reinterpret_cast<uint4*>((val ? vbase : kbase) + pg.slot(pos, page) * ld + e) = *reinterpret_cast<const uint4*>((val ? sv : sk) + e);
-    }
+  if (s == 0 && tid < HD / 4 && new_page >= 0) {
+    const int e = tid % (HD / 8) * 8;
+    const bool val = tid >= HD / 8;
+    *reinterpret_cast<uint4*>((val ? vbase : kbase) + pg.slot(pos, new_page) * ld + e) = *reinterpret_cast<const uint4*>((val ? sv : sk) + e);
   }
 
   uint4 qf[KB];
@@ -877,7 +864,10 @@ SSDK_DEVINL void ds_attention_unit(const DsParams& p, int layer, int b, int h, i
         mma_bf16_16816(sc[j], a1, kf[j][i].z, kf[j][i].w);
       }
     }
-    if (more) ds_load_k<HD>(kbase, pg, ld, lane, tb + kDsUnitKeys, t1, pos, kf);
+    if (more) {
+      slots = ds_slots(pg, lane, tb + kDsUnitKeys, t1, pos);
+      ds_load_k<HD>(kbase, slots, ld, lane, kf);
+    }
     float mn = m;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
@@ -914,7 +904,7 @@ SSDK_DEVINL void ds_attention_unit(const DsParams& p, int layer, int b, int h, i
           for (int q = 0; q < 3; ++q) mma_bf16_16816(o[4 * i + d], a, w[0][q], w[1][q]);
         }
     }
-    if (more) ds_load_v<HD>(vbase, pg, ld, lane, tb + kDsUnitKeys, t1, pos, vf);
+    if (more) ds_load_v<HD>(vbase, slots, ld, lane, vf);
   }
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
