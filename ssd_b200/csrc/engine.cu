@@ -510,8 +510,12 @@ static void derive(Model& m) {
 // ---- streaming draft kernel: which models and batches it serves, and with what shared memory ----
 constexpr int kMaxDynSmem = 227 * 1024 - (int)sizeof(DsShared) - 256;  // opt-in limit per CTA minus the kernel's static shared memory
 static int ds_tokens(int B) { return B == 1 ? 1 : (B <= 4 ? 4 : 8); }   // the kernel's instances
-// slots of up to 2048 columns; narrow models: 1024 (twice as many slots in the same room, and no half-empty ones)
-static int ds_max_chunk(const Model& m) { return m.d <= 1024 ? 1024 : kDsMaxChunk; }
+// slots of up to 2048 columns; narrow models: 1024 (twice as many slots in the same room, and no half-empty ones) where four of them hold every row
+static bool ds_rows_fit(const Model& m, int max_chunk) {
+  DsGeom g;
+  return ds_geometry(m.d, m.qkv_dim, max_chunk, &g) && ds_geometry(m.H * m.hd, m.d, max_chunk, &g) && ds_geometry(m.ffn, m.d, max_chunk, &g);
+}
+static int ds_max_chunk(const Model& m) { return m.d <= 1024 && ds_rows_fit(m, 1024) ? 1024 : kDsMaxChunk; }
 static size_t ds_fixed_smem(const Model& m, int B) {
   const int MT = ds_tokens(B);
   size_t scratch = std::max((size_t)B * (2 * m.d + kDsPad), ds_attn_bytes(m.H / m.KV, m.hd));
@@ -525,12 +529,11 @@ static int ds_ring_slots(const Model& m, int B) {
   return fixed > (size_t)kMaxDynSmem ? 0 : (int)std::min<size_t>(kDsMaxSlots, ((size_t)kMaxDynSmem - fixed) / slot);
 }
 static bool draft_stream_supported(const Model& m, int B) {
-  const int G = m.KV ? m.H / m.KV : 0, mc = ds_max_chunk(m);
-  DsGeom g;
+  const int G = m.KV ? m.H / m.KV : 0;
   // (a row of every matrix on every CTA is what makes the exchange without barriers sound, see draft_stream.cuh)
   return B >= 1 && B <= kDsMaxBatch && m.cfg.tp_size == 1 && m.cfg.layers <= kDsMaxLayers && (m.hd == 64 || m.hd == 128) && G >= 1 && G <= 8 &&
          m.H % m.KV == 0 && m.KV <= 32 && m.d <= 8 * kDsConsumers && m.d >= num_sms() && m.ffn >= num_sms() && m.cfg.vocab >= num_sms() &&
-         ds_geometry(m.d, m.qkv_dim, mc, &g) && ds_geometry(m.H * m.hd, m.d, mc, &g) && ds_geometry(m.ffn, m.d, mc, &g) && ds_ring_slots(m, B) >= 4;
+         ds_rows_fit(m, ds_max_chunk(m)) && ds_ring_slots(m, B) >= 4;
 }
 
 // workspace carve-up (pass base = nullptr to measure)
