@@ -1187,29 +1187,50 @@ static bool draft_stream_enabled() {
   if (v < 0) v = env_int("SSDK_DRAFT_STREAM", 1) != 0 ? 1 : 0;
   return v == 1;
 }
-// Which draft path a step takes (both compute the same step; ctx_bound = the longest context of the batch before it).  Steps of k = 4 with two target layers, us, kernels per op -> streaming kernel:
-//   1B draft (16 layers, d = 2048): 1 sequence of 200, 900, 2000, 8000 tokens 4364 -> 3101, 4444 -> 3339, 4565 -> 3500, 4827 -> 3982; 2 of 500, 2000 4512 -> 4072, 4688 -> 4434;
-//     4 of 200, 2000 4699 -> 3821, 5005 -> 4451; 5 of 500, 900, 1500 4735 -> 4437, 4861 -> 4696, 4910 -> 4796; 8 of 200, 500, 900 4872 -> 4631, 4964 -> 4836, 5056 -> 5122
-//   0.6B draft (28 layers, d = 1024, heads of 128): 1 of 60, 200, 500, 900 4439 -> 3988, 4484 -> 4136, 4512 -> 4738, 4723 -> 4708; 2, 4, 8 of 200 4652 -> 5777, 4719 -> 5850, 5047 -> 7595
-// Wide models stream their weights for most of a layer, so that what the kernel saves between stages counts; its attention, a few CTAs per sequence, costs more per key, which
-// bounds the keys of a call (more than four sequences: half of the tokens' fragments come from other CTAs' words one chunk at a time, and the line lies lower).  Narrow ones are all exchange, and from two sequences on every CTA reads more words than the weights it multiplies.
-// SSDK_DRAFT_STREAM_MAX_CTX replaces the rule by a bound on the context alone.
-static int64_t stream_keys(int B) { return B > 4 ? 5120 : 8192; }   // of all sequences
+// Which calls take the streaming kernel (both forms compute the same; they differ in the order of sums).  A model has a number of tokens per sequence up to which it does.  One sequence: its own tokens
+// decide.  More: the page table's capacity, never the contexts of the moment, so that lengths of the neighbours do not move a sequence's result (their number may, as everywhere).
+// What decides is the bytes of a layer's weights, under which the kernel hides its exchange; the keys, of which a few CTAs per sequence fetch more slowly than paged_attn_kernel; and from five
+// sequences on that half of the tokens' fragments come from other CTAs' words one chunk at a time.  Steps of k = 4 with a target of one small layer, us, kernels per op -> streaming kernel, sequences x tokens
+// (drafts of 16 layers; MiB of a layer, width, size of a head):
+//   116, 2048, 64: 1 x 200, 2000, 8000 3964 -> 2582, 4256 -> 2836, 4445 -> 3392; 2 x 500, 2000, 4000 4099 -> 3518, 4302 -> 3725, 4435 -> 4109; 3 x 500, 4000 4213 -> 3375, 4644 -> 4111;
+//     4 x 200, 2000, 4000 4307 -> 3349, 4601 -> 3876, 4813 -> 4279; 5 x 200, 750 4298 -> 3897, 4353 -> 4188; 6 x 650 4399 -> 4177; 8 x 200, 500 4414 -> 4211, 4486 -> 4428
+//   88, 1792, 64: 1 x 8000 4997 -> 3504; 2 x 500, 4000 4760 -> 3967, 5016 -> 4418; 4 x 500, 4000 4953 -> 3779, 5278 -> 4339; 5 x 500 4025 -> 4269 (seven steps a slot)
+//   68, 2048, 64: 1 x 200 3595 -> 2093; 2 x 500, 4000 3676 -> 2941, 3993 -> 3448; 4 x 500, 4000 3833 -> 2858, 4299 -> 3680; 8 x 500 3921 -> 3689
+//   44, 2048, 64: 1 x 200, 8000 2608 -> 1938, 3013 -> 2698; 2 x 500 2712 -> 2687; 4 x 500 2765 -> 2767; 5 x 750 3485 -> 2966; 8 x 500 3635 -> 3169
+//   48, 1536, 64: 1 x 200, 8000 2691 -> 2206, 3199 -> 2982; 2 x 500 2827 -> 3043; 4 x 200 2892 -> 2847.  45, 1280, 64: 1 x 200, 3000, 8000 2716 -> 2489, 2936 -> 2793, 3159 -> 3232; 2 x 200 2761 -> 3496; 4 x 200 2854 -> 3427
+//   96, 2048, 128: 1 x 200, 8000 4487 -> 2668, 5146 -> 3837; 2 x 500, 4000 4599 -> 3730, 5085 -> 4602; 4 x 200, 2000, 4000 4697 -> 3564, 5157 -> 4471, 5513 -> 5558; 5 x 200 4050 -> 4179
+//   68, 2048, 128: 2 x 500, 2000, 4000 3755 -> 3339, 4056 -> 3574, 4251 -> 4323; 4 x 500, 2000, 3000 3943 -> 3459, 4283 -> 4129, 4495 -> 4678
+//   narrow, 28 layers: 30, 1024, 128 (0.6B): 1 x 60, 200, 500, 900 3798 -> 3419, 3837 -> 3555, 3867 -> 3796, 4036 -> 3998; 2 x 200 3964 -> 4984.  24, 1024, 64: 1 x 200, 900, 2000 3639 -> 2925, 3824 -> 3207, 3998 -> 3543.
+//     12 layers of 8, 512, 64: 1 x 200, 900 1462 -> 1401, 1522 -> 1522
+// Small layers of a few sequences lose; models of up to four of them keep the form all the same (two layers of 45 MiB, 2 x 200: 651 -> 833): it is where its batches are held against the oracle.
+// SSDK_DRAFT_STREAM_MAX_CTX replaces the rule for drafts by a bound on the longest context alone.
+static int64_t stream_tokens(const Model& m, int B) {
+  const int64_t layer = ((int64_t)m.qkv_dim * m.d + (int64_t)m.H * m.hd * m.d + 3ll * m.ffn * m.d) * 2, MiB = 1 << 20;   // bytes of weights
+  if (B == 1) return m.d > 1024 ? (layer >= 64 * MiB ? 8192 : 6144) : (m.hd == 128 ? 256 : 1024);
+  if (m.d <= 1024) return 0;
+  if (B > 4 && m.hd == 64 && m.d == 8 * kDsConsumers) return 4096 / B;
+  if (layer < 64 * MiB) return m.cfg.layers > 4 ? 0 : (B > 4 ? 512 : 1024);
+  if (B > 4) return 0;
+  return m.hd == 64 || layer >= 96 * MiB ? 4096 : 2048;
+}
+// tokens: the longest sequence's behind the call
+static bool stream_pays(ssdk_engine* e, const Model& m, int B, int64_t tokens) {
+  return (B == 1 ? tokens : (int64_t)e->rt.max_blocks_per_seq * e->rt.block_size) <= stream_tokens(m, B);
+}
 static bool use_draft_stream(ssdk_engine* e, int B, int ctx_bound) {
   const Model& m = e->model[SSDK_DRAFT];
   if (!m.present || !draft_stream_enabled() || !draft_stream_supported(m, B)) return false;
-  const int keys = ctx_bound + e->rt.spec_k + 1;
+  const int tokens = ctx_bound + e->rt.spec_k + 1;
   static const int forced = env_int("SSDK_DRAFT_STREAM_MAX_CTX", -1);
-  if (forced >= 0) return keys <= forced;
-  if (m.d > 1024) return (int64_t)B * keys <= stream_keys(B);
-  return B == 1 && keys <= (m.hd == 128 ? 256 : 1024);
+  return forced >= 0 ? tokens <= forced : stream_pays(e, m, B, tokens);
 }
-// One token per sequence of plain decoding, for the wide models of the rule above: a forward is one launch instead of eight per layer, and no graph.  1B model, 16 layers, us a call with its token:
-//   1 sequence of 200, 2000, 7000 tokens 898 -> 626, 938 -> 699, 990 -> 807; 2 of 200, 4000 924 -> 792, 998 -> 980; 4 of 200, 2000 959 -> 766, 1023 -> 926; 8 of 200 986 -> 917;
-//   two layers of it: 1, 4, 8 of 200 279 -> 248, 268 -> 255, 280 -> 285 (the launch itself, its first barrier and the words of eight tokens: more than four sequences from four layers on)
+// One token per sequence of plain decoding, by the same numbers: a forward is one launch instead of nine per layer, and no graph.  The 1B model (116 MiB), us a call with its token:
+//   16 layers: 1 x 200, 2000, 7000 852 -> 571, 890 -> 624, 940 -> 721; 2 x 200, 4000 873 -> 734, 950 -> 871; 4 x 200, 4000 909 -> 728, 1013 -> 903; 5 x 200 927 -> 825; 8 x 200, 500 939 -> 876, 960 -> 923
+//   4 layers: 4, 5, 8 x 200 327 -> 300, 333 -> 319, 340 -> 334; 2: 1, 4, 8 x 200 225 -> 186, 229 -> 216, 241 -> 244 (the launch itself, its barrier and the words of eight tokens)
+//   heads of 128, 96 MiB, 16 layers: 1, 2, 4 x 200 962 -> 585, 974 -> 759, 1000 -> 755; 4 x 3000 1145 -> 1051
 static bool stream_decode(ssdk_engine* e, const Model& m, int B, int q_len, const int32_t* ctx_len) {
   return q_len == 1 && m.d > 1024 && (B <= 4 || m.cfg.layers >= 4) && draft_stream_enabled() && draft_stream_supported(m, B) &&
-         (int64_t)B * (*std::max_element(ctx_len, ctx_len + B) + 1) <= stream_keys(B);
+         stream_pays(e, m, B, *std::max_element(ctx_len, ctx_len + B) + 1);
 }
 template <int HD, int MT>
 static int launch_draft_stream(Launcher& L, const DsParams& p, size_t smem) {

@@ -44,3 +44,39 @@ def test_narrow_drafts_with_long_or_odd_rows_stream(hidden, hd, ffn):
     hard, _ = check_greedy_step(spec, nacc.tolist(), nrec.tolist(), lp_o, lq_o, EPS)
     assert not hard, hard
     r.close()
+
+
+@pytest.mark.parametrize("capacity,far", [(512, 440), (4096, 2100)])
+def test_lengths_of_the_neighbours_do_not_move_a_sequence(capacity, far):
+    """One sequence beside three short or three long ones, in tables of one capacity: the same bits, of a step and of plain decoding, whichever form the capacity picks."""
+    from oracle.model import ModelCfg, random_weights
+    from ssd_b200 import lib as L
+    from ssd_b200.runner import PairRunner
+    dev = torch.device("cuda:0")
+    B, K, bs, n = 4, 4, 64, 40
+    mb = capacity // bs
+    tc = ModelCfg(hidden=256, layers=1, heads=4, kv_heads=2, head_dim=64, ffn=512, vocab=1024, max_pos=capacity)
+    dc = ModelCfg(hidden=1280, layers=2, heads=20, kv_heads=5, head_dim=64, ffn=2560, vocab=1024, max_pos=capacity)
+    wt, wd = _to_dev(random_weights(tc, 31), dev), _to_dev(random_weights(dc, 32), dev)
+    tables = [list(range(b * mb, (b + 1) * mb)) for b in range(B)]
+    seen = []
+    for other in (20, far):
+        lens = [n] + [other - 3 * b for b in range(B - 1)]
+        r = PairRunner(_spec(tc), _spec(dc), spec_k=K, max_batch=B, block_size=bs, max_model_len=capacity, use_graph=True)
+        r.bind_weights(L.TARGET, wt)
+        r.bind_weights(L.DRAFT, wd)
+        r.finalize()
+        g = torch.Generator().manual_seed(9)
+        own = torch.randint(0, 1024, (n,), generator=g).tolist()
+        for b, m in enumerate(lens):
+            prompt = own if b == 0 else torch.randint(0, 1024, (m,), generator=g).tolist()
+            for which in (L.TARGET, L.DRAFT):
+                r.prefill(which, prompt, tables[b], want_sample=False)
+        out = r.forward_tokens(L.DRAFT, [[5 + b] for b in range(B)], lens, tables)
+        token, logits = int(out[0]), r.logits_last(B)[0].clone()
+        toks, _, _ = r.spec_step(lens, [5 + b for b in range(B)], tables, tables, [0.0] * B, [0.0] * B)
+        kv = r.kv[L.DRAFT].reshape(2, dc.layers, -1, dc.kv_heads, dc.head_dim)[:, :, :n + K + 1]
+        seen.append((token, logits, torch.as_tensor(toks[0]), r.logits_q(B)[0].clone(), r.logits_p(B)[0].clone(), kv.clone()))
+        r.close()
+    for a, b in zip(*seen):
+        assert a == b if isinstance(a, int) else torch.equal(a, b)
