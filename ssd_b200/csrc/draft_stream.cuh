@@ -48,9 +48,13 @@ namespace ssdk {
 constexpr int kDsConsumers = 256;                 // threads 0..255: 8 consumer warps
 constexpr int kDsWarps = kDsConsumers / 32;
 constexpr int kDsThreads = kDsConsumers + 128;    // + a warpgroup whose first warp is the producer
-// registers: the block is launched with 384 x 168; the producer's warpgroup gives most of its own to the consumers (heads of 128: keys and values in flight)
+// registers: the block is meant to be launched with 384 x 168; the producer's warpgroup gives most of its own to the consumers (heads of 128: keys and values in flight)
 constexpr int kDsRegsLaunch = 168, kDsRegsProducer = 40, kDsRegsConsumer = 232;
-static_assert(kDsConsumers * kDsRegsConsumer + 128 * kDsRegsProducer <= kDsThreads * kDsRegsLaunch, "register split");
+// whether a kernel that was built with that many registers can be launched: a split above what the block has would wait for ever
+__host__ inline constexpr bool ds_registers_fit(int regs) {
+  return regs >= kDsRegsProducer && regs <= kDsRegsConsumer && kDsConsumers * kDsRegsConsumer + 128 * kDsRegsProducer <= kDsThreads * regs;
+}
+static_assert(ds_registers_fit(kDsRegsLaunch), "register split");
 constexpr int kDsMaxLayers = 32;
 constexpr int kDsMaxBatch = 8;
 constexpr int kDsSplits = 16;         // most ranges of a sequence's keys in stage B

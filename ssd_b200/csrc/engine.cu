@@ -1182,10 +1182,11 @@ __global__ void advance_kernel(int32_t* __restrict__ ctx, int64_t* __restrict__ 
 // streaming draft kernel: the K+1 draft forwards + K samplings of a step in ONE cooperative launch (draft_stream.cuh)
 // SSDK_DRAFT_STREAM=0 keeps the kernel-per-op path.
 // ------------------------------------------------------------------------------------------
+static std::atomic<bool> ds_unfit{false};   // an instance was built with other registers than its split is for (a property of the build): the form stays off
 static bool draft_stream_enabled() {
   static int v = -1;
   if (v < 0) v = env_int("SSDK_DRAFT_STREAM", 1) != 0 ? 1 : 0;
-  return v == 1;
+  return v == 1 && !ds_unfit.load(std::memory_order_acquire);
 }
 // Which calls take the streaming kernel (both forms compute the same; they differ in the order of sums).  A model has a number of tokens per sequence up to which it does.  One sequence: its own tokens
 // decide.  More: the page table's capacity, never the contexts of the moment, so that lengths of the neighbours do not move a sequence's result (their number may, as everywhere).
@@ -1430,10 +1431,10 @@ static int init_kernel_attrs() {
 #undef SSDK_ATTR_P
 #define SSDK_ATTR_D(HD, MT) \
   CK(cudaFuncSetAttribute(draft_stream_kernel<HD, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem)); \
-  { /* (a register split above what the block is launched with would wait for ever) */ \
+  { \
     cudaFuncAttributes a; \
     CK(cudaFuncGetAttributes(&a, draft_stream_kernel<HD, MT>)); \
-    if (a.numRegs != kDsRegsLaunch) return fail("draft_stream_kernel: built with %d registers", a.numRegs); \
+    if (!ds_registers_fit(a.numRegs)) ds_unfit.store(true, std::memory_order_release); \
   }
   SSDK_ATTR_D(64, 1) SSDK_ATTR_D(64, 4) SSDK_ATTR_D(64, 8) SSDK_ATTR_D(128, 1) SSDK_ATTR_D(128, 4) SSDK_ATTR_D(128, 8)
 #undef SSDK_ATTR_D

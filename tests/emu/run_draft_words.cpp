@@ -2,6 +2,7 @@
 // batch of sequences.  TEST INFRASTRUCTURE.
 //   run_draft_words <input blob> <output blob>
 //   run_draft_words <input blob> <output blob> words|copies <n>   in the first of two launches the last CTA's words, or copies of weights, are lost from the n-th on
+//   run_draft_words registers        the launches that the kernel's register split is for
 //   run_draft_words pieces           the attention's weights against the sum of their pieces
 // blob layout: see tests/test_draft_words_emu_cpu.py (the writer).
 #include "cuda_emu.h"
@@ -55,6 +56,11 @@ static int check_pieces() {
 
 int main(int argc, char** argv) {
   if (argc == 2 && std::string(argv[1]) == "pieces") return check_pieces();
+  if (argc == 2 && std::string(argv[1]) == "registers") {   // the numbers of registers that a build may have, up to what a thread can have
+    for (int regs = 0; regs <= 255; ++regs)
+      if (ssdk::ds_registers_fit(regs)) std::cout << regs << "\n";
+    return 0;
+  }
   if (argc != 3 && argc != 5) return 2;
   const bool lose = argc == 5;
   Reader r(argv[1]);

@@ -141,3 +141,11 @@ def test_waits_that_run_out_end_the_launch(tmp_path, lose):
     """What the last CTA sends, or the weights that it fetches, is lost on the way: every wait for it has a limit, the launch ends with its word set, and the next one is right (the
     runner looks at the word, the barrier's count and the range of the tokens behind both)."""
     _check(tmp_path, 64, 1, 2, 512, [40, 300], 0.7, 256, lose=lose)
+
+
+def test_register_split_fits_the_launch():
+    """Eight consumer warps of 232 registers and four warps of 40 come out of what twelve warps are launched with: fewer would wait for ever, and a build with another number turns the
+    form off (it may have more, up to what the split leaves a consumer)."""
+    _build()
+    res = subprocess.run([BIN, "registers"], capture_output=True, text=True, timeout=60)
+    assert [int(x) for x in res.stdout.split()] == list(range((8 * 232 + 4 * 40 + 11) // 12, 233))
