@@ -32,8 +32,9 @@
 // Measured, us a forward of the 1B draft (16 layers, context 203): with device-wide barriers between the stages and one warp per row on CUDA cores 738 (40.8 a layer, 18.6 of them weights at
 // copy bandwidth); tags 705; all reads of a slot in front of its products, which then go in four chains 665; one rolled copy of the code for all stages, which stays in the instruction
 // caches 622; two steps of k per product and missing words asked for again together 552; no
-// first piece asked for alone in front of gate|up's words 532.  What is left, of 28 us a layer: attention 5 (one CTA per key head fetches the keys), the four other
-// exchanges 1.2 each and a wait of up to 2.5 for the CTA whose weights come last, slots at 0.45 (0.73 is the memory's rate).  Contexts of 60 to 8000 tokens and other batches: use_draft_stream (engine.cu).
+// first piece asked for alone in front of gate|up's words 532; a key's place looked up once for a warp 506 (context 135).  Of the 27.8 us of a layer: attention 4.9 (one CTA per key head fetches
+// the keys), the four other exchanges with their norms 1.7 to 2.1 each (the CTA whose weights come last is waited for in them), rows 15.6 (18.6 is the memory's rate; what the ring holds is ahead);
+// the head 72.  (The code has to stay small: a slot's steps written out for every count, or the attention twice, cost more than 4 % though it is not run.)  Contexts of 60 to 8000 tokens and other batches: use_draft_stream (engine.cu).
 //
 // Tags.  tag = forward * L + layer + 1; the words are zeroed at kernel start (a device-wide barrier follows), so no word of another launch is taken for this one's.
 // A word is overwritten only after everybody has read it: with at least one row of every matrix on every CTA (d, ffn, q|k|v and vocabulary >= #CTAs, checked by

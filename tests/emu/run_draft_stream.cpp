@@ -1,6 +1,6 @@
 // Runs the SOURCE of csrc/draft_stream.cuh on host threads (cuda_emu.h).  TEST INFRASTRUCTURE.
-//   run_draft_persistent <input blob> <output blob>
-// blob layout: see tests/test_draft_persistent_emu_cpu.py (the writer).
+//   run_draft_stream <input blob> <output blob>
+// blob layout: see tests/test_draft_stream_emu_cpu.py (the writer).
 #include "cuda_emu.h"
 #define SSDK_HOST_EMU 1
 #include "../../ssd_b200/csrc/draft_stream.cuh"
@@ -95,7 +95,6 @@ int main(int argc, char** argv) {
   p.temp = &temp; p.dyn = nullptr; p.seed = rng[0]; p.call_base = rng[1];
   p.samp_partial = partial.data();
   p.bar_state = sync;
-  p.attn_ticket = sync + 8;
   p.n_slots = n_stages;
   for (int l = 0; l < L; ++l)
     p.layers[l] = ssdk::DsLayer{lw[l].qkv.data(), lw[l].o.data(), lw[l].gate_up.data(), lw[l].down.data(),
@@ -109,15 +108,8 @@ int main(int argc, char** argv) {
     if (rep == 1) {  // second launch: same inputs again (KV rows are simply rewritten with the same values)
       std::fill(tok_buf.begin() + 1, tok_buf.end(), -1);
     }
-    if (hd == 64 && gmax == 4) emu::launch(ssdk::draft_stream_kernel<64, 4>, p, grid, ssdk::kDsThreads, smem);
-    else if (hd == 64) emu::launch(ssdk::draft_stream_kernel<64, 8>, p, grid, ssdk::kDsThreads, smem);
-    else if (gmax == 4) emu::launch(ssdk::draft_stream_kernel<128, 4>, p, grid, ssdk::kDsThreads, smem);
-    else emu::launch(ssdk::draft_stream_kernel<128, 8>, p, grid, ssdk::kDsThreads, smem);
-    for (int i = 2; i < 64; ++i)
-      if (sync[i] != 0) {
-        std::cerr << "attention ticket " << i << " not back to zero\n";
-        return 3;
-      }
+    if (hd == 64) emu::launch(ssdk::draft_stream_kernel<64, 1>, p, grid, ssdk::kDsThreads, smem);   // (the instance of one sequence, as in the product)
+    else emu::launch(ssdk::draft_stream_kernel<128, 1>, p, grid, ssdk::kDsThreads, smem);
     unsigned long long arrivals;
     std::memcpy(&arrivals, sync, 8);
     if (arrivals % (unsigned long long)grid != 0) {

@@ -1,5 +1,5 @@
 """csrc/draft_stream.cuh on host threads with the exchange of the product (tagged words that their readers poll; tests/test_draft_stream_emu_cpu.py runs the
-same source with barriers in their place), for one sequence and for batches of uneven contexts: logits of every forward, keys and values, tokens (greedy and Philox)
+same source with barriers in their place, and only that form), for one sequence and for batches of uneven contexts: logits of every forward, keys and values, tokens (greedy and Philox)
 against the oracle, two launches over the same words.  What it cannot show is the device's memory model and speed."""
 import os
 import shutil
@@ -15,12 +15,16 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SRC = os.path.join(ROOT, "tests", "emu", "run_draft_words.cpp")
 BIN = os.path.join(ROOT, "tests", "emu", "_build", "run_draft_words")
 ASAN = BIN + "_asan"   # every access outside an array of the runner ends the process
+# SSD_B200_TSAN=1: the words' runner with ThreadSanitizer, which reports what two threads touch without an order between them (the words are atomic, and a value travels in its word)
+TSAN = os.environ.get("SSD_B200_TSAN") == "1"
+if TSAN:
+    BIN += "_tsan"
 
 pytestmark = pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++ (C++20)")
 
 
 def _build(binary=BIN):
-    flags = ["-fsanitize=address", "-g"] if binary == ASAN else []
+    flags = ["-fsanitize=address", "-g"] if binary == ASAN else (["-fsanitize=thread", "-g"] if TSAN else [])
     deps = [SRC, os.path.join(ROOT, "tests", "emu", "cuda_emu.h")] + [os.path.join(ROOT, "ssd_b200", "csrc", n) for n in ("draft_stream.cuh", "common.cuh", "sampling.cuh")]
     if os.path.exists(binary) and all(os.path.getmtime(binary) >= os.path.getmtime(d) for d in deps):
         return
@@ -38,7 +42,7 @@ def _check(tmp_path, hd, kv, grid, ffn, ctx, temp, chunk, bs=16, unnamed=(), bin
     _build(binary)
     torch.manual_seed(3)
     B, n_fwd = len(ctx), 2
-    cfg = ModelCfg(hidden=256, layers=1 if ffn > 4096 else 2, heads=256 // hd, kv_heads=kv, head_dim=hd, ffn=ffn, vocab=264, max_pos=512, rms_eps=1e-6, rope_theta=500000.0, qk_norm=hd == 128)
+    cfg = ModelCfg(hidden=256, layers=1 if ffn > 4096 else 2, heads=256 // hd, kv_heads=kv, head_dim=hd, ffn=ffn, vocab=264, max_pos=1024, rms_eps=1e-6, rope_theta=500000.0, qk_norm=hd == 128)
     w = random_weights(cfg, seed=9)
     per = (max(ctx) + n_fwd) // bs + 1
     nblk = B * per
@@ -79,6 +83,7 @@ def _check(tmp_path, hd, kv, grid, ffn, ctx, temp, chunk, bs=16, unnamed=(), bin
         _u16(kv0[1]).tofile(f)
     res = subprocess.run([binary, str(blob), str(out), *lose], capture_output=True, text=True, timeout=600)
     assert res.returncode == 0, res.stderr[-2000:]
+    assert "ThreadSanitizer" not in res.stderr, res.stderr[:3000]
     raw = np.fromfile(out, dtype=np.uint16)
     nl, nc = B * n_fwd * cfg.vocab, cfg.layers * nblk * bs * kv * hd
     bf = torch.from_numpy(raw[:nl + 2 * nc].astype(np.int16)).view(torch.bfloat16)
@@ -112,6 +117,8 @@ def _check(tmp_path, hd, kv, grid, ffn, ctx, temp, chunk, bs=16, unnamed=(), bin
     (64, 1, 2, 512, [300], 0.7, 256),                # two ranges: exchange of partial results; two slots per tile
     (128, 1, 3, 768, [270, 5, 33], 0.0, 256),        # three sequences on the instance of four, three slots per tile
     (64, 2, 2, 512, [9, 255, 256, 1, 30], 0.8, 512), # five: fragments straight from the words; more units than CTAs, contexts around a round of keys
+    (64, 1, 2, 512, [600], 0.0, 512),                # a table of 38 pages, which stays in global memory; ranges of 320 keys, two rounds
+    (64, 1, 2, 5120, [21], 0.7, 2048),               # an intermediate row of four slots of five steps
     (64, 1, 2, 4608, [40, 3, 7], 0.0, 2048),         # an intermediate row too long for the shared memory of four tokens' instance
 ])
 def test_tagged_exchange_matches_the_oracle(tmp_path, hd, kv, grid, ffn, ctx, temp, chunk):

@@ -2,8 +2,8 @@
 and their samplings) against the kernel-per-op path (SSDK_DRAFT_STREAM=0).
 
     python tools/check_draft_stream.py [--temp 0.7] [--prompt-len 3000] [--parallel]
-                                                         # runs the modes in subprocesses and compares; --prompt-len > 1024
-                                                         # exercises the long-context attention (16 KV splits); --parallel
+                                                         # runs the modes in subprocesses and compares; --prompt-len > 4096
+                                                         # gives every range of the attention a second round of keys; --parallel
                                                          # runs the modes at the same time (correctness only, timings mixed)
 
 Workload: a 2-layer target at Llama-3.1-8B dimensions + the full 16-layer Llama-3.2-1B draft (real draft shapes, synthetic

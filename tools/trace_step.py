@@ -88,9 +88,8 @@ def phases(lo, hi, label):
 # streaming draft kernel: phase points of its second forward (ids 64 + point, draft_stream.cuh: ds_mark)
 pts = sorted((all_ts[i], all_ids[i] - 64) for i in range(n) if all_ids[i] >= 64)
 if pts:
-    label = {0: "A prologue done", 1: "A gemv done", 2: "A barrier", 3: "B attention done", 4: "B barrier", 5: "C gemv done",
-             6: "C barrier", 7: "D prologue done", 8: "D gemv done", 9: "D barrier", 10: "E gemv done", 11: "E barrier",
-             12: "probe barrier"}
+    label = {0: "q|k|v operands", 1: "q|k|v rows", 10: "attention", 2: "o operands", 3: "o rows", 4: "gate|up operands", 5: "gate|up rows",
+             6: "down operands", 7: "down rows", 8: "head operands", 9: "head rows"}   # (operands: the words are there, behind a norm normed)
     gaps = collections.defaultdict(lambda: [0, 0.0])
     for (t0, a), (t1, b) in zip(pts, pts[1:]):
         g = gaps[(a, b)]
@@ -100,7 +99,8 @@ if pts:
     tot = 0.0
     for (a, b), (c, us) in sorted(gaps.items()):
         print(f"  {label.get(a, a):>18s} -> {label.get(b, b):<18s} n={c:3d} {us / c:7.2f}")
-        tot += us / c
+        if 8 not in (a, b) and 9 not in (a, b):   # (the head comes once)
+            tot += us / c
     print(f"  per layer {tot:.1f} us; forward span {(pts[-1][0] - pts[0][0]) / 1e3:.1f} us")
 if len(preps) >= 2:
     phases(preps[0], preps[1], "first draft forward")
