@@ -1194,10 +1194,10 @@ static bool draft_stream_enabled() {
 // sequences on that half of the tokens' fragments come from other CTAs' words one chunk at a time.  Steps of k = 4 with a target of one small layer, us, kernels per op -> streaming kernel, sequences x tokens
 // (drafts of 16 layers; MiB of a layer, width, size of a head):
 //   116, 2048, 64: 1 x 200, 2000, 8000 3964 -> 2582, 4256 -> 2836, 4445 -> 3392; 2 x 500, 2000, 4000 4099 -> 3518, 4302 -> 3725, 4435 -> 4109; 3 x 500, 4000 4213 -> 3375, 4644 -> 4111;
-//     4 x 200, 2000, 4000 4307 -> 3349, 4601 -> 3876, 4813 -> 4279; 5 x 200, 750 4298 -> 3897, 4353 -> 4188; 6 x 650 4399 -> 4177; 8 x 200, 500 4414 -> 4211, 4486 -> 4428
+//     4 x 200, 2000, 4000 4307 -> 3349, 4601 -> 3876, 4813 -> 4279; 5 x 200, 750, 1000 4298 -> 3897, 4353 -> 4188, 4394 -> 4316; 6 x 800 4432 -> 4321; 8 x 200, 500, 640 4414 -> 4211, 4486 -> 4428, 4491 -> 4574
 //   88, 1792, 64: 1 x 8000 4997 -> 3504; 2 x 500, 4000 4760 -> 3967, 5016 -> 4418; 4 x 500, 4000 4953 -> 3779, 5278 -> 4339; 5 x 500 4025 -> 4269 (seven steps a slot)
-//   68, 2048, 64: 1 x 200 3595 -> 2093; 2 x 500, 4000 3676 -> 2941, 3993 -> 3448; 4 x 500, 4000 3833 -> 2858, 4299 -> 3680; 8 x 500 3921 -> 3689
-//   44, 2048, 64: 1 x 200, 8000 2608 -> 1938, 3013 -> 2698; 2 x 500 2712 -> 2687; 4 x 500 2765 -> 2767; 5 x 750 3485 -> 2966; 8 x 500 3635 -> 3169
+//   68, 2048, 64: 1 x 200 3595 -> 2093; 2 x 500, 4000 3676 -> 2941, 3993 -> 3448; 4 x 500, 4000 3833 -> 2858, 4299 -> 3680; 8 x 500, 600 3921 -> 3689, 3950 -> 3822
+//   44, 2048, 64: 1 x 200, 8000 2608 -> 1938, 3013 -> 2698; 2 x 500 2712 -> 2687; 4 x 500 2765 -> 2767; 5 x 1000 3520 -> 3101; 8 x 600 3694 -> 3314
 //   48, 1536, 64: 1 x 200, 8000 2691 -> 2206, 3199 -> 2982; 2 x 500 2827 -> 3043; 4 x 200 2892 -> 2847.  45, 1280, 64: 1 x 200, 3000, 8000 2716 -> 2489, 2936 -> 2793, 3159 -> 3232; 2 x 200 2761 -> 3496; 4 x 200 2854 -> 3427
 //   96, 2048, 128: 1 x 200, 8000 4487 -> 2668, 5146 -> 3837; 2 x 500, 4000 4599 -> 3730, 5085 -> 4602; 4 x 200, 2000, 4000 4697 -> 3564, 5157 -> 4471, 5513 -> 5558; 5 x 200 4050 -> 4179
 //   68, 2048, 128: 2 x 500, 2000, 4000 3755 -> 3339, 4056 -> 3574, 4251 -> 4323; 4 x 500, 2000, 3000 3943 -> 3459, 4283 -> 4129, 4495 -> 4678
@@ -1209,7 +1209,7 @@ static int64_t stream_tokens(const Model& m, int B) {
   const int64_t layer = ((int64_t)m.qkv_dim * m.d + (int64_t)m.H * m.hd * m.d + 3ll * m.ffn * m.d) * 2, MiB = 1 << 20;   // bytes of weights
   if (B == 1) return m.d > 1024 ? (layer >= 64 * MiB ? 8192 : 6144) : (m.hd == 128 ? 256 : 1024);
   if (m.d <= 1024) return 0;
-  if (B > 4 && m.hd == 64 && m.d == 8 * kDsConsumers) return 4096 / B;
+  if (B > 4 && m.hd == 64 && m.d == 8 * kDsConsumers) return 5120 / B;
   if (layer < 64 * MiB) return m.cfg.layers > 4 ? 0 : (B > 4 ? 512 : 1024);
   if (B > 4) return 0;
   return m.hd == 64 || layer >= 96 * MiB ? 4096 : 2048;
@@ -1226,7 +1226,7 @@ static bool use_draft_stream(ssdk_engine* e, int B, int ctx_bound) {
   return forced >= 0 ? tokens <= forced : stream_pays(e, m, B, tokens);
 }
 // One token per sequence of plain decoding, by the same numbers: a forward is one launch instead of nine per layer, and no graph.  The 1B model (116 MiB), us a call with its token:
-//   16 layers: 1 x 200, 2000, 7000 852 -> 571, 890 -> 624, 940 -> 721; 2 x 200, 4000 873 -> 734, 950 -> 871; 4 x 200, 4000 909 -> 728, 1013 -> 903; 5 x 200 927 -> 825; 8 x 200, 500 939 -> 876, 960 -> 923
+//   16 layers: 1 x 200, 2000, 7000 852 -> 571, 890 -> 624, 940 -> 721; 2 x 200, 4000 873 -> 734, 950 -> 871; 4 x 200, 4000 909 -> 728, 1013 -> 903; 5 x 200, 1000 927 -> 825, 950 -> 908; 8 x 200, 600 939 -> 876, 960 -> 948
 //   4 layers: 4, 5, 8 x 200 327 -> 300, 333 -> 319, 340 -> 334; 2: 1, 4, 8 x 200 225 -> 186, 229 -> 216, 241 -> 244 (the launch itself, its barrier and the words of eight tokens)
 //   heads of 128, 96 MiB, 16 layers: 1, 2, 4 x 200 962 -> 585, 974 -> 759, 1000 -> 755; 4 x 3000 1145 -> 1051
 static bool stream_decode(ssdk_engine* e, const Model& m, int B, int q_len, const int32_t* ctx_len) {
