@@ -435,6 +435,24 @@ SSDK_DEVINL uint32_t ld_relaxed_gpu_u32(const uint32_t* p) {
 }
 
 #else  // SSDK_HOST_EMU: host stand-ins for the few PTX helpers the emulated kernels use
+}  // namespace ssdk
+namespace emu {
+// A thread that asks for an address again sleeps: some hundred pollers that only yield, or sleep for a few microseconds, take all cores from the threads that they wait for.
+inline void polled(const void* p) {
+  thread_local const void* last[64];
+  thread_local unsigned n = 0;
+  for (const void* q : last)
+    if (q == p) {
+      std::this_thread::sleep_for(std::chrono::microseconds(500));
+      return;
+    }
+  last[n++ % 64] = p;
+}
+// failures that a test asks for: of the last CTA, what follows the n-th word it stores or copy it makes (-1: none) is lost
+inline std::atomic<int> lost_words{-1}, lost_copies{-1};
+inline bool lost(std::atomic<int>& left) { return blockIdx.x + 1 == gridDim.x && left.load() >= 0 && left.fetch_sub(left.load() > 0 ? 1 : 0) == 0; }
+}  // namespace emu
+namespace ssdk {
 enum { TR_PREP = 1, TR_NORM, TR_GEMM, TR_ROPE, TR_ATTN, TR_SAMPLE, TR_VERIFY, TR_MISC };
 enum { TRF_ATTN = 16, TRF_NORM = 24, TRF_ROPE = 32, TRF_COMB = 40, TRF_GEMM = 48 };
 SSDK_DEVINL void trace_mark(int) {}
@@ -558,7 +576,15 @@ SSDK_DEVINL uint32_t __byte_perm(uint32_t a, uint32_t b, uint32_t sel) {
 }
 SSDK_DEVINL void mma_bf16_16816(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
   emu::Warp* x = emu::tctx.cta->warps[threadIdx.x >> 5].get();
-  uint32_t* mine = x->operands[threadIdx.x & 31];
+  struct Words { uint32_t w[32][6]; };
+  static std::mutex mu;
+  static std::map<emu::Warp*, Words> all;   // (a warp's place may be another launch's later: all of it is written anew by every product)
+  thread_local Words* operands = nullptr;   // (a thread belongs to one warp)
+  if (!operands) {
+    std::lock_guard<std::mutex> lock(mu);
+    operands = &all[x];
+  }
+  uint32_t* mine = operands->w[threadIdx.x & 31];
   for (int i = 0; i < 4; ++i) mine[i] = a[i];
   mine[4] = b0; mine[5] = b1;
   x->bar.arrive_and_wait();
@@ -568,7 +594,7 @@ SSDK_DEVINL void mma_bf16_16816(float* c, const uint32_t* a, uint32_t b0, uint32
     const int row = g, hi = e >> 1, col = 2 * t + (e & 1);   // rows behind the eighth: A's odd words
     for (int k = 0; k < 16; ++k) {
       const int lane_k = (k & 7) >> 1, part = k >> 3;
-      c[e] += val(x->operands[row * 4 + lane_k][2 * part + hi], k & 1) * val(x->operands[col * 4 + lane_k][4 + part], k & 1);
+      c[e] += val(operands->w[row * 4 + lane_k][2 * part + hi], k & 1) * val(operands->w[col * 4 + lane_k][4 + part], k & 1);
     }
   }
   x->bar.arrive_and_wait();

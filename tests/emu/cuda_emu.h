@@ -68,7 +68,7 @@ using std::min;
 
 namespace emu {
 struct Warp {
-  uint32_t slot[32], operands[32][6];   // of shuffles; of mma
+  uint32_t slot[32];
   std::barrier<> bar{32};
 };
 struct Cta {
@@ -143,24 +143,6 @@ inline T __shfl_xor_sync(unsigned, T v, int lane_mask) {
   w.bar.arrive_and_wait();
   return r;
 }
-namespace emu {
-// A thread that asks for an address again sleeps: some hundred pollers that only yield, or sleep for a few microseconds, take all cores from the threads that they wait for.
-inline void polled(const void* p) {
-  thread_local const void* last[64];
-  thread_local unsigned n = 0;
-  for (const void* q : last)
-    if (q == p) {
-      std::this_thread::sleep_for(std::chrono::microseconds(500));
-      return;
-    }
-  last[n++ % 64] = p;
-}
-}  // namespace emu
-namespace emu {
-// failures that a test asks for: of the last CTA, what follows the n-th word it stores or copy it makes (-1: none) is lost
-inline std::atomic<int> lost_words{-1}, lost_copies{-1};
-inline bool lost(std::atomic<int>& left) { return blockIdx.x + 1 == gridDim.x && left.load() >= 0 && left.fetch_sub(left.load() > 0 ? 1 : 0) == 0; }
-}  // namespace emu
 inline unsigned atomicAdd(unsigned* p, unsigned v) { return __atomic_fetch_add(p, v, __ATOMIC_SEQ_CST); }
 template <typename T>
 inline T __ldcg(const T* p) { return *p; }

@@ -3,7 +3,8 @@ persistent launch) compiled for the host with tests/emu/cuda_emu.h — one OS th
 real warp shuffles, the real device-wide barrier, mbarrier / bulk-copy stand-ins — and checked against the pinned oracle:
 logits of every forward, the KV rows written, the greedy tokens chained INSIDE the launch, and (temp > 0) the Philox
 exponential-race tokens against oracle.verify.sample on the kernel's own logits.  This executes the kernel's own C++
-(job sequence per CTA, ring slot / parity arithmetic, stage geometry for K <= 2048 / 4096 / 8192, barrier placement);
+(rows of a CTA, ring slot / parity arithmetic, rows of one to four slots, barrier placement; with a device-wide barrier in the
+place of the exchanged words, which tests/test_draft_words_emu_cpu.py runs);
 what it cannot show is device-only behaviour (async-proxy ordering, occupancy, speed)."""
 import os
 import shutil
@@ -43,15 +44,14 @@ def _u16(t):
 
 
 @pytest.mark.parametrize("family,grid,dims,temp,n_fwd,n,bs", [
-    ("llama", 3, (256, 512), 0.0, 3, 21, 16),     # K = 256 / 512: 8 rows per job, one slot (gate|up: 8 pairs, two slots)
+    ("llama", 3, (256, 512), 0.0, 3, 21, 16),     # rows of one slot
     ("qwen", 2, (256, 512), 0.8, 3, 270, 64),     # q/k norm, head_dim 128, Philox sampling in the kernel; context > 256:
-                                                  # 16 KV splits per head (head_dim 128), partials + ticket + merge by the last split
-    ("llama", 3, (256, 4096), 0.0, 2, 21, 16),    # down-proj K = 4096: 4 rows x 2 segments per job
-    ("llama", 2, (256, 5120), 0.7, 2, 21, 16),    # down-proj K = 5120: 2 rows x 4 segments per job
-    ("llama", 3, (256, 512), 0.0, 2, 1100, 64),   # 16 KV splits per head, 8 tokens per warp iteration, two load rounds per split,
-                                                  # several attention units per CTA
-    ("llama", 2, (256, 512), 0.0, 4, 254, 16),    # context 255 .. 258 inside ONE launch: the forwards switch from 8 KV splits
-                                                  # (4 tokens per warp iteration) to 16 splits (8 tokens) at 257 tokens
+                                                  # two ranges per head, partial results and merge
+    ("llama", 3, (256, 4096), 0.0, 2, 21, 16),    # down-proj rows of two slots; a table of 40 pages in global memory
+    ("llama", 2, (256, 5120), 0.7, 2, 21, 16),    # down-proj rows of four slots
+    ("llama", 3, (256, 512), 0.0, 2, 1100, 64),   # five ranges per head, several attention units per CTA
+    ("llama", 2, (256, 512), 0.0, 4, 254, 16),    # context 255 .. 258 inside ONE launch: the forwards switch from one range
+                                                  # to two at 257 tokens
 ])
 def test_draft_stream_kernel_source_on_host_threads(tmp_path, family, grid, dims, temp, n_fwd, n, bs):
     from oracle import verify as V

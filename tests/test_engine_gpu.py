@@ -357,11 +357,11 @@ def test_packed_prefill_of_ragged_prompts_matches_oracle():
 
 
 def test_spec_steps_across_the_draft_path_switch_match_oracle():
-    """The step graph takes the streaming draft kernel while the context fits one load round of its attention phase
-    (<= 1024 tokens incl. the K+1 new ones) and the kernel-per-op draft beyond (use_draft_stream, csrc/engine.cu).  A
+    """The step graph of a narrow draft takes the streaming kernel up to 1024 tokens incl. the K+1 new ones and the
+    kernel-per-op draft beyond (stream_tokens, csrc/engine.cu).  A
     sequence that starts at 1012 tokens crosses the limit within ten steps: every step — whichever graph ran it, and the
     KV the other one left behind — must agree with the oracle (teacher-forced, near-tie protocol); the contexts in between
-    also run the 16-split layout of the streaming kernel's attention (> 256 tokens)."""
+    also run several ranges of the streaming kernel's attention."""
     from oracle.model import ModelCfg, OracleModel, random_weights
     from oracle.spec import SpecSession, check_greedy_step, contiguous_block_tables
     from ssd_b200 import lib as L
